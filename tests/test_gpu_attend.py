@@ -61,3 +61,28 @@ def test_attend_rows_without_winners_and_bad_arguments():
     with pytest.raises(S.SlhaError) as e:
         S.attend_topk(idx, sc, k, 0.25, values, d_v)  # host values
     assert e.value.code == S.ERR_DEVICE
+
+
+@pytest.mark.parametrize("d_v,stride,shift,bf16,k", [(128, 128, 0, True, 2048), (128, 136, 1, True, 100), (130, 130, 0, True, 9), (2104, 2104, 0, True, 33),
+                                                     (7, 9, 0, False, 1), (128, 132, 0, False, 700), (128, 128, 1, False, 65), (1100, 1100, 0, False, 17)])
+def test_attend_takes_any_row_length_stride_and_alignment(d_v, stride, shift, bf16, k):
+    # 16-byte loads where rows allow them, single elements elsewhere; more than 256 vectors per row take a second sweep
+    n, nq = 3000, 3
+    rng = np.random.default_rng(d_v + k)
+    values = rng.standard_normal((n, d_v)).astype(F)
+    if bf16:
+        values = H.to_bf16_f32(values).reshape(n, d_v)
+    esz = 2 if bf16 else 4
+    flat = np.zeros(n * stride + shift, np.uint16 if bf16 else F)
+    rows = flat[shift:].reshape(n, stride)
+    rows[:, :d_v] = (values.view(np.uint32) >> 16).astype(np.uint16) if bf16 else values
+    buf = S.to_device(flat)
+    idx = np.stack([rng.permutation(n)[:k] for _ in range(nq)]).astype(np.uint32)
+    idx[1, ::3] = 0xFFFFFFFF
+    sc = (10.0 * rng.standard_normal((nq, k))).astype(F)
+    cnt = np.array([k, k, k // 2], np.uint32)
+    w_out = np.zeros((nq, k), F)
+    out = S.attend_topk(idx, sc, k, 0.1, buf.view(shift * esz, flat.nbytes - shift * esz), d_v, value_dtype=S.BF16 if bf16 else S.F32, top_count=cnt,
+                        value_row_stride=stride, weights_out=w_out)
+    want, want_w = ora.attend_topk(idx, sc, 0.1, values, top_count=cnt)
+    assert close(w_out, want_w) and close(out, want)
