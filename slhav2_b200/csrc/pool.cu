@@ -319,6 +319,46 @@ __global__ void phase_commit_kernel(PoolDev p) {
 // A phase the select cannot bound (a deficit worth more than EB_CAP operations) raises `overflow`
 // and ends the kernel; the phases already finished are complete, and the host-driven path then
 // continues from the state they left (a finished phase has no candidates left or met the budget).
+constexpr int EB_BATCH = 4;  // slots a thread of the scans looks at together
+// phase_key of the slots s0, s0 + stride, .. (EB_BATCH of them), the loads of all of them in flight together
+__device__ __forceinline__ void phase_keys(const PoolDev& p, int phase, uint64_t s0, uint64_t stride, uint64_t len, uint32_t max_pos, uint64_t (&key)[EB_BATCH]) {
+    uint8_t st[EB_BATCH];
+#pragma unroll
+    for (int u = 0; u < EB_BATCH; ++u) st[u] = s0 + u * stride < len ? p.state[s0 + u * stride] : ST_COLD;
+    const bool evict = phase >= PH_EVICT;
+    const uint8_t only = phase == PH_CORR_WARM ? ST_WARM : ST_HOT;  // (the other phases act on every live slot)
+    uint2 pf[EB_BATCH];       // position, head | flags
+    uint32_t seq[EB_BATCH];
+    float imp[EB_BATCH];      // importance (eviction), sigma (paging)
+#pragma unroll
+    for (int u = 0; u < EB_BATCH; ++u) {
+        const uint64_t s = s0 + u * stride;
+        const bool look = evict ? st[u] != ST_COLD : st[u] == only;
+        pf[u] = make_uint2(0u, 0u);
+        seq[u] = 0u;
+        imp[u] = 0.0f;
+        if (look) {
+            const unsigned char* t = p.tiles + s * TILE_BYTES;
+            pf[u] = *reinterpret_cast<const uint2*>(t + 112);
+            seq[u] = (uint32_t)p.seq[s];
+            imp[u] = evict ? p.importance[s] : *reinterpret_cast<const float*>(t + 104);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < EB_BATCH; ++u) {
+        key[u] = SENTINEL;
+        const uint32_t flags = pf[u].y >> 16;
+        if (evict) {
+            if (st[u] == ST_COLD) continue;
+            const bool pin = p.evict_policy == SLHA_B200_EVICT_IMPORTANCE && is_pinned(p, pf[u].x, max_pos);
+            if ((phase == PH_EVICT_PINNED) != pin) continue;
+            key[u] = p.evict_policy == SLHA_B200_EVICT_CAUSAL ? (uint64_t)seq[u] : ((uint64_t)f32_total_key(imp[u]) << 32) | seq[u];
+        } else {
+            if (st[u] != only || (phase != PH_PAGE && (!corr_bytes(flags) || (flags & F_NOCORR)))) continue;
+            key[u] = p.page_policy == SLHA_B200_PAGE_LOWEST_IMPACT_FIRST ? ((uint64_t)f32_total_key(imp[u]) << 32) | (uint32_t)(s0 + u * stride) : (uint64_t)seq[u];
+        }
+    }
+}
 constexpr int EB_THREADS = 512, EB_ITEMS = 8, EB_CAP = EB_THREADS * EB_ITEMS, EB_LEVELS = 6, EB_BINS = 4096;
 struct EnforceState {
     unsigned long long inv_min_key, max_key;  // ~min and max over the phase's candidates (zero = none yet)
@@ -338,6 +378,7 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
         typename Scan64::TempStorage scan64;
         typename Scan32::TempStorage scan32;
         uint32_t hist[EB_BINS];
+        struct { uint64_t in[EB_THREADS], key[EB_THREADS]; uint32_t val[EB_THREADS]; } few;
     } sm;
     __shared__ uint32_t cut_bin, cut_hist;
     __shared__ unsigned long long cut_cum, fin_applied;
@@ -347,12 +388,29 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
     const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
     const int lane = threadIdx.x & 31;
     if (cnt->live <= cnt->budget) return;  // (nothing has been written yet: every block sees the same)
+    __shared__ uint32_t warp_n[EB_THREADS / 32], block_base;
+    __shared__ unsigned long long block_min_inv, block_max;
+    const int warp = threadIdx.x >> 5;
     if (p.recent_window) {
         uint32_t m = 0;
-        for (uint64_t s = gtid; s < len; s += stride)
-            if (p.state[s] != ST_COLD) m = max(m, *reinterpret_cast<const uint32_t*>(p.tiles + s * TILE_BYTES + 112));
-        for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-        if (lane == 0 && m) atomicMax(&p.cnt->max_pos, m);
+        for (uint64_t s0 = gtid; s0 < len; s0 += EB_BATCH * stride) {  // (the loads of a batch are in flight together)
+            uint8_t st[EB_BATCH];
+            uint32_t pos[EB_BATCH];
+#pragma unroll
+            for (int u = 0; u < EB_BATCH; ++u) st[u] = s0 + u * stride < len ? p.state[s0 + u * stride] : ST_COLD;
+#pragma unroll
+            for (int u = 0; u < EB_BATCH; ++u)
+                pos[u] = st[u] != ST_COLD ? *reinterpret_cast<const uint32_t*>(p.tiles + (s0 + u * stride) * TILE_BYTES + 112) : 0u;
+#pragma unroll
+            for (int u = 0; u < EB_BATCH; ++u) m = max(m, pos[u]);
+        }
+        m = __reduce_max_sync(0xFFFFFFFFu, m);
+        if (lane == 0) warp_n[warp] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < EB_THREADS / 32; ++w) m = max(m, warp_n[w]);
+            if (m) atomicMax(&p.cnt->max_pos, m);
+        }
         grid.sync();
     }
     const uint32_t max_pos = cnt->max_pos;
@@ -363,33 +421,61 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
         const uint64_t deficit = live - budget;
         // ---- build
         {
+            // One reservation per block and batch, one minimum and maximum per block: an atomic per warp on the same word
+            // costs more than the scan itself (32 k of them for a million slots).
             uint64_t kmin = SENTINEL, kmax = 0;
-            const uint64_t rounds = (len + stride - 1) / stride;
-            for (uint64_t r = 0; r < rounds; ++r) {
-                const uint64_t s = r * stride + gtid;
-                uint64_t key = SENTINEL;
-                if (s < len) key = phase_key(p, phase, s, max_pos);
-                const unsigned hit = __ballot_sync(0xFFFFFFFFu, key != SENTINEL);
-                if (hit) {
-                    uint32_t base = 0;
-                    if (lane == 0) base = atomicAdd(&p.cnt->n_cand, (uint32_t)__popc(hit));
-                    base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                    if (key != SENTINEL) {
-                        const uint32_t i = base + (uint32_t)__popc(hit & ((1u << lane) - 1u));
-                        keys[i] = key;
-                        vals[i] = (uint32_t)s;
-                        kmin = min(kmin, key);
-                        kmax = max(kmax, key);
-                    }
+            const uint64_t batches = (len + EB_BATCH * stride - 1) / (EB_BATCH * stride);
+            for (uint64_t r = 0; r < batches; ++r) {
+                const uint64_t s0 = r * EB_BATCH * stride + gtid;
+                uint64_t key[EB_BATCH];
+                phase_keys(p, phase, s0, stride, len, max_pos, key);
+                uint32_t mine = 0;
+#pragma unroll
+                for (int u = 0; u < EB_BATCH; ++u) mine += key[u] != SENTINEL;
+                uint32_t incl = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += y;
                 }
+                if (lane == 31) warp_n[warp] = incl;
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    uint32_t tot = 0;
+                    for (int w = 0; w < EB_THREADS / 32; ++w) {
+                        const uint32_t x = warp_n[w];
+                        warp_n[w] = tot;
+                        tot += x;
+                    }
+                    block_base = tot ? atomicAdd(&p.cnt->n_cand, tot) : 0u;
+                }
+                __syncthreads();
+                uint32_t at = block_base + warp_n[warp] + incl - mine;
+#pragma unroll
+                for (int u = 0; u < EB_BATCH; ++u)
+                    if (key[u] != SENTINEL) {
+                        keys[at] = key[u];
+                        vals[at] = (uint32_t)(s0 + u * stride);
+                        ++at;
+                        kmin = min(kmin, key[u]);
+                        kmax = max(kmax, key[u]);
+                    }
+                __syncthreads();  // (the counts are reused by the next batch)
             }
             for (int o = 16; o; o >>= 1) {
                 kmin = min(kmin, __shfl_xor_sync(0xFFFFFFFFu, kmin, o));
                 kmax = max(kmax, __shfl_xor_sync(0xFFFFFFFFu, kmax, o));
             }
+            if (threadIdx.x == 0) block_min_inv = block_max = 0ull;
+            __syncthreads();
             if (lane == 0 && kmin != SENTINEL) {
-                atomicMax(&es->inv_min_key, ~kmin);
-                atomicMax(&es->max_key, kmax);
+                atomicMax(&block_min_inv, (unsigned long long)~kmin);
+                atomicMax(&block_max, (unsigned long long)kmax);
+            }
+            __syncthreads();
+            if (threadIdx.x == 0 && block_min_inv) {
+                atomicMax(&es->inv_min_key, block_min_inv);
+                atomicMax(&es->max_key, block_max);
             }
         }
         grid.sync();
@@ -499,7 +585,29 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
                     fin_delta = 0;
                 }
                 __syncthreads();
-                Sort(sm.sort).Sort(k, v);
+                if (n <= EB_THREADS) {
+                    // few candidates (a decode step's page-outs and evictions): every thread counts the keys below its own
+                    // (keys are unique), n reads of shared memory instead of the radix sort's sixteen passes
+                    const uint32_t i = threadIdx.x;
+                    const uint64_t own = i < n ? ks[i] : SENTINEL;
+                    sm.few.in[i] = own;
+                    __syncthreads();
+                    uint32_t rank = 0;
+#pragma unroll 8
+                    for (uint32_t e = 0; e < n; ++e) rank += sm.few.in[e] < own;
+                    if (i < n) {
+                        sm.few.key[rank] = own;
+                        sm.few.val[rank] = vs[i];
+                    }
+                    __syncthreads();
+                    for (int j = 0; j < EB_ITEMS; ++j) {
+                        const uint32_t e = threadIdx.x * EB_ITEMS + j;
+                        k[j] = e < n ? sm.few.key[e] : SENTINEL;
+                        v[j] = e < n ? sm.few.val[e] : 0u;
+                    }
+                } else {
+                    Sort(sm.sort).Sort(k, v);
+                }
                 __syncthreads();
                 uint64_t w[EB_ITEMS], excl[EB_ITEMS];
                 for (int j = 0; j < EB_ITEMS; ++j) {
@@ -560,27 +668,46 @@ struct ObserveTmp {
     uint32_t pad;
     float sum;
 };
-__global__ void observe_pass1(PoolDev p, const uint32_t* slots, const float* scores, uint64_t n, ObserveTmp* tmp) {
-    const uint64_t len = p.cnt->len;
+// (one set of atomics per CTA, and a grid of a few CTAs per SM: an atomic per warp on the same words costs more than the scan)
+__global__ void __launch_bounds__(256) observe_pass1(PoolDev p, const uint32_t* slots, const float* scores, uint64_t n, ObserveTmp* tmp) {
+    __shared__ uint32_t red[3];
+    if (threadIdx.x < 3) red[threadIdx.x] = 0u;
+    __syncthreads();
+    const uint64_t len = p.cnt->len, stride = (uint64_t)gridDim.x * blockDim.x;
     uint32_t mk = 0, bad = 0, live = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t s = slots ? slots[i] : (uint32_t)i;
-        if (s < len && p.state[s] != ST_COLD) {
-            const float v = scores[i];
-            ++live;
-            if (!isfinite(v)) bad = 1;
-            mk = max(mk, f32_total_key(v));
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
+        uint64_t s[4];
+        float v[4];
+        uint8_t st[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t i = i0 + u * stride;
+            s[u] = i < n ? (slots ? slots[i] : i) : len;
+            v[u] = i < n ? scores[i] : 0.0f;
         }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) st[u] = s[u] < len ? p.state[s[u]] : ST_COLD;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (st[u] != ST_COLD) {
+                ++live;
+                if (!isfinite(v[u])) bad = 1;
+                mk = max(mk, f32_total_key(v[u]));
+            }
     }
-    for (int o = 16; o; o >>= 1) {
-        mk = max(mk, __shfl_xor_sync(0xFFFFFFFFu, mk, o));
-        bad |= __shfl_xor_sync(0xFFFFFFFFu, bad, o);
-        live += __shfl_xor_sync(0xFFFFFFFFu, live, o);
-    }
+    mk = __reduce_max_sync(0xFFFFFFFFu, mk);
+    bad = __reduce_or_sync(0xFFFFFFFFu, bad);
+    live = __reduce_add_sync(0xFFFFFFFFu, live);
     if ((threadIdx.x & 31) == 0) {
-        atomicMax(&tmp->max_key, mk);
-        if (bad) atomicOr(&tmp->bad, 1u);
-        if (live) atomicAdd(&tmp->live, live);
+        atomicMax(&red[0], mk);
+        if (bad) atomicOr(&red[1], 1u);
+        atomicAdd(&red[2], live);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0 && red[2]) {
+        atomicMax(&tmp->max_key, red[0]);
+        if (red[1]) atomicOr(&tmp->bad, 1u);
+        atomicAdd(&tmp->live, red[2]);
     }
 }
 __device__ __forceinline__ float key_to_f32(uint32_t k) {
@@ -596,9 +723,21 @@ __global__ void observe_pass2(PoolDev p, const uint32_t* slots, const float* sco
     if (!tmp->bad && tmp->live) {
         const uint64_t per = (n + gridDim.x - 1) / gridDim.x;
         const uint64_t lo = (uint64_t)blockIdx.x * per, hi = min(n, lo + per);
-        for (uint64_t i = lo + threadIdx.x; i < hi; i += blockDim.x) {
-            const uint32_t s = slots ? slots[i] : (uint32_t)i;
-            if (s < len && p.state[s] != ST_COLD) acc += expf((scores[i] - m) / temperature);
+        for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += 4 * blockDim.x) {  // (four entries' loads in flight, added in order)
+            uint64_t s[4];
+            float v[4];
+            uint8_t st[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint64_t i = i0 + u * blockDim.x;
+                s[u] = i < hi ? (slots ? slots[i] : (uint32_t)i) : len;
+                v[u] = i < hi ? scores[i] : 0.0f;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) st[u] = s[u] < len ? p.state[s[u]] : ST_COLD;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (st[u] != ST_COLD) acc += expf((v[u] - m) / temperature);
         }
     }
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
@@ -612,42 +751,73 @@ __global__ void observe_pass2(PoolDev p, const uint32_t* slots, const float* sco
 }
 __global__ void observe_pass3(PoolDev p, const uint32_t* slots, const float* scores, uint64_t n,
                               float temperature, ObserveTmp* tmp, const float* partial, int n_partial) {
-    __shared__ float s_inv;
+    __shared__ float s_inv, part[256];
+    for (int i = threadIdx.x; i < n_partial; i += blockDim.x) part[i] = partial[i];  // (n_partial <= 256)
+    __syncthreads();
     if (threadIdx.x == 0) {
         float sum = 0.0f;
-        for (int i = 0; i < n_partial; ++i) sum += partial[i];
+#pragma unroll 16
+        for (int i = 0; i < n_partial; ++i) sum += part[i];
         s_inv = (tmp->bad || !tmp->live || !isfinite(sum) || sum <= 0.0f) ? 0.0f : 1.0f / sum;
     }
     __syncthreads();
     const float inv = s_inv;
     if (inv == 0.0f) return;
-    const uint64_t len = p.cnt->len;
+    const uint64_t len = p.cnt->len, stride = (uint64_t)gridDim.x * blockDim.x;
     const float m = key_to_f32(tmp->max_key);
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t s = slots ? slots[i] : (uint32_t)i;
-        if (s < len && p.state[s] != ST_COLD) atomicAdd(&p.importance[s], expf((scores[i] - m) / temperature) * inv);
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += 4 * stride) {
+        uint64_t s[4];
+        float v[4], old[4];
+        uint8_t st[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint64_t i = i0 + u * stride;
+            s[u] = i < n ? (slots ? slots[i] : (uint32_t)i) : len;
+            v[u] = i < n ? scores[i] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            st[u] = s[u] < len ? p.state[s[u]] : ST_COLD;
+            old[u] = !slots && s[u] < len ? p.importance[s[u]] : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (st[u] != ST_COLD) {
+                const float w = expf((v[u] - m) / temperature) * inv;
+                if (slots) atomicAdd(&p.importance[s[u]], w);  // (a caller's list may name a slot twice)
+                else p.importance[s[u]] = __fadd_rn(old[u], w);
+            }
     }
 }
 
 // ---- stats / compaction ---------------------------------------------------------
-__global__ void stats_kernel(PoolDev p, unsigned long long* out) {
-    const uint64_t len = p.cnt->len;
-    unsigned long long h = 0, w = 0, c = 0, nc = 0, rec = 0;
-    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < len; s += (uint64_t)gridDim.x * blockDim.x) {
-        const uint8_t st = p.state[s];
-        if (st == ST_HOT) ++h; else if (st == ST_WARM) ++w; else ++c;
-        const uint32_t flags = tile_flags(p.tiles, s);
-        if (st != ST_COLD && (flags & F_NOCORR)) { ++nc; rec += corr_bytes(flags); }
+__global__ void __launch_bounds__(256) stats_kernel(PoolDev p, unsigned long long* out, bool planes) {
+    __shared__ uint32_t red[5];
+    if (threadIdx.x < 5) red[threadIdx.x] = 0u;
+    __syncthreads();
+    const uint64_t len = p.cnt->len, stride = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t v[5] = {0, 0, 0, 0, 0};  // hot, warm, cold, without correction plane, bytes it gave back (per thread: below 2^32 slots)
+    for (uint64_t s0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s0 < len; s0 += 4 * stride) {
+        uint8_t st[4];
+        uint32_t flags[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) st[u] = s0 + u * stride < len ? p.state[s0 + u * stride] : 0xFFu;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) flags[u] = planes && (st[u] == ST_HOT || st[u] == ST_WARM) ? tile_flags(p.tiles, s0 + u * stride) : 0u;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            if (st[u] == 0xFFu) continue;
+            ++v[st[u] == ST_HOT ? 0 : (st[u] == ST_WARM ? 1 : 2)];
+            if (flags[u] & F_NOCORR) { ++v[3]; v[4] += corr_bytes(flags[u]); }
+        }
     }
-    for (int o = 16; o; o >>= 1) {
-        h += __shfl_xor_sync(0xFFFFFFFFu, h, o); w += __shfl_xor_sync(0xFFFFFFFFu, w, o);
-        c += __shfl_xor_sync(0xFFFFFFFFu, c, o); nc += __shfl_xor_sync(0xFFFFFFFFu, nc, o);
-        rec += __shfl_xor_sync(0xFFFFFFFFu, rec, o);
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const uint32_t t = __reduce_add_sync(0xFFFFFFFFu, v[i]);
+        if ((threadIdx.x & 31) == 0 && t) atomicAdd(&red[i], t);
     }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&out[2], h); atomicAdd(&out[3], w); atomicAdd(&out[4], c);
-        atomicAdd(&out[5], nc); atomicAdd(&out[6], rec);
-    }
+    __syncthreads();
+    if (threadIdx.x < 5 && red[threadIdx.x]) atomicAdd(&out[2 + threadIdx.x], (unsigned long long)red[threadIdx.x]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         out[0] = p.cnt->len; out[1] = p.cnt->live; out[7] = p.cnt->free_len;
     }
@@ -991,9 +1161,10 @@ Status pool_observe(Ctx* c, Pool* pl, const uint32_t* d_slots, const float* d_sc
     ObserveTmp* tmp = reinterpret_cast<ObserveTmp*>(pl->d_observe);
     float* partial = reinterpret_cast<float*>(tmp + 1);
     SLHA_CUDA(cudaMemsetAsync(tmp, 0, sizeof(ObserveTmp), c->stream));
-    observe_pass1<<<grid_for(n), 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, tmp);
+    const uint32_t grid = std::min<uint32_t>(grid_for(n), 148 * 4);
+    observe_pass1<<<grid, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, tmp);
     observe_pass2<<<nparts, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial);
-    observe_pass3<<<grid_for(n), 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial, nparts);
+    observe_pass3<<<grid, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial, nparts);
     count_launch(3);
     SLHA_CUDA(cudaGetLastError());
     return Status();
@@ -1003,7 +1174,10 @@ Status pool_stats(Ctx* c, Pool* pl, uint64_t out[8]) {
     unsigned long long* d;
     SLHA_TRY(ctx_device_scratch(c, 256, (void**)&d));
     SLHA_CUDA(cudaMemsetAsync(d, 0, 64, c->stream));
-    stats_kernel<<<grid_for(std::max<uint64_t>(pl->h_cnt.len, 1)), 256, 0, c->stream>>>(pl->dev, d);
+    // (a pool that has only ever been appended to with codecs without a correction plane holds no tile that dropped one)
+    const uint32_t cm = pl->codec_mask;
+    const bool planes = !cm || (cm & (0x80000000u | (1u << SLHA_CODEC_TQ3) | (1u << SLHA_CODEC_MIX3)));
+    stats_kernel<<<std::min<uint32_t>(grid_for(std::max<uint64_t>(pl->h_cnt.len, 1)), 148 * 4), 256, 0, c->stream>>>(pl->dev, d, planes);
     count_launch();
     SLHA_CUDA(cudaGetLastError());
     SLHA_CUDA(cudaMemcpyAsync(out, d, 64, cudaMemcpyDeviceToHost, c->stream));
