@@ -40,6 +40,7 @@ struct EncodeArgs {
     const uint32_t* slots;   // optional scatter: tile i goes to tiles[slots[i]]
     float* q_coarse;         // [n][128]  (query mode)
     uint64_t* q_sign;        // [n][4]    (query mode)
+    uint64_t one;            // (1.0f, 1.0f): the compiler must not know it (see add2)
     int kb;                  // keys per CTA pass (power of two, <= 16)
 };
 
@@ -256,27 +257,35 @@ __device__ __forceinline__ void load_keys(float (&v)[NK], const float* src) {
     }
 }
 
-// Packed pairs of float32 (Blackwell f32x2): one instruction multiplies two independent float32
-// pairs, each product rounded to nearest exactly like the scalar multiply, so the two products of
-// a key pair cost one issue slot.  The additions stay scalar: the assembler contracts a packed
-// multiply followed by a packed add into a packed fused multiply-add even when both carry an
-// explicit rounding mode and contraction is switched off (checked on sm_100a, CUDA 12.9), and a
-// fused multiply-add rounds once where the reference rounds twice.
+// Packed pairs of float32 (Blackwell f32x2): one instruction works on two independent float32 values, each rounded to
+// nearest exactly like the scalar operation.  A multiply-add of a key pair is a packed multiply and a packed sum, two issue
+// slots for two multiplies and two additions.  The sum is written as fma(product, one, acc) with `one` = (1, 1) from the
+// kernel's arguments: product * 1 is exact, so it rounds once, like an addition.  A plain packed addition would be contracted
+// with the multiply before it into one fused multiply-add even when both carry an explicit rounding mode and contraction is
+// switched off (seen on sm_100a, CUDA 12.9), and a fused multiply-add rounds once where the reference rounds twice.
+// Bound: 131 072 multiplies and additions per key at d = 128 on 128 fp32 lanes per SM (284 M keys/s).  262 144 bf16 keys: 1251 us
+// (1327 us with scalar sums, three issue slots instead of two).
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
     return r;
 }
-__device__ __forceinline__ void mul2(uint64_t a, uint64_t b, float& lo, float& hi) {
+__device__ __forceinline__ void unpack2(uint64_t v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
     uint64_t m;
     asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(m) : "l"(a), "l"(b));
-    asm("mov.b64 {%0, %1}, %2;\n" : "=f"(lo), "=f"(hi) : "l"(m));
+    return m;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t p, uint64_t one, uint64_t acc) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(p), "l"(one), "l"(acc));
+    return r;
 }
 
-// acc[r][j] += m[r] * v[j] for an R x K register tile: R output rows (or columns) times K keys.
+// acc[r][j] += m[r] * v[j] for an R x K register tile: R output rows (or columns) times K keys, keys in pairs.
 // Each output still sums its products in contraction order, one multiply and one add at a time.
 template <int R, int K>
-__device__ __forceinline__ void outer_keys(float (&acc)[R][K], const float4& m4, const float* v) {
+__device__ __forceinline__ void outer_keys(uint64_t (&acc)[R][K / 2], const float4& m4, const float* v, uint64_t one) {
     static_assert(R == 4 && K % 4 == 0, "the matrix operand is one 16-byte load");
     uint64_t kv[K / 2];
 #pragma unroll
@@ -289,19 +298,21 @@ __device__ __forceinline__ void outer_keys(float (&acc)[R][K], const float4& m4,
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int j = 0; j < K / 2; ++j) {
-            float p0, p1;
-            mul2(m[r], kv[j], p0, p1);
-            acc[r][2 * j] = __fadd_rn(acc[r][2 * j], p0);
-            acc[r][2 * j + 1] = __fadd_rn(acc[r][2 * j + 1], p1);
-        }
+        for (int j = 0; j < K / 2; ++j) acc[r][j] = add2(mul2(m[r], kv[j]), one, acc[r][j]);
 }
 template <int R, int K>
-__device__ __forceinline__ void zero_tile(float (&acc)[R][K]) {
+__device__ __forceinline__ void zero_tile(uint64_t (&acc)[R][K / 2]) {
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int j = 0; j < K; ++j) acc[r][j] = 0.0f;
+        for (int j = 0; j < K / 2; ++j) acc[r][j] = 0ull;
+}
+template <int R, int K>
+__device__ __forceinline__ void unpack_tile(const uint64_t (&acc)[R][K / 2], float (&out)[R][K]) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int j = 0; j < K / 2; ++j) unpack2(acc[r][j], out[r][2 * j], out[r][2 * j + 1]);
 }
 
 // KB keys per CTA pass (compile time: 32 unless the model dimension leaves no room).  Every
@@ -391,12 +402,14 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
                              reinterpret_cast<uintptr_t>(a.zt) | reinterpret_cast<uintptr_t>(a.scale)) & 15) == 0;
         // ---- latent / q_coarse: rows 4 lane .. +3, keys 4 warp .. +3 ------------
         if (KB == 32 && tiled) {
-            float acc[4][4];
-            zero_tile<4, 4>(acc);
+            uint64_t acc2[4][2];
+            zero_tile<4, 4>(acc2);
             const float4* mp = reinterpret_cast<const float4*>(a.pt) + lane;
 #pragma unroll 16
             for (uint32_t i = 0; i < d; ++i)
-                outer_keys<4, 4>(acc, __ldg(mp + (size_t)i * (D_C / 4)), keyT + (size_t)i * KS + 4 * warp);
+                outer_keys<4, 4>(acc2, __ldg(mp + (size_t)i * (D_C / 4)), keyT + (size_t)i * KS + 4 * warp, a.one);
+            float acc[4][4];
+            unpack_tile<4, 4>(acc2, acc);
             const float4 s4 = __ldg(reinterpret_cast<const float4*>(a.scale) + lane);
             const float sk[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
@@ -455,13 +468,15 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
             // tiled: columns 4 ig .. +3 for keys 4 kg .. +3
             for (uint32_t wi = tid; KB == 32 && tiled && wi < (d / 4) * 8; wi += ENC_THREADS) {
                 const uint32_t ig = wi % (d / 4), kg = wi / (d / 4);
-                float acc[4][4];
-                zero_tile<4, 4>(acc);
+                uint64_t acc2[4][2];
+                zero_tile<4, 4>(acc2);
                 const float4* mp = reinterpret_cast<const float4*>(a.p) + ig;
                 const float* wr = wsT + 4 * kg;
 #pragma unroll 16
                 for (int k = 0; k < D_C; ++k)
-                    outer_keys<4, 4>(acc, __ldg(mp + (size_t)k * (d / 4)), wr + (size_t)k * KS);
+                    outer_keys<4, 4>(acc2, __ldg(mp + (size_t)k * (d / 4)), wr + (size_t)k * KS, a.one);
+                float acc[4][4];
+                unpack_tile<4, 4>(acc2, acc);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
                     float kv[4];
@@ -538,12 +553,14 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
         // ---- sign-LSH, tiled: hyperplanes 4 rg .. +3 for keys 8 kg .. +7 -------
         if (KB == 32 && tiled) {
             const int rg = tid & 63, kg = tid >> 6;
-            float acc[4][8];
-            zero_tile<4, 8>(acc);
+            uint64_t acc2[4][4];
+            zero_tile<4, 8>(acc2);
             const float4* mp = reinterpret_cast<const float4*>(a.zt) + rg;
 #pragma unroll 16
             for (uint32_t i = 0; i < dp; ++i)
-                outer_keys<4, 8>(acc, __ldg(mp + (size_t)i * (D_S / 4)), buf + (size_t)i * KS + 8 * kg);
+                outer_keys<4, 8>(acc2, __ldg(mp + (size_t)i * (D_S / 4)), buf + (size_t)i * KS + 8 * kg, a.one);
+            float acc[4][8];
+            unpack_tile<4, 8>(acc2, acc);
             // bit s of a key = (acc < 0); this thread holds bits 4 rg .. +3, eight lanes fill a 32-bit word
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
@@ -676,6 +693,7 @@ Status fill_args(const Model* m, EncodeArgs& a, int* kb_out) {
     a.zt = m->d_zt;
     a.diag = m->d_diag;
     a.fwht_inv = 1.0f / sqrtf((float)m->d_pad);
+    a.one = 0x3F8000003F800000ull;
     a.lambda_c = sqrtf(3.14159265358979323846f / (2.0f * (float)D_S));
     // 32 keys per CTA pass when two CTAs still share an SM (their registers allow no more), else fewer
     int kb = 32;
