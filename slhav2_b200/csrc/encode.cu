@@ -684,7 +684,7 @@ size_t encode_smem(uint32_t d, uint32_t dp, int kb) {
     return (((d * ks + 3) & ~size_t(3)) + (size_t)kb * D_C + ks * dp + ks * D_C) * 4 + (size_t)kb * TILE_BYTES;
 }
 
-Status fill_args(const Model* m, EncodeArgs& a, int* kb_out) {
+Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
     a.d = (uint32_t)m->d;
     a.d_pad = (uint32_t)m->d_pad;
     a.p = m->d_p;
@@ -700,6 +700,11 @@ Status fill_args(const Model* m, EncodeArgs& a, int* kb_out) {
     while (kb > 1 && encode_smem(a.d, a.d_pad, kb) > (kb == 32 ? 100 : 200) * 1024) kb >>= 1;
     if (encode_smem(a.d, a.d_pad, kb) > 200 * 1024)
         return Status(SLHA_ERR_DIMENSION, "model dimension too large for the encode kernel");
+    // Few keys: the narrowest CTA of at least 4 keys that leaves no SM a second one.  Measured (d = 128, bf16,
+    // us per call at 8 / 592 / 1184 / 2368 / 4736 keys): 32 keys per CTA 39 / 39 / 37 / 37 / 37, 16: 29 / 28 / 29 / 29 / 39,
+    // 8: 21 / 21 / 21 / 27 / 49, 4: 17 / 19 / 21 / 37 / 70, 1: 17 / 31 / 59 / 113 / 221 -- a CTA of 4 keys is as fast as one of a
+    // single key, and a wider form is no slower from where the narrower one fills the SMs twice.
+    while (kb > 4 && n <= (uint64_t)(kb / 2) * 148) kb >>= 1;
     *kb_out = kb;
     a.kb = kb;
     return Status();
@@ -745,7 +750,7 @@ Status launch_encode(Ctx* c, const Model* m, const void* d_keys, int key_dtype, 
     if (n == 0) return Status();
     EncodeArgs a{};
     int kb;
-    SLHA_TRY(fill_args(m, a, &kb));
+    SLHA_TRY(fill_args(m, n, a, &kb));
     a.keys = d_keys;
     a.key_dtype = key_dtype;
     a.n = n;
@@ -763,7 +768,7 @@ Status launch_prepare_queries(Ctx* c, const Model* m, const float* d_q, size_t n
     if (nq == 0) return Status();
     EncodeArgs a{};
     int kb;
-    SLHA_TRY(fill_args(m, a, &kb));
+    SLHA_TRY(fill_args(m, nq, a, &kb));
     a.keys = d_q;
     a.key_dtype = SLHA_B200_F32;
     a.n = nq;

@@ -166,3 +166,18 @@ def test_decode_latent_and_key_for_every_codec(codec, d, rht):
         better += np.linalg.norm(keys[i] - gk) < np.linalg.norm(keys[i] - gl)
     # (with the Hadamard rotation the residual estimate is left out, learned.rs:295-299: both decodes coincide)
     assert better == (0 if rht else len(keys))
+
+
+@pytest.mark.parametrize("d,rht,codec", [(128, False, 2), (128, True, 5), (160, True, 4)])
+def test_small_batches_take_narrower_ctas_and_give_the_same_bytes(d, rht, codec):
+    # the number of keys per CTA (4, 8, 16 or 32) follows the batch size: every prefix gives the bytes of the whole batch
+    _, p = H.make_model_pair(d)
+    m = S.Model.from_projection(p, d, 7, rht=rht)
+    n = 5000
+    keys = H.gaussian_keys(77 + d, n, d, outlier_channels=(7, 93))
+    whole = m.encode_keys(keys, codec)
+    qc, qs = m.prepare_queries(keys)
+    for k in (1, 3, 5, 591, 592, 593, 1184, 1185, 2368, 2369, 4736):
+        assert np.array_equal(m.encode_keys(keys[:k], codec).view(np.uint8), whole[:k].view(np.uint8)), k
+        c, s = m.prepare_queries(keys[:k])
+        assert np.array_equal(c, qc[:k]) and np.array_equal(s, qs[:k]), k
