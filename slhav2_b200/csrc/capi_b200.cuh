@@ -538,14 +538,15 @@ int32_t slha_b200_pool_append_keys(SlhaB200Pool* pool, const SlhaModel* model, c
 }
 
 // What a pool's record of appended codecs says to the scorers: -1 unknown (look at the first tile), -2 only codecs the
-// tensor-core kernels do not decode, else bit 0 = NF4 tiles expected, bit 1 = mixed 8/4 only, bit 2 = TQ3 only.
+// tensor-core kernels do not decode, else bit 0 = NF4 tiles expected, bit 1 = mixed 8/4 only, bit 2 = TQ3 only,
+// bit 3 = MIX3 only.
 static int pool_codec_hint(const Pool* pl) {
     const uint32_t cm = pl->codec_mask;
     if ((cm & 0x80000000u) || !cm) return -1;
-    const bool mixed_only = cm == (1u << SLHA_CODEC_MIXED), tq3_only = cm == (1u << SLHA_CODEC_TQ3);
+    const bool mixed_only = cm == (1u << SLHA_CODEC_MIXED), tq3_only = cm == (1u << SLHA_CODEC_TQ3), mix3_only = cm == (1u << SLHA_CODEC_MIX3);
     const uint32_t nibble = (1u << SLHA_CODEC_INT4_SINGLE) | (1u << SLHA_CODEC_INT4_GROUPED) | (1u << SLHA_CODEC_NF4) | (1u << 6);
-    if (!(cm & nibble) && !mixed_only && !tq3_only) return -2;
-    return (int)(((cm >> SLHA_CODEC_NF4) & 1u) | (mixed_only ? 2u : 0u) | (tq3_only ? 4u : 0u));
+    if (!(cm & nibble) && !mixed_only && !tq3_only && !mix3_only) return -2;
+    return (int)(((cm >> SLHA_CODEC_NF4) & 1u) | (mixed_only ? 2u : 0u) | (tq3_only ? 4u : 0u) | (mix3_only ? 8u : 0u));
 }
 
 int32_t slha_b200_pool_score_all(SlhaB200Pool* pool, const float* q_coarse, const uint64_t* q_sign,
@@ -605,15 +606,10 @@ int32_t slha_b200_pool_score_topk(SlhaB200Pool* pool, const float* q_coarse, con
         SLHA_TRY(stage_out(c, out_score, nq * k * 4, &outs[1], /*in_place_if_pinned=*/true));
         SLHA_TRY(stage_out(c, out_count, nq * 4, &outs[2], /*in_place_if_pinned=*/true));
         SlhaB200Segment seg{0, (uint32_t)pl->h_cnt.len, 0, (uint32_t)nq, 0};
-        const uint32_t cm = pl->codec_mask;
-        const bool known = !(cm & 0x80000000u);
-        const bool mixed_only = known && cm == (1u << SLHA_CODEC_MIXED);
-        const bool tq3_only = known && cm == (1u << SLHA_CODEC_TQ3);
-        const uint32_t nibble = (1u << SLHA_CODEC_INT4_SINGLE) | (1u << SLHA_CODEC_INT4_GROUPED) | (1u << SLHA_CODEC_NF4) | (1u << 6);
+        const int hint = pool_codec_hint(pl);
         SLHA_TRY(score_topk_device(c, reinterpret_cast<const SciRustSlhaTile*>(pl->dev.tiles), pl->dev.state, &seg, 1,
                                    dq, ds, nq, k, (uint32_t*)outs[0].dev, (float*)outs[1].dev,
-                                   (uint32_t*)outs[2].dev, /*prefer_generic=*/known && cm && !(cm & nibble) && !mixed_only && !tq3_only,
-                                   known ? (int)(((cm >> SLHA_CODEC_NF4) & 1u) | (mixed_only ? 2u : 0u) | (tq3_only ? 4u : 0u)) : -1));
+                                   (uint32_t*)outs[2].dev, /*prefer_generic=*/hint == -2, hint == -2 ? 0 : hint));
         return finish_outputs(c, outs, sync_by_default(c));
     });
 }

@@ -301,10 +301,10 @@ struct ScoreArgs {
     uint32_t* ghist;              // per query row: 256 bucket counts of appended candidates
     uint32_t* gcount;             // per query row: candidates appended to the row's buffer
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
+    const uint32_t* only_flagged; // dense mode: optional, per query row: only work items one of whose rows is flagged here
     uint64_t* gbuf;               // per query row: gcap composite keys
     uint32_t gcap;
-    uint32_t nf4_table;           // tensor-core kernel: build the NF4 shared-memory table (else NF4 tiles are handed back)
-    uint32_t mixed;               // tensor-core kernel: query fragments arranged for mixed 8/4 tiles (other tiles are handed back)
+    uint32_t nf4_table;           // score_stream_kernel: build the NF4 shared-memory table (else NF4 tiles are handed back)
 };
 
 template <int G, bool TOPK>
@@ -459,6 +459,7 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
 }  // namespace slha
 
 #include "score_mma.cuh"
+#include "score_tile.cuh"
 #include "score_wide.cuh"
 #include "score_merge.cuh"
 #include "score_host.cuh"
@@ -633,9 +634,6 @@ Status score_topk_noalloc(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Se
 }  // namespace slha
 
 #ifdef SLHA_STREAM_PROBE
-extern "C" int slha_debug_stream_probe(unsigned long long* out) {  // development build only
-    return (int)cudaMemcpyFromSymbol(out, slha::g_stream_probe, sizeof(unsigned long long) * 160 * 8);
-}
 extern "C" int slha_debug_merge_probe(unsigned long long* out) {  // development build only
     return (int)cudaMemcpyFromSymbol(out, slha::g_merge_probe, sizeof(unsigned long long) * 64 * 12);
 }

@@ -21,6 +21,68 @@ size_t mma_smem_bytes(int nwarps, bool nf4_table) {  // (keep in step with the k
     return (size_t)(nf4_table ? NF4_LUT_BYTES : 0) + (size_t)nwarps * MMA_DEPTH * MMA_SET_STRIDE + MMA_BQ_BYTES + 128 + 16 + 32 + 32 + 16;
 }
 constexpr int STREAM_THREADS = SLHA_STREAM_THREADS;
+constexpr uint32_t STREAM_LEAST = 2048;  // tiles a CTA is given at least
+// kind of a launch by the flags of a tile (dequant_at's precedence)
+int stream_kind(uint32_t flags) { return (flags & F_MIXED) ? 1 : ((flags & F_TQ3) ? 2 : ((flags & F_MIX3) ? 4 : ((flags & F_NF4) ? 0 : 3))); }
+// the same for a codec hint: bit 0 NF4 tiles expected, bit 1 mixed 8/4 only, bit 2 TQ3 only, bit 3 MIX3 only
+int hint_kind(int hint) { return (hint & 2) ? 1 : ((hint & 4) ? 2 : ((hint & 8) ? 4 : ((hint & 1) ? 0 : 3))); }
+
+template <typename F>
+Status launch_tc(Ctx* c, F* kernel, bool* configured, const ScoreArgs& a, uint32_t grid, int threads, size_t smem) {
+    if (!configured[c->device & 15]) {  // (the attribute is per device)
+        SLHA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        configured[c->device & 15] = true;
+    }
+    kernel<<<grid, threads, smem, c->stream>>>(a);
+    count_launch();
+    SLHA_CUDA(cudaGetLastError());
+    return Status();
+}
+template <int KIND, bool IL>
+Status launch_stream_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+    static thread_local bool configured[16] = {false};
+    return launch_tc(c, score_stream_kernel<KIND, STREAM_THREADS, IL>, configured, a, grid, STREAM_THREADS, mma_smem_bytes(STREAM_THREADS / 32, KIND == 0));
+}
+template <bool IL>
+Status launch_mix3(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+    static thread_local bool configured[16] = {false};
+    return launch_tc(c, score_mix3_kernel<IL>, configured, a, grid, ST_THREADS, st_smem_bytes(4));
+}
+template <bool IL>
+Status launch_stream(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
+    switch (kind) {
+        case 0: return launch_stream_t<0, IL>(c, a, grid);
+        case 1: return launch_stream_t<1, IL>(c, a, grid);
+        case 2: return launch_stream_t<2, IL>(c, a, grid);
+        case 3: return launch_stream_t<3, IL>(c, a, grid);
+        default: return launch_mix3<IL>(c, a, grid);
+    }
+}
+// tiles a warp takes at a time (also the slots it reserves at a time in a row's buffer), and warps of a CTA
+uint32_t stream_warp_tiles(int kind) { return kind == 4 ? ST_WT : MMA_SET_TILES; }
+uint32_t stream_warps(int kind) { return (uint32_t)(kind == 4 ? ST_THREADS : STREAM_THREADS) / 32; }
+static_assert(ST_CHUNK == ST_WT && MMA_CHUNK == MMA_SET_TILES, "a fresh chunk holds what a warp can append at once");
+Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+    static thread_local bool configured[16] = {false};
+    return launch_tc(c, score_dense_kernel, configured, a, grid, 512, dense_smem_bytes());
+}
+template <int KIND>
+Status launch_wide_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+    static thread_local bool configured[16] = {false};
+    return launch_tc(c, score_wide_kernel<KIND>, configured, a, grid, WIDE_THREADS, wide_smem_bytes());
+}
+Status launch_wide(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
+    switch (kind) {
+        case 1: return launch_wide_t<1>(c, a, grid);
+        case 2: return launch_wide_t<2>(c, a, grid);
+        case 3: return launch_wide_t<3>(c, a, grid);
+        default: return launch_wide_t<4>(c, a, grid);
+    }
+}
+Status launch_wide_dense(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+    static thread_local bool configured[16] = {false};
+    return launch_tc(c, score_wide_dense_kernel, configured, a, grid, WIDE_THREADS, wide_smem_bytes());
+}
 
 size_t score_smem_bytes(int G, int nwarps, bool topk, uint32_t cap) {
     size_t b = (size_t)G * D_C * 4 + 16 * 32 * 4 + (size_t)nwarps * DEPTH * BLK_BYTES;
@@ -131,14 +193,10 @@ struct Plan {
     uint32_t max_parts = 1;  // most candidate lists any query has
     uint32_t list_cap = 0;   // slots per candidate list: k plus the slack the tensor-core kernel's last selection may leave
     bool use_mma = false;
-    bool nf4_table = true;
-    bool mixed = false;
-    bool tq3 = false;
+    int kind = 3;            // 0 NF4, 1 mixed 8/4, 2 TQ3, 3 INT4, 4 MIX3
     int codec_hint_in = -1;
     bool force_generic_in = false;
-    int mma_threads = STREAM_THREADS;
     uint32_t mma_grid = 0;
-    size_t mma_smem = 0;
     DevBuf b_stream_items, b_items, b_qbegin, b_qcount, b_keys, b_cnt, b_cta, b_gpivot, b_gbuf, b_gsel, b_vq, b_tmp, b_wide_items, b_wide_cta;
     // Two-level merge for calls with few queries and many candidate lists per query (a pool scored
     // by one GQA group: 148 lists each): groups of `group_parts` lists are merged by a CTA each into
@@ -150,8 +208,6 @@ struct Plan {
     float* d_tmp_score = nullptr;
     uint64_t last_use = 0;
 };
-
-size_t wide_smem_bytes() { return 3 * WIDE_A_BYTES + 2 * WIDE_RAW_BYTES + 2048 + 256 + 256 + 512 + 512 + 64 + 2048 + 1024; }
 
 Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, size_t nq,
                   uint32_t k, int codec_hint, bool allow_wide, Plan** out) {
@@ -206,34 +262,25 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     p->cap = cap;
 
     // tensor-core kernel: one persistent CTA per SM
-    p->mma_threads = STREAM_THREADS;
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
     {
-        const int mw = p->mma_threads / 32;
-        // Codec hint: the flags of the first tile of the first non-empty segment decide
-        // whether the NF4 table occupies shared memory.  A wrong hint costs speed only
-        // (NF4 tiles met without the table are handed to the generic kernel).
-        // (hint: -1 = look at the first tile, else bit 0 = NF4 tiles expected, bit 1 = mixed 8/4 tiles only,
-        //  bit 2 = TQ3 tiles only)
-        p->nf4_table = codec_hint < 0 || (codec_hint & 1);
-        p->mixed = codec_hint > 0 && (codec_hint & 2);
-        p->tq3 = codec_hint > 0 && (codec_hint & 4);
+        // Codec hint: -1 = the flags of the first tile of the first non-empty segment decide which kind of tile the launch
+        // decodes.  A wrong hint costs speed only (tiles of another kind are handed to the generic kernel).
+        p->kind = codec_hint < 0 ? 3 : hint_kind(codec_hint);
         for (size_t i = 0; i < n_segs && codec_hint < 0; ++i)
             if (segs[i].n_tiles) {
                 uint16_t flags = 0;
                 const unsigned char* t0 = reinterpret_cast<const unsigned char*>(tiles) + segs[i].tile_begin * TILE_BYTES;
                 SLHA_CUDA(cudaMemcpyAsync(&flags, t0 + 118, 2, cudaMemcpyDeviceToHost, c->stream));
                 SLHA_CUDA(cudaStreamSynchronize(c->stream));
-                p->nf4_table = (flags & F_NF4) != 0;
-                p->mixed = (flags & F_MIXED) != 0;
-                p->tq3 = (flags & F_TQ3) != 0;
+                p->kind = stream_kind(flags);
                 break;
             }
-        p->mma_smem = mma_smem_bytes(mw, p->nf4_table);
-        p->use_mma = !g_force_generic && p->mma_smem <= MAX_SMEM;
+        p->use_mma = !g_force_generic;
         p->mma_grid = (uint32_t)sms;
     }
+    const uint32_t st_warps = stream_warps(p->kind), st_tiles = stream_warp_tiles(p->kind), st_unit = p->kind == 4 ? (uint32_t)ST_M : (uint32_t)MMA_SET_TILES;
 
     // Work items.  Generic kernel: fixed-size runs, large enough that candidate
     // traffic stays a few percent of the tile stream and small enough to balance
@@ -246,7 +293,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     while (item_tiles > 2048 && total / item_tiles < 592) item_tiles /= 2;
     item_tiles = std::max(round, (item_tiles + round - 1) / round * round);
     uint64_t share = (total + p->mma_grid - 1) / std::max<uint32_t>(p->mma_grid, 1);
-    share = std::max<uint64_t>(2048, (share + MMA_SET_TILES - 1) / MMA_SET_TILES * MMA_SET_TILES);
+    share = std::max<uint64_t>(STREAM_LEAST, (share + st_unit - 1) / st_unit * st_unit);
     const uint64_t snap = std::min<uint64_t>(share / 16, 2048);
     uint64_t spare = share * std::max<uint32_t>(p->mma_grid, 1) > total ? share * std::max<uint32_t>(p->mma_grid, 1) - total : 0;  // room the equal shares leave
     uint64_t filled = 0;  // tiles already given to the current CTA (tensor-core mode)
@@ -273,7 +320,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
             stream_ctas.resize(st_tiles.size());
             uint32_t used = 0;
             for (size_t j = 0; j < st_tiles.size(); ++j) {
-                const uint64_t most = (st_tiles[j] + 2047) / 2048;  // (no CTA for less than 2048 tiles)
+                const uint64_t most = (st_tiles[j] + STREAM_LEAST - 1) / STREAM_LEAST;
                 stream_ctas[j] = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(most, st_tiles[j] * p->mma_grid / total));
                 used += stream_ctas[j];
             }
@@ -282,7 +329,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
                 uint64_t worst = 0;
                 for (size_t j = 0; j < st_tiles.size(); ++j) {
                     const uint64_t per = st_tiles[j] / stream_ctas[j];
-                    if (per > worst && (uint64_t)stream_ctas[j] < (st_tiles[j] + 2047) / 2048) { worst = per; best = j; }
+                    if (per > worst && (uint64_t)stream_ctas[j] < (st_tiles[j] + STREAM_LEAST - 1) / STREAM_LEAST) { worst = per; best = j; }
                 }
                 if (best == st_tiles.size()) break;
                 ++stream_ctas[best];
@@ -306,7 +353,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
             std::vector<std::pair<uint32_t, uint32_t>> cuts;  // (offset, length)
             if (!stream_ctas.empty() && s.n_tiles) {
                 uint32_t ctas = stream_ctas[stream_no++];
-                const uint32_t per = (uint32_t)(((uint64_t)s.n_tiles + ctas - 1) / ctas + MMA_SET_TILES - 1) / MMA_SET_TILES * MMA_SET_TILES;
+                const uint32_t per = (uint32_t)(((uint64_t)s.n_tiles + ctas - 1) / ctas + st_unit - 1) / st_unit * st_unit;
                 ctas = (s.n_tiles + per - 1) / per;  // (rounding to whole sets can leave the last CTA nothing)
                 for (uint32_t part = 0; part < ctas; ++part) {
                     cuts.push_back({part * per, std::min<uint32_t>(per, s.n_tiles - part * per)});
@@ -402,13 +449,13 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // of up to 64 query rows; the (segment, row group) streams are cut into one share per CTA, in whole 128-tile blocks.
     uint32_t wide_parts = 1;
     {
-        bool all_wide = p->use_mma && allow_wide && n_segs > 0 && (p->mixed || p->tq3 || !p->nf4_table);
+        bool all_wide = p->use_mma && allow_wide && n_segs > 0 && p->kind != 0;
         uint64_t wtotal = 0;
         for (size_t i = 0; i < n_segs && all_wide; ++i) {
             all_wide = segs[i].n_queries >= 16 || segs[i].n_tiles == 0;
             wtotal += (uint64_t)segs[i].n_tiles * ((segs[i].n_queries + WIDE_NQ - 1) / WIDE_NQ);
         }
-        if (all_wide && wtotal > 0 && wide_smem_bytes() <= MAX_SMEM) {
+        if (all_wide && wtotal > 0) {
             uint64_t wshare = (wtotal + sms - 1) / sms;
             wshare = std::max<uint64_t>(WIDE_M, (wshare + WIDE_M - 1) / WIDE_M * WIDE_M);
             std::vector<WorkItem> wi;
@@ -454,12 +501,12 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // the row's candidate buffer.  In random order about k (1 + ln(n / k)) tiles pass the rising threshold
     // plus the unfiltered first sets of every warp; 16 k slots (at most the longest segment) leave a wide
     // margin, and a row that fills its buffer all the same is scored by the generic kernel.
-    // (a warp reserves slots in chunks of 16 per row and work item, so up to 16 slots per warp and item stay unused)
+    // (a warp reserves slots in chunks of 32 per row and work item, so up to 32 slots per warp and item stay unused)
     uint32_t longest = 0;
     for (size_t i = 0; i < n_segs; ++i) longest = std::max(longest, segs[i].n_tiles);
-    const uint64_t all_of_a_row = (uint64_t)longest + (uint64_t)MMA_CHUNK * (uint64_t)(p->mma_threads / 32) * p->max_parts + 64;
-    // (the first set of every warp that scans a row is appended unfiltered: 16 slots per warp and item, twice over)
-    const uint64_t first_sets = (uint64_t)(16 + MMA_CHUNK) * (uint64_t)(p->mma_threads / 32) * p->max_parts;
+    const uint64_t all_of_a_row = (uint64_t)longest + (uint64_t)st_tiles * st_warps * p->max_parts + 64;
+    // (the first set of every warp that scans a row is appended unfiltered: 32 slots per warp and item, twice over)
+    const uint64_t first_sets = (uint64_t)(2 * st_tiles) * st_warps * p->max_parts;
     p->gcap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(std::max<uint64_t>(16ull * k, 4096), first_sets + 4ull * k), all_of_a_row / 64 * 64);
     // (wide scoring: the first 128-tile block of every item is appended unfiltered, and a CTA sees few blocks)
     if (p->wide) p->gcap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(p->gcap, 4ull * WIDE_M * wide_parts + 16ull * k), ((uint64_t)longest + 63) / 64 * 64);
@@ -545,95 +592,87 @@ Status launch_validate_tiles(Ctx* c, const SciRustSlhaTile* tiles, size_t n, uns
     return Status();
 }
 
+// One upload of several small host arrays into the call's scratch (pageable sources: cudaMemcpyAsync returns once they are staged).
+struct Blob {
+    std::vector<unsigned char> bytes;
+    template <typename T>
+    size_t add(const std::vector<T>& v) {
+        const size_t at = (bytes.size() + 15) / 16 * 16;
+        bytes.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+    Status upload(Ctx* c, unsigned char** dev) {
+        SLHA_TRY(ctx_device_scratch(c, bytes.size(), (void**)dev));
+        SLHA_CUDA(cudaMemcpyAsync(*dev, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, c->stream));
+        return Status();
+    }
+};
+
+// Cuts of (segment, group of up to `width` query rows) streams into one share per CTA.
+struct Cuts {
+    std::vector<WorkItem> items;
+    std::vector<uint32_t> cta{0u};
+    uint64_t share = 0, filled = 0;
+    Cuts(uint64_t total, int sms, uint64_t unit, uint64_t least) {
+        share = (total + sms - 1) / sms;
+        share = std::max<uint64_t>(least, (share + unit - 1) / unit * unit);
+    }
+    void add(const SlhaB200Segment& s, uint32_t width) {
+        for (uint32_t q0 = 0; q0 < s.n_queries; q0 += width)
+            for (uint64_t pos = 0; pos < s.n_tiles;) {
+                const uint32_t take = (uint32_t)std::min<uint64_t>(s.n_tiles - pos, share - filled);
+                WorkItem w{};
+                w.tile_begin = s.tile_begin + pos;
+                w.n_tiles = take;
+                w.index_base = s.index_base + (uint32_t)pos;
+                w.query_begin = s.query_begin + q0;
+                w.n_queries = std::min<uint32_t>(width, s.n_queries - q0);
+                items.push_back(w);
+                pos += take;
+                filled += take;
+                if (filled >= share) {
+                    filled = 0;
+                    cta.push_back((uint32_t)items.size());
+                }
+            }
+    }
+    void finish() {
+        if (cta.back() != (uint32_t)items.size()) cta.push_back((uint32_t)items.size());
+    }
+};
+
 Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state, size_t n,
                          const float* q_coarse, const uint64_t* q_sign, size_t nq, float* scores, int codec_hint) {
     if (n == 0 || nq == 0) return Status();
     // Long arenas: the streaming tensor-core kernel in its dense mode (all query groups of four in one launch, every CTA an
     // equal share of the tiles), then the generic kernel for the rows of work items it handed back (a codec it does not
-    // decode, a query outside the fp16 split).  codec_hint as for score_topk_device: -1 = look at the first tile, -2 = generic.
+    // decode, a query outside the fp16 split).  codec_hint -2: codecs the tensor-core kernel does not decode together.
     if (n >= 32768 && n < 0xFFFFFFFFull && codec_hint != -2 && !g_force_generic) {
-        bool nf4 = codec_hint < 0 || (codec_hint & 1), mixed = codec_hint > 0 && (codec_hint & 2), tq3 = codec_hint > 0 && (codec_hint & 4), other = false;
-        if (codec_hint < 0) {
-            uint16_t flags = 0;
-            SLHA_CUDA(cudaMemcpyAsync(&flags, reinterpret_cast<const unsigned char*>(tiles) + 118, 2, cudaMemcpyDeviceToHost, c->stream));
-            SLHA_CUDA(cudaStreamSynchronize(c->stream));
-            nf4 = (flags & F_NF4) != 0;
-            mixed = (flags & F_MIXED) != 0;
-            tq3 = (flags & F_TQ3) != 0;
-            other = (flags & F_MIX3) != 0;
-        }
-        const int kind = tq3 ? 2 : (mixed ? 1 : (nf4 ? 0 : 3));
-        const int mw = STREAM_THREADS / 32;
-        const size_t smem = mma_smem_bytes(mw, kind == 0);
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        if (!other && smem <= MAX_SMEM) {
-            const uint32_t groups = (uint32_t)((nq + 3) / 4);
-            const uint64_t total = (uint64_t)n * groups;
-            uint64_t share = (total + sms - 1) / sms;
-            share = std::max<uint64_t>(2048, (share + MMA_SET_TILES - 1) / MMA_SET_TILES * MMA_SET_TILES);
-            std::vector<WorkItem> items;
-            std::vector<uint32_t> cta(1, 0);
-            uint64_t filled = 0;
-            for (uint32_t grp = 0; grp < groups; ++grp)
-                for (uint64_t pos = 0; pos < n;) {
-                    const uint32_t take = (uint32_t)std::min<uint64_t>(n - pos, share - filled);
-                    WorkItem w{};
-                    w.tile_begin = pos;
-                    w.n_tiles = take;
-                    w.index_base = (uint32_t)pos;
-                    w.query_begin = 4 * grp;
-                    w.n_queries = (uint32_t)std::min<size_t>(4, nq - 4 * (size_t)grp);
-                    w.pad = w.n_queries;
-                    items.push_back(w);
-                    pos += take;
-                    filled += take;
-                    if (filled >= share) {
-                        filled = 0;
-                        cta.push_back((uint32_t)items.size());
-                    }
-                }
-            if (cta.back() != (uint32_t)items.size()) cta.push_back((uint32_t)items.size());
-            WorkItem* d_items;
-            uint32_t *d_cta, *d_gflag;
-            SLHA_TRY(ctx_device_scratch(c, items.size() * sizeof(WorkItem), (void**)&d_items));
-            SLHA_TRY(ctx_device_scratch(c, cta.size() * 4, (void**)&d_cta));
-            SLHA_TRY(ctx_device_scratch(c, nq * 4, (void**)&d_gflag));
-            SLHA_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, c->stream));
-            SLHA_CUDA(cudaMemcpyAsync(d_cta, cta.data(), cta.size() * 4, cudaMemcpyHostToDevice, c->stream));
-            SLHA_CUDA(cudaMemsetAsync(d_gflag, 0, nq * 4, c->stream));
-            SLHA_CUDA(cudaStreamSynchronize(c->stream));  // (the host vectors go away)
-            static thread_local bool configured[16] = {false};
-            if (!configured[c->device & 15]) {
-#define SLHA_DENSE_SMEM(K) SLHA_CUDA(cudaFuncSetAttribute(score_stream_kernel<K, STREAM_THREADS, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM))
-                SLHA_DENSE_SMEM(0); SLHA_DENSE_SMEM(1); SLHA_DENSE_SMEM(2); SLHA_DENSE_SMEM(3);
-#undef SLHA_DENSE_SMEM
-                configured[c->device & 15] = true;
-            }
-            ScoreArgs a{};
-            a.tiles = reinterpret_cast<const unsigned char*>(tiles);
-            a.state = state;
-            a.items = d_items;
-            a.stream_items = d_items;
-            a.n_items = (uint32_t)items.size();
-            a.cta_begin = d_cta;
-            a.q_coarse = q_coarse;
-            a.q_sign = reinterpret_cast<const uint32_t*>(q_sign);
-            a.scores = scores;
-            a.score_stride = n;
-            a.gflag = d_gflag;
-            a.nf4_table = kind == 0 ? 1u : 0u;
-            a.mixed = kind == 1 ? 1u : 0u;
-            const uint32_t grid = (uint32_t)cta.size() - 1;
-#define SLHA_LAUNCH_DENSE(K) score_stream_kernel<K, STREAM_THREADS, false, true><<<grid, STREAM_THREADS, smem, c->stream>>>(a)
-            if (kind == 3) SLHA_LAUNCH_DENSE(3); else if (kind == 2) SLHA_LAUNCH_DENSE(2); else if (kind == 1) SLHA_LAUNCH_DENSE(1); else SLHA_LAUNCH_DENSE(0);
-#undef SLHA_LAUNCH_DENSE
-            count_launch();
-            SLHA_CUDA(cudaGetLastError());
-            // the generic kernel over the same work items, only those whose rows were handed back
-            const int threads = 128, nwarps = threads / 32;
-            return launch_score<false>(c, 4, a, (uint32_t)items.size(), threads, score_smem_bytes(4, nwarps, false, 0));
-        }
+        Cuts cuts((uint64_t)n * ((nq + 3) / 4), sms, ST_M, 2048);
+        cuts.add(SlhaB200Segment{0, (uint32_t)n, 0, (uint32_t)nq, 0}, 4);
+        cuts.finish();
+        Blob blob;
+        const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta), o_flag = blob.add(std::vector<uint32_t>(nq, 0u));
+        unsigned char* dev;
+        SLHA_TRY(blob.upload(c, &dev));
+        ScoreArgs a{};
+        a.tiles = reinterpret_cast<const unsigned char*>(tiles);
+        a.state = state;
+        a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_items);
+        a.n_items = (uint32_t)cuts.items.size();
+        a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_cta);
+        a.q_coarse = q_coarse;
+        a.q_sign = reinterpret_cast<const uint32_t*>(q_sign);
+        a.scores = scores;
+        a.score_stride = n;
+        a.gflag = reinterpret_cast<uint32_t*>(dev + o_flag);
+        SLHA_TRY(launch_dense(c, a, (uint32_t)cuts.cta.size() - 1));
+        // the generic kernel over the same work items, only those whose rows were handed back
+        const int threads = 128, nwarps = threads / 32;
+        return launch_score<false>(c, 4, a, (uint32_t)cuts.items.size(), threads, score_smem_bytes(4, nwarps, false, 0));
     }
     const int threads = 128, nwarps = threads / 32;
     const uint32_t item_tiles = 4096;
@@ -659,146 +698,87 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     return Status();
 }
 
-// Dense scores of whole segments in one launch: every query row of a segment against every tile of the segment,
-// row q written at scores + row_offsets[q] + index_base + tile, the rest of the row up to row_len set to `fill`.
-// Work items: (segment, group of up to four query rows, run of 4096 tiles) on the generic kernel.
 // fill of the rows' tails [tail_begin[q], row_len) (one CTA per row)
 __global__ void fill_rows_kernel(float* scores, const unsigned long long* row_offset, const uint32_t* tail_begin, uint32_t row_len, float fill) {
     float* row = scores + row_offset[blockIdx.x];
     for (uint32_t e = tail_begin[blockIdx.x] + threadIdx.x; e < row_len; e += blockDim.x) row[e] = fill;
 }
 
+// Dense scores of whole segments: every query row of a segment against every tile of the segment, row q written at
+// scores + row_offsets[q] + index_base + tile, the rest of the row up to row_len set to `fill`.  Up to three passes over the
+// same call, each for the rows the one before handed over (the last two end at once when there are none): the 64-row kernel
+// where every segment brings 16 query rows or more, the four-row kernel, the generic kernel.  The host looks at no tile and waits for nothing.
 Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, const float* d_q_coarse,
                              const uint64_t* d_q_sign, size_t nq, float* d_scores, const unsigned long long* d_row_offsets,
                              uint32_t row_len, float fill) {
-    // Sixteen or more query rows per segment and INT4 / MX-INT4, TQ3 or mixed 8/4 tiles (by the first tile): the contraction runs on the
-    // tensor cores (score_wide_kernel in its dense mode); rows it cannot score (a tile of another codec, a query outside the
-    // fp16 split) are flagged and the generic kernel below scores them.
-    bool wide = n_segs > 0 && wide_smem_bytes() <= MAX_SMEM;
-    uint64_t wtotal = 0;
-    for (size_t i = 0; i < n_segs && wide; ++i) {
-        wide = segs[i].n_queries >= 16 || segs[i].n_tiles == 0;
-        wtotal += (uint64_t)segs[i].n_tiles * ((segs[i].n_queries + WIDE_NQ - 1) / WIDE_NQ);
-    }
-    int kindw = -1;
-    for (size_t i = 0; i < n_segs && wide && wtotal && kindw < 0; ++i)
-        if (segs[i].n_tiles) {
-            uint16_t flags = 0;
-            const unsigned char* t0 = reinterpret_cast<const unsigned char*>(tiles) + segs[i].tile_begin * TILE_BYTES;
-            SLHA_CUDA(cudaMemcpyAsync(&flags, t0 + 118, 2, cudaMemcpyDeviceToHost, c->stream));
-            SLHA_CUDA(cudaStreamSynchronize(c->stream));
-            kindw = (flags & (F_NF4 | F_MIX3)) ? 3 : ((flags & F_MIXED) ? 2 : ((flags & F_TQ3) ? 1 : 0));
-        }
-    wide = wide && wtotal > 0 && kindw >= 0 && kindw <= 2;
-    uint32_t* d_gflag = nullptr;
-    if (wide) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-        uint64_t wshare = (wtotal + sms - 1) / sms;
-        wshare = std::max<uint64_t>(WIDE_M, (wshare + WIDE_M - 1) / WIDE_M * WIDE_M);
-        std::vector<WorkItem> wi;
-        std::vector<uint32_t> wcta(1, 0), tail(nq, row_len);
-        uint64_t wfilled = 0;
-        for (size_t i = 0; i < n_segs; ++i) {
-            const SlhaB200Segment& s = segs[i];
-            if ((uint64_t)s.query_begin + s.n_queries > nq) return Status(SLHA_ERR_DIMENSION, "segment query range exceeds n_queries");
-            if ((uint64_t)s.index_base + s.n_tiles > row_len) return Status(SLHA_ERR_DIMENSION, "segment does not fit a row of row_len scores");
-            for (uint32_t q = 0; q < s.n_queries; ++q) tail[s.query_begin + q] = s.index_base + s.n_tiles;
-            for (uint32_t q0 = 0; q0 < s.n_queries; q0 += WIDE_NQ)
-                for (uint32_t pos = 0; pos < s.n_tiles;) {
-                    const uint32_t take = (uint32_t)std::min<uint64_t>(s.n_tiles - pos, wshare - wfilled);
-                    WorkItem w{};
-                    w.tile_begin = s.tile_begin + pos;
-                    w.n_tiles = take;
-                    w.index_base = s.index_base + pos;
-                    w.query_begin = s.query_begin + q0;
-                    w.n_queries = std::min<uint32_t>(WIDE_NQ, s.n_queries - q0);
-                    wi.push_back(w);
-                    pos += take;
-                    wfilled += take;
-                    if (wfilled >= wshare) {
-                        wfilled = 0;
-                        wcta.push_back((uint32_t)wi.size());
-                    }
-                }
-        }
-        if (wcta.back() != (uint32_t)wi.size()) wcta.push_back((uint32_t)wi.size());
-        WorkItem* d_wi;
-        uint32_t *d_wcta, *d_tail;
-        SLHA_TRY(ctx_device_scratch(c, wi.size() * sizeof(WorkItem), (void**)&d_wi));
-        SLHA_TRY(ctx_device_scratch(c, wcta.size() * 4, (void**)&d_wcta));
-        SLHA_TRY(ctx_device_scratch(c, nq * 4, (void**)&d_tail));
-        SLHA_TRY(ctx_device_scratch(c, nq * 4, (void**)&d_gflag));
-        SLHA_CUDA(cudaMemcpyAsync(d_wi, wi.data(), wi.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, c->stream));
-        SLHA_CUDA(cudaMemcpyAsync(d_wcta, wcta.data(), wcta.size() * 4, cudaMemcpyHostToDevice, c->stream));
-        SLHA_CUDA(cudaMemcpyAsync(d_tail, tail.data(), nq * 4, cudaMemcpyHostToDevice, c->stream));
-        SLHA_CUDA(cudaMemsetAsync(d_gflag, 0, nq * 4, c->stream));
-        SLHA_CUDA(cudaStreamSynchronize(c->stream));  // (the host vectors go away)
-        static thread_local bool configured[16] = {false};
-        if (!configured[c->device & 15]) {
-            SLHA_CUDA(cudaFuncSetAttribute(score_wide_kernel<0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-            SLHA_CUDA(cudaFuncSetAttribute(score_wide_kernel<1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-            SLHA_CUDA(cudaFuncSetAttribute(score_wide_kernel<2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-            configured[c->device & 15] = true;
-        }
-        ScoreArgs a{};
-        a.tiles = reinterpret_cast<const unsigned char*>(tiles);
-        a.items = d_wi;
-        a.n_items = (uint32_t)wi.size();
-        a.cta_begin = d_wcta;
-        a.q_coarse = d_q_coarse;
-        a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
-        a.scores = d_scores;
-        a.row_offset = d_row_offsets;
-        a.gflag = d_gflag;
-        const uint32_t grid = (uint32_t)wcta.size() - 1;
-        if (kindw == 1) score_wide_kernel<1, true><<<grid, WIDE_THREADS, wide_smem_bytes(), c->stream>>>(a);
-        else if (kindw == 2) score_wide_kernel<2, true><<<grid, WIDE_THREADS, wide_smem_bytes(), c->stream>>>(a);
-        else score_wide_kernel<0, true><<<grid, WIDE_THREADS, wide_smem_bytes(), c->stream>>>(a);
-        count_launch();
-        SLHA_CUDA(cudaGetLastError());
-        fill_rows_kernel<<<(uint32_t)nq, 256, 0, c->stream>>>(d_scores, d_row_offsets, d_tail, row_len, fill);
-        count_launch();
-        SLHA_CUDA(cudaGetLastError());
-    }
-    const uint32_t item_tiles = 4096;
-    std::vector<WorkItem> items;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    bool wide = !g_force_generic, fills = false;
+    uint64_t total = 0, wtotal = 0;
+    std::vector<uint32_t> tail(nq, row_len);
     for (size_t i = 0; i < n_segs; ++i) {
         const SlhaB200Segment& s = segs[i];
         if ((uint64_t)s.query_begin + s.n_queries > nq) return Status(SLHA_ERR_DIMENSION, "segment query range exceeds n_queries");
         if ((uint64_t)s.index_base + s.n_tiles > row_len) return Status(SLHA_ERR_DIMENSION, "segment does not fit a row of row_len scores");
-        for (uint32_t q0 = 0; q0 < s.n_queries; q0 += 4) {
-            uint32_t pos = 0;
-            do {  // (a segment without tiles still fills its rows)
-                WorkItem w{};
-                w.tile_begin = s.tile_begin + pos;
-                w.n_tiles = std::min<uint32_t>(item_tiles, s.n_tiles - pos);
-                w.index_base = s.index_base + pos;
-                w.query_begin = s.query_begin + q0;
-                w.n_queries = std::min<uint32_t>(4, s.n_queries - q0);
-                pos += w.n_tiles;
-                w.pad = (pos >= s.n_tiles && !wide) ? 1u : 0u;  // (the rows' tails: filled above when the tensor-core kernel ran)
-                items.push_back(w);
-            } while (pos < s.n_tiles);
-        }
+        for (uint32_t q = 0; q < s.n_queries; ++q) tail[s.query_begin + q] = s.index_base + s.n_tiles;
+        fills |= s.index_base + s.n_tiles < row_len;
+        wide = wide && (s.n_queries >= 16 || s.n_tiles == 0);
+        total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
+        wtotal += (uint64_t)s.n_tiles * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
     }
-    if (items.empty()) return Status();
-    WorkItem* d_items;
-    SLHA_TRY(ctx_device_scratch(c, items.size() * sizeof(WorkItem), (void**)&d_items));
-    SLHA_CUDA(cudaMemcpyAsync(d_items, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, c->stream));
-    SLHA_CUDA(cudaStreamSynchronize(c->stream));  // (the host vector goes away)
-    const int threads = 128, nwarps = threads / 32;
+    Cuts narrow(total, sms, ST_M, ST_M * 4), many(wtotal, sms, WIDE_M, WIDE_M);
+    for (size_t i = 0; i < n_segs; ++i) {
+        narrow.add(segs[i], 4);
+        if (wide) many.add(segs[i], WIDE_NQ);
+    }
+    narrow.finish();
+    many.finish();
+    std::vector<WorkItem> generic;  // runs of 4096 tiles for the last pass
+    for (const WorkItem& s : narrow.items)
+        for (uint32_t pos = 0; pos < s.n_tiles; pos += 4096) {
+            WorkItem w = s;
+            w.tile_begin += pos;
+            w.index_base += pos;
+            w.n_tiles = std::min<uint32_t>(4096, s.n_tiles - pos);
+            generic.push_back(w);
+        }
+    Blob blob;
+    const size_t o_narrow = blob.add(narrow.items), o_ncta = blob.add(narrow.cta), o_many = blob.add(many.items), o_mcta = blob.add(many.cta), o_gen = blob.add(generic);
+    const size_t o_tail = blob.add(tail), o_flag = blob.add(std::vector<uint32_t>(2 * nq, 0u));
+    unsigned char* dev;
+    SLHA_TRY(blob.upload(c, &dev));
+    if (fills) {
+        fill_rows_kernel<<<(uint32_t)nq, 256, 0, c->stream>>>(d_scores, d_row_offsets, reinterpret_cast<const uint32_t*>(dev + o_tail), row_len, fill);
+        count_launch();
+        SLHA_CUDA(cudaGetLastError());
+    }
+    if (narrow.items.empty()) return Status();
     ScoreArgs a{};
     a.tiles = reinterpret_cast<const unsigned char*>(tiles);
-    a.items = d_items;
     a.q_coarse = d_q_coarse;
     a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
     a.scores = d_scores;
     a.row_offset = d_row_offsets;
-    a.row_len = row_len;
-    a.row_fill = fill;
-    a.gflag = d_gflag;  // (behind the tensor-core kernel: only the work items of rows it handed back)
-    return launch_score<false>(c, 4, a, (uint32_t)items.size(), threads, score_smem_bytes(4, nwarps, false, 0));
+    uint32_t* flag = reinterpret_cast<uint32_t*>(dev + o_flag);
+    if (wide) {
+        a.items = reinterpret_cast<const WorkItem*>(dev + o_many);
+        a.n_items = (uint32_t)many.items.size();
+        a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_mcta);
+        a.gflag = flag + nq;
+        SLHA_TRY(launch_wide_dense(c, a, (uint32_t)many.cta.size() - 1));
+        a.only_flagged = flag + nq;
+    }
+    a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_narrow);
+    a.n_items = (uint32_t)narrow.items.size();
+    a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_ncta);
+    a.gflag = nullptr;
+    if (!g_force_generic) {
+        a.gflag = flag;
+        SLHA_TRY(launch_dense(c, a, (uint32_t)narrow.cta.size() - 1));
+    }
+    a.items = reinterpret_cast<const WorkItem*>(dev + o_gen);
+    const int threads = 128, nwarps = threads / 32;
+    return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0));
 }
 
 Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state,
@@ -836,46 +816,20 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.gflag = a.gcount + nq;
         a.gbuf = p->d_gbuf;
         a.gcap = p->gcap;
-        a.nf4_table = p->nf4_table ? 1u : 0u;
-        a.mixed = p->mixed ? 1u : 0u;
+        a.nf4_table = p->kind == 0 ? 1u : 0u;
         a.q_coarse = d_q_coarse;
         a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
         a.k = k;
-        static thread_local bool mma_configured[16] = {false};  // the attribute is per device
-        if (!mma_configured[c->device & 15]) {
-#define SLHA_STREAM_SMEM(K, I) SLHA_CUDA(cudaFuncSetAttribute(score_stream_kernel<K, STREAM_THREADS, I>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM))
-            SLHA_STREAM_SMEM(0, false); SLHA_STREAM_SMEM(1, false); SLHA_STREAM_SMEM(2, false); SLHA_STREAM_SMEM(3, false);
-            SLHA_STREAM_SMEM(0, true); SLHA_STREAM_SMEM(1, true); SLHA_STREAM_SMEM(2, true); SLHA_STREAM_SMEM(3, true);
-#undef SLHA_STREAM_SMEM
-            mma_configured[c->device & 15] = true;
-        }
-        // 3: no NF4 tile is expected, so the launch holds INT4 / MX-INT4 tiles only (any other tile hands its rows back)
-        const int kind = p->tq3 ? 2 : (p->mixed ? 1 : (p->nf4_table ? 0 : 3));
         if (p->wide) {
-            static thread_local bool wide_configured[16] = {false};
-            if (!wide_configured[c->device & 15]) {
-                SLHA_CUDA(cudaFuncSetAttribute(score_wide_kernel<0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-                SLHA_CUDA(cudaFuncSetAttribute(score_wide_kernel<1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-                SLHA_CUDA(cudaFuncSetAttribute(score_wide_kernel<2, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)MAX_SMEM));
-                wide_configured[c->device & 15] = true;
-            }
             a.items = p->d_wide_items;
             a.n_items = p->n_wide_items;
             a.cta_begin = p->d_wide_cta;
-            if (kind == 2) score_wide_kernel<1, false><<<p->wide_grid, WIDE_THREADS, wide_smem_bytes(), c->stream>>>(a);
-            else if (kind == 1) score_wide_kernel<2, false><<<p->wide_grid, WIDE_THREADS, wide_smem_bytes(), c->stream>>>(a);
-            else score_wide_kernel<0, false><<<p->wide_grid, WIDE_THREADS, wide_smem_bytes(), c->stream>>>(a);
+            SLHA_TRY(launch_wide(c, p->kind, a, p->wide_grid));
+        } else if (p->d_stream_items) {
+            SLHA_TRY((launch_stream<true>(c, p->kind, a, p->mma_grid)));
         } else {
-#define SLHA_LAUNCH_MMA(K)                                                                                             \
-    do {                                                                                                               \
-        if (p->d_stream_items) score_stream_kernel<K, STREAM_THREADS, true><<<p->mma_grid, p->mma_threads, p->mma_smem, c->stream>>>(a); \
-        else score_stream_kernel<K, STREAM_THREADS, false><<<p->mma_grid, p->mma_threads, p->mma_smem, c->stream>>>(a); \
-    } while (0)
-            if (kind == 3) SLHA_LAUNCH_MMA(3); else if (kind == 2) SLHA_LAUNCH_MMA(2); else if (kind == 1) SLHA_LAUNCH_MMA(1); else SLHA_LAUNCH_MMA(0);
-#undef SLHA_LAUNCH_MMA
+            SLHA_TRY((launch_stream<false>(c, p->kind, a, p->mma_grid)));
         }
-        count_launch();
-        SLHA_CUDA(cudaGetLastError());
         // (timing: the first bracket is the tensor-core kernel alone; the generic kernel's pass over handed-back rows, an
         // early exit when there are none, counts with the compaction and the merge)
         if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));

@@ -1,5 +1,5 @@
-// Tensor-core kernel of the fused score + top-k path (score_stream_kernel) and the selection
-// routine the merge kernel shares with it.  Included by score.cu.
+// Tensor-core kernel of the fused score + top-k path for up to four queries per tile (score_stream_kernel), the pieces the
+// other scoring kernels share with it, and the selection routine of the merge kernel.  Included by score.cu.
 //
 // With a GQA group of four queries the CUDA-core kernel is bound by instruction issue (128 FMAs
 // per tile and query plus the nibble decode), not by HBM.  Here the coarse dot product of eq. 2.3
@@ -44,20 +44,12 @@ constexpr int NF4_LUT_BYTES = 256 * 16 * 8;                // [byte][16 lanes] x
 constexpr int SEL_HIST_INTS = 4 * 256 + 48;                // block_select_multi: 4 histograms + state
 
 #ifdef SLHA_STREAM_PROBE
-// development build only: per-CTA timeline of score_stream_kernel (nanoseconds of %globaltimer)
-__device__ unsigned long long g_stream_probe[160][8];
+// development build only: %globaltimer in nanoseconds
 __device__ __forceinline__ unsigned long long probe_now() {
     unsigned long long t;
     asm volatile("mov.u64 %0, %%globaltimer;\n" : "=l"(t));
     return t;
 }
-#define PROBE_SET(i) do { if (threadIdx.x == 0) g_stream_probe[blockIdx.x][i] = probe_now(); } while (0)
-#define PROBE_MAX(i) do { if ((threadIdx.x & 31) == 0) atomicMax(&g_stream_probe[blockIdx.x][i], probe_now()); } while (0)
-#define PROBE_MIN(i) do { if ((threadIdx.x & 31) == 0) atomicMin(&g_stream_probe[blockIdx.x][i], probe_now()); } while (0)
-#else
-#define PROBE_SET(i)
-#define PROBE_MAX(i)
-#define PROBE_MIN(i)
 #endif
 __device__ __forceinline__ void mma_f16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
                                         uint32_t b0, uint32_t b1) {
@@ -76,11 +68,6 @@ __device__ __forceinline__ void mma_f16_zero(float (&d)[4], uint32_t a0, uint32_
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
     uint32_t d;
     asm("prmt.b32 %0, %1, %2, %3;\n" : "=r"(d) : "r"(a), "r"(b), "r"(sel));
-    return d;
-}
-__device__ __forceinline__ uint32_t lop3_and_or(uint32_t a, uint32_t b, uint32_t c) {  // (a & b) | c
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0xEA;\n" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
 __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
@@ -303,6 +290,71 @@ __device__ __forceinline__ void coarse_set_int4c(uint32_t rb, uint32_t t, uint32
     }
     acc0 = (d[0] + e[0]) + (d[1] + e[1]);
     acc1 = (d[2] + e[2]) + (d[3] + e[3]);
+}
+
+// ---- tcgen05 / mbarrier plumbing ------------------------------------------------------------------
+constexpr uint32_t TC_SPIN = 1u << 22;            // polls of one mbarrier wait before it gives up (~0.2 s)
+
+__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(addr));
+    return v;
+}
+// a threshold's score word as a float; words at or below the key of -inf mean "no threshold yet"
+__device__ __forceinline__ float thr_float(uint32_t key) { return key > 0x00800000u ? key_score(key) : -INFINITY; }
+__device__ __forceinline__ void mbar_init(uint32_t addr, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(addr), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t addr) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(addr) : "memory");
+}
+// false when the phase did not complete within TC_SPIN polls
+__device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
+    for (uint32_t i = 0; i < TC_SPIN; ++i) {
+        uint32_t ok;
+        asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+                     : "=r"(ok) : "r"(addr), "r"(parity) : "memory");
+        if (ok) return true;
+        if (i > 64) __nanosleep(64);
+    }
+    return false;
+}
+// Named barrier `id` over `nthreads` threads that also tells every one of them whether any brought `fail`: the
+// warps of a role leave their loop together, so that none is left waiting at a later barrier of the role.
+__device__ __forceinline__ bool role_any(uint32_t id, uint32_t nthreads, bool fail) {
+    uint32_t any;
+    asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %1, 0;\nbar.red.or.pred p, %2, %3, q;\nselp.u32 %0, 1, 0, p;\n}\n"
+                 : "=r"(any) : "r"((uint32_t)fail), "r"(id), "r"(nthreads) : "memory");
+    return any != 0;
+}
+// K-major, 128-byte swizzle, 8-row groups 1024 bytes apart (tcgen05 shared-memory matrix descriptor)
+__device__ __forceinline__ uint64_t tc_desc(uint32_t saddr) {
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) |
+           ((uint64_t)2 << 61);
+}
+// One lane of a warp, to be called where the warp is known to be converged (a kernel's start; the result stays in a predicate).
+// tcgen05 instructions take uniform registers: behind elect.sync and a warp index taken by shuffle the compiler knows a branch to be one
+// thread's, behind `threadIdx.x == 0` it issues each of them through a loop over the active lanes (a lone tcgen05.mma: 217 against
+// 109 cycles).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred p;\nelect.sync _|p, 0xFFFFFFFF;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(p));
+    return p != 0;
+}
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ void tc_commit(uint32_t mbar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
+}
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
+        "%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
+          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
+          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
+          "=r"(v[31])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
 // Bucket of a score inside [smin, smin + 256 / inv): monotone in the score.
@@ -618,7 +670,42 @@ __device__ uint32_t block_select_multi(uint64_t* keys, uint32_t cap, int* cnt, i
 // warp, query and set), counted in the row's histogram, and the threshold is re-derived from that
 // histogram from time to time - the counts are of real tiles, so the lower edge of the highest
 // bucket whose count from the top reaches k is a proven lower bound of the k-th best score, for
-// all CTAs at once.  Nothing in the hot loop waits for another warp or CTA.
+// all CTAs at once.
+
+// A whole warp: the bound that a row's histogram proves (0 = none): the lower edge of the highest bucket whose count from the
+// top reaches k, minus half a bucket and a few ulps: every counted key of the buckets from there on is above it whatever
+// the rounding of the bucket arithmetic.  r: the row's bucket mapping.
+__device__ __forceinline__ uint32_t hist_bound(const uint32_t* hist, float2 r, uint32_t k, int lane) {
+    const uint32_t* hq = hist + 248 - 8 * lane;
+    uint32_t c[8];  // buckets 255-8l .. 248-8l (descending)
+    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(c[7]), "=r"(c[6]), "=r"(c[5]), "=r"(c[4]) : "l"(hq));
+    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(c[3]), "=r"(c[2]), "=r"(c[1]), "=r"(c[0]) : "l"(hq + 4));
+    uint32_t tot = 0;
+#pragma unroll
+    for (int jj = 0; jj < 8; ++jj) tot += c[jj];
+    uint32_t incl = tot;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    const unsigned ok = __ballot_sync(0xFFFFFFFFu, incl >= k);
+    uint32_t ek = 0;
+    if (ok != 0u && lane == __ffs(ok) - 1) {
+        uint32_t run = incl - tot;
+        int b = 0;
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj) {
+            if (run + c[jj] >= k) { b = 255 - 8 * lane - jj; break; }
+            run += c[jj];
+        }
+        if (b >= 1) {
+            const uint32_t e = score_key(r.x + ((float)b - 0.5f) / r.y);
+            ek = e > 8u ? e - 8u : 0u;
+        }
+    }
+    return __reduce_max_sync(0xFFFFFFFFu, ek);
+}
 
 // A whole warp: raise the threshold of query row Q (shared word *pvh) from the row's histogram
 // and from what other CTAs have proven.
@@ -626,37 +713,7 @@ __device__ __forceinline__ void stream_refresh_threshold(const ScoreArgs& a, uin
     const unsigned long long seen = *reinterpret_cast<volatile unsigned long long*>(a.gpivot + Q);
     uint32_t best = (uint32_t)(seen >> 32);
     if (r.y != 0.0f) {
-        const uint32_t* hq = a.ghist + (size_t)Q * 256 + 248 - 8 * lane;
-        uint32_t c[8];  // buckets 255-8l .. 248-8l (descending)
-        asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(c[7]), "=r"(c[6]), "=r"(c[5]), "=r"(c[4]) : "l"(hq));
-        asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(c[3]), "=r"(c[2]), "=r"(c[1]), "=r"(c[0]) : "l"(hq + 4));
-        uint32_t tot = 0;
-#pragma unroll
-        for (int jj = 0; jj < 8; ++jj) tot += c[jj];
-        uint32_t incl = tot;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const unsigned ok = __ballot_sync(0xFFFFFFFFu, incl >= a.k);
-        uint32_t ek = 0;
-        if (ok != 0u && lane == __ffs(ok) - 1) {
-            uint32_t run = incl - tot;
-            int b = 0;
-#pragma unroll
-            for (int jj = 0; jj < 8; ++jj) {
-                if (run + c[jj] >= a.k) { b = 255 - 8 * lane - jj; break; }
-                run += c[jj];
-            }
-            if (b >= 1) {
-                // half a bucket and a few ulps below the bucket's edge: every counted key of the
-                // buckets b.. is above this bound whatever the rounding of the bucket arithmetic
-                const uint32_t e = score_key(r.x + ((float)b - 0.5f) / r.y);
-                ek = e > 8u ? e - 8u : 0u;
-            }
-        }
-        ek = __reduce_max_sync(0xFFFFFFFFu, ek);
+        const uint32_t ek = hist_bound(a.ghist + (size_t)Q * 256, r, a.k, lane);
         if (ek > best) {
             best = ek;
             if (lane == 0) atomicMax(a.gpivot + Q, (unsigned long long)ek << 32);
@@ -671,10 +728,8 @@ __device__ __forceinline__ void stream_refresh_threshold(const ScoreArgs& a, uin
 // Separate instantiations.  A tile of another codec than the launch was arranged for flags the
 // work item's query rows, which the generic kernel then scores.
 // IL: the work items are interleaved shares of whole streams (see the planner); the plain instantiation keeps the
-// set arithmetic of contiguous ranges out of its loop.  DENSE: every score is written to a.scores (row q at
-// q * a.score_stride, tile i of the item at index_base + i; -inf for COLD slots) and nothing is filtered or appended:
-// full score vectors (slha_score_tiles, score_all, the softmax of observe_scores) at the streaming kernel's speed.
-template <int KIND, int NT, bool IL, bool DENSE = false>
+// set arithmetic of contiguous ranges out of its loop.
+template <int KIND, int NT, bool IL>
 __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
@@ -682,13 +737,6 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
     // shared layout: nf4 table | stage ring | B fragments | query sign words | thresholds | bucket mappings | flag
     const uint32_t lut_bytes = a.nf4_table ? NF4_LUT_BYTES : 0;  // the table is left out when no NF4 tile is expected
     uint2* lut = reinterpret_cast<uint2*>(smem);
-#ifdef SLHA_STREAM_PROBE
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 8; ++i) g_stream_probe[blockIdx.x][i] = i == 6 ? ~0ull : 0ull;
-        g_stream_probe[blockIdx.x][0] = probe_now();
-    }
-    __syncthreads();
-#endif
     unsigned char* tail = smem + lut_bytes + (size_t)nwarps * MMA_DEPTH * MMA_SET_STRIDE;
     uint2* bq_w = reinterpret_cast<uint2*>(tail);                        // [9][32]
     uint32_t* qs_w = reinterpret_cast<uint32_t*>(tail + MMA_BQ_BYTES);   // [4][8]
@@ -779,7 +827,7 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
 #pragma unroll
         for (int i = 0; i < MMA_DEPTH - 1; ++i) issue();
         bool row_warm = true;
-        if (!DENSE && tid < 4) {
+        if (tid < 4) {
             // start from the threshold other CTAs have already proven for the row, and from the
             // row's bucket mapping if one has been published
             const bool have = tid < nq;
@@ -851,13 +899,13 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             bq_w[8 * 32 + lane] = make_uint2(bE, 0u);
             if (__any_sync(0xFFFFFFFFu, big) && lane == 0) bail[0] = 1;  // a query too large for the fp16 split
         }
+        // (from a barrier's vote, not from the flag word: a fast warp may raise the flag for an undecodable tile meanwhile)
+        const bool too_big = __syncthreads_or(big) != 0;
         // The barrier after the first round (below) pays when the round can supply k candidates to a row -- 16 per warp
         // of every CTA that works on the row -- and the rows do not already have thresholds (a CTA that starts its
         // second item on rows other CTAs have been scoring for a while).
         const bool all_warm = __syncthreads_and(row_warm) != 0;
-        const bool first_round_barrier = !DENSE && !all_warm && (uint64_t)a.k <= 16ull * (uint64_t)nwarps * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
-        PROBE_SET(1);
-        const bool too_big = bail[0] != 0;
+        const bool first_round_barrier = !all_warm && (uint64_t)a.k <= 16ull * (uint64_t)nwarps * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
         if (too_big) n_sets = 0;  // (the sets already on their way are waited for at the item's end and never read)
 
         uint32_t slot = 0, polls = 0;
@@ -870,11 +918,9 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
                 // Every warp of the CTA (and, started together, of the grid) has appended its first set
                 // unfiltered, so the rows' histograms hold 16 candidates per warp: first thresholds now,
                 // before the second sets are filtered.  (All warps pass here: `rounds` is the same for all.)
-                PROBE_MAX(2);
                 __syncthreads();
                 if (warp < nq) stream_refresh_threshold(a, it.query_begin + (uint32_t)warp, rng[warp], pvh + warp, lane);
                 __syncthreads();
-                PROBE_SET(3);
             }
             // (the ring advances in every iteration, also when this warp has no set in this round -- the short last round of
             // the stream can come anywhere in a rotated walk -- so that fetches and reads stay in step)
@@ -938,7 +984,7 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             // (257 and the relative slack cover the rounding of the bound itself.)  Only the INT4 launches
             // test for it: with a few CTAs per row and k / n of a few percent (the NF4 decode caches) nearly
             // every set holds a candidate and the test costs more than it saves.
-            const bool need = DENSE || KIND != 3 || round == 0 ||
+            const bool need = KIND != 3 || round == 0 ||
                               __any_sync(0xFFFFFFFFu, (mine && score_key(fmaf(lam0, 257.0f, c0 + fabsf(c0) * 1e-6f)) >= pv) ||
                                                           (mine && score_key(fmaf(lam1, 257.0f, c1 + fabsf(c1) * 1e-6f)) >= pv));
             if (need) {
@@ -959,15 +1005,6 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             if (sbase) {
                 live0 = live0 && sbase[t0] != ST_COLD;
                 live1 = live1 && sbase[t1] != ST_COLD;
-            }
-            if (DENSE) {
-                if (mine) {  // (eight lanes of a query hold eight consecutive tiles: 32-byte runs per row)
-                    float* row = a.scores + (size_t)Qt * a.score_stride + it.index_base;
-                    if (t0 < n) row[t0] = live0 ? sc0 : -INFINITY;
-                    if (t1 < n) row[t1] = live1 ? sc1 : -INFINITY;
-                }
-                __syncwarp();
-                continue;
             }
             if (round == 0) {
                 // First set of the warp: a row without a bucket mapping gets one from the 16 scores
@@ -1051,15 +1088,12 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             }
         }
         cp_async_wait<0>();
-        PROBE_MAX(4);
-        PROBE_MIN(6);
-        if (!DENSE && mine) {  // the unused rest of the warp's last chunk holds absent keys
+        if (mine) {  // the unused rest of the warp's last chunk holds absent keys
             for (uint32_t z = cur + (uint32_t)g; z < end; z += 8u) dst[z] = 0ull;
         }
         __syncthreads();
         // rows this CTA could not score on the tensor cores go to the generic kernel as a whole
         if (bail[0] && tid < nq) a.gflag[it.query_begin + tid] = 1u;
-        PROBE_SET(5);
     }
 }
 

@@ -1,0 +1,91 @@
+"""The tcgen05 scoring kernels at the edges of their blocks: a warp holds 32 tiles, a warpgroup's block 128, a round of a CTA
+384 or 512; up to four query rows go through score_stream_kernel (MIX3: score_mix3_kernel), sixteen or more through
+score_wide_kernel, any number through the dense kernels.  Oracle: compute_score_scalar.  Bound: the reference's own 1e-3 (1 + |s|)."""
+import numpy as np
+import pytest
+
+from oracle import pyoracle as ora
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+S = pytest.importorskip("slhav2_b200")
+F = np.float32
+LENS = [1, 31, 32, 33, 0, 127, 128, 129, 383, 385, 511, 513, 1025, 2111]
+
+
+def _layout(nq):
+    rows, tb = [], 0
+    for i, n in enumerate(LENS):
+        rows.append((tb, n, i * nq, nq, 5 * i))
+        tb += n
+    return rows, tb, nq * len(LENS)
+
+
+def _inputs(codec, nq, seed):
+    rows, n, total = _layout(nq)
+    tiles = H.random_tiles(n, codec, seed=seed + codec, warm_every=7, nocorr_every=5)
+    qc, qs = H.random_queries(total, seed + 50 + codec)
+    return rows, tiles, qc, qs, total
+
+
+@pytest.mark.parametrize("codec", range(7))
+@pytest.mark.parametrize("nq", [1, 4, 6, 17, 64])
+def test_top_k_of_segments_around_the_block_sizes(codec, nq):
+    rows, tiles, qc, qs, total = _inputs(codec, nq, 900)
+    k = 24
+    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, total, k)
+    for tb, n, qb, _, base in rows:
+        for j in range(qb, qb + nq):
+            m = min(n, k)
+            assert cnt[j] == m
+            assert np.all(idx[j, m:] == 0xFFFFFFFF) and np.all(np.isneginf(sc[j, m:]))
+            if not n:
+                continue
+            want = ora.score_tiles(tiles[tb:tb + n], qc[j], qs[j])
+            got = idx[j, :m].astype(np.int64) - base
+            assert len(set(got)) == m and got.min() >= 0 and got.max() < n
+            assert np.all(np.abs(sc[j, :m] - want[got]) <= 1e-3)
+            assert np.all(np.diff(sc[j, :m]) <= 0)
+            # whatever is missing from the winners ties with the last of them
+            rest = np.delete(want, got)
+            assert not len(rest) or rest.max() <= want[got].min() + 2e-3
+
+
+@pytest.mark.parametrize("codec", range(7))
+@pytest.mark.parametrize("nq", [1, 4, 17, 64])
+def test_dense_scores_of_segments_around_the_block_sizes(codec, nq):
+    rows, tiles, qc, qs, total = _inputs(codec, nq, 950)
+    row_len = max(LENS) + 100
+    out = np.full((total, row_len), 9.0, F)
+    S.score_segments(S.to_device(tiles), S.make_segments(rows), qc, qs, total, out, np.arange(total, dtype=np.uint64) * row_len, row_len, fill=-3.0)
+    for tb, n, qb, _, base in rows:
+        for j in range(qb, qb + nq):
+            if n:
+                want = ora.score_tiles(tiles[tb:tb + n], qc[j], qs[j])
+                err = np.abs(out[j, base:base + n] - want)
+                assert np.all(err <= 1e-3) and np.all(err <= 1e-3 * (1 + np.abs(want)))
+            assert np.all(out[j, base + n:] == -3.0)
+
+
+@pytest.mark.parametrize("nq", [3, 16])
+def test_segments_of_different_codecs_in_one_call(nq):
+    # a CTA decodes the kind of its first tile: the rows of the other segments take another pass, the results stay the same
+    parts = [H.random_tiles(n, c, seed=70 + c, warm_every=9, nocorr_every=4) for c, n in zip((2, 5, 0, 3, 4), (700, 513, 129, 2049, 40))]
+    tiles = np.concatenate(parts)
+    qc, qs = H.random_queries(5 * nq, 71)
+    rows, tb = [], 0
+    for i, p in enumerate(parts):
+        rows.append((tb, len(p), i * nq, nq, 0))
+        tb += len(p)
+    row_len = 2049
+    out = np.zeros((5 * nq, row_len), F)
+    dt, seg = S.to_device(tiles), S.make_segments(rows)
+    S.score_segments(dt, seg, qc, qs, 5 * nq, out, np.arange(5 * nq, dtype=np.uint64) * row_len, row_len)
+    idx, sc, _ = S.score_topk(dt, seg, qc, qs, 5 * nq, 32)
+    for tb, n, qb, _, _ in rows:
+        for j in range(qb, qb + nq):
+            want = ora.score_tiles(tiles[tb:tb + n], qc[j], qs[j])
+            assert np.all(np.abs(out[j, :n] - want) <= 1e-3 * (1 + np.abs(want)))
+            m = min(n, 32)
+            assert np.all(np.abs(sc[j, :m] - want[idx[j, :m]]) <= 1e-3)
+            assert np.all(np.abs(sc[j, :m] - np.sort(want)[::-1][:m]) <= 2e-3)
