@@ -21,7 +21,9 @@ size_t mma_smem_bytes(int nwarps, bool nf4_table) {  // (keep in step with the k
     return (size_t)(nf4_table ? NF4_LUT_BYTES : 0) + (size_t)nwarps * MMA_DEPTH * MMA_SET_STRIDE + MMA_BQ_BYTES + 128 + 16 + 32 + 32 + 16;
 }
 constexpr int STREAM_THREADS = SLHA_STREAM_THREADS;
-constexpr uint32_t STREAM_LEAST = 2048;  // tiles a CTA is given at least
+// Tiles a CTA is given at least: two rounds of score_stream_kernel's 24 warps.  us per call with 512 / 768 / 2048: 4096 INT4 tiles,
+// one query 27.4 / 26.7 / 32.9; 8 segments x 2048 tiles 27.4 / 26.9 / 36.2; 4 x 32 768 TQ3 tiles 45.6 / 45.1 / 62.8.
+constexpr uint32_t STREAM_LEAST = 768;
 // kind of a launch by the flags of a tile (dequant_at's precedence)
 int stream_kind(uint32_t flags) { return (flags & F_MIXED) ? 1 : ((flags & F_TQ3) ? 2 : ((flags & F_MIX3) ? 4 : ((flags & F_NF4) ? 0 : 3))); }
 // the same for a codec hint: bit 0 NF4 tiles expected, bit 1 mixed 8/4 only, bit 2 TQ3 only, bit 3 MIX3 only
@@ -181,6 +183,10 @@ struct Plan {
     uint64_t* d_gbuf = nullptr;              // per query: gcap candidate keys of the tensor-core kernel
     uint32_t gcap = 0;
     size_t gstate_bytes = 0;
+    // Short shares (below 4096 tiles per CTA, ten rounds): the thresholds raised while scoring are stale or absent, and the compaction or
+    // the merge takes the row's threshold from its complete histogram first.  Longer shares have just refreshed theirs: there the
+    // extra read of the histogram cost 2 to 6 us of 55 to 100.
+    bool late_threshold = false;
     bool state_clean = false;  // the previous call's merge left the streaming state cleared (see StreamLists::finish)
     uint32_t compact_splits = 0, selcap = 0;  // optional compaction pass before the merge (few rows, long buffers)
     // wide scoring (16 or more queries per segment, INT4 / TQ3 launches): work items of up to 64 query rows for score_wide_kernel
@@ -512,6 +518,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     if (p->wide) p->gcap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(p->gcap, 4ull * WIDE_M * wide_parts + 16ull * k), ((uint64_t)longest + 63) / 64 * 64);
     p->gstate_bytes = nq * (1024 + 8 + 8 + 4 + 4 + 4 + 8);  // histogram, threshold, mapping, count, flag, compacted count, statistics
     p->state_clean = false;
+    p->late_threshold = p->use_mma && total / (uint64_t)sms < 4096;
     // few rows with long buffers: several CTAs per row compact the survivors before the merge
     // (a slice of at most 1024 slots per CTA: one round of four keys per thread)
     p->compact_splits = (p->use_mma && nq < 128 && p->gcap >= 8192) ? (uint32_t)std::min<size_t>(64, std::max<size_t>((296 + nq - 1) / nq, (p->gcap + 1023) / 1024)) : 0;
@@ -858,22 +865,28 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         SLHA_CUDA(cudaFuncSetAttribute(topk_merge_kernel<CompLists>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         SLHA_CUDA(cudaFuncSetAttribute(topk_merge_kernel<PairLists>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         SLHA_CUDA(cudaFuncSetAttribute(topk_merge_kernel<StreamLists>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-        SLHA_CUDA(cudaFuncSetAttribute(stream_compact_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        SLHA_CUDA(cudaFuncSetAttribute(stream_compact_kernel<true>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        SLHA_CUDA(cudaFuncSetAttribute(stream_compact_kernel<false>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         configured[c->device & 15] = true;
     }
     if (mma) {
         uint32_t* gselcnt = am.gflag + nq;
         const uint32_t cap_s = p->selcap;
         if (p->compact_splits) {
-            stream_compact_kernel<<<dim3(p->compact_splits, (uint32_t)nq), 256, 0, c->stream>>>(
-                p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap, (uint64_t*)p->b_gsel.p, gselcnt, cap_s, p->compact_splits);
+            const dim3 cgrid(p->compact_splits, (uint32_t)nq);
+            if (p->late_threshold)
+                stream_compact_kernel<true><<<cgrid, 256, 0, c->stream>>>(p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap, (uint64_t*)p->b_gsel.p, gselcnt,
+                                                                          cap_s, p->compact_splits, am.ghist, k);
+            else
+                stream_compact_kernel<false><<<cgrid, 256, 0, c->stream>>>(p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap, (uint64_t*)p->b_gsel.p, gselcnt,
+                                                                           cap_s, p->compact_splits, am.ghist, k);
             count_launch();
             SLHA_CUDA(cudaGetLastError());
         }
         StreamLists L{p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap,
                       p->compact_splits ? (const uint64_t*)p->b_gsel.p : nullptr, gselcnt, cap_s,
                       CompLists{p->d_cand_keys, p->d_cand_cnt, p->d_q_list_begin, p->d_q_list_count, p->list_cap},
-                      am.ghist, gselcnt + nq};
+                      am.ghist, p->late_threshold ? k : 0u, gselcnt + nq};
         topk_merge_kernel<StreamLists><<<(uint32_t)nq, merge_threads(cap_s), merge_smem(cap_s, p->kp2), c->stream>>>(
             L, k, p->kp2, cap_s, d_out_index, d_out_score, d_out_count);
         p->state_clean = cudaPeekAtLastError() == cudaSuccess;

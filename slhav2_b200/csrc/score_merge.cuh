@@ -82,13 +82,24 @@ struct StreamLists {
     // The merge is the last reader of a row's streaming state: it leaves the state cleared for the next call
     // (which then needs no memset in front of its score kernel) and keeps the row's figures for the statistics call.
     __device__ uint64_t floor_key(uint32_t, uint32_t, uint64_t*, uint32_t, int*) const { return 0ull; }  // (the row's threshold filters already)
-    __device__ bool wait_ready(int*) const { return true; }
+    // (the merge's first step) the row's final threshold, unless the compaction has used it already
+    __device__ bool wait_ready(int*) const {
+        if (!k) return true;
+        const uint32_t Q = blockIdx.x;
+        if (!gsel && !gflag[Q] && threadIdx.x < 32) {
+            const unsigned long long t = final_threshold(ghist + (size_t)Q * 256, gpivot[Q], gpivot[gridDim.x + Q], k, (int)threadIdx.x);
+            if (threadIdx.x == 0) *const_cast<volatile unsigned long long*>(gpivot + Q) = t;
+        }
+        __syncthreads();
+        return true;
+    }
     __device__ ListView view(uint32_t Q, uint32_t part) const {
         if (gflag[Q]) return items.view(Q, part);
         if (compacted(Q)) return ListView{gsel + (size_t)Q * selcap, 0ull, gselcnt[Q]};
         return ListView{gbuf + (size_t)Q * gcap, gpivot[Q], min(gcount[Q], gcap)};
     }
     uint32_t* ghist;     // [nq][256]; the state arrays follow it in one allocation
+    uint32_t k;          // 0: the threshold stays as the scoring kernel left it
     uint32_t* stats;     // [nq][2] candidates appended, handed to the generic kernel
     __device__ void finish(uint32_t Q) const {
         for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x) ghist[(size_t)Q * 256 + i] = 0u;
@@ -232,15 +243,28 @@ struct PairLists {  // (index, score) lists laid out [list][query][k_in]
 // per row would read them alone.  Here `splits` CTAs per row each filter a slice of the row's buffer
 // and append the survivors (keys at or above the threshold) to a compact list; a row whose survivors
 // exceed `selcap` keeps a count above it, which sends the merge back to the full buffer.
+// LATE: the row's threshold from its complete histogram first (else it stays as the scoring kernel left it).
+template <bool LATE>
 __global__ void __launch_bounds__(256) stream_compact_kernel(const uint64_t* gbuf, const uint32_t* gcount, const uint32_t* gflag,
                                                              const unsigned long long* gpivot, uint32_t gcap, uint64_t* gsel,
-                                                             uint32_t* gselcnt, uint32_t selcap, uint32_t splits) {
+                                                             uint32_t* gselcnt, uint32_t selcap, uint32_t splits, const uint32_t* ghist, uint32_t k) {
     const uint32_t Q = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
     if (gflag[Q]) return;
+    uint64_t pv;
+    if (LATE) {
+        __shared__ unsigned long long pv_s;
+        if (tid < 32) {
+            const unsigned long long t = final_threshold(ghist + (size_t)Q * 256, gpivot[Q], gpivot[gridDim.y + Q], k, (int)lane);
+            if (tid == 0) pv_s = t;
+        }
+        __syncthreads();
+        pv = pv_s;
+    } else {
+        pv = gpivot[Q];
+    }
     const uint32_t len = min(gcount[Q], gcap);
     const uint32_t per = ((len + splits - 1) / splits + 3) & ~3u;
     const uint32_t lo = blockIdx.x * per, hi = min(len, lo + per);
-    const uint64_t pv = gpivot[Q];
     const uint64_t* src = gbuf + (size_t)Q * gcap;
     uint64_t* dst = gsel + (size_t)Q * selcap;
     for (uint32_t j0 = lo; j0 < hi; j0 += 4 * blockDim.x) {

@@ -722,6 +722,14 @@ __device__ __forceinline__ void stream_refresh_threshold(const ScoreArgs& a, uin
     if (lane == 0 && best > *reinterpret_cast<volatile uint32_t*>(pvh)) atomicMax(pvh, best);
 }
 
+// A whole warp, once a row's candidates are all in its buffer: the row's threshold from its complete histogram.  Calls whose
+// rows are scored in a round or two have raised none, or a stale one, while scoring.
+__device__ __forceinline__ unsigned long long final_threshold(const uint32_t* hist, unsigned long long pivot, unsigned long long mapping, uint32_t k, int lane) {
+    const float2 r = make_float2(__uint_as_float((uint32_t)mapping), __uint_as_float((uint32_t)(mapping >> 32)));
+    const unsigned long long e = r.y != 0.0f ? (unsigned long long)hist_bound(hist, r, k, lane) << 32 : 0ull;
+    return e > pivot ? e : pivot;
+}
+
 // KIND 0: nibble codecs (INT4, MX-INT4, NF4 through the shared-memory table); 1: the launch scores
 // mixed 8/4 tiles; 2: TQ3 tiles, rewritten in shared memory as nibble rows (2 code + correction
 // bit) before the INT4 path scores them; 3: INT4 / MX-INT4 tiles only (scale folded into A).
