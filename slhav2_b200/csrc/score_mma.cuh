@@ -295,18 +295,10 @@ __device__ __forceinline__ void coarse_set_int4c(uint32_t rb, uint32_t t, uint32
 // ---- tcgen05 / mbarrier plumbing ------------------------------------------------------------------
 constexpr uint32_t TC_SPIN = 1u << 22;            // polls of one mbarrier wait before it gives up (~0.2 s)
 
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-    uint32_t v;
-    asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(v) : "r"(addr));
-    return v;
-}
 // a threshold's score word as a float; words at or below the key of -inf mean "no threshold yet"
 __device__ __forceinline__ float thr_float(uint32_t key) { return key > 0x00800000u ? key_score(key) : -INFINITY; }
 __device__ __forceinline__ void mbar_init(uint32_t addr, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(addr), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint32_t addr) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(addr) : "memory");
 }
 // false when the phase did not complete within TC_SPIN polls
 __device__ __forceinline__ bool mbar_wait(uint32_t addr, uint32_t parity) {
@@ -344,17 +336,6 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
 __device__ __forceinline__ void tc_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(mbar) : "memory");
-}
-__device__ __forceinline__ void tc_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,"
-        "%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]),
-          "=r"(v[31])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
 }
 
 // Bucket of a score inside [smin, smin + 256 / inv): monotone in the score.
