@@ -482,6 +482,9 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
             const uint32_t b = block_of(round);
             // (the ring advances in every iteration, also when this warpgroup has no block in this round -- the short last round
             // of the stream can come anywhere in a rotated walk -- so that fetches and reads stay in step)
+            // issue() refills the slot that was read last, every lane its chunks of other lanes' rows: all lanes have read theirs
+            // (they part company over COLD slots, rows past the end and residual words that only some need)
+            __syncwarp();
             issue();
             cp_async_wait<ST_DEPTH - 1>();
             __syncwarp();
@@ -673,7 +676,6 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                 }
                 continue;
             }
-            __syncwarp();
             // In turn, a warp raises the threshold of query (warp & 3): after its 2nd and 4th block (the first
             // thresholds come from the barrier after the first round), then every 8 blocks, the warps of a
             // query staggered.  A stale threshold costs appends (each one a store, a histogram count and,
