@@ -292,6 +292,12 @@ __device__ __forceinline__ void coarse_set_int4c(uint32_t rb, uint32_t t, uint32
     acc1 = (d[2] + e[2]) + (d[3] + e[3]);
 }
 
+// four consecutive elements of a query row (a caller's query rows start at any float)
+__device__ __forceinline__ float4 load_q4(const float* p) {
+    if (reinterpret_cast<uintptr_t>(p) & 15u) return make_float4(p[0], p[1], p[2], p[3]);
+    return *reinterpret_cast<const float4*>(p);
+}
+
 // ---- tcgen05 / mbarrier plumbing ------------------------------------------------------------------
 constexpr uint32_t TC_SPIN = 1u << 22;            // polls of one mbarrier wait before it gives up (~0.2 s)
 
@@ -851,11 +857,8 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
                     // group 0 = dims 2t, 2t+1 (8-bit levels, plain in both slots, so both carry 16x the
                     // query), groups 1..7 = INT4 groups of dims 16 j - 8 ..
                     const int dim0 = !(KIND == 1) ? 16 * j + 4 * t : (j == 0 ? 0 : 16 * j - 8 + 4 * t);
-                    float4 x = *reinterpret_cast<const float4*>(q + dim0);
-                    if (KIND == 1 && j == 0) {
-                        const float2 y = *reinterpret_cast<const float2*>(q + 2 * t);
-                        x = make_float4(y.x, 16.0f * y.y, 0.0f, 0.0f);
-                    }
+                    float4 x = load_q4(q + dim0);
+                    if (KIND == 1 && j == 0) x = make_float4(q[2 * t], 16.0f * q[2 * t + 1], 0.0f, 0.0f);
                     v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w;
                 }
 #pragma unroll

@@ -420,11 +420,11 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                     const float* q = a.q_coarse + (size_t)(it.query_begin + qi) * D_C;
                     constexpr bool HEAD = KIND == 1 || KIND == 4;
                     if (HEAD && i < 2) {  // slots 0..3: the scale byte's high nibble's products of dims 4 i .., 4..7 the low nibble's
-                        const float4 x = *reinterpret_cast<const float4*>(q + 4 * i);
+                        const float4 x = load_q4(q + 4 * i);
                         v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = x.x; v[5] = x.y; v[6] = x.z; v[7] = x.w;
                     } else if (i < 16) {
                         const int d0 = HEAD ? 8 * (i - 1) : 8 * i;
-                        const float4 x = *reinterpret_cast<const float4*>(q + d0), y = *reinterpret_cast<const float4*>(q + d0 + 4);
+                        const float4 x = load_q4(q + d0), y = load_q4(q + d0 + 4);
                         if (KIND == 0) {
                             v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
                         } else {

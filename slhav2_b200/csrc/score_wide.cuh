@@ -177,7 +177,7 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         if (all_blocks) fetch(0);
         for (int e = tid; e < WIDE_NQ * D_C / 4; e += WIDE_THREADS) {
             const int qi = e >> 5;
-            reinterpret_cast<float4*>(qf)[e] = qi < nq ? reinterpret_cast<const float4*>(a.q_coarse + (size_t)(it.query_begin + qi) * D_C)[e & 31] : make_float4(0, 0, 0, 0);
+            reinterpret_cast<float4*>(qf)[e] = qi < nq ? load_q4(a.q_coarse + (size_t)(it.query_begin + qi) * D_C + 4 * (e & 31)) : make_float4(0, 0, 0, 0);
         }
         qs_w[tid] = (tid >> 3) < nq ? a.q_sign[(size_t)(it.query_begin + (tid >> 3)) * 8 + (tid & 7)] : 0u;
         if (DENSE && tid < WIDE_NQ) roff[tid] = tid < nq ? a.row_offset[it.query_begin + tid] : 0ull;

@@ -33,3 +33,25 @@ def test_dense_scores_of_an_arena_with_scattered_cold_slots(codec):
         assert np.all(np.abs(scores - want) <= 1e-4 * (1 + np.abs(want)))
         first = scores if first is None else first
         assert np.array_equal(scores, first)
+
+
+@pytest.mark.parametrize("codec", range(7))
+@pytest.mark.parametrize("nq", [1, 4, 17])
+def test_query_rows_may_start_at_any_float(codec, nq):
+    # query rows in device memory that start 4, 8 and 12 bytes behind a 16-byte boundary: the same results as from the boundary
+    n, k = 3000, 16
+    tiles = H.random_tiles(n, codec, seed=520 + codec)
+    qc, qs = H.random_queries(nq, 530)
+    dt, ds = S.to_device(tiles), S.to_device(qs)
+    long_tiles = S.to_device(np.tile(tiles, 11))  # (score_tiles takes another kernel from 32 768 tiles on)
+    seg, off = S.make_segments([(0, n, 0, nq, 0)]), np.arange(nq, dtype=np.uint64) * n
+
+    def scores(q):
+        i, s, c = S.score_topk(dt, seg, q, ds, nq, k)
+        return [i, s, c, S.score_segments(dt, seg, q, ds, nq, np.zeros((nq, n), F), off, n), S.score_tiles(long_tiles, 11 * n, q, ds, nq, np.zeros((nq, 11 * n), F))]
+
+    want = scores(S.to_device(qc))
+    for shift in (1, 2, 3):
+        flat = S.to_device(np.concatenate([np.zeros(shift, F), qc.reshape(-1)]))
+        for a, b in zip(scores(flat.view(4 * shift, qc.nbytes)), want):
+            assert np.array_equal(a, b)
