@@ -15,6 +15,7 @@
 namespace slha {
 
 Status cuda_status(cudaError_t e, const char* what) {
+    cudaGetLastError();  // (reported here, not once more by the next call's launch check)
     return Status(SLHA_ERR_DEVICE, std::string("CUDA error: ") + cudaGetErrorString(e) + " in " + what);
 }
 
@@ -28,6 +29,21 @@ struct Block {
     char* p = nullptr;
     size_t cap = 0, off = 0;
 };
+// Page-locked staging of the small tables that calls upload (ctx_upload): a copy reads its slot until the slot's event, so a
+// slot is written again only after that.  Given back when the thread ends.
+constexpr int UPLOAD_SLOTS = 4;                    // uploads of a thread that may wait behind its kernels
+constexpr size_t UPLOAD_MOST = (size_t)1 << 20;    // larger tables are copied from where they lie, and waited for
+struct UploadSlot {
+    void* p = nullptr;
+    size_t cap = 0;
+    cudaEvent_t done = nullptr;
+    bool pending = false;
+    ~UploadSlot() {
+        if (pending) cudaEventSynchronize(done);
+        if (done) cudaEventDestroy(done);
+        if (p) cudaFreeHost(p);
+    }
+};
 struct ThreadState {
     int device = 0;
     bool device_chosen = false;
@@ -37,6 +53,8 @@ struct ThreadState {
     bool ctx_init[16] = {false};
     std::vector<Block> blocks[16];
     std::vector<std::pair<void*, size_t>> hblocks[16];
+    UploadSlot upload[16][UPLOAD_SLOTS];
+    uint32_t upload_next[16] = {0};
     // Arena reuse across streams: a call on a caller-supplied stream may return while its
     // kernels still read the arena; the event marks the end of that work, and a later call on
     // ANOTHER stream waits for it before it reuses the arena (same stream: stream order suffices).
@@ -105,6 +123,47 @@ Status ctx_host_scratch(Ctx* c, size_t bytes, void** out) {
     return Status();
 }
 
+Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SLHA_CUDA(cudaStreamIsCapturing(c->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+        // a graph would keep the address of host memory that this call's successors write again: refused, and the capture ends
+        // as invalid, like everywhere the library has to wait for a stream
+        SLHA_CUDA(cudaStreamSynchronize(c->stream));
+        return Status(SLHA_ERR_DEVICE, "this call cannot be captured into a graph");
+    }
+    SLHA_TRY(ctx_device_scratch(c, bytes, dev));
+    if (bytes > UPLOAD_MOST) {
+        SLHA_CUDA(cudaMemcpyAsync(*dev, src, bytes, cudaMemcpyHostToDevice, c->stream));
+        SLHA_CUDA(cudaStreamSynchronize(c->stream));
+        return Status();
+    }
+    UploadSlot& s = tls.upload[c->device][tls.upload_next[c->device]++ % UPLOAD_SLOTS];
+    if (s.pending) {
+        SLHA_CUDA(cudaEventSynchronize(s.done));
+        s.pending = false;
+    }
+    if (s.cap < bytes) {
+        if (s.p) SLHA_CUDA(cudaFreeHost(s.p));
+        s.p = nullptr;
+        s.cap = 0;
+        size_t want = (size_t)64 << 10;
+        while (want < bytes) want <<= 1;
+        SLHA_CUDA(cudaMallocHost(&s.p, want));
+        s.cap = want;
+    }
+    if (!s.done) SLHA_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
+    std::memcpy(s.p, src, bytes);
+    SLHA_CUDA(cudaMemcpyAsync(*dev, s.p, bytes, cudaMemcpyHostToDevice, c->stream));
+    const cudaError_t e = cudaEventRecord(s.done, c->stream);
+    if (e != cudaSuccess) {
+        cudaStreamSynchronize(c->stream);  // (no event to wait for later: the copy is over before the slot is used again)
+        return cuda_status(e, "cudaEventRecord");
+    }
+    s.pending = true;
+    return Status();
+}
+
 CallScope::CallScope() {
     st = get_ctx(&c);
     if (!st.ok()) return;
@@ -141,7 +200,10 @@ CallScope::~CallScope() {
         cudaStreamSynchronize(c->stream);  // no event to be had: drain instead
         return;
     }
-    cudaEventRecord(ev, c->stream);
+    if (cudaEventRecord(ev, c->stream) != cudaSuccess) {  // (a capture that the call has ended as invalid)
+        cudaGetLastError();
+        return;
+    }
     tls.arena_stream[c->device] = c->stream;
     tls.arena_pending[c->device] = true;
 }

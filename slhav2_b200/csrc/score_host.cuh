@@ -599,7 +599,7 @@ Status launch_validate_tiles(Ctx* c, const SciRustSlhaTile* tiles, size_t n, uns
     return Status();
 }
 
-// One upload of several small host arrays into the call's scratch (pageable sources: cudaMemcpyAsync returns once they are staged).
+// One upload of several small host arrays into the call's scratch.
 struct Blob {
     std::vector<unsigned char> bytes;
     template <typename T>
@@ -610,9 +610,7 @@ struct Blob {
         return at;
     }
     Status upload(Ctx* c, unsigned char** dev) {
-        SLHA_TRY(ctx_device_scratch(c, bytes.size(), (void**)dev));
-        SLHA_CUDA(cudaMemcpyAsync(*dev, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, c->stream));
-        return Status();
+        return ctx_upload(c, bytes.data(), bytes.size(), (void**)dev);
     }
 };
 

@@ -55,3 +55,78 @@ def test_query_rows_may_start_at_any_float(codec, nq):
         flat = S.to_device(np.concatenate([np.zeros(shift, F), qc.reshape(-1)]))
         for a, b in zip(scores(flat.view(4 * shift, qc.nbytes)), want):
             assert np.array_equal(a, b)
+
+
+class _CapturedStream:
+    """A stream of the CUDA runtime in capture mode (relaxed), set as the library's."""
+
+    def __enter__(self):
+        import ctypes as C
+
+        S.load_library()
+        self.rt, self.stream = C.CDLL("libcudart.so.12"), C.c_void_p()
+        assert self.rt.cudaStreamCreateWithFlags(C.byref(self.stream), 1) == 0
+        S.set_stream(self.stream.value)
+        assert self.rt.cudaStreamBeginCapture(self.stream, 2) == 0
+        return self
+
+    def __exit__(self, *exc):
+        import ctypes as C
+
+        graph = C.c_void_p()
+        self.rt.cudaStreamEndCapture(self.stream, C.byref(graph))
+        self.captured = bool(graph.value)
+        self.rt.cudaGetLastError()
+        S.set_stream(None)
+        self.rt.cudaStreamDestroy(self.stream)
+
+
+def test_dense_calls_with_tables_refuse_a_stream_that_is_captured():
+    # a graph would keep the address of the call's host tables: the call fails and so does the capture; afterwards it works as before
+    n, nq = 33000, 3
+    tiles = np.tile(H.random_tiles(1100, 1, seed=540), 30)
+    qc, qs = H.random_queries(nq, 541)
+    dt, dq, ds, out = S.to_device(tiles), S.to_device(qc), S.to_device(qs), S.DeviceBuffer(nq * n * 4)
+    seg, off = S.make_segments([(0, n, 0, nq, 0)]), np.arange(nq, dtype=np.uint64) * n
+    want = S.score_tiles(dt, n, dq, ds, nq, np.zeros((nq, n), F))
+    for call in (lambda: S.score_tiles(dt, n, dq, ds, nq, out), lambda: S.score_segments(dt, seg, dq, ds, nq, out, off, n)):
+        with _CapturedStream() as cap:
+            with pytest.raises(S.SlhaError) as e:
+                call()
+            assert e.value.code == S.ERR_DEVICE
+        assert not cap.captured
+        call()
+        S.synchronize()
+        assert np.array_equal(out.download(F, nq * n).reshape(nq, n), want)
+
+
+def test_dense_calls_of_different_shapes_queued_behind_one_another():
+    # more calls in flight on one stream than the library keeps table slots for, each with tables of its own, some of them large
+    import ctypes as C
+
+    tiles = np.tile(H.random_tiles(3000, 4, seed=550), 12)
+    qc, qs = H.random_queries(40, 551)
+    dt, dq, ds = S.to_device(tiles), S.to_device(qc), S.to_device(qs)
+    rng = np.random.default_rng(552)
+    shapes = [(int(rng.integers(1, 30000)), int(rng.integers(1, 41))) for _ in range(9)] + [(32000, 9)]
+    jobs = []
+    for n, nq in shapes:
+        parts = 30000 if n > 30000 else min(n, 3)  # (30 000 segments: tables of more than a megabyte)
+        cut = np.linspace(0, n, parts + 1).astype(int)
+        rows = [(cut[i], cut[i + 1] - cut[i], 0, nq, cut[i]) for i in range(parts)]
+        jobs.append((n, nq, S.make_segments(rows), np.arange(nq, dtype=np.uint64) * n, S.DeviceBuffer(nq * n * 4)))
+    rt, stream = C.CDLL("libcudart.so.12"), C.c_void_p()
+    assert rt.cudaStreamCreateWithFlags(C.byref(stream), 1) == 0
+    S.set_stream(stream.value)
+    try:
+        for n, nq, seg, off, out in jobs:
+            S.score_segments(dt, seg, dq, ds, nq, out, off, n)
+        S.synchronize()
+    finally:
+        S.set_stream(None)
+        rt.cudaStreamDestroy(stream)
+    for n, nq, _, _, out in jobs:
+        got = out.download(F, nq * n).reshape(nq, n)
+        for j in range(nq):
+            want = ora.score_tiles(tiles[:n], qc[j], qs[j])
+            assert np.all(np.abs(got[j] - want) <= 1e-4 * (1 + np.abs(want)))
