@@ -298,6 +298,17 @@ __device__ __forceinline__ float4 load_q4(const float* p) {
     return *reinterpret_cast<const float4*>(p);
 }
 
+// A query row is multiplied by a power of two before it is split into fp16 hi + lo, and the finished sums by its inverse: with the
+// largest element in [2^target, 2^(target + 1)) the parts hold at least 22 bits of every element down to 2^-(target + 2) of the largest
+// (lo ends at 2^-24; unscaled, a row of elements around 1e-3 kept 15 bits and one of 1e-8 none).  `largest`: the bits
+// of the row's largest absolute value.  (up, its inverse)
+__device__ __forceinline__ float2 split_scale(uint32_t largest, int target) {
+    const int e = max(min(target + 127 - (int)(largest >> 23), 126), -126);  // (126: rows of denormals, exact all the same)
+    return make_float2(__uint_as_float((uint32_t)(127 + e) << 23), __uint_as_float((uint32_t)(127 - e) << 23));
+}
+constexpr uint32_t SPLIT_MOST = (127u + 96u) << 23;  // rows with an element of 2^96 or more, infinities and NaN go to the generic kernel
+__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+
 // ---- tcgen05 / mbarrier plumbing ------------------------------------------------------------------
 constexpr uint32_t TC_SPIN = 1u << 22;            // polls of one mbarrier wait before it gives up (~0.2 s)
 

@@ -3,7 +3,7 @@
 //
 // A thread reads its tile's 64 latent bytes from shared memory, turns them into exact fp16 products (level x scale byte) in
 // registers and writes them as its row of the A operand into TMEM; tcgen05.mma multiplies the 128 rows of a warpgroup with
-// the queries (fp16 hi + lo columns, about 22 bits) and the thread reads its finished coarse scores back.  Scale, lambda, flags
+// the queries (scaled to one size, fp16 hi + lo columns, 22 bits or more) and the thread reads its finished coarse scores back.  Scale, lambda, flags
 // and scale bytes are each read by one thread, where the fragments of warp-level MMAs need them in four lanes each.
 //
 // Bound: the chain of a block (decode, TMEM store, eight or nine MMAs, read-back, filter), about 5000 cycles with four warpgroups in
@@ -22,7 +22,7 @@ constexpr int ST_SLOT = ST_WT * ST_ROW;
 constexpr int ST_DEPTH = 2;                            // ring slots per warp
 constexpr uint32_t ST_CHUNK = 32;                      // slots a warp reserves at a time in a row's candidate buffer
 constexpr int ST_B_BYTES = 8192;                       // B operand: up to 3 slabs of 2 KB (64 K slots of 16 rows)
-constexpr int ST_TAIL_BYTES = 128 + 16 + 16 + 32 + 32 + 64;
+constexpr int ST_TAIL_BYTES = 128 + 16 + 16 + 32 + 32 + 64 + 32;
 // KIND 0: NF4 (and INT4) tiles, 1: mixed 8/4, 2: TQ3, 3: INT4 / MX-INT4, 4: MIX3
 constexpr int ST_WG = 4, ST_THREADS = 128 * ST_WG;     // warpgroups per CTA
 constexpr uint32_t ST_TMEM = 128;                      // TMEM columns of a warpgroup: A in the first 64 (72 for the 3-bit kinds), accumulators behind it
@@ -213,8 +213,8 @@ __device__ __forceinline__ void st_fold_row(uint32_t row, uint32_t ta, uint32_t 
     }
     if (Q1 == 4 && (KIND == 2 || KIND == 4)) {
         // level = (n - 8) / 2 + c / 4 with the nibble n (c = 1, or 2 without the correction plane): eight more K slots carry the
-        // scale bytes times c 2^-17, against the queries' sums over the groups (MIX3: the head's slot meets a zero)
-        const uint32_t f = nocorr ? 0x01000100u : 0x00800080u;
+        // scale bytes times c 2^-13, against a sixteenth of the queries' sums over the groups (MIX3: the head's slot meets a zero)
+        const uint32_t f = nocorr ? 0x0C000C00u : 0x08000800u;
         uint32_t o[8] = {scale_pair(gsl, magic, 0x7150u, f), scale_pair(gsl, magic, 0x7352u, f), scale_pair(gsh, magic, 0x7150u, f),
                          scale_pair(gsh, magic, 0x7352u, f), 0u, 0u, 0u, 0u};
         st_tmem_st8(ta + 64u, o);
@@ -280,7 +280,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
     // the thread that issues its warpgroup's MMAs; the four warpgroups' leaders sit on different schedulers
     const int uw = uniform_warp();
     const bool elected = elect_one(), leader = elected && (uw & 3) == (uw >> 2);
-    // shared layout (1024-byte aligned): B | [NF4 table] | ring | sign words | thresholds (keys, floats) | mappings | barriers, flags
+    // shared layout (1024-byte aligned): B | [NF4 table] | ring | sign words | thresholds (keys, floats) | mappings | barriers, flags | query scales
     const uint32_t base_s = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
     unsigned char* base = smem_raw + (base_s - (uint32_t)__cvta_generic_to_shared(smem_raw));
     constexpr uint32_t LUT_OFF = ST_B_BYTES, RING_OFF = LUT_OFF + (KIND == 0 ? NF4_LUT_BYTES : 0), TAIL_OFF = RING_OFF + NWARPS * ST_DEPTH * ST_SLOT;
@@ -295,6 +295,8 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
     const uint32_t bar_s = tail_s + 224u;
     uint32_t* tmem_slot = flagw + 8;
     uint32_t* bail = flagw + 9;
+    uint32_t* qmax = flagw + 16;                                 // [4] bits of the row's largest element
+    float* qinv = reinterpret_cast<float*>(qmax + 4);            // [4] inverse of the row's scale times the unit of A
 
     if (KIND == 0) {  // NF4 codebook pairs per byte, 16 bank-aligned replicas
         uint2* lut = reinterpret_cast<uint2*>(base + LUT_OFF);
@@ -336,6 +338,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
         // interleaved: this CTA is number il_c of the il_n CTAs that share the stream [tile_begin, + n_tiles); round r of
         // the stream's static deal belongs to CTA r mod il_n.  Otherwise the item is this CTA's own range.
         const uint32_t il_n = IL ? ((it.pad >> 8) & 0x7FFFFFu) : 1u, il_c = IL ? it.list_begin : 0u;
+        if (tid < 4) qmax[tid] = 0u;
         __syncthreads();  // previous item fully retired (and the table is visible)
         const uint8_t* sbase = a.state ? a.state + it.tile_begin : nullptr;
         const uint32_t n = it.n_tiles;
@@ -406,53 +409,63 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
             const int qi = lane >> 3;
             qs_w[lane] = qi < nq ? a.q_sign[(size_t)(it.query_begin + qi) * 8 + (lane & 7)] : 0u;
         }
-        // B: 16-byte chunks of eight k slots, K-major, 128-byte swizzle (chunk i of row r at chunk i ^ (r & 7) of its line).
-        bool big = false;
-        {
-            // row n = 2 q + part (hi / lo of query q), rows 8..15 zero; k slot 8 i + j holds dim 8 i + {0,4,1,5,2,6,3,7}[j] (see
-            // nib_word), NF4: dim 8 i + j
-            for (int u = tid; u < 16 * 18; u += blockDim.x) {
-                const int r = u / 18, i = u % 18, qi = r >> 1;
-                float v[8];
+        // B: 16-byte chunks of eight k slots, K-major, 128-byte swizzle (chunk i of row r at chunk i ^ (r & 7) of its line), one a thread.
+        // Row n = 2 q + part (hi / lo of query q), rows 8..15 zero; k slot 8 i + j holds dim 8 i + {0,4,1,5,2,6,3,7}[j] (see
+        // nib_word), NF4: dim 8 i + j.  A row's scale comes from the elements its chunks hold (the mixed layouts drop the last eight).
+        static_assert(ST_THREADS >= 16 * 18, "a thread per chunk");
+        const int br = tid / 18, bi = tid % 18, bq = br >> 1;
+        float v[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-                if (qi < nq) {
-                    const float* q = a.q_coarse + (size_t)(it.query_begin + qi) * D_C;
-                    constexpr bool HEAD = KIND == 1 || KIND == 4;
-                    if (HEAD && i < 2) {  // slots 0..3: the scale byte's high nibble's products of dims 4 i .., 4..7 the low nibble's
-                        const float4 x = load_q4(q + 4 * i);
-                        v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = x.x; v[5] = x.y; v[6] = x.z; v[7] = x.w;
-                    } else if (i < 16) {
-                        const int d0 = HEAD ? 8 * (i - 1) : 8 * i;
-                        const float4 x = load_q4(q + d0), y = load_q4(q + d0 + 4);
-                        if (KIND == 0) {
-                            v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-                        } else {
-                            v[0] = x.x; v[1] = y.x; v[2] = x.y; v[3] = y.y; v[4] = x.z; v[5] = y.z; v[6] = x.w; v[7] = y.w;
-                        }
-                    } else if (i == 16 && (KIND == 2 || KIND == 4)) {
-#pragma unroll
-                        for (int g = KIND == 4 ? 1 : 0; g < 8; ++g) {
-                            float s = 0.0f;
-                            const float* qg = q + (KIND == 4 ? 16 * g - 8 : 16 * g);
-                            for (int d = 0; d < 16; ++d) s += qg[d];
-                            v[g] = s;
-                        }
-                    }
+        for (int j = 0; j < 8; ++j) v[j] = 0.0f;
+        if (tid < 16 * 18 && bq < nq) {
+            const float* q = a.q_coarse + (size_t)(it.query_begin + bq) * D_C;
+            constexpr bool HEAD = KIND == 1 || KIND == 4;
+            if (HEAD && bi < 2) {  // slots 0..3: the scale byte's high nibble's products of dims 4 i .., 4..7 the low nibble's
+                const float4 x = load_q4(q + 4 * bi);
+                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = x.x; v[5] = x.y; v[6] = x.z; v[7] = x.w;
+            } else if (bi < 16) {
+                const int d0 = HEAD ? 8 * (bi - 1) : 8 * bi;
+                const float4 x = load_q4(q + d0), y = load_q4(q + d0 + 4);
+                if (KIND == 0) {
+                    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+                } else {
+                    v[0] = x.x; v[1] = y.x; v[2] = x.y; v[3] = y.y; v[4] = x.z; v[5] = y.z; v[6] = x.w; v[7] = y.w;
                 }
-                uint32_t w[4];
+            } else if (bi == 16 && (KIND == 2 || KIND == 4)) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float x0 = v[2 * j], x1 = v[2 * j + 1];
-                    big |= fabsf(x0) > 60000.0f || fabsf(x1) > 60000.0f;
-                    if (r & 1) { x0 = half_residual(x0); x1 = half_residual(x1); }
-                    w[j] = pack_half2(x0, x1);
+                for (int g = KIND == 4 ? 1 : 0; g < 8; ++g) {
+                    float s = 0.0f;
+                    const float* qg = q + (KIND == 4 ? 16 * g - 8 : 16 * g);
+                    for (int d = 0; d < 16; ++d) s += qg[d];
+                    v[g] = 0.0625f * s;
                 }
-                const uint32_t slab = (uint32_t)i >> 3, chunk = (uint32_t)i & 7u;
-                sts_v4(B_s + slab * 2048u + (uint32_t)r * 128u + ((chunk ^ ((uint32_t)r & 7u)) << 4), w[0], w[1], w[2], w[3]);
+            }
+            if (bi < 16 && !(br & 1)) {
+                uint32_t largest = 0u;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) largest = max(largest, abs_bits(v[j]));
+                atomicMax(&qmax[bq], largest);
             }
         }
-        if (big) *bail = 1u;  // a query too large for the fp16 split
+        __syncthreads();
+        if (tid < 16 * 18) {
+            const float up = split_scale(qmax[bq & 3], 14).x;  // (rows 8 .. 15 are zero)
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                float x0 = v[2 * j] * up, x1 = v[2 * j + 1] * up;
+                if (br & 1) { x0 = half_residual(x0); x1 = half_residual(x1); }
+                w[j] = pack_half2(x0, x1);
+            }
+            const uint32_t slab = (uint32_t)bi >> 3, chunk = (uint32_t)bi & 7u;
+            sts_v4(B_s + slab * 2048u + (uint32_t)br * 128u + ((chunk ^ ((uint32_t)br & 7u)) << 4), w[0], w[1], w[2], w[3]);
+        }
+        bool big = false;  // a query beyond the fp16 split
+        if (tid < 4) {
+            big = qmax[tid] >= SPLIT_MOST;
+            qinv[tid] = split_scale(qmax[tid], 14).y * (KIND == 0 ? 1.0f : (KIND == 2 || KIND == 4 ? 32768.0f : 65536.0f));
+        }
+        if (big) *bail = 1u;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // B was written with ordinary stores, the MMA reads it through the async proxy
         // The barrier after the first round (below) pays when the round can supply k candidates to a row -- 32 per warp
         // of every CTA that works on the row -- and the rows do not already have thresholds (a CTA that starts its
@@ -557,9 +570,12 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
             }
             if (skip) { wg_dead = true; continue; }
             {
-                const float su = __uint_as_float(meta.x) * ((KIND == 0 ? 1.0f : (KIND == 2 || KIND == 4 ? 32768.0f : 65536.0f)) / 255.0f);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) c[q] = (c[q] + low[q]) * su;
+                const float su = __uint_as_float(meta.x) * (1.0f / 255.0f);
+                const float4 inv = *reinterpret_cast<const float4*>(qinv);
+                c[0] = (c[0] + low[0]) * inv.x * su;
+                c[1] = (c[1] + low[1]) * inv.y * su;
+                c[2] = (c[2] + low[2]) * inv.z * su;
+                c[3] = (c[3] + low[3]) * inv.w * su;
             }
             if (dead) continue;
             const float lam = (flags & F_WARM) ? 0.0f : __uint_as_float(meta.y);
@@ -574,7 +590,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                 const float tq[4] = {th.x, th.y, th.z, th.w};
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (q < nq && live && !(fmaf(lam, 257.0f, fmaf(fabsf(c[q]), 1e-6f, c[q])) < tq[q])) m |= 1u << q;  // (a NaN goes on to the exact test)
+                    if (q < nq && live && !(fmaf(fabsf(lam), 257.0f, fmaf(fabsf(c[q]), 1e-6f, c[q])) < tq[q])) m |= 1u << q;  // (a NaN goes on to the exact test)
             }
             if (__any_sync(0xFFFFFFFFu, m != 0u)) {
                 const uint4 ra = lds_v4<64>(row), rb = lds_v4<80>(row);

@@ -2,8 +2,8 @@
 // score_tile.cuh, whose tile decode it shares.
 //
 // A CTA takes a block of 128 tiles through tcgen05.mma against up to 64 query rows.  Both terms of eq. 2.3 are contractions here:
-//   coarse  A (128 tiles x 128 dims, exact fp16 levels times scale bytes, + 16 K slots for the 3-bit kinds) x the queries as
-//           fp16 hi, then lo (q = hi + lo keeps ~22 bits), accumulated into the same 64 columns,
+//   coarse  A (128 tiles x 128 dims, exact fp16 levels times scale bytes, + 16 K slots for the 3-bit kinds) x the queries, scaled
+//           to one size, as fp16 hi, then lo (22 bits or more), accumulated into the same 64 columns,
 //   sign    A (128 tiles x 256 residual bits, a bit in place as an fp16 subnormal 2^-24 .. 2^-17) x the queries' signs as
 //           +-2^10 .. 2^3: exact integers times 2^-14, from which 256 - 2 hamming = U - 2^15 D, U the sum of the query's signs.
 // The 64 Hamming distances of a tile cost 8 XOR + 8 POPC each on the CUDA cores (POPC at a quarter of the issue rate), about 1100
@@ -34,7 +34,7 @@ constexpr int WIDE_S_BYTES = 4 * WIDE_SLAB;         // signs: K = 256
 constexpr int WIDE_RAW = 128 * ST_ROW;              // one staged block
 constexpr int WIDE_RING = 3;
 constexpr int WIDE_Q_BYTES = WIDE_NQ * D_C * 4;     // the item's queries in fp32 (item set-up only)
-constexpr int WIDE_TAIL = 2048 + 256 + 256 + 512 + 512 + 64 + 2048;  // sign words, threshold keys, sign sums, mappings (2), barrier + flags, minima and maxima / row offsets
+constexpr int WIDE_TAIL = 2048 + 256 + 512 + 512 + 512 + 64 + 2048;  // sign words, threshold keys, sign sums and scales, mappings (2), barrier + flags, minima and maxima / row offsets
 constexpr uint32_t WIDE_A_SIGN = 128, WIDE_D = 256;                   // TMEM columns: A latent 0..71, A signs 128..255, accumulators 256.. and 384..
 constexpr size_t wide_smem_bytes() { return 1024 + 2 * WIDE_B_BYTES + WIDE_S_BYTES + WIDE_Q_BYTES + WIDE_RING * WIDE_RAW + WIDE_TAIL; }
 
@@ -123,13 +123,13 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
     unsigned char* tail = base + TAIL_OFF;
     uint32_t* qs_w = reinterpret_cast<uint32_t*>(tail);            // [64][8]
     uint32_t* pvh = qs_w + 512;                                     // [64] score word of the row's threshold
-    float* usum = reinterpret_cast<float*>(pvh + 64);               // [64] sum of the row's signs
-    float2* rng = reinterpret_cast<float2*>(usum + 64);             // [64] (smin, inv)
+    float2* uq = reinterpret_cast<float2*>(pvh + 64);               // [64] (sum of the row's signs, inverse of the row's scale times the unit of A)
+    float2* rng = uq + 64;                                          // [64] (smin, inv)
     float2* rmap = rng + 64;                                        // [64] (-smin inv, inv)
     uint32_t* ctl = reinterpret_cast<uint32_t*>(rmap + 64);         // mbarrier (8 bytes), [4] TMEM base, [5] error flag, [6] bail
     float2* colmm = reinterpret_cast<float2*>(ctl + 16);            // [4][64] per tile quarter: (min, max) score of a column
     unsigned long long* roff = reinterpret_cast<unsigned long long*>(colmm);  // DENSE: [64] where the item's rows start in a.scores
-    const uint32_t bar_s = base_s + TAIL_OFF + 2048 + 256 + 256 + 512 + 512;
+    const uint32_t bar_s = base_s + TAIL_OFF + 2048 + 256 + 512 + 512 + 512;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, qt = warp & 3, ch = warp >> 2;
     const int uw = uniform_warp();
     const bool elected = elect_one(), leader = elected && uw == 0;  // the thread that issues the MMAs
@@ -175,9 +175,25 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         };
         const uint32_t all_blocks = (n + WIDE_M - 1) / WIDE_M;
         if (all_blocks) fetch(0);
-        for (int e = tid; e < WIDE_NQ * D_C / 4; e += WIDE_THREADS) {
-            const int qi = e >> 5;
-            reinterpret_cast<float4*>(qf)[e] = qi < nq ? load_q4(a.q_coarse + (size_t)(it.query_begin + qi) * D_C + 4 * (e & 31)) : make_float4(0, 0, 0, 0);
+        constexpr bool HEAD = KIND == 1 || KIND == 4, EXTRA = KIND == 2 || KIND == 4;
+        bool big = false;  // a query beyond the fp16 split
+        {   // four rows a warp, scaled on their way into shared memory (the mixed layouts have no levels behind dim 119)
+            constexpr int ROWS = WIDE_NQ / (WIDE_THREADS / 32);
+            float4 x[ROWS];
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const int r = ROWS * warp + i;
+                x[i] = r < nq && !(HEAD && lane >= 30) ? load_q4(a.q_coarse + (size_t)(it.query_begin + r) * D_C + 4 * lane) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int i = 0; i < ROWS; ++i) {
+                const int r = ROWS * warp + i;
+                const uint32_t largest = __reduce_max_sync(0xFFFFFFFFu, max(max(abs_bits(x[i].x), abs_bits(x[i].y)), max(abs_bits(x[i].z), abs_bits(x[i].w))));
+                big |= largest >= SPLIT_MOST;
+                const float2 f = split_scale(largest, 14);
+                reinterpret_cast<float4*>(qf)[32 * r + lane] = make_float4(x[i].x * f.x, x[i].y * f.x, x[i].z * f.x, x[i].w * f.x);
+                if (lane == 0) uq[r].y = f.y * (EXTRA ? 32768.0f : 65536.0f);
+            }
         }
         qs_w[tid] = (tid >> 3) < nq ? a.q_sign[(size_t)(it.query_begin + (tid >> 3)) * 8 + (tid & 7)] : 0u;
         if (DENSE && tid < WIDE_NQ) roff[tid] = tid < nq ? a.row_offset[it.query_begin + tid] : 0ull;
@@ -192,8 +208,6 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         __syncthreads();
         // B rows = queries, K-major, 128-byte swizzle (16-byte chunk i of row r at chunk i ^ (r & 7) of its line); the order of the
         // k slots is that of nib_word / head_word / scale_pair
-        bool big = false;
-        constexpr bool HEAD = KIND == 1 || KIND == 4, EXTRA = KIND == 2 || KIND == 4;
         for (int u = tid; u < WIDE_NQ * 18; u += WIDE_THREADS) {
             const int r = u / 18, i = u % 18;
             const float* q = qf + r * D_C;
@@ -216,14 +230,13 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
                             const float4 x = *reinterpret_cast<const float4*>(qg + d);
                             s = s + x.x + x.y + x.z + x.w;
                         }
-                        v[g] = s;
+                        v[g] = 0.0625f * s;
                     }
                 }
             }
             uint32_t hi[4], lo[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                big |= fabsf(v[2 * j]) > 60000.0f || fabsf(v[2 * j + 1]) > 60000.0f;
                 hi[j] = pack_half2(v[2 * j], v[2 * j + 1]);
                 lo[j] = pack_half2(half_residual(v[2 * j]), half_residual(v[2 * j + 1]));
             }
@@ -245,11 +258,11 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         if (tid < WIDE_NQ) {
             int c = 0;
             for (int w = 0; w < 8; ++w) c += __popc(qs_w[8 * tid + w]);
-            usum[tid] = (float)(256 - 2 * c);
+            uq[tid].x = (float)(256 - 2 * c);
         }
         if (big) ctl[6] = 1u;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // B was written with ordinary stores, the MMA reads it through the async proxy
-        const bool too_big = __syncthreads_or(big) != 0;  // a query too large for the fp16 split (from the vote: the flag word may already be raised for a tile)
+        const bool too_big = __syncthreads_or(big) != 0;  // (from the vote: the flag word may already be raised for a tile)
         const bool need_map = __syncthreads_or(!DENSE && tid < nq && rng[tid].y == 0.0f) != 0;  // a row of the item has no bucket mapping yet
         const uint32_t blocks = too_big ? 0u : all_blocks;
         WPROBE_LAP(0);  // item set-up
@@ -318,7 +331,7 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             const uint32_t flags = lds_u16<118>(row);
             const bool live = t0 < n;
             const float lam = (flags & F_WARM) ? 0.0f : __uint_as_float(meta.y);
-            const float su = __uint_as_float(meta.x) * ((EXTRA ? 32768.0f : 65536.0f) / 255.0f);
+            const float su = __uint_as_float(meta.x) * (1.0f / 255.0f);
             float sc[16];
             if (cols) {
                 uint32_t v[16], s[16];
@@ -326,8 +339,9 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
                 st_tmem_ld16x2(dt, dt + 64u, v, s);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const float h = fmaf(__uint_as_float(s[j]), -32768.0f, usum[16 * ch + j]);  // 256 - 2 hamming, exact
-                    sc[j] = fmaf(lam, h, __uint_as_float(v[j]) * su);
+                    const float2 u = uq[16 * ch + j];
+                    const float h = fmaf(__uint_as_float(s[j]), -32768.0f, u.x);  // 256 - 2 hamming, exact
+                    sc[j] = fmaf(lam, h, __uint_as_float(v[j]) * u.y * su);
                 }
             }
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");

@@ -130,3 +130,85 @@ def test_dense_calls_of_different_shapes_queued_behind_one_another():
         for j in range(nq):
             want = ora.score_tiles(tiles[:n], qc[j], qs[j])
             assert np.all(np.abs(got[j] - want) <= 1e-4 * (1 + np.abs(want)))
+
+
+SPREADS = [1e-30, 1e-6, 1e-4, 1e-3, 0.088, 1.0, 1e3, 1e5, 1e20]
+
+
+def _exact_terms(tiles, qc):
+    """float64 scores of tiles without a residual term, [query][tile], and the sums of their terms' sizes."""
+    lat = np.stack([ora.dequant(tiles[i:i + 1]) for i in range(len(tiles))]).astype(np.float64)
+    q = qc.astype(np.float64)
+    return q @ lat.T, np.abs(q) @ np.abs(lat).T
+
+
+def _spread_inputs(codec, nq, seed):
+    tiles = H.random_tiles(400, codec, seed=seed + codec, nocorr_every=5)
+    tiles["dynamic_lambda"] = 0
+    tiles["scale"][100:200] *= F(1e3)
+    tiles["scale"][200:300] *= F(1e6)
+    tiles["scale"][300:] *= F(1e-6)
+    qc, qs = H.random_queries(nq, seed + 1)
+    qc *= np.array([SPREADS[j % len(SPREADS)] for j in range(nq)], F)[:, None]
+    qc[-1, 5] *= F(300.0)  # (one element far above the others)
+    return tiles, qc, qs
+
+
+# Bound: a query is held to 2^-22 of every element that matters, the levels are exact, and at most 20 sums of float32 are each
+# off by 2^-23 of the terms so far (the reference's own latents by 3 x 2^-24): 2.7e-6 of the terms' sizes, whatever the query's size.
+SCORE_BOUND = 3e-6
+
+
+@pytest.mark.parametrize("codec", range(7))
+@pytest.mark.parametrize("nq", [9, 18, 64])
+def test_dense_scores_are_as_exact_for_small_and_large_queries(codec, nq):
+    tiles, qc, qs = _spread_inputs(codec, nq, 560)
+    n = len(tiles)
+    dt = S.to_device(tiles)
+    want, size = _exact_terms(tiles, qc)
+    got = [S.score_segments(dt, S.make_segments([(0, n, 0, nq, 0)]), qc, qs, nq, np.zeros((nq, n), F), np.arange(nq, dtype=np.uint64) * n, n)]
+    got += [np.concatenate([S.score_segments(dt, S.make_segments([(0, n, 0, 1, 0)]), qc[j:j + 1], qs[j:j + 1], 1, np.zeros((1, n), F), np.zeros(1, np.uint64), n)
+                            for j in range(9)])]
+    got += [S.score_tiles(S.to_device(np.tile(tiles, 82)), 82 * n, qc[:9], qs[:9], 9)[:, -n:]]
+    for g in got:
+        assert np.all(np.abs(g - want[:len(g)]) <= SCORE_BOUND * size[:len(g)] + 1e-44)
+
+
+@pytest.mark.parametrize("codec,nq", [(5, 1), (5, 4), (5, 6)] + [(c, nq) for c in (0, 1, 3, 4, 5, 6) for nq in (18, 64)])
+def test_top_k_scores_are_as_exact_for_small_and_large_queries(codec, nq):
+    # the tile kernel's codec and the 64-row kernel's
+    tiles, qc, qs = _spread_inputs(codec, 9 if nq < 9 else nq, 570)
+    n = k = 100 - codec  # (plans are kept by shape, each for one codec)
+    for part in range(4):  # (tiles of one scale at a time: the winners are all of them)
+        own = tiles[100 * part:100 * part + n]
+        dt = S.to_device(own)
+        want, size = _exact_terms(own, qc)
+        for q0 in range(0, len(qc), nq):
+            m = min(nq, len(qc) - q0)
+            idx, sc, cnt = S.score_topk(dt, S.make_segments([(0, n, 0, m, 0)]), qc[q0:q0 + m], qs[q0:q0 + m], m, k)
+            assert np.all(cnt == k) and S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
+            rows = np.arange(q0, q0 + m)[:, None]
+            assert np.all(np.sort(idx, 1) == np.arange(n))
+            assert np.all(np.abs(sc - want[rows, idx]) <= SCORE_BOUND * size[rows, idx] + 1e-44)
+
+
+@pytest.mark.parametrize("nq", [4, 17])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 1e30])
+def test_query_rows_beyond_the_split_take_the_generic_kernel(nq, value):
+    n, k = 700, 20
+    tiles = H.random_tiles(n, 5, seed=580)
+    qc, qs = H.random_queries(nq, 581)
+    qc[2, 77] = value
+    dt, seg = S.to_device(tiles), S.make_segments([(0, n, 0, nq, 0)])
+    idx, sc, _ = S.score_topk(dt, seg, qc, qs, nq, k)
+    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
+    out = S.score_segments(dt, seg, qc, qs, nq, np.zeros((nq, n), F), np.arange(nq, dtype=np.uint64) * n, n)
+    S.debug_force_generic_score(True)
+    try:
+        gi, gs, _ = S.score_topk(dt, seg, qc, qs, nq, k)
+        gout = S.score_segments(dt, seg, qc, qs, nq, np.zeros((nq, n), F), np.arange(nq, dtype=np.uint64) * n, n)
+    finally:
+        S.debug_force_generic_score(False)
+    assert np.array_equal(idx, gi) and np.array_equal(sc, gs, equal_nan=True)
+    assert np.array_equal(out[:4], gout[:4], equal_nan=True)  # (dense: the group of four rows that holds it)
+    assert np.all(np.abs(out[4:] - gout[4:]) <= 1e-4 * (1 + np.abs(gout[4:])))
