@@ -67,8 +67,8 @@ __device__ __forceinline__ void st_tmem_ld16x2(uint32_t t0, uint32_t t1, uint32_
                  : "r"(t0), "r"(t1)
                  : "memory");
 }
-// the first eight columns of three or four accumulators of sixteen
-__device__ __forceinline__ void st_ld_accs(uint32_t t, uint32_t (&v)[3][8]) {
+// eight columns of three or four accumulators, `step` columns apart
+__device__ __forceinline__ void st_ld_accs(uint32_t t, uint32_t (&v)[3][8], uint32_t step = 16u) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%24];\n"
                  "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%25];\n"
                  "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%26];\n"
@@ -76,10 +76,10 @@ __device__ __forceinline__ void st_ld_accs(uint32_t t, uint32_t (&v)[3][8]) {
                  : "=&r"(v[0][0]), "=&r"(v[0][1]), "=&r"(v[0][2]), "=&r"(v[0][3]), "=&r"(v[0][4]), "=&r"(v[0][5]), "=&r"(v[0][6]), "=&r"(v[0][7]),
                    "=&r"(v[1][0]), "=&r"(v[1][1]), "=&r"(v[1][2]), "=&r"(v[1][3]), "=&r"(v[1][4]), "=&r"(v[1][5]), "=&r"(v[1][6]), "=&r"(v[1][7]),
                    "=&r"(v[2][0]), "=&r"(v[2][1]), "=&r"(v[2][2]), "=&r"(v[2][3]), "=&r"(v[2][4]), "=&r"(v[2][5]), "=&r"(v[2][6]), "=&r"(v[2][7])
-                 : "r"(t), "r"(t + 16u), "r"(t + 32u)
+                 : "r"(t), "r"(t + step), "r"(t + 2u * step)
                  : "memory");
 }
-__device__ __forceinline__ void st_ld_accs(uint32_t t, uint32_t (&v)[4][8]) {
+__device__ __forceinline__ void st_ld_accs(uint32_t t, uint32_t (&v)[4][8], uint32_t step = 16u) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%32];\n"
                  "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8,%9,%10,%11,%12,%13,%14,%15}, [%33];\n"
                  "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16,%17,%18,%19,%20,%21,%22,%23}, [%34];\n"
@@ -89,7 +89,7 @@ __device__ __forceinline__ void st_ld_accs(uint32_t t, uint32_t (&v)[4][8]) {
                    "=&r"(v[1][0]), "=&r"(v[1][1]), "=&r"(v[1][2]), "=&r"(v[1][3]), "=&r"(v[1][4]), "=&r"(v[1][5]), "=&r"(v[1][6]), "=&r"(v[1][7]),
                    "=&r"(v[2][0]), "=&r"(v[2][1]), "=&r"(v[2][2]), "=&r"(v[2][3]), "=&r"(v[2][4]), "=&r"(v[2][5]), "=&r"(v[2][6]), "=&r"(v[2][7]),
                    "=&r"(v[3][0]), "=&r"(v[3][1]), "=&r"(v[3][2]), "=&r"(v[3][3]), "=&r"(v[3][4]), "=&r"(v[3][5]), "=&r"(v[3][6]), "=&r"(v[3][7])
-                 : "r"(t), "r"(t + 16u), "r"(t + 32u), "r"(t + 48u)
+                 : "r"(t), "r"(t + step), "r"(t + 2u * step), "r"(t + 3u * step)
                  : "memory");
 }
 
@@ -221,8 +221,8 @@ __device__ __forceinline__ void st_fold_row(uint32_t row, uint32_t ta, uint32_t 
     }
 }
 
-// NF4: half H of the latent (four scale groups) as the codebook entries' fp16 hi (columns 0..31) and lo (32..63) parts, from the
-// shared-memory table; the scale bytes are applied to the groups' sums instead, because a codebook value times a scale
+// NF4: half H of the latent (four scale groups) as fp16 hi (columns 0..31) and lo (32..63) parts of 1024 times the codebook entries
+// (unscaled, the lo parts of the small entries would be subnormal), from the shared-memory table; the scale bytes are applied to the groups' sums instead, because a codebook value times a scale
 // byte does not fit fp16.
 __device__ __forceinline__ void st_nf4_half(uint32_t row, int h, uint32_t ta, uint32_t flags, uint32_t lut_s, uint32_t lane8, uint32_t magic) {
 #pragma unroll
@@ -243,6 +243,7 @@ __device__ __forceinline__ void st_nf4_half(uint32_t row, int h, uint32_t ta, ui
             for (int e = 0; e < 16; ++e) {
                 const uint32_t b = (w[e >> 2] >> (8 * (e & 3))) & 0xFFu;
                 asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(hi[e]) : "r"(((b | (b << 12)) & 0x000F000Fu) | magic), "r"(0xE408E408u));
+                asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(hi[e]) : "r"(hi[e]), "r"(0x64006400u));
                 lo[e] = 0u;
             }
         }
@@ -302,7 +303,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
         uint2* lut = reinterpret_cast<uint2*>(base + LUT_OFF);
         for (int e = tid; e < 256 * 16; e += blockDim.x) {
             const int b = e >> 4;
-            const float c0 = c_nf4[b & 15], c1 = c_nf4[b >> 4];
+            const float c0 = 1024.0f * c_nf4[b & 15], c1 = 1024.0f * c_nf4[b >> 4];
             lut[e] = make_uint2(pack_half2(c0, c1), pack_half2(half_residual(c0), half_residual(c1)));
         }
     }
@@ -463,7 +464,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
         bool big = false;  // a query beyond the fp16 split
         if (tid < 4) {
             big = qmax[tid] >= SPLIT_MOST;
-            qinv[tid] = split_scale(qmax[tid], 14).y * (KIND == 0 ? 1.0f : (KIND == 2 || KIND == 4 ? 32768.0f : 65536.0f));
+            qinv[tid] = split_scale(qmax[tid], 14).y * (KIND == 0 ? 1.0f / 1024.0f : (KIND == 2 || KIND == 4 ? 32768.0f : 65536.0f));
         }
         if (big) *bail = 1u;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // B was written with ordinary stores, the MMA reads it through the async proxy

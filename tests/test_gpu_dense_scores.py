@@ -212,3 +212,32 @@ def test_query_rows_beyond_the_split_take_the_generic_kernel(nq, value):
     assert np.array_equal(idx, gi) and np.array_equal(sc, gs, equal_nan=True)
     assert np.array_equal(out[:4], gout[:4], equal_nan=True)  # (dense: the group of four rows that holds it)
     assert np.all(np.abs(out[4:] - gout[4:]) <= 1e-4 * (1 + np.abs(gout[4:])))
+
+
+@pytest.mark.parametrize("codec,nq", [(c, nq) for c in range(7) for nq in (1, 4)] + [(2, 20), (2, 64), (5, 20), (5, 64)])
+def test_scores_are_no_further_from_64_bits_than_the_generic_kernels(codec, nq):
+    # the calls that tensor-core kernels took over from it (float32 products in short chains): 2-norm of the error over six sets of
+    # tiles and queries, 5 % for chance (a single set's two errors differ by up to 12 % either way)
+    n = 1500 + codec
+    k = n // 3
+    seg, off = S.make_segments([(0, n, 0, nq, 0)]), np.arange(nq, dtype=np.uint64) * n
+    square = np.zeros((2, 2, 2))  # [dense, top-k][tensor cores, generic][error, size]
+    for seed in range(590, 650, 10):
+        tiles = H.random_tiles(n, codec, seed=seed + codec, nocorr_every=5)
+        tiles["dynamic_lambda"] = 0
+        qc, qs = H.random_queries(nq, seed + 1)
+        want = _exact_terms(tiles, qc)[0]
+        dt = S.to_device(tiles)
+        for generic in (0, 1):
+            S.debug_force_generic_score(bool(generic))
+            try:
+                out = S.score_segments(dt, seg, qc, qs, nq, np.zeros((nq, n), F), off, n)
+                idx, sc, _ = S.score_topk(dt, seg, qc, qs, nq, k)
+            finally:
+                S.debug_force_generic_score(False)
+            w = want[np.arange(nq)[:, None], idx]
+            square[0, generic] += ((out - want) ** 2).sum(), (want ** 2).sum()
+            square[1, generic] += ((sc - w) ** 2).sum(), (w ** 2).sum()
+    error = np.sqrt(square[:, :, 0] / square[:, :, 1])
+    assert error[0, 0] <= 1.05 * error[0, 1], error
+    assert codec != 5 or error[1, 0] <= 1.05 * error[1, 1], error  # (the other codecs' top-k always had kernels of their own)
