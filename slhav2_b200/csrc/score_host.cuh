@@ -48,7 +48,7 @@ Status launch_stream_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
 template <bool IL>
 Status launch_mix3(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_mix3_kernel<IL>, configured, a, grid, ST_THREADS, st_smem_bytes(4));
+    return launch_tc(c, score_mix3_kernel<IL>, configured, a, grid, ST_THREADS, st_smem_bytes(false));
 }
 template <bool IL>
 Status launch_stream(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
@@ -66,7 +66,7 @@ uint32_t stream_warps(int kind) { return (uint32_t)(kind == 4 ? ST_THREADS : STR
 static_assert(ST_CHUNK == ST_WT && MMA_CHUNK == MMA_SET_TILES, "a fresh chunk holds what a warp can append at once");
 Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_dense_kernel, configured, a, grid, 512, dense_smem_bytes());
+    return launch_tc(c, score_dense_kernel, configured, a, grid, ST_THREADS, st_smem_bytes(true));
 }
 template <int KIND>
 Status launch_wide_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {

@@ -31,8 +31,8 @@ constexpr uint32_t ST_TMEM = 128;                      // TMEM columns of a warp
 // one per scale group of a half.
 constexpr int st_accs(int kind) { return kind == 2 || kind == 4 ? 3 : 4; }
 constexpr uint32_t st_d_col(int kind) { return kind == 2 || kind == 4 ? 72u : 64u; }
-constexpr size_t st_smem_bytes(int kind) {
-    return 1024 + (kind == 0 ? NF4_LUT_BYTES : 0) + ST_B_BYTES + (size_t)(ST_THREADS / 32) * ST_DEPTH * ST_SLOT + ST_TAIL_BYTES;
+constexpr size_t st_smem_bytes(bool dense) {  // (only dense calls meet NF4 tiles here)
+    return 1024 + (dense ? NF4_LUT_BYTES : 0) + ST_B_BYTES + (size_t)(ST_THREADS / 32) * ST_DEPTH * ST_SLOT + ST_TAIL_BYTES;
 }
 
 // instruction descriptor: D fp32, A and B fp16, both K-major, N columns, M = 128
@@ -269,22 +269,81 @@ __device__ __forceinline__ bool st_alien(int kind, uint32_t flags) {
     return !(flags & F_MIX3) || (flags & (F_MIXED | F_TQ3 | F_NF4));
 }
 
+// What a thread keeps from one work item to the next.
+struct TileCta {
+    uint32_t base_s;   // shared memory, 1024-byte aligned: B | [NF4 table] | ring | sign words | thresholds (keys, floats) | mappings | barriers, flags | query scales
+    unsigned char* base;
+    uint32_t tmem;
+    int uw;            // warp index, known to be uniform
+    bool leader;       // the thread that issues its warpgroup's MMAs
+    bool table;        // the NF4 table is there
+    uint32_t phase;    // of the warpgroup's mbarrier
+    bool failed;       // a wait of this warp ran out
+};
+template <bool DENSE>
+struct TileLayout {
+    static constexpr uint32_t LUT = ST_B_BYTES, RING = LUT + (DENSE ? NF4_LUT_BYTES : 0), TAIL = RING + (ST_THREADS / 32) * ST_DEPTH * ST_SLOT;
+};
+template <bool DENSE>
+__device__ __forceinline__ TileCta tile_open(unsigned char* smem_raw) {
+    TileCta t;
+    t.uw = uniform_warp();
+    // (the four warpgroups' leaders sit on different schedulers)
+    const bool elected = elect_one();
+    t.leader = elected && (t.uw & 3) == (t.uw >> 2);
+    t.base_s = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
+    t.base = smem_raw + (t.base_s - (uint32_t)__cvta_generic_to_shared(smem_raw));
+    const uint32_t tail_s = t.base_s + TileLayout<DENSE>::TAIL;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t.base + TileLayout<DENSE>::TAIL + 256u);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < ST_WG; ++i) mbar_init(tail_s + 224u + 8 * i, 1);
+        tmem_slot[1] = 0u;  // bail
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    if (threadIdx.x < 32) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tail_s + 256u), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    t.tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+    t.table = false;
+    t.phase = 0u;
+    t.failed = false;
+    return t;
+}
+__device__ __forceinline__ void tile_close(const TileCta& t) {
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x < 32) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(t.tmem), "r"(512u) : "memory");
+}
+// The kind of a work item: what its first tile says.  nf4_too: plain nibble tiles count as NF4 (that kind decodes both).
+__device__ __forceinline__ int item_kind(uint32_t tile_flags, bool nf4_too) {
+    if (tile_flags & F_MIXED) return 1;
+    if (tile_flags & F_TQ3) return 2;
+    if (tile_flags & F_MIX3) return 4;
+    return (tile_flags & F_NF4) || nf4_too ? 0 : 3;
+}
+__device__ __forceinline__ uint32_t first_tile_flags(const ScoreArgs& a, const WorkItem& it) {
+    return *reinterpret_cast<const uint16_t*>(a.tiles + it.tile_begin * TILE_BYTES + 118);
+}
+
+// The work items from item_id on (KINDS: up to the first whose first tile is of another kind); the next item.
 // DENSE: every score is written to a.scores (row q at a.row_offset[q] or q * a.score_stride, tile i of the item at
 // index_base + i; -inf for COLD slots) and nothing is filtered or appended.  IL: the work items are interleaved shares of
-// whole streams (see the planner).  A tile of another codec than the launch's, or a query outside the fp16 split, hands the
+// whole streams (see the planner).  A tile of another codec than KIND's, or a query outside the fp16 split, hands the
 // item's query rows to the generic kernel.
-template <int KIND, bool IL, bool DENSE>
-__device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* smem_raw) {
+template <int KIND, bool IL, bool DENSE, bool KINDS>
+__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, bool nf4_too = false) {
     constexpr int NWG = ST_WG, NWARPS = 4 * NWG, NACC = st_accs(KIND);
     constexpr uint32_t STRIDE = ST_TMEM, DCOL = st_d_col(KIND);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wg = warp >> 2, wq = warp & 3;
-    // the thread that issues its warpgroup's MMAs; the four warpgroups' leaders sit on different schedulers
-    const int uw = uniform_warp();
-    const bool elected = elect_one(), leader = elected && (uw & 3) == (uw >> 2);
-    // shared layout (1024-byte aligned): B | [NF4 table] | ring | sign words | thresholds (keys, floats) | mappings | barriers, flags | query scales
-    const uint32_t base_s = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
-    unsigned char* base = smem_raw + (base_s - (uint32_t)__cvta_generic_to_shared(smem_raw));
-    constexpr uint32_t LUT_OFF = ST_B_BYTES, RING_OFF = LUT_OFF + (KIND == 0 ? NF4_LUT_BYTES : 0), TAIL_OFF = RING_OFF + NWARPS * ST_DEPTH * ST_SLOT;
+    const int uw = cta.uw;
+    const bool leader = cta.leader;
+    const uint32_t base_s = cta.base_s, tmem = cta.tmem;
+    unsigned char* base = cta.base;
+    constexpr uint32_t LUT_OFF = TileLayout<DENSE>::LUT, RING_OFF = TileLayout<DENSE>::RING, TAIL_OFF = TileLayout<DENSE>::TAIL;
     const uint32_t B_s = base_s, lut_s = base_s + LUT_OFF, ring_s = base_s + RING_OFF + (uint32_t)warp * (ST_DEPTH * ST_SLOT), tail_s = base_s + TAIL_OFF;
     unsigned char* tail = base + TAIL_OFF;
     uint32_t* qs_w = reinterpret_cast<uint32_t*>(tail);         // [4][8] sign words
@@ -294,12 +353,12 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
     float2* rmap = rng + 4;                                      // [4] (-smin inv, inv)
     uint32_t* flagw = reinterpret_cast<uint32_t*>(rmap + 4);     // mbarriers of the warpgroups (32 bytes), TMEM base, bail
     const uint32_t bar_s = tail_s + 224u;
-    uint32_t* tmem_slot = flagw + 8;
     uint32_t* bail = flagw + 9;
     uint32_t* qmax = flagw + 16;                                 // [4] bits of the row's largest element
     float* qinv = reinterpret_cast<float*>(qmax + 4);            // [4] inverse of the row's scale times the unit of A
 
-    if (KIND == 0) {  // NF4 codebook pairs per byte, 16 bank-aligned replicas
+    if (KIND == 0 && !cta.table) {  // NF4 codebook pairs per byte, 16 bank-aligned replicas (read by nobody yet)
+        cta.table = true;
         uint2* lut = reinterpret_cast<uint2*>(base + LUT_OFF);
         for (int e = tid; e < 256 * 16; e += blockDim.x) {
             const int b = e >> 4;
@@ -307,19 +366,6 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
             lut[e] = make_uint2(pack_half2(c0, c1), pack_half2(half_residual(c0), half_residual(c1)));
         }
     }
-    if (tid == 0) {
-        for (int i = 0; i < NWG; ++i) mbar_init(bar_s + 8 * i, 1);
-        *bail = 0u;
-        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
-    }
-    if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(tail_s + 256u), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
     const uint32_t ta = tmem + (uint32_t)wg * STRIDE + ((uint32_t)(32 * wq) << 16);  // this warp's lanes of its warpgroup's columns
     uint32_t magic;  // 1024.0h twice, opaque so that it stays in one register
     asm volatile("mov.u32 %0, 0x64006400;\n" : "=r"(magic));
@@ -328,13 +374,13 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
     const uint32_t lt_mask = (1u << lane) - 1u;
     uint64_t stream_policy;
     asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;\n" : "=l"(stream_policy));
-    uint32_t phase = 0;      // of the warpgroup's mbarrier
-    bool wg_dead = false;    // a wait ran out (the same in the whole warpgroup)
-    bool failed = false;
+    uint32_t phase = cta.phase;
+    bool failed = cta.failed;
 
-    const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
-    for (uint32_t item_id = a.cta_begin[blockIdx.x]; item_id < item_end; ++item_id) {
+    for (; item_id < item_end; ++item_id) {
         const WorkItem it = a.stream_items[item_id];
+        if (KINDS && item_kind(first_tile_flags(a, it), nf4_too) != KIND) break;  // (the same in the whole CTA)
+        bool gave_up = false;  // this warpgroup met a tile it cannot decode, or a wait of it ran out (the same in the whole warpgroup)
         const int nq = (int)it.n_queries;
         // interleaved: this CTA is number il_c of the il_n CTAs that share the stream [tile_begin, + n_tiles); round r of
         // the stream's static deal belongs to CTA r mod il_n.  Otherwise the item is this CTA's own range.
@@ -479,7 +525,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
 
         uint32_t slot = 0, polls = 0;
         uint32_t cur[4] = {0, 0, 0, 0}, end[4] = {0, 0, 0, 0};  // this warp's chunk of every row's buffer
-        bool dead = false;                                      // this warp met a tile it cannot decode
+        bool dead = false;                                      // this warp met a tile it cannot decode, or a wait of it ran out
         for (uint32_t round = 0; round < rounds; ++round) {
             if (round == 1 && first_round_barrier) {
                 // Every warp of the CTA (and, started together, of the grid) has appended its first tiles
@@ -493,6 +539,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                 }
                 __syncthreads();
             }
+            if (gave_up) continue;
             const uint32_t b = block_of(round);
             // (the ring advances in every iteration, also when this warpgroup has no block in this round -- the short last round
             // of the stream can come anywhere in a rotated walk -- so that fetches and reads stay in step)
@@ -504,7 +551,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
             __syncwarp();
             const uint32_t row = row_lane + slot;
             slot = slot == (ST_DEPTH - 1) * ST_SLOT ? 0u : slot + ST_SLOT;
-            if (b >= n_blocks || wg_dead) continue;  // (the same in the whole warpgroup)
+            if (b >= n_blocks) continue;  // (the same in the whole warpgroup)
             const uint32_t t0 = b * ST_M + (uint32_t)(wq * ST_WT + lane);
             bool live = t0 < n;
             if (sbase && live) live = sbase[t0] != ST_COLD;
@@ -524,7 +571,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                 else st_fold_row<KIND, 0, 4>(row, ta, flags, x.z, x.w, magic);
                 asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-                if (role_any(1 + wg, 128, failed)) { skip = true; break; }
+                if (role_any(1 + wg, 128, failed || dead)) { skip = true; break; }
                 if (leader) {
                         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                         const uint32_t at = tmem + (uint32_t)(uw >> 2) * STRIDE, dt = at + DCOL;
@@ -545,7 +592,7 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                 failed = !mbar_wait(bar_s + 8 * wg, phase);
                 phase ^= 1u;
                 if (__any_sync(0xFFFFFFFFu, failed)) {
-                    // the wait ran out: this warp's rows go to the generic kernel; the warpgroup stops together at its next barrier
+                    // the wait ran out: the warpgroup stops together at its next barrier, in this item and in all that follow
                     failed = true;
                     if (lane == 0) *bail = 1u;
                     dead = true;
@@ -569,7 +616,11 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
                     }
                 }
             }
-            if (skip) { wg_dead = true; continue; }
+            if (skip) {  // the item's rows go to the generic kernel: this warpgroup has no more to do for it
+                if (lane == 0) *bail = 1u;
+                gave_up = true;
+                continue;
+            }
             {
                 const float su = __uint_as_float(meta.x) * (1.0f / 255.0f);
                 const float4 inv = *reinterpret_cast<const float4*>(qinv);
@@ -718,35 +769,40 @@ __device__ __forceinline__ void tile_body(const ScoreArgs& a, unsigned char* sme
         if (*reinterpret_cast<volatile uint32_t*>(bail) && tid < nq) a.gflag[it.query_begin + tid] = 1u;
         __syncthreads();
         if (tid == 0) *bail = 0u;  // (ordered before the next item's writers by the barrier at its start)
-        if (wg_dead || failed) {   // (a warpgroup that stopped cannot score the items that follow either)
-            for (uint32_t later = item_id + 1; later < item_end; ++later) {
-                const WorkItem li = a.stream_items[later];
-                if ((uint32_t)(tid & 127) < li.n_queries) a.gflag[li.query_begin + (tid & 127)] = 1u;
-            }
-        }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-    __syncthreads();
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(512u) : "memory");
+    cta.phase = phase;
+    cta.failed = failed;
+    return item_id;
 }
 
 template <bool IL>
 __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    tile_body<4, IL, false>(a, smem_raw);
+    TileCta cta = tile_open<false>(smem_raw);
+    tile_run<4, IL, false, false>(a, cta, a.cta_begin[blockIdx.x], a.cta_begin[blockIdx.x + 1]);
+    tile_close(cta);
 }
 
-// Dense scores.  The kind of every CTA's launch is what its first tile says (read here: a host that looked would wait for
-// the stream); tiles of another kind hand their rows over as everywhere.
-constexpr size_t dense_smem_bytes() { return st_smem_bytes(3) > st_smem_bytes(0) ? st_smem_bytes(3) : st_smem_bytes(0); }
-__global__ void __launch_bounds__(512, 1) score_dense_kernel(ScoreArgs a) {
+// Dense scores.  Every work item is decoded as what its first tile says (read here: a host that looked would wait for the
+// stream); a tile of another kind inside the item hands its rows over as everywhere.
+__global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    const uint32_t flags = *reinterpret_cast<const uint16_t*>(a.tiles + a.stream_items[a.cta_begin[blockIdx.x]].tile_begin * TILE_BYTES + 118);
-    if (flags & F_MIXED) tile_body<1, false, true>(a, smem_raw);
-    else if (flags & F_TQ3) tile_body<2, false, true>(a, smem_raw);
-    else if (flags & F_MIX3) tile_body<4, false, true>(a, smem_raw);
-    else if (flags & F_NF4) tile_body<0, false, true>(a, smem_raw);
-    else tile_body<3, false, true>(a, smem_raw);
+    uint32_t i = a.cta_begin[blockIdx.x];
+    const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
+    uint32_t flags = first_tile_flags(a, a.stream_items[i]);  // (on its way while the CTA is set up)
+    TileCta cta = tile_open<true>(smem_raw);
+    for (;;) {
+        switch (item_kind(flags, false)) {
+            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end); break;
+            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end); break;
+            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end); break;
+            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end); break;
+            default: i = tile_run<4, false, true, true>(a, cta, i, item_end); break;
+        }
+        if (i >= item_end) break;
+        flags = first_tile_flags(a, a.stream_items[i]);
+    }
+    tile_close(cta);
 }
 
 }  // namespace

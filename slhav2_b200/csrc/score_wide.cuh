@@ -116,8 +116,9 @@ __device__ __forceinline__ void wide_sign_words(const uint4& x, uint32_t ta) {
 // KIND as in score_stream_kernel (1 mixed 8/4, 2 TQ3, 3 INT4 / MX-INT4, 4 MIX3).  DENSE: every score is written to its row of
 // a.scores (row q starts at a.row_offset[q]) instead of going through the top-k filter: the dense scores of a layer for
 // callers that replace attention logits (the llama.cpp shim).
+// The CTA's work items from first_item on.
 template <int KIND, bool DENSE>
-__device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* smem_raw) {
+__device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* smem_raw, uint32_t first_item) {
     constexpr int ACCS = KIND == 4 ? 3 : 1;                            // coarse accumulators
     constexpr uint32_t SIGN_AT = 64u * ACCS, FLIP = ACCS == 1 ? 128u : 0u;  // the signs' columns behind them; the second set of both
     // shared layout (1024-byte aligned base): B hi | B lo | signs | raw ring | queries | tail
@@ -163,7 +164,7 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
     bool stop = false;
 
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
-    for (uint32_t item_id = a.cta_begin[blockIdx.x]; item_id < item_end && !stop; ++item_id) {
+    for (uint32_t item_id = first_item; item_id < item_end && !stop; ++item_id) {
         const WorkItem it = a.items[item_id];
         const int nq = (int)it.n_queries;
         const uint32_t n = it.n_tiles, idesc = tc_idesc(((uint32_t)nq + 15u) & ~15u);
@@ -517,21 +518,25 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
 template <int KIND>
 __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    wide_body<KIND, false>(a, smem_raw);
+    wide_body<KIND, false>(a, smem_raw, a.cta_begin[blockIdx.x]);
 }
 
-// Dense scores; every CTA decodes the kind of its first tile.  NF4 tiles, whose scale bytes cannot be folded into A, go to
-// score_dense_kernel's pass over the flagged rows.
+// Dense scores; a CTA decodes the kind of its first item that is not NF4.  Items of other kinds, and NF4 tiles, whose scale bytes cannot
+// be folded into A, go to score_dense_kernel's pass over the flagged rows.
 __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_dense_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    const uint32_t flags = *reinterpret_cast<const uint16_t*>(a.tiles + a.items[a.cta_begin[blockIdx.x]].tile_begin * TILE_BYTES + 118);
-    if (flags & F_MIXED) wide_body<1, true>(a, smem_raw);
-    else if (flags & F_TQ3) wide_body<2, true>(a, smem_raw);
-    else if (flags & F_MIX3) wide_body<4, true>(a, smem_raw);
-    else if (flags & F_NF4) {
-        for (uint32_t i = a.cta_begin[blockIdx.x]; i < a.cta_begin[blockIdx.x + 1]; ++i)
-            if (threadIdx.x < a.items[i].n_queries) a.gflag[a.items[i].query_begin + threadIdx.x] = 1u;
-    } else wide_body<3, true>(a, smem_raw);
+    uint32_t i = a.cta_begin[blockIdx.x];
+    const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
+    int kind = item_kind(first_tile_flags(a, a.items[i]), false);
+    while (kind == 0) {
+        if (threadIdx.x < a.items[i].n_queries) a.gflag[a.items[i].query_begin + threadIdx.x] = 1u;
+        if (++i == item_end) return;
+        kind = item_kind(first_tile_flags(a, a.items[i]), false);
+    }
+    if (kind == 1) wide_body<1, true>(a, smem_raw, i);
+    else if (kind == 2) wide_body<2, true>(a, smem_raw, i);
+    else if (kind == 4) wide_body<4, true>(a, smem_raw, i);
+    else wide_body<3, true>(a, smem_raw, i);
 }
 
 }  // namespace

@@ -241,3 +241,60 @@ def test_scores_are_no_further_from_64_bits_than_the_generic_kernels(codec, nq):
     error = np.sqrt(square[:, :, 0] / square[:, :, 1])
     assert error[0, 0] <= 1.05 * error[0, 1], error
     assert codec != 5 or error[1, 0] <= 1.05 * error[1, 1], error  # (the other codecs' top-k always had kernels of their own)
+
+
+def _generic(call):
+    S.debug_force_generic_score(True)
+    try:
+        return call()
+    finally:
+        S.debug_force_generic_score(False)
+
+
+@pytest.mark.parametrize("nq", [2, 16])
+def test_segments_of_different_codecs_in_one_cta_are_decoded_each_as_its_own(nq):
+    # 148 CTAs share about two thousand short segments of six codecs in turn: no row takes the generic kernel, whose sums differ in
+    # their last bits.  (NF4 with 16 rows or more passes through the four-row kernel.)
+    n_seg, lens = 1998, [17, 40, 129, 64, 5, 200]
+    parts = [H.random_tiles(200, c, seed=600 + c, warm_every=5, nocorr_every=3) for c in (1, 3, 4, 5, 2, 6)]
+    rows, chunks, tb = [], [], 0
+    for i in range(n_seg):
+        m = lens[(i // 6) % 6]
+        chunks.append(parts[i % 6][:m])
+        rows.append((tb, m, i * nq, nq, 0))
+        tb += m
+    tiles = np.concatenate(chunks)
+    row_len = 200
+    qc, qs = H.random_queries(n_seg * nq, 601)
+    dt, seg, off = S.to_device(tiles), S.make_segments(rows), np.arange(n_seg * nq, dtype=np.uint64) * row_len
+    call = lambda: S.score_segments(dt, seg, qc, qs, n_seg * nq, np.zeros((n_seg * nq, row_len), F), off, row_len)  # noqa: E731
+    got, gen = call(), _generic(call)
+    handed = 0
+    for i, (t, m, q0, _, _) in enumerate(rows):
+        a, b = got[q0:q0 + nq, :m], gen[q0:q0 + nq, :m]
+        assert np.all(np.abs(a - b) <= 1e-4 * (1 + np.abs(b)))
+        handed += m >= 40 and np.array_equal(a, b)
+        assert np.all(got[q0:q0 + nq, m:] == 0)
+        if i % 97 == 0:
+            want = ora.score_tiles(tiles[t:t + m], qc[q0], qs[q0])
+            assert np.all(np.abs(a[0] - want) <= 1e-4 * (1 + np.abs(want)))
+    assert handed == 0
+
+
+@pytest.mark.parametrize("codecs", [(1, 3), (5, 4), (2, 5), (0, 5)])
+@pytest.mark.parametrize("nq", [3, 18])
+def test_arenas_whose_tiles_change_codec_all_the_time(codecs, nq):
+    # every block holds tiles of two codecs: the tensor-core kernels give such items up, the generic kernel scores them
+    n = 33000
+    a, b = (np.tile(H.random_tiles(500, c, seed=610 + c, warm_every=4), 66) for c in codecs)
+    tiles = np.where((np.arange(n) % 3 == 1), b, a)
+    qc, qs = H.random_queries(nq, 611)
+    dt = S.to_device(tiles)
+    idx, sc, _ = S.score_topk(dt, S.make_segments([(0, n, 0, nq, 0)]), qc, qs, nq, 50)
+    out = S.score_segments(dt, S.make_segments([(0, n, 0, nq, 0)]), qc, qs, nq, np.zeros((nq, n), F), np.arange(nq, dtype=np.uint64) * n, n)
+    full = S.score_tiles(dt, n, qc, qs, nq)
+    for j in range(nq):
+        want = ora.score_tiles(tiles, qc[j], qs[j])
+        for o in (out[j], full[j]):
+            assert np.all(np.abs(o - want) <= 1e-4 * (1 + np.abs(want)))
+        assert np.all(np.abs(sc[j] - np.sort(want)[::-1][:50]) <= 1e-3) and np.all(np.abs(sc[j] - want[idx[j]]) <= 1e-3)
