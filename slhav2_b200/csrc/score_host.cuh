@@ -652,7 +652,8 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     if (n == 0 || nq == 0) return Status();
     // Long arenas: the streaming tensor-core kernel in its dense mode (all query groups of four in one launch, every CTA an
     // equal share of the tiles), then the generic kernel for the rows of work items it handed back (a codec it does not
-    // decode, a query outside the fp16 split).  codec_hint -2: codecs the tensor-core kernel does not decode together.
+    // decode, a query outside the fp16 split).  codec_hint -2: codecs the tensor-core kernel does not decode together;
+    // bit 0: NF4 tiles beside INT4 ones; -1: not known.
     if (n >= 32768 && n < 0xFFFFFFFFull && codec_hint != -2 && !g_force_generic) {
         int sms = 148;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
@@ -673,6 +674,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.q_sign = reinterpret_cast<const uint32_t*>(q_sign);
         a.scores = scores;
         a.score_stride = n;
+        a.nf4_table = codec_hint < 0 ? 2u : (uint32_t)(codec_hint & 1);
         a.gflag = reinterpret_cast<uint32_t*>(dev + o_flag);
         SLHA_TRY(launch_dense(c, a, (uint32_t)cuts.cta.size() - 1));
         // the generic kernel over the same work items, only those whose rows were handed back

@@ -784,20 +784,22 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) 
 }
 
 // Dense scores.  Every work item is decoded as what its first tile says (read here: a host that looked would wait for the
-// stream); a tile of another kind inside the item hands its rows over as everywhere.
+// stream); a tile of another kind inside the item hands its rows over as everywhere.  An arena known to hold NF4 beside INT4
+// tiles is decoded as NF4 throughout.
 __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     uint32_t flags = first_tile_flags(a, a.stream_items[i]);  // (on its way while the CTA is set up)
+    const bool nf4_too = a.nf4_table == 1u || (a.nf4_table == 2u && (first_tile_flags(a, a.stream_items[0]) & F_NF4));
     TileCta cta = tile_open<true>(smem_raw);
     for (;;) {
-        switch (item_kind(flags, false)) {
-            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end); break;
-            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end); break;
-            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end); break;
-            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end); break;
-            default: i = tile_run<4, false, true, true>(a, cta, i, item_end); break;
+        switch (item_kind(flags, nf4_too)) {
+            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, nf4_too); break;
+            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, nf4_too); break;
+            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, nf4_too); break;
+            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, nf4_too); break;
+            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, nf4_too); break;
         }
         if (i >= item_end) break;
         flags = first_tile_flags(a, a.stream_items[i]);

@@ -298,3 +298,31 @@ def test_arenas_whose_tiles_change_codec_all_the_time(codecs, nq):
         for o in (out[j], full[j]):
             assert np.all(np.abs(o - want) <= 1e-4 * (1 + np.abs(want)))
         assert np.all(np.abs(sc[j] - np.sort(want)[::-1][:50]) <= 1e-3) and np.all(np.abs(sc[j] - want[idx[j]]) <= 1e-3)
+
+
+def test_a_pool_of_nf4_and_int4_tiles_is_scored_in_one_pass():
+    # tiles of both in every CTA's share: the kind that decodes both takes all of them (the generic kernel's sums differ in their last bits)
+    n = 36000
+    model = S.Model.from_projection(H.make_model_pair(128)[1], 128, 7)
+    keys = H.gaussian_keys(620, 1500, 128, outlier_channels=(7, 93))
+    qc, qs = H.random_queries(1, 621)
+    for first, second in ((S.CODEC_INT4_GROUPED, S.CODEC_NF4), (S.CODEC_NF4, S.CODEC_INT4_SINGLE)):
+        pool = S.TilePool(n, 2**40)
+        for i in range(n // 1500):
+            pool.append_keys(model, keys, (first, second)[i % 2], want_slots=False)
+        slots, got = pool.score_all(qc[0], qs[0])
+        gen = _generic(lambda: pool.score_all(qc[0], qs[0]))[1]
+        tiles = pool.read()[0]
+        want = ora.score_tiles(tiles, qc[0], qs[0])
+        assert np.array_equal(slots, np.arange(n)) and np.all(np.abs(got - want) <= 1e-4 * (1 + np.abs(want)))
+        nf4 = (tiles["flags"] & S.FLAG_NF4) != 0
+        assert nf4.mean() == 0.5
+        for part in (nf4, ~nf4):
+            for b in range(0, n, 3000):
+                own = part[b:b + 3000]
+                assert not np.array_equal(got[b:b + 3000][own], gen[b:b + 3000][own])
+        # the same tiles in an arena of the caller's whose first tile is an NF4 tile
+        arena = tiles[np.argsort(~nf4[:1500 * 2], kind="stable")]
+        arena = np.tile(arena, 12)
+        call = lambda: S.score_tiles(S.to_device(arena), len(arena), qc, qs, 1)  # noqa: E731
+        assert not np.array_equal(call()[0][-3000:], _generic(call)[0][-3000:])
