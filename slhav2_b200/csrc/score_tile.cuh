@@ -775,11 +775,17 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
     return item_id;
 }
 
+// Top-k of plans made for MIX3 tiles.  Plans are kept by shape: where a later call of that shape brings INT4 / MX-INT4 tiles, they
+// are decoded as those (as the plans of MIX3 tiles did when the generic kernel scored MIX3).
 template <bool IL>
 __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
+    uint32_t i = a.cta_begin[blockIdx.x];
+    const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
+    const bool int4 = item_kind(first_tile_flags(a, a.stream_items[i]), false) == 3;
     TileCta cta = tile_open<false>(smem_raw);
-    tile_run<4, IL, false, false>(a, cta, a.cta_begin[blockIdx.x], a.cta_begin[blockIdx.x + 1]);
+    if (int4) i = tile_run<3, IL, false, true>(a, cta, i, item_end);
+    tile_run<4, IL, false, false>(a, cta, i, item_end);
     tile_close(cta);
 }
 

@@ -518,7 +518,10 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
 template <int KIND>
 __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    wide_body<KIND, false>(a, smem_raw, a.cta_begin[blockIdx.x]);
+    const uint32_t first = a.cta_begin[blockIdx.x];
+    // (a plan made for MIX3 tiles also takes INT4 / MX-INT4 tiles of its shape, see score_mix3_kernel)
+    if (KIND == 4 && item_kind(first_tile_flags(a, a.items[first]), false) == 3) wide_body<3, false>(a, smem_raw, first);
+    else wide_body<KIND, false>(a, smem_raw, first);
 }
 
 // Dense scores; a CTA decodes the kind of its first item that is not NF4.  Items of other kinds, and NF4 tiles, whose scale bytes cannot

@@ -326,3 +326,18 @@ def test_a_pool_of_nf4_and_int4_tiles_is_scored_in_one_pass():
         arena = np.tile(arena, 12)
         call = lambda: S.score_tiles(S.to_device(arena), len(arena), qc, qs, 1)  # noqa: E731
         assert not np.array_equal(call()[0][-3000:], _generic(call)[0][-3000:])
+
+
+@pytest.mark.parametrize("nq,n", [(1, 5000), (4, 9000), (20, 3000)])
+def test_int4_tiles_of_the_shape_of_an_earlier_mix3_call_stay_on_the_tensor_cores(nq, n):
+    # plans are kept by shape: the one made for MIX3 tiles decodes INT4 / MX-INT4 tiles too, and MIX3 again after them
+    k = 33
+    qc, qs = H.random_queries(nq, 630)
+    seg = S.make_segments([(0, n, 0, nq, 0)])
+    for codec in (5, 1, 6, 0, 5):
+        tiles = np.tile(H.random_tiles(1000, codec, seed=631 + codec, warm_every=6), n // 1000)
+        idx, sc, cnt = S.score_topk(S.to_device(tiles), seg, qc, qs, nq, k)
+        assert S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
+        for j in range(nq):
+            want = ora.score_tiles(tiles, qc[j], qs[j])
+            assert cnt[j] == k and np.all(np.abs(sc[j] - np.sort(want)[::-1][:k]) <= 1e-3) and np.all(np.abs(sc[j] - want[idx[j]]) <= 1e-3)
