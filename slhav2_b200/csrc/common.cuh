@@ -53,6 +53,8 @@ Status ctx_device_scratch(Ctx* c, size_t bytes, void** out);
 Status ctx_host_scratch(Ctx* c, size_t bytes, void** out);
 // A small host table into device scratch, on the call's stream: `src` may go away when this returns.  Fails on a stream that is being captured.
 Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
+// The call under way leaves work in a plan's buffers (kept per thread, like the scratch arena): see CallScope.
+void ctx_mark_queued(Ctx* c);
 void count_launch(int n = 1);
 uint64_t launch_count();
 void tls_set_device(int dev);

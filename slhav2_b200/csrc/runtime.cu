@@ -36,7 +36,7 @@ constexpr size_t UPLOAD_MOST = (size_t)1 << 20;    // larger tables are copied f
 struct UploadSlot {
     void* p = nullptr;
     size_t cap = 0;
-    cudaEvent_t done = nullptr;
+    cudaEvent_t done = nullptr;  // recorded where the call that used the slot ends
     bool pending = false;
     ~UploadSlot() {
         if (pending) cudaEventSynchronize(done);
@@ -55,12 +55,14 @@ struct ThreadState {
     std::vector<std::pair<void*, size_t>> hblocks[16];
     UploadSlot upload[16][UPLOAD_SLOTS];
     uint32_t upload_next[16] = {0};
-    // Arena reuse across streams: a call on a caller-supplied stream may return while its
-    // kernels still read the arena; the event marks the end of that work, and a later call on
-    // ANOTHER stream waits for it before it reuses the arena (same stream: stream order suffices).
-    cudaEvent_t arena_done[16] = {nullptr};
-    cudaStream_t arena_stream[16] = {nullptr};
-    bool arena_pending[16] = {false};
+    UploadSlot* upload_used[16] = {nullptr};  // by the call under way
+    // Working memory (the arena, the plans' buffers) across streams: a call on a caller-supplied stream may return while its
+    // kernels still use it; the event marks the end of that work, and every later call on ANOTHER stream (by its id: the
+    // handle of a destroyed stream may come again) waits for it first.  On the same stream, stream order suffices.
+    cudaEvent_t own_event[16] = {nullptr};
+    cudaEvent_t work_done[16] = {nullptr};   // own_event or an upload slot's, whichever the latest call recorded
+    unsigned long long work_stream[16] = {0};
+    bool work_queued[16] = {false};          // the call under way uses a plan
 };
 thread_local ThreadState tls;
 }  // namespace
@@ -123,10 +125,23 @@ Status ctx_host_scratch(Ctx* c, size_t bytes, void** out) {
     return Status();
 }
 
-Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
+namespace {
+// (an error means that another stream's capture forbids to ask)
+bool capturing(cudaStream_t s) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    SLHA_CUDA(cudaStreamIsCapturing(c->stream, &cap));
-    if (cap != cudaStreamCaptureStatusNone) {
+    if (cudaStreamIsCapturing(s, &cap) == cudaSuccess) return cap != cudaStreamCaptureStatusNone;
+    cudaGetLastError();
+    return true;
+}
+unsigned long long stream_id(cudaStream_t s) {
+    unsigned long long id = 0;
+    if (cudaStreamGetId(s, &id) != cudaSuccess) cudaGetLastError();
+    return id;
+}
+}  // namespace
+
+Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
+    if (capturing(c->stream)) {
         // a graph would keep the address of host memory that this call's successors write again: refused, and the capture ends
         // as invalid, like everywhere the library has to wait for a stream
         SLHA_CUDA(cudaStreamSynchronize(c->stream));
@@ -137,6 +152,10 @@ Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
         SLHA_CUDA(cudaMemcpyAsync(*dev, src, bytes, cudaMemcpyHostToDevice, c->stream));
         SLHA_CUDA(cudaStreamSynchronize(c->stream));
         return Status();
+    }
+    if (UploadSlot* before = tls.upload_used[c->device]) {  // a second table of the same call
+        SLHA_CUDA(cudaEventRecord(before->done, c->stream));
+        before->pending = true;
     }
     UploadSlot& s = tls.upload[c->device][tls.upload_next[c->device]++ % UPLOAD_SLOTS];
     if (s.pending) {
@@ -155,23 +174,20 @@ Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
     if (!s.done) SLHA_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
     std::memcpy(s.p, src, bytes);
     SLHA_CUDA(cudaMemcpyAsync(*dev, s.p, bytes, cudaMemcpyHostToDevice, c->stream));
-    const cudaError_t e = cudaEventRecord(s.done, c->stream);
-    if (e != cudaSuccess) {
-        cudaStreamSynchronize(c->stream);  // (no event to wait for later: the copy is over before the slot is used again)
-        return cuda_status(e, "cudaEventRecord");
-    }
-    s.pending = true;
+    tls.upload_used[c->device] = &s;  // (its event is recorded at the call's end)
     return Status();
 }
+void ctx_mark_queued(Ctx* c) { tls.work_queued[c->device] = true; }
 
 CallScope::CallScope() {
     st = get_ctx(&c);
     if (!st.ok()) return;
     auto& blocks = tls.blocks[c->device];
-    if (tls.arena_pending[c->device] && tls.arena_stream[c->device] != c->stream) {
-        cudaStreamWaitEvent(c->stream, tls.arena_done[c->device], 0);
-        tls.arena_pending[c->device] = false;
-    }
+    tls.upload_used[c->device] = nullptr;
+    tls.work_queued[c->device] = false;
+    // (a stream under capture runs nothing now, a graph may not wait for work outside it, and asking for the stream's id would end the capture)
+    if (tls.work_done[c->device] && !capturing(c->stream) && stream_id(c->stream) != tls.work_stream[c->device])
+        cudaStreamWaitEvent(c->stream, tls.work_done[c->device], 0);
     // the previous call has returned, so its staging memory may be reused; when
     // the arena had to chain blocks, replace them by one block of the total size
     if (blocks.size() > 1) {
@@ -190,22 +206,21 @@ CallScope::CallScope() {
 }
 
 CallScope::~CallScope() {
-    if (!c || c->own_stream) return;  // library stream: the call drained it before returning
-    bool used = false;
+    if (!c) return;
+    UploadSlot* up = tls.upload_used[c->device];
+    if (c->own_stream && !up) return;  // library stream: the call drained it before returning
+    bool used = up != nullptr || tls.work_queued[c->device];
     for (const Block& b : tls.blocks[c->device]) used |= b.off != 0;
-    if (!used) return;
-    cudaEvent_t& ev = tls.arena_done[c->device];
-    if (!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) {
+    if (!used || capturing(c->stream)) return;
+    cudaEvent_t& ev = up ? up->done : tls.own_event[c->device];
+    if ((!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) || cudaEventRecord(ev, c->stream) != cudaSuccess) {
         cudaGetLastError();
         cudaStreamSynchronize(c->stream);  // no event to be had: drain instead
         return;
     }
-    if (cudaEventRecord(ev, c->stream) != cudaSuccess) {  // (a capture that the call has ended as invalid)
-        cudaGetLastError();
-        return;
-    }
-    tls.arena_stream[c->device] = c->stream;
-    tls.arena_pending[c->device] = true;
+    if (up) up->pending = true;
+    tls.work_done[c->device] = ev;
+    tls.work_stream[c->device] = stream_id(c->stream);
 }
 
 bool is_device_ptr(const void* p) {
