@@ -17,6 +17,7 @@
 // shared memory); full score vectors are never written in top-k mode.
 #include <cuda_fp16.h>
 
+#include <atomic>
 #include <cfloat>
 #include <cstring>
 #include <mutex>

@@ -213,7 +213,11 @@ struct Plan {
     uint32_t* d_tmp_index = nullptr;
     float* d_tmp_score = nullptr;
     uint64_t last_use = 0;
+    bool captured = false;  // a graph of the library's own names this plan's buffers (see plan_epoch)
 };
+thread_local Plan* g_last_plan = nullptr;    // of the thread's latest score_topk
+thread_local uint32_t g_plans_recycled = 0;  // of this thread's captured plans
+std::atomic<uint32_t> g_plan_threads{0};
 
 Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, size_t nq,
                   uint32_t k, int codec_hint, bool allow_wide, Plan** out) {
@@ -241,6 +245,8 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
         p = cache[0].get();
         for (auto& e : cache)
             if (e->last_use < p->last_use) p = e.get();
+        if (p->captured) ++g_plans_recycled;
+        p->captured = false;
         p->classes.clear();
         p->max_parts = 1;
     }
@@ -799,6 +805,7 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     ctx_mark_queued(c);
     Plan* p = nullptr;
     SLHA_TRY(build_plan(c, tiles, segs, n_segs, nq, k, codec_hint, /*allow_wide=*/state == nullptr, &p));
+    g_last_plan = p;
     const int nwarps = p->threads / 32;
     const bool timed = g_timing.calls < g_timing.max_calls;
     cudaEvent_t* tev = timed ? &g_timing.ev[3 * g_timing.calls] : nullptr;
@@ -916,6 +923,16 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         ++g_timing.calls;
     }
     return Status();
+}
+
+// A captured score_topk names the buffers of one of the calling thread's plans: its graph may run as long as plan_epoch()
+// returns what it returned at the capture (this thread, none of its captured plans rebuilt for another shape).
+uint64_t plan_epoch() {
+    static thread_local const uint32_t thread_no = ++g_plan_threads;
+    return ((uint64_t)thread_no << 32) | g_plans_recycled;
+}
+void plan_was_captured() {
+    if (g_last_plan) g_last_plan->captured = true;
 }
 
 void debug_force_generic_score(bool on) { g_force_generic = on; }

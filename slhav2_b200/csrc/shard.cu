@@ -409,8 +409,8 @@ Status shard_step_device(Ctx* c, Shard* s, const SciRustSlhaTile* tiles, const S
     } step_done{s};
     if (s->timed || s->graphs_off || timing_active()) return shard_enqueue(c, s, tiles, h_segs, n_segs, d_qc, d_qs, nq, k, d_out_index, d_out_score);
     // the call's identity: every pointer and size the enqueued work depends on
-    std::vector<unsigned char> key(sizeof(SlhaB200Segment) * n_segs + 8 * 8);
-    const uint64_t head[8] = {(uint64_t)(uintptr_t)tiles, (uint64_t)(uintptr_t)d_qc, (uint64_t)(uintptr_t)d_qs,
+    std::vector<unsigned char> key(sizeof(SlhaB200Segment) * n_segs + 9 * 8);
+    const uint64_t head[9] = {plan_epoch(), (uint64_t)(uintptr_t)tiles, (uint64_t)(uintptr_t)d_qc, (uint64_t)(uintptr_t)d_qs,
                               (uint64_t)(uintptr_t)d_out_index, (uint64_t)(uintptr_t)d_out_score, (uint64_t)nq, (uint64_t)k,
                               (uint64_t)(uintptr_t)c->stream};
     std::memcpy(key.data(), head, sizeof(head));
@@ -441,6 +441,7 @@ Status shard_step_device(Ctx* c, Shard* s, const SciRustSlhaTile* tiles, const S
         s->graph_exec[gp] = exec;
         s->graph_key[gp] = key;
         s->graph_launches = launches;
+        plan_was_captured();
         cudaGraphDestroy(graph);
         SLHA_CUDA(cudaGraphLaunch(s->graph_exec[gp], c->stream));
         return Status();

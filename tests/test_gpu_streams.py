@@ -140,3 +140,28 @@ def test_score_topk_is_captured_after_calls_on_another_stream():
             assert np.array_equal(a, b)
         rt.cudaGraphExecDestroy(exe)
         rt.cudaGraphDestroy(graph)
+
+
+def test_a_sharded_step_outlives_the_plans_of_other_shapes():
+    # the repeated step is a graph over a plan's buffers; five other shapes rebuild all four plans, then the step comes again
+    n, nq, k = 60000, 4, 40
+    tiles = S.to_device(np.tile(H.random_tiles(5000, 1, seed=750), n // 5000))
+    job = Job(tiles, n, nq, k, 751)
+    others = [Job(tiles, n - 7000 * (i + 1), 4, 500, 760 + i) for i in range(5)]
+    shard = S.Shard(None, 0, 1)
+    job.run()
+    S.synchronize()
+    want = job.result()
+    with Streams(1) as st:
+        for _ in range(2):
+            S.set_stream(st.all[0].value)
+            for _ in range(4):  # plain, captured, replayed twice
+                job.clear()
+                shard.score_topk(*job.args, *job.q, nq, k, *job.out[:2])
+                S.synchronize()
+                for a, b in zip(job.result()[:2], want):
+                    assert np.array_equal(a, b)
+            for o in others:
+                o.run()
+            S.synchronize()
+    shard.destroy()
