@@ -5,7 +5,7 @@
 // The k (index, score) pairs stay in HBM; what crosses PCIe afterwards is one d_v-vector per query
 // row instead of k pairs.
 //
-// One query row is shared by the ATT_SPLIT CTAs of a cluster, each taking a contiguous run of the winners.  Every CTA
+// One query row is shared by the ATT_SPLIT CTAs of a cluster, each taking an equal run of the winners the row has.  Every CTA
 // finds the row's maximum itself (k scores, a few KB from the L2) and weighs its own run; the normalisers and the
 // partial sums of the value rows meet in distributed shared memory, added in a fixed order, so a call is one launch and
 // writes nothing but its results.  Bound: the gather of k value rows per query row (HBM); a thread keeps twelve 16-byte
@@ -73,7 +73,7 @@ __global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
                   size_t d_v, size_t row_stride, const uint64_t* row_base, float* out, float* weights_out) {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ float sm[];  // [run] weights | [run] indices
+    extern __shared__ float sm[];  // weights | indices of the CTA's run
     __shared__ float red[8], own_sum, slot[ATT_THREADS * VEC], part_out[ATT_THREADS * VEC];
     const uint32_t Q = blockIdx.y, part = cluster.block_rank(), tid = threadIdx.x;
     const uint32_t n = top_count ? min(top_count[Q], k) : k;
@@ -84,13 +84,13 @@ __global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
     for (uint32_t i = tid; i < n; i += ATT_THREADS)
         if (ix[i] != 0xFFFFFFFFu) mx = fmaxf(mx, sc[i] * scale);
     mx = block_reduce(mx, red, true);
-    const uint32_t run = (k + ATT_SPLIT - 1) / ATT_SPLIT, lo = min(k, part * run), len = min(k, lo + run) - lo;  // this CTA's winners
+    const uint32_t run = (n + ATT_SPLIT - 1) / ATT_SPLIT, lo = min(n, part * run), len = min(n, lo + run) - lo;  // this CTA's winners
     float* w = sm;
-    uint32_t* wi = reinterpret_cast<uint32_t*>(sm + run);
+    uint32_t* wi = reinterpret_cast<uint32_t*>(sm + (k + ATT_SPLIT - 1) / ATT_SPLIT);
     float sum = 0.0f;
     for (uint32_t j = tid; j < len; j += ATT_THREADS) {
         const uint32_t i = lo + j, id = ix[i];
-        const bool have = i < n && id != 0xFFFFFFFFu;
+        const bool have = id != 0xFFFFFFFFu;
         const float e = have && mx > -INFINITY ? expf(sc[i] * scale - mx) : 0.0f;
         w[j] = e;
         wi[j] = have ? id : 0xFFFFFFFFu;
@@ -152,6 +152,8 @@ __global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
         }
         cluster.sync();  // the peers have read this CTA's sums
     }
+    if (weights_out && n < k)
+        for (uint32_t i = n + part * ATT_THREADS + tid; i < k; i += ATT_SPLIT * ATT_THREADS) weights_out[(size_t)Q * k + i] = 0.0f;
 }
 
 template <typename T, int VEC>

@@ -86,3 +86,25 @@ def test_attend_takes_any_row_length_stride_and_alignment(d_v, stride, shift, bf
                         value_row_stride=stride, weights_out=w_out)
     want, want_w = ora.attend_topk(idx, sc, 0.1, values, top_count=cnt)
     assert close(w_out, want_w) and close(out, want)
+
+
+@pytest.mark.parametrize("k,bf16", [(64, False), (1000, True), (2048, True)])
+def test_attend_rows_that_have_fewer_winners_than_k(k, bf16):
+    # the winners a row has are shared by the eight CTAs of its cluster: counts around their multiples, up to k and beyond
+    n, d_v = 4000, 128
+    counts = np.array([0, 1, 7, 8, 9, k // 8 - 1, k // 8, k // 8 + 1, k // 2 + 3, k - 1, k, k + 5], np.uint32)
+    nq = len(counts)
+    rng = np.random.default_rng(k)
+    values = rng.standard_normal((n, d_v)).astype(F)
+    if bf16:
+        values = H.to_bf16_f32(values).reshape(n, d_v)
+    buf = S.to_device((values.view(np.uint32) >> 16).astype(np.uint16) if bf16 else values)
+    idx = np.stack([rng.permutation(n)[:k] for _ in range(nq)]).astype(np.uint32)
+    idx[8, ::5] = 0xFFFFFFFF
+    sc = (10.0 * rng.standard_normal((nq, k))).astype(F)
+    w_out = np.full((nq, k), 7.0, F)
+    out = S.attend_topk(idx, sc, k, 0.1, buf, d_v, value_dtype=S.BF16 if bf16 else S.F32, top_count=counts, weights_out=w_out)
+    want, want_w = ora.attend_topk(idx, sc, 0.1, values, top_count=np.minimum(counts, k))
+    assert close(w_out, want_w) and close(out, want)
+    for j in range(nq):
+        assert np.all(w_out[j, min(counts[j], k):] == 0)
