@@ -133,32 +133,41 @@ __device__ __forceinline__ bool is_pinned(const PoolDev& p, uint32_t pos, uint32
     return p.recent_window && (max_pos - pos) < p.recent_window;
 }
 
-// the sort key of slot s in `phase`, or SENTINEL when the phase cannot act on it
-__device__ __forceinline__ uint64_t phase_key(const PoolDev& p, int phase, uint64_t s, uint32_t max_pos) {
-    const uint8_t st = p.state[s];
-    if (st == ST_COLD) return SENTINEL;
+// What phase_key needs of a slot: loaded first, so that a scan can have several slots' loads in flight.
+struct SlotMeta {
+    uint8_t st;
+    uint32_t pos, flags, seq;
+    float weight;  // sigma (paging phases) or importance (eviction)
+};
+// state only: may `phase` act on a slot in state st at all
+__device__ __forceinline__ bool phase_looks(int phase, uint8_t st) {
+    return phase >= PH_EVICT ? st != ST_COLD : st == (phase == PH_CORR_WARM ? ST_WARM : ST_HOT);
+}
+// (st is set; the rest is loaded where the phase looks at such slots)
+__device__ __forceinline__ void load_meta(const PoolDev& p, int phase, uint64_t s, SlotMeta& m) {
+    m.pos = m.flags = m.seq = 0u;
+    m.weight = 0.0f;
+    if (!phase_looks(phase, m.st)) return;
     const unsigned char* t = p.tiles + s * TILE_BYTES;
-    const uint32_t flags = *reinterpret_cast<const uint16_t*>(t + 118);
-    bool cand = false;
-    if (phase == PH_CORR_HOT) cand = st == ST_HOT && corr_bytes(flags) && !(flags & F_NOCORR);
-    else if (phase == PH_PAGE) cand = st == ST_HOT;
-    else if (phase == PH_CORR_WARM) cand = st == ST_WARM && corr_bytes(flags) && !(flags & F_NOCORR);
-    else {
-        const bool pin = p.evict_policy == SLHA_B200_EVICT_IMPORTANCE &&
-                         is_pinned(p, *reinterpret_cast<const uint32_t*>(t + 112), max_pos);
-        cand = (phase == PH_EVICT_PINNED) == pin;
+    const uint2 pf = *reinterpret_cast<const uint2*>(t + 112);  // position, head | flags
+    m.pos = pf.x;
+    m.flags = pf.y >> 16;
+    m.seq = (uint32_t)p.seq[s];
+    m.weight = phase >= PH_EVICT ? p.importance[s] : *reinterpret_cast<const float*>(t + 104);
+}
+// the sort key of slot s in `phase`, or SENTINEL when the phase cannot act on it
+__device__ __forceinline__ uint64_t phase_key(const PoolDev& p, int phase, uint64_t s, const SlotMeta& m, uint32_t max_pos) {
+    if (!phase_looks(phase, m.st)) return SENTINEL;
+    if (phase >= PH_EVICT) {
+        const bool pin = p.evict_policy == SLHA_B200_EVICT_IMPORTANCE && is_pinned(p, m.pos, max_pos);
+        if ((phase == PH_EVICT_PINNED) != pin) return SENTINEL;
+        // ccos.rs:586-603: causal = by seq; importance = (importance, seq)
+        return p.evict_policy == SLHA_B200_EVICT_CAUSAL ? (uint64_t)m.seq : ((uint64_t)f32_total_key(m.weight) << 32) | m.seq;
     }
-    if (!cand) return SENTINEL;
-    const uint32_t seq32 = (uint32_t)p.seq[s];
-    if (phase <= PH_CORR_WARM) {
-        // slots_in_paging_order, ccos.rs:526-539: stable sort of the
-        // slot-ascending list by sigma (total order) or by seq
-        return p.page_policy == SLHA_B200_PAGE_LOWEST_IMPACT_FIRST
-                   ? ((uint64_t)f32_total_key(*reinterpret_cast<const float*>(t + 104)) << 32) | (uint32_t)s
-                   : (uint64_t)seq32;
-    }
-    // ccos.rs:586-603: causal = by seq; importance = (importance, seq)
-    return p.evict_policy == SLHA_B200_EVICT_CAUSAL ? (uint64_t)seq32 : ((uint64_t)f32_total_key(p.importance[s]) << 32) | seq32;
+    if (phase != PH_PAGE && (!corr_bytes(m.flags) || (m.flags & F_NOCORR))) return SENTINEL;
+    // slots_in_paging_order, ccos.rs:526-539: stable sort of the
+    // slot-ascending list by sigma (total order) or by seq
+    return p.page_policy == SLHA_B200_PAGE_LOWEST_IMPACT_FIRST ? ((uint64_t)f32_total_key(m.weight) << 32) | (uint32_t)s : (uint64_t)m.seq;
 }
 
 // candidate (key, slot) pairs of one phase, compacted in arbitrary order (keys are unique, so the
@@ -177,7 +186,12 @@ __global__ void phase_build_kernel(PoolDev p, int phase, uint64_t* keys, uint32_
     for (uint64_t r = 0; r < rounds; ++r) {
         const uint64_t s = r * stride + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
         uint64_t key = SENTINEL;
-        if (s < len) key = phase_key(p, phase, s, max_pos);
+        if (s < len) {
+            SlotMeta m;
+            m.st = p.state[s];
+            load_meta(p, phase, s, m);
+            key = phase_key(p, phase, s, m, max_pos);
+        }
         const unsigned hit = __ballot_sync(0xFFFFFFFFu, key != SENTINEL);
         if (hit) {
             const int lane = threadIdx.x & 31;
@@ -322,42 +336,13 @@ __global__ void phase_commit_kernel(PoolDev p) {
 constexpr int EB_BATCH = 4;  // slots a thread of the scans looks at together
 // phase_key of the slots s0, s0 + stride, .. (EB_BATCH of them), the loads of all of them in flight together
 __device__ __forceinline__ void phase_keys(const PoolDev& p, int phase, uint64_t s0, uint64_t stride, uint64_t len, uint32_t max_pos, uint64_t (&key)[EB_BATCH]) {
-    uint8_t st[EB_BATCH];
+    SlotMeta m[EB_BATCH];
 #pragma unroll
-    for (int u = 0; u < EB_BATCH; ++u) st[u] = s0 + u * stride < len ? p.state[s0 + u * stride] : ST_COLD;
-    const bool evict = phase >= PH_EVICT;
-    const uint8_t only = phase == PH_CORR_WARM ? ST_WARM : ST_HOT;  // (the other phases act on every live slot)
-    uint2 pf[EB_BATCH];       // position, head | flags
-    uint32_t seq[EB_BATCH];
-    float imp[EB_BATCH];      // importance (eviction), sigma (paging)
+    for (int u = 0; u < EB_BATCH; ++u) m[u].st = s0 + u * stride < len ? p.state[s0 + u * stride] : ST_COLD;
 #pragma unroll
-    for (int u = 0; u < EB_BATCH; ++u) {
-        const uint64_t s = s0 + u * stride;
-        const bool look = evict ? st[u] != ST_COLD : st[u] == only;
-        pf[u] = make_uint2(0u, 0u);
-        seq[u] = 0u;
-        imp[u] = 0.0f;
-        if (look) {
-            const unsigned char* t = p.tiles + s * TILE_BYTES;
-            pf[u] = *reinterpret_cast<const uint2*>(t + 112);
-            seq[u] = (uint32_t)p.seq[s];
-            imp[u] = evict ? p.importance[s] : *reinterpret_cast<const float*>(t + 104);
-        }
-    }
+    for (int u = 0; u < EB_BATCH; ++u) load_meta(p, phase, s0 + u * stride, m[u]);
 #pragma unroll
-    for (int u = 0; u < EB_BATCH; ++u) {
-        key[u] = SENTINEL;
-        const uint32_t flags = pf[u].y >> 16;
-        if (evict) {
-            if (st[u] == ST_COLD) continue;
-            const bool pin = p.evict_policy == SLHA_B200_EVICT_IMPORTANCE && is_pinned(p, pf[u].x, max_pos);
-            if ((phase == PH_EVICT_PINNED) != pin) continue;
-            key[u] = p.evict_policy == SLHA_B200_EVICT_CAUSAL ? (uint64_t)seq[u] : ((uint64_t)f32_total_key(imp[u]) << 32) | seq[u];
-        } else {
-            if (st[u] != only || (phase != PH_PAGE && (!corr_bytes(flags) || (flags & F_NOCORR)))) continue;
-            key[u] = p.page_policy == SLHA_B200_PAGE_LOWEST_IMPACT_FIRST ? ((uint64_t)f32_total_key(imp[u]) << 32) | (uint32_t)(s0 + u * stride) : (uint64_t)seq[u];
-        }
-    }
+    for (int u = 0; u < EB_BATCH; ++u) key[u] = phase_key(p, phase, s0 + u * stride, m[u], max_pos);
 }
 constexpr int EB_THREADS = 512, EB_ITEMS = 8, EB_CAP = EB_THREADS * EB_ITEMS, EB_LEVELS = 6, EB_BINS = 4096;
 struct EnforceState {
