@@ -56,6 +56,7 @@ Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
 // The call under way leaves work in a plan's buffers (kept per thread, like the scratch arena): see CallScope.
 void ctx_mark_queued(Ctx* c);
 void count_launch(int n = 1);
+int sm_count(int device);  // multiprocessors of a device
 uint64_t launch_count();
 void tls_set_device(int dev);
 void tls_set_stream(void* s);

@@ -704,7 +704,7 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
     // us per call at 8 / 592 / 1184 / 2368 / 4736 keys): 32 keys per CTA 39 / 39 / 37 / 37 / 37, 16: 29 / 28 / 29 / 29 / 39,
     // 8: 21 / 21 / 21 / 27 / 49, 4: 17 / 19 / 21 / 37 / 70, 1: 17 / 31 / 59 / 113 / 221 -- a CTA of 4 keys is as fast as one of a
     // single key, and a wider form is no slower from where the narrower one fills the SMs twice.
-    while (kb > 4 && n <= (uint64_t)(kb / 2) * 148) kb >>= 1;
+    while (kb > 4 && n <= (uint64_t)(kb / 2) * (uint64_t)sm_count(m->device)) kb >>= 1;
     *kb_out = kb;
     a.kb = kb;
     return Status();

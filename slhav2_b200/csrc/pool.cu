@@ -1146,7 +1146,7 @@ Status pool_observe(Ctx* c, Pool* pl, const uint32_t* d_slots, const float* d_sc
     ObserveTmp* tmp = reinterpret_cast<ObserveTmp*>(pl->d_observe);
     float* partial = reinterpret_cast<float*>(tmp + 1);
     SLHA_CUDA(cudaMemsetAsync(tmp, 0, sizeof(ObserveTmp), c->stream));
-    const uint32_t grid = std::min<uint32_t>(grid_for(n), 148 * 4);
+    const uint32_t grid = std::min<uint32_t>(grid_for(n), (uint32_t)sm_count(c->device) * 4);
     observe_pass1<<<grid, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, tmp);
     observe_pass2<<<nparts, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial);
     observe_pass3<<<grid, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial, nparts);
@@ -1162,7 +1162,7 @@ Status pool_stats(Ctx* c, Pool* pl, uint64_t out[8]) {
     // (a pool that has only ever been appended to with codecs without a correction plane holds no tile that dropped one)
     const uint32_t cm = pl->codec_mask;
     const bool planes = !cm || (cm & (0x80000000u | (1u << SLHA_CODEC_TQ3) | (1u << SLHA_CODEC_MIX3)));
-    stats_kernel<<<std::min<uint32_t>(grid_for(std::max<uint64_t>(pl->h_cnt.len, 1)), 148 * 4), 256, 0, c->stream>>>(pl->dev, d, planes);
+    stats_kernel<<<std::min<uint32_t>(grid_for(std::max<uint64_t>(pl->h_cnt.len, 1)), (uint32_t)sm_count(c->device) * 4), 256, 0, c->stream>>>(pl->dev, d, planes);
     count_launch();
     SLHA_CUDA(cudaGetLastError());
     SLHA_CUDA(cudaMemcpyAsync(out, d, 64, cudaMemcpyDeviceToHost, c->stream));

@@ -21,6 +21,19 @@ Status cuda_status(cudaError_t e, const char* what) {
 
 static std::atomic<uint64_t> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
+int sm_count(int device) {
+    static std::atomic<int> known[16];
+    std::atomic<int>& n = known[device & 15];
+    int v = n.load(std::memory_order_relaxed);
+    if (v == 0) {
+        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, device) != cudaSuccess || v < 1) {
+            cudaGetLastError();
+            return 148;
+        }
+        n.store(v, std::memory_order_relaxed);
+    }
+    return v;
+}
 uint64_t launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
 // ---- per-thread context ------------------------------------------------------

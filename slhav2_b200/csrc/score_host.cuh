@@ -274,8 +274,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     p->cap = cap;
 
     // tensor-core kernel: one persistent CTA per SM
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const int sms = sm_count(c->device);
     {
         // Codec hint: -1 = the flags of the first tile of the first non-empty segment decide which kind of tile the launch
         // decodes.  A wrong hint costs speed only (tiles of another kind are handed to the generic kernel).
@@ -661,8 +660,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     // decode, a query outside the fp16 split).  codec_hint -2: codecs the tensor-core kernel does not decode together;
     // bit 0: NF4 tiles beside INT4 ones; -1: not known.
     if (n >= 32768 && n < 0xFFFFFFFFull && codec_hint != -2 && !g_force_generic) {
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+        const int sms = sm_count(c->device);
         Cuts cuts((uint64_t)n * ((nq + 3) / 4), sms, ST_M, 2048);
         cuts.add(SlhaB200Segment{0, (uint32_t)n, 0, (uint32_t)nq, 0}, 4);
         cuts.finish();
@@ -724,8 +722,7 @@ __global__ void fill_rows_kernel(float* scores, const unsigned long long* row_of
 Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, const float* d_q_coarse,
                              const uint64_t* d_q_sign, size_t nq, float* d_scores, const unsigned long long* d_row_offsets,
                              uint32_t row_len, float fill) {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const int sms = sm_count(c->device);
     bool wide = !g_force_generic, fills = false;
     uint64_t total = 0, wtotal = 0;
     std::vector<uint32_t> tail(nq, row_len);
