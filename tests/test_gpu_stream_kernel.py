@@ -89,3 +89,77 @@ def test_segments_of_different_codecs_in_one_call(nq):
             m = min(n, 32)
             assert np.all(np.abs(sc[j, :m] - want[idx[j, :m]]) <= 1e-3)
             assert np.all(np.abs(sc[j, :m] - np.sort(want)[::-1][:m]) <= 2e-3)
+
+
+def _check_rows(tiles, rows, qc, qs, idx, sc, cnt, k, every=1):
+    for i, (tb, n, qb, q, base) in enumerate(rows):
+        if i % every:
+            continue
+        for j in range(qb, qb + q):
+            m = min(n, k)
+            assert cnt[j] == m and np.all(idx[j, m:] == 0xFFFFFFFF)
+            if not n:
+                continue
+            want = ora.score_tiles(tiles[tb:tb + n], qc[j], qs[j])
+            got = idx[j, :m].astype(np.int64) - base
+            assert len(set(got)) == m and got.min() >= 0 and got.max() < n
+            assert np.all(np.abs(sc[j, :m] - want[got]) <= 1e-3) and np.all(np.abs(sc[j, :m] - np.sort(want)[::-1][:m]) <= 2e-3)
+
+
+@pytest.mark.parametrize("codec", [3, 5])
+@pytest.mark.parametrize("n_seg,longest,nq,k", [(100, 3000, 3, 40), (90, 2500, 6, 300), (3000, 20, 2, 7), (160, 9000, 4, 16), (1, 700, 5, 64), (8, 20011, 4, 512)])
+def test_top_k_of_many_ragged_segments(codec, n_seg, longest, nq, k):
+    # more streams than half the CTAs: equal shares instead of interleaved ones, several items per CTA, thresholds carried from one
+    # item to the next; thousands of short segments; and a few long ones, interleaved
+    rng = np.random.default_rng(n_seg + k + 1000 * codec)  # (plans are kept by shape, each for one codec)
+    base = H.random_tiles(4000, codec, seed=800 + codec, warm_every=7, nocorr_every=5)
+    rows, tb = [], 0
+    for i in range(n_seg):
+        n = int(rng.integers(0 if i % 3 else 1, longest + 1))
+        rows.append((tb, n, i * nq, nq, 3 * i))
+        tb += n
+    tiles = base[rng.integers(0, len(base), tb)]
+    qc, qs = H.random_queries(n_seg * nq, 801)
+    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, n_seg * nq, k)
+    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
+    _check_rows(tiles, rows, qc, qs, idx, sc, cnt, k, every=max(1, n_seg // 60))
+
+
+@pytest.mark.parametrize("seed", range(6))
+def test_mix3_top_k_of_random_shapes(seed):
+    rng = np.random.default_rng(900 + seed)
+    n_seg = int(rng.integers(1, 12))
+    base = H.random_tiles(3000, 5, seed=810 + seed, warm_every=9, nocorr_every=4)
+    rows, tb, qb = [], 0, 0
+    for i in range(n_seg):
+        n, nq = int(rng.choice([0, 1, 33, int(rng.integers(2, 2000)), int(rng.integers(2000, 30000))])), int(rng.choice([1, 2, 4, 5, 9]))
+        rows.append((tb, n, qb, nq, int(rng.integers(0, 1000))))
+        tb, qb = tb + n, qb + nq
+    tiles = base[rng.integers(0, len(base), max(tb, 1))]
+    qc, qs = H.random_queries(qb, 820 + seed)
+    k = int(rng.choice([1, 17, 256, 1500]))
+    dt, seg = S.to_device(tiles), S.make_segments(rows)
+    for _ in range(2):
+        idx, sc, cnt = S.score_topk(dt, seg, qc, qs, qb, k)
+        _check_rows(tiles, rows, qc, qs, idx, sc, cnt, k)
+
+
+@pytest.mark.parametrize("nq,n_seg,n", [(2, 1, 5000), (4, 100, 900), (20, 3, 2000)])
+def test_mix3_rows_that_are_handed_back(nq, n_seg, n):
+    # a stretch of another codec in one segment, an element beyond the split in another: the rows of those, and no others
+    tiles = np.tile(H.random_tiles(n, 5, seed=830, nocorr_every=4), n_seg)
+    other = n_seg - 1
+    tiles[other * n + n // 2:other * n + n // 2 + 70] = H.random_tiles(70, 4, seed=831)
+    rows = [(i * n, n, i * nq, nq, 0) for i in range(n_seg)]
+    qc, qs = H.random_queries(n_seg * nq, 832)
+    handed = nq
+    if n_seg > 1:
+        qc[nq + 1, 100] = 1e30
+        handed = 2 * nq
+    k = 25
+    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, n_seg * nq, k)
+    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == handed
+    if n_seg > 1:
+        qc[nq + 1] = 0  # (a row of 1e30: its winners are those of one element)
+        rows = rows[:1] + rows[2:]
+    _check_rows(tiles, rows, qc, qs, idx, sc, cnt, k, every=7 if n_seg > 9 else 1)
