@@ -796,6 +796,12 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a)
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
+    if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
+        uint32_t f = 0;
+        for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS)
+            for (uint32_t q = 0; q < a.stream_items[e].n_queries; ++q) f |= a.only_flagged[a.stream_items[e].query_begin + q];
+        if (!__syncthreads_or(f != 0u)) return;
+    }
     uint32_t flags = first_tile_flags(a, a.stream_items[i]);  // (on its way while the CTA is set up)
     const bool nf4_too = a.nf4_table == 1u || (a.nf4_table == 2u && (first_tile_flags(a, a.stream_items[0]) & F_NF4));
     TileCta cta = tile_open<true>(smem_raw);
