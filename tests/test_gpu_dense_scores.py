@@ -111,7 +111,7 @@ def test_dense_calls_of_different_shapes_queued_behind_one_another():
     shapes = [(int(rng.integers(1, 30000)), int(rng.integers(1, 41))) for _ in range(9)] + [(32000, 9)]
     jobs = []
     for n, nq in shapes:
-        parts = 30000 if n > 30000 else min(n, 3)  # (30 000 segments: tables of more than a megabyte)
+        parts = 30000 if n > 30000 else (900 if n > 20000 else min(n, 3))  # (30 000 segments: tables of more than a megabyte; 900: of some 200 KB)
         cut = np.linspace(0, n, parts + 1).astype(int)
         rows = [(cut[i], cut[i + 1] - cut[i], 0, nq, cut[i]) for i in range(parts)]
         jobs.append((n, nq, S.make_segments(rows), np.arange(nq, dtype=np.uint64) * n, S.DeviceBuffer(nq * n * 4)))
@@ -119,8 +119,9 @@ def test_dense_calls_of_different_shapes_queued_behind_one_another():
     assert rt.cudaStreamCreateWithFlags(C.byref(stream), 1) == 0
     S.set_stream(stream.value)
     try:
-        for n, nq, seg, off, out in jobs:
-            S.score_segments(dt, seg, dq, ds, nq, out, off, n)
+        for _ in range(4):
+            for n, nq, seg, off, out in jobs:
+                S.score_segments(dt, seg, dq, ds, nq, out, off, n)
         S.synchronize()
     finally:
         S.set_stream(None)
