@@ -51,7 +51,10 @@ struct Ctx {
 Status get_ctx(Ctx** out);  // fails with SLHA_ERR_DEVICE when there is no GPU
 Status ctx_device_scratch(Ctx* c, size_t bytes, void** out);
 Status ctx_host_scratch(Ctx* c, size_t bytes, void** out);
-// A small host table into device scratch, on the call's stream: `src` may go away when this returns.  Fails on a stream that is being captured.
+// Host tables to the device, on the call's stream: `src` may go away when this returns.  ctx_upload: into the call's scratch.  Only on a stream
+// that is not being captured: ctx_no_capture fails on one that is, and ends the capture as invalid.
+Status ctx_no_capture(Ctx* c);
+Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes);
 Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
 // The call under way leaves work in a plan's buffers (kept per thread, like the scratch arena): see CallScope.
 void ctx_mark_queued(Ctx* c);

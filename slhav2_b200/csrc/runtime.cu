@@ -158,16 +158,21 @@ unsigned long long stream_id(cudaStream_t s) {
 }
 }  // namespace
 
+Status ctx_no_capture(Ctx* c) {
+    if (!capturing(c->stream)) return Status();
+    // a graph would keep the address of host memory that this call's successors write again: refused, and the capture ends
+    // as invalid, like everywhere the library has to wait for a stream
+    SLHA_CUDA(cudaStreamSynchronize(c->stream));
+    return Status(SLHA_ERR_DEVICE, "this call cannot be captured into a graph");
+}
 Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
-    if (capturing(c->stream)) {
-        // a graph would keep the address of host memory that this call's successors write again: refused, and the capture ends
-        // as invalid, like everywhere the library has to wait for a stream
-        SLHA_CUDA(cudaStreamSynchronize(c->stream));
-        return Status(SLHA_ERR_DEVICE, "this call cannot be captured into a graph");
-    }
+    SLHA_TRY(ctx_no_capture(c));
     SLHA_TRY(ctx_device_scratch(c, bytes, dev));
+    return ctx_copy_table(c, *dev, src, bytes);
+}
+Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
     if (bytes > UPLOAD_MOST) {
-        SLHA_CUDA(cudaMemcpyAsync(*dev, src, bytes, cudaMemcpyHostToDevice, c->stream));
+        SLHA_CUDA(cudaMemcpyAsync(dev, src, bytes, cudaMemcpyHostToDevice, c->stream));
         SLHA_CUDA(cudaStreamSynchronize(c->stream));
         return Status();
     }
@@ -199,7 +204,7 @@ Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev) {
     if (!s.done) SLHA_CUDA(cudaEventCreateWithFlags(&s.done, cudaEventDisableTiming));
     if (brief) s.table.assign(static_cast<const unsigned char*>(src), static_cast<const unsigned char*>(src) + bytes);
     else std::memcpy(s.p, src, bytes);
-    SLHA_CUDA(cudaMemcpyAsync(*dev, brief ? s.table.data() : s.p, bytes, cudaMemcpyHostToDevice, c->stream));
+    SLHA_CUDA(cudaMemcpyAsync(dev, brief ? s.table.data() : s.p, bytes, cudaMemcpyHostToDevice, c->stream));
     tls.upload_used[c->device] = &s;  // (its event is recorded at the call's end)
     return Status();
 }

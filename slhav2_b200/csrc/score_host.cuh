@@ -165,6 +165,21 @@ struct DevBuf {
     ~DevBuf() { cudaFree(p); }
 };
 
+// Several small host arrays in one upload.
+struct Blob {
+    std::vector<unsigned char> bytes;
+    template <typename T>
+    size_t add(const std::vector<T>& v) {
+        const size_t at = (bytes.size() + 15) / 16 * 16;
+        bytes.resize(at + v.size() * sizeof(T));
+        if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
+        return at;
+    }
+    Status upload(Ctx* c, unsigned char** dev) {
+        return ctx_upload(c, bytes.data(), bytes.size(), (void**)dev);
+    }
+};
+
 // The cached decomposition of one score_topk call shape.
 struct Plan {
     std::vector<unsigned char> key;
@@ -203,7 +218,7 @@ struct Plan {
     int codec_hint_in = -1;
     bool force_generic_in = false;
     uint32_t mma_grid = 0;
-    DevBuf b_stream_items, b_items, b_qbegin, b_qcount, b_keys, b_cnt, b_cta, b_gpivot, b_gbuf, b_gsel, b_vq, b_tmp, b_wide_items, b_wide_cta;
+    DevBuf b_tables, b_keys, b_cnt, b_gpivot, b_gbuf, b_gsel, b_tmp;
     // Two-level merge for calls with few queries and many candidate lists per query (a pool scored
     // by one GQA group: 148 lists each): groups of `group_parts` lists are merged by a CTA each into
     // `n_groups` intermediate (index, score) lists per query, which a second launch merges.
@@ -237,6 +252,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
             *out = e.get();
             return Status();
         }
+    SLHA_TRY(ctx_no_capture(c));  // (a new plan has tables to copy)
     Plan* p;
     if (cache.size() < 4) {
         cache.push_back(std::make_unique<Plan>());
@@ -444,21 +460,15 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     std::vector<uint32_t> q_stride(nq, 1);
     for (const WorkItem& w : all)
         for (uint32_t g = 0; g < w.n_queries; ++g) q_stride[w.query_begin + g] = w.pad & 0xFFu;
-    SLHA_TRY(p->b_items.ensure(all.size() * sizeof(WorkItem)));
     if (!stream_items.empty() && stream_items.size() != all.size()) return Status(SLHA_ERR_PANIC, "score plan: stream items out of step");
-    SLHA_TRY(p->b_stream_items.ensure(stream_items.size() * sizeof(WorkItem)));
-    p->d_stream_items = stream_items.empty() ? nullptr : (WorkItem*)p->b_stream_items.p;
-    if (p->d_stream_items)
-        SLHA_CUDA(cudaMemcpyAsync(p->d_stream_items, stream_items.data(), stream_items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, c->stream));
-    SLHA_TRY(p->b_qbegin.ensure(nq * 4));
-    SLHA_TRY(p->b_qcount.ensure(nq * 4));
     p->list_cap = (k + std::max<uint32_t>(64, k / 2) + 31) / 32 * 32;
     SLHA_TRY(p->b_keys.ensure((size_t)n_lists * p->list_cap * 8));
     SLHA_TRY(p->b_cnt.ensure((size_t)n_lists * 4));
-    SLHA_TRY(p->b_cta.ensure(cta_begin.size() * 4));
     // Wide scoring: every segment brings 16 or more queries and the launch holds INT4 / MX-INT4 or TQ3 tiles.  Work items
     // of up to 64 query rows; the (segment, row group) streams are cut into one share per CTA, in whole 128-tile blocks.
     uint32_t wide_parts = 1;
+    std::vector<WorkItem> wi;
+    std::vector<uint32_t> wcta;
     {
         bool all_wide = p->use_mma && allow_wide && n_segs > 0 && p->kind != 0;
         uint64_t wtotal = 0;
@@ -469,8 +479,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
         if (all_wide && wtotal > 0) {
             uint64_t wshare = (wtotal + sms - 1) / sms;
             wshare = std::max<uint64_t>(WIDE_M, (wshare + WIDE_M - 1) / WIDE_M * WIDE_M);
-            std::vector<WorkItem> wi;
-            std::vector<uint32_t> wcta(1, 0);
+            wcta.push_back(0);
             uint64_t wfilled = 0;
             for (size_t i = 0; i < n_segs; ++i) {
                 const SlhaB200Segment& s = segs[i];
@@ -497,12 +506,6 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
                 }
             }
             if (wcta.back() != (uint32_t)wi.size()) wcta.push_back((uint32_t)wi.size());
-            SLHA_TRY(p->b_wide_items.ensure(wi.size() * sizeof(WorkItem)));
-            SLHA_TRY(p->b_wide_cta.ensure(wcta.size() * 4));
-            p->d_wide_items = (WorkItem*)p->b_wide_items.p;
-            p->d_wide_cta = (uint32_t*)p->b_wide_cta.p;
-            SLHA_CUDA(cudaMemcpyAsync(p->d_wide_items, wi.data(), wi.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, c->stream));
-            SLHA_CUDA(cudaMemcpyAsync(p->d_wide_cta, wcta.data(), wcta.size() * 4, cudaMemcpyHostToDevice, c->stream));
             p->n_wide_items = (uint32_t)wi.size();
             p->wide_grid = (uint32_t)wcta.size() - 1;
             p->wide = true;
@@ -532,42 +535,45 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     SLHA_TRY(p->b_gpivot.ensure(p->gstate_bytes));
     if (p->use_mma) SLHA_TRY(p->b_gbuf.ensure(nq * (size_t)p->gcap * 8));
     p->d_gbuf = (uint64_t*)p->b_gbuf.p;
-    p->d_items = (WorkItem*)p->b_items.p;
-    p->d_q_list_begin = (uint32_t*)p->b_qbegin.p;
-    p->d_q_list_count = (uint32_t*)p->b_qcount.p;
     p->d_cand_keys = (uint64_t*)p->b_keys.p;
     p->d_cand_cnt = (uint32_t*)p->b_cnt.p;
-    p->d_cta_begin = (uint32_t*)p->b_cta.p;
     p->d_gpivot = (unsigned long long*)p->b_gpivot.p;
     p->n_items = (uint32_t)all.size();
-    // (pageable sources: cudaMemcpyAsync returns once they are staged, so the vectors may die)
-    SLHA_CUDA(cudaMemcpyAsync(p->d_cta_begin, cta_begin.data(), cta_begin.size() * 4, cudaMemcpyHostToDevice, c->stream));
     p->n_groups = 0;
+    std::vector<uint32_t> vq;
     if (nq <= 64 && p->max_parts >= 24 && !p->use_mma) {
         uint32_t G = 1;
         while (G * G < p->max_parts) ++G;
         const uint32_t ng = (p->max_parts + G - 1) / G;
-        std::vector<uint32_t> vq(2 * (size_t)ng * nq);
+        vq.resize(2 * (size_t)ng * nq);
         for (uint32_t g = 0; g < ng; ++g)
             for (size_t Q = 0; Q < nq; ++Q) {
                 const uint32_t parts = q_count[Q], lo = g * G;
                 vq[g * nq + Q] = q_begin[Q] + lo * q_stride[Q];
                 vq[(size_t)ng * nq + g * nq + Q] = (parts > lo ? std::min(G, parts - lo) : 0u) | (q_stride[Q] << 24);
             }
-        SLHA_TRY(p->b_vq.ensure(vq.size() * 4));
         SLHA_TRY(p->b_tmp.ensure((size_t)ng * nq * k * 8));
-        p->d_vq_begin = (uint32_t*)p->b_vq.p;
-        p->d_vq_count = p->d_vq_begin + (size_t)ng * nq;
         p->d_tmp_index = (uint32_t*)p->b_tmp.p;
         p->d_tmp_score = reinterpret_cast<float*>(p->d_tmp_index + (size_t)ng * nq * k);
-        SLHA_CUDA(cudaMemcpyAsync(p->d_vq_begin, vq.data(), vq.size() * 4, cudaMemcpyHostToDevice, c->stream));
         p->n_groups = ng;
         p->group_parts = G;
     }
     for (size_t Q = 0; Q < nq; ++Q) q_count[Q] |= q_stride[Q] << 24;
-    SLHA_CUDA(cudaMemcpyAsync(p->d_items, all.data(), all.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, c->stream));
-    SLHA_CUDA(cudaMemcpyAsync(p->d_q_list_begin, q_begin.data(), nq * 4, cudaMemcpyHostToDevice, c->stream));
-    SLHA_CUDA(cudaMemcpyAsync(p->d_q_list_count, q_count.data(), nq * 4, cudaMemcpyHostToDevice, c->stream));
+    Blob tables;
+    const size_t o_items = tables.add(all), o_stream = tables.add(stream_items), o_cta = tables.add(cta_begin), o_qb = tables.add(q_begin), o_qc = tables.add(q_count);
+    const size_t o_vq = tables.add(vq), o_wi = tables.add(wi), o_wcta = tables.add(wcta);
+    SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
+    unsigned char* dev = static_cast<unsigned char*>(p->b_tables.p);
+    SLHA_TRY(ctx_copy_table(c, dev, tables.bytes.data(), tables.bytes.size()));
+    p->d_items = reinterpret_cast<WorkItem*>(dev + o_items);
+    p->d_stream_items = stream_items.empty() ? nullptr : reinterpret_cast<WorkItem*>(dev + o_stream);
+    p->d_cta_begin = reinterpret_cast<uint32_t*>(dev + o_cta);
+    p->d_q_list_begin = reinterpret_cast<uint32_t*>(dev + o_qb);
+    p->d_q_list_count = reinterpret_cast<uint32_t*>(dev + o_qc);
+    p->d_vq_begin = reinterpret_cast<uint32_t*>(dev + o_vq);
+    p->d_vq_count = p->d_vq_begin + vq.size() / 2;
+    p->d_wide_items = reinterpret_cast<WorkItem*>(dev + o_wi);
+    p->d_wide_cta = reinterpret_cast<uint32_t*>(dev + o_wcta);
     p->key = std::move(key);
     p->device = c->device;
     *out = p;
@@ -603,21 +609,6 @@ Status launch_validate_tiles(Ctx* c, const SciRustSlhaTile* tiles, size_t n, uns
     SLHA_CUDA(cudaGetLastError());
     return Status();
 }
-
-// One upload of several small host arrays into the call's scratch.
-struct Blob {
-    std::vector<unsigned char> bytes;
-    template <typename T>
-    size_t add(const std::vector<T>& v) {
-        const size_t at = (bytes.size() + 15) / 16 * 16;
-        bytes.resize(at + v.size() * sizeof(T));
-        if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
-        return at;
-    }
-    Status upload(Ctx* c, unsigned char** dev) {
-        return ctx_upload(c, bytes.data(), bytes.size(), (void**)dev);
-    }
-};
 
 // Cuts of (segment, group of up to `width` query rows) streams into one share per CTA.
 struct Cuts {

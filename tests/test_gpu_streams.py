@@ -165,3 +165,29 @@ def test_a_sharded_step_outlives_the_plans_of_other_shapes():
                 o.run()
             S.synchronize()
     shard.destroy()
+
+
+def test_a_new_plan_is_not_made_under_capture():
+    # its tables come from host memory that goes away with the call; a pool knows its codec, so no look at a tile stops the call earlier
+    n = 3000
+    pool = S.TilePool(n + 64, 2**40)
+    model = S.Model.from_projection(H.make_model_pair(128)[1], 128, 7)
+    pool.append_keys(model, H.gaussian_keys(770, n, 128), S.CODEC_MIXED, want_slots=False)
+    qc, qs = H.random_queries(2, 771)
+    dq, ds = S.to_device(qc), S.to_device(qs)
+    out = S.DeviceBuffer(2 * 29 * 4), S.DeviceBuffer(2 * 29 * 4), S.DeviceBuffer(8)
+    with Streams(1) as st:
+        graph = C.c_void_p()
+        S.set_stream(st.all[0].value)
+        assert st.rt.cudaStreamBeginCapture(st.all[0], 2) == 0
+        with pytest.raises(S.SlhaError) as e:
+            pool.score_topk(dq, ds, 2, 29, *out)
+        assert e.value.code == S.ERR_DEVICE
+        st.rt.cudaStreamEndCapture(st.all[0], C.byref(graph))
+        st.rt.cudaGetLastError()
+        assert not graph.value
+        pool.score_topk(dq, ds, 2, 29, *out)
+        S.synchronize()
+        idx = out[0].download(np.uint32, 58).reshape(2, 29)
+    want = pool.score_topk(qc, qs, 2, 29)
+    assert np.array_equal(idx, want[0])
