@@ -8,8 +8,9 @@
 //
 // Bound: the chain of a block (decode, TMEM store, eight or nine MMAs, read-back, filter), about 5000 cycles with four warpgroups in
 // flight.  MIX3 top-k of 32 ragged segments (485 k tiles x 4 queries): 367 -> 72 us a call; dense MIX3 scores of 8 x 4096 tiles x 4
-// rows: 278 -> 33 us a call (8.7 us of kernel), both from the generic kernel.  Top-k of the codecs that score_stream_kernel
-// decodes stays there: the same chain took 295 us against 255 us on 8.4 M MX-INT4 tiles and 565 us against 410 us on as many NF4 tiles.
+// rows: 278 -> 37 us a call (8.7 us of kernel), both from the generic kernel.  Top-k of the codecs that score_stream_kernel
+// decodes stays there: with this kernel a call took 301 us against 292 us on 8.4 M MX-INT4 tiles and 573 us against 462 us on as many
+// NF4 tiles.
 #pragma once
 
 namespace slha {
@@ -621,13 +622,14 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                 gave_up = true;
                 continue;
             }
+            // (the row's power of two is exact; the tile's scale comes in the last step, so that the coarse term is rounded once there)
+            const float su = __uint_as_float(meta.x) * (1.0f / 255.0f);
             {
-                const float su = __uint_as_float(meta.x) * (1.0f / 255.0f);
                 const float4 inv = *reinterpret_cast<const float4*>(qinv);
-                c[0] = (c[0] + low[0]) * inv.x * su;
-                c[1] = (c[1] + low[1]) * inv.y * su;
-                c[2] = (c[2] + low[2]) * inv.z * su;
-                c[3] = (c[3] + low[3]) * inv.w * su;
+                c[0] = (c[0] + low[0]) * inv.x;
+                c[1] = (c[1] + low[1]) * inv.y;
+                c[2] = (c[2] + low[2]) * inv.z;
+                c[3] = (c[3] + low[3]) * inv.w;
             }
             if (dead) continue;
             const float lam = (flags & F_WARM) ? 0.0f : __uint_as_float(meta.y);
@@ -641,8 +643,10 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                 asm volatile("ld.volatile.shared.v4.f32 {%0,%1,%2,%3}, [%4];\n" : "=f"(th.x), "=f"(th.y), "=f"(th.z), "=f"(th.w) : "r"(tail_s + 144u));
                 const float tq[4] = {th.x, th.y, th.z, th.w};
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    if (q < nq && live && !(fmaf(fabsf(lam), 257.0f, fmaf(fabsf(c[q]), 1e-6f, c[q])) < tq[q])) m |= 1u << q;  // (a NaN goes on to the exact test)
+                for (int q = 0; q < 4; ++q) {
+                    const float x = c[q] * su;
+                    if (q < nq && live && !(fmaf(fabsf(lam), 257.0f, fmaf(fabsf(x), 1e-6f, x)) < tq[q])) m |= 1u << q;  // (a NaN goes on to the exact test)
+                }
             }
             if (__any_sync(0xFFFFFFFFu, m != 0u)) {
                 const uint4 ra = lds_v4<64>(row), rb = lds_v4<80>(row);
@@ -653,7 +657,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                         const int h = __popc(ra.x ^ qw[0]) + __popc(ra.y ^ qw[1]) + __popc(ra.z ^ qw[2]) + __popc(ra.w ^ qw[3]) +
                                       __popc(rb.x ^ qw[4]) + __popc(rb.y ^ qw[5]) + __popc(rb.z ^ qw[6]) + __popc(rb.w ^ qw[7]);
                         // 256 - 2 h without an integer conversion: (2^23 + h) as a bit pattern, times -2, plus 2^24 + 256 (exact)
-                        c[q] = fmaf(lam, fmaf(__uint_as_float(0x4B000000u | (uint32_t)h), -2.0f, 16777472.0f), c[q]);
+                        c[q] = fmaf(c[q], su, lam * fmaf(__uint_as_float(0x4B000000u | (uint32_t)h), -2.0f, 16777472.0f));
                     }
                 if (!DENSE) {
                     if (round == 0) {

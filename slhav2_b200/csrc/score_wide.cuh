@@ -368,7 +368,7 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
                 for (int j = 0; j < 16; ++j) {
                     const float2 u = uq[16 * ch + j];
                     const float h = fmaf(__uint_as_float(s[j]), -32768.0f, u.x);  // 256 - 2 hamming, exact
-                    sc[j] = fmaf(lam, h, sc[j] * u.y * su);
+                    sc[j] = fmaf(sc[j] * u.y, su, lam * h);  // (u.y is a power of two: the coarse term is rounded once)
                 }
             }
             if (ACCS > 1 && b + 1 < blocks) stage(b + 1);  // (its barrier: every warp has read this block's accumulators)

@@ -215,8 +215,9 @@ def test_query_rows_beyond_the_split_take_the_generic_kernel(nq, value):
     assert np.all(np.abs(out[4:] - gout[4:]) <= 1e-4 * (1 + np.abs(gout[4:])))
 
 
+@pytest.mark.parametrize("residual", [False, True])
 @pytest.mark.parametrize("codec,nq", [(c, nq) for c in range(7) for nq in (1, 4)] + [(2, 20), (2, 64), (5, 20), (5, 64)])
-def test_scores_are_no_further_from_64_bits_than_the_generic_kernels(codec, nq):
+def test_scores_are_no_further_from_64_bits_than_the_generic_kernels(codec, nq, residual):
     # the calls that tensor-core kernels took over from it (float32 products in short chains): 2-norm of the error over six sets of
     # tiles and queries, 5 % for chance (a single set's two errors differ by up to 12 % either way)
     n = 1500 + codec
@@ -225,9 +226,13 @@ def test_scores_are_no_further_from_64_bits_than_the_generic_kernels(codec, nq):
     square = np.zeros((2, 2, 2))  # [dense, top-k][tensor cores, generic][error, size]
     for seed in range(590, 650, 10):
         tiles = H.random_tiles(n, codec, seed=seed + codec, nocorr_every=5)
-        tiles["dynamic_lambda"] = 0
         qc, qs = H.random_queries(nq, seed + 1)
         want = _exact_terms(tiles, qc)[0]
+        # a residual a third of the key's size, or none
+        tiles["dynamic_lambda"] = 0.0235 * want.std() / 128**0.5 if residual else 0
+        lam = tiles["dynamic_lambda"].astype(np.float64)
+        bits = np.unpackbits(np.ascontiguousarray(tiles["residual_bitmap"]).view(np.uint8).reshape(n, 32), axis=1)
+        want += lam * np.stack([256.0 - 2.0 * (bits != np.unpackbits(q.view(np.uint8))).sum(1) for q in qs])
         dt = S.to_device(tiles)
         for generic in (0, 1):
             S.debug_force_generic_score(bool(generic))
