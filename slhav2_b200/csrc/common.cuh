@@ -56,8 +56,8 @@ Status ctx_host_scratch(Ctx* c, size_t bytes, void** out);
 Status ctx_no_capture(Ctx* c);
 Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes);
 Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
-// The call under way leaves work in a plan's buffers (kept per thread, like the scratch arena): see CallScope.
-void ctx_mark_queued(Ctx* c);
+// The call under way uses a plan's buffers (kept per thread, like the scratch arena): waits for another stream's use of them, see LastUse.
+void ctx_uses_plans(Ctx* c);
 void count_launch(int n = 1);
 int sm_count(int device);  // multiprocessors of a device
 uint64_t launch_count();

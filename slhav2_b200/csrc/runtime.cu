@@ -43,8 +43,8 @@ struct Block {
     size_t cap = 0, off = 0;
 };
 // The small tables that calls upload (ctx_upload): a copy may read its slot until the slot's event, so a slot is written again
-// only after that.  The calls of a thread that leave work behind run one after another (see work_done below), so one wait for the
-// newest event of half the ring covers the half; a wait for an event that is long over still costs 1.4 us.  Short tables lie
+// only after that.  One wait per stream, for its newest event in half the ring, covers the half; a wait for an event that is long
+// over still costs 1.4 us.  Short tables lie
 // in ordinary memory, whose copies the driver sends along with its commands (8 KB: 2.0 us against 3.6 us for the copy
 // engine), longer ones in page-locked memory (60 KB: 5.1 us against 2.3 us of the host's time).  Given back when the thread ends.
 constexpr int UPLOAD_SLOTS = 16, UPLOAD_HALF = UPLOAD_SLOTS / 2;
@@ -55,12 +55,22 @@ struct UploadSlot {
     void* p = nullptr;
     size_t cap = 0;
     cudaEvent_t done = nullptr;  // recorded where the call that used the slot ends
+    unsigned long long stream = 0;
     bool pending = false;
     ~UploadSlot() {
         if (pending) cudaEventSynchronize(done);
         if (done) cudaEventDestroy(done);
         if (p) cudaFreeHost(p);
     }
+};
+// Working memory (the scratch arena, the plans' buffers) across streams: a call on a caller-supplied stream may return while its
+// kernels still use it; the event marks the end of that work, and a later call that uses the same memory on ANOTHER stream (by its
+// id: the handle of a destroyed stream may come again) waits for it first.  On the same stream, stream order suffices.  The two are
+// told apart so that a call without a plan (a merge on a second stream) runs beside the scoring of the next step.
+struct LastUse {
+    cudaEvent_t done = nullptr;
+    unsigned long long stream = 0;
+    bool queued = false;
 };
 struct ThreadState {
     int device = 0;
@@ -74,13 +84,8 @@ struct ThreadState {
     UploadSlot upload[16][UPLOAD_SLOTS];
     uint32_t upload_next[16] = {0};
     UploadSlot* upload_used[16] = {nullptr};  // by the call under way
-    // Working memory (the arena, the plans' buffers) across streams: a call on a caller-supplied stream may return while its
-    // kernels still use it; the event marks the end of that work, and every later call on ANOTHER stream (by its id: the
-    // handle of a destroyed stream may come again) waits for it first.  On the same stream, stream order suffices.
-    cudaEvent_t own_event[16] = {nullptr};
-    cudaEvent_t work_done[16] = {nullptr};   // own_event or an upload slot's, whichever the latest call recorded
-    unsigned long long work_stream[16] = {0};
-    bool work_queued[16] = {false};          // the call under way uses a plan
+    LastUse arena[16], plans[16];
+    bool plans_used[16] = {false};            // by the call under way
 };
 thread_local ThreadState tls;
 }  // namespace
@@ -156,6 +161,17 @@ unsigned long long stream_id(cudaStream_t s) {
     if (cudaStreamGetId(s, &id) != cudaSuccess) cudaGetLastError();
     return id;
 }
+// (a stream under capture runs nothing now, a graph may not wait for work outside it, and asking for the stream's id would end the capture)
+void wait_for(const LastUse& u, cudaStream_t s) {
+    if (u.queued && !capturing(s) && stream_id(s) != u.stream) cudaStreamWaitEvent(s, u.done, 0);
+}
+bool mark(LastUse& u, cudaStream_t s, unsigned long long id) {
+    if (!u.done && cudaEventCreateWithFlags(&u.done, cudaEventDisableTiming) != cudaSuccess) return false;
+    if (cudaEventRecord(u.done, s) != cudaSuccess) return false;
+    u.stream = id;
+    u.queued = true;
+    return true;
+}
 }  // namespace
 
 Status ctx_no_capture(Ctx* c) {
@@ -178,17 +194,18 @@ Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
     }
     if (UploadSlot* before = tls.upload_used[c->device]) {  // a second table of the same call
         SLHA_CUDA(cudaEventRecord(before->done, c->stream));
+        before->stream = stream_id(c->stream);
         before->pending = true;
     }
     const uint32_t at = tls.upload_next[c->device]++ % UPLOAD_SLOTS;
     UploadSlot* const ring = tls.upload[c->device];
     if (at % UPLOAD_HALF == 0) {
-        for (int i = UPLOAD_HALF - 1; i >= 0; --i)
-            if (ring[at + i].pending) {
-                SLHA_CUDA(cudaEventSynchronize(ring[at + i].done));
-                break;
-            }
-        for (int i = 0; i < UPLOAD_HALF; ++i) ring[at + i].pending = false;
+        for (int i = UPLOAD_HALF - 1; i >= 0; --i) {
+            if (!ring[at + i].pending) continue;
+            SLHA_CUDA(cudaEventSynchronize(ring[at + i].done));
+            for (int j = i; j >= 0; --j)
+                if (ring[at + j].stream == ring[at + i].stream) ring[at + j].pending = false;
+        }
     }
     UploadSlot& s = ring[at];
     const bool brief = bytes <= UPLOAD_SHORT;
@@ -208,17 +225,18 @@ Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
     tls.upload_used[c->device] = &s;  // (its event is recorded at the call's end)
     return Status();
 }
-void ctx_mark_queued(Ctx* c) { tls.work_queued[c->device] = true; }
+void ctx_uses_plans(Ctx* c) {
+    wait_for(tls.plans[c->device], c->stream);
+    tls.plans_used[c->device] = true;
+}
 
 CallScope::CallScope() {
     st = get_ctx(&c);
     if (!st.ok()) return;
     auto& blocks = tls.blocks[c->device];
     tls.upload_used[c->device] = nullptr;
-    tls.work_queued[c->device] = false;
-    // (a stream under capture runs nothing now, a graph may not wait for work outside it, and asking for the stream's id would end the capture)
-    if (tls.work_done[c->device] && !capturing(c->stream) && stream_id(c->stream) != tls.work_stream[c->device])
-        cudaStreamWaitEvent(c->stream, tls.work_done[c->device], 0);
+    tls.plans_used[c->device] = false;
+    wait_for(tls.arena[c->device], c->stream);
     // the previous call has returned, so its staging memory may be reused; when
     // the arena had to chain blocks, replace them by one block of the total size
     if (blocks.size() > 1) {
@@ -240,18 +258,23 @@ CallScope::~CallScope() {
     if (!c) return;
     UploadSlot* up = tls.upload_used[c->device];
     if (c->own_stream && !up) return;  // library stream: the call drained it before returning
-    bool used = up != nullptr || tls.work_queued[c->device];
-    for (const Block& b : tls.blocks[c->device]) used |= b.off != 0;
-    if (!used || capturing(c->stream)) return;
-    cudaEvent_t& ev = up ? up->done : tls.own_event[c->device];
-    if ((!ev && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) || cudaEventRecord(ev, c->stream) != cudaSuccess) {
+    bool arena = false;
+    for (const Block& b : tls.blocks[c->device]) arena |= b.off != 0;
+    const bool plans = tls.plans_used[c->device];
+    if ((!up && !arena && !plans) || capturing(c->stream)) return;
+    const unsigned long long id = stream_id(c->stream);
+    bool ok = true;
+    if (up) {
+        ok = cudaEventRecord(up->done, c->stream) == cudaSuccess;
+        up->stream = id;
+        up->pending = ok;
+    }
+    if (arena) ok &= mark(tls.arena[c->device], c->stream, id);
+    if (plans) ok &= mark(tls.plans[c->device], c->stream, id);
+    if (!ok) {
         cudaGetLastError();
         cudaStreamSynchronize(c->stream);  // no event to be had: drain instead
-        return;
     }
-    if (up) up->pending = true;
-    tls.work_done[c->device] = ev;
-    tls.work_stream[c->device] = stream_id(c->stream);
 }
 
 bool is_device_ptr(const void* p) {

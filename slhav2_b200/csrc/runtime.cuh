@@ -12,8 +12,8 @@ namespace slha {
 // Resets the calling thread's scratch arena when constructed; the C ABI creates
 // one per entry point so that staging buffers live exactly as long as the call.
 // On a caller-supplied stream the call may return with its kernels still queued: the destructor
-// then records an event, and scopes on a different stream wait for it before they use the thread's
-// working memory.
+// then records events, and calls on a different stream wait for them before they use the same
+// working memory of the thread.
 struct CallScope {
     Ctx* c = nullptr;
     Status st;

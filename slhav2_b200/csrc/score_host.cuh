@@ -790,7 +790,7 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     // (4096 winners per row is what the generic kernel's block-wide selection state holds in shared memory beside its
     // tile ring; the plan builder checks the exact figure)
     if (k == 0 || k > 4096) return Status(SLHA_ERR_DIMENSION, "top-k: k must be in 1..4096");
-    ctx_mark_queued(c);
+    ctx_uses_plans(c);
     Plan* p = nullptr;
     SLHA_TRY(build_plan(c, tiles, segs, n_segs, nq, k, codec_hint, /*allow_wide=*/state == nullptr, &p));
     g_last_plan = p;

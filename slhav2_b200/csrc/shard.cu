@@ -387,7 +387,7 @@ Status shard_step_device(Ctx* c, Shard* s, const SciRustSlhaTile* tiles, const S
                          const float* d_qc, const uint64_t* d_qs, size_t nq, uint32_t k, uint32_t* d_out_index,
                          float* d_out_score) {
     if (s->device != c->device) return Status(SLHA_ERR_DEVICE, "shard handle lives on another device than the calling thread's");
-    ctx_mark_queued(c);  // (a captured step uses a plan's buffers too)
+    ctx_uses_plans(c);  // (a captured step uses a plan's buffers too)
     if (s->world > 1) {
         const size_t block = 2 * nq * (size_t)k;
         // (every rank makes the same calls with the same shapes, so all take the same branch here)

@@ -191,3 +191,32 @@ def test_a_new_plan_is_not_made_under_capture():
         idx = out[0].download(np.uint32, 58).reshape(2, 29)
     want = pool.score_topk(qc, qs, 2, 29)
     assert np.array_equal(idx, want[0])
+
+
+def test_a_merge_on_a_second_stream_runs_beside_the_scoring_on_the_first():
+    # a pipelined step: the merge uses no plan and no scratch, so it may not wait for score calls queued before it
+    n, nq, k = 1 << 22, 4, 64
+    tiles = S.to_device(np.tile(H.random_tiles(4096, 1, seed=780), n // 4096))
+    jobs = [Job(tiles, n, nq, k, 781 + i) for i in range(2)]
+    for j in jobs:
+        j.run()
+    S.synchronize()
+    lists = 2
+    cand_i = S.to_device(np.concatenate([j.result()[0] for j in jobs]))
+    cand_s = S.to_device(np.concatenate([j.result()[1] for j in jobs]))
+    out = S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * k * 4)
+    S.topk_merge(cand_i, cand_s, lists, nq, k, k, *out)
+    S.synchronize()
+    want = out[0].download(np.uint32, nq * k), out[1].download(F, nq * k)
+    with Streams(2) as st:
+        for _ in range(3):
+            S.set_stream(st.all[0].value)
+            for _ in range(200):  # some 25 ms
+                jobs[0].run()
+            S.set_stream(st.all[1].value)
+            S.topk_merge(cand_i, cand_s, lists, nq, k, k, *out)
+            assert st.rt.cudaStreamSynchronize(st.all[1]) == 0
+            assert st.rt.cudaStreamQuery(st.all[0]) == 600  # cudaErrorNotReady: the scoring still runs
+            st.rt.cudaGetLastError()
+            assert st.rt.cudaStreamSynchronize(st.all[0]) == 0
+            assert np.array_equal(out[0].download(np.uint32, nq * k), want[0]) and np.array_equal(out[1].download(F, nq * k), want[1])
