@@ -5,7 +5,7 @@
 // The k (index, score) pairs stay in HBM; what crosses PCIe afterwards is one d_v-vector per query
 // row instead of k pairs.
 //
-// One query row is shared by the ATT_SPLIT CTAs of a cluster, each taking an equal run of the winners the row has.  Every CTA
+// One query row is shared by the SPLIT CTAs of a cluster (eight or fewer, see launch_attend_topk), each taking an equal run of the winners the row has.  Every CTA
 // finds the row's maximum itself (k scores, a few KB from the L2) and weighs its own run; the normalisers and the
 // partial sums of the value rows meet in distributed shared memory, added in a fixed order, so a call is one launch and
 // writes nothing but its results.  Bound: the gather of k value rows per query row (HBM); a thread keeps twelve 16-byte
@@ -22,7 +22,6 @@ namespace slha {
 namespace {
 
 constexpr int ATT_THREADS = 256;
-constexpr int ATT_SPLIT = 8;   // CTAs per row = cluster size (the portable maximum)
 constexpr int ATT_FLIGHT = 12; // value loads a thread issues before it uses the first
 
 // VEC columns of a value row (4 or 16 bytes; one element of a float32 or bfloat16 row), loaded when `p` holds, else zero.
@@ -67,8 +66,8 @@ __device__ __forceinline__ float block_reduce(float v, float* sh, bool is_max) {
 }
 
 // weights_out (optional): [nq][k] softmax weights (0 for absent entries).  VEC 1 takes any alignment, stride and d_v.
-template <typename T, int VEC>
-__global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
+template <typename T, int VEC, int SPLIT>
+__global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
     attend_kernel(const uint32_t* top_index, const float* top_score, const uint32_t* top_count, uint32_t k, float scale, const T* values,
                   size_t d_v, size_t row_stride, const uint64_t* row_base, float* out, float* weights_out) {
     namespace cg = cooperative_groups;
@@ -84,9 +83,9 @@ __global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
     for (uint32_t i = tid; i < n; i += ATT_THREADS)
         if (ix[i] != 0xFFFFFFFFu) mx = fmaxf(mx, sc[i] * scale);
     mx = block_reduce(mx, red, true);
-    const uint32_t run = (n + ATT_SPLIT - 1) / ATT_SPLIT, lo = min(n, part * run), len = min(n, lo + run) - lo;  // this CTA's winners
+    const uint32_t run = (n + SPLIT - 1) / SPLIT, lo = min(n, part * run), len = min(n, lo + run) - lo;  // this CTA's winners
     float* w = sm;
-    uint32_t* wi = reinterpret_cast<uint32_t*>(sm + (k + ATT_SPLIT - 1) / ATT_SPLIT);
+    uint32_t* wi = reinterpret_cast<uint32_t*>(sm + (k + SPLIT - 1) / SPLIT);
     float sum = 0.0f;
     for (uint32_t j = tid; j < len; j += ATT_THREADS) {
         const uint32_t i = lo + j, id = ix[i];
@@ -100,7 +99,7 @@ __global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
     if (tid == 0) own_sum = sum;
     cluster.sync();  // (also: this CTA's weights and indices are visible to all its threads)
     float total = 0.0f;
-    for (int r = 0; r < ATT_SPLIT; ++r) total += *cluster.map_shared_rank(&own_sum, r);
+    for (int r = 0; r < SPLIT; ++r) total += *cluster.map_shared_rank(&own_sum, r);
     const float inv = (total > 0.0f && isfinite(total)) ? 1.0f / total : 0.0f;
     if (weights_out)
         for (uint32_t j = tid; j < len; j += ATT_THREADS) weights_out[(size_t)Q * k + lo + j] = w[j] * inv;
@@ -143,24 +142,25 @@ __global__ void __cluster_dims__(ATT_SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
             part_out[c] = t;
         }
         cluster.sync();
-        const uint32_t share = (cols * VEC + ATT_SPLIT - 1) / ATT_SPLIT, c0 = part * share;
+        const uint32_t share = (cols * VEC + SPLIT - 1) / SPLIT, c0 = part * share;
         for (uint32_t c = c0 + tid; c < min(c0 + share, cols * VEC); c += ATT_THREADS) {
             float t = 0.0f;
 #pragma unroll
-            for (int r = 0; r < ATT_SPLIT; ++r) t += cluster.map_shared_rank(part_out, r)[c];
+            for (int r = 0; r < SPLIT; ++r) t += cluster.map_shared_rank(part_out, r)[c];
             out[(size_t)Q * d_v + (size_t)v0 * VEC + c] = t * inv;
         }
         cluster.sync();  // the peers have read this CTA's sums
     }
     if (weights_out && n < k)
-        for (uint32_t i = n + part * ATT_THREADS + tid; i < k; i += ATT_SPLIT * ATT_THREADS) weights_out[(size_t)Q * k + i] = 0.0f;
+        for (uint32_t i = n + part * ATT_THREADS + tid; i < k; i += SPLIT * ATT_THREADS) weights_out[(size_t)Q * k + i] = 0.0f;
 }
 
-template <typename T, int VEC>
+template <typename T, int VEC, int SPLIT>
 Status launch_attend_t(Ctx* c, const uint32_t* d_index, const float* d_score, const uint32_t* d_count, size_t nq, uint32_t k, float scale,
                        const void* d_values, size_t d_v, size_t row_stride, const uint64_t* d_row_base, float* d_out, float* d_weights) {
-    const size_t smem = (size_t)((k + ATT_SPLIT - 1) / ATT_SPLIT) * 8;
-    attend_kernel<T, VEC><<<dim3(ATT_SPLIT, (uint32_t)nq), ATT_THREADS, smem, c->stream>>>(d_index, d_score, d_count, k, scale, (const T*)d_values, d_v,
+    const size_t smem = (size_t)((k + SPLIT - 1) / SPLIT) * 8;
+    if (smem > 16 * 1024) SLHA_CUDA(cudaFuncSetAttribute(attend_kernel<T, VEC, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 8));
+    attend_kernel<T, VEC, SPLIT><<<dim3(SPLIT, (uint32_t)nq), ATT_THREADS, smem, c->stream>>>(d_index, d_score, d_count, k, scale, (const T*)d_values, d_v,
                                                                                          row_stride, d_row_base, d_out, d_weights);
     count_launch();
     SLHA_CUDA(cudaGetLastError());
@@ -178,9 +178,16 @@ Status launch_attend_topk(Ctx* c, const uint32_t* d_index, const float* d_score,
     // 16-byte loads where every value row starts and ends on a 16-byte boundary, else one element at a time
     const size_t esz = value_dtype == SLHA_B200_BF16 ? 2 : 4;
     const bool vec = reinterpret_cast<uintptr_t>(d_values) % 16 == 0 && d_v * esz % 16 == 0 && row_stride * esz % 16 == 0;
-#define SLHA_ATTEND(T, V) launch_attend_t<T, V>(c, d_index, d_score, d_count, nq, k, scale, d_values, d_v, row_stride, d_row_base, d_out, d_weights)
+    // CTAs per row: the most that keep the grid within two CTAs an SM.  With eight for every row, calls of many rows ran in waves of CTAs
+    // with little to gather each: 128 bf16 values, 100 rows of 64 winners 22.4 us (now 8.6), of 2048 31.1 (16.7), 256 rows of 64
+    // 43.4 (8.8), of 2048 63.9 (35.1).
+    int split = 8;
+    while (split > 1 && nq * (size_t)split > 2 * (size_t)sm_count(c->device)) split >>= 1;
+#define SLHA_ATTEND_S(T, V, S) launch_attend_t<T, V, S>(c, d_index, d_score, d_count, nq, k, scale, d_values, d_v, row_stride, d_row_base, d_out, d_weights)
+#define SLHA_ATTEND(T, V) (split == 8 ? SLHA_ATTEND_S(T, V, 8) : split == 4 ? SLHA_ATTEND_S(T, V, 4) : split == 2 ? SLHA_ATTEND_S(T, V, 2) : SLHA_ATTEND_S(T, V, 1))
     if (value_dtype == SLHA_B200_BF16) return vec ? SLHA_ATTEND(__nv_bfloat16, 8) : SLHA_ATTEND(__nv_bfloat16, 1);
     return vec ? SLHA_ATTEND(float, 4) : SLHA_ATTEND(float, 1);
+#undef SLHA_ATTEND_S
 #undef SLHA_ATTEND
 }
 

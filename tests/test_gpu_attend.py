@@ -108,3 +108,19 @@ def test_attend_rows_that_have_fewer_winners_than_k(k, bf16):
     assert close(w_out, want_w) and close(out, want)
     for j in range(nq):
         assert np.all(w_out[j, min(counts[j], k):] == 0)
+
+
+@pytest.mark.parametrize("nq,k", [(1, 8192), (36, 33), (38, 100), (75, 64), (150, 16), (300, 300), (700, 1), (320, 4096)])
+def test_attend_of_many_rows_takes_smaller_clusters(nq, k):
+    # eight, four, two and one CTA per row; a CTA alone holds all of a row's weights
+    n, d_v = 9000, 96
+    rng = np.random.default_rng(nq)
+    values = rng.standard_normal((n, d_v)).astype(F)
+    idx = np.stack([rng.permutation(n)[:k] for _ in range(nq)]).astype(np.uint32)
+    sc = (10.0 * rng.standard_normal((nq, k))).astype(F)
+    counts = rng.integers(0, k + 1, nq).astype(np.uint32)
+    w_out = np.full((nq, k), 7.0, F)
+    out = S.attend_topk(idx, sc, k, 0.1, S.to_device(values), d_v, top_count=counts, weights_out=w_out)
+    some = rng.choice(nq, min(nq, 40), replace=False)
+    want, want_w = ora.attend_topk(idx[some], sc[some], 0.1, values, top_count=counts[some])
+    assert close(w_out[some], want_w) and close(out[some], want)
