@@ -181,8 +181,12 @@ Status launch_attend_topk(Ctx* c, const uint32_t* d_index, const float* d_score,
     // CTAs per row: the most that keep the grid within two CTAs an SM.  With eight for every row, calls of many rows ran in waves of CTAs
     // with little to gather each: 128 bf16 values, 100 rows of 64 winners 22.4 us (now 8.6), of 2048 31.1 (16.7), 256 rows of 64
     // 43.4 (8.8), of 2048 63.9 (35.1).
+    // Three an SM where a row's values are long: from 320 KB rather two CTAs a row than one (150 rows of 2048 winners of 256 bf16 values
+    // 57.8 -> 35.0 us), from 768 KB of float32 also four and eight (75 rows of 2048 x 256 29.0 -> 24.9; bf16 there 22.8 -> 24.9).
+    const size_t long_row = (size_t)k * d_v * esz, sms = (size_t)sm_count(c->device);
+    auto per_sm = [&](int ctas) { return (ctas == 2 ? long_row >= (320u << 10) : esz == 4 && long_row >= (768u << 10)) ? 3u : 2u; };
     int split = 8;
-    while (split > 1 && nq * (size_t)split > 2 * (size_t)sm_count(c->device)) split >>= 1;
+    while (split > 1 && nq * (size_t)split > per_sm(split) * sms) split >>= 1;
 #define SLHA_ATTEND_S(T, V, S) launch_attend_t<T, V, S>(c, d_index, d_score, d_count, nq, k, scale, d_values, d_v, row_stride, d_row_base, d_out, d_weights)
 #define SLHA_ATTEND(T, V) (split == 8 ? SLHA_ATTEND_S(T, V, 8) : split == 4 ? SLHA_ATTEND_S(T, V, 4) : split == 2 ? SLHA_ATTEND_S(T, V, 2) : SLHA_ATTEND_S(T, V, 1))
     if (value_dtype == SLHA_B200_BF16) return vec ? SLHA_ATTEND(__nv_bfloat16, 8) : SLHA_ATTEND(__nv_bfloat16, 1);
