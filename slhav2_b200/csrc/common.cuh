@@ -93,12 +93,15 @@ struct Model {
     size_t d = 0, d_pad = 0;
     bool rht = false;
     int device = 0;
+    void* block = nullptr;     // the arrays below
     float* d_p = nullptr;      // 128 x d   projection rows
     float* d_pt = nullptr;     // d x 128   transposed copy (coalesced column access)
     float* d_scale = nullptr;  // 128
     float* d_z = nullptr;      // 256 x d_pad
     float* d_zt = nullptr;     // d_pad x 256 transposed copy
     float* d_diag = nullptr;   // d_pad (+-1) or null
+    uint4* d_zf = nullptr;     // z in fp16 as m16n8k16 B fragments [d_pad / 32][32 hyperplane groups of 8][32 lanes], or null
+    float z_guard = 0.0f, z_norm = 0.0f;  // see signs_mma
 };
 
 // ---- kernels' host launchers (score.cu / encode.cu / pool.cu) -------------

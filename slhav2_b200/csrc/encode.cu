@@ -13,22 +13,27 @@
 // __fmul_rn / __fadd_rn (never contracted into FMA), divisions are __fdiv_rn and
 // square roots __fsqrt_rn.  Parallelism comes from rows x keys, not from
 // splitting a sum, so the tile bytes equal the scalar reference's bit for bit.
+#include <cuda_fp16.h>
+
 #include "common.cuh"
 
 namespace slha {
 namespace {
 
-constexpr int ENC_THREADS = 256;
+constexpr int enc_threads(int kb) { return kb == 32 ? 128 : 256; }  // threads of a CTA that takes kb keys at a time
 
 struct EncodeArgs {
     const void* keys;        // [n][d] f32 or bf16
     int key_dtype;
     uint64_t n;
-    uint32_t d, d_pad, log2_pad;
+    uint32_t d, d_pad;
     const float* p;          // [128][d]
     const float* pt;         // [d][128]
     const float* scale;      // [128]
     const float* zt;         // [d_pad][256]
+    const float* z;          // [256][d_pad]
+    const uint4* zf;         // fp16 B fragments of z, rows at one norm (model_build), or null: every sign from its exact sum
+    float z_guard, z_norm;   // a sum further from zero than z_guard |e| + z_norm |e - e'| has the exact sum's sign (see signs_mma)
     const float* diag;       // [d_pad] or null
     float fwht_inv;          // 1/sqrt(d_pad), rounded as the reference rounds it
     float lambda_c;          // sqrt(pi/512) in f32
@@ -45,13 +50,7 @@ struct EncodeArgs {
 };
 
 __device__ __forceinline__ float rnd_half_away(float x) { return roundf(x); }
-__device__ __forceinline__ int sat_i32(float x) {
-    // Rust `x as i32`: NaN -> 0, saturating
-    if (x != x) return 0;
-    if (x >= 2147483648.0f) return 2147483647;
-    if (x <= -2147483648.0f) return (-2147483647 - 1);
-    return (int)x;
-}
+__device__ __forceinline__ int sat_i32(float x) { return __float2int_rz(x); }  // Rust `x as i32`: NaN -> 0, saturating, like cvt.rzi.s32.f32
 __device__ __forceinline__ int clampi(int v, int lo, int hi) { return min(max(v, lo), hi); }
 __device__ __forceinline__ uint32_t scale_byte(float step, float global) {
     // `(step / global * 255.0).round().clamp(1.0, 255.0) as u8`  (int4.rs:48-49)
@@ -59,156 +58,144 @@ __device__ __forceinline__ uint32_t scale_byte(float step, float global) {
     if (r != r) return 0;
     return (uint32_t)fminf(fmaxf(r, 1.0f), 255.0f);
 }
-__device__ __forceinline__ uint32_t int4_nibble(float v, float step) {
-    return (uint32_t)(clampi(sat_i32(rnd_half_away(__fdiv_rn(v, step))), -8, 7) + 8) & 15u;
+// `gap`: lowered to the distance of t from the nearest float between two entries.
+__device__ __forceinline__ uint32_t nf4_nearest(float t, float& gap) {
+    // nf4.rs:7-18: linear scan over the codebook by rounded distance, first minimum wins.  Entry i + 1 beats entry i from a certain float on
+    // (rounded differences are monotone in t), so four comparisons with those floats find the entry; each is the smallest t in
+    // [-1, 1] with |fl(t - c[i+1])| < |fl(t - c[i])|.  (A difference of two floats is negative exactly where the first is smaller.)
+    constexpr uint32_t from[15] = {0xBF5A8F5Bu, 0xBF1FF2E4u, 0xBEF566CFu, 0xBEBA3054u, 0xBE86CF41u, 0xBE2F9DB2u, 0xBDAD5CFBu, 0x31000000u,
+                                   0x3DAD5CFCu, 0x3E2F9DB3u, 0x3E86CF42u, 0x3EBA3056u, 0x3EF566D0u, 0x3F1FF2E5u, 0x3F5A8F5Du};
+    const auto f = [&](int i) { return __uint_as_float(from[i]); };
+    const float d3 = __fsub_rn(t, f(7));
+    const bool b3 = d3 >= 0.0f;
+    const float d2 = __fsub_rn(t, b3 ? f(11) : f(3));
+    const bool b2 = d2 >= 0.0f;
+    const float d1 = __fsub_rn(t, b3 ? (b2 ? f(13) : f(9)) : (b2 ? f(5) : f(1)));
+    const bool b1 = d1 >= 0.0f;
+    const float lo = b2 ? (b1 ? f(6) : f(4)) : (b1 ? f(2) : f(0)), hi = b2 ? (b1 ? f(14) : f(12)) : (b1 ? f(10) : f(8));
+    const float d0 = __fsub_rn(t, b3 ? hi : lo);
+    const bool b0 = d0 >= 0.0f;
+    gap = fminf(fminf(gap, fminf(fabsf(d3), fabsf(d2))), fminf(fabsf(d1), fabsf(d0)));
+    return (b3 ? 8u : 0u) | (b2 ? 4u : 0u) | (b1 ? 2u : 0u) | (b0 ? 1u : 0u);
 }
-__device__ __forceinline__ uint32_t nf4_nearest(float t) {
-    // nf4.rs:7-18: linear scan, first minimum wins
-    const float cb[16] = {-1.0f,   -0.7075f, -0.5421f, -0.4165f, -0.3108f, -0.2158f,
-                          -0.1272f, -0.0421f, 0.0421f,  0.1272f,  0.2158f,  0.3108f,
-                          0.4165f,  0.5421f,  0.7075f,  1.0f};
-    uint32_t best = 0;
-    float best_d = INFINITY;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        const float dd = fabsf(__fsub_rn(t, cb[i]));
-        if (dd < best_d) { best_d = dd; best = i; }
-    }
-    return best;
-}
-__device__ __forceinline__ float quad_max(float v) {  // max over the 4 lanes sharing lane>>2
+// Rows of h in shared memory hold their 16-byte chunks in an order in which eight lanes that each read the same chunk of their own 16 dimensions
+// meet all banks.
+__device__ __forceinline__ int h_chunk(int c) { return (c & ~3) | ((c & 3) ^ (c >> 3)); }
+__device__ __forceinline__ float octet_max(float v) {  // max over the 8 lanes sharing lane >> 3
     v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 1));
-    return fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 2));
-}
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
-    return v;
+    v = fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 2));
+    return fmaxf(v, __shfl_xor_sync(0xFFFFFFFFu, v, 4));
 }
 
-// Quantise one 128-float latent held as 4 consecutive dims per lane into the
-// 64 latent bytes + scale + 8 scale bytes of a tile in shared memory.
-// One warp per key.  `tile` points at 128 zeroed bytes.
-__device__ void quantize_warp(const float* h, int codec, unsigned char* tile, int lane) {
-    float v[4];
+// Code of a value from its quotient q by the unit's step: a nibble, an 8-bit head level, or a 3-bit code (corr: its correction bit).  False where q
+// may lie on the other side of the next place at which the code changes than a quotient up to 2^-22 (relative) away: halves of
+// integers, for 3-bit codes all multiples of a half (a sum with 3.5 is rounded on the way: 2^-21 more), NF4: the floats between two entries.
+enum { Q_INT4, Q_NF4, Q_HEAD, Q_CODE3 };
+template <int MODE>
+__device__ __forceinline__ bool code_of(float q, uint32_t& code, uint32_t& corr) {
+    corr = 0u;
+    if (MODE == Q_NF4) {
+        float gap = 1.0f;
+        code = nf4_nearest(fminf(fmaxf(q, -1.0f), 1.0f), gap);
+        return gap > 5e-7f && fabsf(q) < 1e30f;
+    }
+    if (MODE == Q_CODE3) {
+        code = (uint32_t)clampi(sat_i32(rnd_half_away(__fadd_rn(q, 3.5f))), 0, 7);
+        corr = __fsub_rn(q, __fsub_rn((float)code, 3.5f)) > 0.0f ? 1u : 0u;
+        const float h = __fadd_rn(q, q);
+        return fabsf(__fsub_rn(h, rintf(h))) > 8e-6f && fabsf(q) < 8.0f;
+    }
+    constexpr int lo = MODE == Q_HEAD ? -128 : -8, hi = MODE == Q_HEAD ? 127 : 7;
+    code = (uint32_t)(clampi(sat_i32(rnd_half_away(q)), lo, hi) - lo);
+    return fabsf(__fsub_rn(q, rintf(q))) < 0.5f - (MODE == Q_HEAD ? 6e-5f : 4e-6f) && fabsf(q) < 1.5f * hi;
+}
+// The codes of a unit's values v (nibbles, head levels, or 3-bit codes two times eight with their correction bits).  Every decision is taken on the
+// rounded quotient v / eff; v * (1 / eff) is within 2^-22 of it (half an ulp each for the reciprocal, the product and the quotient), so only
+// the values for which that is not enough are divided -- one in 10^5, and the largest of a key's 3-bit codes.  A division is a branch of its
+// own to the compiler: sixteen of them in a row, one after the other, took a fifth of the kernel.
+template <int MODE>
+__device__ __forceinline__ void quantize_values(const float (&v)[16], const float* h, int first, float eff, uint32_t (&w)[2], uint32_t& corr) {
+    constexpr int N = MODE == Q_HEAD ? 8 : 16, BITS = MODE == Q_HEAD ? 8 : (MODE == Q_CODE3 ? 3 : 4), PER = N / 2;
+    const bool usual = eff >= 8.6736174e-19f && eff <= 1.1529215e18f;  // 2^-60 .. 2^60
+    const float inv = __fdiv_rn(1.0f, eff);
+    uint32_t again = 0, code, c;
+    w[0] = w[1] = corr = 0u;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) v[j] = h[4 * lane + j];
-    uint32_t* tw = reinterpret_cast<uint32_t*>(tile);
-    const float amax4 = fmaxf(fmaxf(fabsf(v[0]), fabsf(v[1])), fmaxf(fabsf(v[2]), fabsf(v[3])));
+    for (int i = 0; i < N; ++i) {
+        const bool sure = code_of<MODE>(__fmul_rn(v[i], inv), code, c);
+        w[i / PER] |= code << (BITS * (i % PER));
+        corr |= c << i;
+        again |= sure ? 0u : 1u << i;
+    }
+    if (!usual) again = (1u << N) - 1u;
+    while (again) {
+        const int i = __ffs(again) - 1, dim = first + i;
+        again &= again - 1u;
+        const float x = h[4 * h_chunk(dim >> 2) + (dim & 3)];
+        code_of<MODE>(MODE != Q_NF4 || eff > 0.0f ? __fdiv_rn(x, eff) : 0.0f, code, c);
+        const uint32_t at = BITS * (i % PER), keep = ~(((1u << BITS) - 1u) << at);
+        if (i < PER) w[0] = (w[0] & keep) | code << at;
+        else w[1] = (w[1] & keep) | code << at;
+        corr = (corr & ~(1u << i)) | c << i;
+    }
+}
+
+// Quantise one latent into the 64 latent bytes + scale + 8 scale bytes of a tile in shared memory: eight lanes per key, lane u has scale
+// unit u -- 16 dimensions from 16 u on, or for the head + body codecs (mixed.rs:15-33, mix3.rs:13-31) dimensions 0..7 (u = 0) and 16
+// from 16 u - 8 on, the last eight dropped.  A lane finds its step and its scale byte for itself, the key's scale takes three shuffles,
+// and the lane's bytes lie together in the tile.  All lanes of the warp call; on: the lane has a key.
+__device__ __forceinline__ void quantize_unit(const float* h, int codec, unsigned char* tile, int u, bool on) {
+    const bool headbody = codec == SLHA_CODEC_MIXED || codec == SLHA_CODEC_MIX3, head = headbody && u == 0;
+    float v[16];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        const int at = h_chunk(headbody ? (u ? 4 * u - 2 + c : (c & 1)) : 4 * u + c);
+        const float4 x = reinterpret_cast<const float4*>(h)[at];
+        const bool in = !head || c < 2;
+        v[4 * c] = in ? x.x : 0.0f;
+        v[4 * c + 1] = in ? x.y : 0.0f;
+        v[4 * c + 2] = in ? x.z : 0.0f;
+        v[4 * c + 3] = in ? x.w : 0.0f;
+    }
+    float mx = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) mx = fmaxf(mx, fabsf(v[i]));
     float global;
-    uint32_t gsb;  // this lane's scale byte
-    const bool headbody = codec == SLHA_CODEC_MIXED || codec == SLHA_CODEC_MIX3;
-    int unit;      // scale-byte index of this lane's dims
+    uint32_t gsb = 255;
     if (codec == SLHA_CODEC_INT4_SINGLE) {  // int4.rs:9-24
-        const float mx = warp_max(amax4);
+        mx = octet_max(mx);
         global = mx > 0.0f ? __fdiv_rn(mx, 7.0f) : 1.0f;
-        gsb = 255;
-        unit = lane >> 2;
-    } else if (!headbody) {
-        // grouped codecs: step = absmax / {7, 1, 3.5}; int4.rs:34-63, nf4.rs:23-57, tq3.rs:10-49
-        float mx = quad_max(amax4);
-        if (codec == SLHA_B200_CODEC_INT4_GROUPED32) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 4));
-        const float div = codec == SLHA_CODEC_NF4 ? 1.0f : (codec == SLHA_CODEC_TQ3 ? 3.5f : 7.0f);
+    } else {
+        // step = absmax / {7, 1, 3.5} (int4.rs:34-63, nf4.rs:23-57, tq3.rs:10-49), of the 8-bit head absmax / 127
+        if (codec == SLHA_B200_CODEC_INT4_GROUPED32) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1));
+        const float div = head ? 127.0f : (codec == SLHA_CODEC_TQ3 || codec == SLHA_CODEC_MIX3 ? 3.5f : 7.0f);
         const float step = codec == SLHA_CODEC_NF4 ? mx : __fdiv_rn(mx, div);
-        const float g = warp_max(step);
+        const float g = octet_max(step);
         global = g > 0.0f ? g : 1.0f;
         gsb = scale_byte(step, global);
-        unit = lane >> 2;
-    } else {
-        // head (dims 0..7 = lanes 0,1) + 7 body groups of 16 dims starting at dim 8
-        // (mixed.rs:15-33, mix3.rs:13-31): body group of dim D is (D-8)/16, i.e.
-        // unit u >= 1 spans lanes 4u-2 .. 4u+1; lanes 30,31 hold the dropped tail.
-        const int d0 = 4 * lane;
-        unit = lane < 2 ? 0 : (d0 < 120 ? 1 + (d0 - 8) / 16 : 8);
-        const int first = lane < 2 ? 0 : (unit < 8 ? 4 * unit - 2 : lane);
-        const int span = lane < 2 ? 2 : (unit < 8 ? 4 : 1);
-        float mx = 0.0f;
-#pragma unroll
-        for (int l = 0; l < 4; ++l) {
-            const float o = __shfl_sync(0xFFFFFFFFu, amax4, min(first + l, 31));
-            if (l < span) mx = fmaxf(mx, o);
-        }
-        const float step = lane < 2 ? __fdiv_rn(mx, 127.0f)
-                                    : __fdiv_rn(mx, codec == SLHA_CODEC_MIXED ? 7.0f : 3.5f);
-        const float g = warp_max(unit < 8 ? step : 0.0f);
-        global = g > 0.0f ? g : 1.0f;
-        gsb = unit < 8 ? scale_byte(step, global) : 0;
     }
-    // publish scale bytes: the first lane of every unit writes its byte
-    if (codec == SLHA_CODEC_INT4_SINGLE) {
-        if (lane < 8) tile[120 + lane] = 255;
-    } else if (!headbody) {
-        if ((lane & 3) == 0) tile[120 + unit] = (unsigned char)gsb;
+    const float eff = codec == SLHA_CODEC_INT4_SINGLE ? global : __fmul_rn(global, __fdiv_rn((float)gsb, 255.0f));
+    if (!on) return;
+    tile[120 + u] = (unsigned char)gsb;
+    if (u == 0) *reinterpret_cast<float*>(tile + 96) = global;
+    const int first = headbody && !head ? 16 * u - 8 : 16 * u;
+    uint32_t w[2], corr;
+    if (head) {
+        quantize_values<Q_HEAD>(v, h, first, eff, w, corr);
+        *reinterpret_cast<uint2*>(tile) = make_uint2(w[0], w[1]);
+    } else if (codec == SLHA_CODEC_TQ3 || codec == SLHA_CODEC_MIX3) {
+        quantize_values<Q_CODE3>(v, h, first, eff, w, corr);
+        // code plane: 6 bytes per unit from byte 0 (TQ3) or 8 (MIX3, whose unit 0 is the head); correction plane behind it
+        const int cu = headbody ? u - 1 : u;
+        uint16_t* cp = reinterpret_cast<uint16_t*>(tile + (headbody ? 8 : 0) + 6 * cu);
+        cp[0] = (uint16_t)w[0];
+        cp[1] = (uint16_t)(w[0] >> 16 | w[1] << 8);
+        cp[2] = (uint16_t)(w[1] >> 8);
+        *reinterpret_cast<uint16_t*>(tile + (headbody ? 50 : 48) + 2 * cu) = (uint16_t)corr;
     } else {
-        if (lane == 0 || (lane >= 2 && lane < 30 && ((lane - 2) & 3) == 0)) tile[120 + unit] = (unsigned char)gsb;
-    }
-    if (lane == 0) *reinterpret_cast<float*>(tile + 96) = global;
-    const float eff = __fmul_rn(global, __fdiv_rn((float)gsb, 255.0f));
-
-    if (codec == SLHA_CODEC_INT4_SINGLE || codec == SLHA_CODEC_INT4_GROUPED ||
-        codec == SLHA_B200_CODEC_INT4_GROUPED32 || codec == SLHA_CODEC_NF4) {
-        uint32_t nib[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            if (codec == SLHA_CODEC_INT4_SINGLE) {
-                nib[j] = int4_nibble(v[j], global);
-            } else if (codec == SLHA_CODEC_NF4) {
-                float tt = 0.0f;
-                if (eff > 0.0f) tt = fminf(fmaxf(__fdiv_rn(v[j], eff), -1.0f), 1.0f);
-                nib[j] = nf4_nearest(tt);
-            } else {
-                nib[j] = int4_nibble(v[j], eff);
-            }
-        }
-        reinterpret_cast<uint16_t*>(tile)[lane] =
-            (uint16_t)(nib[0] | (nib[1] << 4) | (nib[2] << 8) | (nib[3] << 12));
-    } else if (codec == SLHA_CODEC_TQ3) {
-        uint32_t codes = 0, corr = 0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float tt = __fdiv_rn(v[j], eff);
-            const int code = clampi(sat_i32(rnd_half_away(__fadd_rn(tt, 3.5f))), 0, 7);
-            codes |= (uint32_t)code << (3 * j);
-            if (__fsub_rn(tt, __fsub_rn((float)code, 3.5f)) > 0.0f) corr |= 1u << j;
-        }
-        const int bit = 12 * lane;  // 4 dims x 3 bits
-        atomicOr(&tw[bit >> 5], codes << (bit & 31));
-        if ((bit & 31) > 20) atomicOr(&tw[(bit >> 5) + 1], codes >> (32 - (bit & 31)));
-        atomicOr(&tw[12 + (lane >> 3)], corr << (4 * (lane & 7)));
-    } else {
-        // head+body
-        const int d0 = 4 * lane;
-        if (lane < 2) {
-            uint32_t w = 0;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int q = clampi(sat_i32(rnd_half_away(__fdiv_rn(v[j], eff))), -128, 127) + 128;
-                w |= (uint32_t)q << (8 * j);
-            }
-            tw[lane] = w;
-        } else if (d0 < 120) {
-            const int ld0 = d0 - 8;
-            if (codec == SLHA_CODEC_MIXED) {
-                uint32_t nibs = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) nibs |= int4_nibble(v[j], eff) << (4 * j);
-                reinterpret_cast<uint16_t*>(tile)[4 + (ld0 >> 2)] = (uint16_t)nibs;
-            } else {
-                uint32_t codes = 0, corr = 0;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float tt = __fdiv_rn(v[j], eff);
-                    const int code = clampi(sat_i32(rnd_half_away(__fadd_rn(tt, 3.5f))), 0, 7);
-                    codes |= (uint32_t)code << (3 * j);
-                    if (__fsub_rn(tt, __fsub_rn((float)code, 3.5f)) > 0.0f) corr |= 1u << j;
-                }
-                const int bit = 64 + 3 * ld0;  // code plane starts at byte 8
-                atomicOr(&tw[bit >> 5], codes << (bit & 31));
-                if ((bit & 31) > 20) atomicOr(&tw[(bit >> 5) + 1], codes >> (32 - (bit & 31)));
-                const int cbit = 400 + ld0;    // correction plane starts at byte 50
-                atomicOr(&tw[cbit >> 5], corr << (cbit & 31));
-            }
-        }
+        if (codec == SLHA_CODEC_NF4) quantize_values<Q_NF4>(v, h, first, eff, w, corr);
+        else quantize_values<Q_INT4>(v, h, first, eff, w, corr);
+        *reinterpret_cast<uint2*>(tile + 8 * u) = make_uint2(w[0], w[1]);
     }
 }
 
@@ -315,56 +302,364 @@ __device__ __forceinline__ void unpack_tile(const uint64_t (&acc)[R][K / 2], flo
         for (int j = 0; j < K / 2; ++j) unpack2(acc[r][j], out[r][2 * j], out[r][2 * j + 1]);
 }
 
+// floats between the rows of the transposed [..][KB] arrays in shared memory
+__host__ __device__ constexpr int enc_row_stride(int kb) { return kb >= 8 ? kb + 4 : kb; }
+
+// ---- sign bits on the tensor cores ---------------------------------------------------------------------------------------
+// A tile stores only the signs of the 256 projections Z e, and e is exact (in the reference's order) before they are taken.  So the
+// sums run as m16n8k16 MMAs over fp16 roundings of Z (its rows scaled to one norm) and of e (scaled by a power of two), and only a sum
+// closer to zero than its error bound is taken again in the reference's order.  With z' and e' the roundings, n = d_pad terms:
+//   rounding of both factors               |z - z'| |e| + |z'| |e - e'|   (norms, measured: about 2^-12.3 |z| |e| each)
+//   fp32 accumulation in the MMAs          2^-13.9 |z| |e|                (17 addends an MMA, each cut at 2^-22 of the largest, 16 MMAs)
+//   the reference's own sequential sum     2^-16 |z| |e|                  (n + 1 roundings of 2^-24, n <= 256)
+// (model_build gives no fragments for n > 256 or a Z of unusual size).  Gaussian rows of Z leave about 1.1 of 256 signs of a key inside
+// the bound at d = 128, 1.6 at d_pad = 256.
+constexpr int SIGN_LIST = 32;                    // sums of a key that may be taken again before the whole pass is summed exactly
+__host__ __device__ constexpr int sign_stride(int kb) { return kb == 32 ? 40 : (kb == 16 ? 24 : kb); }  // words between pairs of rows: conflict-free fragment loads
+__host__ __device__ constexpr uint32_t sign_rows(uint32_t dp) { return (dp + 31) / 32 * 32; }
+// words of the phase's own shared memory: count | bound [KB] | list | fp16 pairs [rows / 2][stride], later rows of z
+__host__ __device__ constexpr uint32_t sign_fixed(int kb) { return 4u + (uint32_t)kb + (uint32_t)(kb * SIGN_LIST / 2); }
+__host__ __device__ constexpr uint32_t sign_words(uint32_t dp, int kb) {
+    return sign_fixed(kb) + (sign_rows(dp) / 2 * (uint32_t)sign_stride(kb) + 8u > dp + 7u ? sign_rows(dp) / 2 * (uint32_t)sign_stride(kb) + 8u : dp + 7u);
+}
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+template <int N>
+__device__ __forceinline__ void load_words(float (&v)[N], const float* src) {  // N = 8, 4, 2, 1, aligned to min(N, 4) words
+    if (N >= 4) {
+#pragma unroll
+        for (int q = 0; q < N / 4; ++q) {
+            const float4 x = reinterpret_cast<const float4*>(src)[q];
+            v[4 * q] = x.x; v[(4 * q + 1) % N] = x.y; v[(4 * q + 2) % N] = x.z; v[(4 * q + 3) % N] = x.w;
+        }
+    } else if (N == 2) {
+        const float2 x = *reinterpret_cast<const float2*>(src);
+        v[0] = x.x; v[1 % N] = x.y;
+    } else {
+        v[0] = *src;
+    }
+}
+
+// Signs of Z e for the KB columns of buf [dp][KS], into the sign words of the tiles at tl.  All threads of the CTA; buf is complete
+// (a barrier lies between its writers and this call) and the `words` words at `w` are free.  meanwhile: work that only reads buf.  False (for
+// all threads alike): too many sums lie too close to zero, nothing usable was written.
+template <int KB, typename F>
+__device__ __forceinline__ bool signs_mma(const EncodeArgs& a, const float* buf, unsigned char* tl, uint32_t* w, uint32_t words, F&& meanwhile) {
+    constexpr int KS = enc_row_stride(KB), STR = sign_stride(KB), MT = KB == 32 ? 2 : 1, NT = enc_threads(KB), WARPS = NT / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t dp = a.d_pad, rows = sign_rows(dp);
+    uint32_t* cnt = w;
+    float* bound = reinterpret_cast<float*>(cnt + 4);
+    uint16_t* list = reinterpret_cast<uint16_t*>(bound + KB);
+    uint32_t* eh = w + sign_fixed(KB);
+    if (tid == 0) *cnt = 0u;
+    // the first fragments are on their way while the keys are scaled; those of every further two steps follow one turn ahead
+    const uint4* zf = a.zf + (size_t)(4 * warp) * 32 + lane;
+    uint4 ahead[4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n) ahead[n] = __ldg(zf + n * 32);
+    // a warp's keys (KW consecutive columns): largest element, then the scaled fp16 pairs with the norms of what they hold and of what they lost
+    constexpr int KW = KB >= WARPS ? KB / WARPS : 1;
+    if (KW * warp < KB) {
+        const float* col = buf + KW * warp;
+        uint32_t mx[KW];
+        float ss[KW], lost[KW], sc[KW];
+#pragma unroll
+        for (int j = 0; j < KW; ++j) { mx[j] = 0u; ss[j] = lost[j] = 0.0f; }
+#pragma unroll 4
+        for (uint32_t i = lane; i < dp; i += 32) {
+            float x[KW];
+            load_words<KW>(x, col + (size_t)i * KS);
+#pragma unroll
+            for (int j = 0; j < KW; ++j) mx[j] = max(mx[j], __float_as_uint(x[j]) & 0x7FFFFFFFu);
+        }
+#pragma unroll
+        for (int j = 0; j < KW; ++j) {
+            mx[j] = __reduce_max_sync(0xFFFFFFFFu, mx[j]);
+            // 2^p with the largest element in [2^12, 2^13); elements of ordinary size only, so that nothing leaves the normal range
+            // (other keys, infinities and NaN among them, become zeros within an infinite bound: summed exactly)
+            const bool usual = mx[j] >= (67u << 23) && mx[j] < (187u << 23);  // [2^-60, 2^60)
+            sc[j] = usual ? __uint_as_float((266u - (mx[j] >> 23)) << 23) : 0.0f;
+        }
+#pragma unroll 2
+        for (uint32_t r = lane; r < rows / 2; r += 32) {
+            float x[KW] = {}, y[KW] = {};
+            if (2 * r < dp) load_words<KW>(x, col + (size_t)(2 * r) * KS);
+            if (2 * r + 1 < dp) load_words<KW>(y, col + (size_t)(2 * r + 1) * KS);
+            float h[KW];
+#pragma unroll
+            for (int j = 0; j < KW; ++j) {
+                const float u = sc[j] != 0.0f ? x[j] * sc[j] : 0.0f, v = sc[j] != 0.0f ? y[j] * sc[j] : 0.0f;
+                const __half2 p = __floats2half2_rn(u, v);
+                const float2 q = __half22float2(p);
+                ss[j] = fmaf(u, u, fmaf(v, v, ss[j]));
+                lost[j] = fmaf(u - q.x, u - q.x, fmaf(v - q.y, v - q.y, lost[j]));
+                h[j] = *reinterpret_cast<const float*>(&p);
+            }
+            store_keys<KW>(reinterpret_cast<float*>(eh) + r * STR + KW * warp, h);
+        }
+#pragma unroll
+        for (int j = 0; j < KW; ++j) {
+            // sums over the warp in fixed point, rounded up: a lane's eight squares are below 2^29, its lost parts (half an ulp, at most 2) below 2^6
+            const float e2 = 8.0f * (float)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)(ss[j] * 0.125f) + 1u);
+            const float l2 = 9.5367431640625e-7f * (float)__reduce_add_sync(0xFFFFFFFFu, (uint32_t)(lost[j] * 1048576.0f) + 1u);
+            const float lim = a.z_guard * (e2 * rsqrtf(e2)) + a.z_norm * (l2 * rsqrtf(l2));  // (rounding: slack of the two factors)
+            if (lane == j) bound[KW * warp + j] = sc[j] != 0.0f ? lim : (mx[j] == 0u ? -1.0f : INFINITY);  // (an all-zero key has no negative sum)
+        }
+    }
+    __syncthreads();
+    meanwhile();
+    // M = keys (rows of no key give sums nobody reads), N = hyperplanes 32 word .. + 31: one word of every key at a time
+    constexpr int HALVES = KB > 8 ? 2 : 1, WORDS = 8 / WARPS;
+    uint32_t near[WORDS][MT * HALVES], nears = 0;
+    const bool mine = KB >= 8 || g < KB;
+#pragma unroll
+    for (int wd = 0; wd < WORDS; ++wd) {
+        const int word = warp + wd * WARPS;
+        float acc[MT][4][4];
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < 4; ++n)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[m][n][c] = 0.0f;
+#pragma unroll 2
+        for (uint32_t k2 = 0; k2 < rows / 32; ++k2) {
+            uint4 b[4];
+            const bool last = k2 + 1 == rows / 32;
+            const uint4* next = last ? zf + (size_t)(wd + 1) * (4 * WARPS * 32) : zf + (size_t)wd * (4 * WARPS * 32) + (size_t)(k2 + 1) * 1024;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                b[n] = ahead[n];
+                if (!last || wd + 1 < WORDS) ahead[n] = __ldg(next + n * 32);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint32_t* er = eh + (16 * k2 + 8 * h + t) * STR + g;
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    uint32_t x[4];
+                    x[0] = er[16 * m];
+                    x[1] = KB > 8 ? er[16 * m + 8] : 0u;
+                    x[2] = er[4 * STR + 16 * m];
+                    x[3] = KB > 8 ? er[4 * STR + 16 * m + 8] : 0u;
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) mma_16816(acc[m][n], x, h ? b[n].z : b[n].x, h ? b[n].w : b[n].y);
+                }
+            }
+        }
+        // bit 8 n + 2 t + c of the word of key 16 m + 8 half + g
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int half = 0; half < HALVES; ++half) {
+                const int key = 16 * m + 8 * half + g;
+                const float lim = mine ? bound[key] : -1.0f;
+                uint32_t v = 0, close = 0;  // sign bits shifted in: a sum is close where |sum| - bound is negative
+#pragma unroll
+                for (int n = 3; n >= 0; --n) {
+                    v <<= 6;
+                    close <<= 6;
+#pragma unroll
+                    for (int c = 1; c >= 0; --c) {
+                        const float x = acc[m][n][2 * half + c];
+                        v = __funnelshift_l(__float_as_uint(x), v, 1);
+                        close = __funnelshift_l(__float_as_uint(__fsub_rn(fabsf(x), lim)), close, 1);
+                    }
+                }
+                v &= ~close;
+                if (!mine) close = 0u;
+                v <<= 2 * t;
+                near[wd][m * HALVES + half] = close << (2 * t);
+                nears += __popc(close);
+                v |= __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+                v |= __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+                if (t == 0 && mine) reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64)[word] = v;
+            }
+    }
+    // the sums to take again go to the list, one reservation per warp
+    if (__any_sync(0xFFFFFFFFu, nears != 0u)) {
+        uint32_t at = nears;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, at, o);
+            if (lane >= o) at += y;
+        }
+        uint32_t base = 0;
+        if (lane == 31) base = atomicAdd(cnt, at);
+        at += __shfl_sync(0xFFFFFFFFu, base, 31) - nears;
+#pragma unroll
+        for (int wd = 0; wd < WORDS; ++wd)
+#pragma unroll
+            for (int i = 0; i < MT * HALVES; ++i)
+                for (uint32_t b = near[wd][i]; b; b &= b - 1u, ++at)
+                    if (at < KB * SIGN_LIST) list[at] = (uint16_t)((8 * i + g) << 8 | (32 * (warp + wd * WARPS) + __ffs(b) - 1));
+    }
+    __syncthreads();
+    const uint32_t again = *cnt;
+    if (again > KB * SIGN_LIST) return false;
+    // The rows of Z are copied together, a warp per row, to the place of the fp16 pairs; then a thread per sum.  (With every thread loading its
+    // own row each load met 32 lines, and the phase was bound by the L1's tags.)
+    float* zs = reinterpret_cast<float*>(eh);
+    const uint32_t stride = (dp + 7) / 4 * 4, room = min((words - sign_fixed(KB)) / stride, (uint32_t)NT);  // (4 words over a multiple of 32: no bank conflicts)
+    for (uint32_t e0 = 0; e0 < again; e0 += room) {
+        const uint32_t n = min(room, again - e0);
+        for (uint32_t e = warp; e < n; e += WARPS) {
+            const float* z = a.z + (size_t)(list[e0 + e] & 255u) * dp;
+            if (dp % 4 == 0) {
+                const uint32_t to = (uint32_t)__cvta_generic_to_shared(zs + e * stride);
+                for (uint32_t i = 4 * lane; i < dp; i += 128)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to + 4 * i), "l"(z + i) : "memory");
+            } else {
+                for (uint32_t i = lane; i < dp; i += 32) zs[e * stride + i] = __ldg(z + i);
+            }
+        }
+        asm volatile("cp.async.wait_all;\n" ::: "memory");
+        __syncthreads();
+        if (tid < n) {
+            const uint32_t key = list[e0 + tid] >> 8, s = list[e0 + tid] & 255u;
+            const float* z = zs + tid * stride;
+            const float* x = buf + key;
+            float sum = 0.0f;
+            uint32_t i = 0;
+#pragma unroll 4
+            for (; i + 4 <= dp; i += 4) {
+                const float4 z4 = *reinterpret_cast<const float4*>(z + i);
+                sum = __fadd_rn(sum, __fmul_rn(z4.x, x[(size_t)i * KS]));
+                sum = __fadd_rn(sum, __fmul_rn(z4.y, x[(size_t)(i + 1) * KS]));
+                sum = __fadd_rn(sum, __fmul_rn(z4.z, x[(size_t)(i + 2) * KS]));
+                sum = __fadd_rn(sum, __fmul_rn(z4.w, x[(size_t)(i + 3) * KS]));
+            }
+            for (; i < dp; ++i) sum = __fadd_rn(sum, __fmul_rn(z[i], x[(size_t)i * KS]));
+            if (sum < 0.0f) atomicOr(reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64) + (s >> 5), 1u << (s & 31u));
+        }
+        if (e0 + room < again) __syncthreads();
+    }
+    return true;
+}
+
+// Residuals of 32 keys for up to 32 C columns, C columns (32 apart) times 8 keys a thread: e = key - sum_k w_k P[k][column], in place of the key.
+template <int C>
+__device__ __forceinline__ void residual_columns(const EncodeArgs& a, float* buf, const float* wsT) {
+    constexpr int KS = enc_row_stride(32);
+    const uint32_t d = a.d, c0 = 8 * (threadIdx.x >> 5) + (threadIdx.x & 7), kg = (threadIdx.x & 31) >> 3;
+    const float* mp = a.p + c0;
+    const float* wr = wsT + 8 * kg;
+    uint64_t acc[C][4] = {};
+#pragma unroll 4
+    for (int k = 0; k < D_C; ++k) {
+        uint64_t kv[4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float4 x = reinterpret_cast<const float4*>(wr + (size_t)k * KS)[j];
+            kv[2 * j] = pack2(x.x, x.y);
+            kv[2 * j + 1] = pack2(x.z, x.w);
+        }
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+            const float m = c0 + 32 * c < d ? __ldg(mp + (size_t)k * d + 32 * c) : 0.0f;
+            const uint64_t mm = pack2(m, m);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) acc[c][j] = add2(mul2(mm, kv[j]), a.one, acc[c][j]);
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+        if (c0 + 32 * c >= d) continue;
+        float* row = buf + (size_t)(c0 + 32 * c) * KS + 8 * kg;
+        float e[8], kv[8];
+        load_keys<8>(kv, row);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) unpack2(acc[c][j], e[2 * j], e[2 * j + 1]);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) e[j] = __fsub_rn(kv[j], e[j]);
+        store_keys<8>(row, e);
+    }
+}
+
+// 2^R-point stretches of the Hadamard butterflies of buf [dp][KS] in registers: the stages h, 2 h, .. 2^(R-1) h, each sum and difference the
+// reference's.  first: the inputs times the diagonal; last: the outputs times 1/sqrt(dp).
+template <int KB, int R>
+__device__ __forceinline__ void fwht_stages(float* buf, uint32_t dp, uint32_t log2_h, const float* diag, float inv) {
+    constexpr int KS = enc_row_stride(KB), P = 1 << R, NT = enc_threads(KB);
+    const bool last = (1u << (log2_h + R)) == dp;
+    const uint32_t h = 1u << log2_h;
+    for (uint32_t e = threadIdx.x; e < (dp >> R) * KB; e += NT) {
+        const uint32_t q = e / KB, at = ((q >> log2_h) << (log2_h + R)) + (q & (h - 1u));
+        float* col = buf + (size_t)at * KS + e % KB;
+        float x[P];
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+            x[r] = col[(size_t)(r * h) * KS];
+            if (log2_h == 0) x[r] = __fmul_rn(x[r], __ldg(diag + at + r));
+        }
+#pragma unroll
+        for (int o = 1; o < P; o <<= 1)
+#pragma unroll
+            for (int r = 0; r < P; ++r)
+                if (!(r & o)) {
+                    const float u = x[r], v = x[r + o];
+                    x[r] = __fadd_rn(u, v);
+                    x[r + o] = __fsub_rn(u, v);
+                }
+#pragma unroll
+        for (int r = 0; r < P; ++r) col[(size_t)(r * h) * KS] = last ? __fmul_rn(x[r], inv) : x[r];
+    }
+}
+
 // KB keys per CTA pass (compile time: 32 unless the model dimension leaves no room).  Every
 // contraction is walked sequentially by the thread that owns the output element, for all the keys
-// the thread holds at once: one matrix element and KB/8 (latent, residual: half the keys per thread)
-// or KB/4 (sign bits) vector loads feed KB or 2 KB multiply-adds.
-constexpr int enc_row_stride(int kb) { return kb >= 8 ? kb + 4 : kb; }
+// the thread holds at once.
 
 template <bool QUERY, int KB>
-// (three CTAs of 32 keys share an SM at head dimension 128: 80 registers, 74 KB of shared memory each)
-__global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(EncodeArgs a) {
+// (four CTAs of 32 keys share an SM at head dimension 128: up to 128 registers, 57 KB of shared memory each)
+__global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kernel(EncodeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int PER = KB >= 2 ? KB / 2 : 1;  // keys per thread where two threads share an output row
+    constexpr int NT = enc_threads(KB);
     const uint32_t d = a.d, dp = a.d_pad;
-    // shared: tiles [KB][128 B] | h [KB][128] | keyT [d][KS] | bufT [d_pad][KS] | wsT [128][KS]
-    // (keys and the sign-LSH input are stored transposed so that one thread
+    // shared: tiles [KB][128 B] | buf [d_pad][KS] | h [KB][128] | wsT [128][KS]
+    // (buf holds the keys, then in their place the residuals, the sign-LSH input, transposed so that one thread
     // reads the KB values of a contraction index with 16-byte loads).  Rows are KS = KB + 4
     // floats apart: a warp whose lanes walk the rows then spreads its 16-byte accesses over
-    // all banks, while lanes that walk the keys of one row stay on consecutive banks.
+    // all banks, while lanes that walk the keys of one row stay on consecutive banks.  The sign phase works in the
+    // space of h and wsT.
     constexpr int KS = enc_row_stride(KB);
     unsigned char* tl = smem;
-    float* hs = reinterpret_cast<float*>(tl + (size_t)KB * TILE_BYTES);
-    float* keyT = hs + (size_t)KB * D_C;
-    float* buf = keyT + (((size_t)d * KS + 3) & ~size_t(3));
-    float* wsT = buf + (size_t)dp * KS;  // h_k * s_k of every key, transposed like keyT
+    float* buf = reinterpret_cast<float*>(tl + (size_t)KB * TILE_BYTES);
+    float* hs = buf + (((size_t)dp * KS + 3) & ~size_t(3));
+    float* wsT = hs + (size_t)KB * D_C;  // h_k * s_k of every key, transposed like buf
 
     for (uint64_t base = (uint64_t)blockIdx.x * KB; base < a.n; base += (uint64_t)gridDim.x * KB) {
         const int nk = (int)min((uint64_t)KB, a.n - base);
         __syncthreads();
-        // ---- load keys (transposed: keyT[i][j]); absent keys are zero ------
+        // ---- load keys (transposed: buf[i][j]); absent keys and padding rows are zero ------
         const bool f32 = a.key_dtype == SLHA_B200_F32;
         const uint32_t epc = f32 ? 4u : 8u;  // elements per 16-byte chunk
         if (KB >= 8 && d % epc == 0 && (reinterpret_cast<uintptr_t>(a.keys) & 15) == 0) {
             // 16-byte chunks; the lanes of a warp take the same chunk of consecutive keys, so
-            // that their transposed stores fall on consecutive banks.  Both loads of a thread
+            // that their transposed stores fall on consecutive banks.  All loads of a thread
             // are in flight before the first store.
+            constexpr int U = 512 / NT;
             const uint32_t cpk = d / epc, total = cpk * (uint32_t)KB;
             const uint4* src = reinterpret_cast<const uint4*>(a.keys) + base * cpk;
-            for (uint32_t c0 = tid; c0 < total; c0 += 2 * ENC_THREADS) {
-                uint4 v[2];
+            for (uint32_t c0 = tid; c0 < total; c0 += U * NT) {
+                uint4 v[U];
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const uint32_t c = c0 + u * ENC_THREADS, j = c % KB, ic = c / KB;
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t c = c0 + u * NT, j = c % KB, ic = c / KB;
                     v[u] = make_uint4(0u, 0u, 0u, 0u);
                     if (c < total && (int)j < nk) v[u] = __ldg(src + (size_t)j * cpk + ic);
                 }
 #pragma unroll
-                for (int u = 0; u < 2; ++u) {
-                    const uint32_t c = c0 + u * ENC_THREADS, j = c % KB, ic = c / KB;
+                for (int u = 0; u < U; ++u) {
+                    const uint32_t c = c0 + u * NT, j = c % KB, ic = c / KB;
                     if (c >= total) continue;
-                    float* dst = keyT + (size_t)(ic * epc) * KS + j;
+                    float* dst = buf + (size_t)(ic * epc) * KS + j;
                     const uint32_t w[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
@@ -378,7 +673,7 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
                 }
             }
         } else {
-            for (uint32_t e = tid; e < d * (uint32_t)KB; e += ENC_THREADS) {
+            for (uint32_t e = tid; e < d * (uint32_t)KB; e += NT) {
                 const int j = e / d;
                 const uint32_t i = e % d;
                 float x = 0.0f;
@@ -387,61 +682,65 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
                     x = f32 ? reinterpret_cast<const float*>(a.keys)[o]
                             : __uint_as_float((uint32_t)reinterpret_cast<const uint16_t*>(a.keys)[o] << 16);
                 }
-                keyT[(size_t)i * KS + j] = x;
+                buf[(size_t)i * KS + j] = x;
             }
         }
-        for (int e = tid; e < KB * 32; e += ENC_THREADS) reinterpret_cast<uint32_t*>(tl)[e] = 0;
+        for (uint32_t e = d * KS + tid; e < dp * KS; e += NT) buf[e] = 0.0f;
         __syncthreads();
 
-        // With 32 keys per pass every thread holds a 4 x 4 (latent, residual) or 4 x 8 (sign bits)
-        // tile of outputs: four matrix elements (one 16-byte load) and four or eight key values
-        // (one or two 16-byte broadcast loads) feed 16 or 32 multiply-adds, a third of the
-        // register fills per multiply-add of a one-row tile.
+        // With 32 keys per pass every thread holds a 4 x 8 tile of outputs: four matrix elements (one 16-byte load) and eight key
+        // values (two 16-byte loads) feed 32 multiply-adds.  An SM's load path fills 128 bytes of registers a cycle, whether
+        // lanes load the same address or not, and its fp32 lanes take 64 cycles for the four warps' steps: 48 cycles of fills here, as many
+        // as the arithmetic with 4 x 4 tiles (encode of 262 144 bf16 keys, NF4: 888 us with those and 256 threads).  A warp's tiles
+        // form 32 outputs x 32 keys, so that a CTA reads each matrix once.
         const bool tiled = KB == 32 && d % 4 == 0 &&
                            ((reinterpret_cast<uintptr_t>(a.pt) | reinterpret_cast<uintptr_t>(a.p) |
                              reinterpret_cast<uintptr_t>(a.zt) | reinterpret_cast<uintptr_t>(a.scale)) & 15) == 0;
-        // ---- latent / q_coarse: rows 4 lane .. +3, keys 4 warp .. +3 ------------
+        // ---- latent / q_coarse: rows 4 rl .. +3, keys 8 kl .. +7 ------------
         if (KB == 32 && tiled) {
-            uint64_t acc2[4][2];
-            zero_tile<4, 4>(acc2);
-            const float4* mp = reinterpret_cast<const float4*>(a.pt) + lane;
-#pragma unroll 16
+            const int rl = 8 * warp + (lane & 7), kl = lane >> 3;
+            uint64_t acc2[4][4];
+            zero_tile<4, 8>(acc2);
+            const float4* mp = reinterpret_cast<const float4*>(a.pt) + rl;
+#pragma unroll 8
             for (uint32_t i = 0; i < d; ++i)
-                outer_keys<4, 4>(acc2, __ldg(mp + (size_t)i * (D_C / 4)), keyT + (size_t)i * KS + 4 * warp, a.one);
-            float acc[4][4];
-            unpack_tile<4, 4>(acc2, acc);
-            const float4 s4 = __ldg(reinterpret_cast<const float4*>(a.scale) + lane);
+                outer_keys<4, 8>(acc2, __ldg(mp + (size_t)i * (D_C / 4)), buf + (size_t)i * KS + 8 * kl, a.one);
+            float acc[4][8];
+            unpack_tile<4, 8>(acc2, acc);
+            const float4 s4 = __ldg(reinterpret_cast<const float4*>(a.scale) + rl);
             const float sk[4] = {s4.x, s4.y, s4.z, s4.w};
+            const bool whiten = s4.x != 1.0f || s4.y != 1.0f || s4.z != 1.0f || s4.w != 1.0f;  // (a division by one changes nothing, but takes a branch each)
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                float hv[4];
+            for (int j = 0; j < 8; ++j) {
+                float hv[4] = {acc[0][j], acc[1][j], acc[2][j], acc[3][j]};
+                if (whiten) {
 #pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    hv[r] = QUERY ? __fmul_rn(acc[r][j], sk[r]) : __fdiv_rn(acc[r][j], sk[r]);
-                    acc[r][j] = __fmul_rn(hv[r], sk[r]);  // w[k][j] = h_j[k] * s_k, the factor of P[k][:] in the reconstruction
+                    for (int r = 0; r < 4; ++r) {
+                        hv[r] = QUERY ? __fmul_rn(acc[r][j], sk[r]) : __fdiv_rn(acc[r][j], sk[r]);
+                        acc[r][j] = __fmul_rn(hv[r], sk[r]);  // w[k][j] = h_j[k] * s_k, the factor of P[k][:] in the reconstruction
+                    }
                 }
-                store_keys<4>(hs + (size_t)(4 * warp + j) * D_C + 4 * lane, hv);
+                store_keys<4>(hs + (size_t)(8 * kl + j) * D_C + 4 * h_chunk(rl), hv);
             }
             if (!QUERY) {
 #pragma unroll
-                for (int r = 0; r < 4; ++r) store_keys<4>(wsT + (size_t)(4 * lane + r) * KS + 4 * warp, acc[r]);
+                for (int r = 0; r < 4; ++r) store_keys<8>(wsT + (size_t)(4 * rl + r) * KS + 8 * kl, acc[r]);
             }
         } else {
-            // row k = tid & 127, keys of half (tid >> 7)
-            const int k = tid & 127, half = tid >> 7;
-            const int j0 = (KB >= 2) ? half * PER : 0;
-            if (KB >= 2 || half == 0) {
+            // row k = u & 127, keys of half (u >> 7)
+            for (int u = tid; u < (KB >= 2 ? 2 : 1) * D_C; u += NT) {
+                const int k = u & 127, j0 = (u >> 7) * PER;
                 float acc[PER];
 #pragma unroll
                 for (int j = 0; j < PER; ++j) acc[j] = 0.0f;
-#pragma unroll 8
+#pragma unroll KB <= 8 ? 32 : 8
                 for (uint32_t i = 0; i < d; ++i)
-                    axpy_keys<PER>(acc, a.pt[(size_t)i * D_C + k], keyT + (size_t)i * KS + j0);
+                    axpy_keys<PER>(acc, a.pt[(size_t)i * D_C + k], buf + (size_t)i * KS + j0);
                 const float sk = a.scale[k];
 #pragma unroll
                 for (int j = 0; j < PER; ++j) {
                     const float hv = QUERY ? __fmul_rn(acc[j], sk) : __fdiv_rn(acc[j], sk);
-                    hs[(size_t)(j0 + j) * D_C + k] = hv;
+                    hs[(size_t)(j0 + j) * D_C + 4 * h_chunk(k >> 2) + (k & 3)] = hv;
                     // w[k][j] = h_j[k] * s_k, the factor the reconstruction multiplies P[k][:] by
                     acc[j] = __fmul_rn(hv, sk);
                 }
@@ -451,63 +750,70 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
         __syncthreads();
 
         if (QUERY) {
-            for (int e = tid; e < nk * D_C; e += ENC_THREADS)
-                a.q_coarse[(base + e / D_C) * D_C + (e % D_C)] = hs[e];
-            // sign-LSH input is the raw query
-            for (uint32_t e = tid; e < dp * (uint32_t)KS; e += ENC_THREADS)
-                buf[e] = (e / KS) < d ? keyT[e] : 0.0f;
+            for (int e = tid; e < nk * D_C; e += NT)
+                a.q_coarse[(base + e / D_C) * D_C + (e % D_C)] = hs[(e & ~(D_C - 1)) + 4 * h_chunk((e % D_C) >> 2) + (e & 3)];
+            // (the sign-LSH input is the raw query)
         } else {
-            // ---- quantise: one warp per key ---------------------------------
-            for (int j = warp; j < KB; j += ENC_THREADS / 32)
-                quantize_warp(hs + (size_t)j * D_C, a.codec, tl + (size_t)j * TILE_BYTES, lane);
+            // ---- quantise ---------------------------------
+            for (int e = tid; e < (KB > 4 ? KB * 8 : 32); e += NT) {
+                const int j = min(e >> 3, KB - 1);
+                quantize_unit(hs + (size_t)j * D_C, a.codec, tl + (size_t)j * TILE_BYTES, e & 7, (e >> 3) < KB);
+            }
             // (no barrier: the residual phase reads the keys and the reconstruction factors, which
             //  the barrier after the latent phase already covers, and does not touch the tiles)
             // ---- residual e = key - sum_k (h_k*s_k) * P[k][:]  (k outer, sequential): a thread owns
             //      column i for half of the keys ---------------------------------------------------
             constexpr int HALVES = KB >= 2 ? 2 : 1;
-            // tiled: columns 4 ig .. +3 for keys 4 kg .. +3
-            for (uint32_t wi = tid; KB == 32 && tiled && wi < (d / 4) * 8; wi += ENC_THREADS) {
-                const uint32_t ig = wi % (d / 4), kg = wi / (d / 4);
-                uint64_t acc2[4][2];
-                zero_tile<4, 4>(acc2);
+            // tiled: columns 4 ig .. +3 for keys 8 kg .. +7 (or five or six columns a thread, where fours would take the warps two rounds)
+            if (KB == 32 && tiled && d > 128 && d <= 192) {
+                if (d <= 160) residual_columns<5>(a, buf, wsT);
+                else residual_columns<6>(a, buf, wsT);
+            }
+            for (uint32_t wt = warp; KB == 32 && tiled && !(d > 128 && d <= 192) && wt < (d + 31) / 32; wt += NT / 32) {
+                const uint32_t ig = 8 * wt + (lane & 7), kg = lane >> 3;
+                if (ig >= d / 4) continue;
+                uint64_t acc2[4][4];
+                zero_tile<4, 8>(acc2);
                 const float4* mp = reinterpret_cast<const float4*>(a.p) + ig;
-                const float* wr = wsT + 4 * kg;
-#pragma unroll 16
+                const float* wr = wsT + 8 * kg;
+#pragma unroll 8
                 for (int k = 0; k < D_C; ++k)
-                    outer_keys<4, 4>(acc2, __ldg(mp + (size_t)k * (d / 4)), wr + (size_t)k * KS, a.one);
-                float acc[4][4];
-                unpack_tile<4, 4>(acc2, acc);
+                    outer_keys<4, 8>(acc2, __ldg(mp + (size_t)k * (d / 4)), wr + (size_t)k * KS, a.one);
+                float acc[4][8];
+                unpack_tile<4, 8>(acc2, acc);
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    float kv[4];
-                    load_keys<4>(kv, keyT + (size_t)(4 * ig + r) * KS + 4 * kg);
+                    float kv[8];
+                    load_keys<8>(kv, buf + (size_t)(4 * ig + r) * KS + 8 * kg);
 #pragma unroll
-                    for (int j = 0; j < 4; ++j) acc[r][j] = __fsub_rn(kv[j], acc[r][j]);
-                    store_keys<4>(buf + (size_t)(4 * ig + r) * KS + 4 * kg, acc[r]);
+                    for (int j = 0; j < 8; ++j) acc[r][j] = __fsub_rn(kv[j], acc[r][j]);
+                    store_keys<8>(buf + (size_t)(4 * ig + r) * KS + 8 * kg, acc[r]);
                 }
             }
-            for (uint32_t wi = tid; !(KB == 32 && tiled) && wi < HALVES * d; wi += ENC_THREADS) {
+            for (uint32_t wi = tid; !(KB == 32 && tiled) && wi < HALVES * d; wi += NT) {
                 const uint32_t i = wi % d, half = wi / d;
                 float acc[PER];
 #pragma unroll
                 for (int j = 0; j < PER; ++j) acc[j] = 0.0f;
                 const float* wr = wsT + half * PER;
-#pragma unroll 8
+#pragma unroll KB <= 8 ? 32 : 8
                 for (int k = 0; k < D_C; ++k) axpy_keys<PER>(acc, a.p[(size_t)k * d + i], wr + (size_t)k * KS);
                 float kv[PER];
-                load_keys<PER>(kv, keyT + (size_t)i * KS + half * PER);
+                load_keys<PER>(kv, buf + (size_t)i * KS + half * PER);
 #pragma unroll
                 for (int j = 0; j < PER; ++j) acc[j] = __fsub_rn(kv[j], acc[j]);
                 store_keys<PER>(buf + (size_t)i * KS + half * PER, acc);
             }
-            for (uint32_t e = d * KS + tid; e < dp * KS; e += ENC_THREADS) buf[e] = 0.0f;  // padding rows
         }
         __syncthreads();
 
-        // ---- sigma_E (f32, sequential over i) and tile metadata ---------------
-        if (!QUERY && tid < nk) {
-            const int j = tid;
+        // ---- sigma_E (f32, sequential over i) and tile metadata: the last warp (the others go on with the signs where no rotation
+        //      changes the residual first) ---------------
+        auto metadata = [&]() {
+            const int j = tid - (NT - 32);
+            if (QUERY || j < 0 || j >= nk) return;
             float ss = 0.0f;
+#pragma unroll 8
             for (uint32_t i = 0; i < d; ++i) {
                 const float x = buf[(size_t)i * KS + j];
                 ss = __fadd_rn(ss, __fmul_rn(x, x));
@@ -526,33 +832,38 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
             else if (a.codec == SLHA_CODEC_TQ3) cflag = F_TQ3;
             else if (a.codec == SLHA_CODEC_MIX3) cflag = F_MIX3;
             *reinterpret_cast<uint32_t*>(tile + 116) = head | (cflag << 16);
-        }
-        __syncthreads();
+        };
 
         // ---- optional randomised Hadamard transform of buf ------------------
         if (a.diag) {
-            for (uint32_t e = tid; e < dp * (uint32_t)KS; e += ENC_THREADS)
-                buf[e] = __fmul_rn(buf[e], a.diag[e / KS]);
-            __syncthreads();
-            for (uint32_t h = 1; h < dp; h <<= 1) {
-                for (uint32_t e = tid; e < (dp / 2) * (uint32_t)KB; e += ENC_THREADS) {
-                    const uint32_t j = e % KB, pr = e / KB;
-                    const uint32_t lo = ((pr / h) * 2 * h) + (pr % h);
-                    float* col = buf + j;
-                    const float x = col[(size_t)lo * KS], y = col[(size_t)(lo + h) * KS];
-                    col[(size_t)lo * KS] = __fadd_rn(x, y);
-                    col[(size_t)(lo + h) * KS] = __fsub_rn(x, y);
-                }
+            metadata();
+            if (!QUERY) __syncthreads();
+            uint32_t at = 0, left = 31 - __clz(dp);
+            for (; left >= 4; left -= 4, at += 4) {
+                fwht_stages<KB, 4>(buf, dp, at, a.diag, a.fwht_inv);
                 __syncthreads();
             }
-            for (uint32_t e = tid; e < dp * (uint32_t)KS; e += ENC_THREADS)
-                buf[e] = __fmul_rn(buf[e], a.fwht_inv);
-            __syncthreads();
+            if (dp == 1) fwht_stages<KB, 0>(buf, dp, 0, a.diag, a.fwht_inv);
+            if (left == 3) fwht_stages<KB, 3>(buf, dp, at, a.diag, a.fwht_inv);
+            if (left == 2) fwht_stages<KB, 2>(buf, dp, at, a.diag, a.fwht_inv);
+            if (left == 1) fwht_stages<KB, 1>(buf, dp, at, a.diag, a.fwht_inv);
+            if (left || at == 0) __syncthreads();
         }
 
-        // ---- sign-LSH, tiled: hyperplanes 4 rg .. +3 for keys 8 kg .. +7 -------
-        if (KB == 32 && tiled) {
-            const int rg = tid & 63, kg = tid >> 6;
+        // ---- sign-LSH ----------------------------------------------------------
+        bool signs_done = false;
+        if constexpr (KB >= 4) {
+            if (a.zf) signs_done = signs_mma<KB>(a, buf, tl, reinterpret_cast<uint32_t*>(hs), (uint32_t)(D_C * (KB + KS)), [&]() { if (!a.diag) metadata(); });
+            else if (!a.diag) metadata();
+        } else if (!a.diag) {
+            metadata();
+        }
+        if (!signs_done) __syncthreads();
+        // every sum in the reference's order, tiled: hyperplanes 4 rg .. +3 for keys 8 kg .. +7
+        if (signs_done) {
+        } else if (KB == 32 && tiled) {
+            for (int u = tid; u < 256; u += NT) {
+            const int rg = u & 63, kg = u >> 6;
             uint64_t acc2[4][4];
             zero_tile<4, 8>(acc2);
             const float4* mp = reinterpret_cast<const float4*>(a.zt) + rg;
@@ -571,16 +882,12 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
                 v |= __shfl_xor_sync(0xFFFFFFFFu, v, 2);
                 v |= __shfl_xor_sync(0xFFFFFFFFu, v, 4);
                 const int key = 8 * kg + j, word = (rg >> 3);
-                if ((lane & 7) == 0 && key < nk) {
-                    if (QUERY)
-                        reinterpret_cast<uint32_t*>(a.q_sign)[(base + key) * 8 + word] = v;
-                    else
-                        reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64)[word] = v;
-                }
+                if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64)[word] = v;
+            }
             }
         } else {
-            // thread s owns hyperplane s for all KB keys
-            const int s = tid;  // ENC_THREADS == D_S
+            // a thread owns hyperplane s for all KB keys
+            for (int s = tid; s < D_S; s += NT) {
             float acc[KB];
 #pragma unroll
             for (int j = 0; j < KB; ++j) acc[j] = 0.0f;
@@ -589,19 +896,18 @@ __global__ void __launch_bounds__(ENC_THREADS, KB == 32 ? 3 : 1) encode_kernel(E
 #pragma unroll
             for (int j = 0; j < KB; ++j) {
                 const unsigned b = __ballot_sync(0xFFFFFFFFu, acc[j] < 0.0f);
-                if (lane == 0 && j < nk) {
-                    if (QUERY)
-                        reinterpret_cast<uint32_t*>(a.q_sign)[(base + j) * 8 + warp] = b;
-                    else
-                        reinterpret_cast<uint32_t*>(tl + (size_t)j * TILE_BYTES + 64)[warp] = b;
-                }
+                if (lane == 0) reinterpret_cast<uint32_t*>(tl + (size_t)j * TILE_BYTES + 64)[s >> 5] = b;
+            }
             }
         }
         __syncthreads();
 
-        // ---- write tiles: 8 x 16 B per tile ------------------------------------
-        if (!QUERY) {
-            for (int e = tid; e < nk * 8; e += ENC_THREADS) {
+        // ---- write tiles: 8 x 16 B per tile (query mode: their 32 sign bytes) -----
+        if (QUERY) {
+            for (int e = tid; e < nk * 8; e += NT)
+                reinterpret_cast<uint32_t*>(a.q_sign)[base * 8 + e] = reinterpret_cast<const uint32_t*>(tl + (size_t)(e >> 3) * TILE_BYTES + 64)[e & 7];
+        } else {
+            for (int e = tid; e < nk * 8; e += NT) {
                 const int j = e >> 3, c = e & 7;
                 const uint64_t dst = a.slots ? a.slots[base + j] : base + j;
                 reinterpret_cast<uint4*>(a.tiles + dst * TILE_BYTES)[c] =
@@ -679,9 +985,9 @@ __global__ void decode_kernel(const unsigned char* tile, const float* p, const f
     }
 }
 
-size_t encode_smem(uint32_t d, uint32_t dp, int kb) {
+size_t encode_smem(uint32_t d_pad, int kb) {
     const size_t ks = (size_t)enc_row_stride(kb);
-    return (((d * ks + 3) & ~size_t(3)) + (size_t)kb * D_C + ks * dp + ks * D_C) * 4 + (size_t)kb * TILE_BYTES;
+    return (((d_pad * ks + 3) & ~size_t(3)) + (size_t)kb * D_C + ks * D_C) * 4 + (size_t)kb * TILE_BYTES;
 }
 
 Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
@@ -691,14 +997,17 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
     a.pt = m->d_pt;
     a.scale = m->d_scale;
     a.zt = m->d_zt;
+    a.z = m->d_z;
+    a.z_guard = m->z_guard;
+    a.z_norm = m->z_norm;
     a.diag = m->d_diag;
     a.fwht_inv = 1.0f / sqrtf((float)m->d_pad);
     a.one = 0x3F8000003F800000ull;
     a.lambda_c = sqrtf(3.14159265358979323846f / (2.0f * (float)D_S));
     // 32 keys per CTA pass when two CTAs still share an SM (their registers allow no more), else fewer
     int kb = 32;
-    while (kb > 1 && encode_smem(a.d, a.d_pad, kb) > (kb == 32 ? 100 : 200) * 1024) kb >>= 1;
-    if (encode_smem(a.d, a.d_pad, kb) > 200 * 1024)
+    while (kb > 1 && encode_smem(a.d_pad, kb) > (kb == 32 ? 100 : 200) * 1024) kb >>= 1;
+    if (encode_smem(a.d_pad, kb) > 200 * 1024)
         return Status(SLHA_ERR_DIMENSION, "model dimension too large for the encode kernel");
     // Few keys: the narrowest CTA of at least 4 keys that leaves no SM a second one.  Measured (d = 128, bf16,
     // us per call at 8 / 592 / 1184 / 2368 / 4736 keys): 32 keys per CTA 39 / 39 / 37 / 37 / 37, 16: 29 / 28 / 29 / 29 / 39,
@@ -707,12 +1016,14 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
     while (kb > 4 && n <= (uint64_t)(kb / 2) * (uint64_t)sm_count(m->device)) kb >>= 1;
     *kb_out = kb;
     a.kb = kb;
+    // (the sign phase works in the space of h and the reconstruction factors)
+    a.zf = kb >= 4 && sign_words(a.d_pad, kb) <= (uint32_t)(D_C * (kb + enc_row_stride(kb))) ? m->d_zf : nullptr;
     return Status();
 }
 
 template <bool QUERY, int KB>
 Status run_encode_kb(Ctx* c, EncodeArgs& a) {
-    const size_t smem = encode_smem(a.d, a.d_pad, KB);
+    const size_t smem = encode_smem(a.d_pad, KB);
     static thread_local bool configured[16] = {false};  // the attribute is per device
     if (!configured[c->device & 15]) {
         SLHA_CUDA(cudaFuncSetAttribute(encode_kernel<QUERY, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
@@ -724,7 +1035,7 @@ Status run_encode_kb(Ctx* c, EncodeArgs& a) {
     // different phases, so that the arithmetic of one covers the loads, quantisation and barriers
     // of the others.  One resident wave measured 182 M keys/s, 8 CTAs per SM 191, one CTA per pass 199.
     const uint32_t grid = (uint32_t)std::min<uint64_t>(groups, 148ull * 64);
-    encode_kernel<QUERY, KB><<<grid, ENC_THREADS, smem, c->stream>>>(a);
+    encode_kernel<QUERY, KB><<<grid, enc_threads(KB), smem, c->stream>>>(a);
     count_launch();
     SLHA_CUDA(cudaGetLastError());
     return Status();

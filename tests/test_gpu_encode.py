@@ -181,3 +181,51 @@ def test_small_batches_take_narrower_ctas_and_give_the_same_bytes(d, rht, codec)
         assert np.array_equal(m.encode_keys(keys[:k], codec).view(np.uint8), whole[:k].view(np.uint8)), k
         c, s = m.prepare_queries(keys[:k])
         assert np.array_equal(c, qc[:k]) and np.array_equal(s, qs[:k]), k
+
+
+@pytest.mark.parametrize("n", [5, 700, 1500, 5000])  # 4, 8, 16 and 32 keys per CTA
+@pytest.mark.parametrize("d,rht", [(128, False), (160, True), (72, False), (129, True), (256, False)])
+def test_sign_bits_near_and_at_zero_follow_the_exact_sums(n, d, rht):
+    """The signs come from fp16 sums unless those are too close to zero: residuals that are orthogonal to hyperplanes up to
+    rounding, equal to zero, sparse, of extreme size or not finite give the bits of the sequential float32 sums."""
+    rng = np.random.default_rng(n + d)
+    p = H.orthogonal_projection(11, d) if d >= 128 else np.ascontiguousarray(rng.standard_normal((128, d)) / 11, F)
+    om, gm = ora.Model(p, d, seed=7, rht=rht), S.Model.from_projection(p, d, 7, rht=rht)
+    q = H.gaussian_keys(n, n, d, outlier_channels=(7,))
+    z = ora.Rng(7).gaussian(256 * d).reshape(256, d).astype(np.float64) if not rht else rng.standard_normal((256, d))
+    for j in range(1, n, 5):  # a query with a sum of almost nothing: orthogonal to four hyperplanes
+        rows = z[rng.choice(256, 4, replace=False)]
+        q[j] -= (np.linalg.lstsq(rows.T, q[j].astype(np.float64), rcond=None)[0] @ rows).astype(F)
+    q[0::50] *= F(1e-37)
+    q[2::50] *= F(1e25)
+    q[3::50] = 0.0
+    q[4::50, 1:] = 0.0
+    q[8::100, 3] = np.inf
+    q[9::100, 5] = np.nan
+    qc, qs = gm.prepare_queries(q)
+    some = range(n) if n < 1000 else rng.choice(n, 700, replace=False)
+    for j in some:
+        wc, ws = om.prepare_query(q[j])
+        assert np.array_equal(qs[j], ws), j
+    keys = np.where(np.isfinite(q), q, F(1.0))
+    got, want = gm.encode_keys(keys, 2), om.encode_batch(keys, 2)
+    assert got.tobytes() == want.tobytes(), _diff(got, want)
+
+
+def test_nf4_codes_at_the_floats_between_two_entries():
+    # identity projection and a group maximum of 1: the quantised value is the key's element itself, here the floats around every midpoint
+    p = np.zeros((128, 128), F)
+    p[np.arange(128), np.arange(128)] = 1.0
+    om, gm = ora.Model(p, 128, seed=3), S.Model.from_projection(p, 128, 3)
+    book = np.array([-1.0, -0.7075, -0.5421, -0.4165, -0.3108, -0.2158, -0.1272, -0.0421, 0.0421, 0.1272, 0.2158, 0.3108, 0.4165, 0.5421, 0.7075, 1.0], F)
+    mid = ((book[1:] + book[:-1]) / F(2)).astype(F)
+    near = (mid[mid != 0].view(np.int32)[:, None] + np.arange(-60, 60)).astype(np.int32).view(F).reshape(-1)
+    near = np.concatenate([near, np.linspace(-3e-9, 3e-9, 240).astype(F)])
+    keys = np.ones((len(near) // 120 + 1, 128), F)
+    keys[:, 0::16] = -1.0
+    inner = np.arange(128) % 16 != 0
+    for i in range(len(keys)):
+        part = near[i * 120:(i + 1) * 120]
+        keys[i, np.nonzero(inner)[0][:len(part)]] = part
+    got, want = gm.encode_keys(keys, 2), om.encode_batch(keys, 2)
+    assert got.tobytes() == want.tobytes(), _diff(got, want)
