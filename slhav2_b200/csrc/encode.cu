@@ -507,14 +507,22 @@ __device__ __forceinline__ bool signs_mma(const EncodeArgs& a, const float* buf,
     const uint32_t stride = (dp + 7) / 4 * 4, room = min((words - sign_fixed(KB)) / stride, (uint32_t)NT);  // (4 words over a multiple of 32: no bank conflicts)
     for (uint32_t e0 = 0; e0 < again; e0 += room) {
         const uint32_t n = min(room, again - e0);
-        for (uint32_t e = warp; e < n; e += WARPS) {
-            const float* z = a.z + (size_t)(list[e0 + e] & 255u) * dp;
+        // (eight rows a warp at a time: their numbers are read before the first copy is issued)
+        for (uint32_t e = warp; e < n; e += 8 * WARPS) {
+            uint32_t row[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) row[q] = e + q * WARPS < n ? (list[e0 + e + q * WARPS] & 255u) * dp : ~0u;
             if (dp % 4 == 0) {
                 const uint32_t to = (uint32_t)__cvta_generic_to_shared(zs + e * stride);
                 for (uint32_t i = 4 * lane; i < dp; i += 128)
-                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to + 4 * i), "l"(z + i) : "memory");
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (row[q] != ~0u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to + 4 * (q * WARPS * stride + i)), "l"(a.z + row[q] + i));
             } else {
-                for (uint32_t i = lane; i < dp; i += 32) zs[e * stride + i] = __ldg(z + i);
+                for (uint32_t i = lane; i < dp; i += 32)
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        if (row[q] != ~0u) zs[(e + q * WARPS) * stride + i] = __ldg(a.z + row[q] + i);
             }
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
@@ -525,13 +533,18 @@ __device__ __forceinline__ bool signs_mma(const EncodeArgs& a, const float* buf,
             const float* x = buf + key;
             float sum = 0.0f;
             uint32_t i = 0;
-#pragma unroll 4
-            for (; i + 4 <= dp; i += 4) {
-                const float4 z4 = *reinterpret_cast<const float4*>(z + i);
-                sum = __fadd_rn(sum, __fmul_rn(z4.x, x[(size_t)i * KS]));
-                sum = __fadd_rn(sum, __fmul_rn(z4.y, x[(size_t)(i + 1) * KS]));
-                sum = __fadd_rn(sum, __fmul_rn(z4.z, x[(size_t)(i + 2) * KS]));
-                sum = __fadd_rn(sum, __fmul_rn(z4.w, x[(size_t)(i + 3) * KS]));
+            for (; i + 32 <= dp; i += 32) {  // all products of a turn before its sums
+                float p[32];
+#pragma unroll
+                for (int j = 0; j < 32; j += 4) {
+                    const float4 z4 = *reinterpret_cast<const float4*>(z + i + j);
+                    p[j] = __fmul_rn(z4.x, x[(size_t)(i + j) * KS]);
+                    p[j + 1] = __fmul_rn(z4.y, x[(size_t)(i + j + 1) * KS]);
+                    p[j + 2] = __fmul_rn(z4.z, x[(size_t)(i + j + 2) * KS]);
+                    p[j + 3] = __fmul_rn(z4.w, x[(size_t)(i + j + 3) * KS]);
+                }
+#pragma unroll
+                for (int j = 0; j < 32; ++j) sum = __fadd_rn(sum, p[j]);
             }
             for (; i < dp; ++i) sum = __fadd_rn(sum, __fmul_rn(z[i], x[(size_t)i * KS]));
             if (sum < 0.0f) atomicOr(reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64) + (s >> 5), 1u << (s & 31u));
