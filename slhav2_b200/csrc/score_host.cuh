@@ -16,11 +16,6 @@ thread_local bool g_force_generic = false;
 struct Plan;
 thread_local const Plan* g_last_stream_plan = nullptr;  // the calling thread's latest tensor-core call (for its counters)
 
-size_t mma_smem_bytes(int nwarps, bool nf4_table) {  // (keep in step with the kernel's layout)
-    // nf4 table | stage ring | B fragments | sign words, thresholds, bucket mappings, flag
-    return (size_t)(nf4_table ? NF4_LUT_BYTES : 0) + (size_t)nwarps * MMA_DEPTH * MMA_SET_STRIDE + MMA_BQ_BYTES + 128 + 16 + 32 + 32 + 16;
-}
-constexpr int STREAM_THREADS = SLHA_STREAM_THREADS;
 // Tiles a CTA is given at least: two rounds of score_stream_kernel's 24 warps.  us per call with 512 / 768 / 2048: 4096 INT4 tiles,
 // one query 27.4 / 26.7 / 32.9; 8 segments x 2048 tiles 27.4 / 26.9 / 36.2; 4 x 32 768 TQ3 tiles 45.6 / 45.1 / 62.8.
 constexpr uint32_t STREAM_LEAST = 768;
@@ -40,10 +35,10 @@ Status launch_tc(Ctx* c, F* kernel, bool* configured, const ScoreArgs& a, uint32
     SLHA_CUDA(cudaGetLastError());
     return Status();
 }
-template <int KIND, bool IL>
+template <int KIND, bool IL, int U>
 Status launch_stream_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_stream_kernel<KIND, STREAM_THREADS, IL>, configured, a, grid, STREAM_THREADS, mma_smem_bytes(STREAM_THREADS / 32, KIND == 0));
+    return launch_tc(c, score_stream_kernel<KIND, IL, U>, configured, a, grid, stream_threads(KIND, U), stream_smem_bytes(KIND, U));
 }
 template <bool IL>
 Status launch_mix3(Ctx* c, const ScoreArgs& a, uint32_t grid) {
@@ -53,17 +48,17 @@ Status launch_mix3(Ctx* c, const ScoreArgs& a, uint32_t grid) {
 template <bool IL>
 Status launch_stream(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
     switch (kind) {
-        case 0: return launch_stream_t<0, IL>(c, a, grid);
-        case 1: return launch_stream_t<1, IL>(c, a, grid);
-        case 2: return launch_stream_t<2, IL>(c, a, grid);
-        case 3: return launch_stream_t<3, IL>(c, a, grid);
+        case 0: return launch_stream_t<0, IL, stream_sets(0, IL)>(c, a, grid);
+        case 1: return launch_stream_t<1, IL, stream_sets(1, IL)>(c, a, grid);
+        case 2: return launch_stream_t<2, IL, stream_sets(2, IL)>(c, a, grid);
+        case 3: return launch_stream_t<3, IL, stream_sets(3, IL)>(c, a, grid);
         default: return launch_mix3<IL>(c, a, grid);
     }
 }
-// tiles a warp takes at a time (also the slots it reserves at a time in a row's buffer), and warps of a CTA
-uint32_t stream_warp_tiles(int kind) { return kind == 4 ? ST_WT : MMA_SET_TILES; }
-uint32_t stream_warps(int kind) { return (uint32_t)(kind == 4 ? ST_THREADS : STREAM_THREADS) / 32; }
-static_assert(ST_CHUNK == ST_WT && MMA_CHUNK == MMA_SET_TILES, "a fresh chunk holds what a warp can append at once");
+// tiles a warp takes at a time, and warps of a CTA
+uint32_t stream_warp_tiles(int kind, bool il) { return kind == 4 ? ST_WT : (uint32_t)(MMA_SET_TILES * stream_sets(kind, il)); }
+uint32_t stream_warps(int kind, bool il) { return (uint32_t)(kind == 4 ? ST_THREADS : stream_threads(kind, stream_sets(kind, il))) / 32; }
+static_assert(ST_CHUNK == ST_WT, "a fresh chunk holds what a warp can append at once");
 Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
     return launch_tc(c, score_dense_kernel, configured, a, grid, ST_THREADS, st_smem_bytes(true));
@@ -307,7 +302,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
         p->use_mma = !g_force_generic;
         p->mma_grid = (uint32_t)sms;
     }
-    const uint32_t st_warps = stream_warps(p->kind), st_tiles = stream_warp_tiles(p->kind), st_unit = p->kind == 4 ? (uint32_t)ST_M : (uint32_t)MMA_SET_TILES;
+    const uint32_t st_unit = p->kind == 4 ? (uint32_t)ST_M : (uint32_t)MMA_SET_TILES;
 
     // Work items.  Generic kernel: fixed-size runs, large enough that candidate
     // traffic stays a few percent of the tile stream and small enough to balance
@@ -515,21 +510,25 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // the row's candidate buffer.  In random order about k (1 + ln(n / k)) tiles pass the rising threshold
     // plus the unfiltered first sets of every warp; 16 k slots (at most the longest segment) leave a wide
     // margin, and a row that fills its buffer all the same is scored by the generic kernel.
-    // (a warp reserves slots in chunks of 32 per row and work item, so up to 32 slots per warp and item stay unused)
+    // (a warp reserves slots in chunks of up to the tiles it takes at a time, so up to that many per warp and item stay unused)
     uint32_t longest = 0;
     for (size_t i = 0; i < n_segs; ++i) longest = std::max(longest, segs[i].n_tiles);
+    const uint32_t st_warps = stream_warps(p->kind, !stream_items.empty()), st_tiles = stream_warp_tiles(p->kind, !stream_items.empty());
     const uint64_t all_of_a_row = (uint64_t)longest + (uint64_t)st_tiles * st_warps * p->max_parts + 64;
-    // (the first set of every warp that scans a row is appended unfiltered: 32 slots per warp and item, twice over)
+    // (the first set of every warp that scans a row is appended unfiltered: its tiles per warp and item, twice over)
     const uint64_t first_sets = (uint64_t)(2 * st_tiles) * st_warps * p->max_parts;
-    p->gcap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(std::max<uint64_t>(16ull * k, 4096), first_sets + 4ull * k), all_of_a_row / 64 * 64);
+    uint32_t expect = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(std::max<uint64_t>(16ull * k, 4096), first_sets + 4ull * k), all_of_a_row / 64 * 64);
+    // Scores that rise along a long segment bring more (18 to 23 k slots for k = 1024 of 524 288 mixed tiles, 16 k + 10 % of which sent four of
+    // 32 rows to the generic kernel: 1860 us instead of 184), so rows have up to 64 k slots where all rows' together stay within 64 MB.
+    p->gcap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(expect, std::min<uint64_t>(65536, (8ull << 20) / nq)), all_of_a_row / 64 * 64);
     // (wide scoring: the first 128-tile block of every item is appended unfiltered, and a CTA sees few blocks)
-    if (p->wide) p->gcap = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(p->gcap, 4ull * WIDE_M * wide_parts + 16ull * k), ((uint64_t)longest + 63) / 64 * 64);
+    if (p->wide) p->gcap = expect = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(expect, 4ull * WIDE_M * wide_parts + 16ull * k), ((uint64_t)longest + 63) / 64 * 64);
     p->gstate_bytes = nq * (1024 + 8 + 8 + 4 + 4 + 4 + 8);  // histogram, threshold, mapping, count, flag, compacted count, statistics
     p->state_clean = false;
     p->late_threshold = p->use_mma && total / (uint64_t)sms < 4096;
     // few rows with long buffers: several CTAs per row compact the survivors before the merge
     // (a slice of at most 1024 slots per CTA: one round of four keys per thread)
-    p->compact_splits = (p->use_mma && nq < 128 && p->gcap >= 8192) ? (uint32_t)std::min<size_t>(64, std::max<size_t>((296 + nq - 1) / nq, (p->gcap + 1023) / 1024)) : 0;
+    p->compact_splits = (p->use_mma && nq < 128 && expect >= 8192) ? (uint32_t)std::min<size_t>(64, std::max<size_t>((296 + nq - 1) / nq, (expect + 1023) / 1024)) : 0;
     p->selcap = merge_cap((uint64_t)p->gcap, p->kp2, k);
     if (p->compact_splits) SLHA_TRY(p->b_gsel.ensure(nq * (size_t)p->selcap * 8));
     SLHA_TRY(p->b_gpivot.ensure(p->gstate_bytes));

@@ -27,20 +27,32 @@ namespace slha {
 namespace {
 
 constexpr int MMA_SET_TILES = 16;
-constexpr int MMA_SET_BYTES = MMA_SET_TILES * TILE_BYTES;  // 2 KiB of tiles in global memory
 constexpr int MMA_ROW = TILE_BYTES + 16;                   // padded row of the staging ring
-constexpr int MMA_SET_STRIDE = MMA_SET_TILES * MMA_ROW;    // one staged set
 constexpr int MMA_HALF = 8 * MMA_ROW;                      // row g -> row g + 8
 #ifndef SLHA_MMA_DEPTH
 #define SLHA_MMA_DEPTH 2
 #endif
 constexpr uint32_t MMA_CHUNK = 16;  // slots a warp reserves at a time in a row's candidate buffer (larger chunks measured no faster)
-#ifndef SLHA_STREAM_THREADS
-#define SLHA_STREAM_THREADS 768  // 24 warps at 80 registers: the streaming kernel hides its latencies with warps
+// score_stream_kernel: a warp takes sets of U x 16 tiles.  Shared layout: query fragments, sign words, thresholds (the tail) | stage ring, and
+// for launches with NF4 tiles (KIND 0) tail | ring of the first warps | NF4 table at 64 KB | ring of the others.
+#ifndef SLHA_U12
+#define SLHA_U12 2
 #endif
+constexpr int stream_sets(int kind, bool il) { return il || kind == 0 ? 1 : (kind == 3 ? 2 : SLHA_U12); }
+constexpr int stream_threads(int kind, int u) { return 768; }
 constexpr int MMA_DEPTH = SLHA_MMA_DEPTH;                  // cp.async ring slots per warp
 constexpr int MMA_BQ_BYTES = 9 * 32 * 8;                   // B fragments of a work item: [9][32 lanes] x 8 bytes
-constexpr int NF4_LUT_BYTES = 256 * 16 * 8;                // [byte][16 lanes] x (hi pair, lo pair)
+constexpr int MMA_TAIL_BYTES = 2560;                       // fragments | sign words 128 | thresholds 16 | bucket mappings 32 + 32 | flag 16
+constexpr int STREAM_LUT_BYTES = 256 * 32 * 8;             // NF4 table: [byte][32 lanes] x (hi pair, lo pair)
+constexpr uint32_t STREAM_LUT_AT = 0x10000;                // its shared-memory address
+constexpr int stream_slot(int u) { return MMA_DEPTH * u * MMA_SET_TILES * MMA_ROW; }  // a warp's ring
+constexpr int stream_low_warps(int u) { return ((int)STREAM_LUT_AT - 2048 - MMA_TAIL_BYTES) / stream_slot(u); }  // (dynamic shared memory starts below 2 KB)
+constexpr size_t stream_smem_bytes(int kind, int u) {
+    const int warps = stream_threads(kind, u) / 32;
+    if (kind != 0) return MMA_TAIL_BYTES + (size_t)warps * stream_slot(u);
+    return STREAM_LUT_AT + STREAM_LUT_BYTES + (size_t)(warps > stream_low_warps(u) ? warps - stream_low_warps(u) : 0) * stream_slot(u);
+}
+constexpr int NF4_LUT_BYTES = 256 * 16 * 8;                // score_dense_kernel: [byte][16 lanes] x (hi pair, lo pair)
 constexpr int SEL_HIST_INTS = 4 * 256 + 48;                // block_select_multi: 4 histograms + state
 
 #ifdef SLHA_STREAM_PROBE
@@ -169,127 +181,153 @@ __device__ __forceinline__ int popc8(const uint4& a, const uint4& b, const uint3
            __popc(b.x ^ q[4]) + __popc(b.y ^ q[5]) + __popc(b.z ^ q[6]) + __popc(b.w ^ q[7]);
 }
 
-// Coarse sums of one 16-tile set for rows g (acc0) and g+8 (acc1), query t.
+// Pairs of float32 (sm_100's f32x2): each half rounds like the scalar operation
+__device__ __forceinline__ uint64_t f2_pack(float lo, float hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_add(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;\n" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Coarse sums of U sub-sets of 16 tiles for rows g + 16 u (low half of acc[u]) and g + 8 + 16 u (high half), query t.
 // hb = shared address of row g of the set + 2t: halfword t of every 8-byte scale
 // group holds the four nibbles this thread feeds to the MMA of that group.
 // MODE 0: every row uniform INT4, 1: every row NF4, 2: per-row choice, 3: every row mixed 8/4
 // (group 0 holds the eight 8-bit head levels, halfword t = dims 2t and 2t+1, which fill k slots
 // 2t and 2t+1 as byte - 128 while slots 2t+8 and 2t+9 stay empty; groups 1..7 are INT4 groups of
 // dims 16 J - 8 ..; the B operand is arranged to match when the launch scores mixed tiles).
-template <int MODE, int J>
-__device__ __forceinline__ void coarse_group(uint32_t hb, uint32_t lut_lane, uint32_t magic, uint32_t bqa, uint32_t f0,
-                                             uint32_t f1, const uint4& x0, const uint4& x1, float& acc0, float& acc1) {
+// lut: shared address of this lane's column of the NF4 table, whose entry of byte b lies 256 b further (the table starts at a multiple of
+// 64 KB, so that one byte permutation makes an entry's address).
+template <int MODE, int J, int U>
+__device__ __forceinline__ void coarse_group(uint32_t hb, uint32_t lut, uint32_t magic, uint32_t bqa, const uint32_t (&f)[2 * U],
+                                             const uint2 (&gs)[2 * U], uint64_t (&acc)[U]) {
     const uint2 bq = lds_v2<256 * J>(bqa);  // this lane's B fragment of group J
-    const uint32_t h0 = lds_u16<8 * J>(hb), h1 = lds_u16<8 * J + MMA_HALF>(hb);
-    uint32_t a0, a1, a2, a3, l0 = 0, l1 = 0, l2 = 0, l3 = 0;
-    const bool n0 = MODE == 1 || (MODE == 2 && (f0 & F_NF4));
-    const bool n1 = MODE == 1 || (MODE == 2 && (f1 & F_NF4));
-    (void)n0;
-    (void)n1;
-    if (MODE == 3 && J == 0) {
-        // bytes (b0, b1) -> half2 (1024 + b0, 1024 + b1) - 1152
-        asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(a0) : "r"(prmt(h0, magic, 0x7150u)), "r"(0xE480E480u));
-        asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(a1) : "r"(prmt(h1, magic, 0x7150u)), "r"(0xE480E480u));
-        a2 = 0u;
-        a3 = 0u;
-    } else {
-    if (MODE != 0 && n0) {
-        // table entry of byte b at lut_lane + 128 b
-        const uint2 e0 = lds_v2<0>(lut_lane + ((h0 & 0xFFu) << 7));
-        const uint2 e1 = lds_v2<0>(lut_lane + ((h0 >> 8) << 7));
-        a0 = e0.x; a2 = e1.x; l0 = e0.y; l2 = e1.y;
-    } else {
-        int4_quad(h0, magic, a0, a2);
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+        const uint32_t rb = hb + (uint32_t)(2 * u * MMA_HALF);
+        const uint32_t h0 = lds_u16<8 * J>(rb), h1 = lds_u16<8 * J + MMA_HALF>(rb);
+        uint32_t a0, a1, a2, a3, l0 = 0, l1 = 0, l2 = 0, l3 = 0;
+        if (MODE == 3 && J == 0) {
+            // bytes (b0, b1) -> half2 (1024 + b0, 1024 + b1) - 1152
+            asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(a0) : "r"(prmt(h0, magic, 0x7150u)), "r"(0xE480E480u));
+            asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(a1) : "r"(prmt(h1, magic, 0x7150u)), "r"(0xE480E480u));
+            a2 = 0u;
+            a3 = 0u;
+        } else {
+            if (MODE == 1 || (MODE == 2 && (f[2 * u] & F_NF4))) {
+                const uint2 e0 = lds_v2<0>(prmt(h0, lut, 0x7604u)), e1 = lds_v2<0>(prmt(h0, lut, 0x7614u));
+                a0 = e0.x; a2 = e1.x; l0 = e0.y; l2 = e1.y;
+            } else {
+                int4_quad(h0, magic, a0, a2);
+            }
+            if (MODE == 1 || (MODE == 2 && (f[2 * u + 1] & F_NF4))) {
+                const uint2 e0 = lds_v2<0>(prmt(h1, lut, 0x7604u)), e1 = lds_v2<0>(prmt(h1, lut, 0x7614u));
+                a1 = e0.x; a3 = e1.x; l1 = e0.y; l3 = e1.y;
+            } else {
+                int4_quad(h1, magic, a1, a3);
+            }
+        }
+        float d[4];
+        mma_f16_zero(d, a0, a1, a2, a3, bq.x, bq.y);
+        if (MODE == 1 || MODE == 2) mma_f16(d, l0, l1, l2, l3, bq.x, bq.y);
+        // gs[J] as float (on the ALU / FMA pipes: 2^23 + b as a bit pattern, minus 2^23)
+        const uint32_t gw0 = J < 4 ? gs[2 * u].x : gs[2 * u].y, gw1 = J < 4 ? gs[2 * u + 1].x : gs[2 * u + 1].y;
+        const uint64_t g2 = f2_add(f2_pack(__uint_as_float(__byte_perm(gw0, 0x4B000000u, 0x7440 + (J & 3))),
+                                           __uint_as_float(__byte_perm(gw1, 0x4B000000u, 0x7440 + (J & 3)))),
+                                   0xCB000000CB000000ull);
+        acc[u] = f2_fma(f2_pack(d[0] + d[1], d[2] + d[3]), g2, acc[u]);
     }
-    if (MODE != 0 && n1) {
-        const uint2 e0 = lds_v2<0>(lut_lane + ((h1 & 0xFFu) << 7));
-        const uint2 e1 = lds_v2<0>(lut_lane + ((h1 >> 8) << 7));
-        a1 = e0.x; a3 = e1.x; l1 = e0.y; l3 = e1.y;
-    } else {
-        int4_quad(h1, magic, a1, a3);
-    }
-    }
-    float d[4];
-    mma_f16_zero(d, a0, a1, a2, a3, bq.x, bq.y);
-    if (MODE == 1 || MODE == 2) mma_f16(d, l0, l1, l2, l3, bq.x, bq.y);
-    // gs[J] as float: byte J of (x.z, x.w)
-    const uint32_t gw0 = J < 4 ? x0.z : x0.w, gw1 = J < 4 ? x1.z : x1.w;
-    // (byte -> float on the ALU / FMA pipes: 2^23 + b as a bit pattern, minus 2^23)
-    acc0 = fmaf(d[0] + d[1], __uint_as_float(__byte_perm(gw0, 0x4B000000u, 0x7440 + (J & 3))) - 8388608.0f, acc0);
-    acc1 = fmaf(d[2] + d[3], __uint_as_float(__byte_perm(gw1, 0x4B000000u, 0x7440 + (J & 3))) - 8388608.0f, acc1);
 }
 
-template <int MODE>
-__device__ __forceinline__ void coarse_set(uint32_t hb, uint32_t lut_lane, uint32_t magic, uint32_t bq, uint32_t f0,
-                                           uint32_t f1, const uint4& x0, const uint4& x1, float& acc0, float& acc1) {
-    acc0 = 0.0f;
-    acc1 = 0.0f;
-    coarse_group<MODE, 0>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 1>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 2>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 3>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 4>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 5>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 6>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
-    coarse_group<MODE, 7>(hb, lut_lane, magic, bq, f0, f1, x0, x1, acc0, acc1);
+template <int MODE, int U>
+__device__ __forceinline__ void coarse_set(uint32_t hb, uint32_t lut, uint32_t magic, uint32_t bq, const uint32_t (&f)[2 * U],
+                                           const uint2 (&gs)[2 * U], float (&out)[2 * U]) {
+    uint64_t acc[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) acc[u] = 0ull;
+    coarse_group<MODE, 0, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 1, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 2, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 3, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 4, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 5, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 6, U>(hb, lut, magic, bq, f, gs, acc);
+    coarse_group<MODE, 7, U>(hb, lut, magic, bq, f, gs, acc);
+#pragma unroll
+    for (int u = 0; u < U; ++u) asm("mov.b64 {%0, %1}, %2;\n" : "=f"(out[2 * u]), "=f"(out[2 * u + 1]) : "l"(acc[u]));
 }
 
 // ---- launches that hold only INT4 / MX-INT4 tiles (KIND 3) --------------------------------
-// Thread (g, t) of the warp owns the 16 latent bytes 16t..16t+15 of rows g and g+8: dims
+// Thread (g, t) of the warp owns the 16 latent bytes 16t..16t+15 of its rows: dims
 // 32t..32t+31, i.e. the two scale groups 2t and 2t+1, fetched with one 16-byte load per row.
-// The group scale is folded into the A operand, so the eight MMAs of a set chain on one
-// accumulator and nothing is scaled per group afterwards:
-//   a nibble n masked in place at bits 4..7 of a 16-bit half is the fp16 value n * 2^-20;
-//   fma(n * 2^-20, gs * 2^8, -8 gs * 2^-12) = (n - 8) gs * 2^-12, exact: |(n - 8) gs| <= 2040
-//   has 11 significant bits and the result is a normal fp16 number (>= 2^-12).
+// The group scale is folded into the A operand, so the eight MMAs of a set chain on two
+// accumulators and nothing is scaled per group afterwards:
+//   a nibble n masked in place at bits 0..3 of a 16-bit half is the fp16 value n * 2^-24, at bits 4..7 n * 2^-20;
+//   fma(n * 2^-24, gs * 2^8, -8 gs * 2^-16) = fma(n * 2^-20, gs * 2^4, ..) = (n - 8) gs * 2^-16, exact: |(n - 8) gs| <= 2040
+//   has 11 significant bits and is a multiple of 2^-24 (one shift per word of eight nibbles; with the nibbles all brought to bits 4..7 it took three).
 // k slot pairs (2t, 2t+1) / (2t+8, 2t+9) of MMA 2i take nibbles (0, 4) / (1, 5) of the
 // thread's word i, those of MMA 2i+1 nibbles (2, 6) / (3, 7); the B fragments carry the
-// queries' dims in the same order.  Sum = 2^-12 sum_d level_d gs_g q_d.
-__device__ __forceinline__ void int4c_scales(uint32_t h, uint32_t magic, uint32_t& G0, uint32_t& C0, uint32_t& G1, uint32_t& C1) {
-    // h = the two scale bytes (groups 2t, 2t+1) -> half2 (gs * 256) twice and (-gs * 2^-9) twice
-    uint32_t b0, b1;
-    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(b0) : "r"(prmt(h, magic, 0x5050u)), "r"(0xE400E400u));
-    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(b1) : "r"(prmt(h, magic, 0x5151u)), "r"(0xE400E400u));
-    asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(G0) : "r"(b0), "r"(0x5C005C00u));
-    asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(C0) : "r"(b0), "r"(0x98009800u));
-    asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(G1) : "r"(b1), "r"(0x5C005C00u));
-    asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(C1) : "r"(b1), "r"(0x98009800u));
+// queries' dims in the same order.  Sum = 2^-16 sum_d level_d gs_g q_d.
+struct Int4Scale {
+    uint32_t lo, hi, c;  // half2 (gs * 2^8), (gs * 2^4), (-gs * 2^-13), twice each
+};
+__device__ __forceinline__ Int4Scale int4c_scale(uint32_t h, uint32_t magic, uint32_t sel) {  // sel: which byte of h
+    const uint32_t p = prmt(h, magic, sel);  // 1024 + gs
+    Int4Scale s;
+    s.hi = hfma2_u32(p, 0x4C004C00u, 0xF400F400u);  // 16 p - 16384
+    s.c = hfma2_u32(p, 0x88008800u, 0x30003000u);   // -2^-13 p + 2^-3
+    asm("mul.rn.f16x2 %0, %1, %2;\n" : "=r"(s.lo) : "r"(s.hi), "r"(0x4C004C00u));
+    return s;
 }
-__device__ __forceinline__ void int4c_word(uint32_t w, uint32_t G, uint32_t C, uint32_t (&o)[4]) {
-    o[0] = hfma2_u32((w << 4) & 0x00F000F0u, G, C);  // nibbles 0, 4
-    o[1] = hfma2_u32(w & 0x00F000F0u, G, C);         // nibbles 1, 5
-    o[2] = hfma2_u32((w >> 4) & 0x00F000F0u, G, C);  // nibbles 2, 6
-    o[3] = hfma2_u32((w >> 8) & 0x00F000F0u, G, C);  // nibbles 3, 7
+__device__ __forceinline__ void int4c_word(uint32_t w, const Int4Scale& s, uint32_t (&o)[4]) {
+    const uint32_t v = w >> 8;
+    o[0] = hfma2_u32(w & 0x000F000Fu, s.lo, s.c);  // nibbles 0, 4
+    o[1] = hfma2_u32(w & 0x00F000F0u, s.hi, s.c);  // nibbles 1, 5
+    o[2] = hfma2_u32(v & 0x000F000Fu, s.lo, s.c);  // nibbles 2, 6
+    o[3] = hfma2_u32(v & 0x00F000F0u, s.hi, s.c);  // nibbles 3, 7
 }
 // rb = shared address of row g of the staged set; t = lane & 3
-__device__ __forceinline__ void coarse_set_int4c(uint32_t rb, uint32_t t, uint32_t magic, uint32_t bqa, float& acc0, float& acc1) {
+template <int U>
+__device__ __forceinline__ void coarse_set_int4c(uint32_t rb, uint32_t t, uint32_t magic, uint32_t bqa, float (&out)[2 * U]) {
     const uint32_t cb = rb + 16u * t, hb = rb + 2u * t;
-    const uint4 L0 = lds_v4<0>(cb), L1 = lds_v4<MMA_HALF>(cb);
-    const uint32_t h0 = lds_u16<120>(hb), h1 = lds_u16<120 + MMA_HALF>(hb);
-    uint32_t G00, C00, G01, C01, G10, C10, G11, C11;
-    int4c_scales(h0, magic, G00, C00, G01, C01);
-    int4c_scales(h1, magic, G10, C10, G11, C11);
-    const uint32_t w0[4] = {L0.x, L0.y, L0.z, L0.w}, w1[4] = {L1.x, L1.y, L1.z, L1.w};
-    // two accumulator chains (even / odd MMAs) halve the dependent MMA latency of a set
-    float d[4], e[4];
     const uint2 b0 = lds_v2<0>(bqa), b1 = lds_v2<256>(bqa), b2 = lds_v2<512>(bqa), b3 = lds_v2<768>(bqa);
     const uint2 b4 = lds_v2<1024>(bqa), b5 = lds_v2<1280>(bqa), b6 = lds_v2<1536>(bqa), b7 = lds_v2<1792>(bqa);
     const uint2 bq[8] = {b0, b1, b2, b3, b4, b5, b6, b7};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        uint32_t o0[4], o1[4];
-        int4c_word(w0[i], i < 2 ? G00 : G01, i < 2 ? C00 : C01, o0);
-        int4c_word(w1[i], i < 2 ? G10 : G11, i < 2 ? C10 : C11, o1);
-        if (i == 0) {
-            mma_f16_zero(d, o0[0], o1[0], o0[1], o1[1], bq[0].x, bq[0].y);
-            mma_f16_zero(e, o0[2], o1[2], o0[3], o1[3], bq[1].x, bq[1].y);
-        } else {
-            mma_f16(d, o0[0], o1[0], o0[1], o1[1], bq[2 * i].x, bq[2 * i].y);
-            mma_f16(e, o0[2], o1[2], o0[3], o1[3], bq[2 * i + 1].x, bq[2 * i + 1].y);
+    for (int u = 0; u < U; ++u) {
+        const uint32_t cu = cb + (uint32_t)(2 * u * MMA_HALF), hu = hb + (uint32_t)(2 * u * MMA_HALF);
+        const uint4 L0 = lds_v4<0>(cu), L1 = lds_v4<MMA_HALF>(cu);
+        const uint32_t h0 = lds_u16<120>(hu), h1 = lds_u16<120 + MMA_HALF>(hu);
+        const Int4Scale s0[2] = {int4c_scale(h0, magic, 0x5050u), int4c_scale(h0, magic, 0x5151u)};
+        const Int4Scale s1[2] = {int4c_scale(h1, magic, 0x5050u), int4c_scale(h1, magic, 0x5151u)};
+        const uint32_t w0[4] = {L0.x, L0.y, L0.z, L0.w}, w1[4] = {L1.x, L1.y, L1.z, L1.w};
+        // two accumulator chains (even / odd MMAs) halve the dependent MMA latency of a set
+        float d[4], e[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            uint32_t o0[4], o1[4];
+            int4c_word(w0[i], s0[i >> 1], o0);
+            int4c_word(w1[i], s1[i >> 1], o1);
+            if (i == 0) {
+                mma_f16_zero(d, o0[0], o1[0], o0[1], o1[1], bq[0].x, bq[0].y);
+                mma_f16_zero(e, o0[2], o1[2], o0[3], o1[3], bq[1].x, bq[1].y);
+            } else {
+                mma_f16(d, o0[0], o1[0], o0[1], o1[1], bq[2 * i].x, bq[2 * i].y);
+                mma_f16(e, o0[2], o1[2], o0[3], o1[3], bq[2 * i + 1].x, bq[2 * i + 1].y);
+            }
         }
+        out[2 * u] = (d[0] + e[0]) + (d[1] + e[1]);
+        out[2 * u + 1] = (d[2] + e[2]) + (d[3] + e[3]);
     }
-    acc0 = (d[0] + e[0]) + (d[1] + e[1]);
-    acc1 = (d[2] + e[2]) + (d[3] + e[3]);
 }
 
 // four consecutive elements of a query row (a caller's query rows start at any float)
@@ -735,37 +773,44 @@ __device__ __forceinline__ unsigned long long final_threshold(const uint32_t* hi
 // work item's query rows, which the generic kernel then scores.
 // IL: the work items are interleaved shares of whole streams (see the planner); the plain instantiation keeps the
 // set arithmetic of contiguous ranges out of its loop.
-template <int KIND, int NT, bool IL>
-__global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
+// U: a warp takes U x 16 tiles at a time.  The kernel is bound by instruction issue, and what a set costs beside its sums (fetch, flags, votes, thresholds,
+// query fragments) is paid once for both halves of a set of 32.
+template <int KIND, bool IL, int U>
+__global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    constexpr int nwarps = stream_threads(KIND, U) / 32, R = 2 * U, SET_TILES = MMA_SET_TILES * U, SET_STRIDE = SET_TILES * MMA_ROW;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
-    // shared layout: nf4 table | stage ring | B fragments | query sign words | thresholds | bucket mappings | flag
-    const uint32_t lut_bytes = a.nf4_table ? NF4_LUT_BYTES : 0;  // the table is left out when no NF4 tile is expected
-    uint2* lut = reinterpret_cast<uint2*>(smem);
-    unsigned char* tail = smem + lut_bytes + (size_t)nwarps * MMA_DEPTH * MMA_SET_STRIDE;
-    uint2* bq_w = reinterpret_cast<uint2*>(tail);                        // [9][32]
-    uint32_t* qs_w = reinterpret_cast<uint32_t*>(tail + MMA_BQ_BYTES);   // [4][8]
+    uint2* bq_w = reinterpret_cast<uint2*>(smem);                        // [9][32]
+    uint32_t* qs_w = reinterpret_cast<uint32_t*>(smem + MMA_BQ_BYTES);   // [4][8]
     uint32_t* pvh = qs_w + 32;                                           // [4] score word of the row's threshold
     float2* rng = reinterpret_cast<float2*>(pvh + 4);                    // [4] (smin, inv), inv 0 = none yet
     float2* rmap = rng + 4;                                              // [4] (-smin * inv, inv): the same mapping as the hot path uses it
     int* bail = reinterpret_cast<int*>(rmap + 4);                        // [1]
     const uint32_t smem_s = (uint32_t)__cvta_generic_to_shared(smem);
-    const uint32_t stage_s = smem_s + lut_bytes + (uint32_t)warp * MMA_DEPTH * MMA_SET_STRIDE;
-    const uint32_t bqa = smem_s + lut_bytes + (uint32_t)nwarps * MMA_DEPTH * MMA_SET_STRIDE + (uint32_t)lane * 8u;
-    const uint32_t qsa = bqa - (uint32_t)lane * 8u + MMA_BQ_BYTES + (uint32_t)t * 32u;
+    const uint32_t bqa = smem_s + (uint32_t)lane * 8u;
+    const uint32_t qsa = smem_s + MMA_BQ_BYTES + (uint32_t)t * 32u;
+    constexpr int LOW = KIND == 0 ? stream_low_warps(U) : nwarps;
+    const uint32_t stage_s = warp < LOW ? smem_s + MMA_TAIL_BYTES + (uint32_t)warp * stream_slot(U) : STREAM_LUT_AT + STREAM_LUT_BYTES + (uint32_t)(warp - LOW) * stream_slot(U);
 
-    // NF4 codebook as fp16 hi + lo pairs per byte (two nibbles), 16 bank-aligned replicas
-    for (int e = tid; e < (a.nf4_table ? 256 * 16 : 0); e += blockDim.x) {
-        const int b = e >> 4;
-        const float c0 = c_nf4[b & 15], c1 = 16.0f * c_nf4[b >> 4];  // odd slots carry 16x (see int4_quad)
-        lut[e] = make_uint2(pack_half2(c0, c1), pack_half2(half_residual(c0), half_residual(c1)));
+    if (KIND == 0 && smem_s > 2048u) {  // (never: the layout above needs dynamic shared memory to start below 2 KB)
+        for (uint32_t i = a.cta_begin[blockIdx.x]; i < a.cta_begin[blockIdx.x + 1]; ++i)
+            if (tid < (int)a.stream_items[i].n_queries) a.gflag[a.stream_items[i].query_begin + tid] = 1u;
+        return;
     }
-    const uint32_t lut_lane = smem_s + (uint32_t)(lane & 15) * 8u;
+    if (KIND == 0) {
+        // NF4 codebook as fp16 hi + lo pairs per byte (two nibbles), a column for every lane
+        uint2* lut = reinterpret_cast<uint2*>(smem + (STREAM_LUT_AT - smem_s));
+        for (int e = tid; e < 256 * 32; e += 32 * nwarps) {
+            const int b = e >> 5;
+            const float c0 = c_nf4[b & 15], c1 = 16.0f * c_nf4[b >> 4];  // odd slots carry 16x (see int4_quad)
+            lut[e] = make_uint2(pack_half2(c0, c1), pack_half2(half_residual(c0), half_residual(c1)));
+        }
+    }
+    const uint32_t lut_lane = STREAM_LUT_AT + (uint32_t)lane * 8u;
     uint32_t magic;  // 1024.0h twice, opaque so that it stays in one register
     asm volatile("mov.u32 %0, 0x64006400;\n" : "=r"(magic));
-    // cp.async of a set: lane copies the 16-byte chunks lane, lane+32, lane+64, lane+96,
-    // i.e. chunk (lane & 7) of rows (lane >> 3) + {0, 4, 8, 12}
+    // cp.async of a set: lane copies the 16-byte chunks lane, lane+32, .., i.e. chunk (lane & 7) of rows (lane >> 3) + {0, 4, 8, ..}
     const uint32_t dst_lane = (uint32_t)((lane >> 3) * MMA_ROW + (lane & 7) * 16);
     const uint32_t row_lane = (uint32_t)g * MMA_ROW;
     const uint32_t lt_mask = (1u << lane) - 1u, t_mask = 0x11111111u << t;
@@ -785,8 +830,8 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
         // fragments are built.
         const uint8_t* sbase = a.state ? a.state + it.tile_begin : nullptr;
         const uint32_t n = it.n_tiles;
-        uint32_t n_sets = (n + MMA_SET_TILES - 1) / MMA_SET_TILES;
-        const uint32_t n_full = n / MMA_SET_TILES;
+        uint32_t n_sets = (n + SET_TILES - 1) / SET_TILES;
+        const uint32_t n_full = n / SET_TILES;
         const bool mine = t < nq;
         const uint32_t Qt = it.query_begin + (mine ? (uint32_t)t : 0u);  // the row whose scores this thread finishes
         uint64_t* const dst = a.gbuf + (size_t)Qt * a.gcap;                // the row's candidate buffer
@@ -812,23 +857,30 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             ++iss_no;
             if (s_next < n_sets) {
                 const uint32_t dst = stage_s + slot_next + dst_lane;
-                const unsigned char* src = tbase + (size_t)s_next * MMA_SET_BYTES;
+                const unsigned char* src = tbase + (size_t)s_next * (SET_TILES * TILE_BYTES);
                 if (s_next < n_full) {
                     cp_async16_sp<0, 0>(dst, src, 16, stream_policy);
                     cp_async16_sp<512, 4 * MMA_ROW>(dst, src, 16, stream_policy);
                     cp_async16_sp<1024, 8 * MMA_ROW>(dst, src, 16, stream_policy);
                     cp_async16_sp<1536, 12 * MMA_ROW>(dst, src, 16, stream_policy);
+                    if (U == 2) {
+                        cp_async16_sp<2048, 16 * MMA_ROW>(dst, src, 16, stream_policy);
+                        cp_async16_sp<2560, 20 * MMA_ROW>(dst, src, 16, stream_policy);
+                        cp_async16_sp<3072, 24 * MMA_ROW>(dst, src, 16, stream_policy);
+                        cp_async16_sp<3584, 28 * MMA_ROW>(dst, src, 16, stream_policy);
+                    }
                 } else {
                     // ragged last set: rows past the end are zero-filled (source not read)
-                    const uint32_t r = s_next * MMA_SET_TILES + (uint32_t)(lane >> 3);
-                    cp_async16_s<0, 0>(dst, r < n ? src : a.tiles, r < n ? 16 : 0);
-                    cp_async16_s<0, 4 * MMA_ROW>(dst, r + 4 < n ? src + 512 : a.tiles, r + 4 < n ? 16 : 0);
-                    cp_async16_s<0, 8 * MMA_ROW>(dst, r + 8 < n ? src + 1024 : a.tiles, r + 8 < n ? 16 : 0);
-                    cp_async16_s<0, 12 * MMA_ROW>(dst, r + 12 < n ? src + 1536 : a.tiles, r + 12 < n ? 16 : 0);
+                    const uint32_t r = s_next * SET_TILES + (uint32_t)(lane >> 3);
+#pragma unroll 1
+                    for (uint32_t q = 0; q < 4u * U; ++q) {
+                        const bool in = r + 4u * q < n;
+                        cp_async16_s<0, 0>(dst + q * (4u * MMA_ROW), in ? src + 512u * q : a.tiles, in ? 16 : 0);
+                    }
                 }
             }
             cp_async_commit();
-            slot_next = slot_next == (MMA_DEPTH - 1) * MMA_SET_STRIDE ? 0u : slot_next + MMA_SET_STRIDE;
+            slot_next = slot_next == (MMA_DEPTH - 1) * SET_STRIDE ? 0u : slot_next + SET_STRIDE;
         };
 #pragma unroll
         for (int i = 0; i < MMA_DEPTH - 1; ++i) issue();
@@ -904,11 +956,11 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
         }
         // (from a barrier's vote, not from the flag word: a fast warp may raise the flag for an undecodable tile meanwhile)
         const bool too_big = __syncthreads_or(big) != 0;
-        // The barrier after the first round (below) pays when the round can supply k candidates to a row -- 16 per warp
+        // The barrier after the first round (below) pays when the round can supply k candidates to a row -- a set per warp
         // of every CTA that works on the row -- and the rows do not already have thresholds (a CTA that starts its
         // second item on rows other CTAs have been scoring for a while).
         const bool all_warm = __syncthreads_and(row_warm) != 0;
-        const bool first_round_barrier = !all_warm && (uint64_t)a.k <= 16ull * (uint64_t)nwarps * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
+        const bool first_round_barrier = !all_warm && (uint64_t)a.k <= (uint64_t)SET_TILES * (uint64_t)nwarps * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
         if (too_big) n_sets = 0;  // (the sets already on their way are waited for at the item's end and never read)
 
         uint32_t slot = 0, polls = 0;
@@ -919,7 +971,7 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             const uint32_t s = set_of(round);
             if (round == 1 && first_round_barrier) {
                 // Every warp of the CTA (and, started together, of the grid) has appended its first set
-                // unfiltered, so the rows' histograms hold 16 candidates per warp: first thresholds now,
+                // unfiltered, so the rows' histograms hold a set's candidates per warp: first thresholds now,
                 // before the second sets are filtered.  (All warps pass here: `rounds` is the same for all.)
                 __syncthreads();
                 if (warp < nq) stream_refresh_threshold(a, it.query_begin + (uint32_t)warp, rng[warp], pvh + warp, lane);
@@ -931,90 +983,122 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
             cp_async_wait<MMA_DEPTH - 1>();
             __syncwarp();
             const uint32_t rb = stage_s + slot + row_lane;
-            slot = slot == (MMA_DEPTH - 1) * MMA_SET_STRIDE ? 0u : slot + MMA_SET_STRIDE;
+            slot = slot == (MMA_DEPTH - 1) * SET_STRIDE ? 0u : slot + SET_STRIDE;
             if (dead || s >= n_sets) continue;
-            const uint2 m0 = lds_v2<96>(rb), m1 = lds_v2<96 + MMA_HALF>(rb);    // scale, lambda
-            const uint4 x0 = lds_v4<112>(rb), x1 = lds_v4<112 + MMA_HALF>(rb);  // position, head|flags, gs[8]
-            const uint32_t f0 = x0.y >> 16, f1 = x1.y >> 16;
-            const uint32_t fo = __reduce_or_sync(0xFFFFFFFFu, f0 | f1);
             const bool ragged = s >= n_full;
-            const uint32_t t0 = s * MMA_SET_TILES + (uint32_t)g, t1 = t0 + 8;
-            // a launch arranged for mixed 8/4 (TQ3) tiles takes nothing else (rows past the end of a ragged
-            // last set are zero-filled and their scores dropped, so they count as such tiles)
-            const bool all_mixed = KIND == 1 && (__reduce_and_sync(0xFFFFFFFFu, (t0 < n ? f0 : F_MIXED) & (t1 < n ? f1 : F_MIXED)) & F_MIXED);
-            const bool all_tq3 = KIND == 2 && (__reduce_and_sync(0xFFFFFFFFu, (t0 < n ? f0 : F_TQ3) & (t1 < n ? f1 : F_TQ3)) & F_TQ3);
-            if ((fo & F_MIX3) || ((fo & F_TQ3) && !all_tq3) || (KIND == 2 && !all_tq3) ||
-                ((fo & F_MIXED) && !all_mixed) || (KIND == 1 && !all_mixed) || ((fo & F_NF4) && (KIND == 3 || !a.nf4_table))) {
+            const uint32_t t0 = s * SET_TILES + (uint32_t)g;  // row r of this thread is tile t0 + 8 r
+            uint32_t f[R], fo = 0, fa = 0xFFFFFFFFu;
+            uint2 gs[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                if (KIND == 3) {
+                    f[r] = lds_u16<118>(rb + (uint32_t)(r * MMA_HALF));
+                } else {
+                    const uint4 x = lds_v4<112>(rb + (uint32_t)(r * MMA_HALF));  // position, head|flags, gs[8]
+                    f[r] = x.y >> 16;
+                    gs[r] = make_uint2(x.z, x.w);
+                }
+                fo |= f[r];
+                // (rows past the end of a ragged last set are zero-filled and their scores dropped: they count as tiles of the launch's codec)
+                if (KIND == 1 || KIND == 2) fa &= !ragged || t0 + 8u * r < n ? f[r] : 0xFFFFFFFFu;
+                if (KIND == 0) fa &= f[r];
+            }
+            fo = __reduce_or_sync(0xFFFFFFFFu, fo);
+            if (KIND != 3) fa = __reduce_and_sync(0xFFFFFFFFu, fa);
+            // a launch arranged for mixed 8/4 (TQ3) tiles takes nothing else
+            const bool odd = KIND == 3 ? (fo & (F_MIX3 | F_TQ3 | F_MIXED | F_NF4)) != 0
+                           : KIND == 2 ? (fo & (F_MIX3 | F_MIXED)) || !(fa & F_TQ3)
+                           : KIND == 1 ? (fo & (F_MIX3 | F_TQ3)) || !(fa & F_MIXED)
+                                       : (fo & (F_MIX3 | F_TQ3 | F_MIXED)) != 0;
+            if (odd) {
                 if (lane == 0) bail[0] = 1;  // a codec this launch does not decode: the generic kernel takes the rows
                 dead = true;
                 continue;
             }
-            float acc0, acc1;
+            float c[R];
             const uint32_t hb = rb + 2u * (uint32_t)t;
             if (KIND == 3) {
-                coarse_set_int4c(rb, (uint32_t)t, magic, bqa, acc0, acc1);
-            } else if (KIND == 2) {  // (all_tq3 holds here)
-                tq3_to_nibbles(rb - row_lane, lane);
-                coarse_set<0>(hb, lut_lane, magic, bqa, f0, f1, x0, x1, acc0, acc1);
+                coarse_set_int4c<U>(rb, (uint32_t)t, magic, bqa, c);
+            } else if (KIND == 2) {
+#pragma unroll
+                for (int u = 0; u < U; ++u) tq3_to_nibbles(rb - row_lane + (uint32_t)(2 * u * MMA_HALF), lane);
+                coarse_set<0, U>(hb, lut_lane, magic, bqa, f, gs, c);
                 // level = (2 nibble - 15) / 4, or (2 nibble - 14) / 4 without the correction plane:
                 // beside the nibble sums X the score needs 8 c sum_g gs_g Q_g (c = 1 or 2, Q_g = the
                 // query's sum over group g), one more MMA with the scale bytes as the A operand
                 const uint32_t sel = (t & 1) ? 0x7352u : 0x7150u;
-                uint32_t ga0, ga1;
-                asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(ga0) : "r"(prmt(t < 2 ? x0.z : x0.w, magic, sel)), "r"(0xE400E400u));
-                asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(ga1) : "r"(prmt(t < 2 ? x1.z : x1.w, magic, sel)), "r"(0xE400E400u));
-                float e[4];
-                mma_f16_zero(e, ga0, ga1, 0u, 0u, lds_v2<256 * 8>(bqa).x, 0u);
-                acc0 = fmaf((f0 & F_NOCORR) ? 16.0f : 8.0f, e[0] + e[1], acc0);
-                acc1 = fmaf((f1 & F_NOCORR) ? 16.0f : 8.0f, e[2] + e[3], acc1);
-            } else if (KIND == 1) {  // (all_mixed holds here)
-                coarse_set<3>(hb, lut_lane, magic, bqa, f0, f1, x0, x1, acc0, acc1);
+#pragma unroll
+                for (int u = 0; u < U; ++u) {
+                    uint32_t ga0, ga1;
+                    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(ga0) : "r"(prmt(t < 2 ? gs[2 * u].x : gs[2 * u].y, magic, sel)), "r"(0xE400E400u));
+                    asm("add.rn.f16x2 %0, %1, %2;\n" : "=r"(ga1) : "r"(prmt(t < 2 ? gs[2 * u + 1].x : gs[2 * u + 1].y, magic, sel)), "r"(0xE400E400u));
+                    float e[4];
+                    mma_f16_zero(e, ga0, ga1, 0u, 0u, lds_v2<256 * 8>(bqa).x, 0u);
+                    c[2 * u] = fmaf((f[2 * u] & F_NOCORR) ? 16.0f : 8.0f, e[0] + e[1], c[2 * u]);
+                    c[2 * u + 1] = fmaf((f[2 * u + 1] & F_NOCORR) ? 16.0f : 8.0f, e[2] + e[3], c[2 * u + 1]);
+                }
+            } else if (KIND == 1) {
+                coarse_set<3, U>(hb, lut_lane, magic, bqa, f, gs, c);
+            } else if (fa & F_NF4) {
+                coarse_set<1, U>(hb, lut_lane, magic, bqa, f, gs, c);
             } else if (!(fo & F_NF4)) {
-                coarse_set<0>(hb, lut_lane, magic, bqa, f0, f1, x0, x1, acc0, acc1);
-            } else if (__reduce_and_sync(0xFFFFFFFFu, f0 & f1) & F_NF4) {
-                coarse_set<1>(hb, lut_lane, magic, bqa, f0, f1, x0, x1, acc0, acc1);
+                coarse_set<0, U>(hb, lut_lane, magic, bqa, f, gs, c);
             } else {
-                coarse_set<2>(hb, lut_lane, magic, bqa, f0, f1, x0, x1, acc0, acc1);
+                coarse_set<2, U>(hb, lut_lane, magic, bqa, f, gs, c);
             }
-            const float lam0 = (f0 & F_WARM) ? 0.0f : __uint_as_float(m0.y);
-            const float lam1 = (f1 & F_WARM) ? 0.0f : __uint_as_float(m1.y);
-            // 1 / (255 x 16 [x 2]); KIND 3: the sums carry 2^-12
-            constexpr float unit = KIND == 3 ? 4096.0f / 255.0f : (KIND == 2 ? 1.0f / 8160.0f : 1.0f / 4080.0f);
-            const float c0 = acc0 * (__uint_as_float(m0.x) * unit), c1 = acc1 * (__uint_as_float(m1.x) * unit);
-            const uint32_t pv = reinterpret_cast<const volatile uint32_t*>(pvh)[t];
-            // The residual term lies in [-256 lambda, 256 lambda]: a set none of whose tiles can reach its
-            // row's threshold even with the largest term needs no Hamming distances (and appends nothing).
-            // (257 and the relative slack cover the rounding of the bound itself.)  Only the INT4 launches
-            // test for it: with a few CTAs per row and k / n of a few percent (the NF4 decode caches) nearly
-            // every set holds a candidate and the test costs more than it saves.
-            const bool need = KIND != 3 || round == 0 ||
-                              __any_sync(0xFFFFFFFFu, (mine && score_key(fmaf(lam0, 257.0f, c0 + fabsf(c0) * 1e-6f)) >= pv) ||
-                                                          (mine && score_key(fmaf(lam1, 257.0f, c1 + fabsf(c1) * 1e-6f)) >= pv));
-            if (need) {
-            // Hamming term of query t for both rows
-            int h0, h1;
-            {
-                const uint4 qa = lds_v4<0>(qsa), qb = lds_v4<16>(qsa);
-                const uint32_t qs[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
-                h0 = popc8(lds_v4<64>(rb), lds_v4<80>(rb), qs);
-                h1 = popc8(lds_v4<64 + MMA_HALF>(rb), lds_v4<80 + MMA_HALF>(rb), qs);
+            // 1 / (255 x 16 [x 2]); KIND 3: the sums carry 2^-16
+            constexpr float unit = KIND == 3 ? 65536.0f / 255.0f : (KIND == 2 ? 1.0f / 8160.0f : 1.0f / 4080.0f);
+            const float thr = thr_float(reinterpret_cast<const volatile uint32_t*>(pvh)[t]);
+            // The residual term lies in [-256 |lambda|, 256 |lambda|]: rows none of whose tiles can reach the threshold even with the largest
+            // term need no Hamming distances (and append nothing).  (257 and the relative slack cover the rounding of the bound
+            // itself; a NaN passes.)  INT4 launches ask for eight tiles at a time; the others, whose rows are mostly short beside
+            // k (a decode step's caches: one tile in seven is appended, and some tile of a set nearly always), for the set.
+            constexpr int GATE = KIND == 3 ? 1 : R;  // rows asked for at a time
+            float sc[R], lam[R];
+            uint32_t b[R], some = 0;
+            bool p[R];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const uint2 m = lds_v2<96>(rb + (uint32_t)(r * MMA_HALF));  // scale, lambda
+                lam[r] = (f[r] & F_WARM) ? 0.0f : __uint_as_float(m.y);
+                sc[r] = c[r] * (__uint_as_float(m.x) * unit);
+                p[r] = mine && !(fmaf(fabsf(lam[r]), 257.0f, fmaf(fabsf(sc[r]), 1e-6f, sc[r])) < thr);
+                b[r] = 0u;
             }
-            // 256 - 2 h without an integer conversion: (2^23 + h) as a bit pattern, times -2, plus 2^24 + 256 (exact)
-            const float x0f = fmaf(__uint_as_float(0x4B000000u | (uint32_t)h0), -2.0f, 16777472.0f);
-            const float x1f = fmaf(__uint_as_float(0x4B000000u | (uint32_t)h1), -2.0f, 16777472.0f);
-            const float sc0 = fmaf(lam0, x0f, c0);
-            const float sc1 = fmaf(lam1, x1f, c1);
-            bool live0 = mine && (!ragged || t0 < n), live1 = mine && (!ragged || t1 < n);
-            if (sbase) {
-                live0 = live0 && sbase[t0] != ST_COLD;
-                live1 = live1 && sbase[t1] != ST_COLD;
+#pragma unroll
+            for (int r0 = 0; r0 < R; r0 += GATE) {
+                bool any = false;
+#pragma unroll
+                for (int r = r0; r < r0 + GATE; ++r) any = any || p[r];
+                if (__any_sync(0xFFFFFFFFu, any)) {
+                    const uint4 qa = lds_v4<0>(qsa), qb = lds_v4<16>(qsa);
+                    const uint32_t qs[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+#pragma unroll
+                    for (int r = r0; r < r0 + GATE; ++r) {
+                        // Hamming term of query t for the row
+                        const uint32_t row = rb + (uint32_t)(r * MMA_HALF);
+                        const int h = popc8(lds_v4<64>(row), lds_v4<80>(row), qs);
+                        // 256 - 2 h without an integer conversion: (2^23 + h) as a bit pattern, times -2, plus 2^24 + 256 (exact)
+                        sc[r] = fmaf(lam[r], fmaf(__uint_as_float(0x4B000000u | (uint32_t)h), -2.0f, 16777472.0f), sc[r]);
+                        // (a superset of the composite comparison: the merge drops keys below the final threshold)
+                        p[r] = p[r] && !(sc[r] < thr) && (!ragged || t0 + 8u * r < n);
+                        if (sbase) p[r] = p[r] && sbase[t0 + 8u * r] != ST_COLD;
+                        b[r] = __ballot_sync(0xFFFFFFFFu, p[r]);
+                        some |= b[r];
+                    }
+                }
             }
             if (round == 0) {
-                // First set of the warp: a row without a bucket mapping gets one from the 16 scores
+                // First set of the warp: a row without a bucket mapping gets one from the scores
                 // this warp has just computed for it - their range widened by 1.5 spans on both sides.
                 // Any monotone mapping is valid; this one only has to put the final threshold somewhere
                 // inside its 256 buckets.  The first CTA to publish wins.
-                float mn = fminf(live0 ? sc0 : INFINITY, live1 ? sc1 : INFINITY), mx = fmaxf(live0 ? sc0 : -INFINITY, live1 ? sc1 : -INFINITY);
+                float mn = INFINITY, mx = -INFINITY;
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    mn = fminf(mn, p[r] ? sc[r] : INFINITY);
+                    mx = fmaxf(mx, p[r] ? sc[r] : -INFINITY);
+                }
 #pragma unroll
                 for (int o = 4; o < 32; o <<= 1) {
                     mn = fminf(mn, __shfl_xor_sync(0xFFFFFFFFu, mn, o));
@@ -1037,54 +1121,55 @@ __global__ void __launch_bounds__(NT, 1) score_stream_kernel(ScoreArgs a) {
                 }
                 __syncwarp();
             }
-            // filter on the score word alone (a superset of the composite comparison: the merge drops
-            // keys below the final threshold)
-            const uint32_t k0 = score_key(sc0), k1 = score_key(sc1);
-            const bool p0 = live0 && k0 >= pv, p1 = live1 && k1 >= pv;
-            if (__any_sync(0xFFFFFFFFu, p0 || p1)) {
+            if (some) {
                 // The eight lanes of query t append to the row's buffer, slots by ballot.  The warp owns a
-                // chunk of 16 slots per row, [cur, end), reserved with one atomic; a set brings at most 16
-                // candidates per row, so a fresh chunk always fits them.  The unused rest of a chunk is
-                // zeroed (an absent key) before the next one is taken and at the end of the work item.
-                const unsigned b0 = __ballot_sync(0xFFFFFFFFu, p0) & t_mask, b1 = __ballot_sync(0xFFFFFFFFu, p1) & t_mask;
-                const uint32_t n0 = (uint32_t)__popc(b0), nn = n0 + (uint32_t)__popc(b1);
-                if (cur + nn > end) {  // (the same in the eight lanes of a query, which are the lanes of t_mask)
-                    for (uint32_t z = cur + (uint32_t)g; z < end; z += 8u) dst[z] = 0ull;
+                // chunk of slots per row, [cur, end); a set that does not fit takes what is left of it and the start of a new chunk,
+                // reserved with one atomic.  What is unused at the end of the work item is zeroed (absent keys).
+                uint32_t nn = 0, first[R];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    first[r] = nn + (uint32_t)__popc(b[r] & t_mask & lt_mask);
+                    nn += (uint32_t)__popc(b[r] & t_mask);
+                }
+                const uint32_t left = end - cur;
+                uint32_t fresh = cur;  // where the candidates beyond `left` go, minus `left`
+                if (nn > left) {  // (the same in the eight lanes of a query, which are the lanes of t_mask)
+                    const uint32_t size = nn - left > MMA_CHUNK ? 2 * MMA_CHUNK : MMA_CHUNK;
                     uint32_t base = 0;
                     if (g == 0) {
-                        base = atomicAdd(a.gcount + Qt, MMA_CHUNK);
-                        if (base + MMA_CHUNK > a.gcap) {
+                        base = atomicAdd(a.gcount + Qt, size);
+                        if (base + size > a.gcap) {
                             // the row's buffer is full: the generic kernel scores the row; this warp's further
-                            // candidates of the row land in the buffer's last chunk, which nobody reads then
+                            // candidates of the row land in the buffer's last slots, which nobody reads then
                             a.gflag[Qt] = 1u;
-                            base = a.gcap - MMA_CHUNK;
+                            base = a.gcap - size;
                         }
                     }
-                    cur = __shfl_sync(t_mask, base, t);  // lane t is (g = 0, t)
-                    end = cur + MMA_CHUNK;
+                    base = __shfl_sync(t_mask, base, t);  // lane t is (g = 0, t)
+                    fresh = base - left;
+                    end = base + size;
                 }
                 // bucket of the row's histogram: (int)(score * inv - smin * inv), clamped; scores below the
                 // mapping (and all scores while the row has no mapping) count in bucket 0, which never decides
-                const float2 r = rmap[t];
-                if (p0) {
-                    dst[cur + (uint32_t)__popc(b0 & lt_mask)] = ((uint64_t)k0 << 32) | (uint64_t)(~(it.index_base + t0));
-                    atomicAdd(hrow + min(max(__float2int_rz(fmaf(sc0, r.y, r.x)), 0), 255), 1u);
+                const float2 map = rmap[t];
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    if (p[r]) {
+                        dst[(first[r] < left ? cur : fresh) + first[r]] = ((uint64_t)score_key(sc[r]) << 32) | (uint64_t)(~(it.index_base + t0 + 8u * r));
+                        atomicAdd(hrow + min(max(__float2int_rz(fmaf(sc[r], map.y, map.x)), 0), 255), 1u);
+                    }
                 }
-                if (p1) {
-                    dst[cur + n0 + (uint32_t)__popc(b1 & lt_mask)] = ((uint64_t)k1 << 32) | (uint64_t)(~(it.index_base + t1));
-                    atomicAdd(hrow + min(max(__float2int_rz(fmaf(sc1, r.y, r.x)), 0), 255), 1u);
-                }
-                cur += nn;
+                cur = nn > left ? fresh + nn : cur + nn;
             }
-            }  // need
             __syncwarp();
-            // In turn, a warp raises the threshold of query (warp & 3): after its 3rd and 7th set (the first
-            // thresholds come from the barrier after the first round), then every 16 sets, the warps of a
+            // In turn, a warp raises the threshold of query (warp & 3): early on (the first
+            // thresholds come from the barrier after the first round), then every 256 tiles, the warps of a
             // query staggered.  A stale threshold costs appends (each one a store, a
             // histogram count and, downstream, merge work), a refresh costs one 1 KB read of the row's
             // histogram by one warp.
             ++polls;
-            if ((polls & 15u) == (uint32_t)((warp >> 2) & 3) * 4u + 3u || polls == 3u || polls == 7u) {
+            constexpr uint32_t every = 16 / U;
+            if ((polls & (every - 1u)) == (uint32_t)((warp >> 2) & 3) * (every / 4u) + (every / 4u - 1u) || polls == 4u / U - (U == 1) || polls == 8u / U - (U == 1)) {
                 const int q = warp & 3;
                 if (q < nq) stream_refresh_threshold(a, it.query_begin + (uint32_t)q, rng[q], pvh + q, lane);
                 __syncwarp();
