@@ -7,6 +7,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 
 #include "../../include/slha_b200.h"
 
@@ -59,6 +60,28 @@ Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
 // The call under way uses a plan's buffers (kept per thread, like the scratch arena): waits for another stream's use of them, see LastUse.
 void ctx_uses_plans(Ctx* c);
 void count_launch(int n = 1);
+// A kernel launched beside the end of the one before it on the stream (programmatic dependent launch): its CTAs may be on their SMs while
+// the last ones of that kernel still run, and wait for it (dep_wait, before anything that kernel wrote is read or anything it reads is written).
+template <typename... P, typename... A>
+inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
+#ifdef __CUDACC__
+// Every thread of a kernel launched with launch_behind calls dep_wait, also in CTAs that have nothing to do: a kernel counts as finished
+// when its CTAs are, and the next but one may rely on it.  Without that attribute both do nothing.
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+__device__ __forceinline__ void dep_launch() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+#endif
 int sm_count(int device);  // multiprocessors of a device
 uint64_t launch_count();
 void tls_set_device(int dev);
@@ -158,6 +181,7 @@ Status launch_attend_topk(Ctx* c, const uint32_t* d_index, const float* d_score,
                           float scale, const void* d_values, int value_dtype, size_t d_v, size_t row_stride,
                           const uint64_t* d_row_base, float* d_out, float* d_weights);
 
+Status build_sign_fragments(Ctx* c, Model* m, uint4* d_zf, void* d_stats);  // fills d_zf from d_z and sets the model's sign members; synchronises
 Status launch_encode(Ctx* c, const Model* m, const void* d_keys, int key_dtype, size_t n,
                      const uint32_t* d_positions, uint32_t position_base, const uint16_t* d_heads,
                      int codec, SciRustSlhaTile* d_tiles, const uint32_t* d_slots);

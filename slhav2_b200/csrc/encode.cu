@@ -998,6 +998,42 @@ __global__ void decode_kernel(const unsigned char* tile, const float* p, const f
     }
 }
 
+// Z in fp16 as the B operand of m16n8k16 MMAs (columns = hyperplanes), every row scaled to the norm SIGN_NORM: lane (g, t) of a group of 8
+// hyperplanes holds k = 2 t, 2 t + 1 and 2 t + 8, 2 t + 9 of hyperplane g for two steps of 16 in one 16-byte word.  A CTA per
+// row; stats[row] = (norm of what the rounding lost, norm of what it kept), negative where the row is not of ordinary size.
+constexpr double SIGN_NORM = 16.0;
+__global__ void __launch_bounds__(128) sign_fragments_kernel(const float* z, uint32_t dp, uint32_t* out, float2* stats) {
+    __shared__ double part[4];
+    const uint32_t s = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const auto total = [&](double v) {
+        for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+        __syncthreads();
+        if (lane == 0) part[warp] = v;
+        __syncthreads();
+        return part[0] + part[1] + part[2] + part[3];
+    };
+    double n2 = 0.0, lost = 0.0, kept = 0.0;
+    for (uint32_t i = threadIdx.x; i < dp; i += 128) n2 += (double)z[(size_t)s * dp + i] * z[(size_t)s * dp + i];
+    n2 = total(n2);
+    const bool usual = n2 >= 1e-12 && n2 <= 1e12;  // (false for NaN)
+    const double scale = usual ? SIGN_NORM / sqrt(n2) : 0.0;
+    for (uint32_t i = 2 * threadIdx.x; i < sign_rows(dp); i += 256) {
+        uint32_t word = 0;
+        for (uint32_t h = 0; h < 2; ++h) {
+            const double x = i + h < dp && usual ? z[(size_t)s * dp + i + h] * scale : 0.0;
+            const __half r = __float2half_rn((float)x);
+            const double k = (double)__half2float(r), l = k - x;
+            kept += k * k;
+            lost += l * l;
+            word |= (uint32_t)__half_as_ushort(r) << (16 * h);
+        }
+        out[((i / 32 * 32 + s / 8) * 32 + 4 * (s % 8) + i / 2 % 4) * 4 + i / 8 % 4] = word;
+    }
+    lost = total(lost);
+    kept = total(kept);
+    if (threadIdx.x == 0) stats[s] = usual ? make_float2((float)sqrt(lost), (float)sqrt(kept)) : make_float2(-1.0f, -1.0f);
+}
+
 size_t encode_smem(uint32_t d_pad, int kb) {
     const size_t ks = (size_t)enc_row_stride(kb);
     return (((d_pad * ks + 3) & ~size_t(3)) + (size_t)kb * D_C + ks * D_C) * 4 + (size_t)kb * TILE_BYTES;
@@ -1067,6 +1103,28 @@ Status run_encode(Ctx* c, EncodeArgs& a) {
 }
 
 }  // namespace
+
+// No fragments (every sign from its exact sum) where the error bound of signs_mma does not hold: more than 256 dimensions, or rows far
+// from ordinary size.
+Status build_sign_fragments(Ctx* c, Model* m, uint4* d_zf, void* d_stats) {
+    float2 stats[D_S];
+    sign_fragments_kernel<<<D_S, 128, 0, c->stream>>>(m->d_z, (uint32_t)m->d_pad, reinterpret_cast<uint32_t*>(d_zf), static_cast<float2*>(d_stats));
+    count_launch();
+    SLHA_CUDA(cudaGetLastError());
+    SLHA_CUDA(cudaMemcpyAsync(stats, d_stats, sizeof stats, cudaMemcpyDeviceToHost, c->stream));
+    SLHA_CUDA(cudaStreamSynchronize(c->stream));
+    float lost = 0.0f, kept = 0.0f;
+    for (const float2& r : stats) {
+        if (!(r.y > 0.0f)) return Status();
+        lost = std::max(lost, r.x);
+        kept = std::max(kept, r.y);
+    }
+    // MMA accumulation and the reference's own sum: 2^-13.9 + 2^-16 of the norms' product; 2e-4 for the rounding of the bound itself
+    m->z_guard = (float)(1.0002 * (lost + (1.0 / 15286.0 + 1.0 / 65536.0) * SIGN_NORM));
+    m->z_norm = (float)(1.0002 * kept);
+    m->d_zf = d_zf;
+    return Status();
+}
 
 Status launch_encode(Ctx* c, const Model* m, const void* d_keys, int key_dtype, size_t n,
                      const uint32_t* d_positions, uint32_t position_base, const uint16_t* d_heads,

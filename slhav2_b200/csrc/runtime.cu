@@ -2,7 +2,6 @@
 // model construction (.slhw parsing, sign-LSH matrix generation) and registry.
 #include "runtime.cuh"
 
-#include <cuda_fp16.h>
 #include <sys/stat.h>
 
 #include <atomic>
@@ -412,42 +411,6 @@ void free_model(Model* m) {
     cudaFree(m->block);
     delete m;
 }
-// Z in fp16 as the B operand of m16n8k16 MMAs (columns = hyperplanes), every row scaled to the norm SIGN_NORM: lane (g, t) of a group of 8
-// hyperplanes holds k = 2 t, 2 t + 1 and 2 t + 8, 2 t + 9 of hyperplane g for two steps of 16 in one 16-byte word.  False (every sign from
-// its exact sum) where the error bound of signs_mma does not hold: more than 256 dimensions, or elements or rows far from ordinary size.
-constexpr double SIGN_NORM = 16.0;
-bool sign_fragments(const std::vector<float>& Z, size_t dp, uint32_t* out, float* guard, float* most) {
-    if (dp > 256) return false;
-    double lost = 0.0, kept = 0.0;  // largest |z - z'| and |z'| of any row
-    double scale[D_S];
-    for (size_t s = 0; s < (size_t)D_S; ++s) {
-        double n2 = 0.0;
-        for (size_t i = 0; i < dp; ++i) n2 += (double)Z[s * dp + i] * Z[s * dp + i];
-        if (!(n2 >= 1e-12 && n2 <= 1e12)) return false;
-        scale[s] = SIGN_NORM / std::sqrt(n2);
-    }
-    for (size_t s = 0; s < (size_t)D_S; ++s) {
-        uint16_t row[256] = {};
-        double l2 = 0.0, k2 = 0.0;
-        for (size_t i = 0; i < dp; ++i) {
-            const __half h = __float2half_rn((float)(Z[s * dp + i] * scale[s]));
-            std::memcpy(&row[i], &h, 2);
-            const double kept_i = __half2float(h), lost_i = kept_i - Z[s * dp + i] * scale[s];
-            l2 += lost_i * lost_i;
-            k2 += kept_i * kept_i;
-        }
-        lost = std::max(lost, std::sqrt(l2));
-        kept = std::max(kept, std::sqrt(k2));
-        for (size_t i = 0; i < (dp + 31) / 32 * 32; i += 2) {
-            const size_t lane = 4 * (s % 8) + i / 2 % 4, w = i / 8 % 4;
-            out[((i / 32 * 32 + s / 8) * 32 + lane) * 4 + w] = row[i] | (uint32_t)row[i + 1] << 16;
-        }
-    }
-    // MMA accumulation and the reference's own sum: 2^-13.9 + 2^-16 of the norms' product; 2e-4 for the rounding of the bound itself
-    *guard = (float)(1.0002 * (lost + (1.0 / 15286.0 + 1.0 / 65536.0) * SIGN_NORM));
-    *most = (float)(1.0002 * kept);
-    return true;
-}
 }  // namespace
 
 Status model_build(Ctx* c, const float* p, size_t d, uint64_t seed, bool rht, const float* scale,
@@ -495,7 +458,7 @@ Status model_build(Ctx* c, const float* p, size_t d, uint64_t seed, bool rht, co
     at[4] = at[3] + pad256(zb);
     at[5] = at[4] + pad256(zb);
     at[6] = at[5] + pad256(diag.size() * 4);
-    std::vector<unsigned char> blob(at[6] + (dp <= 256 ? zfb : 0));
+    std::vector<unsigned char> blob(at[6]);
     const auto put = [&](int i, const std::vector<float>& v) { if (!v.empty()) std::memcpy(blob.data() + at[i], v.data(), v.size() * 4); };
     put(0, P);
     put(1, Pt);
@@ -503,9 +466,8 @@ Status model_build(Ctx* c, const float* p, size_t d, uint64_t seed, bool rht, co
     put(3, Z);
     put(4, Zt);
     put(5, diag);
-    const bool signs = sign_fragments(Z, dp, reinterpret_cast<uint32_t*>(blob.data() + at[6]), &m->z_guard, &m->z_norm);
-    SLHA_CUDA(cudaMalloc(&m->block, blob.size() + 256));
-    SLHA_CUDA(cudaMemcpyAsync(m->block, blob.data(), blob.size(), cudaMemcpyHostToDevice, c->stream));
+    SLHA_CUDA(cudaMalloc(&m->block, at[6] + (dp <= 256 ? zfb + D_S * 8 : 0) + 256));
+    SLHA_CUDA(cudaMemcpyAsync(m->block, blob.data(), at[6], cudaMemcpyHostToDevice, c->stream));
     const auto array = [&](int i) { return reinterpret_cast<float*>((char*)m->block + at[i]); };
     m->d_p = array(0);
     m->d_pt = array(1);
@@ -513,7 +475,7 @@ Status model_build(Ctx* c, const float* p, size_t d, uint64_t seed, bool rht, co
     m->d_z = array(3);
     m->d_zt = array(4);
     m->d_diag = rht ? array(5) : nullptr;
-    m->d_zf = signs ? reinterpret_cast<uint4*>(array(6)) : nullptr;
+    if (dp <= 256) SLHA_TRY(build_sign_fragments(c, m.get(), reinterpret_cast<uint4*>(array(6)), (char*)m->block + at[6] + zfb));
     SLHA_CUDA(cudaStreamSynchronize(c->stream));
     *out = std::move(m);
     return Status();

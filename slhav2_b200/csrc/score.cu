@@ -310,6 +310,8 @@ struct ScoreArgs {
 template <int G, bool TOPK>
 __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    dep_launch();
+    dep_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int t = lane >> 3, s = lane & 7;
     WorkItem it;

@@ -25,12 +25,13 @@ int stream_kind(uint32_t flags) { return (flags & F_MIXED) ? 1 : ((flags & F_TQ3
 int hint_kind(int hint) { return (hint & 2) ? 1 : ((hint & 4) ? 2 : ((hint & 8) ? 4 : ((hint & 1) ? 0 : 3))); }
 
 template <typename F>
-Status launch_tc(Ctx* c, F* kernel, bool* configured, const ScoreArgs& a, uint32_t grid, int threads, size_t smem) {
+Status launch_tc(Ctx* c, F* kernel, bool* configured, const ScoreArgs& a, uint32_t grid, int threads, size_t smem, bool behind = false) {
     if (!configured[c->device & 15]) {  // (the attribute is per device)
         SLHA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         configured[c->device & 15] = true;
     }
-    kernel<<<grid, threads, smem, c->stream>>>(a);
+    if (behind) SLHA_CUDA(launch_behind(kernel, dim3(grid), dim3(threads), smem, c->stream, a));
+    else kernel<<<grid, threads, smem, c->stream>>>(a);
     count_launch();
     SLHA_CUDA(cudaGetLastError());
     return Status();
@@ -59,9 +60,9 @@ Status launch_stream(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
 uint32_t stream_warp_tiles(int kind, bool il) { return kind == 4 ? ST_WT : (uint32_t)(MMA_SET_TILES * stream_sets(kind, il)); }
 uint32_t stream_warps(int kind, bool il) { return (uint32_t)(kind == 4 ? ST_THREADS : stream_threads(kind, stream_sets(kind, il))) / 32; }
 static_assert(ST_CHUNK == ST_WT, "a fresh chunk holds what a warp can append at once");
-Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_dense_kernel, configured, a, grid, ST_THREADS, st_smem_bytes(true));
+    return launch_tc(c, score_dense_kernel, configured, a, grid, ST_THREADS, st_smem_bytes(true), behind);
 }
 template <int KIND>
 Status launch_wide_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
@@ -89,7 +90,7 @@ size_t score_smem_bytes(int G, int nwarps, bool topk, uint32_t cap) {
 }
 
 template <int G, bool TOPK>
-Status launch_score_t(Ctx* c, const ScoreArgs& a, uint32_t grid, int threads, size_t smem) {
+Status launch_score_t(Ctx* c, const ScoreArgs& a, uint32_t grid, int threads, size_t smem, bool behind) {
     static thread_local size_t configured[16] = {0};
     int dev = c->device & 15;
     if (configured[dev] < smem) {
@@ -100,18 +101,20 @@ Status launch_score_t(Ctx* c, const ScoreArgs& a, uint32_t grid, int threads, si
         SLHA_CUDA(cudaFuncSetAttribute(score_kernel<G, TOPK>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         configured[dev] = MAX_SMEM;
     }
-    score_kernel<G, TOPK><<<grid, threads, smem, c->stream>>>(a);
+    if (behind) SLHA_CUDA(launch_behind(score_kernel<G, TOPK>, dim3(grid), dim3(threads), smem, c->stream, a));
+    else score_kernel<G, TOPK><<<grid, threads, smem, c->stream>>>(a);
     count_launch();
     SLHA_CUDA(cudaGetLastError());
     return Status();
 }
 
 template <bool TOPK>
-Status launch_score(Ctx* c, int G, const ScoreArgs& a, uint32_t grid, int threads, size_t smem) {
+// behind: right after a kernel of the same call (see launch_behind)
+Status launch_score(Ctx* c, int G, const ScoreArgs& a, uint32_t grid, int threads, size_t smem, bool behind) {
     switch (G) {
-        case 1: return launch_score_t<1, TOPK>(c, a, grid, threads, smem);
-        case 2: return launch_score_t<2, TOPK>(c, a, grid, threads, smem);
-        default: return launch_score_t<4, TOPK>(c, a, grid, threads, smem);
+        case 1: return launch_score_t<1, TOPK>(c, a, grid, threads, smem, behind);
+        case 2: return launch_score_t<2, TOPK>(c, a, grid, threads, smem, behind);
+        default: return launch_score_t<4, TOPK>(c, a, grid, threads, smem, behind);
     }
 }
 
@@ -670,10 +673,10 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.score_stride = n;
         a.nf4_table = codec_hint < 0 ? 2u : (uint32_t)(codec_hint & 1);
         a.gflag = reinterpret_cast<uint32_t*>(dev + o_flag);
-        SLHA_TRY(launch_dense(c, a, (uint32_t)cuts.cta.size() - 1));
+        SLHA_TRY(launch_dense(c, a, (uint32_t)cuts.cta.size() - 1, false));
         // the generic kernel over the same work items, only those whose rows were handed back
         const int threads = 128, nwarps = threads / 32;
-        return launch_score<false>(c, 4, a, (uint32_t)cuts.items.size(), threads, score_smem_bytes(4, nwarps, false, 0));
+        return launch_score<false>(c, 4, a, (uint32_t)cuts.items.size(), threads, score_smem_bytes(4, nwarps, false, 0), true);
     }
     const int threads = 128, nwarps = threads / 32;
     const uint32_t item_tiles = 4096;
@@ -693,7 +696,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.total_tiles = n;
         a.item_tiles = item_tiles;
         a.nq_launch = (uint32_t)gq;
-        SLHA_TRY(launch_score<false>(c, G, a, chunks, threads, score_smem_bytes(G, nwarps, false, 0)));
+        SLHA_TRY(launch_score<false>(c, G, a, chunks, threads, score_smem_bytes(G, nwarps, false, 0), false));
         q0 += gq;
     }
     return Status();
@@ -774,11 +777,11 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     a.gflag = nullptr;
     if (!g_force_generic) {
         a.gflag = flag;
-        SLHA_TRY(launch_dense(c, a, (uint32_t)narrow.cta.size() - 1));
+        SLHA_TRY(launch_dense(c, a, (uint32_t)narrow.cta.size() - 1, wide));
     }
     a.items = reinterpret_cast<const WorkItem*>(dev + o_gen);
     const int threads = 128, nwarps = threads / 32;
-    return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0));
+    return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0), !g_force_generic);
 }
 
 Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state,
@@ -849,7 +852,7 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.cap = p->cap;
         a.cand_keys = p->d_cand_keys;
         a.cand_cnt = p->d_cand_cnt;
-        SLHA_TRY(launch_score<true>(c, cl.G, a, cl.count, p->threads, score_smem_bytes(cl.G, nwarps, true, p->cap)));
+        SLHA_TRY(launch_score<true>(c, cl.G, a, cl.count, p->threads, score_smem_bytes(cl.G, nwarps, true, p->cap), mma));
     }
     if (timed && !mma) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));
     static thread_local bool configured[16] = {false};  // the attribute is per device
@@ -870,11 +873,11 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         if (p->compact_splits) {
             const dim3 cgrid(p->compact_splits, (uint32_t)nq);
             if (p->late_threshold)
-                stream_compact_kernel<true><<<cgrid, 256, 0, c->stream>>>(p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap, (uint64_t*)p->b_gsel.p, gselcnt,
-                                                                          cap_s, p->compact_splits, am.ghist, k);
+                SLHA_CUDA(launch_behind(stream_compact_kernel<true>, cgrid, dim3(256), 0, c->stream, p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap,
+                                        (uint64_t*)p->b_gsel.p, gselcnt, cap_s, p->compact_splits, am.ghist, k));
             else
-                stream_compact_kernel<false><<<cgrid, 256, 0, c->stream>>>(p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap, (uint64_t*)p->b_gsel.p, gselcnt,
-                                                                           cap_s, p->compact_splits, am.ghist, k);
+                SLHA_CUDA(launch_behind(stream_compact_kernel<false>, cgrid, dim3(256), 0, c->stream, p->d_gbuf, am.gcount, am.gflag, am.gpivot, p->gcap,
+                                        (uint64_t*)p->b_gsel.p, gselcnt, cap_s, p->compact_splits, am.ghist, k));
             count_launch();
             SLHA_CUDA(cudaGetLastError());
         }
@@ -882,9 +885,9 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
                       p->compact_splits ? (const uint64_t*)p->b_gsel.p : nullptr, gselcnt, cap_s,
                       CompLists{p->d_cand_keys, p->d_cand_cnt, p->d_q_list_begin, p->d_q_list_count, p->list_cap},
                       am.ghist, p->late_threshold ? k : 0u, gselcnt + nq};
-        topk_merge_kernel<StreamLists><<<(uint32_t)nq, merge_threads(cap_s), merge_smem(cap_s, p->kp2), c->stream>>>(
-            L, k, p->kp2, cap_s, d_out_index, d_out_score, d_out_count);
-        p->state_clean = cudaPeekAtLastError() == cudaSuccess;
+        SLHA_CUDA(launch_behind(topk_merge_kernel<StreamLists>, dim3((uint32_t)nq), dim3(merge_threads(cap_s)), merge_smem(cap_s, p->kp2), c->stream, L, k, p->kp2, cap_s,
+                                d_out_index, d_out_score, d_out_count));
+        p->state_clean = true;
     } else if (p->n_groups) {
         // few queries, many lists each: groups of lists first, then the groups' results
         CompLists L1{p->d_cand_keys, p->d_cand_cnt, p->d_vq_begin, p->d_vq_count, p->list_cap};

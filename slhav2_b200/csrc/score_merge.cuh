@@ -248,6 +248,8 @@ template <bool LATE>
 __global__ void __launch_bounds__(256) stream_compact_kernel(const uint64_t* gbuf, const uint32_t* gcount, const uint32_t* gflag,
                                                              const unsigned long long* gpivot, uint32_t gcap, uint64_t* gsel,
                                                              uint32_t* gselcnt, uint32_t selcap, uint32_t splits, const uint32_t* ghist, uint32_t k) {
+    dep_launch();
+    dep_wait();
     const uint32_t Q = blockIdx.y, tid = threadIdx.x, lane = tid & 31;
     if (gflag[Q]) return;
     uint64_t pv;
@@ -725,6 +727,7 @@ __global__ void __launch_bounds__(512) topk_merge_kernel(Lists L, uint32_t k, ui
                                                          uint32_t* out_index, float* out_score,
                                                          uint32_t* out_count) {
     extern __shared__ __align__(16) unsigned char smem[];
+    dep_wait();
     if (L.wait_ready(reinterpret_cast<int*>(smem))) {
         topk_merge_body(L, k, kp2, cap_s, out_index, out_score, out_count, smem);
     } else {

@@ -778,6 +778,7 @@ __device__ __forceinline__ unsigned long long final_threshold(const uint32_t* hi
 template <int KIND, bool IL, int U>
 __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    dep_launch();
     constexpr int nwarps = stream_threads(KIND, U) / 32, R = 2 * U, SET_TILES = MMA_SET_TILES * U, SET_STRIDE = SET_TILES * MMA_ROW;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
@@ -1051,9 +1052,9 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
             const float thr = thr_float(reinterpret_cast<const volatile uint32_t*>(pvh)[t]);
             // The residual term lies in [-256 |lambda|, 256 |lambda|]: rows none of whose tiles can reach the threshold even with the largest
             // term need no Hamming distances (and append nothing).  (257 and the relative slack cover the rounding of the bound
-            // itself; a NaN passes.)  INT4 launches ask for eight tiles at a time; the others, whose rows are mostly short beside
+            // itself; a NaN passes.)  Long INT4 launches ask for eight tiles at a time; the others, whose rows are mostly short beside
             // k (a decode step's caches: one tile in seven is appended, and some tile of a set nearly always), for the set.
-            constexpr int GATE = KIND == 3 ? 1 : R;  // rows asked for at a time
+            constexpr int GATE = KIND == 3 && U == 2 ? 1 : R;  // rows asked for at a time
             float sc[R], lam[R];
             uint32_t b[R], some = 0;
             bool p[R];

@@ -784,6 +784,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
 template <bool IL>
 __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
+    dep_launch();
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     const bool int4 = item_kind(first_tile_flags(a, a.stream_items[i]), false) == 3;
@@ -798,6 +799,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) 
 // tiles is decoded as NF4 throughout.
 __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
+    dep_launch();
+    dep_wait();
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
