@@ -210,24 +210,46 @@ int32_t slha_b200_score_segments(const SciRustSlhaTile* tiles, const SlhaB200Seg
         std::vector<uint64_t> hoff(n_queries);
         if (is_device_ptr(segments)) { SLHA_CUDA(cudaMemcpyAsync(hseg.data(), segments, n_segments * sizeof(SlhaB200Segment), cudaMemcpyDeviceToHost, c->stream)); SLHA_CUDA(cudaStreamSynchronize(c->stream)); }  // (after the caller's work on this stream)
         else std::memcpy(hseg.data(), segments, n_segments * sizeof(SlhaB200Segment));
-        if (is_device_ptr(row_offsets)) { SLHA_CUDA(cudaMemcpyAsync(hoff.data(), row_offsets, n_queries * 8, cudaMemcpyDeviceToHost, c->stream)); SLHA_CUDA(cudaStreamSynchronize(c->stream)); }  // (after the caller's work on this stream)
-        else std::memcpy(hoff.data(), row_offsets, n_queries * 8);
-        for (size_t q = 0; q < n_queries; ++q)
-            if (hoff[q] > scores_len || (uint64_t)row_len > scores_len - hoff[q])
-                return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+        // Offsets in device memory may still be on their way on this stream: a kernel checks them there, the scoring kernels behind
+        // it write nothing where it objects, and the host, which has to say so, waits for that kernel while they run.  (Copied to
+        // the host and checked before anything was launched, the GPU lay idle for the round trip: 89 us per call of 8 x 32 768 tiles
+        // and 64 rows, of which the kernels take 50.)
+        const bool dev_off = is_device_ptr(row_offsets);
+        const uint64_t* doff;
+        const uint32_t* refused = nullptr;
+        if (dev_off) {
+            SLHA_TRY(launch_check_offsets(c, row_offsets, n_queries, scores_len, row_len, &doff, &refused));
+        } else {
+            std::memcpy(hoff.data(), row_offsets, n_queries * 8);
+            for (size_t q = 0; q < n_queries; ++q)
+                if (hoff[q] > scores_len || (uint64_t)row_len > scores_len - hoff[q])
+                    return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+            SLHA_TRY(stage_in_t(c, row_offsets, n_queries, &doff));
+        }
+        const auto scored = [&]() -> Status {
         const float* dq;
         const uint64_t* ds;
-        const uint64_t* doff;
         SLHA_TRY(stage_in_t(c, q_coarse, n_queries * D_C, &dq));
         SLHA_TRY(stage_in_t(c, q_sign, n_queries * 4, &ds));
-        SLHA_TRY(stage_in_t(c, row_offsets, n_queries, &doff));
         std::vector<StagedOut> outs(1);
         SLHA_TRY(stage_out(c, scores_out, scores_len * 4, &outs[0]));
         // a host destination comes back whole: what no row covers is zero
         if (outs[0].is_host) SLHA_CUDA(cudaMemsetAsync(outs[0].dev, 0, scores_len * 4, c->stream));
         SLHA_TRY(launch_score_segments(c, tiles, hseg.data(), n_segments, dq, ds, n_queries, (float*)outs[0].dev,
-                                       reinterpret_cast<const unsigned long long*>(doff), row_len, fill));
+                                       reinterpret_cast<const unsigned long long*>(doff), row_len, fill, refused));
+        if (dev_off) {
+            bool bad;
+            SLHA_TRY(checked_offsets(c, &bad));
+            if (bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+        }
         return finish_outputs(c, outs, sync_by_default(c));
+        };
+        Status st = scored();
+        if (dev_off && !st.ok()) {  // (what else was wrong is reported behind the offsets)
+            bool bad;
+            if (checked_offsets(c, &bad).ok() && bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+        }
+        return st;
     });
 }
 

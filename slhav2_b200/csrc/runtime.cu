@@ -72,6 +72,18 @@ struct LastUse {
     unsigned long long stream = 0;
     bool queued = false;
 };
+struct Answer {
+    uint32_t* host = nullptr;
+    uint32_t* dev = nullptr;
+    cudaEvent_t event = nullptr;
+    ~Answer() {
+        if (event) {
+            cudaEventSynchronize(event);
+            cudaEventDestroy(event);
+        }
+        if (host) cudaFreeHost(host);
+    }
+};
 struct ThreadState {
     int device = 0;
     bool device_chosen = false;
@@ -85,6 +97,7 @@ struct ThreadState {
     uint32_t upload_next[16] = {0};
     UploadSlot* upload_used[16] = {nullptr};  // by the call under way
     LastUse arena[16], plans[16];
+    Answer answer[16];
     bool plans_used[16] = {false};            // by the call under way
 };
 thread_local ThreadState tls;
@@ -223,6 +236,18 @@ Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
     else std::memcpy(s.p, src, bytes);
     SLHA_CUDA(cudaMemcpyAsync(dev, brief ? s.table.data() : s.p, bytes, cudaMemcpyHostToDevice, c->stream));
     tls.upload_used[c->device] = &s;  // (its event is recorded at the call's end)
+    return Status();
+}
+Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, cudaEvent_t* event) {
+    Answer& a = tls.answer[c->device];
+    if (!a.event) {
+        if (!a.host) SLHA_CUDA(cudaHostAlloc((void**)&a.host, 64, cudaHostAllocMapped | cudaHostAllocPortable));
+        SLHA_CUDA(cudaHostGetDevicePointer((void**)&a.dev, a.host, 0));
+        SLHA_CUDA(cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming));
+    }
+    *host = a.host;
+    *dev = a.dev;
+    *event = a.event;
     return Status();
 }
 void ctx_uses_plans(Ctx* c) {

@@ -283,6 +283,7 @@ struct ScoreArgs {
     // full mode
     float* scores;            // [nq][score_stride]
     uint64_t score_stride;
+    const uint32_t* refused;  // optional (full-score mode): nothing is written where it holds 1
     const unsigned long long* row_offset;  // optional (full-score mode): row q starts at scores + row_offset[q] instead of q * score_stride
     // top-k mode
     uint32_t k, cap;
@@ -312,6 +313,7 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     dep_launch();
     dep_wait();
+    if (!TOPK && a.refused && *a.refused) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
     const int t = lane >> 3, s = lane & 7;
     WorkItem it;

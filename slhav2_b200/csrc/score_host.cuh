@@ -702,8 +702,51 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     return Status();
 }
 
+__global__ void __launch_bounds__(256) check_offsets_kernel(const uint64_t* offsets, uint32_t nq, uint64_t scores_len, uint32_t row_len, uint64_t* copy, uint32_t* refused, uint32_t* answer) {
+    bool bad = false;
+    for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x) {
+        const uint64_t o = offsets[q];
+        copy[q] = o;
+        bad |= o > scores_len || row_len > scores_len - o;
+    }
+    bad = __syncthreads_or(bad) != 0;
+    if (threadIdx.x == 0) {
+        *refused = bad;
+        *reinterpret_cast<volatile uint32_t*>(answer) = bad;
+    }
+}
+Status launch_check_offsets(Ctx* c, const uint64_t* d_offsets, size_t nq, uint64_t scores_len, uint32_t row_len, const uint64_t** d_copy, const uint32_t** d_refused) {
+    SLHA_TRY(ctx_no_capture(c));
+    if (nq > 0xFFFFFFFFull) return Status(SLHA_ERR_DIMENSION, "too many query rows");
+    void* dev;
+    SLHA_TRY(ctx_device_scratch(c, nq * 8 + 8, &dev));
+    volatile uint32_t* host;
+    uint32_t* answer;
+    cudaEvent_t event;
+    SLHA_TRY(ctx_answer(c, &host, &answer, &event));
+    uint64_t* copy = static_cast<uint64_t*>(dev);
+    uint32_t* refused = reinterpret_cast<uint32_t*>(copy + nq);
+    check_offsets_kernel<<<1, 256, 0, c->stream>>>(d_offsets, (uint32_t)nq, scores_len, row_len, copy, refused, answer);
+    count_launch();
+    SLHA_CUDA(cudaGetLastError());
+    SLHA_CUDA(cudaEventRecord(event, c->stream));
+    *d_copy = copy;
+    *d_refused = refused;
+    return Status();
+}
+Status checked_offsets(Ctx* c, bool* refused) {
+    volatile uint32_t* host;
+    uint32_t* answer;
+    cudaEvent_t event;
+    SLHA_TRY(ctx_answer(c, &host, &answer, &event));
+    SLHA_CUDA(cudaEventSynchronize(event));
+    *refused = *host != 0;
+    return Status();
+}
+
 // fill of the rows' tails [tail_begin[q], row_len) (one CTA per row)
-__global__ void fill_rows_kernel(float* scores, const unsigned long long* row_offset, const uint32_t* tail_begin, uint32_t row_len, float fill) {
+__global__ void fill_rows_kernel(float* scores, const unsigned long long* row_offset, const uint32_t* tail_begin, uint32_t row_len, float fill, const uint32_t* refused) {
+    if (refused && *refused) return;
     float* row = scores + row_offset[blockIdx.x];
     for (uint32_t e = tail_begin[blockIdx.x] + threadIdx.x; e < row_len; e += blockDim.x) row[e] = fill;
 }
@@ -714,7 +757,7 @@ __global__ void fill_rows_kernel(float* scores, const unsigned long long* row_of
 // where every segment brings 16 query rows or more, the four-row kernel, the generic kernel.  The host looks at no tile and waits for nothing.
 Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, const float* d_q_coarse,
                              const uint64_t* d_q_sign, size_t nq, float* d_scores, const unsigned long long* d_row_offsets,
-                             uint32_t row_len, float fill) {
+                             uint32_t row_len, float fill, const uint32_t* refused) {
     const int sms = sm_count(c->device);
     bool wide = !g_force_generic, fills = false;
     uint64_t total = 0, wtotal = 0;
@@ -751,7 +794,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     unsigned char* dev;
     SLHA_TRY(blob.upload(c, &dev));
     if (fills) {
-        fill_rows_kernel<<<(uint32_t)nq, 256, 0, c->stream>>>(d_scores, d_row_offsets, reinterpret_cast<const uint32_t*>(dev + o_tail), row_len, fill);
+        fill_rows_kernel<<<(uint32_t)nq, 256, 0, c->stream>>>(d_scores, d_row_offsets, reinterpret_cast<const uint32_t*>(dev + o_tail), row_len, fill, refused);
         count_launch();
         SLHA_CUDA(cudaGetLastError());
     }
@@ -762,6 +805,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
     a.scores = d_scores;
     a.row_offset = d_row_offsets;
+    a.refused = refused;
     uint32_t* flag = reinterpret_cast<uint32_t*>(dev + o_flag);
     if (wide) {
         a.items = reinterpret_cast<const WorkItem*>(dev + o_many);

@@ -801,6 +801,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a)
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     dep_launch();
     dep_wait();
+    if (a.refused && *a.refused) return;
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)

@@ -530,6 +530,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_kernel(ScoreArgs a
 __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_dense_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     dep_launch();
+    if (a.refused && *a.refused) return;
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     int kind = item_kind(first_tile_flags(a, a.items[i]), false);

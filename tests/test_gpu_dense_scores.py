@@ -347,3 +347,31 @@ def test_int4_tiles_of_the_shape_of_an_earlier_mix3_call_stay_on_the_tensor_core
         for j in range(nq):
             want = ora.score_tiles(tiles, qc[j], qs[j])
             assert cnt[j] == k and np.all(np.abs(sc[j] - np.sort(want)[::-1][:k]) <= 1e-3) and np.all(np.abs(sc[j] - want[idx[j]]) <= 1e-3)
+
+
+@pytest.mark.parametrize("nq,codec", [(1, 0), (4, 5), (20, 3), (20, 2), (300, 0)])
+@pytest.mark.parametrize("tail", [0, 7])
+def test_row_offsets_in_device_memory_are_checked_there(nq, codec, tail):
+    # the same scores as with offsets in host memory; a row that reaches beyond the destination refuses the call, and no row is written
+    n = 700
+    tiles = S.to_device(H.random_tiles(n, codec, seed=540 + codec))
+    qc, qs = H.random_queries(nq, 541)
+    dq, ds = S.to_device(qc), S.to_device(qs)
+    seg, row = S.make_segments([(0, n, 0, nq, 0)]), n + tail
+    off = np.random.default_rng(nq).permutation(nq).astype(np.uint64) * row
+    want = S.score_segments(tiles, seg, dq, ds, nq, np.zeros(nq * row, F), off, row, fill=-3.0)
+    out = S.to_device(np.full(nq * row, 9.0, F))
+    S.score_segments(tiles, seg, dq, ds, nq, out, S.to_device(off), row, fill=-3.0)
+    assert np.array_equal(out.download(F, nq * row), want)
+    for bad in (1, 2**63, 2**64 - row):  # (one element too far, and sums that wrap around)
+        wrong = off.copy()
+        wrong[nq // 2] = (int(wrong.max()) + bad) % 2**64 if bad == 1 else bad
+        out = S.to_device(np.full(nq * row, 9.0, F))
+        host = np.full(nq * row, 9.0, F)
+        for dst in (out, host):
+            with pytest.raises(S.SlhaError) as e:
+                S.score_segments(tiles, seg, dq, ds, nq, dst, S.to_device(wrong), row, fill=-3.0)
+            assert e.value.code == S.ERR_DIMENSION
+        assert np.all(out.download(F, nq * row) == 9.0) and np.all(host == 9.0)
+    S.score_segments(tiles, seg, dq, ds, nq, out, S.to_device(off), row, fill=-3.0)  # a refused call leaves nothing behind
+    assert np.array_equal(out.download(F, nq * row), want)
