@@ -344,12 +344,102 @@ __device__ __forceinline__ void phase_keys(const PoolDev& p, int phase, uint64_t
 #pragma unroll
     for (int u = 0; u < EB_BATCH; ++u) key[u] = phase_key(p, phase, s0 + u * stride, m[u], max_pos);
 }
+constexpr int EB_KEYS = 16;  // slots of a thread whose keys stay in its registers (1.2 million on 148 SMs)
 constexpr int EB_THREADS = 512, EB_ITEMS = 8, EB_CAP = EB_THREADS * EB_ITEMS, EB_LEVELS = 6, EB_BINS = 4096;
 struct EnforceState {
     unsigned long long inv_min_key, max_key;  // ~min and max over the phase's candidates (zero = none yet)
     uint32_t n_keep, overflow, pad[2];
+    unsigned long long bound_inv[5];          // ~bound of the phase's candidates, see below
+    uint32_t few[5], pad2;                    // how many lie within it
     uint32_t hist[5][EB_LEVELS][EB_BINS];
 };
+
+using EbScan32 = cub::BlockScan<uint32_t, EB_THREADS>;
+struct CutShared {
+    union {
+        uint32_t hist[EB_BINS];
+        typename EbScan32::TempStorage scan;
+    };
+    unsigned long long lo_inv, hi;
+    uint32_t count, bin, in_bin, cum;
+};
+// A key bound that at least `reach` of the block's keys (N a thread, SENTINEL where there is none) do not exceed, or all of
+// them where there are fewer: a radix select in shared memory, 12 key bits a level from the highest in which the keys differ, until at most `slack`
+// more than reach are kept.  All threads of the block call; kept: how many keys are within the bound.
+template <int N>
+__device__ __forceinline__ uint64_t block_cut(const uint64_t (&k)[N], uint64_t reach, uint32_t slack, CutShared& sm, uint32_t& kept) {
+    uint64_t lo = SENTINEL, hi = 0;
+    uint32_t n = 0;
+#pragma unroll
+    for (int j = 0; j < N; ++j)
+        if (k[j] != SENTINEL) {
+            lo = min(lo, k[j]);
+            hi = max(hi, k[j]);
+            ++n;
+        }
+    for (int o = 16; o; o >>= 1) {
+        lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
+        hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
+    }
+    n = __reduce_add_sync(0xFFFFFFFFu, n);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sm.lo_inv = sm.hi = 0ull;
+        sm.count = 0u;
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0 && n) {
+        atomicMax(&sm.lo_inv, (unsigned long long)~lo);
+        atomicMax(&sm.hi, (unsigned long long)hi);
+        atomicAdd(&sm.count, n);
+    }
+    __syncthreads();
+    lo = ~sm.lo_inv;
+    hi = sm.hi;
+    kept = sm.count;
+    if (kept <= reach + slack) return hi;
+    uint64_t base = lo, below = 0;
+    int shift = max(0, 64 - __clzll((long long)(hi - lo)) - 12);
+    for (;;) {
+        __syncthreads();
+        for (uint32_t b = threadIdx.x; b < EB_BINS; b += EB_THREADS) sm.hist[b] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < N; ++j)
+            if (k[j] != SENTINEL && k[j] >= base && ((k[j] - base) >> shift) < (uint64_t)EB_BINS) atomicAdd(&sm.hist[(uint32_t)((k[j] - base) >> shift)], 1u);
+        __syncthreads();
+        uint32_t h[EB_ITEMS], mine = 0, before;
+#pragma unroll
+        for (int j = 0; j < EB_ITEMS; ++j) {
+            h[j] = sm.hist[threadIdx.x * EB_ITEMS + j];
+            mine += h[j];
+        }
+        __syncthreads();
+        EbScan32(sm.scan).ExclusiveSum(mine, before);
+        uint64_t cum = below + before;
+        if (cum < reach && cum + mine >= reach) {  // (one thread: there are more than reach keys)
+            for (int j = 0; j < EB_ITEMS; ++j) {
+                cum += h[j];
+                if (cum >= reach) {
+                    sm.bin = threadIdx.x * EB_ITEMS + j;
+                    sm.in_bin = h[j];
+                    sm.cum = (uint32_t)cum;
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        const uint32_t b = sm.bin;
+        kept = sm.cum;
+        if (kept <= reach + slack || shift == 0) {
+            const uint64_t bound = base + ((((uint64_t)b + 1) << shift) - 1);
+            return bound < base ? SENTINEL - 1 : bound;
+        }
+        below = kept - sm.in_bin;
+        base += (uint64_t)b << shift;
+        shift = max(0, shift - 12);
+    }
+}
 
 __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t phase_mask, uint64_t* keys, uint32_t* vals,
                                                              uint64_t* skeys, uint32_t* svals, EnforceState* es) {
@@ -364,6 +454,7 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
         typename Scan32::TempStorage scan32;
         uint32_t hist[EB_BINS];
         struct { uint64_t in[EB_THREADS], key[EB_THREADS]; uint32_t val[EB_THREADS]; } few;
+        CutShared cut;
     } sm;
     __shared__ uint32_t cut_bin, cut_hist;
     __shared__ unsigned long long cut_cum, fin_applied;
@@ -404,8 +495,57 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
         const uint64_t live = cnt->live, budget = cnt->budget;
         if (live <= budget) break;
         const uint64_t deficit = live - budget;
+        const uint64_t min_freed = phase == PH_PAGE ? 32 : (phase >= PH_EVICT ? 80 : 14);
+        const uint64_t reach = deficit / min_freed + 1;
+        // ---- a decode step's deficit (a few operations): every block finds a bound that `reach` of its own keys do not exceed, and the
+        //      smallest of the blocks' bounds is one for all candidates.  The few keys within it go to the last block's sort from
+        //      registers: one scan and two grid barriers, where the list of all candidates below takes a write and three reads,
+        //      global histograms and three barriers.
+        bool few = len <= EB_KEYS * stride && reach * gridDim.x <= 4ull * EB_CAP;
+        if (few) {
+            uint64_t key[EB_KEYS];
+#pragma unroll
+            for (int b = 0; b < EB_KEYS; b += EB_BATCH) {
+                uint64_t part[EB_BATCH];
+                phase_keys(p, phase, gtid + b * stride, stride, len, max_pos, part);
+#pragma unroll
+                for (int u = 0; u < EB_BATCH; ++u) key[b + u] = part[u];
+            }
+            uint32_t kept;
+            const uint64_t own = block_cut(key, reach, 4u, sm.cut, kept);
+            if (threadIdx.x == 0 && kept >= reach) atomicMax(&es->bound_inv[phase], (unsigned long long)~own);  // (a block with fewer keys bounds nothing)
+            grid.sync();
+            const uint64_t bound = ~*(volatile unsigned long long*)&es->bound_inv[phase];
+            uint32_t mine = 0;
+#pragma unroll
+            for (int j = 0; j < EB_KEYS; ++j) mine += key[j] != SENTINEL && key[j] <= bound;
+            if (__any_sync(0xFFFFFFFFu, mine != 0u)) {
+                uint32_t incl = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                uint32_t at = 0;
+                if (lane == 31) at = atomicAdd(&es->few[phase], incl);
+                at = __shfl_sync(0xFFFFFFFFu, at, 31) + incl - mine;
+#pragma unroll
+                for (int j = 0; j < EB_KEYS; ++j)
+                    if (key[j] != SENTINEL && key[j] <= bound) {
+                        if (at < (uint32_t)EB_CAP) {
+                            skeys[at] = key[j];
+                            svals[at] = (uint32_t)(gtid + j * stride);
+                        }
+                        ++at;
+                    }
+            }
+            grid.sync();
+            const uint32_t got = *(volatile uint32_t*)&es->few[phase];
+            if (got == 0) continue;                 // no candidates (every block sees the same)
+            few = got <= (uint32_t)EB_CAP;          // (else the general path below)
+        }
         // ---- build
-        {
+        if (!few) {
             // One reservation per block and batch, one minimum and maximum per block: an atomic per warp on the same word
             // costs more than the scan itself (32 k of them for a million slots).
             uint64_t kmin = SENTINEL, kmax = 0;
@@ -463,15 +603,13 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
                 atomicMax(&es->max_key, block_max);
             }
         }
-        grid.sync();
+        if (!few) grid.sync();
         const uint64_t nc = cnt->n_cand;
-        if (nc) {
-            const uint64_t min_freed = phase == PH_PAGE ? 32 : (phase >= PH_EVICT ? 80 : 14);
-            const uint64_t reach = deficit / min_freed + 1;
-            const bool take_all = nc <= (uint64_t)EB_CAP;
+        if (nc || few) {
+            const bool take_all = !few && nc <= (uint64_t)EB_CAP;
             uint64_t base = ~*(volatile unsigned long long*)&es->inv_min_key, thr_rel = ~0ull, below = 0;
-            bool bounded = take_all;
-            if (!take_all && reach <= (uint64_t)EB_CAP) {
+            bool bounded = take_all || few;
+            if (!bounded && reach <= (uint64_t)EB_CAP) {
                 const uint64_t span = *(volatile unsigned long long*)&es->max_key - base;
                 int shift = max(0, 64 - __clzll((long long)span) - 12);
                 for (int level = 0; level < EB_LEVELS && !bounded; ++level) {
@@ -530,7 +668,7 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
                 if (gtid == 0) es->overflow = 1;
                 return;  // every block takes this branch
             }
-            if (!take_all) {
+            if (!take_all && !few) {
                 const uint64_t rounds = (nc + stride - 1) / stride;
                 for (uint64_t r = 0; r < rounds; ++r) {
                     const uint64_t i = r * stride + gtid;
@@ -557,13 +695,31 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
             if (blockIdx.x == 0) {
                 const uint64_t* ks = take_all ? keys : skeys;
                 const uint32_t* vs = take_all ? vals : svals;
-                const uint32_t n = take_all ? (uint32_t)nc : min(*(volatile uint32_t*)&es->n_keep, (uint32_t)EB_CAP);
+                uint32_t n = take_all ? (uint32_t)nc : (few ? *(volatile uint32_t*)&es->few[phase] : min(*(volatile uint32_t*)&es->n_keep, (uint32_t)EB_CAP));
                 uint64_t k[EB_ITEMS];
                 uint32_t v[EB_ITEMS];
                 for (int j = 0; j < EB_ITEMS; ++j) {
                     const uint32_t i = threadIdx.x * EB_ITEMS + j;
                     k[j] = i < n ? ks[i] : SENTINEL;
                     v[j] = i < n ? vs[i] : 0u;
+                }
+                if (n > EB_THREADS && reach <= EB_THREADS / 2) {  // the blocks' smallest keys together: down to what the count below orders
+                    uint32_t kept;
+                    const uint64_t bound = block_cut(k, reach, EB_THREADS / 2, sm.cut, kept);
+                    if (kept <= EB_THREADS) {
+                        if (threadIdx.x == 0) warp_n[0] = 0u;
+                        __syncthreads();
+                        for (int j = 0; j < EB_ITEMS; ++j)
+                            if (k[j] != SENTINEL && k[j] <= bound) {
+                                const uint32_t o = atomicAdd(&warp_n[0], 1u);
+                                skeys[o] = k[j];  // (every key has been read: block_cut's barriers)
+                                svals[o] = v[j];
+                            }
+                        __syncthreads();
+                        ks = skeys;
+                        vs = svals;
+                        n = kept;
+                    }
                 }
                 if (threadIdx.x == 0) {
                     fin_applied = 0;

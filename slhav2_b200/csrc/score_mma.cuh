@@ -961,7 +961,18 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
         // of every CTA that works on the row -- and the rows do not already have thresholds (a CTA that starts its
         // second item on rows other CTAs have been scoring for a while).
         const bool all_warm = __syncthreads_and(row_warm) != 0;
-        const bool first_round_barrier = !all_warm && (uint64_t)a.k <= (uint64_t)SET_TILES * (uint64_t)nwarps * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
+        const bool first_round_barrier = !all_warm && !too_big && (uint64_t)a.k <= (uint64_t)SET_TILES * (uint64_t)nwarps * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
+        // Of the first round only some warps append unfiltered; the others wait at that barrier with their first set, and filter it by the
+        // thresholds of these seeds.  With N tiles in the first round of all CTAs on the row, S seeds and (N - S) k / S of the rest are appended,
+        // least at S = sqrt(N k).  (With all 24 warps of 148 CTAs on one row 57 k tiles a row were appended at once: a million MX tiles, k = 100,
+        // 81 us, with 7 seeds a CTA 60.)
+        const uint32_t parts = max((it.pad >> 8) & 0x7FFFFFu, 1u);
+        int seeds = nwarps;
+        // (from N = 9 k on, where the seeds number 3 k: with k = 2048 of N = 6912 the seeds hardly prove a threshold before the rest is due,
+        // 8 x 131 072 INT4 tiles 85 -> 100 us; and calls of two rounds have little to append: 8 x 8192 mixed tiles 29.1 -> 29.6 us)
+        const uint64_t first_tiles = (uint64_t)SET_TILES * (uint64_t)nwarps * parts;
+        if (first_round_barrier && my_rounds > 1u && first_tiles >= 9ull * a.k && (my_rounds > 2u || first_tiles >= 8192u))
+            seeds = min(nwarps, max(1, (int)ceilf(sqrtf((float)nwarps * (float)a.k / ((float)SET_TILES * (float)parts)))));
         if (too_big) n_sets = 0;  // (the sets already on their way are waited for at the item's end and never read)
 
         uint32_t slot = 0, polls = 0;
@@ -970,12 +981,20 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
         const uint32_t rounds = too_big ? 0u : my_rounds;
         for (uint32_t round = 0; round < rounds; ++round) {
             const uint32_t s = set_of(round);
-            if (round == 1 && first_round_barrier) {
-                // Every warp of the CTA (and, started together, of the grid) has appended its first set
-                // unfiltered, so the rows' histograms hold a set's candidates per warp: first thresholds now,
-                // before the second sets are filtered.  (All warps pass here: `rounds` is the same for all.)
+            if (round == (warp < seeds ? 1u : 0u) && first_round_barrier) {
+                // The seeds of the CTA (and, started together, of the grid) have appended their first sets
+                // unfiltered, so the rows' histograms hold a set's candidates per seed: first thresholds now,
+                // before the other sets are filtered.  (All warps pass here: `rounds` is the same for all, and at least two where there are
+                // fewer seeds than warps.)  Other CTAs may be a little behind: a few tries.
                 __syncthreads();
-                if (warp < nq) stream_refresh_threshold(a, it.query_begin + (uint32_t)warp, rng[warp], pvh + warp, lane);
+                if (warp < nq) {
+                    for (int tries = seeds < nwarps ? 4 : 1; tries; --tries) {
+                        stream_refresh_threshold(a, it.query_begin + (uint32_t)warp, rng[warp], pvh + warp, lane);
+                        __syncwarp();
+                        if (reinterpret_cast<volatile uint32_t*>(pvh)[warp] != 0u || tries == 1) break;
+                        __nanosleep(400);
+                    }
+                }
                 __syncthreads();
             }
             // (the ring advances in every iteration, also when this warp has no set in this round -- the short last round of
