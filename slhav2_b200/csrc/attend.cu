@@ -70,6 +70,8 @@ template <typename T, int VEC, int SPLIT>
 __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
     attend_kernel(const uint32_t* top_index, const float* top_score, const uint32_t* top_count, uint32_t k, float scale, const T* values,
                   size_t d_v, size_t row_stride, const uint64_t* row_base, float* out, float* weights_out) {
+    dep_launch();
+    dep_wait();
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ float sm[];  // weights | indices of the CTA's run
@@ -160,10 +162,9 @@ Status launch_attend_t(Ctx* c, const uint32_t* d_index, const float* d_score, co
                        const void* d_values, size_t d_v, size_t row_stride, const uint64_t* d_row_base, float* d_out, float* d_weights) {
     const size_t smem = (size_t)((k + SPLIT - 1) / SPLIT) * 8;
     if (smem > 16 * 1024) SLHA_CUDA(cudaFuncSetAttribute(attend_kernel<T, VEC, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8192 * 8));
-    attend_kernel<T, VEC, SPLIT><<<dim3(SPLIT, (uint32_t)nq), ATT_THREADS, smem, c->stream>>>(d_index, d_score, d_count, k, scale, (const T*)d_values, d_v,
-                                                                                         row_stride, d_row_base, d_out, d_weights);
+    SLHA_CUDA(launch_behind(attend_kernel<T, VEC, SPLIT>, dim3(SPLIT, (uint32_t)nq), dim3(ATT_THREADS), smem, c->stream, d_index, d_score, d_count, k, scale,
+                            (const T*)d_values, d_v, row_stride, d_row_base, d_out, d_weights));
     count_launch();
-    SLHA_CUDA(cudaGetLastError());
     return Status();
 }
 

@@ -631,6 +631,8 @@ template <bool QUERY, int KB>
 // (four CTAs of 32 keys share an SM at head dimension 128: up to 128 registers, 57 KB of shared memory each)
 __global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kernel(EncodeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    dep_launch();
+    dep_wait();
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int PER = KB >= 2 ? KB / 2 : 1;  // keys per thread where two threads share an output row
     constexpr int NT = enc_threads(KB);
@@ -1084,9 +1086,8 @@ Status run_encode_kb(Ctx* c, EncodeArgs& a) {
     // different phases, so that the arithmetic of one covers the loads, quantisation and barriers
     // of the others.  One resident wave measured 182 M keys/s, 8 CTAs per SM 191, one CTA per pass 199.
     const uint32_t grid = (uint32_t)std::min<uint64_t>(groups, 148ull * 64);
-    encode_kernel<QUERY, KB><<<grid, enc_threads(KB), smem, c->stream>>>(a);
+    SLHA_CUDA(launch_behind(encode_kernel<QUERY, KB>, dim3(grid), dim3(enc_threads(KB)), smem, c->stream, a));
     count_launch();
-    SLHA_CUDA(cudaGetLastError());
     return Status();
 }
 

@@ -43,6 +43,8 @@ __device__ __forceinline__ uint32_t tile_flags(const unsigned char* tiles, uint6
 // (LIFO pops), then fresh slots len, len+1, ...
 __global__ void insert_kernel(PoolDev p, const unsigned char* src, uint64_t n, uint64_t pops,
                               uint64_t len0, uint64_t free0, uint64_t seq0, uint32_t* slots_out) {
+    dep_launch();
+    dep_wait();
     const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t bytes = 0;
     if (j < n) {
@@ -811,6 +813,8 @@ struct ObserveTmp {
 };
 // (one set of atomics per CTA, and a grid of a few CTAs per SM: an atomic per warp on the same words costs more than the scan)
 __global__ void __launch_bounds__(256) observe_pass1(PoolDev p, const uint32_t* slots, const float* scores, uint64_t n, ObserveTmp* tmp) {
+    dep_launch();
+    dep_wait();
     __shared__ uint32_t red[3];
     if (threadIdx.x < 3) red[threadIdx.x] = 0u;
     __syncthreads();
@@ -857,6 +861,8 @@ __device__ __forceinline__ float key_to_f32(uint32_t k) {
 // per-CTA partial sums of exp((s-m)/T) in a fixed order (deterministic)
 __global__ void observe_pass2(PoolDev p, const uint32_t* slots, const float* scores, uint64_t n,
                               float temperature, const ObserveTmp* tmp, float* partial) {
+    dep_launch();
+    dep_wait();
     __shared__ float red[32];
     const uint64_t len = p.cnt->len;
     const float m = key_to_f32(tmp->max_key);
@@ -892,6 +898,8 @@ __global__ void observe_pass2(PoolDev p, const uint32_t* slots, const float* sco
 }
 __global__ void observe_pass3(PoolDev p, const uint32_t* slots, const float* scores, uint64_t n,
                               float temperature, ObserveTmp* tmp, const float* partial, int n_partial) {
+    dep_launch();
+    dep_wait();
     __shared__ float s_inv, part[256];
     for (int i = threadIdx.x; i < n_partial; i += blockDim.x) part[i] = partial[i];  // (n_partial <= 256)
     __syncthreads();
@@ -1060,10 +1068,9 @@ Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t
     const uint64_t pops = std::min<uint64_t>(n, h.free_len);
     if (h.len + (n - pops) > pl->cfg.capacity_tiles)
         return Status(SLHA_ERR_CAPACITY, "pool: capacity_tiles exceeded");
-    insert_kernel<<<(uint32_t)((n + 255) / 256), 256, 0, c->stream>>>(pl->dev, d_src_tiles, n, pops, h.len,
-                                                                      h.free_len, h.next_seq, d_slots);
+    SLHA_CUDA(launch_behind(insert_kernel, dim3((uint32_t)((n + 255) / 256)), dim3(256), 0, c->stream, pl->dev, d_src_tiles, n, pops, h.len, h.free_len,
+                            h.next_seq, d_slots));
     count_launch();
-    SLHA_CUDA(cudaGetLastError());
     h.free_len -= pops;
     h.len += n - pops;
     h.next_seq += n;
@@ -1304,8 +1311,8 @@ Status pool_observe(Ctx* c, Pool* pl, const uint32_t* d_slots, const float* d_sc
     SLHA_CUDA(cudaMemsetAsync(tmp, 0, sizeof(ObserveTmp), c->stream));
     const uint32_t grid = std::min<uint32_t>(grid_for(n), (uint32_t)sm_count(c->device) * 4);
     observe_pass1<<<grid, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, tmp);
-    observe_pass2<<<nparts, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial);
-    observe_pass3<<<grid, 256, 0, c->stream>>>(pl->dev, d_slots, d_scores, n, temperature, tmp, partial, nparts);
+    SLHA_CUDA(launch_behind(observe_pass2, dim3(nparts), dim3(256), 0, c->stream, pl->dev, d_slots, d_scores, n, temperature, tmp, partial));
+    SLHA_CUDA(launch_behind(observe_pass3, dim3(grid), dim3(256), 0, c->stream, pl->dev, d_slots, d_scores, n, temperature, tmp, partial, nparts));
     count_launch(3);
     SLHA_CUDA(cudaGetLastError());
     return Status();

@@ -39,12 +39,12 @@ Status launch_tc(Ctx* c, F* kernel, bool* configured, const ScoreArgs& a, uint32
 template <int KIND, bool IL, int U>
 Status launch_stream_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_stream_kernel<KIND, IL, U>, configured, a, grid, stream_threads(KIND, U), stream_smem_bytes(KIND, U));
+    return launch_tc(c, score_stream_kernel<KIND, IL, U>, configured, a, grid, stream_threads(KIND, U), stream_smem_bytes(KIND, U), true);
 }
 template <bool IL>
 Status launch_mix3(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_mix3_kernel<IL>, configured, a, grid, ST_THREADS, st_smem_bytes(false));
+    return launch_tc(c, score_mix3_kernel<IL>, configured, a, grid, ST_THREADS, st_smem_bytes(false), true);
 }
 template <bool IL>
 Status launch_stream(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
@@ -67,7 +67,7 @@ Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
 template <int KIND>
 Status launch_wide_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_wide_kernel<KIND>, configured, a, grid, WIDE_THREADS, wide_smem_bytes());
+    return launch_tc(c, score_wide_kernel<KIND>, configured, a, grid, WIDE_THREADS, wide_smem_bytes(), true);
 }
 Status launch_wide(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
     switch (kind) {
@@ -703,6 +703,8 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
 }
 
 __global__ void __launch_bounds__(256) check_offsets_kernel(const uint64_t* offsets, uint32_t nq, uint64_t scores_len, uint32_t row_len, uint64_t* copy, uint32_t* refused, uint32_t* answer) {
+    dep_launch();
+    dep_wait();
     bool bad = false;
     for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x) {
         const uint64_t o = offsets[q];
@@ -726,9 +728,8 @@ Status launch_check_offsets(Ctx* c, const uint64_t* d_offsets, size_t nq, uint64
     SLHA_TRY(ctx_answer(c, &host, &answer, &event));
     uint64_t* copy = static_cast<uint64_t*>(dev);
     uint32_t* refused = reinterpret_cast<uint32_t*>(copy + nq);
-    check_offsets_kernel<<<1, 256, 0, c->stream>>>(d_offsets, (uint32_t)nq, scores_len, row_len, copy, refused, answer);
+    SLHA_CUDA(launch_behind(check_offsets_kernel, dim3(1), dim3(256), 0, c->stream, d_offsets, (uint32_t)nq, scores_len, row_len, copy, refused, answer));
     count_launch();
-    SLHA_CUDA(cudaGetLastError());
     SLHA_CUDA(cudaEventRecord(event, c->stream));
     *d_copy = copy;
     *d_refused = refused;

@@ -779,6 +779,7 @@ template <int KIND, bool IL, int U>
 __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     dep_launch();
+    dep_wait();
     constexpr int nwarps = stream_threads(KIND, U) / 32, R = 2 * U, SET_TILES = MMA_SET_TILES * U, SET_STRIDE = SET_TILES * MMA_ROW;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;

@@ -785,6 +785,7 @@ template <bool IL>
 __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     dep_launch();
+    dep_wait();
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     const bool int4 = item_kind(first_tile_flags(a, a.stream_items[i]), false) == 3;

@@ -519,6 +519,7 @@ template <int KIND>
 __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     dep_launch();
+    dep_wait();
     const uint32_t first = a.cta_begin[blockIdx.x];
     // (a plan made for MIX3 tiles also takes INT4 / MX-INT4 tiles of its shape, see score_mix3_kernel)
     if (KIND == 4 && item_kind(first_tile_flags(a, a.items[first]), false) == 3) wide_body<3, false>(a, smem_raw, first);
@@ -530,6 +531,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_kernel(ScoreArgs a
 __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_dense_kernel(ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     dep_launch();
+    dep_wait();
     if (a.refused && *a.refused) return;
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
