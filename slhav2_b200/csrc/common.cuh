@@ -186,7 +186,7 @@ Status launch_attend_topk(Ctx* c, const uint32_t* d_index, const float* d_score,
                           float scale, const void* d_values, int value_dtype, size_t d_v, size_t row_stride,
                           const uint64_t* d_row_base, float* d_out, float* d_weights);
 
-Status build_sign_fragments(Ctx* c, Model* m, uint4* d_zf, void* d_stats);  // fills d_zf from d_z and sets the model's sign members; synchronises
+Status build_model_arrays(Ctx* c, Model* m, uint4* d_zf, void* d_stats);  // d_pt, d_zt, d_zf from d_p and d_z, and the model's sign members; synchronises
 Status launch_encode(Ctx* c, const Model* m, const void* d_keys, int key_dtype, size_t n,
                      const uint32_t* d_positions, uint32_t position_base, const uint16_t* d_heads,
                      int codec, SciRustSlhaTile* d_tiles, const uint32_t* d_slots);

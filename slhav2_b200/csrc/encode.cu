@@ -1036,6 +1036,10 @@ __global__ void __launch_bounds__(128) sign_fragments_kernel(const float* z, uin
     if (threadIdx.x == 0) stats[s] = usual ? make_float2((float)sqrt(lost), (float)sqrt(kept)) : make_float2(-1.0f, -1.0f);
 }
 
+__global__ void __launch_bounds__(256) transpose_kernel(const float* in, float* out, uint64_t rows, uint64_t cols) {
+    for (uint64_t i = (uint64_t)blockIdx.x * 256 + threadIdx.x; i < rows * cols; i += (uint64_t)gridDim.x * 256) out[i] = in[i % rows * cols + i / rows];
+}
+
 size_t encode_smem(uint32_t d_pad, int kb) {
     const size_t ks = (size_t)enc_row_stride(kb);
     return (((d_pad * ks + 3) & ~size_t(3)) + (size_t)kb * D_C + ks * D_C) * 4 + (size_t)kb * TILE_BYTES;
@@ -1107,7 +1111,13 @@ Status run_encode(Ctx* c, EncodeArgs& a) {
 
 // No fragments (every sign from its exact sum) where the error bound of signs_mma does not hold: more than 256 dimensions, or rows far
 // from ordinary size.
-Status build_sign_fragments(Ctx* c, Model* m, uint4* d_zf, void* d_stats) {
+Status build_model_arrays(Ctx* c, Model* m, uint4* d_zf, void* d_stats) {
+    const auto grid = [](size_t n) { return (uint32_t)std::min<size_t>((n + 255) / 256, 1184); };
+    transpose_kernel<<<grid(D_C * m->d), 256, 0, c->stream>>>(m->d_p, m->d_pt, D_C, m->d);
+    transpose_kernel<<<grid(D_S * m->d_pad), 256, 0, c->stream>>>(m->d_z, m->d_zt, D_S, m->d_pad);
+    count_launch(2);
+    SLHA_CUDA(cudaGetLastError());
+    if (m->d_pad > 256) return Status();
     float2 stats[D_S];
     sign_fragments_kernel<<<D_S, 128, 0, c->stream>>>(m->d_z, (uint32_t)m->d_pad, reinterpret_cast<uint32_t*>(d_zf), static_cast<float2*>(d_stats));
     count_launch();

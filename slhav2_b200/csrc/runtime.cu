@@ -8,6 +8,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <shared_mutex>
 #include <unordered_map>
@@ -453,54 +454,45 @@ Status model_build(Ctx* c, const float* p, size_t d, uint64_t seed, bool rht, co
         while (dp < d) dp <<= 1;
     }
     m->d_pad = dp;
-    std::vector<float> P(p, p + (size_t)D_C * d), Pt((size_t)D_C * d), S(D_C, 1.0f);
-    for (size_t k = 0; k < (size_t)D_C; ++k)
-        for (size_t i = 0; i < d; ++i) Pt[i * D_C + k] = P[k * d + i];
-    if (scale) {
-        for (int k = 0; k < D_C; ++k) {
-            if (!std::isfinite(scale[k]) || scale[k] <= 0.0f)
-                return Status(SLHA_ERR_NONFINITE, "whitening scale must be finite and positive");
-            S[k] = scale[k];
-        }
+    // one allocation; P, scale, Z and the diagonal go up in one copy, the transposed copies and the fragments of Z are made there
+    const size_t zfb = (dp + 31) / 32 * 32 * 32 * 16;
+    size_t at[8] = {0};
+    at[1] = pad256(D_C * d * 4);              // 0 P, 1 scale
+    at[2] = at[1] + pad256(D_C * 4);          // 2 Z
+    at[3] = at[2] + pad256(D_S * dp * 4);     // 3 diagonal
+    at[4] = at[3] + pad256(rht ? dp * 4 : 0); // 4 P transposed, from here on made on the device
+    at[5] = at[4] + pad256(D_C * d * 4);      // 5 Z transposed
+    at[6] = at[5] + pad256(D_S * dp * 4);     // 6 fragments
+    at[7] = at[6] + (dp <= 256 ? zfb : 0);    // 7 figures of the fragments' rounding
+    std::unique_ptr<float[]> host(new float[at[4] / 4]);
+    const auto part = [&](int i) { return host.get() + at[i] / 4; };
+    std::memcpy(part(0), p, D_C * d * 4);
+    for (int k = 0; k < D_C; ++k) {
+        if (scale && (!std::isfinite(scale[k]) || scale[k] <= 0.0f))
+            return Status(SLHA_ERR_NONFINITE, "whitening scale must be finite and positive");
+        part(1)[k] = scale ? scale[k] : 1.0f;
     }
-    std::vector<float> Z((size_t)D_S * dp), Zt((size_t)D_S * dp), diag;
     if (rht) {  // learned.rs:158-165 + incoherence.rs:89-97
         Rng r(seed ^ 0xA2A2A2A2A2A2A2A2ull);
-        diag.resize(dp);
-        for (size_t i = 0; i < dp; ++i) diag[i] = r.next_unit() < 0.5f ? -1.0f : 1.0f;
+        for (size_t i = 0; i < dp; ++i) part(3)[i] = r.next_unit() < 0.5f ? -1.0f : 1.0f;
     }
     if (z) {
-        std::memcpy(Z.data(), z, Z.size() * 4);
+        std::memcpy(part(2), z, D_S * dp * 4);
     } else {  // learned.rs:168-170
         Rng r(seed);
-        for (float& v : Z) v = r.next_gaussian();
+        float* zp = part(2);
+        for (size_t i = 0; i < D_S * dp; ++i) zp[i] = r.next_gaussian();
     }
-    for (size_t s = 0; s < (size_t)D_S; ++s)
-        for (size_t i = 0; i < dp; ++i) Zt[i * D_S + s] = Z[s * dp + i];
-    // one allocation and one copy for all arrays
-    const size_t dim = D_C * d * 4, zb = D_S * dp * 4, zfb = (dp + 31) / 32 * 32 * 32 * 16;
-    size_t at[7] = {0, pad256(dim), 2 * pad256(dim), 2 * pad256(dim) + pad256(D_C * 4)};
-    at[4] = at[3] + pad256(zb);
-    at[5] = at[4] + pad256(zb);
-    at[6] = at[5] + pad256(diag.size() * 4);
-    std::vector<unsigned char> blob(at[6]);
-    const auto put = [&](int i, const std::vector<float>& v) { if (!v.empty()) std::memcpy(blob.data() + at[i], v.data(), v.size() * 4); };
-    put(0, P);
-    put(1, Pt);
-    put(2, S);
-    put(3, Z);
-    put(4, Zt);
-    put(5, diag);
-    SLHA_CUDA(cudaMalloc(&m->block, at[6] + (dp <= 256 ? zfb + D_S * 8 : 0) + 256));
-    SLHA_CUDA(cudaMemcpyAsync(m->block, blob.data(), at[6], cudaMemcpyHostToDevice, c->stream));
+    SLHA_CUDA(cudaMalloc(&m->block, at[7] + D_S * 8 + 256));
+    SLHA_CUDA(cudaMemcpyAsync(m->block, host.get(), at[4], cudaMemcpyHostToDevice, c->stream));
     const auto array = [&](int i) { return reinterpret_cast<float*>((char*)m->block + at[i]); };
     m->d_p = array(0);
-    m->d_pt = array(1);
-    m->d_scale = array(2);
-    m->d_z = array(3);
-    m->d_zt = array(4);
-    m->d_diag = rht ? array(5) : nullptr;
-    if (dp <= 256) SLHA_TRY(build_sign_fragments(c, m.get(), reinterpret_cast<uint4*>(array(6)), (char*)m->block + at[6] + zfb));
+    m->d_scale = array(1);
+    m->d_z = array(2);
+    m->d_diag = rht ? array(3) : nullptr;
+    m->d_pt = array(4);
+    m->d_zt = array(5);
+    SLHA_TRY(build_model_arrays(c, m.get(), reinterpret_cast<uint4*>(array(6)), array(7)));
     SLHA_CUDA(cudaStreamSynchronize(c->stream));
     *out = std::move(m);
     return Status();

@@ -27,6 +27,7 @@ struct ListView {
 // Candidate accessors: element e of query Q as a composite key, 0 = absent.
 struct CompLists {  // lists written by score_kernel
     static constexpr bool kFiltered = false;
+    static constexpr bool kDistinct = true;  // no key comes twice
     const uint64_t* keys;      // [n_lists][k] (k here = slots per list, >= the k asked for)
     const uint32_t* cnt;       // [n_lists]
     const uint32_t* q_list_begin;  // [nq]
@@ -57,6 +58,7 @@ struct CompLists {  // lists written by score_kernel
 // generic kernel's per-work-item lists.
 struct StreamLists {
     static constexpr bool kFiltered = true;
+    static constexpr bool kDistinct = true;  // no key comes twice
     const uint64_t* gbuf;                // [nq][gcap]
     const uint32_t* gcount;              // [nq]
     const uint32_t* gflag;               // [nq]
@@ -116,6 +118,7 @@ struct StreamLists {
 };
 struct PairLists {  // (index, score) lists laid out [list][query][k_in]
     static constexpr bool kFiltered = false;
+    static constexpr bool kDistinct = false;  // no key comes twice
     const uint32_t* idx;
     const float* score;
     uint32_t n_lists, n_queries, k_in;
@@ -436,6 +439,36 @@ __device__ void sort_and_emit(uint64_t* buf, uint32_t cap_s, int* hist, uint32_t
     emit_sorted(sorted, m, k, Q, out_index, out_score, out_count);
 }
 
+// The k best of buf[0..m), m <= RANK_MOST distinct keys, written where they belong: a key's place is the number of larger ones.  Every thread compares
+// its key with all of them, two per shared-memory load: no barrier after the gathering, where bucket placement takes eight and a
+// selection before it a dozen.  For short lists only: 64 winners of 4096 tiles 21.6 -> 20.7 us a call, but 256 of 8 x 8192 (300 keys)
+// 27.1 -> 34.9.
+constexpr uint32_t RANK_MOST = 128;  // (at most a thread each)
+__device__ __forceinline__ void rank_and_emit(uint64_t* buf, uint32_t m, uint32_t k, uint32_t Q, uint32_t* out_index, float* out_score, uint32_t* out_count) {
+    const uint32_t tid = threadIdx.x;
+    if (tid == 0) buf[m] = 0ull;  // (pairs)
+    __syncthreads();
+    if (tid < m) {
+        const ulonglong2* pairs = reinterpret_cast<const ulonglong2*>(buf);
+        const uint64_t x = buf[tid];
+        uint32_t r = 0;
+#pragma unroll 8
+        for (uint32_t e = 0; e < (m + 1) / 2; ++e) {
+            const ulonglong2 v = pairs[e];
+            r += (v.x > x) + (v.y > x);
+        }
+        if (r < k) {
+            out_index[(size_t)Q * k + r] = 0xFFFFFFFFu - (uint32_t)x;
+            out_score[(size_t)Q * k + r] = key_score((uint32_t)(x >> 32));
+        }
+    }
+    for (uint32_t r = m + tid; r < k; r += blockDim.x) {
+        out_index[(size_t)Q * k + r] = 0xFFFFFFFFu;
+        out_score[(size_t)Q * k + r] = -INFINITY;
+    }
+    if (out_count && tid == 0) out_count[Q] = min(m, k);
+}
+
 // cap_s: candidate slots of the shared-memory buffer (>= kp2).  When the query's
 // candidates fit they are gathered once and selected / sorted in shared memory;
 // otherwise the radix select runs over global memory.
@@ -525,6 +558,10 @@ __device__ __forceinline__ void topk_merge_body(const Lists& L, uint32_t k, uint
         const uint32_t present = (uint32_t)*n_s;
         __syncthreads();
         MPROBE_VAL(11, present);
+        if (Lists::kDistinct && present <= RANK_MOST && present < cap_s) {
+            rank_and_emit(buf, present, k, Q, out_index, out_score, out_count);
+            return;
+        }
         if (present > k) {
             // Lists filtered by a threshold that is proven to keep k candidates hold little more than k (up to 1.5 k here):
             // ordering them all and writing the first k is cheaper than selecting the k first.

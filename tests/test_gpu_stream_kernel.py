@@ -163,3 +163,62 @@ def test_mix3_rows_that_are_handed_back(nq, n_seg, n):
         qc[nq + 1] = 0  # (a row of 1e30: its winners are those of one element)
         rows = rows[:1] + rows[2:]
     _check_rows(tiles, rows, qc, qs, idx, sc, cnt, k, every=7 if n_seg > 9 else 1)
+
+
+@pytest.mark.parametrize("codec", [0, 2, 3, 4, 6])
+@pytest.mark.parametrize("nq", [1, 3, 4])
+def test_plain_shares_around_the_sets_of_sixteen_and_thirty_two(codec, nq):
+    # more than 74 streams: CTAs take contiguous shares, in sets of 32 tiles (NF4: 16), several segments in turn, some of them with WARM
+    # tiles, tiles without their correction plane and, in one segment, tiles of another codec (handed to the generic kernel)
+    lens = [1, 15, 16, 17, 31, 32, 33, 47, 63, 65, 767, 768, 769, 800, 1537, 0, 5, 24, 49, 2000] * 4
+    n, k = sum(lens), 40 + codec  # (plans are kept by shape, each for one codec)
+    tiles = H.random_tiles(3000, codec, seed=970 + codec, warm_every=9, nocorr_every=6)
+    tiles = np.tile(tiles, n // 3000 + 1)[:n].copy()
+    rng = np.random.default_rng(codec)
+    rng.shuffle(tiles)
+    rows, tb = [], 0
+    for i, m in enumerate(lens):
+        rows.append((tb, m, i * nq, nq, i))
+        tb += m
+    odd = rows[12]
+    tiles[odd[0] + 400:odd[0] + 403] = H.random_tiles(3, 3 if codec != 3 else 4, seed=5)
+    qc, qs = H.random_queries(nq * len(lens), 971)
+    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, nq * len(lens), k)
+    for tb, m, qb, _, base in rows:
+        for j in range(qb, qb + nq):
+            have = min(m, k)
+            assert cnt[j] == have
+            if not have:
+                continue
+            want = ora.score_tiles(tiles[tb:tb + m], qc[j], qs[j])
+            got = idx[j, :have].astype(np.int64) - base
+            assert len(set(got)) == have and got.min() >= 0 and got.max() < m
+            assert np.all(np.abs(sc[j, :have] - want[got]) <= 1e-3)
+            rest = np.delete(want, got)
+            assert not len(rest) or rest.max() <= want[got].min() + 2e-3
+
+
+@pytest.mark.parametrize("order", ["random", "rising", "falling", "equal", "negative lambda"])
+@pytest.mark.parametrize("codec,nq,k", [(0, 4, 16), (2, 1, 100), (3, 2, 300), (4, 4, 7)])
+def test_seeds_of_a_long_row(order, codec, nq, k):
+    # one row over all CTAs: few warps append their first sets unfiltered and the others wait for the thresholds these prove, whatever the
+    # scores' order.  (The residual term of a negative lambda has the same size: its tiles must not be passed over.)
+    n = 150_001
+    tiles = np.tile(H.random_tiles(5000, codec, seed=980 + codec), n // 5000 + 1)[:n].copy()
+    qc, qs = H.random_queries(nq, 981)
+    if order in ("rising", "falling"):
+        s = ora.score_tiles(tiles, qc[0], qs[0])
+        tiles = tiles[np.argsort(s if order == "rising" else -s, kind="stable")]
+    elif order == "equal":
+        tiles[:] = tiles[0]
+    elif order == "negative lambda":
+        tiles["dynamic_lambda"] = np.where(np.arange(n) % 3 == 0, -0.05, 0.0).astype(F)
+    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments([(0, n, 0, nq, 0)]), qc, qs, nq, k)
+    for j in range(nq):
+        want = ora.score_tiles(tiles, qc[j], qs[j])
+        assert cnt[j] == k and len(set(idx[j])) == k
+        assert np.all(np.abs(sc[j] - want[idx[j]]) <= 1e-3 * (1 + np.abs(want[idx[j]])))
+        rest = np.delete(want, idx[j])
+        assert rest.max() <= want[idx[j]].min() + 2e-3 * (1 + np.abs(want).max())
+        if order == "equal":
+            assert np.array_equal(idx[j], np.arange(k))  # ties go to the lower index
