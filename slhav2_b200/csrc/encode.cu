@@ -12,7 +12,9 @@
 // owns whole output rows and walks the contraction index sequentially with
 // __fmul_rn / __fadd_rn (never contracted into FMA), divisions are __fdiv_rn and
 // square roots __fsqrt_rn.  Parallelism comes from rows x keys, not from
-// splitting a sum, so the tile bytes equal the scalar reference's bit for bit.
+// splitting a sum, so the tile bytes equal the scalar reference's bit for bit.  Where
+// only a decision is stored (sign bits, codes), it is taken on a cheaper value with a
+// bound on its error, and on the exact one where the bound does not settle it.
 #include <cuda_fp16.h>
 
 #include "common.cuh"
@@ -250,8 +252,8 @@ __device__ __forceinline__ void load_keys(float (&v)[NK], const float* src) {
 // kernel's arguments: product * 1 is exact, so it rounds once, like an addition.  A plain packed addition would be contracted
 // with the multiply before it into one fused multiply-add even when both carry an explicit rounding mode and contraction is
 // switched off (seen on sm_100a, CUDA 12.9), and a fused multiply-add rounds once where the reference rounds twice.
-// Bound: 131 072 multiplies and additions per key at d = 128 on 128 fp32 lanes per SM (284 M keys/s).  262 144 bf16 keys: 1251 us
-// (1327 us with scalar sums, three issue slots instead of two).
+// Bound: 65 536 multiplies and additions per key (latent and residual) at d = 128 on 128 fp32 lanes per SM: 568 M keys/s, 461 us for
+// 262 144 bf16 keys, which take 747 us.  (With the signs in the same form 1251 us, with scalar sums, three issue slots instead of two, 1327.)
 __device__ __forceinline__ uint64_t pack2(float lo, float hi) {
     uint64_t r;
     asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "f"(lo), "f"(hi));
@@ -1065,9 +1067,9 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
     if (encode_smem(a.d_pad, kb) > 200 * 1024)
         return Status(SLHA_ERR_DIMENSION, "model dimension too large for the encode kernel");
     // Few keys: the narrowest CTA of at least 4 keys that leaves no SM a second one.  Measured (d = 128, bf16,
-    // us per call at 8 / 592 / 1184 / 2368 / 4736 keys): 32 keys per CTA 39 / 39 / 37 / 37 / 37, 16: 29 / 28 / 29 / 29 / 39,
-    // 8: 21 / 21 / 21 / 27 / 49, 4: 17 / 19 / 21 / 37 / 70, 1: 17 / 31 / 59 / 113 / 221 -- a CTA of 4 keys is as fast as one of a
-    // single key, and a wider form is no slower from where the narrower one fills the SMs twice.
+    // us per call at 8 / 592 / 1184 / 2368 / 4736 keys): 32 keys per CTA 35 / 32 / 29 / 29 / 30, 16: 23 / 19 / 19 / 20 / 38,
+    // 8: 13 / 14 / 14 / 27 / 50, 4: 12 / 13 / 25 / 44 / 83 -- a wider form is no slower from where the narrower one fills the SMs
+    // twice.
     while (kb > 4 && n <= (uint64_t)(kb / 2) * (uint64_t)sm_count(m->device)) kb >>= 1;
     *kb_out = kb;
     a.kb = kb;
@@ -1085,10 +1087,10 @@ Status run_encode_kb(Ctx* c, EncodeArgs& a) {
         configured[c->device & 15] = true;
     }
     const uint64_t groups = (a.n + KB - 1) / KB;
-    // far more CTAs than fit at once (444 are resident at head dimension 128): the hardware hands
+    // far more CTAs than fit at once (592 are resident at head dimension 128): the hardware hands
     // out a CTA whenever one finishes, which balances the tail and keeps the CTAs sharing an SM in
     // different phases, so that the arithmetic of one covers the loads, quantisation and barriers
-    // of the others.  One resident wave measured 182 M keys/s, 8 CTAs per SM 191, one CTA per pass 199.
+    // of the others.  (One resident wave measured 182 M keys/s, 8 CTAs per SM 191, one CTA per pass 199, when the signs were summed in order.)
     const uint32_t grid = (uint32_t)std::min<uint64_t>(groups, 148ull * 64);
     SLHA_CUDA(launch_behind(encode_kernel<QUERY, KB>, dim3(grid), dim3(enc_threads(KB)), smem, c->stream, a));
     count_launch();

@@ -35,11 +35,11 @@ constexpr int MMA_HALF = 8 * MMA_ROW;                      // row g -> row g + 8
 constexpr uint32_t MMA_CHUNK = 16;  // slots a warp reserves at a time in a row's candidate buffer (larger chunks measured no faster)
 // score_stream_kernel: a warp takes sets of U x 16 tiles.  Shared layout: query fragments, sign words, thresholds (the tail) | stage ring, and
 // for launches with NF4 tiles (KIND 0) tail | ring of the first warps | NF4 table at 64 KB | ring of the others.
-#ifndef SLHA_U12
-#define SLHA_U12 2
-#endif
-constexpr int stream_sets(int kind, bool il) { return il || kind == 0 ? 1 : (kind == 3 ? 2 : SLHA_U12); }
-constexpr int stream_threads(int kind, int u) { return 768; }
+// U = 2 on long shares: 8 x 1M MX-32 tiles 274 -> 247 us a call (16 tiles at a time cost 483 instructions, 32 tiles 2 x 291), 8 x 524 288 mixed and TQ3
+// tiles the same as with 1.  Not for NF4, whose 128 registers leave 16 warps an SM (457 us for 256 x 32 768 tiles; 439 with sets of 16 and
+// 24 warps), nor for interleaved shares, whose first sets are appended unfiltered (a million MX-16 tiles on one row, k = 100: 81 us, with U = 2 102).
+constexpr int stream_sets(int kind, bool il) { return il || kind == 0 ? 1 : 2; }
+constexpr int stream_threads(int, int) { return 768; }  // 24 warps at 80 registers: latencies are hidden with warps (U = 2 with 20 or 16 warps: 251, 254 us)
 constexpr int MMA_DEPTH = SLHA_MMA_DEPTH;                  // cp.async ring slots per warp
 constexpr int MMA_BQ_BYTES = 9 * 32 * 8;                   // B fragments of a work item: [9][32 lanes] x 8 bytes
 constexpr int MMA_TAIL_BYTES = 2560;                       // fragments | sign words 128 | thresholds 16 | bucket mappings 32 + 32 | flag 16
