@@ -532,8 +532,8 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // few rows with long buffers: several CTAs per row compact the survivors before the merge
     // (a slice of at most 1024 slots per CTA: one round of four keys per thread)
     // (up to 256 rows: 128 rows of 15 k MIX3 tiles 69.4 -> 65.0 us, 160 rows of 30 000 INT4 tiles 86.9 -> 82.2; with 1024 rows of 32 768 NF4 tiles the
-    // merge's own CTAs fill the GPU and the extra pass costs 28 us of 441, with 512 of the 64-row kernel 10 of 85)
-    p->compact_splits = (p->use_mma && nq <= 256 && expect >= 8192) ? (uint32_t)std::min<size_t>(64, std::max<size_t>((296 + nq - 1) / nq, (expect + 1023) / 1024)) : 0;
+    // merge's own CTAs fill the GPU and the extra pass costs 28 us of 441; rows of the 64-row kernel are short: 512 of them 10 of 85, 192 7 of 133)
+    p->compact_splits = (p->use_mma && (nq < 128 || (nq <= 256 && !p->wide)) && expect >= 8192) ? (uint32_t)std::min<size_t>(64, std::max<size_t>((296 + nq - 1) / nq, (expect + 1023) / 1024)) : 0;
     p->selcap = merge_cap((uint64_t)p->gcap, p->kp2, k);
     if (p->compact_splits) SLHA_TRY(p->b_gsel.ensure(nq * (size_t)p->selcap * 8));
     SLHA_TRY(p->b_gpivot.ensure(p->gstate_bytes));
