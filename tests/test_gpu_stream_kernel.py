@@ -198,6 +198,20 @@ def test_plain_shares_around_the_sets_of_sixteen_and_thirty_two(codec, nq):
             assert not len(rest) or rest.max() <= want[got].min() + 2e-3
 
 
+@pytest.mark.parametrize("codec,nq,k", [(0, 4, 60), (3, 3, 61), (4, 1, 62), (2, 4, 63)])
+def test_plain_shares_of_long_segments_end_inside_a_set_of_thirty_two(codec, nq, k):
+    # work items of more than 10 000 tiles take sets of 32 (NF4: 16); segments end at every place of a set, and the last segments share tiles
+    lens = [12_000 + i for i in range(33)] + [16_384, 10_001, 20_000] + [13_000 + 5 * i for i in range(40)]
+    base = np.tile(H.random_tiles(4000, codec, seed=960 + codec, warm_every=9, nocorr_every=6), 6)
+    rng = np.random.default_rng(codec)
+    rng.shuffle(base)
+    rows = [(int(rng.integers(0, len(base) - m + 1)), m, i * nq, nq, 2 * i) for i, m in enumerate(lens)]
+    qc, qs = H.random_queries(nq * len(lens), 961)
+    idx, sc, cnt = S.score_topk(S.to_device(base), S.make_segments(rows), qc, qs, nq * len(lens), k)
+    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
+    _check_rows(base, rows, qc, qs, idx, sc, cnt, k, every=3)
+
+
 @pytest.mark.parametrize("order", ["random", "rising", "falling", "equal", "negative lambda"])
 @pytest.mark.parametrize("codec,nq,k", [(0, 4, 16), (2, 1, 100), (3, 2, 300), (4, 4, 7)])
 def test_seeds_of_a_long_row(order, codec, nq, k):
