@@ -25,20 +25,21 @@ constexpr int ATT_THREADS = 256;
 constexpr int ATT_FLIGHT = 12; // value loads a thread issues before it uses the first
 
 // VEC columns of a value row (4 or 16 bytes; one element of a float32 or bfloat16 row), loaded when `p` holds, else zero.
-// (Predicated loads in volatile statements, so that a thread's loads stay together in front of their uses.)
+// (Predicated loads in volatile statements, so that a thread's loads stay together in front of their uses.  Coherent ones: this grid may be
+// resident while the values are written, see dep_wait.)
 template <typename T, int VEC>
 struct Values {
     uint32_t x[VEC == 1 ? 1 : 4];
     __device__ __forceinline__ void load(const T* src, bool p) {
         if constexpr (VEC > 1) {
             asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %5, 0;\nmov.u32 %0, 0;\nmov.u32 %1, 0;\nmov.u32 %2, 0;\nmov.u32 %3, 0;\n"
-                         "@p ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];\n}\n"
+                         "@p ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n}\n"
                          : "=&r"(x[0]), "=&r"(x[1]), "=&r"(x[2]), "=&r"(x[3]) : "l"(src), "r"((uint32_t)p));
         } else if constexpr (sizeof(T) == 4) {
-            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\nmov.u32 %0, 0;\n@p ld.global.nc.u32 %0, [%1];\n}\n" : "=&r"(x[0]) : "l"(src), "r"((uint32_t)p));
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\nmov.u32 %0, 0;\n@p ld.global.u32 %0, [%1];\n}\n" : "=&r"(x[0]) : "l"(src), "r"((uint32_t)p));
         } else {
             uint16_t h;
-            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\nmov.u16 %0, 0;\n@p ld.global.nc.u16 %0, [%1];\n}\n" : "=&h"(h) : "l"(src), "r"((uint32_t)p));
+            asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %2, 0;\nmov.u16 %0, 0;\n@p ld.global.u16 %0, [%1];\n}\n" : "=&h"(h) : "l"(src), "r"((uint32_t)p));
             x[0] = h;
         }
     }

@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kern
         if (KB >= 8 && d % epc == 0 && (reinterpret_cast<uintptr_t>(a.keys) & 15) == 0) {
             // 16-byte chunks; the lanes of a warp take the same chunk of consecutive keys, so
             // that their transposed stores fall on consecutive banks.  All loads of a thread
-            // are in flight before the first store.
+            // are in flight before the first store.  (Ordinary loads: this grid may be resident while the keys are written, see dep_wait.)
             constexpr int U = 512 / NT;
             const uint32_t cpk = d / epc, total = cpk * (uint32_t)KB;
             const uint4* src = reinterpret_cast<const uint4*>(a.keys) + base * cpk;
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kern
                 for (int u = 0; u < U; ++u) {
                     const uint32_t c = c0 + u * NT, j = c % KB, ic = c / KB;
                     v[u] = make_uint4(0u, 0u, 0u, 0u);
-                    if (c < total && (int)j < nk) v[u] = __ldg(src + (size_t)j * cpk + ic);
+                    if (c < total && (int)j < nk) v[u] = src[(size_t)j * cpk + ic];
                 }
 #pragma unroll
                 for (int u = 0; u < U; ++u) {

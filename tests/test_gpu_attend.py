@@ -124,3 +124,40 @@ def test_attend_of_many_rows_takes_smaller_clusters(nq, k):
     some = rng.choice(nq, min(nq, 40), replace=False)
     want, want_w = ora.attend_topk(idx[some], sc[some], 0.1, values, top_count=counts[some])
     assert close(w_out[some], want_w) and close(out[some], want)
+
+
+def test_attention_feeds_attention_queries_and_keys_without_a_wait_between():
+    # attend's grids let the next kernel on the stream start early: what they write is the next call's values, queries or keys, in the same
+    # buffers call after call (1500 rows: the wide loads of the encoder, full 16-byte value loads)
+    n, k, d = 1500, 8, 128
+    rng = np.random.default_rng(5)
+    gm = S.Model.from_projection(H.orthogonal_projection(11, d), d, 7)
+    idx = S.to_device(rng.integers(0, n, (n, k)).astype(np.uint32))
+    sc = S.to_device(rng.standard_normal((n, k)).astype(F))
+    idx.numel = lambda: n * k  # (attend_topk takes the number of rows from it)
+    values = [S.to_device(rng.standard_normal((n, d)).astype(F)) for _ in range(3)]
+    mid, out, qc, qs, tiles = [S.DeviceBuffer(n * m) for m in (4 * d, 4 * d, 512, 32, 128)]
+
+    def step(v, wait):
+        S.attend_topk(idx, sc, k, 0.7, v, d, out=mid)
+        wait()
+        S.attend_topk(idx, sc, k, 0.7, mid, d, out=out)
+        wait()
+        gm.prepare_queries(out, nq=n, q_coarse_out=qc, q_sign_out=qs)
+        wait()
+        S.attend_topk(idx, sc, k, 0.3, mid, d, out=out)
+        wait()
+        gm.encode_keys(out, 2, n=n, out=tiles)
+
+    def results():
+        S.synchronize()
+        return [b.download(np.uint8, b.nbytes) for b in (qc, qs, tiles)]
+
+    want = []
+    for v in values:
+        step(v, S.synchronize)
+        want.append(results())
+    for r in range(30):
+        for i in range(r % 3 + 1):
+            step(values[i], lambda: None)
+        assert all(np.array_equal(g, w) for g, w in zip(results(), want[r % 3])), r

@@ -1,0 +1,32 @@
+"""Rules of the CUDA sources that no run shows: they are read as text."""
+import glob
+import os
+import re
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+def _sources():
+    for path in sorted(glob.glob(os.path.join(ROOT, "slhav2_b200", "csrc", "*.cu*"))):
+        text = re.sub(r"/\*.*?\*/|//[^\n]*", "", open(path).read(), flags=re.S)
+        yield os.path.basename(path), text
+
+
+def test_only_the_models_own_arrays_are_read_through_the_non_coherent_path():
+    # Kernels are launched while their predecessor on the stream still runs and wait for it on the device.  Non-coherent loads need memory that
+    # nobody writes from the grid's start on: a model's arrays, complete before the model is handed out, but no argument of a call.
+    models = r"^(zf|next|mp|diag|a\.z|reinterpret_cast<const float4\*>\(a\.scale\))(?!\w)"
+    for name, text in _sources():
+        assert "global.nc" not in text, name
+        for m in re.finditer(r"__ldg\(((?:[^()]|\([^()]*\))*)", text):
+            assert name == "encode.cu" and re.match(models, m.group(1)), (name, m.group(0))
+        if "__ldg" in text:  # what those names point to
+            for var, arrays in (("zf", "a.zf"), ("next", "zf"), ("mp", "a.p|a.pt|a.zt"), ("diag", None)):
+                for d in re.finditer(r"\bconst \w+\* %s = ([^;]*);" % var, text):
+                    assert arrays and re.search(r"\b(%s)\b" % arrays.replace(".", r"\."), d.group(1)), (var, d.group(0))
+
+
+def test_every_kernel_that_lets_the_next_one_start_waits_for_the_one_before_it():
+    for name, text in _sources():
+        for m in re.finditer(r"\bdep_launch\(\);\s*(\S+)", text):
+            assert m.group(1).startswith("dep_wait()"), (name, m.group(0))
