@@ -510,22 +510,23 @@ __device__ __forceinline__ bool signs_mma(const EncodeArgs& a, const float* buf,
     for (uint32_t e0 = 0; e0 < again; e0 += room) {
         const uint32_t n = min(room, again - e0);
         // (eight rows a warp at a time: their numbers are read before the first copy is issued)
-        for (uint32_t e = warp; e < n; e += 8 * WARPS) {
+        for (uint32_t e = warp; dp % 4 == 0 && e < n; e += 8 * WARPS) {
             uint32_t row[8];
 #pragma unroll
             for (int q = 0; q < 8; ++q) row[q] = e + q * WARPS < n ? (list[e0 + e + q * WARPS] & 255u) * dp : ~0u;
-            if (dp % 4 == 0) {
-                const uint32_t to = (uint32_t)__cvta_generic_to_shared(zs + e * stride);
-                for (uint32_t i = 4 * lane; i < dp; i += 128)
+            const uint32_t to = (uint32_t)__cvta_generic_to_shared(zs + e * stride);
+            for (uint32_t i = 4 * lane; i < dp; i += 128)
 #pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (row[q] != ~0u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to + 4 * (q * WARPS * stride + i)), "l"(a.z + row[q] + i));
-            } else {
-                for (uint32_t i = lane; i < dp; i += 32)
-#pragma unroll
-                    for (int q = 0; q < 8; ++q)
-                        if (row[q] != ~0u) zs[(e + q * WARPS) * stride + i] = __ldg(a.z + row[q] + i);
-            }
+                for (int q = 0; q < 8; ++q)
+                    if (row[q] != ~0u) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to + 4 * (q * WARPS * stride + i)), "l"(a.z + row[q] + i));
+        }
+        // (rows that start at any word: by words, and copied all the same; through registers 300 queries of 202 dimensions took 24.5 us a call, now 15.8)
+#pragma unroll 1
+        for (uint32_t e = warp; dp % 4 != 0 && e < n; e += WARPS) {
+            const float* z = a.z + (list[e0 + e] & 255u) * dp;
+            const uint32_t to = (uint32_t)__cvta_generic_to_shared(zs + e * stride);
+#pragma unroll 1
+            for (uint32_t i = lane; i < dp; i += 32) asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(to + 4 * i), "l"(z + i));
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
@@ -629,9 +630,12 @@ __device__ __forceinline__ void fwht_stages(float* buf, uint32_t dp, uint32_t lo
 // contraction is walked sequentially by the thread that owns the output element, for all the keys
 // the thread holds at once.
 
+// CTAs of KB keys whose registers fit on an SM together: four of 32 keys at head dimension 128 (57 KB of shared memory each), two of 16 or 8.  (16
+// keys with 180 registers, one CTA an SM: 20 011 keys of 512 dimensions 772 us, with 123 registers 593.)
+constexpr int enc_ctas(int kb) { return kb == 32 ? 4 : (kb >= 8 ? 2 : 1); }
+
 template <bool QUERY, int KB>
-// (four CTAs of 32 keys share an SM at head dimension 128: up to 128 registers, 57 KB of shared memory each)
-__global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kernel(EncodeArgs a) {
+__global__ void __launch_bounds__(enc_threads(KB), enc_ctas(KB)) encode_kernel(EncodeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     dep_launch();
     dep_wait();
@@ -750,7 +754,7 @@ __global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kern
                 float acc[PER];
 #pragma unroll
                 for (int j = 0; j < PER; ++j) acc[j] = 0.0f;
-#pragma unroll KB <= 8 ? 32 : 8
+#pragma unroll KB <= 8 ? 32 : (KB == 16 ? 16 : 8)
                 for (uint32_t i = 0; i < d; ++i)
                     axpy_keys<PER>(acc, a.pt[(size_t)i * D_C + k], buf + (size_t)i * KS + j0);
                 const float sk = a.scale[k];
@@ -813,7 +817,7 @@ __global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kern
 #pragma unroll
                 for (int j = 0; j < PER; ++j) acc[j] = 0.0f;
                 const float* wr = wsT + half * PER;
-#pragma unroll KB <= 8 ? 32 : 8
+#pragma unroll KB <= 8 ? 32 : (KB == 16 ? 16 : 8)
                 for (int k = 0; k < D_C; ++k) axpy_keys<PER>(acc, a.p[(size_t)k * d + i], wr + (size_t)k * KS);
                 float kv[PER];
                 load_keys<PER>(kv, buf + (size_t)i * KS + half * PER);
@@ -908,7 +912,8 @@ __global__ void __launch_bounds__(enc_threads(KB), KB == 32 ? 4 : 1) encode_kern
             float acc[KB];
 #pragma unroll
             for (int j = 0; j < KB; ++j) acc[j] = 0.0f;
-#pragma unroll 8
+// (16 keys: loads of 16 steps in flight together, as in the two phases above: 7000 keys of 448 dimensions 182 us, with 8 steps 231)
+#pragma unroll KB == 16 ? 16 : 8
             for (uint32_t i = 0; i < dp; ++i) axpy_keys<KB>(acc, a.zt[(size_t)i * D_S + s], buf + (size_t)i * KS);
 #pragma unroll
             for (int j = 0; j < KB; ++j) {
@@ -1061,16 +1066,21 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
     a.fwht_inv = 1.0f / sqrtf((float)m->d_pad);
     a.one = 0x3F8000003F800000ull;
     a.lambda_c = sqrtf(3.14159265358979323846f / (2.0f * (float)D_S));
-    // 32 keys per CTA pass when two CTAs still share an SM (their registers allow no more), else fewer
+    // 32 keys per CTA pass up to 100 KB of shared memory (d_pad <= 440: 20 011 keys of 440 dimensions 411 us, with 16 keys 530), else fewer
     int kb = 32;
     while (kb > 1 && encode_smem(a.d_pad, kb) > (kb == 32 ? 100 : 200) * 1024) kb >>= 1;
     if (encode_smem(a.d_pad, kb) > 200 * 1024)
         return Status(SLHA_ERR_DIMENSION, "model dimension too large for the encode kernel");
-    // Few keys: the narrowest CTA of at least 4 keys that leaves no SM a second one.  Measured (d = 128, bf16,
-    // us per call at 8 / 592 / 1184 / 2368 / 4736 keys): 32 keys per CTA 35 / 32 / 29 / 29 / 30, 16: 23 / 19 / 19 / 20 / 38,
-    // 8: 13 / 14 / 14 / 27 / 50, 4: 12 / 13 / 25 / 44 / 83 -- a wider form is no slower from where the narrower one fills the SMs
-    // twice.
-    while (kb > 4 && n <= (uint64_t)(kb / 2) * (uint64_t)sm_count(m->device)) kb >>= 1;
+    // The 4 x 8 register tiles, which make 32 keys pay, need d % 4 == 0.  Without them 16 keys are faster where the signs are summed in order too
+    // (2400 keys of 258 dimensions 73 us, with 32 keys 117; 60 000: 930, 910) and up to two waves of their CTAs (9000 keys of 202 dimensions 92, 115;
+    // 12 000: 131, 117).
+    const uint64_t sms = (uint64_t)sm_count(m->device);
+    if (kb == 32 && m->d % 4 != 0 && (!m->d_zf || n <= 16 * 2 * 2 * sms)) kb = 16;
+    // Few keys: the narrowest CTA of at least 4 keys whose CTAs are all on the GPU at once, one (4 keys) or two (8, 16) an SM.  Measured (us per call,
+    // float32, at 592 / 1184 / 2368 / 4736 keys): d = 128: 4 keys 14 / 25 / 45 / 84, 8: 14 / 15 / 19 / 36, 16: 19 / 19 / 20 / 27, 32: 33 / 30 / 30 / 31;
+    // d = 320: 4: 30 / 58 / 113 / 224, 8: 36 / 36 / 52 / 102, 16: 59 / 59 / 59 / 84, 32: 89 / 88 / 89 / 89.  With the next width from one CTA an SM on, 2400 keys
+    // of 288 dimensions took 89 us instead of 78, 1800 queries of 512 dimensions 85 instead of 54.
+    while (kb > 4 && n <= (uint64_t)(kb / 2 * enc_ctas(kb / 2)) * sms) kb >>= 1;
     *kb_out = kb;
     a.kb = kb;
     // (the sign phase works in the space of h and the reconstruction factors)
@@ -1080,13 +1090,16 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
 
 template <bool QUERY, int KB>
 Status run_encode_kb(Ctx* c, EncodeArgs& a) {
-    const size_t smem = encode_smem(a.d_pad, KB);
+    size_t smem = encode_smem(a.d_pad, KB);
+    const uint64_t groups = (a.n + KB - 1) / KB;
+    // (Where an SM holds two CTAs and every CTA can have one to itself, more than half of an SM's shared memory keeps them apart: 900 keys of 512 dimensions,
+    // 113 CTAs, took 76 us and 1184, 148 CTAs, 54.)
+    if (enc_ctas(KB) == 2 && groups <= (uint64_t)sm_count(c->device)) smem = std::max<size_t>(smem, 116 * 1024);
     static thread_local bool configured[16] = {false};  // the attribute is per device
     if (!configured[c->device & 15]) {
         SLHA_CUDA(cudaFuncSetAttribute(encode_kernel<QUERY, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         configured[c->device & 15] = true;
     }
-    const uint64_t groups = (a.n + KB - 1) / KB;
     // far more CTAs than fit at once (592 are resident at head dimension 128): the hardware hands
     // out a CTA whenever one finishes, which balances the tail and keeps the CTAs sharing an SM in
     // different phases, so that the arithmetic of one covers the loads, quantisation and barriers

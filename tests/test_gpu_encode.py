@@ -183,7 +183,29 @@ def test_small_batches_take_narrower_ctas_and_give_the_same_bytes(d, rht, codec)
         assert np.array_equal(c, qc[:k]) and np.array_equal(s, qs[:k]), k
 
 
-@pytest.mark.parametrize("n", [5, 700, 1500, 5000])  # 4, 8, 16 and 32 keys per CTA
+@pytest.mark.parametrize("d,rht", [(130, False), (202, False), (257, False), (258, True), (320, False), (440, False), (448, False), (300, True), (640, False)])
+def test_models_of_every_width_give_the_same_bytes_at_every_number_of_keys_per_cta(d, rht):
+    """Dimensions that are no multiple of four, above 256 (every sign from its exact sum) and above 440 (16 keys per CTA at most), at the batch sizes around
+    which the number of keys per CTA changes: the oracle's bytes for a sample of a large batch, and for every prefix the bytes of the whole."""
+    om, gm = _models(d, rht, seed=7)
+    n, rng = 9500, np.random.default_rng(d)
+    keys = H.gaussian_keys(d, n, d, outlier_channels=(7, d - 1))
+    pos = rng.integers(0, 2**32, n, dtype=np.uint32)
+    whole = gm.encode_keys(keys, 2, positions=pos)
+    qc, qs = gm.prepare_queries(keys)
+    some = np.unique(np.concatenate([[0, n - 1], rng.choice(n, 150, replace=False)]))
+    want = om.encode_batch(keys[some], 2, pos=pos[some])
+    assert whole[some].tobytes() == want.tobytes(), _diff(whole[some], want)
+    for j in some[::10]:
+        wc, ws = om.prepare_query(keys[j])
+        assert np.array_equal(qs[j], ws) and np.array_equal(qc[j].view(np.uint32), wc.view(np.uint32))
+    for k in (1, 592, 593, 1184, 1185, 2368, 2369, 4736, 4737, 9472, 9473):
+        assert np.array_equal(gm.encode_keys(keys[:k], 2, positions=pos[:k]).view(np.uint8), whole[:k].view(np.uint8)), k
+        c, s = gm.prepare_queries(keys[:k])
+        assert np.array_equal(c.view(np.uint32), qc[:k].view(np.uint32)) and np.array_equal(s, qs[:k]), k
+
+
+@pytest.mark.parametrize("n", [5, 700, 1500, 2500, 5000])  # 4, 8 (one and two CTAs an SM), 16 and 32 keys per CTA
 @pytest.mark.parametrize("d,rht", [(128, False), (160, True), (72, False), (129, True), (256, False)])
 def test_sign_bits_near_and_at_zero_follow_the_exact_sums(n, d, rht):
     """The signs come from fp16 sums unless those are too close to zero: residuals that are orthogonal to hyperplanes up to
