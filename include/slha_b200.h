@@ -201,6 +201,10 @@ int32_t slha_b200_debug_force_generic_score(int32_t on);
  * out[2] candidates the rows' buffers received in all, out[3] slots per buffer.
  * Waits for the stream.  All zero when no such call has run. */
 int32_t slha_b200_last_score_stats(uint64_t* out /* 4 values */);
+/* Checking aid: how many tiles a warp took at a time (16 or 32) in that call; 0 for
+ * calls of the kernels that do not work in such sets (MIX3 tiles, 16 rows or more a
+ * segment) and when no such call has run. */
+int32_t slha_b200_debug_last_score_set(uint32_t* out);
 /* Device timing of the fused score + top-k path: after timing_begin, each of
  * the calling thread's next `max_calls` slha_b200_score_topk /
  * slha_b200_pool_score_topk calls records CUDA events on its stream around the

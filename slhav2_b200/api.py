@@ -75,6 +75,7 @@ SIGNATURES = {
     "slha_b200_launch_count": (_u64, []),
     "slha_b200_debug_force_generic_score": (_i32, [_i32]),
     "slha_b200_last_score_stats": (_i32, [_vp]),
+    "slha_b200_debug_last_score_set": (_i32, [_vp]),
     "slha_b200_timing_begin": (_i32, [_u32]),
     "slha_b200_timing_end": (_i32, [_vp, _vp, _u32, _vp]),
     "slha_b200_malloc": (_i32, [_sz, C.POINTER(_vp)]),
@@ -206,6 +207,13 @@ def last_score_stats():
     out = np.zeros(4, np.uint64)
     _check(load_library().slha_b200_last_score_stats(ptr(out)))
     return {"rows": int(out[0]), "rows_handed_to_generic_kernel": int(out[1]), "candidates_appended": int(out[2]), "buffer_slots": int(out[3])}
+
+
+def debug_last_score_set():
+    """Checking aid: tiles a warp took at a time in this thread's latest tensor-core score_topk call (16 or 32; 0: a kernel without such sets)."""
+    out = np.zeros(1, np.uint32)
+    _check(load_library().slha_b200_debug_last_score_set(ptr(out)))
+    return int(out[0])
 
 
 def timing_begin(max_calls):

@@ -58,6 +58,15 @@ int32_t slha_b200_last_score_stats(uint64_t* out) {
         return last_score_stats(c, out);
     });
 }
+int32_t slha_b200_debug_last_score_set(uint32_t* out) {
+    return ffi([&]() -> Status {
+        if (!out) return Status(SLHA_ERR_NULL, "slha_b200_debug_last_score_set received a NULL pointer");
+        Ctx* c;
+        SLHA_TRY(get_ctx(&c));
+        *out = last_score_set(c);
+        return Status();
+    });
+}
 int32_t slha_b200_timing_begin(uint32_t max_calls) {
     return ffi([&]() -> Status {
         Ctx* c;

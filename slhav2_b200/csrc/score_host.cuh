@@ -1000,6 +1000,12 @@ Status last_score_stats(Ctx* c, uint64_t* out4) {
     return Status();
 }
 
+// Tiles a warp of that call took at a time.
+uint32_t last_score_set(Ctx* c) {
+    const Plan* p = g_last_stream_plan;
+    return !p || p->device != c->device || !p->use_mma || p->wide || p->kind == 4 ? 0u : (uint32_t)(MMA_SET_TILES * p->sets);
+}
+
 bool timing_active() { return g_timing.calls < g_timing.max_calls; }
 
 Status timing_begin(uint32_t max_calls) {

@@ -38,9 +38,11 @@ constexpr uint32_t MMA_CHUNK = 16;  // slots a warp reserves at a time in a row'
 // U = 2 on long shares: 8 x 1M MX-32 tiles 274 -> 247 us a call (16 tiles at a time cost 483 instructions, 32 tiles 2 x 291), 8 x 524 288 mixed and TQ3
 // tiles the same as with 1.  Not for NF4, whose 128 registers leave 16 warps an SM (457 us for 256 x 32 768 tiles; 439 with sets of 16 and
 // 24 warps), nor for interleaved shares, whose first sets are appended unfiltered (a million MX-16 tiles on one row, k = 100: 81 us, with U = 2 102).
-// From 10 000 tiles a work item on (the plan's average): a CTA's first sets of an item are appended unfiltered, twice as many of them with U = 2 (us a call
-// with 1 / 2: 200 segments of 3000 INT4 tiles 58 / 65, of 8000 106 / 110, of 12 000 mixed tiles 139 / 138, 150 of 16 000 INT4 tiles 151 / 144).
-constexpr int stream_sets(int kind, bool il, uint64_t item_tiles) { return il || kind == 0 || item_tiles < 10000 ? 1 : 2; }
+// From 6400 (INT4, MX-INT4) or 10 000 tiles a work item on (the plan's average: segments are cut at the CTAs' shares too): a CTA's first sets of an item are
+// appended unfiltered, twice as many of them with U = 2.  us a call with 1 / 2 at average items of 4878 (200 segments of 8000 tiles, k = 64), 6521 (150 of 12 000), 8510
+// (150 of 16 000), 14 545 (80 of 40 000): INT4 92 / 94, 88 / 86, 104 / 102, 113 / 104; mixed 96 / 101, 95 / 96, 115 / 116, 129 / 126; TQ3 119 / 128, 123 / 126,
+// 151 / 155, 173 / 173; with k = 1024 at 8510 and 14 545: INT4 152 / 147, 158 / 152, mixed 156 / 149, 164 / 160, TQ3 189 / 185, 209 / 208.
+constexpr int stream_sets(int kind, bool il, uint64_t item_tiles) { return il || kind == 0 || item_tiles < (kind == 3 ? 6400 : 10000) ? 1 : 2; }
 constexpr int stream_threads(int, int) { return 768; }  // 24 warps at 80 registers: latencies are hidden with warps (U = 2 with 20 or 16 warps: 251, 254 us)
 constexpr int MMA_DEPTH = SLHA_MMA_DEPTH;                  // cp.async ring slots per warp
 constexpr int MMA_BQ_BYTES = 9 * 32 * 8;                   // B fragments of a work item: [9][32 lanes] x 8 bytes

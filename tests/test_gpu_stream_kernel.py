@@ -168,7 +168,7 @@ def test_mix3_rows_that_are_handed_back(nq, n_seg, n):
 @pytest.mark.parametrize("codec", [0, 2, 3, 4, 6])
 @pytest.mark.parametrize("nq", [1, 3, 4])
 def test_plain_shares_around_the_sets_of_sixteen_and_thirty_two(codec, nq):
-    # more than 74 streams: CTAs take contiguous shares, in sets of 32 tiles (NF4: 16), several segments in turn, some of them with WARM
+    # more than 74 streams: CTAs take contiguous shares, in sets of 16 tiles (items are short), several segments in turn, some of them with WARM
     # tiles, tiles without their correction plane and, in one segment, tiles of another codec (handed to the generic kernel)
     lens = [1, 15, 16, 17, 31, 32, 33, 47, 63, 65, 767, 768, 769, 800, 1537, 0, 5, 24, 49, 2000] * 4
     n, k = sum(lens), 40 + codec  # (plans are kept by shape, each for one codec)
@@ -184,6 +184,7 @@ def test_plain_shares_around_the_sets_of_sixteen_and_thirty_two(codec, nq):
     tiles[odd[0] + 400:odd[0] + 403] = H.random_tiles(3, 3 if codec != 3 else 4, seed=5)
     qc, qs = H.random_queries(nq * len(lens), 971)
     idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, nq * len(lens), k)
+    assert S.debug_last_score_set() == 16
     for tb, m, qb, _, base in rows:
         for j in range(qb, qb + nq):
             have = min(m, k)
@@ -198,18 +199,75 @@ def test_plain_shares_around_the_sets_of_sixteen_and_thirty_two(codec, nq):
             assert not len(rest) or rest.max() <= want[got].min() + 2e-3
 
 
-@pytest.mark.parametrize("codec,nq,k", [(0, 4, 60), (3, 3, 61), (4, 1, 62), (2, 4, 63)])
-def test_plain_shares_of_long_segments_end_inside_a_set_of_thirty_two(codec, nq, k):
-    # work items of more than 10 000 tiles take sets of 32 (NF4: 16); segments end at every place of a set, and the last segments share tiles
-    lens = [12_000 + i for i in range(33)] + [16_384, 10_001, 20_000] + [13_000 + 5 * i for i in range(40)]
-    base = np.tile(H.random_tiles(4000, codec, seed=960 + codec, warm_every=9, nocorr_every=6), 6)
+def _planned_items(lens, sms=148):
+    """Work items of a plain plan for four query rows or fewer a segment on `sms` CTAs, as the planner cuts them: at equal shares, and nowhere that leaves a sliver."""
+    share = -(-max(768, -(-sum(lens) // sms)) // 16) * 16
+    snap, spare, filled, items = min(share // 16, 2048), max(0, share * sms - sum(lens)), 0, []
+    for n in lens:
+        at = 0
+        while at < n:
+            if at == 0 and 0 < share - filled < snap and filled and spare >= share - filled:
+                spare, filled = spare - (share - filled), 0
+            take = min(n - at, share - filled)
+            rest = n - at - take
+            if 0 < rest < snap:
+                take, spare = take + rest, spare + rest
+            filled, at = filled + take, at + take
+            items.append(take)
+            if filled >= share:
+                filled = 0
+    return items
+
+
+# Segments that share one buffer of tiles.  INT4 takes sets of 32 from items of 6400 tiles on the average, mixed 8/4 and TQ3 from 10 000, NF4 never.
+LONG = [40_000 + 617 * i for i in range(33)] + [65_536, 40_001, 59_999] + [48_000 + 5 * i for i in range(44)]
+MIDDLE = [12_000 + 3 * i for i in range(150)]
+
+
+@pytest.mark.parametrize("codec,nq,k,lens,sets", [(0, 4, 60, LONG, 32), (1, 1, 1024, LONG, 32), (3, 3, 61, LONG, 32), (4, 2, 62, LONG, 32), (2, 4, 63, LONG, 16),
+                                                  (6, 2, 64, MIDDLE, 32), (3, 2, 65, MIDDLE, 16)])
+def test_plain_shares_of_long_segments_end_inside_a_set_of_thirty_two(codec, nq, k, lens, sets):
+    # segments end at every place of a set; some tiles are WARM or without their correction plane; the last segment ends in tiles of another codec
+    # and is handed to the generic kernel
+    items = _planned_items(lens)
+    assert (np.mean(items) >= 10_000) == (lens is LONG) and len({m % 32 for m in lens}) > 16
+    base = np.tile(H.random_tiles(4000, codec, seed=960 + codec, warm_every=9, nocorr_every=6), 17)
     rng = np.random.default_rng(codec)
     rng.shuffle(base)
-    rows = [(int(rng.integers(0, len(base) - m + 1)), m, i * nq, nq, 2 * i) for i, m in enumerate(lens)]
+    base[-5:] = H.random_tiles(5, 3 if codec != 3 else 4, seed=6)
+    free = len(base) - 5
+    rows = [(int(rng.integers(0, free - m + 1)), m, i * nq, nq, 2 * i) for i, m in enumerate(lens)]
+    rows[-1] = (len(base) - lens[-1], lens[-1]) + rows[-1][2:]
     qc, qs = H.random_queries(nq * len(lens), 961)
     idx, sc, cnt = S.score_topk(S.to_device(base), S.make_segments(rows), qc, qs, nq * len(lens), k)
-    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
-    _check_rows(base, rows, qc, qs, idx, sc, cnt, k, every=3)
+    assert S.debug_last_score_set() == sets
+    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
+    _check_rows(base, rows[:33] + rows[-1:], qc, qs, idx, sc, cnt, k, every=3)
+
+
+@pytest.mark.parametrize("codec", [1, 3])
+def test_a_pool_of_three_million_slots_skips_its_cold_tiles_in_sets_of_thirty_two(codec):
+    # one stream so long that its CTAs take contiguous shares; the slots' states are looked at for both halves of a set
+    n, k = 3_000_017, 48 + codec  # (plans are kept by shape, each for one codec)
+    base = H.random_tiles(5000, codec, seed=57)
+    pool = S.TilePool(n, 2**40, S.PAGE_OLDEST_FIRST, S.EVICT_CAUSAL)
+    rng = np.random.default_rng(codec)
+    pick = rng.integers(0, len(base), n)
+    for b in range(0, n, 500_000):
+        pool.insert(base[pick[b:b + 500_000]])
+    qc, qs = H.random_queries(2, 58)
+    scores = [ora.score_tiles(base, qc[j], qs[j])[pick] for j in range(2)]
+    # a hole among the best, and slots all over the stream
+    cold = np.unique(np.concatenate([rng.choice(n, 400, replace=False), np.argsort(-scores[0])[:300:2], np.argsort(-scores[1])[:300:2], np.arange(n - 40, n, 3)]))
+    for s in cold:
+        assert pool.evict(int(s))
+    ti, tv, tc = pool.score_topk(qc, qs, 2, k)
+    assert S.debug_last_score_set() == 32 and S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
+    for j in range(2):
+        live = scores[j].copy()
+        live[cold] = -np.inf
+        assert tc[j] == k and len(set(ti[j])) == k and not set(ti[j]) & set(cold)
+        assert np.all(np.abs(tv[j] - live[ti[j]]) <= 1e-3) and np.all(np.abs(tv[j] - np.sort(live)[::-1][:k]) <= 2e-3)
 
 
 @pytest.mark.parametrize("order", ["random", "rising", "falling", "equal", "negative lambda"])
