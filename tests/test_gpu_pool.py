@@ -182,6 +182,104 @@ def test_large_pool_enforce_budget_with_long_candidate_lists(codec, page, evict,
     assert_same(pool, cache, 1e-3)  # (the oracle sums 90 000 softmax terms sequentially in f32, the pool in a tree)
 
 
+def _evict_route(pool, sink, recent, budget):
+    """Which of its ways the single cooperative launch takes for the coming eviction of the lowest importances, told from the keys: every block
+    (512 threads, at most 148 blocks) bounds its own `reach` smallest keys with up to four more, and the smallest of those bounds counts."""
+    tiles, state, imp, seq = pool.read()
+    st, pos = pool.stats(), tiles["position"]
+    deficit = st["live_bytes"] - 32 * st["hot"] - budget
+    reach = deficit // 80 + 1
+    live = state != ora.COLD
+    last = pos[live].max()
+    slots = np.nonzero(live & (pos >= sink) & (pos + recent <= last))[0]
+    order = slots[np.lexsort((seq[slots], imp[slots]))]
+    rank = np.empty(len(state), np.int64)
+    rank[order] = np.arange(len(order))
+    grid = min(148, (len(state) + 511) // 512)
+    if reach * grid > 4 * 4096 or len(state) > 16 * grid * 512:
+        return "list of all"
+    block = (slots % (grid * 512)) // 512
+    own = [np.sort(rank[slots[block == b]]) for b in range(grid)]
+    fewest, most = [min((r[reach - 1 + more] for r in own if len(r) > reach - 1 + more), default=len(order)) + 1 for more in (0, 4)]
+    return "counted" if most <= 512 else "cut, then counted" if fewest > 512 and most <= 4096 else "too many" if fewest > 4096 else "?"
+
+
+def test_small_deficits_take_every_way_through_the_cooperative_launch():
+    # evictions of 1 to 300 tiles of 90 000 with importances in random order: the blocks' smallest keys together fit the last block's count, are cut
+    # down to it, are too many for it (the general path then lists all candidates), or are not tried; slots, states and accounting as the oracle's
+    n, sink, recent = 90_000, 4, 64
+    budget = int(0.6 * 128 * n)
+    pool, cache = S.TilePool(n + 512, budget, 1, 1, sink, recent), ora.Cache(budget, 1, 1, sink, recent)
+    tiles = H.random_tiles(n + 700, 3, seed=91)
+    tiles["position"] = np.arange(n + 700)
+    assert list(pool.insert(tiles[:n])) == [cache.insert(tiles[j:j + 1]) for j in range(n)]
+    sc = ora.Rng(6).gaussian(n) * 4
+    live = np.arange(n, dtype=np.uint32)
+    pool.observe_scores(live, sc, 0.9)
+    cache.observe_scores(live, sc, 0.9)
+    assert pool.enforce_budget() == cache.enforce_budget()
+    at, routes = n, []
+    for m in (1, 2, 300, 3, 5, 20, 100, 14, 60, 90, 1):
+        more = tiles[at:at + m]
+        at += m
+        assert list(pool.insert(more)) == [cache.insert(more[j:j + 1]) for j in range(m)]
+        routes.append(_evict_route(pool, sink, recent, budget))
+        assert pool.enforce_budget() == cache.enforce_budget()
+        h, w, c = cache.counts()
+        st = pool.stats()
+        assert (st["live_bytes"], st["hot"], st["warm"], st["cold"]) == (cache.live_bytes(), h, w, c)
+    assert {"counted", "cut, then counted", "too many", "list of all"} <= set(routes), routes
+    assert_same(pool, cache, 1e-3)  # (the oracle sums 90 000 softmax terms sequentially in f32, the pool in a tree)
+
+
+def test_a_pool_that_grows_past_the_slots_its_threads_hold_in_registers():
+    # 16 slots a thread of 148 blocks of 512: up to 1 212 416 slots the smallest keys are found from registers, beyond them from the list of all
+    # candidates; both give what the phases run from the host give
+    limit = 16 * 148 * 512
+    n, sink, recent = limit - 40, 4, 2048
+    base = H.random_tiles(4000, 3, seed=92)
+    rng = np.random.default_rng(3)
+    tiles = base[rng.integers(0, len(base), n + 200)]
+    tiles["position"] = np.arange(n + 200)
+    pools = [S.TilePool(n + 400, 2**40, 1, 1, sink, recent) for _ in range(2)]
+
+    def enforce(pool, from_host):
+        S.debug_force_generic_score(from_host)
+        try:
+            return pool.enforce_budget()
+        finally:
+            S.debug_force_generic_score(False)
+
+    for b in range(0, n, 400_000):
+        for p in pools:
+            p.insert(tiles[b:min(n, b + 400_000)])
+    live = np.arange(n, dtype=np.uint32)
+    sc = (rng.standard_normal(n) * 4).astype(F)
+    for i, p in enumerate(pools):
+        p.observe_scores(live, sc, 0.9)
+    at, lens = n, []
+    budget = pools[0].stats()["live_bytes"]  # (everything still fits: page-outs for the new tiles only, no slot is reused)
+
+    def step(m, budget):
+        for p in pools:
+            p.set_budget(budget)
+        assert np.array_equal(*[p.insert(tiles[at:at + m]) for p in pools])
+        assert enforce(pools[0], False) and enforce(pools[1], True)
+        assert pools[0].stats() == pools[1].stats()
+        lens.append(pools[0].stats()["len"])
+
+    for m in (8, 8, 40, 8):
+        step(m, budget)
+        at += m
+    assert lens[0] < limit < lens[-1]
+    for m in (4, 9, 30):  # everything paged out, then evictions, whose slots the next tiles take in the same order
+        step(m, 96 * (lens[3] - 20))
+        at += m
+    assert pools[0].stats()["cold"] >= 20
+    for g, w in zip(pools[0].read(), pools[1].read()):
+        assert g.tobytes() == w.tobytes()
+
+
 def test_scoring_a_pool_whose_oldest_slots_are_cold_stays_on_the_tensor_core_kernel():
     # One long stream scored by every CTA, with nothing to score at its start (the oldest third of the slots is COLD):
     # the first thresholds must still form early, otherwise the rows' candidate buffers overflow and the rows are handed
