@@ -347,11 +347,12 @@ __device__ __forceinline__ void phase_keys(const PoolDev& p, int phase, uint64_t
     for (int u = 0; u < EB_BATCH; ++u) key[u] = phase_key(p, phase, s0 + u * stride, m[u], max_pos);
 }
 constexpr int EB_KEYS = 16;  // slots of a thread whose keys stay in its registers (1.2 million on 148 SMs)
+constexpr int EB_FEW = 6;    // and from how many slots a thread on they do (455 000)
 constexpr int EB_THREADS = 512, EB_ITEMS = 8, EB_CAP = EB_THREADS * EB_ITEMS, EB_LEVELS = 6, EB_BINS = 4096;
 struct EnforceState {
     unsigned long long inv_min_key, max_key;  // ~min and max over the phase's candidates (zero = none yet)
     uint32_t n_keep, overflow, pad[2];
-    unsigned long long bound_inv[5];          // ~bound of the phase's candidates, see below
+    ulonglong2 bounds[5];                     // ~bound of the phase's candidates and the largest of the blocks' smallest keys, see below
     uint32_t few[5], pad2;                    // how many lie within it
     uint32_t hist[5][EB_LEVELS][EB_BINS];
 };
@@ -443,6 +444,9 @@ __device__ __forceinline__ uint64_t block_cut(const uint64_t (&k)[N], uint64_t r
     }
 }
 
+// FEW: for pools in which a phase's smallest keys are found from registers where that can be done (see below); the other form is the faster one without that code
+// (100 000 slots, 1 to 80 evictions: 62 to 71 us of the kernel, 69 to 76 with it).
+template <bool FEW>
 __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t phase_mask, uint64_t* keys, uint32_t* vals,
                                                              uint64_t* skeys, uint32_t* svals, EnforceState* es) {
     namespace cg = cooperative_groups;
@@ -499,12 +503,15 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
         const uint64_t deficit = live - budget;
         const uint64_t min_freed = phase == PH_PAGE ? 32 : (phase >= PH_EVICT ? 80 : 14);
         const uint64_t reach = deficit / min_freed + 1;
-        // ---- a decode step's deficit (a few operations): every block finds a bound that `reach` of its own keys do not exceed, and the
-        //      smallest of the blocks' bounds is one for all candidates.  The few keys within it go to the last block's sort from
-        //      registers: one scan and two grid barriers, where the list of all candidates below takes a write and three reads,
-        //      global histograms and three barriers.
-        bool few = len <= EB_KEYS * stride && reach * gridDim.x <= 4ull * EB_CAP;
-        if (few) {
+        // ---- a decode step's deficit (a few operations) in a large pool: every block finds a bound that `reach` of its own keys do not
+        //      exceed, and the smallest of the blocks' bounds is one for all candidates; so is the largest of the blocks' smallest keys, where
+        //      there are `reach` blocks or more (the better one where keys lie in random order: 1 000 000 slots, 80 evictions 179 -> 132 us).  The few keys
+        //      within both go to the last block's sort from registers: one scan and two grid barriers, where the list of all
+        //      candidates below takes a write and three reads, global histograms and three barriers.  The block's own selection costs more than the list while
+        //      that is read in a round or two (us of the kernel, 16 evictions by importance, without and with: 100 000 slots 65 / 84, 300 000 73 / 88,
+        //      500 000 93 / 96, 650 000 101 / 102, 1 000 000 136 / 120; in causal order 59 / 71, 69 / 76, 84 / 81, 93 / 87, 126 / 108).
+        bool few = FEW && reach * gridDim.x <= 4ull * EB_CAP;
+        if (FEW && few) {
             uint64_t key[EB_KEYS];
 #pragma unroll
             for (int b = 0; b < EB_KEYS; b += EB_BATCH) {
@@ -515,9 +522,11 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
             }
             uint32_t kept;
             const uint64_t own = block_cut(key, reach, 4u, sm.cut, kept);
-            if (threadIdx.x == 0 && kept >= reach) atomicMax(&es->bound_inv[phase], (unsigned long long)~own);  // (a block with fewer keys bounds nothing)
+            if (threadIdx.x == 0 && kept >= reach) atomicMax(&es->bounds[phase].x, (unsigned long long)~own);  // (a block with fewer keys bounds nothing)
+            if (threadIdx.x == 32) atomicMax(&es->bounds[phase].y, ~sm.cut.lo_inv);                            // (SENTINEL from a block without keys)
             grid.sync();
-            const uint64_t bound = ~*(volatile unsigned long long*)&es->bound_inv[phase];
+            const ulonglong2 bounds = __ldcg(&es->bounds[phase]);
+            const uint64_t bound = reach <= gridDim.x ? min(~bounds.x, bounds.y) : ~bounds.x;
             uint32_t mine = 0;
 #pragma unroll
             for (int j = 0; j < EB_KEYS; ++j) mine += key[j] != SENTINEL && key[j] <= bound;
@@ -705,7 +714,7 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
                     k[j] = i < n ? ks[i] : SENTINEL;
                     v[j] = i < n ? vs[i] : 0u;
                 }
-                if (n > EB_THREADS && reach <= EB_THREADS / 2) {  // the blocks' smallest keys together: down to what the count below orders
+                if (FEW && n > EB_THREADS && reach <= EB_THREADS / 2) {  // the blocks' smallest keys together: down to what the count below orders
                     uint32_t kept;
                     const uint64_t bound = block_cut(k, reach, EB_THREADS / 2, sm.cut, kept);
                     if (kept <= EB_THREADS) {
@@ -1126,10 +1135,12 @@ static Status pool_enforce_budget_fused(Ctx* c, Pool* pl, int32_t* within, bool*
     static int blocks_per_sm[64] = {0}, sms[64] = {0};
     const int dev = pl->device & 63;
     if (!blocks_per_sm[dev]) {
-        int coop = 0, n = 0, b = 0;
+        int coop = 0, n = 0, b = 0, f = 0;
         SLHA_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, pl->device));
         SLHA_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, pl->device));
-        SLHA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, enforce_kernel, EB_THREADS, 0));
+        SLHA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, enforce_kernel<false>, EB_THREADS, 0));
+        SLHA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&f, enforce_kernel<true>, EB_THREADS, 0));
+        b = std::min(b, f);
         sms[dev] = n;
         blocks_per_sm[dev] = coop && b > 0 ? std::min(b, 2) : -1;
     }
@@ -1154,7 +1165,9 @@ static Status pool_enforce_budget_fused(Ctx* c, Pool* pl, int32_t* within, bool*
     void* args[] = {&d, &mask, &keys, &vals, &skeys, &svals, &es};
     const uint64_t want = (len + EB_THREADS - 1) / EB_THREADS;
     const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sms[dev] * blocks_per_sm[dev]));
-    SLHA_CUDA(cudaLaunchCooperativeKernel((const void*)enforce_kernel, dim3(grid), dim3(EB_THREADS), args, 0, c->stream));
+    const uint64_t stride = (uint64_t)grid * EB_THREADS;
+    const bool few = len > EB_FEW * stride && len <= EB_KEYS * stride;
+    SLHA_CUDA(cudaLaunchCooperativeKernel(few ? (const void*)enforce_kernel<true> : (const void*)enforce_kernel<false>, dim3(grid), dim3(EB_THREADS), args, 0, c->stream));
     count_launch();
     uint32_t overflow = 0;
     SLHA_CUDA(cudaMemcpyAsync(&overflow, &es->overflow, 4, cudaMemcpyDeviceToHost, c->stream));

@@ -184,7 +184,8 @@ def test_large_pool_enforce_budget_with_long_candidate_lists(codec, page, evict,
 
 def _evict_route(pool, sink, recent, budget):
     """Which of its ways the single cooperative launch takes for the coming eviction of the lowest importances, told from the keys: every block
-    (512 threads, at most 148 blocks) bounds its own `reach` smallest keys with up to four more, and the smallest of those bounds counts."""
+    (512 threads, 148 blocks) bounds its own `reach` smallest keys with up to four more; the smallest of those bounds counts, or the largest of
+    the blocks' smallest keys where that is smaller."""
     tiles, state, imp, seq = pool.read()
     st, pos = pool.stats(), tiles["position"]
     deficit = st["live_bytes"] - 32 * st["hot"] - budget
@@ -195,25 +196,32 @@ def _evict_route(pool, sink, recent, budget):
     order = slots[np.lexsort((seq[slots], imp[slots]))]
     rank = np.empty(len(state), np.int64)
     rank[order] = np.arange(len(order))
-    grid = min(148, (len(state) + 511) // 512)
-    if reach * grid > 4 * 4096 or len(state) > 16 * grid * 512:
+    grid = 148
+    if reach * grid > 4 * 4096 or not 6 * grid * 512 < len(state) <= 16 * grid * 512:
         return "list of all"
     block = (slots % (grid * 512)) // 512
     own = [np.sort(rank[slots[block == b]]) for b in range(grid)]
+    firsts = max(r[0] if len(r) else len(order) for r in own) + 1
     fewest, most = [min((r[reach - 1 + more] for r in own if len(r) > reach - 1 + more), default=len(order)) + 1 for more in (0, 4)]
+    fewest, most = min(fewest, firsts), min(most, firsts)
     return "counted" if most <= 512 else "cut, then counted" if fewest > 512 and most <= 4096 else "too many" if fewest > 4096 else "?"
 
 
-def test_small_deficits_take_every_way_through_the_cooperative_launch():
-    # evictions of 1 to 300 tiles of 90 000 with importances in random order: the blocks' smallest keys together fit the last block's count, are cut
-    # down to it, are too many for it (the general path then lists all candidates), or are not tried; slots, states and accounting as the oracle's
-    n, sink, recent = 90_000, 4, 64
+@pytest.mark.parametrize("skewed", [False, True])
+def test_small_deficits_take_every_way_through_the_cooperative_launch(skewed):
+    # evictions of 1 to 300 tiles of 470 000: the blocks' smallest keys together fit the last block's count, are cut down to it, are too many for
+    # it (the general path then lists all candidates), or are not tried; slots, states and accounting as the oracle's.  Skewed: one block's
+    # tiles all weigh more than the others'
+    n, sink, recent = 470_000, 4, 64
     budget = int(0.6 * 128 * n)
     pool, cache = S.TilePool(n + 512, budget, 1, 1, sink, recent), ora.Cache(budget, 1, 1, sink, recent)
-    tiles = H.random_tiles(n + 700, 3, seed=91)
+    base = H.random_tiles(4000, 3, seed=91)
+    tiles = base[np.random.default_rng(4).integers(0, len(base), n + 700)]
     tiles["position"] = np.arange(n + 700)
     assert list(pool.insert(tiles[:n])) == [cache.insert(tiles[j:j + 1]) for j in range(n)]
-    sc = ora.Rng(6).gaussian(n) * 4
+    sc = ora.Rng(6).gaussian(n)
+    if skewed:
+        sc[np.arange(n) % (148 * 512) < 512] += 6
     live = np.arange(n, dtype=np.uint32)
     pool.observe_scores(live, sc, 0.9)
     cache.observe_scores(live, sc, 0.9)
@@ -228,8 +236,8 @@ def test_small_deficits_take_every_way_through_the_cooperative_launch():
         h, w, c = cache.counts()
         st = pool.stats()
         assert (st["live_bytes"], st["hot"], st["warm"], st["cold"]) == (cache.live_bytes(), h, w, c)
-    assert {"counted", "cut, then counted", "too many", "list of all"} <= set(routes), routes
-    assert_same(pool, cache, 1e-3)  # (the oracle sums 90 000 softmax terms sequentially in f32, the pool in a tree)
+    assert {"counted", "cut, then counted", "list of all"} <= set(routes) and ("too many" in routes) == skewed, routes
+    assert_same(pool, cache, 1e-3)  # (the oracle sums 470 000 softmax terms sequentially in f32, the pool in a tree)
 
 
 def test_a_pool_that_grows_past_the_slots_its_threads_hold_in_registers():
