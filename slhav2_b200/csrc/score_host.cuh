@@ -36,33 +36,33 @@ Status launch_tc(Ctx* c, F* kernel, bool* configured, const ScoreArgs& a, uint32
     SLHA_CUDA(cudaGetLastError());
     return Status();
 }
-template <int KIND, bool IL, int U>
+template <int KIND, bool IL, bool LONG>
 Status launch_stream_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_stream_kernel<KIND, IL, U>, configured, a, grid, stream_threads(KIND, U), stream_smem_bytes(KIND, U), true);
+    return launch_tc(c, score_stream_kernel<KIND, IL, LONG>, configured, a, grid, STREAM_THREADS, stream_smem_bytes(KIND, stream_sets(KIND, LONG)), true);
 }
 template <bool IL>
 Status launch_mix3(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
     return launch_tc(c, score_mix3_kernel<IL>, configured, a, grid, ST_THREADS, st_smem_bytes(false), true);
 }
-template <bool IL, int U>
-Status launch_stream_u(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
+template <bool IL, bool LONG>
+Status launch_stream_i(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
     switch (kind) {
-        case 0: return launch_stream_t<0, IL, 1>(c, a, grid);
-        case 1: return launch_stream_t<1, IL, U>(c, a, grid);
-        case 2: return launch_stream_t<2, IL, U>(c, a, grid);
-        case 3: return launch_stream_t<3, IL, U>(c, a, grid);
+        case 0: return launch_stream_t<0, IL, LONG>(c, a, grid);
+        case 1: return launch_stream_t<1, IL, LONG>(c, a, grid);
+        case 2: return launch_stream_t<2, IL, LONG>(c, a, grid);
+        case 3: return launch_stream_t<3, IL, LONG>(c, a, grid);
         default: return launch_mix3<IL>(c, a, grid);
     }
 }
-Status launch_stream(Ctx* c, int kind, bool il, int sets, const ScoreArgs& a, uint32_t grid) {
-    if (il) return launch_stream_u<true, 1>(c, kind, a, grid);
-    return sets == 2 ? launch_stream_u<false, 2>(c, kind, a, grid) : launch_stream_u<false, 1>(c, kind, a, grid);
+Status launch_stream(Ctx* c, int kind, bool il, bool long_items, const ScoreArgs& a, uint32_t grid) {
+    if (il) return launch_stream_i<true, false>(c, kind, a, grid);
+    return long_items ? launch_stream_i<false, true>(c, kind, a, grid) : launch_stream_i<false, false>(c, kind, a, grid);
 }
 // tiles a warp takes at a time, and warps of a CTA
 uint32_t stream_warp_tiles(int kind, int sets) { return kind == 4 ? ST_WT : (uint32_t)(MMA_SET_TILES * sets); }
-uint32_t stream_warps(int kind, int sets) { return (uint32_t)(kind == 4 ? ST_THREADS : stream_threads(kind, sets)) / 32; }
+uint32_t stream_warps(int kind) { return (uint32_t)(kind == 4 ? ST_THREADS : STREAM_THREADS) / 32; }
 static_assert(ST_CHUNK == ST_WT, "a fresh chunk holds what a warp can append at once");
 Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
     static thread_local bool configured[16] = {false};
@@ -220,6 +220,7 @@ struct Plan {
     int codec_hint_in = -1;
     bool force_generic_in = false;
     uint32_t mma_grid = 0;
+    bool long_items = false; // score_stream_kernel's form for them
     int sets = 1;            // sub-sets of 16 tiles that a warp takes at a time
     DevBuf b_tables, b_keys, b_cnt, b_gpivot, b_gbuf, b_gsel, b_tmp;
     // Two-level merge for calls with few queries and many candidate lists per query (a pool scored
@@ -318,7 +319,12 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // concatenated tile stream is cut into one equal share per persistent CTA
     // (and at segment ends), so per-item costs are paid once per ~total/grid tiles.
     uint64_t total = 0;
-    for (size_t i = 0; i < n_segs; ++i) total += (uint64_t)segs[i].n_tiles * ((segs[i].n_queries + 3) / 4);
+    size_t streams = 0;  // (segment, group of up to four query rows)
+    for (size_t i = 0; i < n_segs; ++i) {
+        const size_t groups = (segs[i].n_queries + 3) / 4;
+        total += (uint64_t)segs[i].n_tiles * groups;
+        streams += segs[i].n_tiles ? groups : 0;
+    }
     uint32_t item_tiles = std::max<uint32_t>(8192, 8 * k);
     while (item_tiles > 2048 && total / item_tiles < 592) item_tiles /= 2;
     item_tiles = std::max(round, (item_tiles + round - 1) / round * round);
@@ -521,8 +527,9 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // (a warp reserves slots in chunks of up to the tiles it takes at a time, so up to that many per warp and item stay unused)
     uint32_t longest = 0;
     for (size_t i = 0; i < n_segs; ++i) longest = std::max(longest, segs[i].n_tiles);
-    p->sets = stream_sets(p->kind, !stream_items.empty(), all.empty() ? 0 : total / all.size());
-    const uint32_t st_warps = stream_warps(p->kind, p->sets), st_tiles = stream_warp_tiles(p->kind, p->sets);
+    p->long_items = stream_long(p->kind, !stream_items.empty(), total / std::max<size_t>(all.size(), 1), total / std::max<size_t>(streams, 1), k);
+    p->sets = stream_sets(p->kind, p->long_items);
+    const uint32_t st_warps = stream_warps(p->kind), st_tiles = stream_warp_tiles(p->kind, p->sets);
     const uint64_t all_of_a_row = (uint64_t)longest + (uint64_t)st_tiles * st_warps * p->max_parts + 64;
     // (the first set of every warp that scans a row is appended unfiltered: its tiles per warp and item, twice over)
     const uint64_t first_sets = (uint64_t)(2 * st_tiles) * st_warps * p->max_parts;
@@ -884,9 +891,9 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
             a.cta_begin = p->d_wide_cta;
             SLHA_TRY(launch_wide(c, p->kind, a, p->wide_grid));
         } else if (p->d_stream_items) {
-            SLHA_TRY(launch_stream(c, p->kind, true, 1, a, p->mma_grid));
+            SLHA_TRY(launch_stream(c, p->kind, true, false, a, p->mma_grid));
         } else {
-            SLHA_TRY(launch_stream(c, p->kind, false, p->sets, a, p->mma_grid));
+            SLHA_TRY(launch_stream(c, p->kind, false, p->long_items, a, p->mma_grid));
         }
         // (timing: the first bracket is the tensor-core kernel alone; the generic kernel's pass over handed-back rows, an
         // early exit when there are none, counts with the compaction and the merge)

@@ -38,12 +38,19 @@ constexpr uint32_t MMA_CHUNK = 16;  // slots a warp reserves at a time in a row'
 // U = 2 on long shares: 8 x 1M MX-32 tiles 274 -> 247 us a call (16 tiles at a time cost 483 instructions, 32 tiles 2 x 291), 8 x 524 288 mixed and TQ3
 // tiles the same as with 1.  Not for NF4, whose 128 registers leave 16 warps an SM (457 us for 256 x 32 768 tiles; 439 with sets of 16 and
 // 24 warps), nor for interleaved shares, whose first sets are appended unfiltered (a million MX-16 tiles on one row, k = 100: 81 us, with U = 2 102).
-// From 6400 (INT4, MX-INT4) or 10 000 tiles a work item on (the plan's average: segments are cut at the CTAs' shares too): a CTA's first sets of an item are
-// appended unfiltered, twice as many of them with U = 2.  us a call with 1 / 2 at average items of 4878 (200 segments of 8000 tiles, k = 64), 6521 (150 of 12 000), 8510
-// (150 of 16 000), 14 545 (80 of 40 000): INT4 92 / 94, 88 / 86, 104 / 102, 113 / 104; mixed 96 / 101, 95 / 96, 115 / 116, 129 / 126; TQ3 119 / 128, 123 / 126,
-// 151 / 155, 173 / 173; with k = 1024 at 8510 and 14 545: INT4 152 / 147, 158 / 152, mixed 156 / 149, 164 / 160, TQ3 189 / 185, 209 / 208.
-constexpr int stream_sets(int kind, bool il, uint64_t item_tiles) { return il || kind == 0 || item_tiles < (kind == 3 ? 6400 : 10000) ? 1 : 2; }
-constexpr int stream_threads(int, int) { return 768; }  // 24 warps at 80 registers: latencies are hidden with warps (U = 2 with 20 or 16 warps: 251, 254 us)
+// Plain shares come in two forms.  LONG: U = 2 (not NF4), a first round with few seeds, Hamming distances only where a tile can reach the threshold.  Short ones
+// have none of the three (INT4 has the latter two in both forms): each costs set-up or instructions and saves where items are long or few tiles are appended.  Taken
+//   INT4, MX-INT4: from 6400 tiles a work item on (the plan's average: segments are cut at the CTAs' shares too), mixed 8/4 and TQ3 from 18 000.  us a call short / long
+//     at items of 4878 (200 segments of 8000 tiles, k = 64), 6521 (150 of 12 000), 9756 (200 of 16 000, k = 256), 14 545 (80 of 40 000, k = 1024), 21 399 (256 of 32 768,
+//     k = 1024), 27 594 (8 of 524 288): INT4 92 / 94, 88 / 86, 161 / 156, 158 / 152; mixed 91 / 100, 91 / 97, 160 / 164, 158 / 159, 368 / 365, 155 / 139;
+//     TQ3 117 / 125, 121 / 126, 211 / 211, 205 / 206, 493 / 485, 219 / 201;
+//   NF4: where rows have 200 k tiles or more on the average, so that few are appended: 256 rows of 32 768 tiles, k = 1024 428 / 443, 200 of 20 000, k = 256 218 / 223, 100 of
+//     40 000 190 / 190, 200 of 16 000, k = 32 160 / 155, 8 of a million, k = 2048 347 / 324.
+constexpr bool stream_long(int kind, bool il, uint64_t item_tiles, uint64_t row_tiles, uint32_t k) {
+    return !il && (kind == 0 ? row_tiles >= 200ull * k : item_tiles >= (kind == 3 ? 6400 : 18000));
+}
+constexpr int stream_sets(int kind, bool long_items) { return long_items && kind != 0 ? 2 : 1; }
+constexpr int STREAM_THREADS = 768;  // 24 warps at 80 registers: latencies are hidden with warps (U = 2 with 20 or 16 warps: 251, 254 us)
 constexpr int MMA_DEPTH = SLHA_MMA_DEPTH;                  // cp.async ring slots per warp
 constexpr int MMA_BQ_BYTES = 9 * 32 * 8;                   // B fragments of a work item: [9][32 lanes] x 8 bytes
 constexpr int MMA_TAIL_BYTES = 2560;                       // fragments | sign words 128 | thresholds 16 | bucket mappings 32 + 32 | flag 16
@@ -52,7 +59,7 @@ constexpr uint32_t STREAM_LUT_AT = 0x10000;                // its shared-memory 
 constexpr int stream_slot(int u) { return MMA_DEPTH * u * MMA_SET_TILES * MMA_ROW; }  // a warp's ring
 constexpr int stream_low_warps(int u) { return ((int)STREAM_LUT_AT - 2048 - MMA_TAIL_BYTES) / stream_slot(u); }  // (dynamic shared memory starts below 2 KB)
 constexpr size_t stream_smem_bytes(int kind, int u) {
-    const int warps = stream_threads(kind, u) / 32;
+    const int warps = STREAM_THREADS / 32;
     if (kind != 0) return MMA_TAIL_BYTES + (size_t)warps * stream_slot(u);
     return STREAM_LUT_AT + STREAM_LUT_BYTES + (size_t)(warps > stream_low_warps(u) ? warps - stream_low_warps(u) : 0) * stream_slot(u);
 }
@@ -777,14 +784,16 @@ __device__ __forceinline__ unsigned long long final_threshold(const uint32_t* hi
 // work item's query rows, which the generic kernel then scores.
 // IL: the work items are interleaved shares of whole streams (see the planner); the plain instantiation keeps the
 // set arithmetic of contiguous ranges out of its loop.
+// LONG: see stream_long.  FULL: what its rows pay for is there (seeds, and the question whether a tile can reach the threshold).
 // U: a warp takes U x 16 tiles at a time.  The kernel is bound by instruction issue, and what a set costs beside its sums (fetch, flags, votes, thresholds,
 // query fragments) is paid once for both halves of a set of 32.
-template <int KIND, bool IL, int U>
-__global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kernel(ScoreArgs a) {
+template <int KIND, bool IL, bool LONG>
+__global__ void __launch_bounds__(STREAM_THREADS, 1) score_stream_kernel(ScoreArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     dep_launch();
     dep_wait();
-    constexpr int nwarps = stream_threads(KIND, U) / 32, R = 2 * U, SET_TILES = MMA_SET_TILES * U, SET_STRIDE = SET_TILES * MMA_ROW;
+    constexpr int U = stream_sets(KIND, LONG), nwarps = STREAM_THREADS / 32, R = 2 * U, SET_TILES = MMA_SET_TILES * U, SET_STRIDE = SET_TILES * MMA_ROW;
+    constexpr bool FULL = IL || LONG || KIND == 3;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     uint2* bq_w = reinterpret_cast<uint2*>(smem);                        // [9][32]
@@ -976,7 +985,7 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
         // (from N = 9 k on, where the seeds number 3 k: with k = 2048 of N = 6912 the seeds hardly prove a threshold before the rest is due,
         // 8 x 131 072 INT4 tiles 85 -> 100 us; and calls of two rounds have little to append: 8 x 8192 mixed tiles 29.1 -> 29.6 us)
         const uint64_t first_tiles = (uint64_t)SET_TILES * (uint64_t)nwarps * parts;
-        if (first_round_barrier && my_rounds > 1u && first_tiles >= 9ull * a.k && (my_rounds > 2u || first_tiles >= 8192u))
+        if (FULL && first_round_barrier && my_rounds > 1u && first_tiles >= 9ull * a.k && (my_rounds > 2u || first_tiles >= 8192u))
             seeds = min(nwarps, max(1, (int)ceilf(sqrtf((float)nwarps * (float)a.k / ((float)SET_TILES * (float)parts)))));
         if (too_big) n_sets = 0;  // (the sets already on their way are waited for at the item's end and never read)
 
@@ -986,14 +995,14 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
         const uint32_t rounds = too_big ? 0u : my_rounds;
         for (uint32_t round = 0; round < rounds; ++round) {
             const uint32_t s = set_of(round);
-            if (round == (warp < seeds ? 1u : 0u) && first_round_barrier) {
+            if (round == (!FULL || warp < seeds ? 1u : 0u) && first_round_barrier) {
                 // The seeds of the CTA (and, started together, of the grid) have appended their first sets
                 // unfiltered, so the rows' histograms hold a set's candidates per seed: first thresholds now,
                 // before the other sets are filtered.  (All warps pass here: `rounds` is the same for all, and at least two where there are
                 // fewer seeds than warps.)  Other CTAs may be a little behind: a few tries.
                 __syncthreads();
                 if (warp < nq) {
-                    for (int tries = seeds < nwarps ? 4 : 1; tries; --tries) {
+                    for (int tries = FULL && seeds < nwarps ? 4 : 1; tries; --tries) {
                         stream_refresh_threshold(a, it.query_begin + (uint32_t)warp, rng[warp], pvh + warp, lane);
                         __syncwarp();
                         if (reinterpret_cast<volatile uint32_t*>(pvh)[warp] != 0u || tries == 1) break;
@@ -1076,8 +1085,8 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
             const float thr = thr_float(reinterpret_cast<const volatile uint32_t*>(pvh)[t]);
             // The residual term lies in [-256 |lambda|, 256 |lambda|]: rows none of whose tiles can reach the threshold even with the largest
             // term need no Hamming distances (and append nothing).  (257 and the relative slack cover the rounding of the bound
-            // itself; a NaN passes.)  Long INT4 launches ask for eight tiles at a time; the others, whose rows are mostly short beside
-            // k (a decode step's caches: one tile in seven is appended, and some tile of a set nearly always), for the set.
+            // itself; a NaN passes.)  Long INT4 launches ask for eight tiles at a time, the others for the set; not asked where most rows are short
+            // beside k (a decode step's caches: one tile in seven is appended, and some tile of a set nearly always), see stream_long.
             constexpr int GATE = KIND == 3 && U == 2 ? 1 : R;  // rows asked for at a time
             float sc[R], lam[R];
             uint32_t b[R], some = 0;
@@ -1087,7 +1096,7 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
                 const uint2 m = lds_v2<96>(rb + (uint32_t)(r * MMA_HALF));  // scale, lambda
                 lam[r] = (f[r] & F_WARM) ? 0.0f : __uint_as_float(m.y);
                 sc[r] = c[r] * (__uint_as_float(m.x) * unit);
-                p[r] = mine && !(fmaf(fabsf(lam[r]), 257.0f, fmaf(fabsf(sc[r]), 1e-6f, sc[r])) < thr);
+                p[r] = mine && (!FULL || !(fmaf(fabsf(lam[r]), 257.0f, fmaf(fabsf(sc[r]), 1e-6f, sc[r])) < thr));
                 b[r] = 0u;
             }
 #pragma unroll
@@ -1095,7 +1104,7 @@ __global__ void __launch_bounds__(stream_threads(KIND, U), 1) score_stream_kerne
                 bool any = false;
 #pragma unroll
                 for (int r = r0; r < r0 + GATE; ++r) any = any || p[r];
-                if (__any_sync(0xFFFFFFFFu, any)) {
+                if (!FULL || __any_sync(0xFFFFFFFFu, any)) {
                     const uint4 qa = lds_v4<0>(qsa), qb = lds_v4<16>(qsa);
                     const uint32_t qs[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
 #pragma unroll
