@@ -9,7 +9,7 @@
 // finds the row's maximum itself (k scores, a few KB from the L2) and weighs its own run; the normalisers and the
 // partial sums of the value rows meet in distributed shared memory, added in a fixed order, so a call is one launch and
 // writes nothing but its results.  Bound: the gather of k value rows per query row (HBM); a thread keeps twelve 16-byte
-// loads in flight.  32 rows x 2048 winners of 128 bf16 values (17 MB): 10.3 us a call, 8.7 us of it the kernel (2.0 TB/s); with
+// loads in flight.  32 rows x 2048 winners of 128 bf16 values (17 MB): 8.7 us a call (2.0 TB/s); with
 // one-element loads, four in flight, partial sums through memory and a second launch to add them it was 31.9 us.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -71,8 +71,7 @@ template <typename T, int VEC, int SPLIT>
 __global__ void __cluster_dims__(SPLIT, 1, 1) __launch_bounds__(ATT_THREADS)
     attend_kernel(const uint32_t* top_index, const float* top_score, const uint32_t* top_count, uint32_t k, float scale, const T* values,
                   size_t d_v, size_t row_stride, const uint64_t* row_base, float* out, float* weights_out) {
-    dep_launch();
-    dep_wait();
+    dep_wait();  // (no dep_launch: CTAs of the next call that came to wait here were spread unevenly, 256 rows x 2048 winners 37 us -> 49, now 35)
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ float sm[];  // weights | indices of the CTA's run

@@ -81,6 +81,7 @@ inline cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, si
 #ifdef __CUDACC__
 // Every thread of a kernel launched with launch_behind calls dep_wait, also in CTAs that have nothing to do: a kernel counts as finished
 // when its CTAs are, and the next but one may rely on it.  Without that attribute both do nothing.
+// dep_launch at a kernel's start suits kernels whose CTAs fill an SM each; behind others the waiting CTAs of the next grid are spread unevenly.
 // What a caller or another kernel writes is read with ordinary loads there (or cp.async), not through the non-coherent path: that one asks that
 // nobody writes the memory while the grid lives, and the grid may live before the kernel that writes it has ended.
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }

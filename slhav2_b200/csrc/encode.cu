@@ -637,8 +637,7 @@ constexpr int enc_ctas(int kb) { return kb == 32 ? 4 : (kb >= 8 ? 2 : 1); }
 template <bool QUERY, int KB>
 __global__ void __launch_bounds__(enc_threads(KB), enc_ctas(KB)) encode_kernel(EncodeArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
-    dep_launch();
-    dep_wait();
+    dep_wait();  // (no dep_launch: CTAs of the next call that came to wait here were spread unevenly over the SMs, 7000 keys of 128 dimensions 42 us -> 55)
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int PER = KB >= 2 ? KB / 2 : 1;  // keys per thread where two threads share an output row
     constexpr int NT = enc_threads(KB);
@@ -1090,11 +1089,8 @@ Status fill_args(const Model* m, size_t n, EncodeArgs& a, int* kb_out) {
 
 template <bool QUERY, int KB>
 Status run_encode_kb(Ctx* c, EncodeArgs& a) {
-    size_t smem = encode_smem(a.d_pad, KB);
+    const size_t smem = encode_smem(a.d_pad, KB);
     const uint64_t groups = (a.n + KB - 1) / KB;
-    // (Where an SM holds two CTAs and every CTA can have one to itself, more than half of an SM's shared memory keeps them apart: 900 keys of 512 dimensions,
-    // 113 CTAs, took 76 us and 1184, 148 CTAs, 54.)
-    if (enc_ctas(KB) == 2 && groups <= (uint64_t)sm_count(c->device)) smem = std::max<size_t>(smem, 116 * 1024);
     static thread_local bool configured[16] = {false};  // the attribute is per device
     if (!configured[c->device & 15]) {
         SLHA_CUDA(cudaFuncSetAttribute(encode_kernel<QUERY, KB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
