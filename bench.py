@@ -465,7 +465,7 @@ def run_scoring_workload(args, w, S, torch, dist, rank, local, world, dev, strea
         failed = []
         slowest = [0.0] * callers
         n_rounds = 3  # the median round is reported (a round is short: one stalled call would dominate it)
-        t_end = [[0.0] * callers for _ in range(n_rounds)]
+        t_begin, t_end = [[[0.0] * callers for _ in range(n_rounds)] for _ in range(2)]
 
         def caller(i, n_calls):
             # the thread lives through all rounds: its set-up (stream, staging memory, plan) and its tear-down at thread exit
@@ -476,6 +476,7 @@ def run_scoring_workload(args, w, S, torch, dist, rank, local, world, dev, strea
                     S.score_topk(tiles, segs, hq, hs, nq, k, out_index=outs[i][0], out_score=outs[i][1])
                 for r in range(n_rounds):
                     go.wait()
+                    t_begin[r][i] = time.perf_counter()  # (each caller's own: the main thread may come from the barrier after the calls are done)
                     for _ in range(n_calls):
                         t_call = time.perf_counter()
                         S.score_topk(tiles, segs, hq, hs, nq, k, out_index=outs[i][0], out_score=outs[i][1])
@@ -494,9 +495,8 @@ def run_scoring_workload(args, w, S, torch, dist, rank, local, world, dev, strea
         try:
             for r in range(n_rounds):
                 go.wait()
-                t0 = time.perf_counter()
                 done.wait()
-                rounds_ms.append(1e3 * (max(t_end[r]) - t0) / (per * callers))
+                rounds_ms.append(1e3 * (max(t_end[r]) - min(t_begin[r])) / (per * callers))
         except threading.BrokenBarrierError:
             pass
         for th in threads:
