@@ -236,22 +236,22 @@ int32_t slha_b200_score_segments(const SciRustSlhaTile* tiles, const SlhaB200Seg
             SLHA_TRY(stage_in_t(c, row_offsets, n_queries, &doff));
         }
         const auto scored = [&]() -> Status {
-        const float* dq;
-        const uint64_t* ds;
-        SLHA_TRY(stage_in_t(c, q_coarse, n_queries * D_C, &dq));
-        SLHA_TRY(stage_in_t(c, q_sign, n_queries * 4, &ds));
-        std::vector<StagedOut> outs(1);
-        SLHA_TRY(stage_out(c, scores_out, scores_len * 4, &outs[0]));
-        // a host destination comes back whole: what no row covers is zero
-        if (outs[0].is_host) SLHA_CUDA(cudaMemsetAsync(outs[0].dev, 0, scores_len * 4, c->stream));
-        SLHA_TRY(launch_score_segments(c, tiles, hseg.data(), n_segments, dq, ds, n_queries, (float*)outs[0].dev,
-                                       reinterpret_cast<const unsigned long long*>(doff), row_len, fill, refused));
-        if (dev_off) {
-            bool bad;
-            SLHA_TRY(checked_offsets(c, &bad));
-            if (bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
-        }
-        return finish_outputs(c, outs, sync_by_default(c));
+            const float* dq;
+            const uint64_t* ds;
+            SLHA_TRY(stage_in_t(c, q_coarse, n_queries * D_C, &dq));
+            SLHA_TRY(stage_in_t(c, q_sign, n_queries * 4, &ds));
+            std::vector<StagedOut> outs(1);
+            SLHA_TRY(stage_out(c, scores_out, scores_len * 4, &outs[0]));
+            // a host destination comes back whole: what no row covers is zero
+            if (outs[0].is_host) SLHA_CUDA(cudaMemsetAsync(outs[0].dev, 0, scores_len * 4, c->stream));
+            SLHA_TRY(launch_score_segments(c, tiles, hseg.data(), n_segments, dq, ds, n_queries, (float*)outs[0].dev,
+                                           reinterpret_cast<const unsigned long long*>(doff), row_len, fill, refused));
+            if (dev_off) {
+                bool bad;
+                SLHA_TRY(checked_offsets(c, &bad));
+                if (bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+            }
+            return finish_outputs(c, outs, sync_by_default(c));
         };
         Status st = scored();
         if (dev_off && !st.ok()) {  // (what else was wrong is reported behind the offsets)

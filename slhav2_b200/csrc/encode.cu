@@ -312,7 +312,9 @@ __host__ __device__ constexpr int enc_row_stride(int kb) { return kb >= 8 ? kb +
 // sums run as m16n8k16 MMAs over fp16 roundings of Z (its rows scaled to one norm) and of e (scaled by a power of two), and only a sum
 // closer to zero than its error bound is taken again in the reference's order.  With z' and e' the roundings, n = d_pad terms:
 //   rounding of both factors               |z - z'| |e| + |z'| |e - e'|   (norms, measured: about 2^-12.3 |z| |e| each)
-//   fp32 accumulation in the MMAs          2^-13.9 |z| |e|                (17 addends an MMA, each cut at 2^-22 of the largest, 16 MMAs)
+//   fp32 accumulation in the MMAs          2^-13.9 |z| |e|                (17 addends an MMA, each cut at 2^-22 of the largest, 16 MMAs; no document
+//                                                                          says how they are summed: measured, addends are kept to 2^-25 of the
+//                                                                          largest, and 256 products beside one large end within 2^-17.7)
 //   the reference's own sequential sum     2^-16 |z| |e|                  (n + 1 roundings of 2^-24, n <= 256)
 // (model_build gives no fragments for n > 256 or a Z of unusual size).  Gaussian rows of Z leave about 1.1 of 256 signs of a key inside
 // the bound at d = 128, 1.6 at d_pad = 256.
@@ -631,7 +633,7 @@ __device__ __forceinline__ void fwht_stages(float* buf, uint32_t dp, uint32_t lo
 // the thread holds at once.
 
 // CTAs of KB keys whose registers fit on an SM together: four of 32 keys at head dimension 128 (57 KB of shared memory each), two of 16 or 8.  (16
-// keys with 180 registers, one CTA an SM: 20 011 keys of 512 dimensions 772 us, with 123 registers 593.)
+// keys with 180 registers, one CTA an SM: 20 011 keys of 512 dimensions 772 us, with 127 registers 564.)
 constexpr int enc_ctas(int kb) { return kb == 32 ? 4 : (kb >= 8 ? 2 : 1); }
 
 template <bool QUERY, int KB>
@@ -883,42 +885,42 @@ __global__ void __launch_bounds__(enc_threads(KB), enc_ctas(KB)) encode_kernel(E
         if (signs_done) {
         } else if (KB == 32 && tiled) {
             for (int u = tid; u < 256; u += NT) {
-            const int rg = u & 63, kg = u >> 6;
-            uint64_t acc2[4][4];
-            zero_tile<4, 8>(acc2);
-            const float4* mp = reinterpret_cast<const float4*>(a.zt) + rg;
+                const int rg = u & 63, kg = u >> 6;
+                uint64_t acc2[4][4];
+                zero_tile<4, 8>(acc2);
+                const float4* mp = reinterpret_cast<const float4*>(a.zt) + rg;
 #pragma unroll 16
-            for (uint32_t i = 0; i < dp; ++i)
-                outer_keys<4, 8>(acc2, __ldg(mp + (size_t)i * (D_S / 4)), buf + (size_t)i * KS + 8 * kg, a.one);
-            float acc[4][8];
-            unpack_tile<4, 8>(acc2, acc);
-            // bit s of a key = (acc < 0); this thread holds bits 4 rg .. +3, eight lanes fill a 32-bit word
+                for (uint32_t i = 0; i < dp; ++i)
+                    outer_keys<4, 8>(acc2, __ldg(mp + (size_t)i * (D_S / 4)), buf + (size_t)i * KS + 8 * kg, a.one);
+                float acc[4][8];
+                unpack_tile<4, 8>(acc2, acc);
+                // bit s of a key = (acc < 0); this thread holds bits 4 rg .. +3, eight lanes fill a 32-bit word
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                uint32_t v = (acc[0][j] < 0.0f ? 1u : 0u) | (acc[1][j] < 0.0f ? 2u : 0u) |
-                             (acc[2][j] < 0.0f ? 4u : 0u) | (acc[3][j] < 0.0f ? 8u : 0u);
-                v <<= 4 * (lane & 7);
-                v |= __shfl_xor_sync(0xFFFFFFFFu, v, 1);
-                v |= __shfl_xor_sync(0xFFFFFFFFu, v, 2);
-                v |= __shfl_xor_sync(0xFFFFFFFFu, v, 4);
-                const int key = 8 * kg + j, word = (rg >> 3);
-                if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64)[word] = v;
-            }
+                for (int j = 0; j < 8; ++j) {
+                    uint32_t v = (acc[0][j] < 0.0f ? 1u : 0u) | (acc[1][j] < 0.0f ? 2u : 0u) |
+                                 (acc[2][j] < 0.0f ? 4u : 0u) | (acc[3][j] < 0.0f ? 8u : 0u);
+                    v <<= 4 * (lane & 7);
+                    v |= __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+                    v |= __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+                    v |= __shfl_xor_sync(0xFFFFFFFFu, v, 4);
+                    const int key = 8 * kg + j, word = (rg >> 3);
+                    if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(tl + (size_t)key * TILE_BYTES + 64)[word] = v;
+                }
             }
         } else {
             // a thread owns hyperplane s for all KB keys
             for (int s = tid; s < D_S; s += NT) {
-            float acc[KB];
+                float acc[KB];
 #pragma unroll
-            for (int j = 0; j < KB; ++j) acc[j] = 0.0f;
-// (16 keys: loads of 16 steps in flight together, as in the two phases above: 7000 keys of 448 dimensions 182 us, with 8 steps 231)
+                for (int j = 0; j < KB; ++j) acc[j] = 0.0f;
+                // (16 keys: loads of 16 steps in flight together, as in the two phases above: 7000 keys of 448 dimensions 182 us, with 8 steps 231)
 #pragma unroll KB == 16 ? 16 : 8
-            for (uint32_t i = 0; i < dp; ++i) axpy_keys<KB>(acc, a.zt[(size_t)i * D_S + s], buf + (size_t)i * KS);
+                for (uint32_t i = 0; i < dp; ++i) axpy_keys<KB>(acc, a.zt[(size_t)i * D_S + s], buf + (size_t)i * KS);
 #pragma unroll
-            for (int j = 0; j < KB; ++j) {
-                const unsigned b = __ballot_sync(0xFFFFFFFFu, acc[j] < 0.0f);
-                if (lane == 0) reinterpret_cast<uint32_t*>(tl + (size_t)j * TILE_BYTES + 64)[s >> 5] = b;
-            }
+                for (int j = 0; j < KB; ++j) {
+                    const unsigned b = __ballot_sync(0xFFFFFFFFu, acc[j] < 0.0f);
+                    if (lane == 0) reinterpret_cast<uint32_t*>(tl + (size_t)j * TILE_BYTES + 64)[s >> 5] = b;
+                }
             }
         }
         __syncthreads();

@@ -304,8 +304,8 @@ struct ScoreArgs {
     const uint32_t* only_flagged; // dense mode: optional, per query row: only work items one of whose rows is flagged here
     uint64_t* gbuf;               // per query row: gcap composite keys
     uint32_t gcap;
-    uint32_t nf4_table;           // score_stream_kernel: build the NF4 shared-memory table (else NF4 tiles are handed back); score_dense_kernel: decode
-                                  // items that start on an INT4 tile as NF4, which takes both (1 always, 2 if the launch's first tile is NF4)
+    uint32_t nf4_table;           // score_dense_kernel: decode items that start on an INT4 tile as NF4, which takes both (1 always, 2 if the
+                                  // launch's first tile is NF4)
 };
 
 template <int G, bool TOPK>

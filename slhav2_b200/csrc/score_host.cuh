@@ -112,8 +112,8 @@ Status launch_score_t(Ctx* c, const ScoreArgs& a, uint32_t grid, int threads, si
     return Status();
 }
 
-template <bool TOPK>
 // behind: right after a kernel of the same call (see launch_behind)
+template <bool TOPK>
 Status launch_score(Ctx* c, int G, const ScoreArgs& a, uint32_t grid, int threads, size_t smem, bool behind) {
     switch (G) {
         case 1: return launch_score_t<1, TOPK>(c, a, grid, threads, smem, behind);
@@ -881,7 +881,6 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.gflag = a.gcount + nq;
         a.gbuf = p->d_gbuf;
         a.gcap = p->gcap;
-        a.nf4_table = p->kind == 0 ? 1u : 0u;
         a.q_coarse = d_q_coarse;
         a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
         a.k = k;

@@ -27,7 +27,7 @@ struct ListView {
 // Candidate accessors: element e of query Q as a composite key, 0 = absent.
 struct CompLists {  // lists written by score_kernel
     static constexpr bool kFiltered = false;
-    static constexpr bool kDistinct = true;  // no key comes twice
+    static constexpr bool kDistinct = true;  // no key comes twice: a row belongs to one segment, whose indices differ
     const uint64_t* keys;      // [n_lists][k] (k here = slots per list, >= the k asked for)
     const uint32_t* cnt;       // [n_lists]
     const uint32_t* q_list_begin;  // [nq]
@@ -118,7 +118,7 @@ struct StreamLists {
 };
 struct PairLists {  // (index, score) lists laid out [list][query][k_in]
     static constexpr bool kFiltered = false;
-    static constexpr bool kDistinct = false;  // no key comes twice
+    static constexpr bool kDistinct = false;  // a key may come twice: the lists are the caller's
     const uint32_t* idx;
     const float* score;
     uint32_t n_lists, n_queries, k_in;
@@ -439,7 +439,8 @@ __device__ void sort_and_emit(uint64_t* buf, uint32_t cap_s, int* hist, uint32_t
     emit_sorted(sorted, m, k, Q, out_index, out_score, out_count);
 }
 
-// The k best of buf[0..m), m <= RANK_MOST distinct keys, written where they belong: a key's place is the number of larger ones.  Every thread compares
+// The k best of buf[0..m), m <= RANK_MOST distinct keys, written where they belong: a key's place is the number of larger ones (equal keys
+// would share a place and leave one unwritten: only for lists with kDistinct).  Every thread compares
 // its key with all of them, two per shared-memory load: no barrier after the gathering, where bucket placement takes eight and a
 // selection before it a dozen.  For short lists only: 64 winners of 4096 tiles 21.6 -> 20.7 us a call, but 256 of 8 x 8192 (300 keys)
 // 27.1 -> 34.9.

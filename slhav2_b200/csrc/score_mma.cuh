@@ -35,7 +35,7 @@ constexpr int MMA_HALF = 8 * MMA_ROW;                      // row g -> row g + 8
 constexpr uint32_t MMA_CHUNK = 16;  // slots a warp reserves at a time in a row's candidate buffer (larger chunks measured no faster)
 // score_stream_kernel: a warp takes sets of U x 16 tiles.  Shared layout: query fragments, sign words, thresholds (the tail) | stage ring, and
 // for launches with NF4 tiles (KIND 0) tail | ring of the first warps | NF4 table at 64 KB | ring of the others.
-// U = 2 on long shares: 8 x 1M MX-32 tiles 274 -> 247 us a call (16 tiles at a time cost 483 instructions, 32 tiles 2 x 291), 8 x 524 288 mixed and TQ3
+// U = 2 on long shares: 8 x 1M MX-32 tiles 274 -> 247 us a call (16 tiles at a time cost 483 instructions, 32 tiles 2 x 308), 8 x 524 288 mixed and TQ3
 // tiles the same as with 1.  Not for NF4, whose 128 registers leave 16 warps an SM (457 us for 256 x 32 768 tiles; 439 with sets of 16 and
 // 24 warps), nor for interleaved shares, whose first sets are appended unfiltered (a million MX-16 tiles on one row, k = 100: 81 us, with U = 2 102).
 // Plain shares come in two forms.  LONG: U = 2 (not NF4), a first round with few seeds, Hamming distances only where a tile can reach the threshold.  Short ones
