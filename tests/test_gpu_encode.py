@@ -214,7 +214,13 @@ def test_sign_bits_near_and_at_zero_follow_the_exact_sums(n, d, rht):
     p = H.orthogonal_projection(11, d) if d >= 128 else np.ascontiguousarray(rng.standard_normal((128, d)) / 11, F)
     om, gm = ora.Model(p, d, seed=7, rht=rht), S.Model.from_projection(p, d, 7, rht=rht)
     q = H.gaussian_keys(n, n, d, outlier_channels=(7,))
-    z = ora.Rng(7).gaussian(256 * d).reshape(256, d).astype(np.float64) if not rht else rng.standard_normal((256, d))
+    z = ora.Rng(7).gaussian(256 * om.d_pad).reshape(256, om.d_pad).astype(np.float64)
+    if rht:  # the rows as a query meets them, behind the rotation
+        r, h = ora.Rng(7 ^ 0xA2A2A2A2A2A2A2A2), np.ones((1, 1))
+        diag = np.array([-1.0 if r.next_unit() < 0.5 else 1.0 for _ in range(om.d_pad)])
+        while len(h) < om.d_pad:
+            h = np.block([[h, h], [h, -h]])
+        z = (z @ h / np.sqrt(om.d_pad) * diag)[:, :d]
     for j in range(1, n, 5):  # a query with a sum of almost nothing: orthogonal to four hyperplanes
         rows = z[rng.choice(256, 4, replace=False)]
         q[j] -= (np.linalg.lstsq(rows.T, q[j].astype(np.float64), rcond=None)[0] @ rows).astype(F)
@@ -231,6 +237,45 @@ def test_sign_bits_near_and_at_zero_follow_the_exact_sums(n, d, rht):
         assert np.array_equal(qs[j], ws), j
     keys = np.where(np.isfinite(q), q, F(1.0))
     got, want = gm.encode_keys(keys, 2), om.encode_batch(keys, 2)
+    assert got.tobytes() == want.tobytes(), _diff(got, want)
+
+
+@pytest.mark.parametrize("n", [700, 2500, 5000])  # 8, 16 and 32 keys per CTA
+@pytest.mark.parametrize("d,rht", [(128, False), (256, False), (160, True), (256, True)])
+def test_sign_bits_around_the_edge_of_the_error_bound_follow_the_exact_sums(n, d, rht):
+    """Every key has one planted sum, 0.02 to 2 times what the fp16 sums may be wrong by (about 2^-11 of the norms' product), against rows of the model's own Z --
+    behind the rotation, where there is one.  Half of the keys make the products with that row large, equal in size, positive in the first half of the row and
+    negative in the second, so that the sum runs up and cancels.  A projection of zeros makes the key its own residual."""
+    rng = np.random.default_rng(n + d)
+    p, seed = np.zeros((128, d), F), 7
+    om, gm = ora.Model(p, d, seed=seed, rht=rht), S.Model.from_projection(p, d, seed, rht=rht)
+    dp = om.d_pad
+    z = ora.Rng(seed).gaussian(256 * dp).reshape(256, dp).astype(np.float64)
+    rows = z
+    if rht:  # the row as the key meets it: z (H D / sqrt(dp)) over the key's d coordinates
+        r = ora.Rng(seed ^ 0xA2A2A2A2A2A2A2A2)
+        diag = np.array([-1.0 if r.next_unit() < 0.5 else 1.0 for _ in range(dp)])
+        h = np.ones((1, 1))
+        while len(h) < dp:
+            h = np.block([[h, h], [h, -h]])
+        rows = (z @ h / np.sqrt(dp) * diag)[:, :d]
+    q = np.empty((n, d))
+    for j in range(n):
+        s = int(rng.integers(256))
+        w = rows[s]
+        if j % 2:
+            v = np.where(np.abs(z[s]) > 0.2, 1.0 / np.where(z[s] == 0, 1.0, z[s]), 0.0) * np.where(np.arange(dp) < dp // 2, 1.0, -1.0)
+            x = ((v * (1 + 1e-3 * rng.standard_normal(dp))) @ h / np.sqrt(dp) * diag)[:d] if rht else v * (1 + 1e-3 * rng.standard_normal(dp))
+        else:
+            x = rng.standard_normal(d)
+        x -= (w @ x) / (w @ w) * w
+        want = 0.02 * 100.0 ** rng.random() * rng.choice([-1.0, 1.0]) * 2.0**-11 * np.linalg.norm(x) * np.linalg.norm(w)
+        q[j] = (x + want / (w @ w) * w) * 2.0 ** rng.integers(-20, 20)
+    q = q.astype(F)
+    qc, qs = gm.prepare_queries(q)
+    for j in rng.choice(n, 600, replace=False):
+        assert np.array_equal(qs[j], om.prepare_query(q[j])[1]), j
+    got, want = gm.encode_keys(q, 2), om.encode_batch(q, 2)
     assert got.tobytes() == want.tobytes(), _diff(got, want)
 
 
