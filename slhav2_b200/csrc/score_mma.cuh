@@ -40,14 +40,15 @@ constexpr uint32_t MMA_CHUNK = 16;  // slots a warp reserves at a time in a row'
 // 24 warps), nor for interleaved shares, whose first sets are appended unfiltered (a million MX-16 tiles on one row, k = 100: 81 us, with U = 2 102).
 // Plain shares come in two forms.  LONG: U = 2 (not NF4), a first round with few seeds, Hamming distances only where a tile can reach the threshold.  Short ones
 // have none of the three (INT4 has the latter two in both forms): each costs set-up or instructions and saves where items are long or few tiles are appended.  Taken
-//   INT4, MX-INT4: from 6400 tiles a work item on (the plan's average: segments are cut at the CTAs' shares too), mixed 8/4 and TQ3 from 18 000.  us a call short / long
+//   INT4, MX-INT4: from 6400 tiles a work item on (the plan's average: segments are cut at the CTAs' shares too), mixed 8/4 and TQ3 from 18 000, or
+//     from 10 000 where rows have 1000 k tiles or more (99 segments of 30 303 TQ3 tiles, k = 16 161 / 157, k = 64 166 / 168).  us a call short / long
 //     at items of 4878 (200 segments of 8000 tiles, k = 64), 6521 (150 of 12 000), 9756 (200 of 16 000, k = 256), 14 545 (80 of 40 000, k = 1024), 21 399 (256 of 32 768,
 //     k = 1024), 27 594 (8 of 524 288): INT4 92 / 94, 88 / 86, 161 / 156, 158 / 152; mixed 91 / 100, 91 / 97, 160 / 164, 158 / 159, 368 / 365, 155 / 139;
 //     TQ3 117 / 125, 121 / 126, 211 / 211, 205 / 206, 493 / 485, 219 / 201;
 //   NF4: where rows have 200 k tiles or more on the average, so that few are appended: 256 rows of 32 768 tiles, k = 1024 428 / 443, 200 of 20 000, k = 256 218 / 223, 100 of
 //     40 000 190 / 190, 200 of 16 000, k = 32 160 / 155, 8 of a million, k = 2048 347 / 324.
 constexpr bool stream_long(int kind, bool il, uint64_t item_tiles, uint64_t row_tiles, uint32_t k) {
-    return !il && (kind == 0 ? row_tiles >= 200ull * k : item_tiles >= (kind == 3 ? 6400 : 18000));
+    return !il && (kind == 0 ? row_tiles >= 200ull * k : item_tiles >= (kind == 3 ? 6400 : row_tiles >= 1000ull * k ? 10000 : 18000));
 }
 constexpr int stream_sets(int kind, bool long_items) { return long_items && kind != 0 ? 2 : 1; }
 constexpr int STREAM_THREADS = 768;  // 24 warps at 80 registers: latencies are hidden with warps (U = 2 with 20 or 16 warps: 251, 254 us)

@@ -219,18 +219,20 @@ def _planned_items(lens, sms=148):
     return items
 
 
-# Segments that share one buffer of tiles.  INT4 takes sets of 32 from items of 6400 tiles on the average, mixed 8/4 and TQ3 from 18 000, NF4 never.
+# Segments that share one buffer of tiles.  INT4 takes sets of 32 from items of 6400 tiles on the average, mixed 8/4 and TQ3 from 18 000, or
+# 10 000 where rows have 1000 k tiles, NF4 never.
 LONG = [40_000 + 617 * i for i in range(33)] + [65_536, 40_001, 59_999] + [48_000 + 5 * i for i in range(44)]
 MIDDLE = [12_000 + 3 * i for i in range(150)]
+BETWEEN = [30_000 + 7 * i for i in range(99)]
 
 
 @pytest.mark.parametrize("codec,nq,k,lens,sets", [(0, 4, 60, LONG, 32), (1, 1, 1024, LONG, 32), (3, 3, 61, LONG, 32), (4, 2, 62, LONG, 32), (2, 4, 63, LONG, 16), (2, 3, 301, LONG, 16),
-                                                  (6, 2, 64, MIDDLE, 32), (3, 2, 65, MIDDLE, 16)])
+                                                  (6, 2, 64, MIDDLE, 32), (3, 2, 65, MIDDLE, 16), (4, 3, 20, BETWEEN, 32), (3, 1, 66, BETWEEN, 16)])
 def test_plain_shares_of_long_segments_end_inside_a_set_of_thirty_two(codec, nq, k, lens, sets):
     # segments end at every place of a set; some tiles are WARM or without their correction plane; the last segment ends in tiles of another codec
     # and is handed to the generic kernel
     items = _planned_items(lens)
-    assert (np.mean(items) >= 18_000) == (lens is LONG) and np.mean(items) >= 6400 and len({m % 32 for m in lens}) > 16
+    assert (np.mean(items) >= 18_000) == (lens is LONG) and (np.mean(items) >= 10_000) == (lens is not MIDDLE) and np.mean(items) >= 6400 and len({m % 32 for m in lens}) > 16
     base = np.tile(H.random_tiles(4000, codec, seed=960 + codec, warm_every=9, nocorr_every=6), 17)
     rng = np.random.default_rng(codec)
     rng.shuffle(base)
