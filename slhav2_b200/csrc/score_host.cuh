@@ -732,6 +732,8 @@ __global__ void __launch_bounds__(256) check_offsets_kernel(const uint64_t* offs
         *reinterpret_cast<volatile uint32_t*>(answer) = bad;
     }
 }
+// A check whose answer nobody has waited for (a call that ended by an exception): its kernel may still write the word.
+thread_local bool g_check_pending[16] = {false};
 Status launch_check_offsets(Ctx* c, const uint64_t* d_offsets, size_t nq, uint64_t scores_len, uint32_t row_len, const uint64_t** d_copy, const uint32_t** d_refused) {
     SLHA_TRY(ctx_no_capture(c));
     if (nq > 0xFFFFFFFFull) return Status(SLHA_ERR_DIMENSION, "too many query rows");
@@ -741,11 +743,13 @@ Status launch_check_offsets(Ctx* c, const uint64_t* d_offsets, size_t nq, uint64
     uint32_t* answer;
     cudaEvent_t event;
     SLHA_TRY(ctx_answer(c, &host, &answer, &event));
+    if (g_check_pending[c->device & 15]) SLHA_CUDA(cudaEventSynchronize(event));
     uint64_t* copy = static_cast<uint64_t*>(dev);
     uint32_t* refused = reinterpret_cast<uint32_t*>(copy + nq);
     SLHA_CUDA(launch_behind(check_offsets_kernel, dim3(1), dim3(256), 0, c->stream, d_offsets, (uint32_t)nq, scores_len, row_len, copy, refused, answer));
     count_launch();
     SLHA_CUDA(cudaEventRecord(event, c->stream));
+    g_check_pending[c->device & 15] = true;
     *d_copy = copy;
     *d_refused = refused;
     return Status();
@@ -756,6 +760,7 @@ Status checked_offsets(Ctx* c, bool* refused) {
     cudaEvent_t event;
     SLHA_TRY(ctx_answer(c, &host, &answer, &event));
     SLHA_CUDA(cudaEventSynchronize(event));
+    g_check_pending[c->device & 15] = false;
     *refused = *host != 0;
     return Status();
 }
