@@ -283,6 +283,7 @@ struct ScoreArgs {
     // full mode
     float* scores;            // [nq][score_stride]
     uint64_t score_stride;
+    uint32_t cold_bits;       // what a COLD slot's score is written as
     const uint32_t* refused;  // optional (full-score mode): nothing is written where it holds 1
     const unsigned long long* row_offset;  // optional (full-score mode): row q starts at scores + row_offset[q] instead of q * score_stride
     // top-k mode
@@ -301,6 +302,8 @@ struct ScoreArgs {
     uint32_t* ghist;              // per query row: 256 bucket counts of appended candidates
     uint32_t* gcount;             // per query row: candidates appended to the row's buffer
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
+    uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): 1, or 2 where that pass is to
+    uint32_t handoff_as;          // score them in score_kernel's arithmetic (NF4 rows always 1)
     const uint32_t* only_flagged; // dense mode: optional, per query row: only work items one of whose rows is flagged here
     uint64_t* gbuf;               // per query row: gcap composite keys
     uint32_t gcap;
@@ -417,7 +420,7 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
                         }
                     } else if (ti < n) {
                         const size_t row0 = a.row_offset ? (size_t)a.row_offset[it.query_begin + g] : (size_t)(it.query_begin + g) * a.score_stride;
-                        a.scores[row0 + it.index_base + ti] = live ? sc : -INFINITY;
+                        a.scores[row0 + it.index_base + ti] = live ? sc : __uint_as_float(a.cold_bits);
                     }
                 }
             }
@@ -452,6 +455,83 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
     }
 }
 
+// Work items that a dense kernel's CTA could not score on the tensor cores (a tile of another codec than its item's first, a query outside the fp16
+// split), to be scored in score_kernel's arithmetic once the CTA is through: in its loop the call would cost registers.
+struct Undone {
+    uint32_t n;
+    uint32_t item[31];  // (more than these: all of the CTA's items)
+};
+__device__ __forceinline__ void undone_add(Undone& u, uint32_t item) {  // one thread of the CTA
+    if (u.n < 31u) u.item[u.n] = item;
+    ++u.n;
+}
+// Dense scores of one work item by the whole CTA, rows query_begin .. + nq (four at most).  smem: 4 KB, and 4 KB a warp.
+__device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem& it, uint32_t query_begin, int nq, unsigned char* smem) {
+    constexpr int G = 4;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
+    const int t = lane >> 3, s = lane & 7;
+    float* qsm = reinterpret_cast<float*>(smem);
+    float* lut = qsm + G * D_C;
+    unsigned char* stage = smem + 4096 + (size_t)warp * BLK_BYTES;
+    const uint32_t n = it.n_tiles;
+    __syncthreads();
+    for (int i = tid; i < G * D_C; i += blockDim.x) qsm[i] = i / D_C < nq ? a.q_coarse[(size_t)(query_begin + i / D_C) * D_C + (i % D_C)] : 0.0f;
+    for (int i = tid; i < 16 * 32; i += blockDim.x) lut[i] = c_nf4[i >> 5];
+    __syncthreads();
+    float qreg[G][16];
+    uint32_t qs[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) qreg[g][j] = qsm[g * D_C + 16 * s + j];
+        qs[g] = g < nq ? a.q_sign[(size_t)(query_begin + g) * 8 + s] : 0u;
+    }
+    for (uint32_t blk = warp; blk < (n + BLK_TILES - 1) / BLK_TILES; blk += nwarps) {
+        const uint32_t my = blk * BLK_TILES + lane;
+        const uint32_t st_lane = a.state && my < n ? a.state[it.tile_begin + my] : ST_HOT;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < ITER; ++i) {
+            const uint32_t ti = blk * BLK_TILES + i * 4 + t;
+            const uint32_t stt = __shfl_sync(0xFFFFFFFFu, st_lane, i * 4 + t);
+            const bool live = ti < n && stt != ST_COLD;
+            cp_async16(stage + i * ITER_BYTES + stage_off(t, s * 16), a.tiles + (it.tile_begin + (live ? ti : 0)) * TILE_BYTES + s * 16, live ? 16 : 0);
+        }
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncwarp();
+        float part[G][ITER];
+#pragma unroll
+        for (int i = 0; i < ITER; ++i) {
+            float o[G];
+            tile_partial<G>(stage + i * ITER_BYTES, t, s, lane, qreg, qs, qsm, lut, o);
+#pragma unroll
+            for (int g = 0; g < G; ++g) part[g][i] = o[g];
+        }
+        const uint32_t ti = blk * BLK_TILES + 4 * s + t;
+        const uint32_t stt = __shfl_sync(0xFFFFFFFFu, st_lane, 4 * s + t);
+        const bool live = ti < n && stt != ST_COLD;
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const float sc = transpose_reduce8(part[g], s);
+            if (g < nq && ti < n) {
+                const size_t row0 = a.row_offset ? (size_t)a.row_offset[query_begin + g] : (size_t)(query_begin + g) * a.score_stride;
+                a.scores[row0 + it.index_base + ti] = live ? sc : __uint_as_float(a.cold_bits);
+            }
+        }
+    }
+    __syncthreads();
+}
+// What is left at a CTA's end (all of its shared memory is free).
+__device__ __noinline__ void finish_undone(const ScoreArgs& a, const WorkItem* items, const Undone& u, unsigned char* smem) {
+    __syncthreads();
+    const uint32_t m = u.n, first = a.cta_begin[blockIdx.x], end = a.cta_begin[blockIdx.x + 1];
+    for (uint32_t j = 0; j < (m > 31u ? end - first : m); ++j) {
+        const WorkItem it = items[m > 31u ? first + j : u.item[j]];
+        for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
+    }
+}
+
 }  // namespace
 }  // namespace slha
 
@@ -459,6 +539,7 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
 #include "score_tile.cuh"
 #include "score_wide.cuh"
 #include "score_merge.cuh"
+#include "score_select.cuh"
 #include "score_host.cuh"
 
 // ---------------------------------------------------------------------------

@@ -81,9 +81,29 @@ Status launch_wide(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
         default: return launch_wide_t<4>(c, a, grid);
     }
 }
-Status launch_wide_dense(Ctx* c, const ScoreArgs& a, uint32_t grid) {
+Status launch_wide_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_wide_dense_kernel, configured, a, grid, WIDE_THREADS, wide_smem_bytes());
+    return launch_tc(c, score_wide_dense_kernel, configured, a, grid, WIDE_THREADS, wide_smem_bytes(), behind);
+}
+template <int NT, int R>
+Status launch_rows_t(Ctx* c, const RowsArgs& a, uint32_t nq) {
+    static thread_local bool configured[16] = {false};
+    if (!configured[c->device & 15]) {
+        SLHA_CUDA(cudaFuncSetAttribute(topk_rows_kernel<NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)row_smem(row_cap(4096, 4096), NT, R)));
+        SLHA_CUDA(cudaFuncSetAttribute(topk_rows_kernel<NT, R>, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        configured[c->device & 15] = true;
+    }
+    SLHA_CUDA(launch_behind(topk_rows_kernel<NT, R>, dim3(nq), dim3(NT), row_smem(a.cap, NT, R), c->stream, a));
+    count_launch();
+    return Status();
+}
+constexpr uint32_t ROWS_MOST = 32768;  // scores of a row that topk_rows_kernel takes
+Status launch_rows(Ctx* c, const RowsArgs& a, uint32_t nq, uint32_t longest) {
+    if (longest <= 2048) return launch_rows_t<256, 2>(c, a, nq);
+    if (longest <= 4096) return launch_rows_t<512, 2>(c, a, nq);
+    if (longest <= 8192) return launch_rows_t<512, 4>(c, a, nq);
+    if (longest <= 16384) return launch_rows_t<512, 8>(c, a, nq);
+    return launch_rows_t<512, 16>(c, a, nq);
 }
 
 size_t score_smem_bytes(int G, int nwarps, bool topk, uint32_t cap) {
@@ -231,6 +251,12 @@ struct Plan {
     uint32_t* d_vq_count = nullptr;
     uint32_t* d_tmp_index = nullptr;
     float* d_tmp_score = nullptr;
+    // Rows whose scores are written as a whole and selected from (score_select.cuh)
+    bool rows = false, allow_rows_in = false;
+    uint32_t longest = 0, grid_narrow = 0, grid_wide = 0;
+    uint64_t row_stride = 0;
+    RowInfo* d_rows = nullptr;
+    uint32_t* d_row_flags = nullptr;  // [nq] generic arithmetic, [nq] handed on by the 64-row kernel, [nq][2] statistics
     uint64_t last_use = 0;
     bool captured = false;  // a graph of the library's own names this plan's buffers (see plan_epoch)
 };
@@ -238,8 +264,107 @@ thread_local Plan* g_last_plan = nullptr;    // of the thread's latest score_top
 thread_local uint32_t g_plans_recycled = 0;  // of this thread's captured plans
 std::atomic<uint32_t> g_plan_threads{0};
 
+// Cuts of (segment, group of up to `width` query rows) streams into one share per CTA.
+struct Cuts {
+    std::vector<WorkItem> items;
+    std::vector<uint32_t> cta{0u};
+    uint64_t share = 0, filled = 0;
+    Cuts(uint64_t total, int sms, uint64_t unit, uint64_t least) {
+        share = (total + sms - 1) / sms;
+        share = std::max<uint64_t>(least, (share + unit - 1) / unit * unit);
+    }
+    void add(const SlhaB200Segment& s, uint32_t width) {
+        for (uint32_t q0 = 0; q0 < s.n_queries; q0 += width)
+            for (uint64_t pos = 0; pos < s.n_tiles;) {
+                const uint32_t take = (uint32_t)std::min<uint64_t>(s.n_tiles - pos, share - filled);
+                WorkItem w{};
+                w.tile_begin = s.tile_begin + pos;
+                w.n_tiles = take;
+                w.index_base = s.index_base + (uint32_t)pos;
+                w.query_begin = s.query_begin + q0;
+                w.n_queries = std::min<uint32_t>(width, s.n_queries - q0);
+                items.push_back(w);
+                pos += take;
+                filled += take;
+                if (filled >= share) {
+                    filled = 0;
+                    cta.push_back((uint32_t)items.size());
+                }
+            }
+    }
+    void finish() {
+        if (cta.back() != (uint32_t)items.size()) cta.push_back((uint32_t)items.size());
+    }
+};
+
+// Whether a call's rows are scored as a whole (score_select.cuh) rather than streamed: rows of up to ROWS_MOST tiles, scores of 64 MB at most.  `passes`: tiles times
+// groups of four query rows, `wide`: 16 rows or more a segment, which the 64-row kernel takes (512 rows of 16 384 TQ3 tiles, k = 256 86 -> 51 us; 1232 of
+// 3553 MX tiles 111 -> 53).  Streaming reads a million tiles in 25 us where score_dense_kernel takes 40 (NF4 60), but its first sets, hand-over check, compaction and
+// merge cost 20 to 50 us more, most with many winners.  us a call, streamed / whole, k = 64 and 1024: 8192 INT4 tiles 22.9 / 15.6, 27.7 / 16.0; 32 segments of
+// 8192 mixed tiles 35.8 / 26.2, 46.0 / 29.2; 64 of 16 384 INT4 61 / 54, 89 / 59, TQ3 80 / 67, 108 / 72, NF4 73 / 78, 100 / 82; 100 of 16 384 INT4 80 / 81, 108 / 88,
+// NF4 95 / 117, 120 / 124; 128 of 32 768 INT4 137 / 193, 187 / 212; MIX3 16 of 32 768 59 / 45, 76 / 49.
+enum RowsRule { ROWS_NO, ROWS_YES, ROWS_UNLESS_NF4 };
+RowsRule rows_rule(uint64_t passes, bool wide, size_t nq, uint32_t longest, uint32_t k) {
+    if (longest == 0 || longest > ROWS_MOST || nq * (((uint64_t)longest + 31) / 32 * 32) > (16ull << 20)) return ROWS_NO;
+    const uint64_t more = k >= 512 ? 2 : 1;
+    if (wide || passes <= 640000 * more) return ROWS_YES;
+    return passes <= 1280000 * more ? ROWS_UNLESS_NF4 : ROWS_NO;
+}
+
+Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_segs, size_t nq, uint32_t longest, bool allow_wide) {
+    const int sms = sm_count(c->device);
+    bool wide = true;
+    uint64_t total = 0, wtotal = 0;
+    std::vector<RowInfo> rows(nq, RowInfo{0u, 0u});
+    std::vector<uint8_t> taken(nq, 0);
+    for (size_t i = 0; i < n_segs; ++i) {
+        const SlhaB200Segment& s = segs[i];
+        if ((uint64_t)s.query_begin + s.n_queries > nq) return Status(SLHA_ERR_DIMENSION, "segment query range exceeds n_queries");
+        for (uint32_t q = 0; q < s.n_queries; ++q) {
+            if (taken[s.query_begin + q]) return Status(SLHA_ERR_DIMENSION, "a query row belongs to two segments");
+            taken[s.query_begin + q] = s.n_tiles != 0;
+            rows[s.query_begin + q] = RowInfo{s.n_tiles, s.index_base};
+        }
+        wide = wide && (s.n_queries >= 16 || s.n_tiles == 0);
+        total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
+        wtotal += (uint64_t)s.n_tiles * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
+    }
+    Cuts narrow(total, sms, ST_M, ST_M), many(wtotal, sms, WIDE_M, WIDE_M);
+    for (size_t i = 0; i < n_segs; ++i) {
+        SlhaB200Segment s = segs[i];
+        s.index_base = 0;  // (where the scores go: a place in the row)
+        narrow.add(s, 4);
+        if (wide) many.add(s, WIDE_NQ);
+    }
+    narrow.finish();
+    many.finish();
+    Blob tables;
+    const size_t o_n = tables.add(narrow.items), o_nc = tables.add(narrow.cta), o_w = tables.add(many.items), o_wc = tables.add(many.cta), o_r = tables.add(rows);
+    SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
+    SLHA_TRY(p->b_gpivot.ensure(4 * nq * 4));
+    p->row_stride = ((uint64_t)longest + 31) / 32 * 32;
+    SLHA_TRY(p->b_gbuf.ensure(nq * p->row_stride * 4));
+    unsigned char* dev = static_cast<unsigned char*>(p->b_tables.p);
+    SLHA_TRY(ctx_copy_table(c, dev, tables.bytes.data(), tables.bytes.size()));
+    p->d_row_flags = (uint32_t*)p->b_gpivot.p;
+    SLHA_CUDA(cudaMemsetAsync(p->d_row_flags, 0, 4 * nq * 4, c->stream));
+    p->d_items = reinterpret_cast<WorkItem*>(dev + o_n);
+    p->d_cta_begin = reinterpret_cast<uint32_t*>(dev + o_nc);
+    p->d_wide_items = reinterpret_cast<WorkItem*>(dev + o_w);
+    p->d_wide_cta = reinterpret_cast<uint32_t*>(dev + o_wc);
+    p->d_rows = reinterpret_cast<RowInfo*>(dev + o_r);
+    p->wide = wide && allow_wide && !many.items.empty();
+    p->grid_narrow = (uint32_t)narrow.cta.size() - 1;
+    p->grid_wide = (uint32_t)many.cta.size() - 1;
+    p->n_items = (uint32_t)narrow.items.size();
+    p->n_wide_items = (uint32_t)many.items.size();
+    p->longest = longest;
+    p->rows = true;
+    return Status();
+}
+
 Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, size_t nq,
-                  uint32_t k, int codec_hint, bool allow_wide, Plan** out) {
+                  uint32_t k, int codec_hint, bool allow_wide, bool allow_rows, Plan** out) {
     std::vector<unsigned char> key(sizeof(SlhaB200Segment) * n_segs + 16);
     std::memcpy(key.data(), segs, sizeof(SlhaB200Segment) * n_segs);
     uint64_t nq64 = nq;
@@ -251,7 +376,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     static thread_local uint64_t tick = 0;
     ++tick;
     for (auto& e : cache)
-        if (e->device == c->device && e->codec_hint_in == codec_hint && e->force_generic_in == g_force_generic && e->allow_wide_in == allow_wide && e->key == key) {
+        if (e->device == c->device && e->codec_hint_in == codec_hint && e->force_generic_in == g_force_generic && e->allow_wide_in == allow_wide && e->allow_rows_in == allow_rows && e->key == key) {
             e->last_use = tick;
             *out = e.get();
             return Status();
@@ -278,12 +403,53 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     p->codec_hint_in = codec_hint;
     p->force_generic_in = g_force_generic;
     p->allow_wide_in = allow_wide;
-    p->wide = false;
+    p->allow_rows_in = allow_rows;
+    p->wide = p->rows = false;
     p->k = k;
     p->n_lists = 0;
     p->nq = (uint32_t)nq;
     p->kp2 = 2;
     while (p->kp2 < k) p->kp2 <<= 1;
+    // Codec hint: -1 = the flags of the first tile of the first non-empty segment decide which kind of tile a streaming launch
+    // decodes.  A wrong hint costs speed only (tiles of another kind are handed to the generic kernel).
+    auto look = [&]() -> Status {
+        p->kind = codec_hint < 0 ? 3 : hint_kind(codec_hint);
+        for (size_t i = 0; i < n_segs && codec_hint < 0; ++i)
+            if (segs[i].n_tiles) {
+                uint16_t flags = 0;
+                const unsigned char* t0 = reinterpret_cast<const unsigned char*>(tiles) + segs[i].tile_begin * TILE_BYTES;
+                SLHA_CUDA(cudaMemcpyAsync(&flags, t0 + 118, 2, cudaMemcpyDeviceToHost, c->stream));
+                SLHA_CUDA(cudaStreamSynchronize(c->stream));
+                p->kind = stream_kind(flags);
+                break;
+            }
+        return Status();
+    };
+    bool looked = false;
+    if (allow_rows && !g_force_generic) {
+        uint32_t longest = 0;
+        uint64_t passes = 0;
+        bool wide = true;
+        for (size_t i = 0; i < n_segs; ++i) {
+            if (segs[i].n_queries) longest = std::max(longest, segs[i].n_tiles);
+            wide = wide && (segs[i].n_queries >= 16 || segs[i].n_tiles == 0);
+            passes += (uint64_t)segs[i].n_tiles * ((segs[i].n_queries + 3) / 4);
+        }
+        RowsRule rule = rows_rule(passes, wide && allow_wide, nq, longest, k);
+        if (rule == ROWS_UNLESS_NF4) {
+            SLHA_TRY(look());
+            looked = true;
+            rule = p->kind == 0 ? ROWS_NO : ROWS_YES;
+        }
+        if (rule == ROWS_YES) {
+            SLHA_TRY(build_rows_plan(c, p, segs, n_segs, nq, longest, allow_wide));
+            p->use_mma = true;
+            p->key = std::move(key);
+            p->device = c->device;
+            *out = p;
+            return Status();
+        }
+    }
     p->threads = k > 1024 ? 256 : 128;
     const int nwarps = p->threads / 32;
     const uint32_t round = (uint32_t)nwarps * BLK_TILES;
@@ -296,18 +462,7 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
     // tensor-core kernel: one persistent CTA per SM
     const int sms = sm_count(c->device);
     {
-        // Codec hint: -1 = the flags of the first tile of the first non-empty segment decide which kind of tile the launch
-        // decodes.  A wrong hint costs speed only (tiles of another kind are handed to the generic kernel).
-        p->kind = codec_hint < 0 ? 3 : hint_kind(codec_hint);
-        for (size_t i = 0; i < n_segs && codec_hint < 0; ++i)
-            if (segs[i].n_tiles) {
-                uint16_t flags = 0;
-                const unsigned char* t0 = reinterpret_cast<const unsigned char*>(tiles) + segs[i].tile_begin * TILE_BYTES;
-                SLHA_CUDA(cudaMemcpyAsync(&flags, t0 + 118, 2, cudaMemcpyDeviceToHost, c->stream));
-                SLHA_CUDA(cudaStreamSynchronize(c->stream));
-                p->kind = stream_kind(flags);
-                break;
-            }
+        if (!looked) SLHA_TRY(look());
         p->use_mma = !g_force_generic;
         p->mma_grid = (uint32_t)sms;
     }
@@ -627,45 +782,11 @@ Status launch_validate_tiles(Ctx* c, const SciRustSlhaTile* tiles, size_t n, uns
     return Status();
 }
 
-// Cuts of (segment, group of up to `width` query rows) streams into one share per CTA.
-struct Cuts {
-    std::vector<WorkItem> items;
-    std::vector<uint32_t> cta{0u};
-    uint64_t share = 0, filled = 0;
-    Cuts(uint64_t total, int sms, uint64_t unit, uint64_t least) {
-        share = (total + sms - 1) / sms;
-        share = std::max<uint64_t>(least, (share + unit - 1) / unit * unit);
-    }
-    void add(const SlhaB200Segment& s, uint32_t width) {
-        for (uint32_t q0 = 0; q0 < s.n_queries; q0 += width)
-            for (uint64_t pos = 0; pos < s.n_tiles;) {
-                const uint32_t take = (uint32_t)std::min<uint64_t>(s.n_tiles - pos, share - filled);
-                WorkItem w{};
-                w.tile_begin = s.tile_begin + pos;
-                w.n_tiles = take;
-                w.index_base = s.index_base + (uint32_t)pos;
-                w.query_begin = s.query_begin + q0;
-                w.n_queries = std::min<uint32_t>(width, s.n_queries - q0);
-                items.push_back(w);
-                pos += take;
-                filled += take;
-                if (filled >= share) {
-                    filled = 0;
-                    cta.push_back((uint32_t)items.size());
-                }
-            }
-    }
-    void finish() {
-        if (cta.back() != (uint32_t)items.size()) cta.push_back((uint32_t)items.size());
-    }
-};
-
 Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state, size_t n,
                          const float* q_coarse, const uint64_t* q_sign, size_t nq, float* scores, int codec_hint) {
     if (n == 0 || nq == 0) return Status();
     // Long arenas: the streaming tensor-core kernel in its dense mode (all query groups of four in one launch, every CTA an
-    // equal share of the tiles), then the generic kernel for the rows of work items it handed back (a codec it does not
-    // decode, a query outside the fp16 split).  codec_hint -2: codecs the tensor-core kernel does not decode together;
+    // equal share of the tiles).  codec_hint -2: codecs the tensor-core kernel does not decode together;
     // bit 0: NF4 tiles beside INT4 ones; -1: not known.
     if (n >= 32768 && n < 0xFFFFFFFFull && codec_hint != -2 && !g_force_generic) {
         const int sms = sm_count(c->device);
@@ -673,10 +794,11 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         cuts.add(SlhaB200Segment{0, (uint32_t)n, 0, (uint32_t)nq, 0}, 4);
         cuts.finish();
         Blob blob;
-        const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta), o_flag = blob.add(std::vector<uint32_t>(nq, 0u));
+        const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta);
         unsigned char* dev;
         SLHA_TRY(blob.upload(c, &dev));
         ScoreArgs a{};
+        a.cold_bits = 0xFF800000u;
         a.tiles = reinterpret_cast<const unsigned char*>(tiles);
         a.state = state;
         a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_items);
@@ -687,11 +809,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.scores = scores;
         a.score_stride = n;
         a.nf4_table = codec_hint < 0 ? 2u : (uint32_t)(codec_hint & 1);
-        a.gflag = reinterpret_cast<uint32_t*>(dev + o_flag);
-        SLHA_TRY(launch_dense(c, a, (uint32_t)cuts.cta.size() - 1, false));
-        // the generic kernel over the same work items, only those whose rows were handed back
-        const int threads = 128, nwarps = threads / 32;
-        return launch_score<false>(c, 4, a, (uint32_t)cuts.items.size(), threads, score_smem_bytes(4, nwarps, false, 0), true);
+        return launch_dense(c, a, (uint32_t)cuts.cta.size() - 1, false);
     }
     const int threads = 128, nwarps = threads / 32;
     const uint32_t item_tiles = 4096;
@@ -707,6 +825,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.q_coarse = q_coarse + q0 * D_C;
         a.q_sign = reinterpret_cast<const uint32_t*>(q_sign + q0 * 4);
         a.scores = scores + q0 * n;
+        a.cold_bits = 0xFF800000u;
         a.score_stride = n;
         a.total_tiles = n;
         a.item_tiles = item_tiles;
@@ -773,9 +892,9 @@ __global__ void fill_rows_kernel(float* scores, const unsigned long long* row_of
 }
 
 // Dense scores of whole segments: every query row of a segment against every tile of the segment, row q written at
-// scores + row_offsets[q] + index_base + tile, the rest of the row up to row_len set to `fill`.  Up to three passes over the
-// same call, each for the rows the one before handed over (the last two end at once when there are none): the 64-row kernel
-// where every segment brings 16 query rows or more, the four-row kernel, the generic kernel.  The host looks at no tile and waits for nothing.
+// scores + row_offsets[q] + index_base + tile, the rest of the row up to row_len set to `fill`.  Where every segment brings 16 query rows or
+// more the 64-row kernel comes first and the four-row kernel takes the rows it hands over (it ends at once when there are none).  The host looks at no tile and
+// waits for nothing.
 Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, const float* d_q_coarse,
                              const uint64_t* d_q_sign, size_t nq, float* d_scores, const unsigned long long* d_row_offsets,
                              uint32_t row_len, float fill, const uint32_t* refused) {
@@ -800,18 +919,19 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     }
     narrow.finish();
     many.finish();
-    std::vector<WorkItem> generic;  // runs of 4096 tiles for the last pass
-    for (const WorkItem& s : narrow.items)
-        for (uint32_t pos = 0; pos < s.n_tiles; pos += 4096) {
-            WorkItem w = s;
-            w.tile_begin += pos;
-            w.index_base += pos;
-            w.n_tiles = std::min<uint32_t>(4096, s.n_tiles - pos);
-            generic.push_back(w);
-        }
+    std::vector<WorkItem> generic;  // runs of 4096 tiles where score_kernel takes the call
+    if (g_force_generic)
+        for (const WorkItem& s : narrow.items)
+            for (uint32_t pos = 0; pos < s.n_tiles; pos += 4096) {
+                WorkItem w = s;
+                w.tile_begin += pos;
+                w.index_base += pos;
+                w.n_tiles = std::min<uint32_t>(4096, s.n_tiles - pos);
+                generic.push_back(w);
+            }
     Blob blob;
     const size_t o_narrow = blob.add(narrow.items), o_ncta = blob.add(narrow.cta), o_many = blob.add(many.items), o_mcta = blob.add(many.cta), o_gen = blob.add(generic);
-    const size_t o_tail = blob.add(tail), o_flag = blob.add(std::vector<uint32_t>(2 * nq, 0u));
+    const size_t o_tail = blob.add(tail), o_flag = blob.add(std::vector<uint32_t>(nq, 0u));
     unsigned char* dev;
     SLHA_TRY(blob.upload(c, &dev));
     if (fills) {
@@ -826,27 +946,65 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
     a.scores = d_scores;
     a.row_offset = d_row_offsets;
+    a.cold_bits = 0xFF800000u;
     a.refused = refused;
     uint32_t* flag = reinterpret_cast<uint32_t*>(dev + o_flag);
     if (wide) {
         a.items = reinterpret_cast<const WorkItem*>(dev + o_many);
         a.n_items = (uint32_t)many.items.size();
         a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_mcta);
-        a.gflag = flag + nq;
-        SLHA_TRY(launch_wide_dense(c, a, (uint32_t)many.cta.size() - 1));
-        a.only_flagged = flag + nq;
+        a.handoff = flag;
+        a.handoff_as = 1u;
+        SLHA_TRY(launch_wide_dense(c, a, (uint32_t)many.cta.size() - 1, false));
+        a.only_flagged = flag;
     }
     a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_narrow);
     a.n_items = (uint32_t)narrow.items.size();
     a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_ncta);
-    a.gflag = nullptr;
-    if (!g_force_generic) {
-        a.gflag = flag;
-        SLHA_TRY(launch_dense(c, a, (uint32_t)narrow.cta.size() - 1, wide));
-    }
+    if (!g_force_generic) return launch_dense(c, a, (uint32_t)narrow.cta.size() - 1, wide);
     a.items = reinterpret_cast<const WorkItem*>(dev + o_gen);
     const int threads = 128, nwarps = threads / 32;
-    return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0), !g_force_generic);
+    return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0), false);
+}
+
+// Every score of every row, then the rows' best.
+static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, const uint8_t* state, const float* d_q_coarse, const uint64_t* d_q_sign, size_t nq, uint32_t k,
+                              uint32_t* d_out_index, float* d_out_score, uint32_t* d_out_count, int codec_hint) {
+    const bool timed = g_timing.calls < g_timing.max_calls;
+    cudaEvent_t* tev = timed ? &g_timing.ev[3 * g_timing.calls] : nullptr;
+    if (timed) SLHA_CUDA(cudaEventRecord(tev[0], c->stream));
+    g_last_stream_plan = p;
+    ScoreArgs a{};
+    a.tiles = reinterpret_cast<const unsigned char*>(tiles);
+    a.state = state;
+    a.q_coarse = d_q_coarse;
+    a.q_sign = reinterpret_cast<const uint32_t*>(d_q_sign);
+    a.scores = reinterpret_cast<float*>(p->b_gbuf.p);
+    a.score_stride = p->row_stride;
+    a.cold_bits = ROW_ABSENT;
+    a.nf4_table = codec_hint < 0 ? 2u : (uint32_t)(codec_hint & 1);
+    a.gflag = p->d_row_flags;
+    if (p->wide) {
+        a.items = p->d_wide_items;
+        a.n_items = p->n_wide_items;
+        a.cta_begin = p->d_wide_cta;
+        a.handoff = p->d_row_flags + nq;
+        a.handoff_as = 2u;
+        SLHA_TRY(launch_wide_dense(c, a, p->grid_wide, true));
+        a.only_flagged = a.handoff;
+    }
+    a.items = a.stream_items = p->d_items;
+    a.n_items = p->n_items;
+    a.cta_begin = p->d_cta_begin;
+    SLHA_TRY(launch_dense(c, a, p->grid_narrow, true));
+    if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));
+    RowsArgs r{a.scores, p->row_stride, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, p->kp2, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
+    SLHA_TRY(launch_rows(c, r, (uint32_t)nq, p->longest));
+    if (timed) {
+        SLHA_CUDA(cudaEventRecord(tev[2], c->stream));
+        ++g_timing.calls;
+    }
+    return Status();
 }
 
 Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state,
@@ -859,8 +1017,9 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     if (k == 0 || k > 4096) return Status(SLHA_ERR_DIMENSION, "top-k: k must be in 1..4096");
     ctx_uses_plans(c);
     Plan* p = nullptr;
-    SLHA_TRY(build_plan(c, tiles, segs, n_segs, nq, k, codec_hint, /*allow_wide=*/state == nullptr, &p));
+    SLHA_TRY(build_plan(c, tiles, segs, n_segs, nq, k, codec_hint, /*allow_wide=*/state == nullptr, /*allow_rows=*/!prefer_generic, &p));
     g_last_plan = p;
+    if (p->rows) return score_topk_rows(c, p, tiles, state, d_q_coarse, d_q_sign, nq, k, d_out_index, d_out_score, d_out_count, codec_hint);
     const int nwarps = p->threads / 32;
     const bool timed = g_timing.calls < g_timing.max_calls;
     cudaEvent_t* tev = timed ? &g_timing.ev[3 * g_timing.calls] : nullptr;
@@ -999,7 +1158,7 @@ Status last_score_stats(Ctx* c, uint64_t* out4) {
     if (!p || p->device != c->device || !p->use_mma) return Status();
     const size_t nq = p->nq;
     std::vector<uint32_t> h(2 * nq);
-    const uint32_t* stats = reinterpret_cast<const uint32_t*>(p->d_gpivot + 128 * nq + 2 * nq) + 3 * nq;  // kept by the merge
+    const uint32_t* stats = p->rows ? p->d_row_flags + 2 * nq : reinterpret_cast<const uint32_t*>(p->d_gpivot + 128 * nq + 2 * nq) + 3 * nq;  // kept by the merge
     SLHA_CUDA(cudaMemcpyAsync(h.data(), stats, 8 * nq, cudaMemcpyDeviceToHost, c->stream));
     SLHA_CUDA(cudaStreamSynchronize(c->stream));
     out4[0] = nq;
@@ -1007,14 +1166,14 @@ Status last_score_stats(Ctx* c, uint64_t* out4) {
         out4[1] += h[2 * q + 1] != 0;
         out4[2] += h[2 * q];
     }
-    out4[3] = p->gcap;
+    out4[3] = p->rows ? p->row_stride : p->gcap;
     return Status();
 }
 
 // Tiles a warp of that call took at a time.
 uint32_t last_score_set(Ctx* c) {
     const Plan* p = g_last_stream_plan;
-    return !p || p->device != c->device || !p->use_mma || p->wide || p->kind == 4 ? 0u : (uint32_t)(MMA_SET_TILES * p->sets);
+    return !p || p->device != c->device || !p->use_mma || p->wide || (!p->rows && p->kind == 4) ? 0u : (uint32_t)(MMA_SET_TILES * (p->rows ? 1 : p->sets));
 }
 
 bool timing_active() { return g_timing.calls < g_timing.max_calls; }

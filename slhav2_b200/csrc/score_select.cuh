@@ -1,0 +1,347 @@
+// Top-k of rows whose scores have all been written: one CTA per query row.  Included by score.cu after score_merge.cuh.
+//
+// Where a row is short (a decode step over an ordinary context, a batch of queries on one cache) the streaming top-k has little to stream: its thresholds come
+// from the first tiles of every warp, which are appended unfiltered, and the passes behind it (hand-over check, compaction, merge) each cost
+// a launch and a chain of latencies.  Scores written as a whole cost four bytes a tile and row, which the L2 keeps, and need no threshold while they
+// are made.  Here a row's scores go to registers, a sample of them gives a bound that little more than k reach, every thread keeps the few of its own that do,
+// a histogram between the bound and the largest score of the sample gives each of those its bucket, and its place is the bucket's plus the number of larger
+// ones in the bucket.
+// Bound: the latencies between eight block barriers, and for many rows the instructions a score costs.
+#pragma once
+
+namespace slha {
+namespace {
+
+constexpr int ROW_BUCKETS = 1024;
+constexpr uint32_t ROW_ABSENT = 0xFFFFFFFFu;      // bits of a score that is not there (no arithmetic gives this NaN)
+constexpr int row_own(int r) { return 4 * r < 16 ? 4 * r : 16; }  // candidates a thread keeps
+struct RowInfo {
+    uint32_t n, index_base;  // scores of the row, reported index of the first
+};
+struct RowsArgs {
+    const float* scores;     // row q starts at q * stride
+    uint64_t stride;
+    const RowInfo* rows;
+    uint32_t* flag;          // [nq] a work item of the row took the generic arithmetic, [nq] it was handed on by the 64-row kernel (cleared here)
+    uint32_t* stats;         // [nq][2] candidates, the flag
+    uint32_t k, kp2, cap;    // cap: slots for candidates, row_cap(k, kp2)
+    uint32_t* out_index;
+    float* out_score;
+    uint32_t* out_count;
+};
+// slots: what a sample's bound lets through, see below, and kp2 winners
+inline uint32_t row_cap(uint32_t k, uint32_t kp2) { return std::max(kp2, std::min(4u * k + 1024u, 2u * k + 2560u)); }
+constexpr int ROW_HIST_INTS = ROW_BUCKETS + 64;
+inline size_t row_smem(uint32_t cap, int nt, int r) { return (size_t)cap * 8 + (size_t)nt * row_own(r) * 8 + (size_t)(ROW_HIST_INTS + 64) * 4; }
+
+// R: 4 R scores a thread, n <= 4 R x threads
+template <int NT, int R>
+__global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    dep_launch();
+    dep_wait();
+    constexpr int OWN = row_own(R), PER = ROW_BUCKETS / NT;
+    const uint32_t k = a.k, cap = a.cap, Q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint64_t* buf = reinterpret_cast<uint64_t*>(smem);                     // [cap]
+    uint64_t* own = buf + cap + tid;                                       // [OWN], NT apart
+    int* hist = reinterpret_cast<int*>(buf + cap + NT * OWN);              // [ROW_BUCKETS + 1]
+    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket, 4 a thread holds too many, 8.. of a selection step, 16.. warp totals
+    const RowInfo info = a.rows[Q];
+    const uint32_t n = info.n;
+    const float* row = a.scores + (size_t)Q * a.stride;
+    // thread t holds the scores 4 (t + NT j) .. + 3
+    auto load4 = [&](int j) {
+        const uint32_t e = 4u * (tid + (uint32_t)NT * j);
+        uint4 x = e < n ? __ldcg(reinterpret_cast<const uint4*>(row + e)) : make_uint4(ROW_ABSENT, ROW_ABSENT, ROW_ABSENT, ROW_ABSENT);
+        if (e + 3u >= n) {
+            if (e + 1u >= n) x.y = ROW_ABSENT;
+            if (e + 2u >= n) x.z = ROW_ABSENT;
+            x.w = ROW_ABSENT;
+        }
+        return x;
+    };
+    uint4 v[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) v[j] = load4(j);
+    if (tid < 16) st[tid] = tid == 1 ? 0xFFFFFFFFu : 0u;
+    for (int b = (int)tid; b <= ROW_BUCKETS; b += NT) hist[b] = 0;
+    __syncthreads();
+    // (What one pass over the row computed from the scores is not kept for the next: it would take as many registers as they do.)
+    auto fresh = [&]() {
+#pragma unroll
+        for (int j = 0; j < R; ++j) asm volatile("" : "+r"(v[j].x), "+r"(v[j].y), "+r"(v[j].z), "+r"(v[j].w));
+    };
+    fresh();
+    // Long rows: a bound from a sample, every fourth to sixteenth score all along the row (neighbours resemble one another).  Where `part` of the sample should lie above the k-th score, it is the lower edge of the bucket
+    // in which the sample's count from the top reaches 1.25 part + 3 sqrt(part) + 2.
+    constexpr int STEP = R >= 16 ? 4 : (R >= 8 ? 2 : 1);
+    const bool sampled = R > 2 || n > cap / 2u;
+    {
+        uint32_t mn = 0xFFFFFFFFu, mx = 0u;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const uint32_t x[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (sampled ? c == 0 && ((tid + j) & (STEP - 1)) == 0 : R <= 2) {
+                    const float s = __uint_as_float(x[c]);
+                    if (fabsf(s) < INFINITY) {
+                        mn = min(mn, score_key(s));
+                        mx = max(mx, score_key(s));
+                    }
+                }
+        }
+        mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+        mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+        if (lane == 0 && mx) {
+            atomicMin(&st[1], mn);
+            atomicMax(&st[2], mx);
+        }
+    }
+    __syncthreads();
+    // places of the buckets: the counts before them
+    auto scan = [&](int (&c)[PER]) {
+        int sum = 0;
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            c[j] = hist[tid * PER + j];
+            sum += c[j];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if ((int)lane >= o) incl += y;
+        }
+        if (lane == 31) st[16 + warp] = (uint32_t)incl;
+        __syncthreads();
+        int before = lane < warp ? (int)st[16 + lane] : 0;
+        return incl - sum + __reduce_add_sync(0xFFFFFFFFu, before);
+    };
+    const bool ranged = st[2] > st[1];
+    float low = key_score(ranged ? st[1] : score_key(0.0f)), bound = -INFINITY;
+    const float top = key_score(ranged ? st[2] : score_key(1.0f));
+    if (sampled && ranged) {
+        const float inv = (float)ROW_BUCKETS / (top - low);  // (a range that overflows puts all in one bucket)
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const float s = __uint_as_float(v[j].x);
+            if (((tid + j) & (STEP - 1)) == 0 && fabsf(s) < INFINITY) atomicAdd(&hist[min(max(__float2int_rz((top - s) * inv), 0), ROW_BUCKETS - 1)], 1);
+        }
+        __syncthreads();
+        const float part = (float)k * (0.25f / (float)STEP);
+        const int want = (int)(1.25f * part + 3.0f * sqrtf(part)) + 2;
+        int c[PER], at = scan(c);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            if (at < want && at + c[j] >= want) st[3] = tid * PER + j + 1;
+            at += c[j];
+            hist[tid * PER + j] = 0;
+        }
+        __syncthreads();
+        if (st[3] && st[3] < (uint32_t)ROW_BUCKETS) bound = top - (float)st[3] / inv;  // (zero: the sample holds too few, all are candidates)
+    }
+    // what reaches the bound: the thread's own candidates
+    uint32_t mine;
+    for (;;) {
+        fresh();
+        mine = 0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const uint32_t x[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (__uint_as_float(x[c]) >= bound) {
+                    if (OWN == 4 * R || mine < (uint32_t)OWN) own[mine * NT] = (uint64_t)x[c] << 32 | (uint32_t)(4 * NT * j + c);
+                    ++mine;
+                }
+            asm volatile("" : "+r"(mine) : : "memory");  // (four at a time: all comparisons first would take a register each)
+        }
+        if (bound <= 0.0f) {  // a NaN counts as -0, as score_kernel's keys have it
+#pragma unroll
+            for (int j = 0; j < R; ++j) {
+                const uint32_t x[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if ((x[c] & 0x7FFFFFFFu) > 0x7F800000u && x[c] != ROW_ABSENT) {
+                        if (OWN == 4 * R || mine < (uint32_t)OWN) own[mine * NT] = (uint64_t)0x80000000u << 32 | (uint32_t)(4 * NT * j + c);
+                        ++mine;
+                    }
+                asm volatile("" : "+r"(mine) : : "memory");
+            }
+        }
+        const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, mine);
+        if (lane == 0 && sum) atomicAdd(&st[0], sum);
+        if (OWN < 4 * R && mine > (uint32_t)OWN) st[4] = 1u;
+        __syncthreads();
+        if (st[0] >= k || bound == -INFINITY) break;
+        bound = -INFINITY;  // (the sample misled)
+        __syncthreads();
+        if (tid == 0) st[0] = st[4] = 0u;
+        __syncthreads();
+    }
+    const uint32_t got = st[0], m = min(got, k);
+    uint32_t* const out_index = a.out_index + (size_t)Q * k;
+    float* const out_score = a.out_score + (size_t)Q * k;
+    if (got <= cap && (OWN == 4 * R || !st[4])) {
+        if (bound > low) low = bound;
+        const float inv = (float)ROW_BUCKETS / (top - low);
+        const bool apart = inv > 0.0f && inv < INFINITY;
+        auto bucket = [&](uint32_t bits) {
+            return apart ? min(max(__float2int_rz((top - __uint_as_float(bits)) * inv), 0), ROW_BUCKETS - 1) : 0;
+        };
+        for (uint32_t h = 0; h < mine; ++h) {
+            const uint64_t e = own[h * NT];
+            const int b = bucket((uint32_t)(e >> 32));
+            const int r = atomicAdd(&hist[b], 1);  // (any order inside the bucket)
+            own[h * NT] = e & 0xFFFFFFFF0000FFFFull | (uint64_t)r << 16;
+        }
+        __syncthreads();
+        int c[PER], at = scan(c);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            hist[tid * PER + j] = at;
+            at += c[j];
+        }
+        if (tid == NT - 1) hist[ROW_BUCKETS] = at;
+        __syncthreads();
+        for (uint32_t h = 0; h < mine; ++h) {
+            const uint64_t e = own[h * NT];
+            const uint32_t bits = (uint32_t)(e >> 32);
+            buf[hist[bucket(bits)] + (int)((uint32_t)e >> 16)] = make_comp(__uint_as_float(bits), info.index_base + 4u * tid + ((uint32_t)e & 0xFFFFu));
+        }
+        __syncthreads();
+        for (uint32_t i = tid; i < got; i += NT) {
+            const uint64_t key = buf[i];
+            const int b = bucket(__float_as_uint(key_score((uint32_t)(key >> 32))));
+            const int s0 = hist[b], e0 = hist[b + 1];
+            uint32_t r = (uint32_t)s0;
+            for (int x = s0; x < e0; ++x) r += buf[x] > key;
+            if (r < m) {
+                out_index[r] = 0xFFFFFFFFu - (uint32_t)key;
+                out_score[r] = key_score((uint32_t)(key >> 32));
+            }
+        }
+        for (uint32_t r = m + tid; r < k; r += NT) {
+            out_index[r] = 0xFFFFFFFFu;
+            out_score[r] = -INFINITY;
+        }
+    } else {
+        // Too many candidates (many equal scores, or outliers far from the rest): a radix selection of the k-th largest score word, what
+        // lies above it, and of the scores equal to it those with the lowest indices.  (At least k are there.  The row is read again: held on to for
+        // this, it would cost every launch registers.)
+        auto word = [](uint32_t bits) { return (bits & 0x7FFFFFFFu) > 0x7F800000u ? 0x7FFFFFFFu : score_key(__uint_as_float(bits)); };
+        uint32_t prefix = 0, need = k;
+        for (int shift = 24;; shift -= 8) {
+            __syncthreads();
+            for (int b = (int)tid; b < 256; b += NT) hist[b] = 0;
+            __syncthreads();
+#pragma unroll 1
+            for (int j = 0; j < R; ++j) {
+                const uint4 w = load4(j);
+                const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const uint32_t h = word(x[c]);
+                    const bool in = x[c] != ROW_ABSENT && (shift == 24 || (h >> (shift + 8)) == prefix);
+                    const uint32_t b = in ? (h >> shift) & 255u : 256u;
+                    // (equal scores meet in one bucket: one atomic per warp and bucket)
+                    const uint32_t same = __match_any_sync(0xFFFFFFFFu, b);
+                    if (in && (uint32_t)__ffs(same) - 1u == lane) atomicAdd(&hist[b], __popc(same));
+                }
+            }
+            __syncthreads();
+            if (tid < 32) {  // lane l owns bins 255-8l .. 248-8l (descending)
+                int c[8], tot = 0;
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    c[j] = hist[255 - 8 * (int)tid - j];
+                    tot += c[j];
+                }
+                int incl = tot;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                    if ((int)lane >= o) incl += y;
+                }
+                const unsigned ok = __ballot_sync(0xFFFFFFFFu, incl >= (int)need);
+                if ((int)tid == __ffs(ok) - 1) {
+                    int run = incl - tot;
+#pragma unroll
+                    for (int j = 0; j < 8; ++j) {
+                        if (run + c[j] >= (int)need) {
+                            st[8] = 255u - 8u * tid - (uint32_t)j;
+                            st[9] = (uint32_t)run;
+                            break;
+                        }
+                        run += c[j];
+                    }
+                }
+            }
+            __syncthreads();
+            prefix = (prefix << 8) | st[8];
+            need -= st[9];
+            if (shift == 0) break;
+        }
+        __syncthreads();
+        if (tid == 0) st[5] = 0u;
+        for (uint32_t i = tid; i < a.kp2; i += NT) buf[i] = 0ull;
+        __syncthreads();
+#pragma unroll 1
+        for (int j = 0; j < R; ++j) {  // (4 NT scores at a time in index order, so that the lowest indices among the equal ones come first)
+            const uint4 w = load4(j);
+            const uint32_t x[4] = {w.x, w.y, w.z, w.w}, e = info.index_base + 4u * (tid + (uint32_t)NT * j);
+            uint32_t eq = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (x[c] == ROW_ABSENT) continue;
+                const uint32_t h = word(x[c]);
+                if (h > prefix) buf[atomicAdd(&st[5], 1u)] = ((uint64_t)word(x[c]) << 32 | (0xFFFFFFFFu - (e + c)));
+                else if (h == prefix) ++eq;
+            }
+            uint32_t incl = eq;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            if (lane == 31) st[16 + warp] = incl;
+            __syncthreads();
+            uint32_t rank = incl - eq, all = 0;
+            for (uint32_t w2 = 0; w2 < NT / 32; ++w2) {
+                if (w2 < warp) rank += st[16 + w2];
+                all += st[16 + w2];
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (x[c] != ROW_ABSENT && word(x[c]) == prefix) {
+                    if (rank < need) buf[atomicAdd(&st[5], 1u)] = ((uint64_t)word(x[c]) << 32 | (0xFFFFFFFFu - (e + c)));
+                    ++rank;
+                }
+            need -= min(need, all);
+            __syncthreads();
+        }
+        for (uint32_t size = 2; size <= a.kp2; size <<= 1)
+            for (uint32_t stride = size >> 1; stride; stride >>= 1) {
+                for (uint32_t i = tid; i < a.kp2 / 2; i += NT) {
+                    const uint32_t p = 2 * i - (i & (stride - 1)), q = p + stride;
+                    const uint64_t x = buf[p], y = buf[q];
+                    if ((x < y) == ((p & size) == 0)) {
+                        buf[p] = y;
+                        buf[q] = x;
+                    }
+                }
+                __syncthreads();
+            }
+        emit_sorted(buf, k, k, Q, a.out_index, a.out_score, nullptr);
+    }
+    if (tid == 0) {
+        if (a.out_count) a.out_count[Q] = m;
+        a.stats[2 * Q] = got;
+        a.stats[2 * Q + 1] = a.flag[Q];
+        a.flag[Q] = a.flag[gridDim.x + Q] = 0u;
+    }
+}
+
+}  // namespace
+}  // namespace slha

@@ -336,7 +336,7 @@ __device__ __forceinline__ uint32_t first_tile_flags(const ScoreArgs& a, const W
 // whole streams (see the planner).  A tile of another codec than KIND's, or a query outside the fp16 split, hands the
 // item's query rows to the generic kernel.
 template <int KIND, bool IL, bool DENSE, bool KINDS>
-__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, bool nf4_too = false) {
+__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, bool nf4_too = false, Undone* undone = nullptr) {
     constexpr int NWG = ST_WG, NWARPS = 4 * NWG, NACC = st_accs(KIND);
     constexpr uint32_t STRIDE = ST_TMEM, DCOL = st_d_col(KIND);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wg = warp >> 2, wq = warp & 3;
@@ -408,6 +408,11 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             uint32_t f = 0;
             for (int q = 0; q < nq; ++q) f |= a.only_flagged[it.query_begin + q];
             if (!f) continue;  // (the same in the whole CTA)
+            if (f & 2u) {
+                if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
+                if (tid == 0) undone_add(*undone, item_id);
+                continue;
+            }
         }
         const unsigned char* tbase = a.tiles + it.tile_begin * TILE_BYTES + (size_t)wq * (ST_WT * TILE_BYTES) + lane * 16;
         uint32_t iss_no = 0, slot_next = 0;
@@ -743,7 +748,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                         if (q < nq) {
                             const uint32_t Q = it.query_begin + (uint32_t)q;
                             const size_t row0 = a.row_offset ? (size_t)a.row_offset[Q] : (size_t)Q * a.score_stride;
-                            a.scores[row0 + it.index_base + t0] = live ? c[q] : -INFINITY;
+                            a.scores[row0 + it.index_base + t0] = live ? c[q] : __uint_as_float(a.cold_bits);
                         }
                 }
                 continue;
@@ -769,8 +774,11 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                 if (cur[q] + (uint32_t)lane < end[q]) a.gbuf[(size_t)(it.query_begin + (uint32_t)q) * a.gcap + cur[q] + (uint32_t)lane] = 0ull;
         }
         __syncthreads();
-        // rows this CTA could not score on the tensor cores go to the generic kernel as a whole
-        if (*reinterpret_cast<volatile uint32_t*>(bail) && tid < nq) a.gflag[it.query_begin + tid] = 1u;
+        if (*reinterpret_cast<volatile uint32_t*>(bail)) {  // (the same in the whole CTA)
+            // rows this CTA could not score on the tensor cores go to the generic kernel as a whole; of dense calls the item, at the CTA's end
+            if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
+            if (DENSE && tid == 0) undone_add(*undone, item_id);
+        }
         __syncthreads();
         if (tid == 0) *bail = 0u;  // (ordered before the next item's writers by the barrier at its start)
     }
@@ -798,13 +806,15 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) 
 // Dense scores.  Every work item is decoded as what its first tile says (read here: a host that looked would wait for the
 // stream); a tile of another kind inside the item hands its rows over as everywhere.  An arena known to hold NF4 beside INT4
 // tiles is decoded as NF4 throughout.
-__global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a) {
+__global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid_constant__ ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
+    __shared__ Undone undone;
     dep_launch();
     dep_wait();
     if (a.refused && *a.refused) return;
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
+    if (threadIdx.x == 0) undone.n = 0u;
     if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
         uint32_t f = 0;
         for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS)
@@ -816,16 +826,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(ScoreArgs a)
     TileCta cta = tile_open<true>(smem_raw);
     for (;;) {
         switch (item_kind(flags, nf4_too)) {
-            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, nf4_too); break;
-            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, nf4_too); break;
-            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, nf4_too); break;
-            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, nf4_too); break;
-            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, nf4_too); break;
+            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
+            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
+            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
+            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
+            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
         }
         if (i >= item_end) break;
         flags = first_tile_flags(a, a.stream_items[i]);
     }
     tile_close(cta);
+    finish_undone(a, a.stream_items, undone, smem_raw);
 }
 
 }  // namespace

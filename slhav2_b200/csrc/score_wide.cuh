@@ -203,7 +203,7 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             }
         }
         qs_w[tid] = (tid >> 3) < nq ? a.q_sign[(size_t)(it.query_begin + (tid >> 3)) * 8 + (tid & 7)] : 0u;
-        if (DENSE && tid < WIDE_NQ) roff[tid] = tid < nq ? a.row_offset[it.query_begin + tid] : 0ull;
+        if (DENSE && tid < WIDE_NQ) roff[tid] = tid >= nq ? 0ull : (a.row_offset ? a.row_offset[it.query_begin + tid] : (it.query_begin + tid) * a.score_stride);
         if (!DENSE && tid < WIDE_NQ) {
             const bool have = tid < nq;
             const unsigned long long pv = have ? *reinterpret_cast<volatile unsigned long long*>(a.gpivot + it.query_begin + tid) : ~0ull;
@@ -500,15 +500,17 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         if (warp == 0) WPROBE_OUT(0, 12);
         if (stop && tid == 0) ctl[5] = 1u;
         __syncthreads();
-        // rows this CTA could not score (another codec, a query outside the fp16 split, a wait that ran out) go to the generic kernel
-        if ((*reinterpret_cast<volatile uint32_t*>(ctl + 6) || stop) && tid < nq) a.gflag[it.query_begin + tid] = 1u;
+        // rows this CTA could not score (another codec, a query outside the fp16 split, a wait that ran out) go to the generic kernel, of a dense call to
+        // the four-row kernel
+        if ((*reinterpret_cast<volatile uint32_t*>(ctl + 6) || stop) && tid < nq) (DENSE ? a.handoff : a.gflag)[it.query_begin + tid] = DENSE ? a.handoff_as : 1u;
         __syncthreads();
         if (tid == 0) ctl[6] = 0u;  // (ordered before the next item's writers by the barrier at its start)
     }
     if (stop) {
-        // a wait ran out (the same in all threads): the barrier's phases are no longer known, the remaining items go to the generic kernel too
+        // a wait ran out (the same in all threads): the barrier's phases are no longer known, the remaining items go to the generic kernel too (of a
+        // dense call to the four-row kernel)
         for (uint32_t item_id = a.cta_begin[blockIdx.x]; item_id < item_end; ++item_id)
-            for (uint32_t q = tid; q < a.items[item_id].n_queries; q += WIDE_THREADS) a.gflag[a.items[item_id].query_begin + q] = 1u;
+            for (uint32_t q = tid; q < a.items[item_id].n_queries; q += WIDE_THREADS) (DENSE ? a.handoff : a.gflag)[a.items[item_id].query_begin + q] = DENSE ? a.handoff_as : 1u;
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -537,7 +539,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_dense_kernel(Score
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     int kind = item_kind(first_tile_flags(a, a.items[i]), false);
     while (kind == 0) {
-        if (threadIdx.x < a.items[i].n_queries) a.gflag[a.items[i].query_begin + threadIdx.x] = 1u;
+        if (threadIdx.x < a.items[i].n_queries) a.handoff[a.items[i].query_begin + threadIdx.x] = 1u;
         if (++i == item_end) return;
         kind = item_kind(first_tile_flags(a, a.items[i]), false);
     }

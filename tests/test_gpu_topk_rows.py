@@ -1,0 +1,99 @@
+"""Top-k of calls whose rows are scored as a whole (topk_rows_kernel): rows at the edges of what a thread, a sample and the candidates' slots hold, scores that a
+sample does not tell apart, absent and non-finite ones, against an exact selection of the same scores."""
+import numpy as np
+import pytest
+
+import slhav2_b200 as S
+from tests import helpers as H
+
+pytestmark = pytest.mark.gpu
+F = np.float32
+TAKEN = S.last_score_stats  # (rows of a whole-row plan are reported as sets of sixteen tiles with as many slots as the row has, in multiples of 32)
+
+
+def _check(tiles, rows, nq, k, qc, qs, state_cold=None):
+    """The dense call scores the same rows with the same kernels: the winners are its k largest, ties towards the lower index, bit for bit."""
+    dt, seg = S.to_device(tiles), S.make_segments(rows)
+    longest = max(r[1] for r in rows)
+    idx, sc, cnt = S.score_topk(dt, seg, qc, qs, nq, k)
+    assert TAKEN()["buffer_slots"] == (longest + 31) // 32 * 32
+    flat = S.make_segments([(t, n, q, m, 0) for t, n, q, m, _ in rows])
+    dense = S.score_segments(dt, flat, qc, qs, nq, np.zeros((nq, longest), F), np.arange(nq, dtype=np.uint64) * longest, longest, fill=0.0)
+    for t, n, q0, m, base in rows:
+        for q in range(q0, q0 + m):
+            want = dense[q, :n]
+            key = np.where(np.isnan(want), F(-0.0), want).view(np.int32).astype(np.int64)
+            key = np.where(key < 0, -2**31 - 1 - key, key)  # total order: -0 below 0
+            order = np.lexsort((np.arange(n), -key))[:k]
+            have = min(n, k)
+            assert cnt[q] == have and np.all(idx[q, have:] == 0xFFFFFFFF) and np.all(sc[q, have:] == -np.inf)
+            assert np.array_equal(idx[q, :have], order + base)
+            assert np.array_equal(sc[q, :have].view(np.uint32), np.where(np.isnan(want), F(-0.0), want)[order].view(np.uint32))
+    return idx, sc
+
+
+@pytest.mark.parametrize("n", [1, 3, 127, 1025, 2047, 2048, 2049, 4095, 4097, 8191, 8193, 16383, 16385, 20011, 32767, 32768])
+@pytest.mark.parametrize("k", [1, 17, 256, 1000, 4096])
+def test_rows_of_every_length(n, k):
+    # around the scores a thread holds (1024, 2048, .. 16 384 a block's round) and the candidates' slots (from n = cap / 2 on a sample gives the bound)
+    codec = [0, 3, 4, 5][n % 4]
+    base = H.random_tiles(2000, codec, seed=n, warm_every=9, nocorr_every=5)
+    tiles = base[np.random.default_rng(n + k).integers(0, len(base), 2 * n)]  # (with equal scores)
+    qc, qs = H.random_queries(5, 900 + k)
+    _check(tiles, [(0, n, 0, 3, 5), (n, n, 3, 2, 1000)], 5, k, qc, qs)
+
+
+@pytest.mark.parametrize("n", [900, 9000, 30000])
+@pytest.mark.parametrize("shape", ["equal", "few values", "outlier", "rising", "last", "zero query", "infinite", "huge"])
+def test_scores_that_a_sample_does_not_tell_apart(n, shape):
+    rng = np.random.default_rng(7)
+    tiles = np.tile(H.random_tiles(1000, 1, seed=31), n // 1000 + 1)[:n].copy()
+    tiles["dynamic_lambda"] = 0
+    qc, qs = H.random_queries(2, 32)
+    if shape == "equal":
+        tiles[:] = tiles[0]
+    elif shape == "few values":
+        tiles = tiles[rng.integers(0, 3, n)]
+    elif shape == "outlier":
+        tiles["scale"][n // 3] *= F(1e6)
+    elif shape == "rising":
+        tiles["scale"] *= np.linspace(0.01, 3.0, n).astype(F)
+    elif shape == "last":
+        tiles["scale"][:-300] *= F(1e-3)
+    elif shape == "zero query":
+        qc[:] = 0
+    elif shape == "infinite":
+        tiles["scale"][::7] = np.inf
+        tiles["scale"][3::11] = np.nan
+    elif shape == "huge":
+        tiles["scale"][:] = rng.choice(np.array([1e37, 1.0, 1e-30], F), n)
+    for k in (1, 200, 2000):
+        _check(tiles, [(0, n, 0, 2, 0)], 2, k, qc, qs)
+
+
+@pytest.mark.parametrize("nq,codec", [(16, 1), (40, 2), (64, 4), (70, 5)])
+def test_rows_of_many_queries(nq, codec):
+    # the 64-row kernel's scores, of NF4 tiles the four-row kernel's; a segment without rows and one without tiles
+    n = 2500
+    tiles = H.random_tiles(2 * n, codec, seed=60 + nq, warm_every=8, nocorr_every=3)
+    qc, qs = H.random_queries(2 * nq + 20, 61)
+    _check(tiles, [(0, n, 0, nq, 3), (n, n - 77, nq, nq, 0), (5, 0, 2 * nq, 20, 9), (9, 400, 0, 0, 0)], 2 * nq + 20, 100, qc, qs)
+
+
+def test_cold_slots_are_no_candidates():
+    n, k = 3000, 500
+    tiles = H.random_tiles(n, 3, seed=70)
+    pool = S.TilePool(n, 2**40)
+    pool.insert(tiles)
+    rng = np.random.default_rng(71)
+    gone = rng.permutation(n)[:2700]
+    for s in gone:
+        pool.evict(int(s))
+    qc, qs = H.random_queries(4, 72)
+    idx, sc, cnt = pool.score_topk(qc, qs, 4, k)
+    assert np.all(cnt == 300) and np.all(idx[:, 300:] == 0xFFFFFFFF)
+    want = S.score_tiles(S.to_device(tiles), n, qc, qs, 4)
+    left = np.setdiff1d(np.arange(n), gone)
+    for j in range(4):
+        order = left[np.lexsort((left, -want[j, left]))]
+        assert np.array_equal(np.sort(idx[j, :300]), left) and np.all(np.abs(sc[j, :300] - want[j, order]) <= 1e-3)
