@@ -525,7 +525,7 @@ __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem&
 // What is left at a CTA's end (all of its shared memory is free).
 __device__ __noinline__ void finish_undone(const ScoreArgs& a, const WorkItem* items, const Undone& u, unsigned char* smem) {
     __syncthreads();
-    const uint32_t m = u.n, first = a.cta_begin[blockIdx.x], end = a.cta_begin[blockIdx.x + 1];
+    const uint32_t m = u.n, first = a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x, end = a.cta_begin ? a.cta_begin[blockIdx.x + 1] : first + 1;
     for (uint32_t j = 0; j < (m > 31u ? end - first : m); ++j) {
         const WorkItem it = items[m > 31u ? first + j : u.item[j]];
         for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);

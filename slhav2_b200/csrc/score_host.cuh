@@ -349,7 +349,7 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     p->d_row_flags = (uint32_t*)p->b_gpivot.p;
     SLHA_CUDA(cudaMemsetAsync(p->d_row_flags, 0, 4 * nq * 4, c->stream));
     p->d_items = reinterpret_cast<WorkItem*>(dev + o_n);
-    p->d_cta_begin = reinterpret_cast<uint32_t*>(dev + o_nc);
+    p->d_cta_begin = narrow.items.size() + 1 == narrow.cta.size() ? nullptr : reinterpret_cast<uint32_t*>(dev + o_nc);
     p->d_wide_items = reinterpret_cast<WorkItem*>(dev + o_w);
     p->d_wide_cta = reinterpret_cast<uint32_t*>(dev + o_wc);
     p->d_rows = reinterpret_cast<RowInfo*>(dev + o_r);
@@ -803,7 +803,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.state = state;
         a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_items);
         a.n_items = (uint32_t)cuts.items.size();
-        a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_cta);
+        a.cta_begin = cuts.items.size() + 1 == cuts.cta.size() ? nullptr : reinterpret_cast<const uint32_t*>(dev + o_cta);
         a.q_coarse = q_coarse;
         a.q_sign = reinterpret_cast<const uint32_t*>(q_sign);
         a.scores = scores;
@@ -960,7 +960,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     }
     a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_narrow);
     a.n_items = (uint32_t)narrow.items.size();
-    a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_ncta);
+    a.cta_begin = narrow.items.size() + 1 == narrow.cta.size() ? nullptr : reinterpret_cast<const uint32_t*>(dev + o_ncta);
     if (!g_force_generic) return launch_dense(c, a, (uint32_t)narrow.cta.size() - 1, wide);
     a.items = reinterpret_cast<const WorkItem*>(dev + o_gen);
     const int threads = 128, nwarps = threads / 32;

@@ -6,10 +6,12 @@
 // the queries (scaled to one size, fp16 hi + lo columns, 22 bits or more) and the thread reads its finished coarse scores back.  Scale, lambda, flags
 // and scale bytes are each read by one thread, where the fragments of warp-level MMAs need them in four lanes each.
 //
-// Bound: the chain of a block (decode, TMEM store, eight or nine MMAs, read-back, filter), about 5000 cycles with four warpgroups in
-// flight.  MIX3 top-k of 32 ragged segments (485 k tiles x 4 queries): 367 -> 72 us a call; dense MIX3 scores of 8 x 4096 tiles x 4
-// rows: 278 -> 37 us a call (8.7 us of kernel), both from the generic kernel.  Top-k of the codecs that score_stream_kernel
-// decodes stays there: with this kernel a call took 301 us against 292 us on 8.4 M MX-INT4 tiles and 573 us against 462 us on as many
+// Bound: the chain of a block (decode, TMEM store, eight or nine MMAs, read-back, filter or finish), 4000 cycles (MIX3 5200, NF4 6700) with four warpgroups in
+// flight, of which the instructions take 1700.  Dense scores of 8 x 131 072 mixed tiles, 4 rows: 4820 cycles a round -> 4020, one row 4250 -> 3330, an item's set-up 4900 ->
+// 3000, by the sums in pairs (f32x2), full adders in front of POPC, row addresses and slot states read ahead, the queries asked for before the tiles.
+// MIX3 top-k of 32 ragged segments (485 k tiles x 4 queries): 367 -> 72 us a call streamed (dense scores and a selection: 42); dense MIX3 scores of 8 x 4096
+// tiles x 4 rows: 278 -> 17 us a call (6 of kernel).  Top-k of the codecs that score_stream_kernel
+// decodes, over long rows, stays there: with this kernel a call took 301 us against 292 us on 8.4 M MX-INT4 tiles and 573 us against 462 us on as many
 // NF4 tiles.
 #pragma once
 
@@ -23,7 +25,7 @@ constexpr int ST_SLOT = ST_WT * ST_ROW;
 constexpr int ST_DEPTH = 2;                            // ring slots per warp
 constexpr uint32_t ST_CHUNK = 32;                      // slots a warp reserves at a time in a row's candidate buffer
 constexpr int ST_B_BYTES = 8192;                       // B operand: up to 3 slabs of 2 KB (64 K slots of 16 rows)
-constexpr int ST_TAIL_BYTES = 128 + 16 + 16 + 32 + 32 + 64 + 32;
+constexpr int ST_TAIL_BYTES = 128 + 16 + 16 + 32 + 32 + 64 + 32 + 256;
 // KIND 0: NF4 (and INT4) tiles, 1: mixed 8/4, 2: TQ3, 3: INT4 / MX-INT4, 4: MIX3
 constexpr int ST_WG = 4, ST_THREADS = 128 * ST_WG;     // warpgroups per CTA
 constexpr uint32_t ST_TMEM = 128;                      // TMEM columns of a warpgroup: A in the first 64 (72 for the 3-bit kinds), accumulators behind it
@@ -260,6 +262,31 @@ __device__ __forceinline__ void two_sum(float& s, float x, float& e) {
     e = __fadd_rn(e, __fadd_rn(__fsub_rn(s, __fsub_rn(t, b)), __fsub_rn(x, b)));
     s = t;
 }
+// the same for pairs (a subtraction is a fused step with -1: exact but for the one rounding)
+__device__ __forceinline__ void two_sum2(uint64_t& s, uint64_t x, uint64_t& e) {
+    constexpr uint64_t M1 = 0xBF800000BF800000ull;
+    const uint64_t t = f2_add(s, x), b = f2_fma(s, M1, t);
+    e = f2_add(e, f2_add(f2_fma(f2_fma(b, M1, t), M1, s), f2_fma(b, M1, x)));
+    s = t;
+}
+__device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;\n" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t u2_pack(uint32_t lo, uint32_t hi) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};\n" : "=l"(r) : "r"(lo), "r"(hi));
+    return r;
+}
+// Set bits of eight words: four full adders leave four words for POPC, which runs at a quarter of the logic's rate.
+__device__ __forceinline__ uint32_t popc8_words(const uint32_t (&x)[8]) {
+    const uint32_t s1 = x[0] ^ x[1] ^ x[2], c1 = (x[0] & x[1]) | (x[2] & (x[0] | x[1]));
+    const uint32_t s2 = x[3] ^ x[4] ^ x[5], c2 = (x[3] & x[4]) | (x[5] & (x[3] | x[4]));
+    const uint32_t s3 = x[6] ^ x[7] ^ s1, c3 = (x[6] & x[7]) | (s1 & (x[6] | x[7]));
+    const uint32_t t = c1 ^ c2 ^ c3, u = (c1 & c2) | (c3 & (c1 | c2));
+    return (uint32_t)__popc(s2) + (uint32_t)__popc(s3) + 2u * (uint32_t)__popc(t) + 4u * (uint32_t)__popc(u);
+}
 
 // a codec a launch of this kind does not decode
 __device__ __forceinline__ bool st_alien(int kind, uint32_t flags) {
@@ -330,13 +357,14 @@ __device__ __forceinline__ uint32_t first_tile_flags(const ScoreArgs& a, const W
     return *reinterpret_cast<const uint16_t*>(a.tiles + it.tile_begin * TILE_BYTES + 118);
 }
 
-// The work items from item_id on (KINDS: up to the first whose first tile is of another kind); the next item.
+// The work items from item_id on (KINDS: up to the first whose first tile is of another kind); the next item.  it, flags0: item_id's item and its first
+// tile's flags, which the caller has read; the next item's when this returns.
 // DENSE: every score is written to a.scores (row q at a.row_offset[q] or q * a.score_stride, tile i of the item at
 // index_base + i; -inf for COLD slots) and nothing is filtered or appended.  IL: the work items are interleaved shares of
 // whole streams (see the planner).  A tile of another codec than KIND's, or a query outside the fp16 split, hands the
 // item's query rows to the generic kernel.
 template <int KIND, bool IL, bool DENSE, bool KINDS>
-__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, bool nf4_too = false, Undone* undone = nullptr) {
+__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, WorkItem& it, uint32_t& flags0, bool nf4_too = false, Undone* undone = nullptr) {
     constexpr int NWG = ST_WG, NWARPS = 4 * NWG, NACC = st_accs(KIND);
     constexpr uint32_t STRIDE = ST_TMEM, DCOL = st_d_col(KIND);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wg = warp >> 2, wq = warp & 3;
@@ -353,10 +381,11 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
     float2* rng = reinterpret_cast<float2*>(thr + 4);            // [4] (smin, inv), inv 0 = none yet
     float2* rmap = rng + 4;                                      // [4] (-smin inv, inv)
     uint32_t* flagw = reinterpret_cast<uint32_t*>(rmap + 4);     // mbarriers of the warpgroups (32 bytes), TMEM base, bail
-    const uint32_t bar_s = tail_s + 224u;
+    const uint32_t bar_s = tail_s + 224u, qsw_s = tail_s;
     uint32_t* bail = flagw + 9;
     uint32_t* qmax = flagw + 16;                                 // [4] bits of the row's largest element
     float* qinv = reinterpret_cast<float*>(qmax + 4);            // [4] inverse of the row's scale times the unit of A
+    float* qsum = qinv + 4;                                      // [4][16] sums of eight elements (3-bit kinds)
 
     if (KIND == 0 && !cta.table) {  // NF4 codebook pairs per byte, 16 bank-aligned replicas (read by nobody yet)
         cta.table = true;
@@ -378,16 +407,18 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
     uint32_t phase = cta.phase;
     bool failed = cta.failed;
 
-    for (; item_id < item_end; ++item_id) {
-        const WorkItem it = a.stream_items[item_id];
-        if (KINDS && item_kind(first_tile_flags(a, it), nf4_too) != KIND) break;  // (the same in the whole CTA)
+    auto next_item = [&]() {  // false at the end, or at an item of another kind (the same in the whole CTA)
+        if (++item_id >= item_end) return false;
+        it = a.stream_items[item_id];
+        if (KINDS) flags0 = first_tile_flags(a, it);
+        return !KINDS || item_kind(flags0, nf4_too) == KIND;
+    };
+    do {
         bool gave_up = false;  // this warpgroup met a tile it cannot decode, or a wait of it ran out (the same in the whole warpgroup)
         const int nq = (int)it.n_queries;
         // interleaved: this CTA is number il_c of the il_n CTAs that share the stream [tile_begin, + n_tiles); round r of
         // the stream's static deal belongs to CTA r mod il_n.  Otherwise the item is this CTA's own range.
         const uint32_t il_n = IL ? ((it.pad >> 8) & 0x7FFFFFu) : 1u, il_c = IL ? it.list_begin : 0u;
-        if (tid < 4) qmax[tid] = 0u;
-        __syncthreads();  // previous item fully retired (and the table is visible)
         const uint8_t* sbase = a.state ? a.state + it.tile_begin : nullptr;
         const uint32_t n = it.n_tiles;
         const uint32_t n_blocks = (n + ST_M - 1) / ST_M;
@@ -443,71 +474,82 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             cp_async_commit();
             slot_next = slot_next == (ST_DEPTH - 1) * ST_SLOT ? 0u : slot_next + ST_SLOT;
         };
+        // B: 16-byte chunks of eight k slots, K-major, 128-byte swizzle (chunk i of row r at chunk i ^ (r & 7) of its line), one a thread.
+        // Row n = 4 part + q (hi / lo of query q), rows 8..15 zero; k slot 8 i + j holds dim 8 i + {0,4,1,5,2,6,3,7}[j] (see
+        // nib_word), NF4: dim 8 i + j.  A row's scale comes from the elements its chunks hold (the mixed layouts drop the last eight).  What the item
+        // brings from memory is asked for before the first barrier, and before the tiles: behind 64 KB of them it took 1100 to 2500 cycles.
+        static_assert(ST_THREADS >= 16 * 18, "a thread per chunk");
+        constexpr bool HEAD = KIND == 1 || KIND == 4, EXTRA = KIND == 2 || KIND == 4;
+        const int br = tid / 18, bi = tid % 18, bq = br & 3;
+        // (one load for all kinds of chunk and no arithmetic on what comes: a branch would wait for its own loads)
+        const bool chunk_of_row = tid < 8 * 18 && bq < nq && bi < 16, head = HEAD && bi < 2;
+        float4 qx = make_float4(0.0f, 0.0f, 0.0f, 0.0f), qy = qx;
+        {
+            const float* q = a.q_coarse + (size_t)(it.query_begin + bq) * D_C + (head ? 4 * bi : 8 * (HEAD ? bi - 1 : bi));
+            const int up = head ? 0 : 4;
+            if (reinterpret_cast<uintptr_t>(a.q_coarse) & 15u) {  // (the same for all rows)
+                if (chunk_of_row) {
+                    qx = make_float4(q[0], q[1], q[2], q[3]);
+                    qy = make_float4(q[up], q[up + 1], q[up + 2], q[up + 3]);
+                }
+            } else if (chunk_of_row) {
+                qx = *reinterpret_cast<const float4*>(q);
+                qy = *reinterpret_cast<const float4*>(q + up);
+            }
+        }
+        uint32_t sign_word = 0u;
+        if (warp == 8 && (lane >> 3) < nq) sign_word = a.q_sign[(size_t)(it.query_begin + (lane >> 3)) * 8 + (lane & 7)];
+        bool row_warm = true;
+        unsigned long long pv = 0ull, pr = 0ull;
+        if (!DENSE && tid < nq) {
+            pv = *reinterpret_cast<volatile unsigned long long*>(a.gpivot + it.query_begin + tid);
+            pr = *reinterpret_cast<volatile unsigned long long*>(a.grange + it.query_begin + tid);
+        }
+        float* rowp[4];  // dense: where the item's rows start
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t Q = it.query_begin + (uint32_t)min(q, nq - 1);
+            rowp[q] = !DENSE ? nullptr : a.scores + (a.row_offset ? (size_t)a.row_offset[Q] : (size_t)Q * a.score_stride) + it.index_base;
+        }
 #pragma unroll
         for (int i = 0; i < ST_DEPTH - 1; ++i) issue();
-        bool row_warm = true;
+        if (warp == 9 && lane < 4) qmax[lane] = 0u;  // (read last in the set-up of the item before)
+        __syncthreads();  // previous item fully retired (and the table is visible)
         if (!DENSE && tid < 4) {
             // start from the threshold other CTAs have already proven for the row, and from the
             // row's bucket mapping if one has been published
-            const bool have = tid < nq;
-            const unsigned long long pv = have ? *reinterpret_cast<volatile unsigned long long*>(a.gpivot + it.query_begin + tid) : 0ull;
             pvh[tid] = (uint32_t)(pv >> 32);
             thr[tid] = thr_float((uint32_t)(pv >> 32));
-            row_warm = !have || (uint32_t)(pv >> 32) != 0u;
-            const unsigned long long pr = have ? *reinterpret_cast<volatile unsigned long long*>(a.grange + it.query_begin + tid) : 0ull;
+            row_warm = tid >= nq || (uint32_t)(pv >> 32) != 0u;
             rng[tid] = make_float2(__uint_as_float((uint32_t)pr), __uint_as_float((uint32_t)(pr >> 32)));
             rmap[tid] = make_float2(-rng[tid].x * rng[tid].y, rng[tid].y);
         }
-        if (warp == 1) {  // sign words of the item's (up to four) queries
-            const int qi = lane >> 3;
-            qs_w[lane] = qi < nq ? a.q_sign[(size_t)(it.query_begin + qi) * 8 + (lane & 7)] : 0u;
-        }
-        // B: 16-byte chunks of eight k slots, K-major, 128-byte swizzle (chunk i of row r at chunk i ^ (r & 7) of its line), one a thread.
-        // Row n = 2 q + part (hi / lo of query q), rows 8..15 zero; k slot 8 i + j holds dim 8 i + {0,4,1,5,2,6,3,7}[j] (see
-        // nib_word), NF4: dim 8 i + j.  A row's scale comes from the elements its chunks hold (the mixed layouts drop the last eight).
-        static_assert(ST_THREADS >= 16 * 18, "a thread per chunk");
-        const int br = tid / 18, bi = tid % 18, bq = br >> 1;
+        if (warp == 8) qs_w[lane] = sign_word;  // sign words of the item's (up to four) queries
         float v[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = 0.0f;
-        if (tid < 16 * 18 && bq < nq) {
-            const float* q = a.q_coarse + (size_t)(it.query_begin + bq) * D_C;
-            constexpr bool HEAD = KIND == 1 || KIND == 4;
-            if (HEAD && bi < 2) {  // slots 0..3: the scale byte's high nibble's products of dims 4 i .., 4..7 the low nibble's
-                const float4 x = load_q4(q + 4 * bi);
-                v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = x.x; v[5] = x.y; v[6] = x.z; v[7] = x.w;
-            } else if (bi < 16) {
-                const int d0 = HEAD ? 8 * (bi - 1) : 8 * bi;
-                const float4 x = load_q4(q + d0), y = load_q4(q + d0 + 4);
-                if (KIND == 0) {
-                    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
-                } else {
-                    v[0] = x.x; v[1] = y.x; v[2] = x.y; v[3] = y.y; v[4] = x.z; v[5] = y.z; v[6] = x.w; v[7] = y.w;
-                }
-            } else if (bi == 16 && (KIND == 2 || KIND == 4)) {
-#pragma unroll
-                for (int g = KIND == 4 ? 1 : 0; g < 8; ++g) {
-                    float s = 0.0f;
-                    const float* qg = q + (KIND == 4 ? 16 * g - 8 : 16 * g);
-                    for (int d = 0; d < 16; ++d) s += qg[d];
-                    v[g] = 0.0625f * s;
-                }
-            }
-            if (bi < 16 && !(br & 1)) {
-                uint32_t largest = 0u;
-#pragma unroll
-                for (int j = 0; j < 8; ++j) largest = max(largest, abs_bits(v[j]));
-                atomicMax(&qmax[bq], largest);
-            }
+        if (KIND == 0 || head) {  // (head: slots 0..3 the scale byte's high nibble's products of dims 4 bi .., 4..7 the low nibble's)
+            v[0] = qx.x; v[1] = qx.y; v[2] = qx.z; v[3] = qx.w; v[4] = qy.x; v[5] = qy.y; v[6] = qy.z; v[7] = qy.w;
+        } else {
+            v[0] = qx.x; v[1] = qy.x; v[2] = qx.y; v[3] = qy.y; v[4] = qx.z; v[5] = qy.z; v[6] = qx.w; v[7] = qy.w;
         }
+        if (tid < 4 * 18 && bi < 16) {
+            uint32_t largest = 0u;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) largest = max(largest, abs_bits(v[j]));
+            atomicMax(&qmax[bq], largest);
+        }
+        if (EXTRA && tid < 4 * 18 && bi < 16) qsum[16 * bq + bi] = ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));  // of a group's half
         __syncthreads();
+        if (EXTRA && tid < 8 * 18 && bi == 16) {
+#pragma unroll
+            for (int g = KIND == 4 ? 1 : 0; g < 8; ++g) v[g] = 0.0625f * (qsum[16 * bq + 2 * g] + qsum[16 * bq + 2 * g + 1]);
+        }
         if (tid < 16 * 18) {
-            const float up = split_scale(qmax[bq & 3], 14).x;  // (rows 8 .. 15 are zero)
+            const float up = split_scale(qmax[bq], 14).x;  // (rows 8 .. 15 are zero)
             uint32_t w[4];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 float x0 = v[2 * j] * up, x1 = v[2 * j + 1] * up;
-                if (br & 1) { x0 = half_residual(x0); x1 = half_residual(x1); }
+                if (br >= 4) { x0 = half_residual(x0); x1 = half_residual(x1); }
                 w[j] = pack_half2(x0, x1);
             }
             const uint32_t slab = (uint32_t)bi >> 3, chunk = (uint32_t)bi & 7u;
@@ -525,10 +567,15 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
         // second item on rows other CTAs have been scoring for a while).
         // (from a barrier's vote, not from the flag word: a fast warp may raise the flag for an undecodable tile meanwhile)
         const bool too_big = __syncthreads_or(big) != 0;
-        const bool all_warm = __syncthreads_and(row_warm) != 0;
+        const bool all_warm = !DENSE && __syncthreads_and(row_warm) != 0;
         const bool first_round_barrier = !DENSE && !all_warm && (uint64_t)a.k <= (uint64_t)(ST_WT * NWARPS) * (uint64_t)max((it.pad >> 8) & 0x7FFFFFu, 1u);
         const uint32_t rounds = too_big ? 0u : my_rounds;  // (copies already on their way are waited for at the item's end and never read)
 
+        auto state_of = [&](uint32_t i) {
+            const uint32_t t = i < my_rounds ? block_of(i) * (uint32_t)ST_M + (uint32_t)(wq * ST_WT + lane) : 0xFFFFFFFFu;
+            return t < n ? sbase[t] : ST_HOT;
+        };
+        uint8_t st_next = sbase ? state_of(0) : ST_HOT;
         uint32_t slot = 0, polls = 0;
         uint32_t cur[4] = {0, 0, 0, 0}, end[4] = {0, 0, 0, 0};  // this warp's chunk of every row's buffer
         bool dead = false;                                      // this warp met a tile it cannot decode, or a wait of it ran out
@@ -557,10 +604,16 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             __syncwarp();
             const uint32_t row = row_lane + slot;
             slot = slot == (ST_DEPTH - 1) * ST_SLOT ? 0u : slot + ST_SLOT;
-            if (b >= n_blocks) continue;  // (the same in the whole warpgroup)
+            if (b >= n_blocks) {  // (the same in the whole warpgroup)
+                if (sbase) st_next = state_of(round + 1);
+                continue;
+            }
             const uint32_t t0 = b * ST_M + (uint32_t)(wq * ST_WT + lane);
             bool live = t0 < n;
-            if (sbase && live) live = sbase[t0] != ST_COLD;
+            if (sbase) {  // (the slot's state came with the block before)
+                live = live && st_next != ST_COLD;
+                st_next = state_of(round + 1);
+            }
             const uint2 meta = lds_v2<96>(row);   // scale, lambda
             const uint4 x = lds_v4<112>(row);     // position, head | flags, scale bytes
             const uint32_t flags = x.y >> 16;
@@ -569,7 +622,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                 if (lane == 0) *bail = 1u;
                 dead = true;
             }
-            float c[4] = {0.0f, 0.0f, 0.0f, 0.0f}, low[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            uint64_t cs[2] = {0ull, 0ull}, low[2] = {0ull, 0ull};  // rows 0, 1 and 2, 3
             bool skip = false;
 #pragma unroll
             for (int h = 0; h < (KIND == 0 ? 2 : 1); ++h) {  // (NF4: the latent in two halves, whose hi and lo parts fill the same columns)
@@ -610,15 +663,27 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                 // The accumulators' sums with their rounding errors kept (two_sum), so that a score is rounded once here: the
                 // generic kernel adds fp32 products in sixteen short chains, and this kernel's error is not to be larger.
 #pragma unroll
-                for (int i = 0; i < NACC; ++i) {
-                    // NF4: the group's scale byte (byte -> float: 2^23 + b as a bit pattern, minus 2^23)
-                    const float gs = KIND == 0 ? __uint_as_float(__byte_perm(h ? x.w : x.z, 0x4B000000u, 0x7440 + i)) - 8388608.0f : 1.0f;
+                for (int p = 0; p < 2; ++p) {
+                    if (p && nq <= 2) break;  // (uniform)
+                    if (KIND == 0) {
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) {
-                        const float hi = __uint_as_float(v[i][2 * q]), lo = __uint_as_float(v[i][2 * q + 1]);
-                        const float p = KIND == 0 ? hi * gs : hi;
-                        low[q] += KIND == 0 ? fmaf(hi, gs, -p) + lo * gs : lo;
-                        two_sum(c[q], p, low[q]);
+                        for (int i = 0; i < NACC; ++i) {
+                            // the group's scale byte (byte -> float: 2^23 + b as a bit pattern, minus 2^23), and its products' rounding errors
+                            const float gs = __uint_as_float(__byte_perm(h ? x.w : x.z, 0x4B000000u, 0x7440 + i)) - 8388608.0f;
+                            const uint64_t hi = u2_pack(v[i][2 * p], v[i][2 * p + 1]), lo = u2_pack(v[i][4 + 2 * p], v[i][4 + 2 * p + 1]);
+                            const uint64_t g2 = f2_pack(gs, gs), n2 = f2_pack(-gs, -gs), prod = f2_mul(hi, g2);
+                            low[p] = f2_fma(f2_fma(lo, n2, f2_fma(hi, n2, prod)), 0xBF800000BF800000ull, low[p]);
+                            if (h == 0 && i == 0) cs[p] = prod;
+                            else two_sum2(cs[p], prod, low[p]);
+                        }
+                    } else {
+                        cs[p] = u2_pack(v[0][2 * p], v[0][2 * p + 1]);
+                        low[p] = u2_pack(v[0][4 + 2 * p], v[0][4 + 2 * p + 1]);
+#pragma unroll
+                        for (int i = 1; i < NACC; ++i) {
+                            low[p] = f2_add(low[p], u2_pack(v[i][4 + 2 * p], v[i][4 + 2 * p + 1]));
+                            two_sum2(cs[p], u2_pack(v[i][2 * p], v[i][2 * p + 1]), low[p]);
+                        }
                     }
                 }
             }
@@ -629,19 +694,34 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             }
             // (the row's power of two is exact; the tile's scale comes in the last step, so that the coarse term is rounded once there)
             const float su = __uint_as_float(meta.x) * (1.0f / 255.0f);
+            float c[4];
             {
-                const float4 inv = *reinterpret_cast<const float4*>(qinv);
-                c[0] = (c[0] + low[0]) * inv.x;
-                c[1] = (c[1] + low[1]) * inv.y;
-                c[2] = (c[2] + low[2]) * inv.z;
-                c[3] = (c[3] + low[3]) * inv.w;
+                const ulonglong2 inv = *reinterpret_cast<const ulonglong2*>(qinv);
+                cs[0] = f2_mul(f2_add(cs[0], low[0]), inv.x);
+                cs[1] = f2_mul(f2_add(cs[1], low[1]), inv.y);
+                asm("mov.b64 {%0, %1}, %2;\n" : "=f"(c[0]), "=f"(c[1]) : "l"(cs[0]));
+                asm("mov.b64 {%0, %1}, %2;\n" : "=f"(c[2]), "=f"(c[3]) : "l"(cs[1]));
             }
             if (dead) continue;
             const float lam = (flags & F_WARM) ? 0.0f : __uint_as_float(meta.y);
+            if (DENSE) {
+                const uint4 ra = lds_v4<64>(row), rb = lds_v4<80>(row);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    if (q >= nq) break;  // (uniform)
+                    const uint4 qa = lds_v4<0>(qsw_s + 32u * q), qb = lds_v4<16>(qsw_s + 32u * q);
+                    const uint32_t d[8] = {ra.x ^ qa.x, ra.y ^ qa.y, ra.z ^ qa.z, ra.w ^ qa.w, rb.x ^ qb.x, rb.y ^ qb.y, rb.z ^ qb.z, rb.w ^ qb.w};
+                    // 256 - 2 h without an integer conversion: (2^23 + h) as a bit pattern, times -2, plus 2^24 + 256 (exact)
+                    const float sc = fmaf(c[q], su, lam * fmaf(__uint_as_float(0x4B000000u | popc8_words(d)), -2.0f, 16777472.0f));
+                    // (the 32 lanes of a warp hold 32 consecutive tiles: one 128-byte run per row)
+                    if (t0 < n) rowp[q][t0] = live ? sc : __uint_as_float(a.cold_bits);
+                }
+                continue;
+            }
             // The residual term lies in [-256 lambda, 256 lambda]: a tile that cannot reach a row's threshold even with the
             // largest term needs no Hamming distance (257 and the relative slack cover the rounding of the bound itself).
             uint32_t m = 0;
-            if (DENSE || round == 0) {
+            if (round == 0) {
                 m = live ? (1u << nq) - 1u : 0u;
             } else {
                 float4 th;
@@ -659,12 +739,10 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                 for (int q = 0; q < 4; ++q)
                     if (m >> q & 1u) {
                         const uint32_t* qw = qs_w + 8 * q;
-                        const int h = __popc(ra.x ^ qw[0]) + __popc(ra.y ^ qw[1]) + __popc(ra.z ^ qw[2]) + __popc(ra.w ^ qw[3]) +
-                                      __popc(rb.x ^ qw[4]) + __popc(rb.y ^ qw[5]) + __popc(rb.z ^ qw[6]) + __popc(rb.w ^ qw[7]);
-                        // 256 - 2 h without an integer conversion: (2^23 + h) as a bit pattern, times -2, plus 2^24 + 256 (exact)
-                        c[q] = fmaf(c[q], su, lam * fmaf(__uint_as_float(0x4B000000u | (uint32_t)h), -2.0f, 16777472.0f));
+                        const uint32_t d[8] = {ra.x ^ qw[0], ra.y ^ qw[1], ra.z ^ qw[2], ra.w ^ qw[3], rb.x ^ qw[4], rb.y ^ qw[5], rb.z ^ qw[6], rb.w ^ qw[7]};
+                        c[q] = fmaf(c[q], su, lam * fmaf(__uint_as_float(0x4B000000u | popc8_words(d)), -2.0f, 16777472.0f));
                     }
-                if (!DENSE) {
+                {
                     if (round == 0) {
                         // First tiles of the warp: a row without a bucket mapping gets one from the scores this warp has just
                         // computed for it - their range widened by 1.5 spans on both sides.  Any monotone mapping is
@@ -741,18 +819,6 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                     }
                 }
             }
-            if (DENSE) {  // (the 32 lanes of a warp hold 32 consecutive tiles: one 128-byte run per row)
-                if (t0 < n) {
-#pragma unroll
-                    for (int q = 0; q < 4; ++q)
-                        if (q < nq) {
-                            const uint32_t Q = it.query_begin + (uint32_t)q;
-                            const size_t row0 = a.row_offset ? (size_t)a.row_offset[Q] : (size_t)Q * a.score_stride;
-                            a.scores[row0 + it.index_base + t0] = live ? c[q] : __uint_as_float(a.cold_bits);
-                        }
-                }
-                continue;
-            }
             // In turn, a warp raises the threshold of query (warp & 3): after its 2nd and 4th block (the first
             // thresholds come from the barrier after the first round), then every 8 blocks, the warps of a
             // query staggered.  A stale threshold costs appends (each one a store, a histogram count and,
@@ -781,7 +847,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
         }
         __syncthreads();
         if (tid == 0) *bail = 0u;  // (ordered before the next item's writers by the barrier at its start)
-    }
+    } while (next_item());
     cta.phase = phase;
     cta.failed = failed;
     return item_id;
@@ -796,10 +862,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) 
     dep_wait();
     uint32_t i = a.cta_begin[blockIdx.x];
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
-    const bool int4 = item_kind(first_tile_flags(a, a.stream_items[i]), false) == 3;
+    WorkItem it = a.stream_items[i];
+    uint32_t flags = first_tile_flags(a, it);
     TileCta cta = tile_open<false>(smem_raw);
-    if (int4) i = tile_run<3, IL, false, true>(a, cta, i, item_end);
-    tile_run<4, IL, false, false>(a, cta, i, item_end);
+    if (item_kind(flags, false) == 3) i = tile_run<3, IL, false, true>(a, cta, i, item_end, it, flags);
+    if (i < item_end) tile_run<4, IL, false, false>(a, cta, i, item_end, it, flags);
     tile_close(cta);
 }
 
@@ -812,8 +879,8 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     dep_launch();
     dep_wait();
     if (a.refused && *a.refused) return;
-    uint32_t i = a.cta_begin[blockIdx.x];
-    const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
+    uint32_t i = a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x;  // (null: an item a CTA)
+    const uint32_t item_end = a.cta_begin ? a.cta_begin[blockIdx.x + 1] : i + 1;
     if (threadIdx.x == 0) undone.n = 0u;
     if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
         uint32_t f = 0;
@@ -821,19 +888,22 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
             for (uint32_t q = 0; q < a.stream_items[e].n_queries; ++q) f |= a.only_flagged[a.stream_items[e].query_begin + q];
         if (!__syncthreads_or(f != 0u)) return;
     }
-    uint32_t flags = first_tile_flags(a, a.stream_items[i]);  // (on its way while the CTA is set up)
+    WorkItem it = a.stream_items[i];
+    uint32_t flags = first_tile_flags(a, it);  // (on its way while the CTA is set up, and the first item's queries with it)
+    if (threadIdx.x < 4u * it.n_queries) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_coarse + (size_t)it.query_begin * D_C + 32u * threadIdx.x));
+    if (threadIdx.x == 32) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_sign + (size_t)it.query_begin * 8));
+    if (threadIdx.x == 64 && a.row_offset) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.row_offset + it.query_begin));
     const bool nf4_too = a.nf4_table == 1u || (a.nf4_table == 2u && (first_tile_flags(a, a.stream_items[0]) & F_NF4));
     TileCta cta = tile_open<true>(smem_raw);
     for (;;) {
         switch (item_kind(flags, nf4_too)) {
-            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
-            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
-            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
-            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
-            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, nf4_too, &undone); break;
+            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
+            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
+            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
+            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
+            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
         }
         if (i >= item_end) break;
-        flags = first_tile_flags(a, a.stream_items[i]);
     }
     tile_close(cta);
     finish_undone(a, a.stream_items, undone, smem_raw);
