@@ -224,16 +224,12 @@ int32_t slha_b200_score_segments(const SciRustSlhaTile* tiles, const SlhaB200Seg
         // the host and checked before anything was launched, the GPU lay idle for the round trip: 89 us per call of 8 x 32 768 tiles
         // and 64 rows, of which the kernels take 50.)
         const bool dev_off = is_device_ptr(row_offsets);
-        const uint64_t* doff;
-        const uint32_t* refused = nullptr;
-        if (dev_off) {
-            SLHA_TRY(launch_check_offsets(c, row_offsets, n_queries, scores_len, row_len, &doff, &refused));
-        } else {
+        RowCheck check{row_offsets, n_queries, scores_len, row_len};
+        if (!dev_off) {
             std::memcpy(hoff.data(), row_offsets, n_queries * 8);
             for (size_t q = 0; q < n_queries; ++q)
                 if (hoff[q] > scores_len || (uint64_t)row_len > scores_len - hoff[q])
                     return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
-            SLHA_TRY(stage_in_t(c, row_offsets, n_queries, &doff));
         }
         const auto scored = [&]() -> Status {
             const float* dq;
@@ -244,11 +240,11 @@ int32_t slha_b200_score_segments(const SciRustSlhaTile* tiles, const SlhaB200Seg
             SLHA_TRY(stage_out(c, scores_out, scores_len * 4, &outs[0]));
             // a host destination comes back whole: what no row covers is zero
             if (outs[0].is_host) SLHA_CUDA(cudaMemsetAsync(outs[0].dev, 0, scores_len * 4, c->stream));
-            SLHA_TRY(launch_score_segments(c, tiles, hseg.data(), n_segments, dq, ds, n_queries, (float*)outs[0].dev,
-                                           reinterpret_cast<const unsigned long long*>(doff), row_len, fill, refused));
+            SLHA_TRY(launch_score_segments(c, tiles, hseg.data(), n_segments, dq, ds, n_queries, (float*)outs[0].dev, dev_off ? nullptr : hoff.data(), row_len, fill,
+                                           dev_off ? &check : nullptr));
             if (dev_off) {
                 bool bad;
-                SLHA_TRY(checked_offsets(c, &bad));
+                SLHA_TRY(checked_offsets(c, check, &bad));
                 if (bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
             }
             return finish_outputs(c, outs, sync_by_default(c));
@@ -256,7 +252,8 @@ int32_t slha_b200_score_segments(const SciRustSlhaTile* tiles, const SlhaB200Seg
         Status st = scored();
         if (dev_off && !st.ok()) {  // (what else was wrong is reported behind the offsets)
             bool bad;
-            if (checked_offsets(c, &bad).ok() && bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+            if (!check.launched) SLHA_TRY(launch_row_check(c, &check));
+            if (checked_offsets(c, check, &bad).ok() && bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
         }
         return st;
     });

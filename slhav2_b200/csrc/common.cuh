@@ -57,8 +57,8 @@ Status ctx_host_scratch(Ctx* c, size_t bytes, void** out);
 Status ctx_no_capture(Ctx* c);
 Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes);
 Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
-// A word of page-locked host memory that kernels of the calling thread's call can write, and an event: one of each per thread and device.
-Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, cudaEvent_t* event);
+// 64 bytes of page-locked host memory that kernels of the calling thread's call can write, per thread and device; *open while one may.
+Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, bool** open);
 // The call under way uses a plan's buffers (kept per thread, like the scratch arena): waits for another stream's use of them, see LastUse.
 void ctx_uses_plans(Ctx* c);
 void count_launch(int n = 1);
@@ -135,12 +135,25 @@ struct Model {
 // ---- kernels' host launchers (score.cu / encode.cu / pool.cu) -------------
 struct ScorePlan;  // cached work decomposition of one slha_b200_score_topk call shape
 
+// Row offsets in device memory: copied and checked there by a kernel of the call, *refused set to 1 where a row reaches beyond scores_len, else 0.  checked_offsets waits for the answer.
+struct RowCheck {
+    const uint64_t* offsets;
+    size_t nq;
+    uint64_t scores_len;
+    uint32_t row_len;
+    bool launched = false;
+    const uint64_t* copy = nullptr;
+    const uint32_t* refused = nullptr;
+    volatile uint32_t* host = nullptr;  // where the kernel answers: twice `no`, plus 1 where it objects
+    uint32_t no = 0;
+    bool* open = nullptr;
+};
+Status launch_row_check(Ctx* c, RowCheck* check);  // alone
+Status checked_offsets(Ctx* c, RowCheck& check, bool* refused);
+// row_offsets: host memory, or null and `check` for offsets in device memory
 Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, const float* d_q_coarse,
-                             const uint64_t* d_q_sign, size_t nq, float* d_scores, const unsigned long long* d_row_offsets,
-                             uint32_t row_len, float fill, const uint32_t* refused = nullptr);
-// Row offsets in device memory: copied to *d_copy and checked there, *d_refused set to 1 where a row reaches beyond scores_len, else 0.  checked_offsets waits for the thread's latest check.
-Status launch_check_offsets(Ctx* c, const uint64_t* d_offsets, size_t nq, uint64_t scores_len, uint32_t row_len, const uint64_t** d_copy, const uint32_t** d_refused);
-Status checked_offsets(Ctx* c, bool* refused);
+                             const uint64_t* d_q_sign, size_t nq, float* d_scores, const uint64_t* row_offsets,
+                             uint32_t row_len, float fill, RowCheck* check);
 Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state, size_t n,
                          const float* q_coarse, const uint64_t* q_sign, size_t nq, float* scores, int codec_hint = -1);
 // d_status must hold ~0ull on entry; receives min over bad tiles of (index << 8 | code) with

@@ -76,12 +76,9 @@ struct LastUse {
 struct Answer {
     uint32_t* host = nullptr;
     uint32_t* dev = nullptr;
-    cudaEvent_t event = nullptr;
+    bool open = false;  // a kernel may still write there: nobody has seen its answer (a call that ended by an exception)
     ~Answer() {
-        if (event) {
-            cudaEventSynchronize(event);
-            cudaEventDestroy(event);
-        }
+        if (open) cudaDeviceSynchronize();
         if (host) cudaFreeHost(host);
     }
 };
@@ -239,16 +236,16 @@ Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
     tls.upload_used[c->device] = &s;  // (its event is recorded at the call's end)
     return Status();
 }
-Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, cudaEvent_t* event) {
+Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, bool** open) {
     Answer& a = tls.answer[c->device];
-    if (!a.event) {
-        if (!a.host) SLHA_CUDA(cudaHostAlloc((void**)&a.host, 64, cudaHostAllocMapped | cudaHostAllocPortable));
-        SLHA_CUDA(cudaHostGetDevicePointer((void**)&a.dev, a.host, 0));
-        SLHA_CUDA(cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming));
+    if (!a.host) {
+        SLHA_CUDA(cudaHostAlloc((void**)&a.host, 64, cudaHostAllocMapped | cudaHostAllocPortable));
+        std::memset(a.host, 0, 64);
     }
+    if (!a.dev) SLHA_CUDA(cudaHostGetDevicePointer((void**)&a.dev, a.host, 0));
     *host = a.host;
     *dev = a.dev;
-    *event = a.event;
+    *open = &a.open;
     return Status();
 }
 void ctx_uses_plans(Ctx* c) {

@@ -302,6 +302,7 @@ struct ScoreArgs {
     uint32_t* ghist;              // per query row: 256 bucket counts of appended candidates
     uint32_t* gcount;             // per query row: candidates appended to the row's buffer
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
+    uint32_t by_fours;            // score_dense_kernel: items are the 64-row kernel's, taken four rows at a time (item e: rows 4 (e mod 16) .. of items[e / 16])
     uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): 1, or 2 where that pass is to
     uint32_t handoff_as;          // score them in score_kernel's arithmetic (NF4 rows always 1)
     const uint32_t* only_flagged; // dense mode: optional, per query row: only work items one of whose rows is flagged here
@@ -455,6 +456,21 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
     }
 }
 
+// Item e of a call of score_dense_kernel.
+__device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e) {
+    if (!a.by_fours) return a.stream_items[e];
+    WorkItem it = a.stream_items[e >> 4];
+    const uint32_t q = 4u * (e & 15u);
+    it.query_begin += q;
+    it.n_queries = it.n_queries > q ? min(4u, it.n_queries - q) : 0u;
+    return it;
+}
+// (null: an item a CTA)
+__device__ __forceinline__ uint32_t dense_first(const ScoreArgs& a, uint32_t cta) {
+    const uint32_t i = a.cta_begin ? a.cta_begin[cta] : cta;
+    return a.by_fours ? 16u * i : i;
+}
+
 // Work items that a dense kernel's CTA could not score on the tensor cores (a tile of another codec than its item's first, a query outside the fp16
 // split), to be scored in score_kernel's arithmetic once the CTA is through: in its loop the call would cost registers.
 struct Undone {
@@ -523,11 +539,11 @@ __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem&
     __syncthreads();
 }
 // What is left at a CTA's end (all of its shared memory is free).
-__device__ __noinline__ void finish_undone(const ScoreArgs& a, const WorkItem* items, const Undone& u, unsigned char* smem) {
+__device__ __noinline__ void finish_undone(const ScoreArgs& a, const Undone& u, unsigned char* smem) {
     __syncthreads();
-    const uint32_t m = u.n, first = a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x, end = a.cta_begin ? a.cta_begin[blockIdx.x + 1] : first + 1;
+    const uint32_t m = u.n, first = dense_first(a, blockIdx.x), end = dense_first(a, blockIdx.x + 1);
     for (uint32_t j = 0; j < (m > 31u ? end - first : m); ++j) {
-        const WorkItem it = items[m > 31u ? first + j : u.item[j]];
+        const WorkItem it = dense_item(a, m > 31u ? first + j : u.item[j]);
         for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
     }
 }

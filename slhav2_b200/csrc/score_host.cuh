@@ -197,9 +197,6 @@ struct Blob {
         if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
         return at;
     }
-    Status upload(Ctx* c, unsigned char** dev) {
-        return ctx_upload(c, bytes.data(), bytes.size(), (void**)dev);
-    }
 };
 
 // The cached decomposition of one score_topk call shape.
@@ -253,7 +250,7 @@ struct Plan {
     float* d_tmp_score = nullptr;
     // Rows whose scores are written as a whole and selected from (score_select.cuh)
     bool rows = false, allow_rows_in = false;
-    uint32_t longest = 0, grid_narrow = 0, grid_wide = 0;
+    uint32_t longest = 0;
     uint64_t row_stride = 0;
     RowInfo* d_rows = nullptr;
     uint32_t* d_row_flags = nullptr;  // [nq] generic arithmetic, [nq] handed on by the 64-row kernel, [nq][2] statistics
@@ -329,17 +326,16 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
         total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
         wtotal += (uint64_t)s.n_tiles * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
     }
-    Cuts narrow(total, sms, ST_M, ST_M), many(wtotal, sms, WIDE_M, WIDE_M);
+    wide = wide && allow_wide && wtotal;
+    Cuts cuts(wide ? wtotal : total, sms, wide ? WIDE_M : ST_M, wide ? WIDE_M : ST_M);
     for (size_t i = 0; i < n_segs; ++i) {
         SlhaB200Segment s = segs[i];
         s.index_base = 0;  // (where the scores go: a place in the row)
-        narrow.add(s, 4);
-        if (wide) many.add(s, WIDE_NQ);
+        cuts.add(s, wide ? WIDE_NQ : 4);
     }
-    narrow.finish();
-    many.finish();
+    cuts.finish();
     Blob tables;
-    const size_t o_n = tables.add(narrow.items), o_nc = tables.add(narrow.cta), o_w = tables.add(many.items), o_wc = tables.add(many.cta), o_r = tables.add(rows);
+    const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows);
     SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
     SLHA_TRY(p->b_gpivot.ensure(4 * nq * 4));
     p->row_stride = ((uint64_t)longest + 31) / 32 * 32;
@@ -349,15 +345,11 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     p->d_row_flags = (uint32_t*)p->b_gpivot.p;
     SLHA_CUDA(cudaMemsetAsync(p->d_row_flags, 0, 4 * nq * 4, c->stream));
     p->d_items = reinterpret_cast<WorkItem*>(dev + o_n);
-    p->d_cta_begin = narrow.items.size() + 1 == narrow.cta.size() ? nullptr : reinterpret_cast<uint32_t*>(dev + o_nc);
-    p->d_wide_items = reinterpret_cast<WorkItem*>(dev + o_w);
-    p->d_wide_cta = reinterpret_cast<uint32_t*>(dev + o_wc);
+    p->wide = wide;
+    p->n_items = (uint32_t)cuts.items.size();
+    p->mma_grid = (uint32_t)cuts.cta.size() - 1;
+    p->d_cta_begin = !wide && p->n_items == p->mma_grid ? nullptr : reinterpret_cast<uint32_t*>(dev + o_nc);  // (null: an item a CTA)
     p->d_rows = reinterpret_cast<RowInfo*>(dev + o_r);
-    p->wide = wide && allow_wide && !many.items.empty();
-    p->grid_narrow = (uint32_t)narrow.cta.size() - 1;
-    p->grid_wide = (uint32_t)many.cta.size() - 1;
-    p->n_items = (uint32_t)narrow.items.size();
-    p->n_wide_items = (uint32_t)many.items.size();
     p->longest = longest;
     p->rows = true;
     return Status();
@@ -782,6 +774,106 @@ Status launch_validate_tiles(Ctx* c, const SciRustSlhaTile* tiles, size_t n, uns
     return Status();
 }
 
+// What a dense call brings from the host, in a kernel's parameters: its tables, copied to `dst`, and with them the check of row offsets in device
+// memory (block 0).  An upload between two kernels cost 8 us (8 x 32 768 tiles x 64 rows 57 us a call, now 50).
+template <int BYTES>
+struct TableParam {
+    uint4 w[BYTES / 16];
+};
+constexpr uint32_t TABLE_SLICE = 2048;  // bytes a block copies (parameters are read one address at a time)
+template <int BYTES>
+__global__ void __launch_bounds__(256) table_kernel(const __grid_constant__ TableParam<BYTES> table, uint32_t n16, uint4* dst, const uint64_t* offsets, uint32_t nq, uint64_t scores_len,
+                                                    uint32_t row_len, uint64_t* copy, uint32_t* refused, uint32_t* answer, uint32_t check_no) {
+    dep_launch();
+    dep_wait();
+    const uint32_t i = blockIdx.x * (TABLE_SLICE / 16) + threadIdx.x;
+    if (threadIdx.x < TABLE_SLICE / 16 && i < n16) dst[i] = table.w[i];
+    if (blockIdx.x || !offsets) return;
+    bool bad = false;
+    for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x) {
+        const uint64_t o = offsets[q];
+        copy[q] = o;
+        bad |= o > scores_len || row_len > scores_len - o;
+    }
+    bad = __syncthreads_or(bad) != 0;
+    if (threadIdx.x == 0) {
+        *refused = bad;
+        *reinterpret_cast<volatile uint32_t*>(answer) = 2u * check_no + bad;  // (page-locked host memory)
+    }
+}
+constexpr uint32_t ANSWERS = 16;  // words that checks answer in, in turn: one of a call that ended early may still write
+thread_local uint32_t g_check_no = 0;
+template <int BYTES>
+Status launch_table_t(Ctx* c, const Blob& blob, uint4* dst, const uint64_t* offsets, uint32_t nq, uint64_t scores_len, uint32_t row_len, uint64_t* copy, uint32_t* refused, uint32_t* answer,
+                      uint32_t check_no) {
+    static thread_local TableParam<BYTES> table;
+    std::memcpy(&table, blob.bytes.data(), blob.bytes.size());
+    const uint32_t n16 = (uint32_t)((blob.bytes.size() + 15) / 16), blocks = std::max<uint32_t>(1, (n16 * 16 + TABLE_SLICE - 1) / TABLE_SLICE);
+    SLHA_CUDA(launch_behind(table_kernel<BYTES>, dim3(blocks), dim3(256), 0, c->stream, table, n16, dst, offsets, nq, scores_len, row_len, copy, refused, answer, check_no));
+    count_launch();
+    return Status();
+}
+// The call's tables to the device (*dev), and the check of `check`'s offsets, if any, with them.
+Status send_tables(Ctx* c, const Blob& blob, unsigned char** dev, RowCheck* check) {
+    SLHA_TRY(ctx_no_capture(c));
+    const bool in_params = blob.bytes.size() <= 16384;
+    uint64_t* copy = nullptr;
+    uint32_t *refused = nullptr, *answer = nullptr, no = 0;
+    if (check) {
+        if (check->nq > 0xFFFFFFFFull) return Status(SLHA_ERR_DIMENSION, "too many query rows");
+        void* mem;
+        SLHA_TRY(ctx_device_scratch(c, check->nq * 8 + 8, &mem));
+        SLHA_TRY(ctx_answer(c, &check->host, &answer, &check->open));
+        g_check_no = g_check_no % 0x7FFFFFFFu + 1u;
+        check->no = no = g_check_no;
+        check->host += no % ANSWERS;
+        answer += no % ANSWERS;
+        copy = static_cast<uint64_t*>(mem);
+        refused = reinterpret_cast<uint32_t*>(copy + check->nq);
+    }
+    const uint64_t* offsets = check ? check->offsets : nullptr;
+    const uint32_t nq = check ? (uint32_t)check->nq : 0u, row_len = check ? check->row_len : 0u;
+    const uint64_t len = check ? check->scores_len : 0ull;
+    if (in_params && !blob.bytes.empty()) SLHA_TRY(ctx_device_scratch(c, (blob.bytes.size() + 15) / 16 * 16, (void**)dev));
+    else if (!blob.bytes.empty()) SLHA_TRY(ctx_upload(c, blob.bytes.data(), blob.bytes.size(), (void**)dev));
+    uint4* dst = in_params ? reinterpret_cast<uint4*>(*dev) : nullptr;
+    static const Blob none;
+    const Blob& sent = in_params ? blob : none;
+    if (in_params || check) {
+        if (sent.bytes.size() <= 2048) SLHA_TRY(launch_table_t<2048>(c, sent, dst, offsets, nq, len, row_len, copy, refused, answer, no));
+        else if (sent.bytes.size() <= 6144) SLHA_TRY(launch_table_t<6144>(c, sent, dst, offsets, nq, len, row_len, copy, refused, answer, no));
+        else SLHA_TRY(launch_table_t<16384>(c, sent, dst, offsets, nq, len, row_len, copy, refused, answer, no));
+    }
+    if (check) {
+        *check->open = check->launched = true;
+        check->copy = copy;
+        check->refused = refused;
+    }
+    return Status();
+}
+Status launch_row_check(Ctx* c, RowCheck* check) {
+    unsigned char* dev = nullptr;
+    return send_tables(c, Blob(), &dev, check);
+}
+// (The host polls the word: recording an event and waiting for it cost 3 us of a call of 17.)
+Status checked_offsets(Ctx* c, RowCheck& check, bool* refused) {
+    for (uint32_t i = 0; (*check.host >> 1) != check.no; ++i) {
+        if (i % 4096 != 4095) continue;
+        const cudaError_t e = cudaStreamQuery(c->stream);
+        if (e == cudaErrorNotReady) continue;
+        SLHA_CUDA(e);
+        uint32_t word = 0;  // the stream is idle: the kernel's own word
+        SLHA_CUDA(cudaMemcpyAsync(&word, check.refused, 4, cudaMemcpyDeviceToHost, c->stream));
+        SLHA_CUDA(cudaStreamSynchronize(c->stream));
+        *refused = word != 0;
+        *check.open = false;
+        return Status();
+    }
+    *refused = (*check.host & 1u) != 0;
+    *check.open = false;
+    return Status();
+}
+
 Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* state, size_t n,
                          const float* q_coarse, const uint64_t* q_sign, size_t nq, float* scores, int codec_hint) {
     if (n == 0 || nq == 0) return Status();
@@ -796,7 +888,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         Blob blob;
         const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta);
         unsigned char* dev;
-        SLHA_TRY(blob.upload(c, &dev));
+        SLHA_TRY(send_tables(c, blob, &dev, nullptr));
         ScoreArgs a{};
         a.cold_bits = 0xFF800000u;
         a.tiles = reinterpret_cast<const unsigned char*>(tiles);
@@ -809,7 +901,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
         a.scores = scores;
         a.score_stride = n;
         a.nf4_table = codec_hint < 0 ? 2u : (uint32_t)(codec_hint & 1);
-        return launch_dense(c, a, (uint32_t)cuts.cta.size() - 1, false);
+        return launch_dense(c, a, (uint32_t)cuts.cta.size() - 1, true);
     }
     const int threads = 128, nwarps = threads / 32;
     const uint32_t item_tiles = 4096;
@@ -836,54 +928,6 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     return Status();
 }
 
-__global__ void __launch_bounds__(256) check_offsets_kernel(const uint64_t* offsets, uint32_t nq, uint64_t scores_len, uint32_t row_len, uint64_t* copy, uint32_t* refused, uint32_t* answer) {
-    dep_launch();
-    dep_wait();
-    bool bad = false;
-    for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x) {
-        const uint64_t o = offsets[q];
-        copy[q] = o;
-        bad |= o > scores_len || row_len > scores_len - o;
-    }
-    bad = __syncthreads_or(bad) != 0;
-    if (threadIdx.x == 0) {
-        *refused = bad;
-        *reinterpret_cast<volatile uint32_t*>(answer) = bad;
-    }
-}
-// A check whose answer nobody has waited for (a call that ended by an exception): its kernel may still write the word.
-thread_local bool g_check_pending[16] = {false};
-Status launch_check_offsets(Ctx* c, const uint64_t* d_offsets, size_t nq, uint64_t scores_len, uint32_t row_len, const uint64_t** d_copy, const uint32_t** d_refused) {
-    SLHA_TRY(ctx_no_capture(c));
-    if (nq > 0xFFFFFFFFull) return Status(SLHA_ERR_DIMENSION, "too many query rows");
-    void* dev;
-    SLHA_TRY(ctx_device_scratch(c, nq * 8 + 8, &dev));
-    volatile uint32_t* host;
-    uint32_t* answer;
-    cudaEvent_t event;
-    SLHA_TRY(ctx_answer(c, &host, &answer, &event));
-    if (g_check_pending[c->device & 15]) SLHA_CUDA(cudaEventSynchronize(event));
-    uint64_t* copy = static_cast<uint64_t*>(dev);
-    uint32_t* refused = reinterpret_cast<uint32_t*>(copy + nq);
-    SLHA_CUDA(launch_behind(check_offsets_kernel, dim3(1), dim3(256), 0, c->stream, d_offsets, (uint32_t)nq, scores_len, row_len, copy, refused, answer));
-    count_launch();
-    SLHA_CUDA(cudaEventRecord(event, c->stream));
-    g_check_pending[c->device & 15] = true;
-    *d_copy = copy;
-    *d_refused = refused;
-    return Status();
-}
-Status checked_offsets(Ctx* c, bool* refused) {
-    volatile uint32_t* host;
-    uint32_t* answer;
-    cudaEvent_t event;
-    SLHA_TRY(ctx_answer(c, &host, &answer, &event));
-    SLHA_CUDA(cudaEventSynchronize(event));
-    g_check_pending[c->device & 15] = false;
-    *refused = *host != 0;
-    return Status();
-}
-
 // fill of the rows' tails [tail_begin[q], row_len) (one CTA per row)
 __global__ void fill_rows_kernel(float* scores, const unsigned long long* row_offset, const uint32_t* tail_begin, uint32_t row_len, float fill, const uint32_t* refused) {
     if (refused && *refused) return;
@@ -896,8 +940,8 @@ __global__ void fill_rows_kernel(float* scores, const unsigned long long* row_of
 // more the 64-row kernel comes first and the four-row kernel takes the rows it hands over (it ends at once when there are none).  The host looks at no tile and
 // waits for nothing.
 Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* segs, size_t n_segs, const float* d_q_coarse,
-                             const uint64_t* d_q_sign, size_t nq, float* d_scores, const unsigned long long* d_row_offsets,
-                             uint32_t row_len, float fill, const uint32_t* refused) {
+                             const uint64_t* d_q_sign, size_t nq, float* d_scores, const uint64_t* row_offsets,
+                             uint32_t row_len, float fill, RowCheck* check) {
     const int sms = sm_count(c->device);
     bool wide = !g_force_generic, fills = false;
     uint64_t total = 0, wtotal = 0;
@@ -912,16 +956,13 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
         total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
         wtotal += (uint64_t)s.n_tiles * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
     }
-    Cuts narrow(total, sms, ST_M, ST_M * 4), many(wtotal, sms, WIDE_M, WIDE_M);
-    for (size_t i = 0; i < n_segs; ++i) {
-        narrow.add(segs[i], 4);
-        if (wide) many.add(segs[i], WIDE_NQ);
-    }
-    narrow.finish();
-    many.finish();
+    // (the four-row kernel's pass behind the 64-row kernel takes that one's items, four rows at a time)
+    Cuts cuts(wide ? wtotal : total, sms, wide ? WIDE_M : ST_M, wide ? WIDE_M : ST_M * 4);
+    for (size_t i = 0; i < n_segs; ++i) cuts.add(segs[i], wide ? WIDE_NQ : 4);
+    cuts.finish();
     std::vector<WorkItem> generic;  // runs of 4096 tiles where score_kernel takes the call
     if (g_force_generic)
-        for (const WorkItem& s : narrow.items)
+        for (const WorkItem& s : cuts.items)
             for (uint32_t pos = 0; pos < s.n_tiles; pos += 4096) {
                 WorkItem w = s;
                 w.tile_begin += pos;
@@ -930,16 +971,19 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
                 generic.push_back(w);
             }
     Blob blob;
-    const size_t o_narrow = blob.add(narrow.items), o_ncta = blob.add(narrow.cta), o_many = blob.add(many.items), o_mcta = blob.add(many.cta), o_gen = blob.add(generic);
-    const size_t o_tail = blob.add(tail), o_flag = blob.add(std::vector<uint32_t>(nq, 0u));
+    const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta), o_gen = blob.add(generic);
+    const size_t o_tail = fills ? blob.add(tail) : 0, o_flag = wide ? blob.add(std::vector<uint32_t>(nq, 0u)) : 0;
+    const size_t o_rows = check ? 0 : blob.add(std::vector<uint64_t>(row_offsets, row_offsets + nq));
     unsigned char* dev;
-    SLHA_TRY(blob.upload(c, &dev));
+    SLHA_TRY(send_tables(c, blob, &dev, check));
+    const unsigned long long* d_row_offsets = reinterpret_cast<const unsigned long long*>(check ? check->copy : reinterpret_cast<const uint64_t*>(dev + o_rows));
+    const uint32_t* refused = check ? check->refused : nullptr;
     if (fills) {
         fill_rows_kernel<<<(uint32_t)nq, 256, 0, c->stream>>>(d_scores, d_row_offsets, reinterpret_cast<const uint32_t*>(dev + o_tail), row_len, fill, refused);
         count_launch();
         SLHA_CUDA(cudaGetLastError());
     }
-    if (narrow.items.empty()) return Status();
+    if (cuts.items.empty()) return Status();
     ScoreArgs a{};
     a.tiles = reinterpret_cast<const unsigned char*>(tiles);
     a.q_coarse = d_q_coarse;
@@ -948,20 +992,20 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     a.row_offset = d_row_offsets;
     a.cold_bits = 0xFF800000u;
     a.refused = refused;
-    uint32_t* flag = reinterpret_cast<uint32_t*>(dev + o_flag);
+    a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_items);
+    a.n_items = (uint32_t)cuts.items.size();
+    a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_cta);
+    const uint32_t grid = (uint32_t)cuts.cta.size() - 1;
     if (wide) {
-        a.items = reinterpret_cast<const WorkItem*>(dev + o_many);
-        a.n_items = (uint32_t)many.items.size();
-        a.cta_begin = reinterpret_cast<const uint32_t*>(dev + o_mcta);
-        a.handoff = flag;
+        a.handoff = reinterpret_cast<uint32_t*>(dev + o_flag);
         a.handoff_as = 1u;
-        SLHA_TRY(launch_wide_dense(c, a, (uint32_t)many.cta.size() - 1, false));
-        a.only_flagged = flag;
+        SLHA_TRY(launch_wide_dense(c, a, grid, true));
+        a.only_flagged = a.handoff;
+        a.by_fours = 1u;
+    } else if (a.n_items == grid) {
+        a.cta_begin = nullptr;
     }
-    a.items = a.stream_items = reinterpret_cast<const WorkItem*>(dev + o_narrow);
-    a.n_items = (uint32_t)narrow.items.size();
-    a.cta_begin = narrow.items.size() + 1 == narrow.cta.size() ? nullptr : reinterpret_cast<const uint32_t*>(dev + o_ncta);
-    if (!g_force_generic) return launch_dense(c, a, (uint32_t)narrow.cta.size() - 1, wide);
+    if (!g_force_generic) return launch_dense(c, a, grid, true);
     a.items = reinterpret_cast<const WorkItem*>(dev + o_gen);
     const int threads = 128, nwarps = threads / 32;
     return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0), false);
@@ -984,19 +1028,17 @@ static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, con
     a.cold_bits = ROW_ABSENT;
     a.nf4_table = codec_hint < 0 ? 2u : (uint32_t)(codec_hint & 1);
     a.gflag = p->d_row_flags;
-    if (p->wide) {
-        a.items = p->d_wide_items;
-        a.n_items = p->n_wide_items;
-        a.cta_begin = p->d_wide_cta;
-        a.handoff = p->d_row_flags + nq;
-        a.handoff_as = 2u;
-        SLHA_TRY(launch_wide_dense(c, a, p->grid_wide, true));
-        a.only_flagged = a.handoff;
-    }
     a.items = a.stream_items = p->d_items;
     a.n_items = p->n_items;
     a.cta_begin = p->d_cta_begin;
-    SLHA_TRY(launch_dense(c, a, p->grid_narrow, true));
+    if (p->wide) {
+        a.handoff = p->d_row_flags + nq;
+        a.handoff_as = 2u;
+        SLHA_TRY(launch_wide_dense(c, a, p->mma_grid, true));
+        a.only_flagged = a.handoff;
+        a.by_fours = 1u;  // (the pass takes the same items, four rows at a time)
+    }
+    SLHA_TRY(launch_dense(c, a, p->mma_grid, true));
     if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));
     RowsArgs r{a.scores, p->row_stride, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, p->kp2, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
     SLHA_TRY(launch_rows(c, r, (uint32_t)nq, p->longest));

@@ -409,7 +409,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
 
     auto next_item = [&]() {  // false at the end, or at an item of another kind (the same in the whole CTA)
         if (++item_id >= item_end) return false;
-        it = a.stream_items[item_id];
+        it = DENSE ? dense_item(a, item_id) : a.stream_items[item_id];
         if (KINDS) flags0 = first_tile_flags(a, it);
         return !KINDS || item_kind(flags0, nf4_too) == KIND;
     };
@@ -879,16 +879,18 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     dep_launch();
     dep_wait();
     if (a.refused && *a.refused) return;
-    uint32_t i = a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x;  // (null: an item a CTA)
-    const uint32_t item_end = a.cta_begin ? a.cta_begin[blockIdx.x + 1] : i + 1;
+    uint32_t i = dense_first(a, blockIdx.x);
+    const uint32_t item_end = dense_first(a, blockIdx.x + 1);
     if (threadIdx.x == 0) undone.n = 0u;
     if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
         uint32_t f = 0;
-        for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS)
-            for (uint32_t q = 0; q < a.stream_items[e].n_queries; ++q) f |= a.only_flagged[a.stream_items[e].query_begin + q];
+        for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS) {
+            const WorkItem own = dense_item(a, e);
+            for (uint32_t q = 0; q < own.n_queries; ++q) f |= a.only_flagged[own.query_begin + q];
+        }
         if (!__syncthreads_or(f != 0u)) return;
     }
-    WorkItem it = a.stream_items[i];
+    WorkItem it = dense_item(a, i);
     uint32_t flags = first_tile_flags(a, it);  // (on its way while the CTA is set up, and the first item's queries with it)
     if (threadIdx.x < 4u * it.n_queries) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_coarse + (size_t)it.query_begin * D_C + 32u * threadIdx.x));
     if (threadIdx.x == 32) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_sign + (size_t)it.query_begin * 8));
@@ -906,7 +908,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
         if (i >= item_end) break;
     }
     tile_close(cta);
-    finish_undone(a, a.stream_items, undone, smem_raw);
+    finish_undone(a, undone, smem_raw);
 }
 
 }  // namespace
