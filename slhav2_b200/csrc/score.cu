@@ -302,6 +302,7 @@ struct ScoreArgs {
     uint32_t* ghist;              // per query row: 256 bucket counts of appended candidates
     uint32_t* gcount;             // per query row: candidates appended to the row's buffer
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
+    uint32_t blocked;             // dense mode: item's scores lie in blocks of 128 tiles, block b's of its row q from list_begin + b * pad + 128 q on
     uint32_t by_fours;            // score_dense_kernel: items are the 64-row kernel's, taken four rows at a time (item e: rows 4 (e mod 16) .. of items[e / 16])
     uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): 1, or 2 where that pass is to
     uint32_t handoff_as;          // score them in score_kernel's arithmetic (NF4 rows always 1)
@@ -463,6 +464,7 @@ __device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e) {
     const uint32_t q = 4u * (e & 15u);
     it.query_begin += q;
     it.n_queries = it.n_queries > q ? min(4u, it.n_queries - q) : 0u;
+    it.list_begin += 128u * q;
     return it;
 }
 // (null: an item a CTA)
@@ -531,8 +533,9 @@ __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem&
         for (int g = 0; g < G; ++g) {
             const float sc = transpose_reduce8(part[g], s);
             if (g < nq && ti < n) {
-                const size_t row0 = a.row_offset ? (size_t)a.row_offset[query_begin + g] : (size_t)(query_begin + g) * a.score_stride;
-                a.scores[row0 + it.index_base + ti] = live ? sc : __uint_as_float(a.cold_bits);
+                const size_t at = a.blocked ? (size_t)((it.index_base + ti) >> 7) * it.pad + it.list_begin + 128u * (query_begin - it.query_begin + g) + (ti & 127u)
+                                            : (a.row_offset ? (size_t)a.row_offset[query_begin + g] : (size_t)(query_begin + g) * a.score_stride) + it.index_base + ti;
+                a.scores[at] = live ? sc : __uint_as_float(a.cold_bits);
             }
         }
     }

@@ -71,7 +71,7 @@ Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
 template <int KIND>
 Status launch_wide_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_wide_kernel<KIND>, configured, a, grid, WIDE_THREADS, wide_smem_bytes(), true);
+    return launch_tc(c, score_wide_kernel<KIND>, configured, a, grid, WIDE_THREADS, wide_smem_bytes(false), true);
 }
 Status launch_wide(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
     switch (kind) {
@@ -83,7 +83,7 @@ Status launch_wide(Ctx* c, int kind, const ScoreArgs& a, uint32_t grid) {
 }
 Status launch_wide_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_wide_dense_kernel, configured, a, grid, WIDE_THREADS, wide_smem_bytes(), behind);
+    return launch_tc(c, score_wide_dense_kernel, configured, a, grid, WIDE_THREADS, wide_smem_bytes(true), behind);
 }
 template <int NT, int R>
 Status launch_rows_t(Ctx* c, const RowsArgs& a, uint32_t nq) {
@@ -265,8 +265,8 @@ std::atomic<uint32_t> g_plan_threads{0};
 struct Cuts {
     std::vector<WorkItem> items;
     std::vector<uint32_t> cta{0u};
-    uint64_t share = 0, filled = 0;
-    Cuts(uint64_t total, int sms, uint64_t unit, uint64_t least) {
+    uint64_t share = 0, filled = 0, unit;
+    Cuts(uint64_t total, int sms, uint64_t unit_tiles, uint64_t least) : unit(unit_tiles) {
         share = (total + sms - 1) / sms;
         share = std::max<uint64_t>(least, (share + unit - 1) / unit * unit);
     }
@@ -282,7 +282,7 @@ struct Cuts {
                 w.n_queries = std::min<uint32_t>(width, s.n_queries - q0);
                 items.push_back(w);
                 pos += take;
-                filled += take;
+                filled += (take + unit - 1) / unit * unit;  // (cuts lie at whole units of a segment)
                 if (filled >= share) {
                     filled = 0;
                     cta.push_back((uint32_t)items.size());
@@ -312,7 +312,7 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     const int sms = sm_count(c->device);
     bool wide = true;
     uint64_t total = 0, wtotal = 0;
-    std::vector<RowInfo> rows(nq, RowInfo{0u, 0u});
+    std::vector<RowInfo> rows(nq, RowInfo{0u, 0u, 0u, 128u});
     std::vector<uint8_t> taken(nq, 0);
     for (size_t i = 0; i < n_segs; ++i) {
         const SlhaB200Segment& s = segs[i];
@@ -320,7 +320,7 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
         for (uint32_t q = 0; q < s.n_queries; ++q) {
             if (taken[s.query_begin + q]) return Status(SLHA_ERR_DIMENSION, "a query row belongs to two segments");
             taken[s.query_begin + q] = s.n_tiles != 0;
-            rows[s.query_begin + q] = RowInfo{s.n_tiles, s.index_base};
+            rows[s.query_begin + q] = RowInfo{s.n_tiles, s.index_base, 0u, 128u};
         }
         wide = wide && (s.n_queries >= 16 || s.n_tiles == 0);
         total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
@@ -334,12 +334,34 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
         cuts.add(s, wide ? WIDE_NQ : 4);
     }
     cuts.finish();
+    // Where the scores go: rows one behind the other, or where the 64-row kernel writes them, a block of 128 tiles' scores of all the item's rows together.
+    p->row_stride = ((uint64_t)longest + 31) / 32 * 32;
+    uint64_t floats = nq * p->row_stride;
+    if (wide) {
+        floats = 0;
+        size_t at = 0;
+        for (size_t i = 0; i < n_segs; ++i)
+            for (uint32_t q0 = 0; q0 < segs[i].n_queries && segs[i].n_tiles; q0 += WIDE_NQ) {
+                const uint32_t m = std::min<uint32_t>(WIDE_NQ, segs[i].n_queries - q0);
+                for (uint32_t q = 0; q < m; ++q) {
+                    rows[segs[i].query_begin + q0 + q].begin = (uint32_t)(floats + 128 * q);
+                    rows[segs[i].query_begin + q0 + q].step = 128 * m;
+                }
+                for (uint64_t done = 0; done < segs[i].n_tiles; ++at) {  // (the cuts of this stream, in order)
+                    cuts.items[at].list_begin = (uint32_t)floats;
+                    cuts.items[at].pad = 128 * m;
+                    done += cuts.items[at].n_tiles;
+                }
+                floats += (uint64_t)(segs[i].n_tiles + 127) / 128 * 128 * m;
+            }
+    } else {
+        for (size_t q = 0; q < nq; ++q) rows[q].begin = (uint32_t)(q * p->row_stride);
+    }
     Blob tables;
     const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows);
     SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
     SLHA_TRY(p->b_gpivot.ensure(4 * nq * 4));
-    p->row_stride = ((uint64_t)longest + 31) / 32 * 32;
-    SLHA_TRY(p->b_gbuf.ensure(nq * p->row_stride * 4));
+    SLHA_TRY(p->b_gbuf.ensure(floats * 4));
     unsigned char* dev = static_cast<unsigned char*>(p->b_tables.p);
     SLHA_TRY(ctx_copy_table(c, dev, tables.bytes.data(), tables.bytes.size()));
     p->d_row_flags = (uint32_t*)p->b_gpivot.p;
@@ -1032,6 +1054,7 @@ static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, con
     a.n_items = p->n_items;
     a.cta_begin = p->d_cta_begin;
     if (p->wide) {
+        a.blocked = 1u;
         a.handoff = p->d_row_flags + nq;
         a.handoff_as = 2u;
         SLHA_TRY(launch_wide_dense(c, a, p->mma_grid, true));
@@ -1040,7 +1063,7 @@ static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, con
     }
     SLHA_TRY(launch_dense(c, a, p->mma_grid, true));
     if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));
-    RowsArgs r{a.scores, p->row_stride, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, p->kp2, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
+    RowsArgs r{a.scores, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, p->kp2, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
     SLHA_TRY(launch_rows(c, r, (uint32_t)nq, p->longest));
     if (timed) {
         SLHA_CUDA(cudaEventRecord(tev[2], c->stream));

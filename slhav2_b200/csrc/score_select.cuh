@@ -17,10 +17,10 @@ constexpr uint32_t ROW_ABSENT = 0xFFFFFFFFu;      // bits of a score that is not
 constexpr int row_own(int r) { return 4 * r < 16 ? 4 * r : 16; }  // candidates a thread keeps
 struct RowInfo {
     uint32_t n, index_base;  // scores of the row, reported index of the first
+    uint32_t begin, step;    // where they lie: 128 from begin on, the next 128 `step` further, ..
 };
 struct RowsArgs {
-    const float* scores;     // row q starts at q * stride
-    uint64_t stride;
+    const float* scores;
     const RowInfo* rows;
     uint32_t* flag;          // [nq] a work item of the row took the generic arithmetic, [nq] it was handed on by the 64-row kernel (cleared here)
     uint32_t* stats;         // [nq][2] candidates, the flag
@@ -48,11 +48,11 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket, 4 a thread holds too many, 8.. of a selection step, 16.. warp totals
     const RowInfo info = a.rows[Q];
     const uint32_t n = info.n;
-    const float* row = a.scores + (size_t)Q * a.stride;
+    const float* row = a.scores + info.begin;
     // thread t holds the scores 4 (t + NT j) .. + 3
     auto load4 = [&](int j) {
         const uint32_t e = 4u * (tid + (uint32_t)NT * j);
-        uint4 x = e < n ? __ldcg(reinterpret_cast<const uint4*>(row + e)) : make_uint4(ROW_ABSENT, ROW_ABSENT, ROW_ABSENT, ROW_ABSENT);
+        uint4 x = e < n ? __ldcg(reinterpret_cast<const uint4*>(row + (size_t)(e >> 7) * info.step + (e & 127u))) : make_uint4(ROW_ABSENT, ROW_ABSENT, ROW_ABSENT, ROW_ABSENT);
         if (e + 3u >= n) {
             if (e + 1u >= n) x.y = ROW_ABSENT;
             if (e + 2u >= n) x.z = ROW_ABSENT;

@@ -122,15 +122,21 @@ __device__ __forceinline__ void nib_word(uint32_t w, const NibScale& s, uint32_t
     o[2] = hfma2_u32(x & 0x000F000Fu, s.g8, s.c);
     o[3] = hfma2_u32(x & 0x00F000F0u, s.g4, s.c);
 }
-// eight 3-bit codes (24 bits) and their correction bits (8 bits) -> a word of nibbles 2 code + bit
+// eight 3-bit codes (the low 24 bits) and their correction bits (the low 8) -> a word of nibbles 2 code + bit.  Every step moves the upper half of each field and takes
+// the rest as it is, one LOP3 a step (x where the mask is set, else y); what that leaves between the fields never reaches a place that the last step keeps.
+__device__ __forceinline__ uint32_t bit_select(uint32_t x, uint32_t y, uint32_t mask) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0xE2;\n" : "=r"(d) : "r"(x), "r"(mask), "r"(y));
+    return d;
+}
 __device__ __forceinline__ uint32_t code3_nibbles(uint32_t x, uint32_t c) {
-    x = (x & 0xFFFu) | ((x & 0xFFF000u) << 4);
-    x = (x & 0x003F003Fu) | ((x & 0x0FC00FC0u) << 2);
-    x = (x & 0x07070707u) | ((x & 0x38383838u) << 1);
-    c = (c | (c << 12)) & 0x000F000Fu;
-    c = (c | (c << 6)) & 0x03030303u;
-    c = (c | (c << 3)) & 0x11111111u;
-    return (x << 1) | c;
+    x = bit_select(x, x << 4, 0x00000FFFu);
+    x = bit_select(x, x << 2, 0x003F003Fu);
+    x = bit_select(x, x << 1, 0x07070707u);
+    c = bit_select(c, c << 12, 0x0000000Fu);
+    c = bit_select(c, c << 6, 0x00030003u);
+    c = bit_select(c, c << 3, 0x01010101u);
+    return bit_select(x << 1, c, 0xEEEEEEEEu);
 }
 // four head bytes b -> (b - 128) gh 2^(U + 4) (two columns) and (b - 128) gl 2^U (two columns), gh / gl the nibbles of the
 // head's scale byte, U = -16 (mixed) or -15 (MIX3, whose other levels are kept halved): products below 2048, exact in fp16
@@ -179,7 +185,7 @@ __device__ __forceinline__ void st_fold_row(uint32_t row, uint32_t ta, uint32_t 
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
                 const int bit = 96 * Q + 24 * m, wi = bit >> 5, sh = bit & 31;
-                w[m] = code3_nibbles(__funnelshift_r(words[wi], words[wi + 1], sh) & 0xFFFFFFu, (cr >> (8 * m)) & 0xFFu);
+                w[m] = code3_nibbles(__funnelshift_r(words[wi], words[wi + 1], sh), cr >> (8 * m));
             }
         } else if (KIND == 4) {
             if (Q == 0) {
@@ -190,8 +196,8 @@ __device__ __forceinline__ void st_fold_row(uint32_t row, uint32_t ta, uint32_t 
             for (int m = Q == 0 ? 2 : 0; m < 4; ++m) {
                 const int j = 4 * Q + m - 2;  // code word j: dims 8 + 8 j .., codes at bit 64 + 24 j, correction bits at bit 400 + 8 j
                 const int bit = 64 + 24 * j, wi = bit >> 5, sh = bit & 31, cb = 400 + 8 * j;
-                const uint32_t cr = nocorr ? 0u : (words[cb >> 5] >> (cb & 31)) & 0xFFu;
-                w[m] = code3_nibbles(__funnelshift_r(words[wi], words[wi + 1 < 16 ? wi + 1 : 15], sh) & 0xFFFFFFu, cr);
+                const uint32_t cr = nocorr ? 0u : words[cb >> 5] >> (cb & 31);
+                w[m] = code3_nibbles(__funnelshift_r(words[wi], words[wi + 1 < 16 ? wi + 1 : 15], sh), cr);
             }
         } else {
             const uint4 L = Q == 0 ? lds_v4<0>(row) : (Q == 1 ? lds_v4<16>(row) : (Q == 2 ? lds_v4<32>(row) : lds_v4<48>(row)));
@@ -509,8 +515,10 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
             const uint32_t Q = it.query_begin + (uint32_t)min(q, nq - 1);
-            rowp[q] = !DENSE ? nullptr : a.scores + (a.row_offset ? (size_t)a.row_offset[Q] : (size_t)Q * a.score_stride) + it.index_base;
+            rowp[q] = !DENSE ? nullptr : a.blocked ? a.scores + it.list_begin + 128u * (uint32_t)q + (size_t)(it.index_base >> 7) * it.pad
+                                                   : a.scores + (a.row_offset ? (size_t)a.row_offset[Q] : (size_t)Q * a.score_stride) + it.index_base;
         }
+        const uint32_t row_step = DENSE && a.blocked ? it.pad : (uint32_t)ST_M;  // from a block's scores of a row to the next block's
 #pragma unroll
         for (int i = 0; i < ST_DEPTH - 1; ++i) issue();
         if (warp == 9 && lane < 4) qmax[lane] = 0u;  // (read last in the set-up of the item before)
@@ -714,7 +722,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
                     // 256 - 2 h without an integer conversion: (2^23 + h) as a bit pattern, times -2, plus 2^24 + 256 (exact)
                     const float sc = fmaf(c[q], su, lam * fmaf(__uint_as_float(0x4B000000u | popc8_words(d)), -2.0f, 16777472.0f));
                     // (the 32 lanes of a warp hold 32 consecutive tiles: one 128-byte run per row)
-                    if (t0 < n) rowp[q][t0] = live ? sc : __uint_as_float(a.cold_bits);
+                    if (t0 < n) rowp[q][(size_t)b * row_step + (uint32_t)(wq * ST_WT + lane)] = live ? sc : __uint_as_float(a.cold_bits);
                 }
                 continue;
             }

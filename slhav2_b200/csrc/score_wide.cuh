@@ -38,9 +38,12 @@ constexpr int WIDE_S_BYTES = 4 * WIDE_SLAB;         // signs: K = 256
 constexpr int WIDE_RAW = 128 * ST_ROW;              // one staged block
 constexpr int WIDE_RING = 3;
 constexpr int WIDE_Q_BYTES = WIDE_NQ * D_C * 4;     // the item's queries in fp32 (item set-up only)
+constexpr int WIDE_OUT_BYTES = WIDE_NQ * 128 * 4;   // dense: a block's scores on their way out, a row of them per query; two of these, over the queries
 constexpr int WIDE_TAIL = 2048 + 256 + 512 + 512 + 512 + 64 + 2048;  // sign words, threshold keys, sign sums and scales, mappings (2), barrier + flags, minima and maxima / row offsets
 constexpr uint32_t WIDE_A_SIGN = 128, WIDE_D = 256;                   // TMEM columns: A latent 0..71, A signs 128..255, accumulators 256.. and 384..
-constexpr size_t wide_smem_bytes() { return 1024 + 2 * WIDE_B_BYTES + WIDE_S_BYTES + WIDE_Q_BYTES + WIDE_RING * WIDE_RAW + WIDE_TAIL; }
+constexpr size_t wide_smem_bytes(bool dense) {
+    return 1024 + 2 * WIDE_B_BYTES + WIDE_S_BYTES + (dense ? 2 * WIDE_OUT_BYTES : WIDE_Q_BYTES) + WIDE_RING * WIDE_RAW + WIDE_TAIL;
+}
 
 // Threshold refresh of NR consecutive query rows by one warp (all loads of the NR histograms in flight
 // together): the lower edge of the highest bucket whose count from the top reaches k, minus half a
@@ -121,17 +124,17 @@ template <int KIND, bool DENSE>
 __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* smem_raw, uint32_t first_item) {
     constexpr int ACCS = KIND == 4 ? 3 : 1;                            // coarse accumulators
     constexpr uint32_t SIGN_AT = 64u * ACCS, FLIP = ACCS == 1 ? 128u : 0u;  // the signs' columns behind them; the second set of both
-    // shared layout (1024-byte aligned base): B hi | B lo | signs | raw ring | queries | tail
+    // shared layout (1024-byte aligned base): B hi | B lo | signs | raw ring | queries, later (dense) scores on their way out | tail
     const uint32_t base_s = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
     unsigned char* base = smem_raw + (base_s - (uint32_t)__cvta_generic_to_shared(smem_raw));
-    constexpr uint32_t S_OFF = 2 * WIDE_B_BYTES, RAW_OFF = S_OFF + WIDE_S_BYTES, Q_OFF = RAW_OFF + WIDE_RING * WIDE_RAW, TAIL_OFF = Q_OFF + WIDE_Q_BYTES;
-    const uint32_t B_s = base_s, S_s = base_s + S_OFF, raw_s = base_s + RAW_OFF;
+    constexpr uint32_t S_OFF = 2 * WIDE_B_BYTES, RAW_OFF = S_OFF + WIDE_S_BYTES, Q_OFF = RAW_OFF + WIDE_RING * WIDE_RAW, TAIL_OFF = Q_OFF + (DENSE ? 2 * WIDE_OUT_BYTES : WIDE_Q_BYTES);
+    const uint32_t B_s = base_s, S_s = base_s + S_OFF, raw_s = base_s + RAW_OFF, out_s = base_s + Q_OFF;
     float* qf = reinterpret_cast<float*>(base + Q_OFF);             // [64][128]
     unsigned char* tail = base + TAIL_OFF;
     uint32_t* qs_w = reinterpret_cast<uint32_t*>(tail);            // [64][8]
     uint32_t* pvh = qs_w + 512;                                     // [64] score word of the row's threshold
-    float2* uq = reinterpret_cast<float2*>(pvh + 64);               // [64] (sum of the row's signs, inverse of the row's scale times the unit of A)
-    float2* rng = uq + 64;                                          // [64] (smin, inv)
+    float* uq = reinterpret_cast<float*>(pvh + 64);                 // [64] sums of the rows' signs, [64] inverses of the rows' scales times the unit of A
+    float2* rng = reinterpret_cast<float2*>(uq + 128);                                          // [64] (smin, inv)
     float2* rmap = rng + 64;                                        // [64] (-smin inv, inv)
     uint32_t* ctl = reinterpret_cast<uint32_t*>(rmap + 64);         // mbarrier (8 bytes), [4] TMEM base, [5] error flag, [6] bail
     float2* colmm = reinterpret_cast<float2*>(ctl + 16);            // [4][64] per tile quarter: (min, max) score of a column
@@ -199,11 +202,11 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
                 big |= largest >= SPLIT_MOST;
                 const float2 f = split_scale(largest, 14);
                 reinterpret_cast<float4*>(qf)[32 * r + lane] = make_float4(x[i].x * f.x, x[i].y * f.x, x[i].z * f.x, x[i].w * f.x);
-                if (lane == 0) uq[r].y = f.y * (EXTRA ? 32768.0f : 65536.0f);
+                if (lane == 0) uq[64 + r] = f.y * (EXTRA ? 32768.0f : 65536.0f);
             }
         }
         qs_w[tid] = (tid >> 3) < nq ? a.q_sign[(size_t)(it.query_begin + (tid >> 3)) * 8 + (tid & 7)] : 0u;
-        if (DENSE && tid < WIDE_NQ) roff[tid] = tid >= nq ? 0ull : (a.row_offset ? a.row_offset[it.query_begin + tid] : (it.query_begin + tid) * a.score_stride);
+        if (DENSE && tid < WIDE_NQ) roff[tid] = tid >= nq || a.blocked ? 0ull : a.row_offset[it.query_begin + tid];
         if (!DENSE && tid < WIDE_NQ) {
             const bool have = tid < nq;
             const unsigned long long pv = have ? *reinterpret_cast<volatile unsigned long long*>(a.gpivot + it.query_begin + tid) : ~0ull;
@@ -213,6 +216,20 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             rmap[tid] = make_float2(-rng[tid].x * rng[tid].y, rng[tid].y);
         }
         __syncthreads();
+        constexpr uint32_t SUMS = WIDE_NQ * D_C;  // behind the queries: [64][8] a sixteenth of their sums over the groups (a group a thread; MIX3: group g is dims 16 g - 8 ..)
+        if (EXTRA && DENSE) {
+            const int r = tid >> 3, g = tid & 7;
+            const float* qg = qf + r * D_C + (KIND == 4 ? 16 * g - 8 : 16 * g);
+            float s = 0.0f;
+            if (KIND == 2 || g)
+#pragma unroll
+                for (int d = 0; d < 16; d += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(qg + d);
+                    s = s + x.x + x.y + x.z + x.w;
+                }
+            qf[SUMS + tid] = 0.0625f * s;
+            __syncthreads();
+        }
         // B rows = queries, K-major, 128-byte swizzle (16-byte chunk i of row r at chunk i ^ (r & 7) of its line); the order of the
         // k slots is that of nib_word / head_word / scale_pair
         for (int u = tid; u < WIDE_NQ * 18; u += WIDE_THREADS) {
@@ -229,8 +246,8 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             } else {
 #pragma unroll
                 for (int g = 0; g < 8; ++g) {
-                    v[g] = 0.0f;
-                    if (i == 16 && EXTRA && (KIND == 2 || g)) {
+                    v[g] = i == 16 && EXTRA && DENSE ? qf[SUMS + 8 * r + g] : 0.0f;
+                    if (i == 16 && EXTRA && !DENSE && (KIND == 2 || g)) {
                         const float* qg = q + (KIND == 4 ? 16 * g - 8 : 16 * g);
                         float s = 0.0f;
                         for (int d = 0; d < 16; d += 4) {
@@ -265,7 +282,7 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         if (tid < WIDE_NQ) {
             int c = 0;
             for (int w = 0; w < 8; ++w) c += __popc(qs_w[8 * tid + w]);
-            uq[tid].x = (float)(256 - 2 * c);
+            uq[tid] = (float)(256 - 2 * c);
         }
         if (big) ctl[6] = 1u;
         asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");  // B was written with ordinary stores, the MMA reads it through the async proxy
@@ -293,7 +310,9 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             }
             asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-            asm volatile("bar.sync 2, 512;\n" ::: "memory");
+            // (only the issuing warp waits for the others: a barrier of its own, since the others may be at the next one by then)
+            if (uw == 0) asm volatile("bar.sync 3, 512;\n" ::: "memory");
+            else asm volatile("bar.arrive 3, 512;\n" ::: "memory");
             if (leader) {
                 asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
                 const uint32_t dt = tmem + WIDE_D + FLIP * (b & 1u);
@@ -311,6 +330,14 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             }
             __syncwarp();
         };
+        // A block's scores of a plan of whole rows, where they lie together, leave shared memory by one bulk copy (a store a score keeps the load-store unit busy for 1300 cycles
+        // a block, the tiles' reads behind them; a bulk copy takes the copy engine 35 cycles to accept, so one for each of 64 rows would be no faster).
+        auto send = [&](uint32_t b) {
+            if (tid != WIDE_THREADS - 32) return;
+            float* const to = a.scores + it.list_begin + (size_t)((it.index_base >> 7) + b) * it.pad;
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;\ncp.async.bulk.commit_group;\n" ::"l"(to), "r"(out_s + (b & 1u) * WIDE_OUT_BYTES),
+                         "r"((uint32_t)nq * 512u) : "memory");
+        };
         const int r = 32 * qt + lane;
         const bool cols = 16 * ch < nq;  // this warp has query columns in this item
         const uint32_t Q0 = it.query_begin + 16u * (uint32_t)ch;
@@ -327,7 +354,10 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
             const bool ok = mbar_wait(bar_s, phase);
             phase ^= 1u;
             cp_async_wait<0>();  // this thread's copies of block b + 1
+            const bool turned = DENSE && a.blocked;
+            if (turned && tid == WIDE_THREADS - 32) asm volatile("cp.async.bulk.wait_group.read 0;\n" ::: "memory");  // (the copy out of the buffer that this block fills)
             if (role_any(1, WIDE_THREADS, !ok)) { stop = true; break; }
+            if (turned && b) send(b - 1);
             asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
             WPROBE_LAP(1);  // wait for the accumulators
             if (b + 2 < blocks) fetch(b + 2);
@@ -364,17 +394,30 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
                         }
                     }
                 }
+                const uint64_t su2 = f2_pack(su, su), lam2 = f2_pack(lam, lam);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float2 u = uq[16 * ch + j];
-                    const float h = fmaf(__uint_as_float(s[j]), -32768.0f, u.x);  // 256 - 2 hamming, exact
-                    sc[j] = fmaf(sc[j] * u.y, su, lam * h);  // (u.y is a power of two: the coarse term is rounded once)
+                for (int j = 0; j < 16; j += 4) {
+                    const ulonglong2 ux = *reinterpret_cast<const ulonglong2*>(uq + 16 * ch + j), uy = *reinterpret_cast<const ulonglong2*>(uq + 64 + 16 * ch + j);
+#pragma unroll
+                    for (int p = 0; p < 2; ++p) {
+                        const uint64_t h = f2_fma(u2_pack(s[j + 2 * p], s[j + 2 * p + 1]), 0xC7000000C7000000ull, p ? ux.y : ux.x);  // 256 - 2 hamming, exact (-32768 s + u)
+                        // (uy is a power of two: the coarse term is rounded once)
+                        const uint64_t r2 = f2_fma(f2_mul(f2_pack(sc[j + 2 * p], sc[j + 2 * p + 1]), p ? uy.y : uy.x), su2, f2_mul(lam2, h));
+                        asm("mov.b64 {%0, %1}, %2;\n" : "=f"(sc[j + 2 * p]), "=f"(sc[j + 2 * p + 1]) : "l"(r2));
+                    }
                 }
             }
             if (ACCS > 1 && b + 1 < blocks) stage(b + 1);  // (its barrier: every warp has read this block's accumulators)
             asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
             if (DENSE) {
-                if (cols) {
+                if (turned) {
+                    const uint32_t to = out_s + (b & 1u) * WIDE_OUT_BYTES + (uint32_t)(16 * ch * 128 + r) * 4u;
+                    if (cols) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) asm volatile("st.shared.f32 [%0], %1;\n" ::"r"(to + (uint32_t)(j * 512)), "f"(sc[j]) : "memory");
+                        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+                    }
+                } else if (cols) {
 #pragma unroll
                     for (int j = 0; j < 16; ++j) {
                         const int q = 16 * ch + j;
@@ -500,6 +543,10 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         if (warp == 0) WPROBE_OUT(0, 12);
         if (stop && tid == 0) ctl[5] = 1u;
         __syncthreads();
+        if (DENSE && a.blocked && blocks && !stop) {
+            send(blocks - 1);
+            if (tid == WIDE_THREADS - 32) asm volatile("cp.async.bulk.wait_group 0;\n" ::: "memory");  // (the next item's first block fills a buffer behind its barriers)
+        }
         // rows this CTA could not score (another codec, a query outside the fp16 split, a wait that ran out) go to the generic kernel, of a dense call to
         // the four-row kernel
         if ((*reinterpret_cast<volatile uint32_t*>(ctl + 6) || stop) && tid < nq) (DENSE ? a.handoff : a.gflag)[it.query_begin + tid] = DENSE ? a.handoff_as : 1u;
