@@ -32,21 +32,24 @@ struct RowsArgs {
 // slots: what a sample's bound lets through, see below, and kp2 winners
 inline uint32_t row_cap(uint32_t k, uint32_t kp2) { return std::max(kp2, std::min(4u * k + 1024u, 2u * k + 2560u)); }
 constexpr int ROW_HIST_INTS = ROW_BUCKETS + 64;
-inline size_t row_smem(uint32_t cap, int nt, int r) { return (size_t)cap * 8 + (size_t)nt * row_own(r) * 8 + (size_t)(ROW_HIST_INTS + 64) * 4; }
+// (the threads' own lists make room for the candidates by buckets)
+__host__ __device__ constexpr size_t row_own_slots(uint32_t cap, int nt, int r) { return (size_t)nt * row_own(r) > cap ? (size_t)nt * row_own(r) : cap; }
+inline size_t row_smem(uint32_t cap, int nt, int r) { return ((size_t)cap + row_own_slots(cap, nt, r)) * 8 + (size_t)(ROW_HIST_INTS + 64) * 4 + (size_t)(cap + 1) / 2 * 4; }
+constexpr uint32_t ROW_RANKED = 192;              // candidates that are ordered by comparing each with all
 
 // R: 4 R scores a thread, n <= 4 R x threads
 template <int NT, int R>
 __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
+    const RowInfo info = a.rows[blockIdx.x];  // (the plan's: no kernel writes it)
     dep_launch();
     dep_wait();
     constexpr int OWN = row_own(R), PER = ROW_BUCKETS / NT;
     const uint32_t k = a.k, cap = a.cap, Q = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem);                     // [cap]
-    uint64_t* own = buf + cap + tid;                                       // [OWN], NT apart
-    int* hist = reinterpret_cast<int*>(buf + cap + NT * OWN);              // [ROW_BUCKETS + 1]
+    uint64_t* own = buf + cap + tid;                                       // [OWN], NT apart; then the candidates' places in their buckets
+    int* hist = reinterpret_cast<int*>(buf + cap + row_own_slots(cap, NT, R));  // [ROW_BUCKETS + 1]
     uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket, 4 a thread holds too many, 8.. of a selection step, 16.. warp totals
-    const RowInfo info = a.rows[Q];
     const uint32_t n = info.n;
     const float* row = a.scores + info.begin;
     // thread t holds the scores 4 (t + NT j) .. + 3
@@ -170,8 +173,21 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
                 asm volatile("" : "+r"(mine) : : "memory");
             }
         }
-        const uint32_t sum = __reduce_add_sync(0xFFFFFFFFu, mine);
-        if (lane == 0 && sum) atomicAdd(&st[0], sum);
+        if (__any_sync(0xFFFFFFFFu, mine != 0u)) {
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= (uint32_t)o) incl += y;
+            }
+            uint32_t at = 0;
+            if (lane == 31) at = atomicAdd(&st[0], incl);
+            at = __shfl_sync(0xFFFFFFFFu, at, 31) + incl - mine;
+            for (uint32_t h = 0; h < min(mine, (uint32_t)OWN); ++h, ++at) {
+                const uint64_t e = own[h * NT];
+                if (at < cap) buf[at] = make_comp(__uint_as_float((uint32_t)(e >> 32)), info.index_base + 4u * tid + (uint32_t)e);
+            }
+        }
         if (OWN < 4 * R && mine > (uint32_t)OWN) st[4] = 1u;
         __syncthreads();
         if (st[0] >= k || bound == -INFINITY) break;
@@ -183,19 +199,35 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     const uint32_t got = st[0], m = min(got, k);
     uint32_t* const out_index = a.out_index + (size_t)Q * k;
     float* const out_score = a.out_score + (size_t)Q * k;
-    if (got <= cap && (OWN == 4 * R || !st[4])) {
+    const bool listed = got <= cap && (OWN == 4 * R || !st[4]);
+    if (listed && got <= ROW_RANKED) {
+        // Few candidates: a candidate's place is the number of larger ones, counted by SPLIT threads in turn (a slice of the list each).
+        constexpr uint32_t SPLIT = 2;
+        const uint32_t i = tid / SPLIT, part = tid % SPLIT;
+        for (uint32_t c = i; c < got; c += NT / SPLIT) {
+            const uint64_t key = buf[c];
+            uint32_t r = 0;
+#pragma unroll 8
+            for (uint32_t x = part; x < got; x += SPLIT) r += buf[x] > key;
+            r += __shfl_xor_sync(3u << (lane & 30u), r, 1);
+            if (part == 0 && r < m) {
+                out_index[r] = 0xFFFFFFFFu - (uint32_t)key;
+                out_score[r] = key_score((uint32_t)(key >> 32));
+            }
+        }
+        for (uint32_t r = m + tid; r < k; r += NT) {
+            out_index[r] = 0xFFFFFFFFu;
+            out_score[r] = -INFINITY;
+        }
+    } else if (listed) {
         if (bound > low) low = bound;
         const float inv = (float)ROW_BUCKETS / (top - low);
         const bool apart = inv > 0.0f && inv < INFINITY;
-        auto bucket = [&](uint32_t bits) {
-            return apart ? min(max(__float2int_rz((top - __uint_as_float(bits)) * inv), 0), ROW_BUCKETS - 1) : 0;
-        };
-        for (uint32_t h = 0; h < mine; ++h) {
-            const uint64_t e = own[h * NT];
-            const int b = bucket((uint32_t)(e >> 32));
-            const int r = atomicAdd(&hist[b], 1);  // (any order inside the bucket)
-            own[h * NT] = e & 0xFFFFFFFF0000FFFFull | (uint64_t)r << 16;
-        }
+        auto bucket = [&](uint64_t key) { return apart ? min(max(__float2int_rz((top - key_score((uint32_t)(key >> 32))) * inv), 0), ROW_BUCKETS - 1) : 0; };
+        // placed[]: the candidates by buckets; a candidate's number in its bucket comes from the counting (any order)
+        uint64_t* const placed = buf + cap;
+        uint16_t* const number = reinterpret_cast<uint16_t*>(st + 64);
+        for (uint32_t i = tid; i < got; i += NT) number[i] = (uint16_t)atomicAdd(&hist[bucket(buf[i])], 1);
         __syncthreads();
         int c[PER], at = scan(c);
 #pragma unroll
@@ -205,18 +237,17 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         }
         if (tid == NT - 1) hist[ROW_BUCKETS] = at;
         __syncthreads();
-        for (uint32_t h = 0; h < mine; ++h) {
-            const uint64_t e = own[h * NT];
-            const uint32_t bits = (uint32_t)(e >> 32);
-            buf[hist[bucket(bits)] + (int)((uint32_t)e >> 16)] = make_comp(__uint_as_float(bits), info.index_base + 4u * tid + ((uint32_t)e & 0xFFFFu));
+        for (uint32_t i = tid; i < got; i += NT) {
+            const uint64_t key = buf[i];
+            placed[hist[bucket(key)] + (int)number[i]] = key;
         }
         __syncthreads();
         for (uint32_t i = tid; i < got; i += NT) {
-            const uint64_t key = buf[i];
-            const int b = bucket(__float_as_uint(key_score((uint32_t)(key >> 32))));
+            const uint64_t key = placed[i];
+            const int b = bucket(key);
             const int s0 = hist[b], e0 = hist[b + 1];
             uint32_t r = (uint32_t)s0;
-            for (int x = s0; x < e0; ++x) r += buf[x] > key;
+            for (int x = s0; x < e0; ++x) r += placed[x] > key;
             if (r < m) {
                 out_index[r] = 0xFFFFFFFFu - (uint32_t)key;
                 out_score[r] = key_score((uint32_t)(key >> 32));
