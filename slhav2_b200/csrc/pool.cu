@@ -444,6 +444,307 @@ __device__ __forceinline__ uint64_t block_cut(const uint64_t (&k)[N], uint64_t r
     }
 }
 
+// Shared memory of a phase's end (block 0) and of what the blocks do before it.
+struct FinishShared {
+    using Sort = cub::BlockRadixSort<uint64_t, EB_THREADS, EB_ITEMS, uint32_t>;
+    using Scan64 = cub::BlockScan<uint64_t, EB_THREADS>;
+    union {
+        typename Sort::TempStorage sort;
+        typename Scan64::TempStorage scan64;
+        typename EbScan32::TempStorage scan32;
+        uint32_t hist[EB_BINS];
+        struct { uint64_t in[EB_THREADS], key[EB_THREADS]; uint32_t val[EB_THREADS]; } few;
+        CutShared cut;
+    };
+    unsigned long long applied;  // of the phase that ended
+    long long delta;
+    uint32_t n;
+};
+// The end of a phase, by one block: the candidates ks / vs [0 .. n), n <= EB_CAP, in order, the operation on exactly the prefix that the reference's loop reaches.  sm.applied and
+// sm.delta: what was evicted, and the change of the live bytes.  CUT: for lists of the blocks' smallest keys, of which few are reached (skeys, svals: room for them).
+template <bool CUT>
+__device__ __forceinline__ void finish_phase(const PoolDev& p, int phase, uint64_t reach, uint64_t deficit, uint64_t free0, const uint64_t* ks, const uint32_t* vs, uint32_t n, uint64_t* skeys,
+                                             uint32_t* svals, FinishShared& sm) {
+    const int lane = threadIdx.x & 31;
+    uint64_t k[EB_ITEMS];
+    uint32_t v[EB_ITEMS];
+#pragma unroll
+    for (int j = 0; j < EB_ITEMS; ++j) {
+        const uint32_t i = threadIdx.x * EB_ITEMS + j;
+        k[j] = i < n ? ks[i] : SENTINEL;
+        v[j] = i < n ? vs[i] : 0u;
+    }
+    if (CUT && n > EB_THREADS && reach <= EB_THREADS / 2) {  // the blocks' smallest keys together: down to what the count below orders
+        uint32_t kept;
+        const uint64_t bound = block_cut(k, reach, EB_THREADS / 2, sm.cut, kept);
+        if (kept <= EB_THREADS) {
+            if (threadIdx.x == 0) sm.n = 0u;
+            __syncthreads();
+#pragma unroll
+            for (int j = 0; j < EB_ITEMS; ++j)
+                if (k[j] != SENTINEL && k[j] <= bound) {
+                    const uint32_t o = atomicAdd(&sm.n, 1u);
+                    skeys[o] = k[j];  // (every key has been read: block_cut's barriers)
+                    svals[o] = v[j];
+                }
+            __syncthreads();
+            ks = skeys;
+            vs = svals;
+            n = kept;
+        }
+    }
+    if (threadIdx.x == 0) {
+        sm.applied = 0;
+        sm.delta = 0;
+    }
+    __syncthreads();
+    int64_t delta = 0;
+    uint32_t applied = 0;
+    auto weight = [&](uint64_t key, uint32_t slot) -> uint64_t {
+        if (key == SENTINEL) return 0;
+        const uint32_t flags = tile_flags(p.tiles, slot);
+        return phase == PH_PAGE ? 32 : phase <= PH_CORR_WARM ? corr_bytes(flags) : live_bytes_of(p.state[slot], flags);
+    };
+    auto apply = [&](uint64_t key, uint32_t slot, uint64_t bytes, uint64_t before, uint32_t place) {
+        if (key == SENTINEL || before >= deficit) return;
+        if (phase == PH_PAGE) {
+            do_page_out(p, slot, &delta);
+        } else if (phase <= PH_CORR_WARM) {
+            do_drop_correction(p, slot, &delta);
+        } else {
+            delta -= (int64_t)bytes;
+            p.state[slot] = ST_COLD;
+            p.free_list[free0 + place] = slot;  // applied items are a prefix of the sorted order
+            ++applied;
+        }
+    };
+    if (n <= EB_THREADS) {
+        // few candidates (a decode step's page-outs and evictions): every thread counts the keys below its own
+        // (keys are unique), n reads of shared memory instead of the radix sort's sixteen passes, and goes on with one of them in order
+        const uint32_t i = threadIdx.x;
+        const uint64_t own = i < n ? ks[i] : SENTINEL;
+        sm.few.in[i] = own;
+        __syncthreads();
+        uint32_t rank = 0;
+#pragma unroll 8
+        for (uint32_t e = 0; e < n; ++e) rank += sm.few.in[e] < own;
+        if (i < n) {
+            sm.few.key[rank] = own;
+            sm.few.val[rank] = vs[i];
+        }
+        __syncthreads();
+        const uint64_t key = i < n ? sm.few.key[i] : SENTINEL;
+        const uint32_t slot = i < n ? sm.few.val[i] : 0u;
+        const uint64_t bytes = weight(key, slot);
+        uint64_t before;
+        __syncthreads();
+        FinishShared::Scan64(sm.scan64).ExclusiveSum(bytes, before);
+        apply(key, slot, bytes, before, i);
+    } else {
+        FinishShared::Sort(sm.sort).Sort(k, v);
+        __syncthreads();
+        uint64_t w[EB_ITEMS], excl[EB_ITEMS];
+#pragma unroll
+        for (int j = 0; j < EB_ITEMS; ++j) w[j] = weight(k[j], v[j]);
+        FinishShared::Scan64(sm.scan64).ExclusiveSum(w, excl);
+#pragma unroll
+        for (int j = 0; j < EB_ITEMS; ++j) apply(k[j], v[j], w[j], excl[j], threadIdx.x * EB_ITEMS + j);
+    }
+    for (int o = 16; o; o >>= 1) {
+        delta += __shfl_xor_sync(0xFFFFFFFFu, delta, o);
+        applied += __shfl_xor_sync(0xFFFFFFFFu, applied, o);
+    }
+    if (lane == 0) {
+        if (delta) atomicAdd((unsigned long long*)&sm.delta, (unsigned long long)delta);
+        if (applied) atomicAdd(&sm.applied, (unsigned long long)applied);
+    }
+    __syncthreads();
+}
+
+// A decode step's budget question in one pass over the slots: no correction planes in the pool, few HOT tiles to page out, few evictions.  Paging every HOT tile
+// frees 32 bytes each, so all blocks know the evictions' deficit as soon as they know how many there are, and the states, positions and the largest position come
+// from the same loads: three grid barriers and one end instead of seven and two, and the host reads the answer from its own memory instead of waiting for the end and for
+// two copies.  Latency bounds it: barriers, a scan whose loads are all in flight at once, and one block's ordering of a few hundred keys.  us of the whole
+// call, 8 tiles appended and 8 evicted, with enforce_kernel and with this one: by importance 20 000 slots 94 / 32, 100 000 81 / 42, 1 000 000 132 / 62; in
+// causal order 69 / 32, 81 / 35, 121 / 37.  Whatever does not fit is left to enforce_kernel, with nothing changed: that costs the first scan, so the host
+// also asks what it knows before (see there).
+constexpr uint32_t STEP_BAIL = 1u;                  // a flag of the answer: nothing was done
+struct StepState {                                  // zero when the kernel starts, and again when it ends
+    struct {
+        unsigned long long bound_inv, bound_low;    // ~bound of the candidates and the largest of the blocks' smallest keys, see enforce_kernel
+        uint32_t few_n, all_n;                      // how many lie within it, and how many there are
+    } set[2];                                       // tiles that are not pinned, then those that are
+    uint32_t hot_n, max_pos;
+};
+struct StepAnswer {                                 // page-locked host memory
+    uint64_t live, free_len;
+    uint64_t hot;                                   // HOT tiles left
+    uint32_t flags, no;                             // no: the call's number, written last
+};
+__global__ void __launch_bounds__(EB_THREADS) enforce_step_kernel(PoolDev p, uint64_t* hkeys, uint32_t* hvals, uint64_t* skeys, uint32_t* svals, StepState* ss,
+                                                                  volatile StepAnswer* answer, uint32_t no) {
+    namespace cg = cooperative_groups;
+    cg::grid_group grid = cg::this_grid();
+    __shared__ FinishShared sm;
+    __shared__ uint32_t warp_n[EB_THREADS / 32];
+    volatile PoolCounters* cnt = p.cnt;
+    const uint64_t len = cnt->len, live = cnt->live, budget = cnt->budget, free0 = cnt->free_len;
+    const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto say = [&](uint64_t live_now, uint64_t free_now, uint64_t hot, uint32_t flags) {  // block 0's first thread, when nobody reads *ss any more
+        *ss = StepState{};
+        answer->live = live_now;
+        answer->free_len = free_now;
+        answer->hot = hot;
+        answer->flags = flags;
+        __threadfence_system();
+        answer->no = no;
+    };
+    if (live <= budget) {
+        if (gtid == 0) say(live, free0, ~0ull, 0u);
+        return;
+    }
+    const bool by_importance = p.evict_policy == SLHA_B200_EVICT_IMPORTANCE, low_impact = p.page_policy == SLHA_B200_PAGE_LOWEST_IMPACT_FIRST;
+    uint8_t st[EB_KEYS];
+    uint32_t pos[EB_KEYS];
+#pragma unroll
+    for (int u = 0; u < EB_KEYS; ++u) st[u] = gtid + u * stride < len ? p.state[gtid + u * stride] : ST_COLD;
+#pragma unroll
+    for (int u = 0; u < EB_KEYS; ++u) pos[u] = by_importance && st[u] != ST_COLD ? *reinterpret_cast<const uint32_t*>(p.tiles + (gtid + u * stride) * TILE_BYTES + 112) : 0u;
+    uint32_t m = 0;
+#pragma unroll
+    for (int u = 0; u < EB_KEYS; ++u) m = max(m, pos[u]);
+#pragma unroll 1
+    for (int u = 0; u < EB_KEYS; ++u) {
+        uint8_t own = st[0];
+#pragma unroll
+        for (int j = 1; j < EB_KEYS; ++j) own = u == j ? st[j] : own;
+        const bool hot = own == ST_HOT;
+        const unsigned hit = __ballot_sync(0xFFFFFFFFu, hot);
+        if (!hit) continue;
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(&ss->hot_n, (uint32_t)__popc(hit));
+        at = __shfl_sync(0xFFFFFFFFu, at, 0) + (uint32_t)__popc(hit & ((1u << lane) - 1u));
+        if (hot && at < (uint32_t)EB_CAP) {
+            const uint64_t s = gtid + u * stride;
+            hkeys[at] = low_impact ? ((uint64_t)f32_total_key(*reinterpret_cast<const float*>(p.tiles + s * TILE_BYTES + 104)) << 32) | (uint32_t)s : (uint64_t)(uint32_t)p.seq[s];
+            hvals[at] = (uint32_t)s;
+        }
+    }
+    if (p.recent_window) {
+        m = __reduce_max_sync(0xFFFFFFFFu, m);
+        if (lane == 0) warp_n[warp] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < EB_THREADS / 32; ++w) m = max(m, warp_n[w]);
+            if (m) atomicMax(&ss->max_pos, m);
+        }
+    }
+    grid.sync();
+    const uint32_t hot_n = *(volatile uint32_t*)&ss->hot_n, max_pos = *(volatile uint32_t*)&ss->max_pos;
+    const uint64_t deficit = live - budget, paged = 32ull * hot_n;
+    const bool evicts = paged < deficit;
+    const uint64_t rest = evicts ? deficit - paged : 0, reach = rest / 80 + 1;
+    const bool fits = hot_n <= (uint32_t)EB_CAP && !(evicts && reach * gridDim.x > 4ull * EB_CAP);
+    if (!fits || !evicts) {  // (the same for every block)
+        grid.sync();         // the counts have been read
+        if (blockIdx.x) return;
+        if (fits) finish_phase<false>(p, PH_PAGE, deficit / 32 + 1, deficit, free0, hkeys, hvals, hot_n, skeys, svals, sm);
+        if (threadIdx.x == 0) {
+            const uint64_t live_now = fits ? (uint64_t)((int64_t)live + sm.delta) : live;
+            if (fits) cnt->live = live_now;
+            say(live_now, free0, hot_n - (live - live_now) / 32, fits ? 0u : STEP_BAIL);
+        }
+        return;
+    }
+    // Pinned tiles go last (by importance only), and only where the others free too little: 96 bytes each, once they are paged.
+    uint32_t got[2] = {0u, 0u};
+#pragma unroll 1
+    for (int pinned = 0; pinned < 2; ++pinned) {
+        uint64_t key[EB_KEYS];
+        float imp[EB_KEYS];
+        uint32_t seq[EB_KEYS];
+        auto looks = [&](int u) { return st[u] != ST_COLD && (by_importance && is_pinned(p, pos[u], max_pos)) == (pinned != 0); };
+#pragma unroll
+        for (int u = 0; u < EB_KEYS; ++u) {
+            imp[u] = by_importance && looks(u) ? p.importance[gtid + u * stride] : 0.0f;
+            seq[u] = looks(u) ? (uint32_t)p.seq[gtid + u * stride] : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < EB_KEYS; ++u) key[u] = !looks(u) ? SENTINEL : by_importance ? ((uint64_t)f32_total_key(imp[u]) << 32) | seq[u] : (uint64_t)seq[u];
+        auto& set = ss->set[pinned];
+        uint64_t* lk = skeys + pinned * EB_CAP;
+        uint32_t* lv = svals + pinned * EB_CAP;
+        uint32_t kept;
+        const uint64_t own = block_cut(key, reach, 4u, sm.cut, kept);
+        if (threadIdx.x == 0 && kept >= reach) atomicMax(&set.bound_inv, (unsigned long long)~own);
+        if (threadIdx.x == 32) atomicMax(&set.bound_low, ~sm.cut.lo_inv);
+        if (threadIdx.x == 64 && sm.cut.count) atomicAdd(&set.all_n, sm.cut.count);
+        grid.sync();
+        const unsigned long long by_blocks = ~*(volatile unsigned long long*)&set.bound_inv, by_least = *(volatile unsigned long long*)&set.bound_low;
+        const uint32_t all_n = *(volatile uint32_t*)&set.all_n;
+        const uint64_t bound = reach <= gridDim.x ? min(by_blocks, by_least) : by_blocks;
+        uint32_t mine = 0;
+#pragma unroll
+        for (int j = 0; j < EB_KEYS; ++j) mine += key[j] != SENTINEL && key[j] <= bound;
+        if (__any_sync(0xFFFFFFFFu, mine != 0u)) {
+            uint32_t incl = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+                if (lane >= o) incl += y;
+            }
+            uint32_t at = 0;
+            if (lane == 31) at = atomicAdd(&set.few_n, incl);
+            at = __shfl_sync(0xFFFFFFFFu, at, 31) + incl - mine;
+#pragma unroll
+            for (int j = 0; j < EB_KEYS; ++j)
+                if (key[j] != SENTINEL && key[j] <= bound) {
+                    if (at < (uint32_t)EB_CAP) {
+                        lk[at] = key[j];
+                        lv[at] = (uint32_t)(gtid + j * stride);
+                    }
+                    ++at;
+                }
+        }
+        grid.sync();
+        got[pinned] = *(volatile uint32_t*)&set.few_n;
+        if (!by_importance || 96ull * all_n >= rest) break;  // (the same for every block)
+    }
+    if (blockIdx.x) return;
+    __syncthreads();
+    if (got[0] > (uint32_t)EB_CAP || got[1] > (uint32_t)EB_CAP) {
+        if (threadIdx.x == 0) say(live, free0, hot_n, STEP_BAIL);
+        return;
+    }
+    int64_t delta = 0;
+    uint64_t freed = free0;
+    if (hot_n) {
+        finish_phase<false>(p, PH_PAGE, hot_n, deficit, free0, hkeys, hvals, hot_n, skeys, svals, sm);  // (all of them: the lists of the evictions stay as they are)
+        delta += sm.delta;
+        __threadfence_block();
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int pinned = 0; pinned < 2; ++pinned) {
+        const uint64_t now = (uint64_t)((int64_t)live + delta);
+        if (!got[pinned] || now <= budget) continue;
+        const uint64_t left = now - budget;
+        uint64_t* lk = skeys + pinned * EB_CAP;
+        uint32_t* lv = svals + pinned * EB_CAP;
+        finish_phase<true>(p, PH_EVICT, left / 80 + 1, left, freed, lk, lv, got[pinned], lk, lv, sm);
+        delta += sm.delta;
+        freed += sm.applied;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        const uint64_t live_now = (uint64_t)((int64_t)live + delta);
+        cnt->live = live_now;
+        cnt->free_len = freed;
+        say(live_now, freed, 0, 0u);
+    }
+}
+
 // FEW: for pools in which a phase's smallest keys are found from registers where that can be done (see below); the other form is the faster one without that code
 // (100 000 slots, 1 to 80 evictions: 62 to 71 us of the kernel, 69 to 76 with it).
 template <bool FEW>
@@ -451,20 +752,10 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
                                                              uint64_t* skeys, uint32_t* svals, EnforceState* es) {
     namespace cg = cooperative_groups;
     cg::grid_group grid = cg::this_grid();
-    using Sort = cub::BlockRadixSort<uint64_t, EB_THREADS, EB_ITEMS, uint32_t>;
-    using Scan64 = cub::BlockScan<uint64_t, EB_THREADS>;
     using Scan32 = cub::BlockScan<uint32_t, EB_THREADS>;
-    __shared__ union {
-        typename Sort::TempStorage sort;
-        typename Scan64::TempStorage scan64;
-        typename Scan32::TempStorage scan32;
-        uint32_t hist[EB_BINS];
-        struct { uint64_t in[EB_THREADS], key[EB_THREADS]; uint32_t val[EB_THREADS]; } few;
-        CutShared cut;
-    } sm;
+    __shared__ FinishShared sm;
     __shared__ uint32_t cut_bin, cut_hist;
-    __shared__ unsigned long long cut_cum, fin_applied;
-    __shared__ long long fin_delta;
+    __shared__ unsigned long long cut_cum;
     volatile PoolCounters* cnt = p.cnt;
     const uint64_t len = cnt->len;
     const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, stride = (uint64_t)gridDim.x * blockDim.x;
@@ -707,99 +998,10 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
                 const uint64_t* ks = take_all ? keys : skeys;
                 const uint32_t* vs = take_all ? vals : svals;
                 uint32_t n = take_all ? (uint32_t)nc : (few ? *(volatile uint32_t*)&es->few[phase] : min(*(volatile uint32_t*)&es->n_keep, (uint32_t)EB_CAP));
-                uint64_t k[EB_ITEMS];
-                uint32_t v[EB_ITEMS];
-                for (int j = 0; j < EB_ITEMS; ++j) {
-                    const uint32_t i = threadIdx.x * EB_ITEMS + j;
-                    k[j] = i < n ? ks[i] : SENTINEL;
-                    v[j] = i < n ? vs[i] : 0u;
-                }
-                if (FEW && n > EB_THREADS && reach <= EB_THREADS / 2) {  // the blocks' smallest keys together: down to what the count below orders
-                    uint32_t kept;
-                    const uint64_t bound = block_cut(k, reach, EB_THREADS / 2, sm.cut, kept);
-                    if (kept <= EB_THREADS) {
-                        if (threadIdx.x == 0) warp_n[0] = 0u;
-                        __syncthreads();
-                        for (int j = 0; j < EB_ITEMS; ++j)
-                            if (k[j] != SENTINEL && k[j] <= bound) {
-                                const uint32_t o = atomicAdd(&warp_n[0], 1u);
-                                skeys[o] = k[j];  // (every key has been read: block_cut's barriers)
-                                svals[o] = v[j];
-                            }
-                        __syncthreads();
-                        ks = skeys;
-                        vs = svals;
-                        n = kept;
-                    }
-                }
+                finish_phase<FEW>(p, phase, reach, deficit, cnt->free_len, ks, vs, n, skeys, svals, sm);
                 if (threadIdx.x == 0) {
-                    fin_applied = 0;
-                    fin_delta = 0;
-                }
-                __syncthreads();
-                if (n <= EB_THREADS) {
-                    // few candidates (a decode step's page-outs and evictions): every thread counts the keys below its own
-                    // (keys are unique), n reads of shared memory instead of the radix sort's sixteen passes
-                    const uint32_t i = threadIdx.x;
-                    const uint64_t own = i < n ? ks[i] : SENTINEL;
-                    sm.few.in[i] = own;
-                    __syncthreads();
-                    uint32_t rank = 0;
-#pragma unroll 8
-                    for (uint32_t e = 0; e < n; ++e) rank += sm.few.in[e] < own;
-                    if (i < n) {
-                        sm.few.key[rank] = own;
-                        sm.few.val[rank] = vs[i];
-                    }
-                    __syncthreads();
-                    for (int j = 0; j < EB_ITEMS; ++j) {
-                        const uint32_t e = threadIdx.x * EB_ITEMS + j;
-                        k[j] = e < n ? sm.few.key[e] : SENTINEL;
-                        v[j] = e < n ? sm.few.val[e] : 0u;
-                    }
-                } else {
-                    Sort(sm.sort).Sort(k, v);
-                }
-                __syncthreads();
-                uint64_t w[EB_ITEMS], excl[EB_ITEMS];
-                for (int j = 0; j < EB_ITEMS; ++j) {
-                    uint32_t bytes = 0;
-                    if (k[j] != SENTINEL) {
-                        const uint32_t flags = tile_flags(p.tiles, v[j]);
-                        if (phase == PH_PAGE) bytes = 32;
-                        else if (phase <= PH_CORR_WARM) bytes = corr_bytes(flags);
-                        else bytes = live_bytes_of(p.state[v[j]], flags);
-                    }
-                    w[j] = bytes;
-                }
-                Scan64(sm.scan64).ExclusiveSum(w, excl);
-                const uint64_t free0 = cnt->free_len;
-                int64_t delta = 0;
-                uint32_t applied = 0;
-                for (int j = 0; j < EB_ITEMS; ++j) {
-                    if (k[j] == SENTINEL || excl[j] >= deficit) continue;
-                    const uint32_t s = v[j];
-                    if (phase == PH_PAGE) do_page_out(p, s, &delta);
-                    else if (phase <= PH_CORR_WARM) do_drop_correction(p, s, &delta);
-                    else {
-                        delta -= (int64_t)w[j];
-                        p.state[s] = ST_COLD;
-                        p.free_list[free0 + threadIdx.x * EB_ITEMS + j] = s;  // applied items are a prefix of the sorted order
-                        ++applied;
-                    }
-                }
-                for (int o = 16; o; o >>= 1) {
-                    delta += __shfl_xor_sync(0xFFFFFFFFu, delta, o);
-                    applied += __shfl_xor_sync(0xFFFFFFFFu, applied, o);
-                }
-                if (lane == 0) {
-                    if (delta) atomicAdd((unsigned long long*)&fin_delta, (unsigned long long)delta);
-                    if (applied) atomicAdd(&fin_applied, (unsigned long long)applied);
-                }
-                __syncthreads();
-                if (threadIdx.x == 0) {
-                    cnt->live = (uint64_t)((int64_t)live + fin_delta);
-                    cnt->free_len = free0 + fin_applied;
+                    cnt->live = (uint64_t)((int64_t)live + sm.delta);
+                    cnt->free_len += sm.applied;
                     cnt->n_cand = 0;
                     es->inv_min_key = 0;
                     es->max_key = 0;
@@ -1022,6 +1224,7 @@ inline uint32_t grid_for(uint64_t n, int threads = 256) {
 Status pool_sync_counters(Ctx* c, Pool* pl) {
     SLHA_CUDA(cudaMemcpyAsync(&pl->h_cnt, pl->dev.cnt, sizeof(PoolCounters), cudaMemcpyDeviceToHost, c->stream));
     SLHA_CUDA(cudaStreamSynchronize(c->stream));
+    pl->unread = 0;
     return Status();
 }
 
@@ -1065,6 +1268,8 @@ void pool_destroy(Pool* pl) {
     cudaFree(pl->dev.free_list);
     cudaFree(pl->dev.cnt);
     cudaFree(pl->d_observe);
+    cudaFree(pl->d_step);
+    if (pl->h_step) cudaFreeHost(pl->h_step);
     if (pl->log) eventlog_close(pl->log);
     delete pl;
 }
@@ -1083,6 +1288,8 @@ Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t
     h.free_len -= pops;
     h.len += n - pops;
     h.next_seq += n;
+    pl->hot_most += n;
+    pl->unread += n;
     return Status();
 }
 
@@ -1145,7 +1352,7 @@ static Status pool_enforce_budget_fused(Ctx* c, Pool* pl, int32_t* within, bool*
         blocks_per_sm[dev] = coop && b > 0 ? std::min(b, 2) : -1;
     }
     if (blocks_per_sm[dev] < 0) return Status();
-    const uint64_t len = pl->h_cnt.len;  // (the host mirror of len is exact: only inserts move it)
+    const uint64_t len = pl->h_cnt.len, free_before = pl->h_cnt.free_len;  // (the host mirror of both is exact: inserts and calls that read them back move them)
     if (len == 0) return Status();
     Scratch sc{c};
     SLHA_TRY(sc.reserve(pad256(len * 8) + pad256(len * 4) + pad256(EB_CAP * 8) + pad256(EB_CAP * 4) + pad256(sizeof(EnforceState)) + 4096));
@@ -1173,6 +1380,74 @@ static Status pool_enforce_budget_fused(Ctx* c, Pool* pl, int32_t* within, bool*
     SLHA_CUDA(cudaMemcpyAsync(&overflow, &es->overflow, 4, cudaMemcpyDeviceToHost, c->stream));
     SLHA_TRY(pool_sync_counters(c, pl));
     if (overflow) return Status();
+    if (pl->h_cnt.free_len > free_before) pl->hot_most = 0;  // evictions follow when every HOT tile is paged
+    *within = pl->h_cnt.live <= pl->h_cnt.budget ? 1 : 0;
+    *done = true;
+    return Status();
+}
+
+// The step kernel (see there), where no tile can have a correction plane and a thread's slots fit its registers (1.2 million on 148 SMs).  Not where the
+// list of HOT tiles may overflow, nor where the appended tiles alone ask for more evictions than the blocks' smallest keys are kept for (110 on 148 blocks):
+// the kernel would find that out after its first scan, 20 to 30 us, and leave the rest to the other.  Sets *done when the budget question is settled.
+static Status pool_enforce_budget_step(Ctx* c, Pool* pl, int32_t* within, bool* done) {
+    *done = false;
+    const uint32_t cm = pl->codec_mask;
+    const bool planes = !cm || (cm & (0x80000000u | (1u << SLHA_CODEC_TQ3) | (1u << SLHA_CODEC_MIX3)));
+    const uint64_t len = pl->h_cnt.len;
+    if (planes || len == 0) return Status();
+    static int ctas[64] = {0};
+    const int dev = pl->device & 63;
+    if (!ctas[dev]) {
+        int coop = 0, n = 0, b = 0;
+        SLHA_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, pl->device));
+        SLHA_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, pl->device));
+        SLHA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, enforce_step_kernel, EB_THREADS, 0));
+        ctas[dev] = coop && b > 0 ? n : -1;
+    }
+    if (ctas[dev] < 0) return Status();
+    const uint64_t want = (len + EB_THREADS - 1) / EB_THREADS;
+    const unsigned grid = (unsigned)std::min<uint64_t>(want, (uint64_t)ctas[dev]);
+    if (len > (uint64_t)EB_KEYS * grid * EB_THREADS) return Status();
+    if (pl->hot_most > (uint64_t)EB_CAP) return Status();
+    const uint64_t about = pl->h_cnt.live + 96 * pl->unread;  // once they are paged
+    if (about > pl->h_cnt.budget && ((about - pl->h_cnt.budget) / 80 + 1) * grid > 4ull * EB_CAP) return Status();
+    SLHA_TRY(ctx_no_capture(c));  // (the host waits for the answer)
+    constexpr size_t LIST = EB_CAP * 12;
+    if (!pl->d_step) {
+        SLHA_CUDA(cudaMalloc(&pl->d_step, 256 + 3 * LIST));
+        pl->step_clean = false;
+    }
+    if (!pl->h_step) SLHA_CUDA(cudaHostAlloc(&pl->h_step, 256, cudaHostAllocMapped | cudaHostAllocPortable));
+    void* d_answer = nullptr;
+    SLHA_CUDA(cudaHostGetDevicePointer(&d_answer, pl->h_step, 0));
+    volatile StepAnswer* h = static_cast<volatile StepAnswer*>(pl->h_step);
+    StepState* ss = static_cast<StepState*>(pl->d_step);
+    uint64_t* hkeys = reinterpret_cast<uint64_t*>(static_cast<char*>(pl->d_step) + 256);
+    uint64_t* skeys = hkeys + EB_CAP;
+    uint32_t* hvals = reinterpret_cast<uint32_t*>(skeys + 2 * EB_CAP);
+    uint32_t* svals = hvals + EB_CAP;
+    if (!pl->step_clean) SLHA_CUDA(cudaMemsetAsync(ss, 0, sizeof(StepState), c->stream));
+    pl->step_clean = false;
+    PoolDev d = pl->dev;
+    uint32_t no = pl->step_no = pl->step_no % 0x7FFFFFFFu + 1u;
+    h->no = 0u;
+    StepAnswer* answer = static_cast<StepAnswer*>(d_answer);
+    void* args[] = {&d, &hkeys, &hvals, &skeys, &svals, &ss, &answer, &no};
+    SLHA_CUDA(cudaLaunchCooperativeKernel((const void*)enforce_step_kernel, dim3(grid), dim3(EB_THREADS), args, 0, c->stream));
+    count_launch();
+    for (uint32_t i = 0; h->no != no; ++i) {
+        if (i % 4096 != 4095) continue;
+        const cudaError_t e = cudaStreamQuery(c->stream);
+        if (e == cudaErrorNotReady) continue;
+        SLHA_CUDA(e);
+        if (h->no != no) return Status(SLHA_ERR_DEVICE, "enforce_budget: the kernel ended without an answer");
+    }
+    pl->h_cnt.live = h->live;
+    pl->h_cnt.free_len = h->free_len;
+    pl->unread = 0;
+    pl->step_clean = true;
+    if (h->hot != ~0ull) pl->hot_most = h->hot;
+    if (h->flags) return Status();
     *within = pl->h_cnt.live <= pl->h_cnt.budget ? 1 : 0;
     *done = true;
     return Status();
@@ -1181,6 +1456,8 @@ static Status pool_enforce_budget_fused(Ctx* c, Pool* pl, int32_t* within, bool*
 Status pool_enforce_budget(Ctx* c, Pool* pl, int32_t* within) {
     if (!pl->log && !pl->require_durable && !debug_general_paths()) {
         bool done = false;
+        SLHA_TRY(pool_enforce_budget_step(c, pl, within, &done));
+        if (done) return Status();
         SLHA_TRY(pool_enforce_budget_fused(c, pl, within, &done));
         if (done) return Status();
     }
