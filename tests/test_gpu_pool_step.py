@@ -76,3 +76,49 @@ def test_a_step_gives_what_the_host_driven_phases_give(page, evict, recent, n):
     step(96 * 2)
     for a, b in zip(pools[0].read(), pools[1].read()):
         assert a.tobytes() == b.tobytes()
+
+
+@pytest.mark.parametrize("n", [1, 15, 256, 257, 65537, 16 * 65536, 16 * 65536 + 1])
+def test_observing_a_query_is_observing_its_scores(n):
+    # up to 16 x 65 536 slots by one kernel, from there on by three, like a list of slots, in the same order; the counts of both forms of the statistics
+    gm = S.Model.from_projection(H.make_model_pair(128, seed=61)[1], 128, 61)
+    base = H.gaussian_keys(64, 2048, 128)
+    pools = [S.TilePool(n, 2**40) for _ in range(2)]
+    for b in range(0, n, 262144):
+        keys = np.resize(base, (min(262144, n - b), 128))
+        for p in pools:
+            p.append_keys(gm, keys, S.CODEC_MIXED)
+    qc, qs = H.random_queries(1, 7)
+    gone = np.unique(np.array([0, n // 3, n // 2]) % n) if n > 1 else []
+    for p in pools:
+        for s in gone:
+            p.evict(int(s))
+    slots, scores = pools[0].score_all(qc, qs)
+    pools[0].observe_query(qc, qs, 20.0)
+    pools[1].observe_scores(slots, scores, 20.0)
+    a, b = pools[0].read()[2], pools[1].read()[2]
+    live = np.ones(n, bool)
+    live[list(gone)] = False
+    assert np.allclose(a[live], b[live], rtol=3e-5, atol=1e-44)  # (a list leaves out COLD slots, so its shares are others: 16 terms a thread, a tree, 256 sums, each way 2^-24 x 280; subnormal weights: their spacing)
+    assert abs(float(a[live].astype(np.float64).sum()) - 1.0) < 1e-4
+    st = pools[0].stats()
+    assert (st["hot"], st["warm"], st["cold"], st["len"]) == (n - len(gone), 0, len(gone), n)
+    extra = S.TilePool(40, 2**40)
+    extra.insert(H.random_tiles(33, 4, seed=3, nocorr_every=5))
+    st = extra.stats()
+    assert st["hot"] == 33 and st["nocorr"] == 7
+
+
+@pytest.mark.parametrize("nq,k", [(1, 1), (256, 1), (257, 1), (4, 64), (5, 64)])
+def test_short_host_outputs(nq, k):
+    # 1024 bytes are the most that kernels write to the host's page
+    tiles = H.random_tiles(300, 0, seed=9)
+    pool = S.TilePool(300, 2**40)
+    pool.insert(tiles)
+    qc, qs = H.random_queries(nq, 11)
+    gi, gs, gc = pool.score_topk(qc, qs, nq, k)
+    di, ds, dc = S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * 4)
+    pool.score_topk(S.to_device(qc), S.to_device(qs), nq, k, di, ds, dc)
+    S.synchronize()
+    assert np.array_equal(np.asarray(gi).reshape(-1), di.download(np.uint32, nq * k)) and np.array_equal(np.asarray(gs).reshape(-1), ds.download(F, nq * k))
+    assert np.array_equal(gc, dc.download(np.uint32, nq)) and np.all(gc == k)
