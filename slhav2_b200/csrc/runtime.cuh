@@ -37,6 +37,7 @@ Status stage_in_t(Ctx* c, const T* p, size_t count, const T** dev) {
 struct StagedOut {
     void* dev = nullptr;
     void* user = nullptr;
+    const unsigned char* page = nullptr;  // page-locked memory behind dev
     size_t bytes = 0;
     bool is_host = false;
 };
