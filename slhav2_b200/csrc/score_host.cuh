@@ -261,14 +261,16 @@ thread_local Plan* g_last_plan = nullptr;    // of the thread's latest score_top
 thread_local uint32_t g_plans_recycled = 0;  // of this thread's captured plans
 std::atomic<uint32_t> g_plan_threads{0};
 
-// Cuts of (segment, group of up to `width` query rows) streams into one share per CTA.
+// Cuts of (segment, group of up to `width` query rows) streams into one share per CTA.  `total`: in whole units of each stream, as the shares are filled (counted in
+// tiles, 200 segments of 8128 made 149 CTAs, one of them behind all others: 136 us instead of 90).
 struct Cuts {
+    static uint64_t whole(uint64_t n, uint64_t unit) { return (n + unit - 1) / unit * unit; }
     std::vector<WorkItem> items;
     std::vector<uint32_t> cta{0u};
     uint64_t share = 0, filled = 0, unit;
     Cuts(uint64_t total, int sms, uint64_t unit_tiles, uint64_t least) : unit(unit_tiles) {
         share = (total + sms - 1) / sms;
-        share = std::max<uint64_t>(least, (share + unit - 1) / unit * unit);
+        share = std::max<uint64_t>(least, whole(share, unit));
     }
     void add(const SlhaB200Segment& s, uint32_t width) {
         for (uint32_t q0 = 0; q0 < s.n_queries; q0 += width)
@@ -282,7 +284,7 @@ struct Cuts {
                 w.n_queries = std::min<uint32_t>(width, s.n_queries - q0);
                 items.push_back(w);
                 pos += take;
-                filled += (take + unit - 1) / unit * unit;  // (cuts lie at whole units of a segment)
+                filled += whole(take, unit);  // (cuts lie at whole units of a segment)
                 if (filled >= share) {
                     filled = 0;
                     cta.push_back((uint32_t)items.size());
@@ -323,8 +325,8 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
             rows[s.query_begin + q] = RowInfo{s.n_tiles, s.index_base, 0u, 128u};
         }
         wide = wide && (s.n_queries >= 16 || s.n_tiles == 0);
-        total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
-        wtotal += (uint64_t)s.n_tiles * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
+        total += Cuts::whole(s.n_tiles, ST_M) * ((s.n_queries + 3) / 4);
+        wtotal += Cuts::whole(s.n_tiles, WIDE_M) * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
     }
     wide = wide && allow_wide && wtotal;
     Cuts cuts(wide ? wtotal : total, sms, wide ? WIDE_M : ST_M, wide ? WIDE_M : ST_M);
@@ -904,7 +906,7 @@ Status launch_score_full(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     // bit 0: NF4 tiles beside INT4 ones; -1: not known.
     if (n >= 32768 && n < 0xFFFFFFFFull && codec_hint != -2 && !g_force_generic) {
         const int sms = sm_count(c->device);
-        Cuts cuts((uint64_t)n * ((nq + 3) / 4), sms, ST_M, 2048);
+        Cuts cuts(Cuts::whole(n, ST_M) * ((nq + 3) / 4), sms, ST_M, 2048);
         cuts.add(SlhaB200Segment{0, (uint32_t)n, 0, (uint32_t)nq, 0}, 4);
         cuts.finish();
         Blob blob;
@@ -975,8 +977,8 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
         for (uint32_t q = 0; q < s.n_queries; ++q) tail[s.query_begin + q] = s.index_base + s.n_tiles;
         fills |= s.index_base + s.n_tiles < row_len;
         wide = wide && (s.n_queries >= 16 || s.n_tiles == 0);
-        total += (uint64_t)s.n_tiles * ((s.n_queries + 3) / 4);
-        wtotal += (uint64_t)s.n_tiles * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
+        total += Cuts::whole(s.n_tiles, ST_M) * ((s.n_queries + 3) / 4);
+        wtotal += Cuts::whole(s.n_tiles, WIDE_M) * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
     }
     // (the four-row kernel's pass behind the 64-row kernel takes that one's items, four rows at a time)
     Cuts cuts(wide ? wtotal : total, sms, wide ? WIDE_M : ST_M, wide ? WIDE_M : ST_M * 4);
