@@ -297,17 +297,20 @@ struct Cuts {
 };
 
 // Whether a call's rows are scored as a whole (score_select.cuh) rather than streamed: rows of up to ROWS_MOST tiles, scores of 64 MB at most.  `passes`: tiles times
-// groups of four query rows, `wide`: 16 rows or more a segment, which the 64-row kernel takes (512 rows of 16 384 TQ3 tiles, k = 256 86 -> 51 us; 1232 of
-// 3553 MX tiles 111 -> 53).  Streaming reads a million tiles in 25 us where score_dense_kernel takes 40 (NF4 60), but its first sets, hand-over check, compaction and
-// merge cost 20 to 50 us more, most with many winners.  us a call, streamed / whole, k = 64 and 1024: 8192 INT4 tiles 22.9 / 15.6, 27.7 / 16.0; 32 segments of
-// 8192 mixed tiles 35.8 / 26.2, 46.0 / 29.2; 64 of 16 384 INT4 61 / 54, 89 / 59, TQ3 80 / 67, 108 / 72, NF4 73 / 78, 100 / 82; 100 of 16 384 INT4 80 / 81, 108 / 88,
-// NF4 95 / 117, 120 / 124; 128 of 32 768 INT4 137 / 193, 187 / 212; MIX3 16 of 32 768 59 / 45, 76 / 49.
+// groups of four query rows, `wide`: 16 rows or more a segment, which the 64-row kernel takes (512 rows of 16 384 TQ3 tiles, k = 256 85 -> 47 us; 1232 of
+// 3553 MX tiles 111 -> 53).  Streaming reads a million tiles in 25 us where score_dense_kernel takes 40 (NF4 34, 59), but its set-up, first sets and compaction
+// cost about 20 us a call, and appending and merging a row 0.04 (k = 64) to 0.08 us (k = 1024), which selecting from whole rows costs hardly: in pico-
+// seconds, 16 a pass (NF4 30, both a little above what was measured) against 18 million a call and per_row a row.  us a call, whole / streamed, k = 64, 256, 1024:
+//   64 segments of 16 384 INT4 tiles 51 / 63, 52 / 72, 60 / 90, TQ3 59 / 82, 60 / 95, 68 / 111, NF4 71 / 73, 71 / 86, 80 / 105; 128 of 16 384 INT4 88 / 94, 89 / 108, 106 / 124,
+//   NF4 126 / 114, 127 / 122, 143 / 140; 48 of 32 768 INT4 76 / 72, 79 / 85, 86 / 103, NF4 105 / 87, 109 / 99, 116 / 117; 96 of 32 768 INT4 131 / 114, 135 / 133, 147 / 157,
+//   mixed 129 / 124, 133 / 136, 144 / 157; 400 of 8192 INT4 141 / 165, 142 / 191, 181 / 234, NF4 201 / 186, 201 / 214, 241 / 256; 1000 of 4096 INT4 198 / 253,
+//   200 / 308, 245 / 396, NF4 272 / 294, 273 / 369, 318 / 475.
 enum RowsRule { ROWS_NO, ROWS_YES, ROWS_UNLESS_NF4 };
 RowsRule rows_rule(uint64_t passes, bool wide, size_t nq, uint32_t longest, uint32_t k) {
     if (longest == 0 || longest > ROWS_MOST || nq * (((uint64_t)longest + 31) / 32 * 32) > (16ull << 20)) return ROWS_NO;
-    const uint64_t more = k >= 512 ? 2 : 1;
-    if (wide || passes <= 640000 * more) return ROWS_YES;
-    return passes <= 1280000 * more ? ROWS_UNLESS_NF4 : ROWS_NO;
+    if (wide || passes <= (k >= 512 ? 1280000 : 640000)) return ROWS_YES;
+    const uint64_t saved = 18000000 + nq * (k >= 1024 ? 85000 : k >= 200 ? 75000 : k >= 32 ? 37000 : 25000);
+    return 30 * passes <= saved ? ROWS_YES : 16 * passes <= saved ? ROWS_UNLESS_NF4 : ROWS_NO;
 }
 
 Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_segs, size_t nq, uint32_t longest, bool allow_wide) {

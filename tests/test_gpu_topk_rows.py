@@ -97,3 +97,14 @@ def test_cold_slots_are_no_candidates():
     for j in range(4):
         order = left[np.lexsort((left, -want[j, left]))]
         assert np.array_equal(np.sort(idx[j, :300]), left) and np.all(np.abs(sc[j, :300] - want[j, order]) <= 1e-3)
+
+
+@pytest.mark.parametrize("codec,n_seg", [(0, 100), (4, 100), (2, 60)])
+def test_many_rows_whose_segments_end_inside_a_block(codec, n_seg):
+    # above what every call's rows are scored as a whole for: the rule's side of them; shares that are cut in blocks of 128 tiles
+    n, nq = 16_000, 4
+    tiles = H.random_tiles(n + 600, codec, seed=80 + codec)
+    qc, qs = H.random_queries(nq * n_seg, 81)
+    rows = [(5 * i, n + i, nq * i, nq, 7 * i) for i in range(n_seg)]
+    assert sum(r[1] for r in rows) > 640_000
+    _check(tiles, rows, nq * n_seg, 300, qc, qs)
