@@ -1732,7 +1732,8 @@ Status pool_observe(Ctx* c, Pool* pl, const uint32_t* d_slots, const float* d_sc
     ObserveTmp* tmp = reinterpret_cast<ObserveTmp*>(pl->d_observe);
     ObserveTmp* all = tmp + 1;  // observe_all_kernel's, zero between its calls
     float* partial = reinterpret_cast<float*>(tmp + 2);
-    if (!d_slots && n <= (uint64_t)OBSERVE_PARTS * 256 * OBSERVE_KEEP) {
+    // (not into a graph: whether the state needs its clear is known when a call is made, not when a graph is launched)
+    if (!d_slots && n <= (uint64_t)OBSERVE_PARTS * 256 * OBSERVE_KEEP && !ctx_capturing(c)) {
         static int fits[64] = {0};
         const int dev = pl->device & 63;
         if (!fits[dev]) {

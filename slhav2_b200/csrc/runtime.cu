@@ -197,6 +197,7 @@ bool mark(LastUse& u, cudaStream_t s, unsigned long long id) {
 }
 }  // namespace
 
+bool ctx_capturing(Ctx* c) { return capturing(c->stream); }
 Status ctx_no_capture(Ctx* c) {
     if (!capturing(c->stream)) return Status();
     // a graph would keep the address of host memory that this call's successors write again: refused, and the capture ends

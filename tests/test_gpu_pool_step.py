@@ -1,9 +1,12 @@
 """The budget question of a decode step, settled by one kernel (pool.cu, enforce_step_kernel): the same slots, states, bytes and order of freed
 slots as the phases run one by one from the host give, on both sides of every condition under which the kernel leaves the work to the others."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from tests import helpers as H
+from tests.test_gpu_streams import Streams
 
 pytestmark = pytest.mark.gpu
 S = pytest.importorskip("slhav2_b200")
@@ -122,3 +125,33 @@ def test_short_host_outputs(nq, k):
     S.synchronize()
     assert np.array_equal(np.asarray(gi).reshape(-1), di.download(np.uint32, nq * k)) and np.array_equal(np.asarray(gs).reshape(-1), ds.download(F, nq * k))
     assert np.array_equal(gc, dc.download(np.uint32, nq)) and np.all(gc == k)
+
+
+def test_observing_a_query_is_captured_before_any_other_call():
+    # a graph made by the pool's first such call, launched behind and before calls that are not
+    gm = S.Model.from_projection(H.make_model_pair(128, seed=61)[1], 128, 61)
+    pools = [S.TilePool(3000, 2**40) for _ in range(2)]
+    for p in pools:
+        p.append_keys(gm, H.gaussian_keys(65, 3000, 128), S.CODEC_MIXED)
+    qc, qs = H.random_queries(1, 12)
+    dq, ds = S.to_device(qc), S.to_device(qs)
+    with Streams(1) as st:
+        rt, graph, exe = st.rt, C.c_void_p(), C.c_void_p()
+        S.set_stream(st.all[0].value)
+        pools[1].observe_query(dq, ds, 3.0)  # (the thread's scratch)
+        assert rt.cudaStreamBeginCapture(st.all[0], 2) == 0
+        pools[0].observe_query(dq, ds, 3.0)
+        assert rt.cudaStreamEndCapture(st.all[0], C.byref(graph)) == 0
+        assert rt.cudaGraphInstantiate(C.byref(exe), graph, C.c_ulonglong(0)) == 0
+        for direct in (True, False, True, False):
+            if direct:
+                pools[0].observe_query(dq, ds, 3.0)
+            else:
+                assert rt.cudaGraphLaunch(exe, st.all[0]) == 0
+        for _ in range(3):
+            pools[1].observe_query(dq, ds, 3.0)
+        S.synchronize()
+        rt.cudaGraphExecDestroy(exe)
+        rt.cudaGraphDestroy(graph)
+        S.set_stream(None)
+    assert pools[0].read()[2].tobytes() == pools[1].read()[2].tobytes()
