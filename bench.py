@@ -538,7 +538,7 @@ def run_scoring_workload(args, w, S, torch, dist, rank, local, world, dev, strea
         "blocks_ms_per_step": {"min": min(block_ms) / args.steps, "median": ms_step, "max": max(block_ms) / args.steps, "blocks": BLOCKS},
         "scores_per_s": value * w["group"],
         "hbm_gbs_whole_step": total_tiles * 128 / (ms_step * 1e-3) / 1e9,
-        "roofline": {"bound": "hbm", "kernel": "score_stream_kernel (fused eq. 2.3 score + streaming top-k)", "achieved": achieved,
+        "roofline": {"bound": "hbm", "kernel": "score_stream_kernel (fused eq. 2.3 score + streaming top-k), of short rows score_dense_kernel or score_wide_dense_kernel", "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak, "peak_kind": peak_kind,
                      "frac_of_nominal_8000": achieved / 8000.0, "kernel_ms": k_ms,
                      "merge_kernel_ms": float(np.median(merge_ms)) if len(merge_ms) else None,  # (early-exit pass of the generic kernel, compaction, merge)
