@@ -557,7 +557,7 @@ int32_t slha_b200_pool_append_keys(SlhaB200Pool* pool, const SlhaModel* model, c
             SLHA_TRY(ctx_device_scratch(c, n * 4, (void**)&dslots));
         }
         // freshly encoded tiles are HOT with their correction plane: 128 live bytes each
-        SLHA_TRY(pool_reserve(c, pl, nullptr, n, dslots));
+        SLHA_TRY(pool_reserve(c, pl, nullptr, n, dslots, dpos, position_base));
         SLHA_TRY(launch_encode(c, m.get(), dk, key_dtype, n, dpos, position_base, dhead, codec,
                                reinterpret_cast<SciRustSlhaTile*>(pl->dev.tiles), dslots));
         pl->codec_mask |= 1u << codec;

@@ -42,7 +42,7 @@ __device__ __forceinline__ uint32_t tile_flags(const unsigned char* tiles, uint6
 // Tile j of the batch takes free_list[free_len-1-j] while the free list lasts
 // (LIFO pops), then fresh slots len, len+1, ...
 __global__ void insert_kernel(PoolDev p, const unsigned char* src, uint64_t n, uint64_t pops,
-                              uint64_t len0, uint64_t free0, uint64_t seq0, uint32_t* slots_out) {
+                              uint64_t len0, uint64_t free0, uint64_t seq0, const uint32_t* positions, uint32_t position_base, uint32_t* slots_out) {
     dep_launch();
     dep_wait();
     const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -55,6 +55,7 @@ __global__ void insert_kernel(PoolDev p, const unsigned char* src, uint64_t n, u
         p.state[slot] = st;
         p.seq[slot] = seq0 + j;
         p.importance[slot] = 0.0f;
+        p.pos[slot] = src ? *reinterpret_cast<const uint32_t*>(src + j * TILE_BYTES + 112) : positions ? positions[j] : position_base + (uint32_t)j;
         slots_out[j] = slot;
         bytes = live_bytes_of(st, flags);
     }
@@ -125,7 +126,7 @@ __global__ void max_pos_kernel(PoolDev p) {
     const uint64_t len = p.cnt->len;
     uint32_t m = 0;
     for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < len; s += (uint64_t)gridDim.x * blockDim.x)
-        if (p.state[s] != ST_COLD) m = max(m, *reinterpret_cast<const uint32_t*>(p.tiles + s * TILE_BYTES + 112));
+        if (p.state[s] != ST_COLD) m = max(m, p.pos[s]);
     for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(&p.cnt->max_pos, m);
 }
@@ -151,9 +152,8 @@ __device__ __forceinline__ void load_meta(const PoolDev& p, int phase, uint64_t 
     m.weight = 0.0f;
     if (!phase_looks(phase, m.st)) return;
     const unsigned char* t = p.tiles + s * TILE_BYTES;
-    const uint2 pf = *reinterpret_cast<const uint2*>(t + 112);  // position, head | flags
-    m.pos = pf.x;
-    m.flags = pf.y >> 16;
+    if (phase >= PH_EVICT) m.pos = p.pos[s];
+    if (phase == PH_CORR_HOT || phase == PH_CORR_WARM) m.flags = tile_flags(p.tiles, s);
     m.seq = (uint32_t)p.seq[s];
     m.weight = phase >= PH_EVICT ? p.importance[s] : *reinterpret_cast<const float*>(t + 104);
 }
@@ -565,8 +565,8 @@ __device__ __forceinline__ void finish_phase(const PoolDev& p, int phase, uint64
 // frees 32 bytes each, so all blocks know the evictions' deficit as soon as they know how many there are, and the states, positions and the largest position come
 // from the same loads: three grid barriers and one end instead of seven and two, and the host reads the answer from its own memory instead of waiting for the end and for
 // two copies.  Latency bounds it: barriers, a scan whose loads are all in flight at once, and one block's ordering of a few hundred keys.  us of the whole
-// call, 8 tiles appended and 8 evicted, with enforce_kernel and with this one: by importance 20 000 slots 94 / 32, 100 000 81 / 42, 1 000 000 132 / 62; in
-// causal order 69 / 32, 81 / 35, 121 / 37.  Whatever does not fit is left to enforce_kernel, with nothing changed: that costs the first scan, so the host
+// call, 8 tiles appended and 8 evicted, with enforce_kernel and with this one: by importance 20 000 slots 94 / 32, 100 000 81 / 42, 1 000 000 132 / 41 (62
+// while the positions were read from the tiles, a sector of every line); in causal order 69 / 32, 81 / 35, 121 / 37.  Whatever does not fit is left to enforce_kernel, with nothing changed: that costs the first scan, so the host
 // also asks what it knows before (see there).
 constexpr uint32_t STEP_BAIL = 1u;                  // a flag of the answer: nothing was done
 struct StepState {                                  // zero when the kernel starts, and again when it ends
@@ -610,10 +610,10 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_step_kernel(PoolDev p, uin
 #pragma unroll
     for (int u = 0; u < EB_KEYS; ++u) st[u] = gtid + u * stride < len ? p.state[gtid + u * stride] : ST_COLD;
 #pragma unroll
-    for (int u = 0; u < EB_KEYS; ++u) pos[u] = by_importance && st[u] != ST_COLD ? *reinterpret_cast<const uint32_t*>(p.tiles + (gtid + u * stride) * TILE_BYTES + 112) : 0u;
+    for (int u = 0; u < EB_KEYS; ++u) pos[u] = by_importance && gtid + u * stride < len ? p.pos[gtid + u * stride] : 0u;
     uint32_t m = 0;
 #pragma unroll
-    for (int u = 0; u < EB_KEYS; ++u) m = max(m, pos[u]);
+    for (int u = 0; u < EB_KEYS; ++u) m = max(m, st[u] != ST_COLD ? pos[u] : 0u);
 #pragma unroll 1
     for (int u = 0; u < EB_KEYS; ++u) {
         uint8_t own = st[0];
@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
             for (int u = 0; u < EB_BATCH; ++u) st[u] = s0 + u * stride < len ? p.state[s0 + u * stride] : ST_COLD;
 #pragma unroll
             for (int u = 0; u < EB_BATCH; ++u)
-                pos[u] = st[u] != ST_COLD ? *reinterpret_cast<const uint32_t*>(p.tiles + (s0 + u * stride) * TILE_BYTES + 112) : 0u;
+                pos[u] = st[u] != ST_COLD ? p.pos[s0 + u * stride] : 0u;
 #pragma unroll
             for (int u = 0; u < EB_BATCH; ++u) m = max(m, pos[u]);
         }
@@ -800,7 +800,8 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_kernel(PoolDev p, uint32_t
         //      within both go to the last block's sort from registers: one scan and two grid barriers, where the list of all
         //      candidates below takes a write and three reads, global histograms and three barriers.  The block's own selection costs more than the list while
         //      that is read in a round or two (us of the kernel, 16 evictions by importance, without and with: 100 000 slots 65 / 84, 300 000 73 / 88,
-        //      500 000 93 / 96, 650 000 101 / 102, 1 000 000 136 / 120; in causal order 59 / 71, 69 / 76, 84 / 81, 93 / 87, 126 / 108).
+        //      500 000 93 / 96, 650 000 101 / 102, 1 000 000 136 / 120; in causal order 59 / 71, 69 / 76, 84 / 81, 93 / 87, 126 / 108;
+        //      all with the positions read from the tiles).
         bool few = FEW && reach * gridDim.x <= 4ull * EB_CAP;
         if (FEW && few) {
             uint64_t key[EB_KEYS];
@@ -1359,6 +1360,7 @@ Status pool_create(Ctx* c, const SlhaB200PoolConfig& cfg, Pool** out) {
     alloc((void**)&d.state, cap);
     alloc((void**)&d.seq, cap * 8);
     alloc((void**)&d.importance, cap * 4);
+    alloc((void**)&d.pos, cap * 4);
     alloc((void**)&d.free_list, cap * 4);
     alloc((void**)&d.cnt, sizeof(PoolCounters));
     if (e != cudaSuccess) {
@@ -1384,6 +1386,7 @@ void pool_destroy(Pool* pl) {
     cudaFree(pl->dev.state);
     cudaFree(pl->dev.seq);
     cudaFree(pl->dev.importance);
+    cudaFree(pl->dev.pos);
     cudaFree(pl->dev.free_list);
     cudaFree(pl->dev.cnt);
     cudaFree(pl->d_observe);
@@ -1394,7 +1397,7 @@ void pool_destroy(Pool* pl) {
 }
 
 // Reserve slots for n tiles (bookkeeping only); d_slots receives the slot ids.
-Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t n, uint32_t* d_slots) {
+Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t n, uint32_t* d_slots, const uint32_t* d_positions, uint32_t position_base) {
     PoolCounters& h = pl->h_cnt;
     if (h.next_seq + n > 0xFFFFFFFFull)
         return Status(SLHA_ERR_CAPACITY, "pool: insertion counter exhausted (2^32 inserts)");
@@ -1402,7 +1405,7 @@ Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t
     if (h.len + (n - pops) > pl->cfg.capacity_tiles)
         return Status(SLHA_ERR_CAPACITY, "pool: capacity_tiles exceeded");
     SLHA_CUDA(launch_behind(insert_kernel, dim3((uint32_t)((n + 255) / 256)), dim3(256), 0, c->stream, pl->dev, d_src_tiles, n, pops, h.len, h.free_len,
-                            h.next_seq, d_slots));
+                            h.next_seq, d_positions, position_base, d_slots));
     count_launch();
     h.free_len -= pops;
     h.len += n - pops;

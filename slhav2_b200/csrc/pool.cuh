@@ -25,6 +25,7 @@ struct PoolDev {
     uint8_t* state = nullptr;        // HOT / WARM / COLD per slot
     uint64_t* seq = nullptr;         // insertion order per slot
     float* importance = nullptr;     // accumulated H2O importance per slot
+    uint32_t* pos = nullptr;         // the tiles' positions once more: a scan of them reads 4 bytes a slot, not a line
     uint32_t* free_list = nullptr;   // LIFO stack of COLD slots
     PoolCounters* cnt = nullptr;
     int32_t page_policy = 0, evict_policy = 0;
@@ -64,7 +65,8 @@ struct Pool {
 Status pool_create(Ctx* c, const SlhaB200PoolConfig& cfg, Pool** out);
 void pool_destroy(Pool* pl);
 Status pool_sync_counters(Ctx* c, Pool* pl);
-Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t n, uint32_t* d_slots);
+Status pool_reserve(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, uint64_t n, uint32_t* d_slots, const uint32_t* d_positions = nullptr,
+                    uint32_t position_base = 0);
 Status pool_scatter(Ctx* c, Pool* pl, const unsigned char* d_src_tiles, const uint32_t* d_slots, uint64_t n);
 Status pool_single_op(Ctx* c, Pool* pl, int op, uint32_t slot, int32_t* result);
 Status pool_enforce_budget(Ctx* c, Pool* pl, int32_t* within);
