@@ -58,8 +58,8 @@ Status ctx_no_capture(Ctx* c);
 bool ctx_capturing(Ctx* c);
 Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes);
 Status ctx_upload(Ctx* c, const void* src, size_t bytes, void** dev);
-// 256 bytes of page-locked host memory that kernels of the calling thread's call can write, per thread and device (64 of them for checks, the upper
-// half for statistics, which are waited for); *open while a check may.
+// 512 bytes of page-locked host memory that kernels of the calling thread's call can write, per thread and device (64 of them for checks, from byte 128 on
+// statistics and from 256 on enforce_budget, which are waited for); *open while a check may.
 Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, bool** open);
 // The call under way uses a plan's buffers (kept per thread, like the scratch arena): waits for another stream's use of them, see LastUse.
 void ctx_uses_plans(Ctx* c);

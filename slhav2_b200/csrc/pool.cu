@@ -1391,7 +1391,6 @@ void pool_destroy(Pool* pl) {
     cudaFree(pl->dev.cnt);
     cudaFree(pl->d_observe);
     cudaFree(pl->d_step);
-    if (pl->h_step) cudaFreeHost(pl->h_step);
     if (pl->log) eventlog_close(pl->log);
     delete pl;
 }
@@ -1457,13 +1456,12 @@ Status pool_single_op(Ctx* c, Pool* pl, int op, uint32_t slot, int32_t* result) 
     return pool_sync_counters(c, pl);
 }
 
-// Device memory of enforce_step_kernel (state, lists), and where it answers.
-static Status pool_answer_memory(Pool* pl) {
+// Device memory of enforce_step_kernel: state, lists.
+static Status pool_step_memory(Pool* pl) {
     if (!pl->d_step) {
         SLHA_CUDA(cudaMalloc(&pl->d_step, 256 + 3 * (size_t)EB_CAP * 12));
         pl->step_clean = false;
     }
-    if (!pl->h_step) SLHA_CUDA(cudaHostAlloc(&pl->h_step, 256, cudaHostAllocMapped | cudaHostAllocPortable));
     return Status();
 }
 // Until a kernel on the stream has answered; an error of the stream, or its end without the answer, ends the wait too.
@@ -1556,10 +1554,12 @@ static Status pool_enforce_budget_step(Ctx* c, Pool* pl, int32_t* within, bool* 
     const uint64_t about = pl->h_cnt.live + 96 * pl->unread;  // once they are paged
     if (about > pl->h_cnt.budget && ((about - pl->h_cnt.budget) / 80 + 1) * grid > 4ull * EB_CAP) return Status();
     SLHA_TRY(ctx_no_capture(c));  // (the host waits for the answer)
-    SLHA_TRY(pool_answer_memory(pl));
-    void* d_answer = nullptr;
-    SLHA_CUDA(cudaHostGetDevicePointer(&d_answer, pl->h_step, 0));
-    volatile StepAnswer* h = static_cast<volatile StepAnswer*>(pl->h_step);
+    SLHA_TRY(pool_step_memory(pl));
+    volatile uint32_t* host;
+    uint32_t* dev_host;
+    bool* open;
+    SLHA_TRY(ctx_answer(c, &host, &dev_host, &open));
+    volatile StepAnswer* h = reinterpret_cast<volatile StepAnswer*>(host + 64);
     StepState* ss = static_cast<StepState*>(pl->d_step);
     uint64_t* hkeys = reinterpret_cast<uint64_t*>(static_cast<char*>(pl->d_step) + 256);
     uint64_t* skeys = hkeys + EB_CAP;
@@ -1568,9 +1568,10 @@ static Status pool_enforce_budget_step(Ctx* c, Pool* pl, int32_t* within, bool* 
     if (!pl->step_clean) SLHA_CUDA(cudaMemsetAsync(ss, 0, sizeof(StepState), c->stream));
     pl->step_clean = false;
     PoolDev d = pl->dev;
-    uint32_t no = pl->step_no = pl->step_no % 0x7FFFFFFFu + 1u;
+    static thread_local uint32_t count = 0;
+    uint32_t no = count = count % 0x7FFFFFFFu + 1u;
     h->no = 0u;
-    StepAnswer* answer = static_cast<StepAnswer*>(d_answer);
+    StepAnswer* answer = reinterpret_cast<StepAnswer*>(dev_host + 64);
     void* args[] = {&d, &hkeys, &hvals, &skeys, &svals, &ss, &answer, &no};
     SLHA_CUDA(cudaLaunchCooperativeKernel((const void*)enforce_step_kernel, dim3(grid), dim3(EB_THREADS), args, 0, c->stream));
     count_launch();

@@ -48,10 +48,8 @@ struct Pool {
     PoolDev dev;
     PoolCounters h_cnt;      // host mirror
     void* d_observe = nullptr;  // scratch of observe_scores (reduction cell + partial sums)
-    void* d_step = nullptr;     // enforce_step_kernel: its state and lists,
-    void* h_step = nullptr;     // and where it answers (page-locked)
+    void* d_step = nullptr;     // enforce_step_kernel: its state and lists
     bool step_clean = false, observe_clean = false;  // that state and observe_all_kernel's are zero
-    uint32_t step_no = 0;
     uint64_t hot_most = 0, unread = 0;  // HOT tiles at the most, and tiles inserted since h_cnt.live was read: what a kernel is chosen by, nothing depends on them
     // codecs the pool may hold: bit i = codec id i appended through append_keys; bit 31 = tiles of
     // unknown codec were inserted. Lets the scorer pick its kernel variant without reading tiles back.

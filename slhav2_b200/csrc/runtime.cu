@@ -252,8 +252,8 @@ Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
 Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, bool** open) {
     Answer& a = tls.answer[c->device];
     if (!a.host) {
-        SLHA_CUDA(cudaHostAlloc((void**)&a.host, 256, cudaHostAllocMapped | cudaHostAllocPortable));
-        std::memset(a.host, 0, 256);
+        SLHA_CUDA(cudaHostAlloc((void**)&a.host, 512, cudaHostAllocMapped | cudaHostAllocPortable));
+        std::memset(a.host, 0, 512);
     }
     if (!a.dev) SLHA_CUDA(cudaHostGetDevicePointer((void**)&a.dev, a.host, 0));
     *host = a.host;
