@@ -601,6 +601,7 @@ __global__ void __launch_bounds__(EB_THREADS) enforce_step_kernel(PoolDev p, uin
         answer->no = no;
     };
     if (live <= budget) {
+        grid.sync();  // every block has read the counters: on the answer the caller may change them, on another stream
         if (gtid == 0) say(live, free0, ~0ull, 0u);
         return;
     }

@@ -156,3 +156,37 @@ def test_observing_a_query_is_captured_before_any_other_call():
         rt.cudaGraphDestroy(graph)
         S.set_stream(None)
     assert pools[0].read()[2].tobytes() == pools[1].read()[2].tobytes()
+
+
+def test_a_pool_is_driven_from_two_streams_in_turn():
+    # every call of a step on the other stream than the one before it, as soon as that has given its answer; budgets that are met and that are not
+    gm = S.Model.from_projection(H.make_model_pair(128, seed=61)[1], 128, 61)
+    keys = H.gaussian_keys(66, 4096, 128)
+    pools = [S.TilePool(150_000, 2**40, 1, 1, 4, 50) for _ in range(2)]
+    with Streams(2) as st:
+        for p in pools:
+            turn = 0
+
+            def other():
+                nonlocal turn
+                turn ^= p is pools[0]
+                S.set_stream(st.all[turn].value)
+
+            for i in range(30):
+                p.append_keys(gm, keys, S.CODEC_MIXED, position_base=4096 * i)
+            S.synchronize()
+            for i in range(60):
+                live = p.stats()["live_bytes"]
+                p.set_budget(live + 1000 if i % 3 else live - 32 * 8 - 96 * 3)
+                assert p.enforce_budget()
+                other()
+                p.append_keys(gm, keys[:8], S.CODEC_MIXED, position_base=130_000 + i)
+                S.synchronize()
+                p.set_budget(2**40)
+                assert p.enforce_budget()
+                other()
+                p.append_keys(gm, keys[8:9], S.CODEC_MIXED, position_base=140_000 + i)
+                S.synchronize()
+    assert pools[0].stats() == pools[1].stats()
+    for a, b in zip(pools[0].read(), pools[1].read()):
+        assert a.tobytes() == b.tobytes()

@@ -30,3 +30,14 @@ def test_every_kernel_that_lets_the_next_one_start_waits_for_the_one_before_it()
     for name, text in _sources():
         for m in re.finditer(r"\bdep_launch\(\);\s*(\S+)", text):
             assert m.group(1).startswith("dep_wait()"), (name, m.group(0))
+
+
+def test_a_kernel_whose_answer_the_host_polls_has_met_at_a_barrier_before_it_answers():
+    # The host returns on the answer: blocks that have not read the pool's counters by then would see what the caller does next.
+    text = dict(_sources())["pool.cu"]
+    for kernel, answer in (("enforce_step_kernel", r"\bsay\("), ("stats_kernel", r"\banswer\[8\] =")):
+        body = re.search(r"\b%s\(PoolDev.*?\n}\n" % kernel, text, flags=re.S).group(0)
+        assert re.search(answer, body)
+        for m in re.finditer(answer, body):
+            block = body[:m.start()]
+            assert ".sync()" in block, (kernel, body[m.start():m.start() + 60])
