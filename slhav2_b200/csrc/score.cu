@@ -304,8 +304,8 @@ struct ScoreArgs {
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
     uint32_t blocked;             // dense mode: item's scores lie in blocks of 128 tiles, block b's of its row q from list_begin + b * pad + 128 q on
     uint32_t by_fours;            // score_dense_kernel: items are the 64-row kernel's, taken four rows at a time (item e: rows 4 (e mod 16) .. of items[e / 16])
-    uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): 1, or 2 where that pass is to
-    uint32_t handoff_as;          // score them in score_kernel's arithmetic (NF4 rows always 1)
+    uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): bit 0, or bit 1 where that pass is to
+    uint32_t handoff_as;          // score them in score_kernel's arithmetic (items that begin with an NF4 tile: always bit 0)
     const uint32_t* only_flagged; // dense mode: optional, per query row: only work items one of whose rows is flagged here
     uint64_t* gbuf;               // per query row: gcap composite keys
     uint32_t gcap;

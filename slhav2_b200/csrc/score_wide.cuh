@@ -116,6 +116,15 @@ __device__ __forceinline__ void wide_sign_words(const uint4& x, uint32_t ta) {
     }
 }
 
+// Dense calls: an item's rows go to the four-row kernel's pass.  (CTAs that share the rows may hand them on for different reasons: the pass sees them all, whichever came last.)
+__device__ __forceinline__ void wide_hand_on(const ScoreArgs& a, const WorkItem& it, uint32_t as) {
+    if (threadIdx.x < it.n_queries) atomicOr(a.handoff + it.query_begin + threadIdx.x, as);
+}
+// what an item that wide_body did not score is handed on as: it is NF4 where its first tile is
+__device__ __forceinline__ uint32_t wide_hand_as(const ScoreArgs& a, const WorkItem& it) {
+    return item_kind(first_tile_flags(a, it), false) == 0 ? 1u : a.handoff_as;
+}
+
 // KIND as in score_stream_kernel (1 mixed 8/4, 2 TQ3, 3 INT4 / MX-INT4, 4 MIX3).  DENSE: every score is written to its row of
 // a.scores (row q starts at a.row_offset[q]) instead of going through the top-k filter: the dense scores of a layer for
 // callers that replace attention logits (the llama.cpp shim).
@@ -549,15 +558,21 @@ __device__ __forceinline__ void wide_body(const ScoreArgs& a, unsigned char* sme
         }
         // rows this CTA could not score (another codec, a query outside the fp16 split, a wait that ran out) go to the generic kernel, of a dense call to
         // the four-row kernel
-        if ((*reinterpret_cast<volatile uint32_t*>(ctl + 6) || stop) && tid < nq) (DENSE ? a.handoff : a.gflag)[it.query_begin + tid] = DENSE ? a.handoff_as : 1u;
+        if (*reinterpret_cast<volatile uint32_t*>(ctl + 6) || stop) {
+            if (DENSE) wide_hand_on(a, it, wide_hand_as(a, it));
+            else if (tid < nq) a.gflag[it.query_begin + tid] = 1u;
+        }
         __syncthreads();
         if (tid == 0) ctl[6] = 0u;  // (ordered before the next item's writers by the barrier at its start)
     }
     if (stop) {
         // a wait ran out (the same in all threads): the barrier's phases are no longer known, the remaining items go to the generic kernel too (of a
         // dense call to the four-row kernel)
-        for (uint32_t item_id = a.cta_begin[blockIdx.x]; item_id < item_end; ++item_id)
-            for (uint32_t q = tid; q < a.items[item_id].n_queries; q += WIDE_THREADS) (DENSE ? a.handoff : a.gflag)[a.items[item_id].query_begin + q] = DENSE ? a.handoff_as : 1u;
+        for (uint32_t item_id = a.cta_begin[blockIdx.x]; item_id < item_end; ++item_id) {
+            const WorkItem it = a.items[item_id];
+            if (DENSE) wide_hand_on(a, it, wide_hand_as(a, it));
+            else if (tid < (int)it.n_queries) a.gflag[it.query_begin + tid] = 1u;
+        }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
     __syncthreads();
@@ -586,7 +601,7 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) score_wide_dense_kernel(Score
     const uint32_t item_end = a.cta_begin[blockIdx.x + 1];
     int kind = item_kind(first_tile_flags(a, a.items[i]), false);
     while (kind == 0) {
-        if (threadIdx.x < a.items[i].n_queries) a.handoff[a.items[i].query_begin + threadIdx.x] = 1u;
+        wide_hand_on(a, a.items[i], 1u);
         if (++i == item_end) return;
         kind = item_kind(first_tile_flags(a, a.items[i]), false);
     }

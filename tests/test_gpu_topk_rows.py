@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import slhav2_b200 as S
+from oracle import pyoracle as ora
 from tests import helpers as H
 
 pytestmark = pytest.mark.gpu
@@ -108,3 +109,30 @@ def test_many_rows_whose_segments_end_inside_a_block(codec, n_seg):
     rows = [(5 * i, n + i, nq * i, nq, 7 * i) for i in range(n_seg)]
     assert sum(r[1] for r in rows) > 640_000
     _check(tiles, rows, nq * n_seg, 300, qc, qs)
+
+
+
+def test_rows_handed_on_for_different_reasons():
+    # A segment of three blocks, the first of which begins on an NF4 tile and the others meet one, scored with 16 rows: alone, and behind 49 short NF4 segments
+    # and before others in shares of 50 blocks (on 148 SMs), where the CTA that hands its rows on for the first block does so last.  The same scores bit for bit.
+    n, nq, k = 384, 16, 384
+    mixed = H.random_tiles(n, 0, seed=85)
+    nf4 = H.random_tiles(60, 2, seed=86)
+    mixed[0], mixed[130:140], mixed[300] = nf4[59], nf4[49:59], nf4[58]
+    rest = np.tile(H.random_tiles(2560, 0, seed=87), 2)
+    tiles = np.concatenate([nf4[:49], mixed, rest])
+    rows = [(i, 1, nq * i, nq, 0) for i in range(49)] + [(49, n, nq * 49, nq, 0)]
+    for _ in range((148 * 50 - 52) // 4):
+        rows.append((49 + n + len(rows), 512, nq * len(rows), nq, 0))
+    total = nq * len(rows)
+    qc, qs = H.random_queries(total, 88)
+    own = slice(49 * nq, 50 * nq)
+    dt = S.to_device(tiles)
+    alone = S.score_topk(dt, S.make_segments([(49, n, 0, nq, 0)]), qc[own], qs[own], nq, k)
+    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
+    want = ora.score_tiles(mixed, qc[own][3], qs[own][3])
+    assert np.all(np.abs(alone[1][3] - want[alone[0][3]]) <= 1e-3)
+    for _ in range(5):
+        idx, sc, cnt = S.score_topk(dt, S.make_segments(rows), qc, qs, total, k)
+        assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
+        assert np.all(cnt[own] == k) and np.array_equal(idx[own], alone[0]) and np.array_equal(sc[own].view(np.uint32), alone[1].view(np.uint32))
