@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem);                     // [cap]
     uint64_t* own = buf + cap + tid;                                       // [OWN], NT apart; then the candidates' places in their buckets
     int* hist = reinterpret_cast<int*>(buf + cap + row_own_slots(cap, NT, R));  // [ROW_BUCKETS + 1]
-    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket, 4 a thread holds too many, 8.. of a selection step, 16.. warp totals
+    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket, 8.. of a selection step, 16.. warp totals
     const uint32_t n = info.n;
     const float* row = a.scores + info.begin;
     // thread t holds the scores 4 (t + NT j) .. + 3
@@ -185,23 +185,38 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
             uint32_t at = 0;
             if (lane == 31) at = atomicAdd(&st[0], incl);
             at = __shfl_sync(0xFFFFFFFFu, at, 31) + incl - mine;
+            if (OWN < 4 * R && mine > (uint32_t)OWN) {  // all of the thread's candidates again, for want of room in its own list (read again: the unrolled form cost all launches 1.4 %)
+#pragma unroll 1
+                for (int j = 0; j < R; ++j) {
+                    const uint4 w = load4(j);
+                    const uint32_t x[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        const float s = __uint_as_float(x[c]);
+                        const bool nan = bound <= 0.0f && s != s && x[c] != ROW_ABSENT;
+                        if (!(s >= bound || nan)) continue;
+                        if (at < cap) buf[at] = make_comp(nan ? -0.0f : s, info.index_base + 4u * (tid + (uint32_t)NT * j) + c);
+                        ++at;
+                    }
+                }
+                mine = 0u;
+            }
             for (uint32_t h = 0; h < min(mine, (uint32_t)OWN); ++h, ++at) {
                 const uint64_t e = own[h * NT];
                 if (at < cap) buf[at] = make_comp(__uint_as_float((uint32_t)(e >> 32)), info.index_base + 4u * tid + (uint32_t)e);
             }
         }
-        if (OWN < 4 * R && mine > (uint32_t)OWN) st[4] = 1u;
         __syncthreads();
         if (st[0] >= k || bound == -INFINITY) break;
         bound = -INFINITY;  // (the sample misled)
         __syncthreads();
-        if (tid == 0) st[0] = st[4] = 0u;
+        if (tid == 0) st[0] = 0u;
         __syncthreads();
     }
     const uint32_t got = st[0], m = min(got, k);
     uint32_t* const out_index = a.out_index + (size_t)Q * k;
     float* const out_score = a.out_score + (size_t)Q * k;
-    const bool listed = got <= cap && (OWN == 4 * R || !st[4]);
+    const bool listed = got <= cap;
     if (listed && got <= ROW_RANKED) {
         // Few candidates: a candidate's place is the number of larger ones, counted by SPLIT threads in turn (a slice of the list each).
         constexpr uint32_t SPLIT = 2;
@@ -261,7 +276,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         }
     } else {
         // Too many candidates (many equal scores, or outliers far from the rest): a radix selection of the k-th largest score word, what
-        // lies above it, and of the scores equal to it those with the lowest indices.  (At least k are there.  The row is read again: held on to for
+        // lies above it, and of the scores equal to it those with the lowest indices.  (More than k are there.  The row is read again: held on to for
         // this, it would cost every launch registers.)
         auto word = [](uint32_t bits) { return (bits & 0x7FFFFFFFu) > 0x7F800000u ? 0x7FFFFFFFu : score_key(__uint_as_float(bits)); };
         uint32_t prefix = 0, need = k;

@@ -100,6 +100,26 @@ def test_cold_slots_are_no_candidates():
         assert np.array_equal(np.sort(idx[j, :300]), left) and np.all(np.abs(sc[j, :300] - want[j, order]) <= 1e-3)
 
 
+@pytest.mark.parametrize("n,k,live", [(16384, 64, lambda s: s // 4 % 512 == 3), (32768, 100, lambda s: s // 4 % 512 == 511), (16384, 2048, lambda s: s // 4 % 512 < 60), (30000, 4096, lambda s: s // 4 % 512 < 64)])
+def test_fewer_slots_than_winners_that_few_threads_hold(n, k, live):
+    # what is left of a pool lies where a thread holds more candidates than its own list has room for, fewer than k in all
+    tiles = np.tile(H.random_tiles(2000, 3, seed=73), n // 2000 + 1)[:n]
+    left = np.flatnonzero(live(np.arange(n)))
+    pool = S.TilePool(n, 2**40)
+    pool.insert(tiles)
+    for s in np.setdiff1d(np.arange(n), left):
+        pool.evict(int(s))
+    qc, qs = H.random_queries(4, 74)
+    idx, sc, cnt = pool.score_topk(qc, qs, 4, k)
+    m = min(k, len(left))
+    assert np.all(cnt == m) and np.all(idx[:, m:] == 0xFFFFFFFF) and np.all(np.isneginf(sc[:, m:]))
+    want = S.score_tiles(S.to_device(tiles), n, qc, qs, 4)
+    for j in range(4):
+        order = left[np.lexsort((left, -want[j, left]))][:m]
+        assert len(set(idx[j, :m])) == m and set(idx[j, :m]) <= set(left)
+        assert np.all(np.abs(sc[j, :m] - want[j, order]) <= 1e-3 * (1 + np.abs(want[j, order])))
+
+
 @pytest.mark.parametrize("codec,n_seg", [(0, 100), (4, 100), (2, 60)])
 def test_many_rows_whose_segments_end_inside_a_block(codec, n_seg):
     # above what every call's rows are scored as a whole for: the rule's side of them; shares that are cut in blocks of 128 tiles
