@@ -5,7 +5,7 @@
 // a launch and a chain of latencies.  Scores written as a whole cost four bytes a tile and row, which the L2 keeps, and need no threshold while they
 // are made.  Here a row's scores go to registers, a sample of them gives a bound that little more than k reach, every thread keeps the few of its own that do,
 // and those are compacted: up to ROW_RANKED are ordered by comparing each with all, more by buckets between the bound and the largest score of the
-// sample and by comparing inside a bucket.
+// sample and by comparing inside a bucket, or, where that is crowded (equal scores, one far from the rest), by a radix sort.
 // Bound: the latencies between the block barriers, and for many rows the instructions a score costs.  us a call, streamed and merged / whole rows: 4096
 // INT4 tiles, k = 64 19.6 / 10.6, 8 x 8192 mixed tiles x 4 rows, k = 256 26.6 / 13.2, 8 x 16 384 TQ3 x 64 rows 85 / 47; the kernel itself about 8 us of the last.  With the
 // candidates ordered by buckets alone 13.6 and 48.1; with a histogram of the whole row in place of the sample 20 us for 512 rows of 16 384.
@@ -38,6 +38,86 @@ constexpr int ROW_HIST_INTS = ROW_BUCKETS + 64;
 __host__ __device__ constexpr size_t row_own_slots(uint32_t cap, int nt, int r) { return (size_t)nt * row_own(r) > cap ? (size_t)nt * row_own(r) : cap; }
 inline size_t row_smem(uint32_t cap, int nt, int r) { return ((size_t)cap + row_own_slots(cap, nt, r)) * 8 + (size_t)(ROW_HIST_INTS + 64) * 4 + (size_t)(cap + 1) / 2 * 4; }
 constexpr uint32_t ROW_RANKED = 192;              // candidates that are ordered by comparing each with all
+// Candidates of a bucket up to which the bucket is ordered by comparing each with all.  Above, all candidates are sorted: comparing goes by the bucket's square (us a call by comparing / sorting:
+// 4 rows of 6000 equal scores 1004 / 38, of 4096 scores with one 10 000 times the others, k = 4096 466 / 54), sorting by the candidates (4 rows of 30 000, each score thirty times, k = 4096, buckets of
+// some hundred 42 / 67).
+constexpr uint32_t ROW_CROWD = 512;
+
+// The CTA's hist[ROW_BUCKETS] into c, ROW_BUCKETS / NT a thread; the sum of the counts before the thread's.  (st[16 ..]: a word a warp.)
+template <int NT>
+__device__ __forceinline__ int row_scan(const int* hist, uint32_t* st, int (&c)[ROW_BUCKETS / NT]) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int sum = 0;
+#pragma unroll
+    for (int j = 0; j < ROW_BUCKETS / NT; ++j) {
+        c[j] = hist[tid * (ROW_BUCKETS / NT) + j];
+        sum += c[j];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+        if ((int)lane >= o) incl += y;
+    }
+    if (lane == 31) st[16 + warp] = (uint32_t)incl;
+    __syncthreads();
+    const int before = lane < warp ? (int)st[16 + lane] : 0;
+    return incl - sum + __reduce_add_sync(0xFFFFFFFFu, before);
+}
+// buf[0 .. count) in descending order, there or behind cap: a stable radix sort, six bits at a time where the keys differ.  A warp takes a run of the keys; hist[16 x digit + warp] holds its
+// counts, then its places.
+template <int NT>
+__device__ __forceinline__ const uint64_t* row_sort(uint64_t* buf, uint32_t cap, uint32_t count, int* hist, uint32_t* st) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int PER = ROW_BUCKETS / NT;
+    uint64_t *from = buf, *to = buf + cap;
+    if (tid == 0) st[8] = st[9] = 0u;
+    __syncthreads();
+    uint64_t differ = 0;
+    for (uint32_t i = tid; i < count; i += NT) differ |= from[i] ^ from[0];
+    const uint32_t lo = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)differ), hi = __reduce_or_sync(0xFFFFFFFFu, (uint32_t)(differ >> 32));
+    if (lane == 0) {
+        atomicOr(&st[8], lo);
+        atomicOr(&st[9], hi);
+    }
+    __syncthreads();
+    differ = (uint64_t)st[9] << 32 | st[8];
+    const uint32_t run = (count + NT - 1) / NT * 32, first = min(count, warp * run), end = min(count, first + run);
+    for (int shift = 0; shift < 64; shift += 6) {
+        if (!(differ >> shift & 63u)) continue;
+        for (uint32_t b = tid; b < (uint32_t)ROW_BUCKETS; b += NT) hist[b] = 0;
+        __syncthreads();
+        for (uint32_t i0 = first; i0 < end; i0 += 32) {
+            const bool in = i0 + lane < end;
+            const uint32_t digit = in ? 63u - (uint32_t)(from[i0 + lane] >> shift & 63u) : 64u, same = __match_any_sync(0xFFFFFFFFu, digit);
+            if (in && (uint32_t)__ffs(same) - 1u == lane) hist[16 * digit + warp] += __popc(same);
+            __syncwarp();
+        }
+        __syncthreads();
+        int c[PER], at = row_scan<NT>(hist, st, c);
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            hist[tid * PER + j] = at;
+            at += c[j];
+        }
+        __syncthreads();
+        for (uint32_t i0 = first; i0 < end; i0 += 32) {
+            const bool in = i0 + lane < end;
+            const uint64_t key = in ? from[i0 + lane] : 0ull;
+            const uint32_t digit = in ? 63u - (uint32_t)(key >> shift & 63u) : 64u, same = __match_any_sync(0xFFFFFFFFu, digit);
+            const int place = in ? hist[16 * digit + warp] : 0;
+            __syncwarp();
+            if (in) to[place + __popc(same & ((1u << lane) - 1u))] = key;
+            if (in && (uint32_t)__ffs(same) - 1u == lane) hist[16 * digit + warp] = place + __popc(same);
+            __syncwarp();
+        }
+        __syncthreads();
+        uint64_t* const was = from;
+        from = to;
+        to = was;
+    }
+    return from;
+}
 
 // R: 4 R scores a thread, n <= 4 R x threads
 template <int NT, int R>
@@ -51,7 +131,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem);                     // [cap]
     uint64_t* own = buf + cap + tid;                                       // [OWN], NT apart; then the candidates' places in their buckets
     int* hist = reinterpret_cast<int*>(buf + cap + row_own_slots(cap, NT, R));  // [ROW_BUCKETS + 1]
-    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket, 8.. of a selection step, 16.. warp totals
+    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket and 10, 11, 13 what a closer look at it needs, 5, 8, 9 of a selection step, 12 a bucket is crowded, 16.. warp totals
     const uint32_t n = info.n;
     const float* row = a.scores + info.begin;
     // thread t holds the scores 4 (t + NT j) .. + 3
@@ -68,7 +148,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     uint4 v[R];
 #pragma unroll
     for (int j = 0; j < R; ++j) v[j] = load4(j);
-    if (tid < 16) st[tid] = tid == 1 ? 0xFFFFFFFFu : 0u;
+    if (tid < 16) st[tid] = tid == 1 || tid == 10 ? 0xFFFFFFFFu : 0u;
     for (int b = (int)tid; b <= ROW_BUCKETS; b += NT) hist[b] = 0;
     __syncthreads();
     // (What one pass over the row computed from the scores is not kept for the next: it would take as many registers as they do.)
@@ -104,47 +184,83 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         }
     }
     __syncthreads();
-    // places of the buckets: the counts before them
-    auto scan = [&](int (&c)[PER]) {
-        int sum = 0;
-#pragma unroll
-        for (int j = 0; j < PER; ++j) {
-            c[j] = hist[tid * PER + j];
-            sum += c[j];
-        }
-        int incl = sum;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if ((int)lane >= o) incl += y;
-        }
-        if (lane == 31) st[16 + warp] = (uint32_t)incl;
-        __syncthreads();
-        int before = lane < warp ? (int)st[16 + lane] : 0;
-        return incl - sum + __reduce_add_sync(0xFFFFFFFFu, before);
-    };
     const bool ranged = st[2] > st[1];
     float low = key_score(ranged ? st[1] : score_key(0.0f)), bound = -INFINITY;
     const float top = key_score(ranged ? st[2] : score_key(1.0f));
     if (sampled && ranged) {
-        const float inv = (float)ROW_BUCKETS / (top - low);  // (a range that overflows puts all in one bucket)
+        const float part = (float)k * (0.25f / (float)STEP);
+        const int want = (int)(1.25f * part + 3.0f * sqrtf(part)) + 2, most = (int)(cap * 3u / (16u * STEP));
+        float inv = (float)ROW_BUCKETS / (top - low);  // (a range that overflows puts all in one bucket)
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             const float s = __uint_as_float(v[j].x);
             if (((tid + j) & (STEP - 1)) == 0 && fabsf(s) < INFINITY) atomicAdd(&hist[min(max(__float2int_rz((top - s) * inv), 0), ROW_BUCKETS - 1)], 1);
         }
         __syncthreads();
-        const float part = (float)k * (0.25f / (float)STEP);
-        const int want = (int)(1.25f * part + 3.0f * sqrtf(part)) + 2;
-        int c[PER], at = scan(c);
+        int c[PER], at = row_scan<NT>(hist, st, c);
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
-            if (at < want && at + c[j] >= want) st[3] = tid * PER + j + 1;
+            if (at < want && at + c[j] >= want) {
+                st[3] = tid * PER + j + 1;
+                if (at + c[j] > most) st[13] = at + 1;
+            }
             at += c[j];
             hist[tid * PER + j] = 0;
         }
         __syncthreads();
         if (st[3] && st[3] < (uint32_t)ROW_BUCKETS) bound = top - (float)st[3] / inv;  // (zero: the sample holds too few, all are candidates)
+        // Scores far from the rest (an attention sink) leave that bucket with more than the candidates' slots hold: its own scores in buckets, up to three times.  (128 rows of 30 000, one score
+        // 10 000 times the others, k = 1024: 449 us a call without, 81 with it.)
+        if (__builtin_expect(st[13] != 0u, 0)) {
+            float upper = top, lower = low;
+#pragma unroll 1
+            for (int zoom = 0; zoom < 3 && st[13]; ++zoom) {
+                const int b = (int)st[3] - 1, above = (int)st[13] - 1;
+                uint32_t mn = 0xFFFFFFFFu, mx = 0u;
+#pragma unroll
+                for (int j = 0; j < R; ++j) {
+                    const float s = __uint_as_float(v[j].x);
+                    if (((tid + j) & (STEP - 1)) == 0 && s >= lower && s <= upper && min(max(__float2int_rz((upper - s) * inv), 0), ROW_BUCKETS - 1) == b) {
+                        mn = min(mn, score_key(s));
+                        mx = max(mx, score_key(s));
+                    }
+                }
+                mn = __reduce_min_sync(0xFFFFFFFFu, mn);
+                mx = __reduce_max_sync(0xFFFFFFFFu, mx);
+                if (lane == 0 && mx) {
+                    atomicMin(&st[10], mn);
+                    atomicMax(&st[11], mx);
+                }
+                __syncthreads();
+                lower = key_score(st[10]);
+                upper = key_score(st[11]);
+                __syncthreads();
+                if (!(lower < upper)) break;  // (all equal, the same in every thread)
+                if (tid == 0) {
+                    st[3] = st[11] = st[13] = 0u;
+                    st[10] = 0xFFFFFFFFu;
+                }
+                inv = (float)ROW_BUCKETS / (upper - lower);
+#pragma unroll
+                for (int j = 0; j < R; ++j) {
+                    const float s = __uint_as_float(v[j].x);
+                    if (((tid + j) & (STEP - 1)) == 0 && s >= lower && s <= upper) atomicAdd(&hist[min(max(__float2int_rz((upper - s) * inv), 0), ROW_BUCKETS - 1)], 1);
+                }
+                __syncthreads();
+                int c[PER], at = row_scan<NT>(hist, st, c) + above;
+#pragma unroll
+                for (int j = 0; j < PER; ++j) {
+                    if (at < want && at + c[j] >= want) {
+                        st[3] = tid * PER + j + 1;
+                        if (at + c[j] > most) st[13] = at + 1;
+                    }
+                    at += c[j];
+                    hist[tid * PER + j] = 0;
+                }
+                __syncthreads();
+                if (st[3]) bound = st[3] < (uint32_t)ROW_BUCKETS ? upper - (float)st[3] / inv : lower;
+            }
+        }
     }
     // what reaches the bound: the thread's own candidates
     uint32_t mine;
@@ -217,6 +333,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     uint32_t* const out_index = a.out_index + (size_t)Q * k;
     float* const out_score = a.out_score + (size_t)Q * k;
     const bool listed = got <= cap;
+    bool crowded = false;
     if (listed && got <= ROW_RANKED) {
         // Few candidates: a candidate's place is the number of larger ones, counted by SPLIT threads in turn (a slice of the list each).
         constexpr uint32_t SPLIT = 2;
@@ -246,11 +363,12 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         uint16_t* const number = reinterpret_cast<uint16_t*>(st + 64);
         for (uint32_t i = tid; i < got; i += NT) number[i] = (uint16_t)atomicAdd(&hist[bucket(buf[i])], 1);
         __syncthreads();
-        int c[PER], at = scan(c);
+        int c[PER], at = row_scan<NT>(hist, st, c);
 #pragma unroll
         for (int j = 0; j < PER; ++j) {
             hist[tid * PER + j] = at;
             at += c[j];
+            if (c[j] > (int)ROW_CROWD) st[12] = 1u;
         }
         if (tid == NT - 1) hist[ROW_BUCKETS] = at;
         __syncthreads();
@@ -259,7 +377,8 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
             placed[hist[bucket(key)] + (int)number[i]] = key;
         }
         __syncthreads();
-        for (uint32_t i = tid; i < got; i += NT) {
+        crowded = st[12] != 0u;
+        for (uint32_t i = tid; i < got && !crowded; i += NT) {
             const uint64_t key = placed[i];
             const int b = bucket(key);
             const int s0 = hist[b], e0 = hist[b + 1];
@@ -333,7 +452,6 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         }
         __syncthreads();
         if (tid == 0) st[5] = 0u;
-        for (uint32_t i = tid; i < a.kp2; i += NT) buf[i] = 0ull;
         __syncthreads();
 #pragma unroll 1
         for (int j = 0; j < R; ++j) {  // (4 NT scores at a time in index order, so that the lowest indices among the equal ones come first)
@@ -369,20 +487,8 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
             need -= min(need, all);
             __syncthreads();
         }
-        for (uint32_t size = 2; size <= a.kp2; size <<= 1)
-            for (uint32_t stride = size >> 1; stride; stride >>= 1) {
-                for (uint32_t i = tid; i < a.kp2 / 2; i += NT) {
-                    const uint32_t p = 2 * i - (i & (stride - 1)), q = p + stride;
-                    const uint64_t x = buf[p], y = buf[q];
-                    if ((x < y) == ((p & size) == 0)) {
-                        buf[p] = y;
-                        buf[q] = x;
-                    }
-                }
-                __syncthreads();
-            }
-        emit_sorted(buf, k, k, Q, a.out_index, a.out_score, nullptr);
     }
+    if (__builtin_expect(crowded || !listed, 0)) emit_sorted(row_sort<NT>(buf, cap, listed ? got : k, hist, st), m, k, Q, a.out_index, a.out_score, nullptr);
     if (tid == 0) {
         if (a.out_count) a.out_count[Q] = m;
         a.stats[2 * Q] = got;

@@ -156,3 +156,28 @@ def test_rows_handed_on_for_different_reasons():
         idx, sc, cnt = S.score_topk(dt, S.make_segments(rows), qc, qs, total, k)
         assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
         assert np.all(cnt[own] == k) and np.array_equal(idx[own], alone[0]) and np.array_equal(sc[own].view(np.uint32), alone[1].view(np.uint32))
+
+
+@pytest.mark.parametrize("n,k", [(3000, 512), (4096, 2048), (6000, 4096), (30000, 1024)])
+def test_equal_scores_and_one_far_from_the_rest_cost_no_multiple(n, k):
+    # the selection's device time beside that of scores that differ: within ten times (comparing equal scores with one another took 30 to 60 times as long)
+    base = H.random_tiles(1000, 0, seed=31)
+    rng = np.random.default_rng(n)
+    nq = 128
+    qc, qs = H.random_queries(nq, 90)
+    seg = S.make_segments([(0, n, 4 * i, 4, 0) for i in range(nq // 4)])
+    took = {}
+    for shape in ("differ", "equal", "far"):
+        tiles = base[rng.integers(0, 1000, n)] if shape != "equal" else np.repeat(base[:1], n)
+        tiles["scale"] *= rng.uniform(0.9, 1.1, n).astype(F) if shape != "equal" else F(1)
+        if shape == "far":
+            tiles["scale"][n // 3] *= F(1e4)
+        dt = S.to_device(tiles)
+        args = dt, seg, S.to_device(qc), S.to_device(qs), nq, k, S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * 4)
+        S.score_topk(*args)
+        S.timing_begin(9)
+        for _ in range(9):
+            S.score_topk(*args)
+        took[shape] = float(np.median(S.timing_end(9)[1]))
+        _check(tiles, [(0, n, 0, 2, 0)], 2, k, qc[:2], qs[:2])
+    assert max(took["equal"], took["far"]) < 10 * took["differ"], took
