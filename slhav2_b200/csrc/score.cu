@@ -474,14 +474,16 @@ __device__ __forceinline__ uint32_t dense_first(const ScoreArgs& a, uint32_t cta
 }
 
 // Work items that a dense kernel's CTA could not score on the tensor cores (a tile of another codec than its item's first, a query outside the fp16
-// split), to be scored in score_kernel's arithmetic once the CTA is through: in its loop the call would cost registers.
-struct Undone {
-    uint32_t n;
-    uint32_t item[31];  // (more than these: all of the CTA's items)
-};
-__device__ __forceinline__ void undone_add(Undone& u, uint32_t item) {  // one thread of the CTA
-    if (u.n < 31u) u.item[u.n] = item;
-    ++u.n;
+// split): a bit each in shared memory, to be scored in score_kernel's arithmetic once the CTA is through.  (In its loop the call would cost registers, 70 of which it spilled.)
+constexpr int UNDONE_WORDS = 4096;
+// 0: a bit an item, as for any call up to 19 million of them; above, 2^shift items share one
+__device__ __forceinline__ uint32_t undone_shift(uint32_t items) {
+    return items <= 32u * UNDONE_WORDS ? 0u : 32u - (uint32_t)__clz((items - 1u) / (32u * UNDONE_WORDS));
+}
+// (one thread of the CTA)
+__device__ __forceinline__ void undone_add(const ScoreArgs& a, uint32_t* bits, uint32_t item) {
+    const uint32_t first = dense_first(a, blockIdx.x), e = (item - first) >> undone_shift(dense_first(a, blockIdx.x + 1) - first);
+    bits[e >> 5] |= 1u << (e & 31u);
 }
 // Dense scores of one work item by the whole CTA, rows query_begin .. + nq (four at most).  smem: 4 KB, and 4 KB a warp.
 __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem& it, uint32_t query_begin, int nq, unsigned char* smem) {
@@ -541,12 +543,14 @@ __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem&
     }
     __syncthreads();
 }
-// What is left at a CTA's end (all of its shared memory is free).
-__device__ __noinline__ void finish_undone(const ScoreArgs& a, const Undone& u, unsigned char* smem) {
+// What is left at a CTA's end (all of its shared memory but the bits is free).
+__device__ __noinline__ void finish_undone(const ScoreArgs& a, const uint32_t* bits, unsigned char* smem) {
     __syncthreads();
-    const uint32_t m = u.n, first = dense_first(a, blockIdx.x), end = dense_first(a, blockIdx.x + 1);
-    for (uint32_t j = 0; j < (m > 31u ? end - first : m); ++j) {
-        const WorkItem it = dense_item(a, m > 31u ? first + j : u.item[j]);
+    const uint32_t first = dense_first(a, blockIdx.x), items = dense_first(a, blockIdx.x + 1) - first, shift = undone_shift(items);
+    for (uint32_t e = 0; e < items; ++e) {
+        const uint32_t bit = e >> shift;
+        if (!(bits[bit >> 5] >> (bit & 31u) & 1u)) continue;
+        const WorkItem it = dense_item(a, first + e);
         for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
     }
 }

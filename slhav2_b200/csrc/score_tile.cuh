@@ -35,7 +35,7 @@ constexpr uint32_t ST_TMEM = 128;                      // TMEM columns of a warp
 constexpr int st_accs(int kind) { return kind == 2 || kind == 4 ? 3 : 4; }
 constexpr uint32_t st_d_col(int kind) { return kind == 2 || kind == 4 ? 72u : 64u; }
 constexpr size_t st_smem_bytes(bool dense) {  // (only dense calls meet NF4 tiles here)
-    return 1024 + (dense ? NF4_LUT_BYTES : 0) + ST_B_BYTES + (size_t)(ST_THREADS / 32) * ST_DEPTH * ST_SLOT + ST_TAIL_BYTES;
+    return 1024 + (dense ? NF4_LUT_BYTES + 4 * UNDONE_WORDS : 0) + ST_B_BYTES + (size_t)(ST_THREADS / 32) * ST_DEPTH * ST_SLOT + ST_TAIL_BYTES;
 }
 
 // instruction descriptor: D fp32, A and B fp16, both K-major, N columns, M = 128
@@ -305,7 +305,7 @@ __device__ __forceinline__ bool st_alien(int kind, uint32_t flags) {
 
 // What a thread keeps from one work item to the next.
 struct TileCta {
-    uint32_t base_s;   // shared memory, 1024-byte aligned: B | [NF4 table] | ring | sign words | thresholds (keys, floats) | mappings | barriers, flags | query scales
+    uint32_t base_s;   // shared memory, 1024-byte aligned: B | [NF4 table] | ring | sign words | thresholds (keys, floats) | mappings | barriers, flags | query scales | [bits of undone items]
     unsigned char* base;
     uint32_t tmem;
     int uw;            // warp index, known to be uniform
@@ -313,11 +313,16 @@ struct TileCta {
     bool table;        // the NF4 table is there
     uint32_t phase;    // of the warpgroup's mbarrier
     bool failed;       // a wait of this warp ran out
+    bool undone;       // dense: an item was left, see undone_add
 };
 template <bool DENSE>
 struct TileLayout {
-    static constexpr uint32_t LUT = ST_B_BYTES, RING = LUT + (DENSE ? NF4_LUT_BYTES : 0), TAIL = RING + (ST_THREADS / 32) * ST_DEPTH * ST_SLOT;
+    static constexpr uint32_t LUT = ST_B_BYTES, RING = LUT + (DENSE ? NF4_LUT_BYTES : 0), TAIL = RING + (ST_THREADS / 32) * ST_DEPTH * ST_SLOT, UNDONE = TAIL + ST_TAIL_BYTES;
 };
+__device__ __forceinline__ unsigned char* tile_base(unsigned char* smem_raw) {
+    const uint32_t at = (uint32_t)__cvta_generic_to_shared(smem_raw);
+    return smem_raw + (((at + 1023u) & ~1023u) - at);
+}
 template <bool DENSE>
 __device__ __forceinline__ TileCta tile_open(unsigned char* smem_raw) {
     TileCta t;
@@ -325,8 +330,8 @@ __device__ __forceinline__ TileCta tile_open(unsigned char* smem_raw) {
     // (the four warpgroups' leaders sit on different schedulers)
     const bool elected = elect_one();
     t.leader = elected && (t.uw & 3) == (t.uw >> 2);
-    t.base_s = ((uint32_t)__cvta_generic_to_shared(smem_raw) + 1023u) & ~1023u;
-    t.base = smem_raw + (t.base_s - (uint32_t)__cvta_generic_to_shared(smem_raw));
+    t.base = tile_base(smem_raw);
+    t.base_s = (uint32_t)__cvta_generic_to_shared(t.base);
     const uint32_t tail_s = t.base_s + TileLayout<DENSE>::TAIL;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(t.base + TileLayout<DENSE>::TAIL + 256u);
     if (threadIdx.x == 0) {
@@ -344,7 +349,7 @@ __device__ __forceinline__ TileCta tile_open(unsigned char* smem_raw) {
     t.tmem = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
     t.table = false;
     t.phase = 0u;
-    t.failed = false;
+    t.failed = t.undone = false;
     return t;
 }
 __device__ __forceinline__ void tile_close(const TileCta& t) {
@@ -370,7 +375,7 @@ __device__ __forceinline__ uint32_t first_tile_flags(const ScoreArgs& a, const W
 // whole streams (see the planner).  A tile of another codec than KIND's, or a query outside the fp16 split, hands the
 // item's query rows to the generic kernel.
 template <int KIND, bool IL, bool DENSE, bool KINDS>
-__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, WorkItem& it, uint32_t& flags0, bool nf4_too = false, Undone* undone = nullptr) {
+__device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, WorkItem& it, uint32_t& flags0, bool nf4_too = false) {
     constexpr int NWG = ST_WG, NWARPS = 4 * NWG, NACC = st_accs(KIND);
     constexpr uint32_t STRIDE = ST_TMEM, DCOL = st_d_col(KIND);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wg = warp >> 2, wq = warp & 3;
@@ -447,7 +452,8 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             if (!f) continue;  // (the same in the whole CTA)
             if (f & 2u) {
                 if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
-                if (tid == 0) undone_add(*undone, item_id);
+                if (tid == 0) undone_add(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
+                cta.undone = true;
                 continue;
             }
         }
@@ -851,7 +857,10 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
         if (*reinterpret_cast<volatile uint32_t*>(bail)) {  // (the same in the whole CTA)
             // rows this CTA could not score on the tensor cores go to the generic kernel as a whole; of dense calls the item, at the CTA's end
             if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
-            if (DENSE && tid == 0) undone_add(*undone, item_id);
+            if (DENSE) {
+                if (tid == 0) undone_add(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
+                cta.undone = true;
+            }
         }
         __syncthreads();
         if (tid == 0) *bail = 0u;  // (ordered before the next item's writers by the barrier at its start)
@@ -883,13 +892,11 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) 
 // tiles is decoded as NF4 throughout.
 __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid_constant__ ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ Undone undone;
     dep_launch();
     dep_wait();
     if (a.refused && *a.refused) return;
     uint32_t i = dense_first(a, blockIdx.x);
     const uint32_t item_end = dense_first(a, blockIdx.x + 1);
-    if (threadIdx.x == 0) undone.n = 0u;
     if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
         uint32_t f = 0;
         for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS) {
@@ -904,19 +911,22 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     if (threadIdx.x == 32) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_sign + (size_t)it.query_begin * 8));
     if (threadIdx.x == 64 && a.row_offset) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.row_offset + it.query_begin));
     const bool nf4_too = a.nf4_table == 1u || (a.nf4_table == 2u && (first_tile_flags(a, a.stream_items[0]) & F_NF4));
+    uint32_t* const bits = reinterpret_cast<uint32_t*>(tile_base(smem_raw) + TileLayout<true>::UNDONE);
+    for (uint32_t w = threadIdx.x; w < min((item_end - i + 31u) / 32u, (uint32_t)UNDONE_WORDS); w += ST_THREADS) bits[w] = 0u;  // (ordered by tile_open's barrier)
     TileCta cta = tile_open<true>(smem_raw);
     for (;;) {
         switch (item_kind(flags, nf4_too)) {
-            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
-            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
-            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
-            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
-            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, it, flags, nf4_too, &undone); break;
+            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
+            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
         }
         if (i >= item_end) break;
     }
     tile_close(cta);
-    finish_undone(a, undone, smem_raw);
+    static_assert(4096 + (ST_THREADS / 32) * BLK_BYTES <= TileLayout<true>::UNDONE, "below the bits");
+    if (cta.undone) finish_undone(a, bits, smem_raw);
 }
 
 }  // namespace

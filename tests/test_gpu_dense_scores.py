@@ -375,3 +375,34 @@ def test_row_offsets_in_device_memory_are_checked_there(nq, codec, tail):
         assert np.all(out.download(F, nq * row) == 9.0) and np.all(host == 9.0)
     S.score_segments(tiles, seg, dq, ds, nq, out, S.to_device(off), row, fill=-3.0)  # a refused call leaves nothing behind
     assert np.array_equal(out.download(F, nq * row), want)
+
+
+@pytest.mark.parametrize("nq,per_cta", [(1, 80), (16, 20)])
+def test_segments_that_are_left_to_the_generic_arithmetic_leave_the_others_as_they_are(nq, per_cta):
+    # more such segments in a CTA (148 SMs) than a short list holds, every second one: the rows of the others keep their bits, in dense calls and in top-k
+    m, n_seg = 5, 148 * per_cta
+    base = H.random_tiles(1000, 3, seed=540)
+    tiles = base[np.random.default_rng(nq).integers(0, 1000, m * n_seg)]
+    mixed = tiles.copy()
+    odd = np.repeat(np.arange(n_seg) % 2 == 1, nq)
+    mixed[m + 2::2 * m] = np.resize(H.random_tiles(100, 4, seed=541), n_seg // 2)
+    total = nq * n_seg
+    qc, qs = (np.resize(x, (total,) + x.shape[1:]) for x in H.random_queries(97, 542))
+    seg = S.make_segments([(m * i, m, nq * i, nq, 0) for i in range(n_seg)])
+    off = np.arange(total, dtype=np.uint64) * m
+
+    def run(t):
+        dt = S.to_device(t)
+        dense = S.score_segments(dt, seg, qc, qs, total, np.zeros((total, m), F), off, m)
+        idx, sc, _ = S.score_topk(dt, seg, qc, qs, total, m)
+        return dense, idx, sc, S.last_score_stats()["rows_handed_to_generic_kernel"]
+
+    clean, now = run(tiles), run(mixed)
+    assert clean[3] == 0 and now[3] == odd.sum()
+    for a, b in zip(clean[:3], now[:3]):
+        assert a[~odd].tobytes() == b[~odd].tobytes()
+    for i in range(1, n_seg, 97):
+        if i % 2:
+            for j in (nq * i, nq * i + nq - 1):
+                want = ora.score_tiles(mixed[m * i:m * i + m], qc[j], qs[j])
+                assert np.all(np.abs(now[0][j] - want) <= 1e-3 * (1 + np.abs(want))) and np.all(np.abs(now[2][j] - want[now[1][j]]) <= 1e-3)
