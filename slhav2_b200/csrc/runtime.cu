@@ -21,7 +21,11 @@ Status cuda_status(cudaError_t e, const char* what) {
 }
 
 static std::atomic<uint64_t> g_launches{0};
-void count_launch(int n) { g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed); }
+static thread_local uint64_t g_thread_launches = 0;
+void count_launch(int n) {
+    g_launches.fetch_add((uint64_t)n, std::memory_order_relaxed);
+    g_thread_launches += (uint64_t)n;
+}
 int sm_count(int device) {
     static std::atomic<int> known[16];
     std::atomic<int>& n = known[device & 15];
@@ -73,23 +77,30 @@ struct LastUse {
     unsigned long long stream = 0;
     bool queued = false;
 };
+// (at the thread's end, when any device may be current)
+void drain(int device) {
+    if (cudaSetDevice(device) == cudaSuccess) cudaDeviceSynchronize();
+}
 struct Answer {
+    int device = 0;
     uint32_t* host = nullptr;
     uint32_t* dev = nullptr;
     bool open = false;  // a kernel may still write there: nobody has seen its answer (a call that ended by an exception)
     ~Answer() {
-        if (open) cudaDeviceSynchronize();
+        if (open) drain(device);
         if (host) cudaFreeHost(host);
     }
 };
-// Where kernels write a call's short host outputs.  A call that fails leaves its part in use for good: its kernels may still write there.
+// Where kernels write a call's short host outputs.  Empty between calls: what a failed call has left is given back at its end (see ~CallScope).
 constexpr size_t OUT_PAGE = 4096, OUT_BYTES = 1024;
 struct OutPage {
+    int device = 0;
     unsigned char* host = nullptr;
     unsigned char* dev = nullptr;
     size_t used = 0;
+    uint64_t launched = 0;  // the thread's launches when the call under way took its first part
     ~OutPage() {
-        if (used) cudaDeviceSynchronize();
+        if (used) drain(device);
         if (host) cudaFreeHost(host);
     }
 };
@@ -252,6 +263,7 @@ Status ctx_copy_table(Ctx* c, void* dev, const void* src, size_t bytes) {
 Status ctx_answer(Ctx* c, volatile uint32_t** host, uint32_t** dev, bool** open) {
     Answer& a = tls.answer[c->device];
     if (!a.host) {
+        a.device = c->device;
         SLHA_CUDA(cudaHostAlloc((void**)&a.host, 512, cudaHostAllocMapped | cudaHostAllocPortable));
         std::memset(a.host, 0, 512);
     }
@@ -292,6 +304,12 @@ CallScope::CallScope() {
 
 CallScope::~CallScope() {
     if (!c) return;
+    // A call that failed behind stage_out: nothing writes its part of the page where nothing was launched, and nothing once the stream is drained.
+    OutPage& page = tls.outs[c->device];
+    if (page.used) {
+        if (page.launched == g_thread_launches || cudaStreamSynchronize(c->stream) == cudaSuccess) page.used = 0;
+        else cudaGetLastError();
+    }
     UploadSlot* up = tls.upload_used[c->device];
     if (c->own_stream && !up) return;  // library stream: the call drained it before returning
     bool arena = false;
@@ -358,11 +376,13 @@ Status stage_out(Ctx* c, void* user, size_t bytes, StagedOut* out, bool in_place
     if (in_place_if_pinned && bytes <= OUT_BYTES && !capturing(c->stream)) {
         OutPage& o = tls.outs[c->device];
         if (!o.host) {
+            o.device = c->device;
             SLHA_CUDA(cudaHostAlloc((void**)&o.host, OUT_PAGE, cudaHostAllocMapped | cudaHostAllocPortable));
             SLHA_CUDA(cudaHostGetDevicePointer((void**)&o.dev, o.host, 0));
         }
         const size_t take = (bytes + 15) / 16 * 16;
         if (o.used + take <= OUT_PAGE) {
+            if (!o.used) o.launched = g_thread_launches;
             out->dev = o.dev + o.used;
             out->page = o.host + o.used;
             o.used += take;

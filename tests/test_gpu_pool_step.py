@@ -190,3 +190,32 @@ def test_a_pool_is_driven_from_two_streams_in_turn():
     assert pools[0].stats() == pools[1].stats()
     for a, b in zip(pools[0].read(), pools[1].read()):
         assert a.tobytes() == b.tobytes()
+
+
+def test_refused_calls_leave_the_page_for_short_outputs_free():
+    # a thread's calls take no longer after hundreds of refused ones (through the device and a copy an output, as without the page, twice as long)
+    import time
+
+    tiles = H.random_tiles(4096, 0, seed=9)
+    qc, qs = H.random_queries(1, 11)
+    dt, dq, ds = S.to_device(tiles), S.to_device(qc), S.to_device(qs)
+    good, bad = S.make_segments([(0, 4096, 0, 1, 0)]), S.make_segments([(0, 4096, 0, 1, 0), (0, 100, 0, 1, 0)])
+    out = np.zeros((1, 64), np.uint32), np.zeros((1, 64), F), np.zeros(1, np.uint32)
+
+    def took():
+        t = []
+        for _ in range(300):
+            t0 = time.perf_counter()
+            S.score_topk(dt, good, dq, ds, 1, 64, *out)
+            t.append(time.perf_counter() - t0)
+        return float(np.median(t))
+
+    took()
+    before = took()
+    for _ in range(300):
+        with pytest.raises(S.SlhaError):
+            S.score_topk(dt, bad, dq, ds, 1, 64, *out)
+        with pytest.raises(S.SlhaError):
+            S.score_topk(dt, good, dq, ds, 1, 5000, np.zeros((1, 5000), np.uint32), np.zeros((1, 5000), F), out[2])
+    after = took()
+    assert after < 1.25 * before, (before, after)
