@@ -202,9 +202,21 @@ int32_t slha_b200_debug_force_generic_score(int32_t on);
  * Waits for the stream.  All zero when no such call has run. */
 int32_t slha_b200_last_score_stats(uint64_t* out /* 4 values */);
 /* Checking aid: how many tiles a warp took at a time (16 or 32) in that call; 0 for
- * calls of the kernels that do not work in such sets (MIX3 tiles, 16 rows or more a
- * segment) and when no such call has run. */
+ * calls of the kernels that do not work in such sets (all but SLHA_B200_KERNEL_STREAM)
+ * and when no such call has run. */
 int32_t slha_b200_debug_last_score_set(uint32_t* out);
+/* Checking aid: the kernel of that call, 0 when no such call has run.  The first three
+ * stream the tiles and merge what they have appended; the other two write whole rows
+ * of scores, which a selection follows. */
+#define SLHA_B200_KERNEL_STREAM 1     /* warps take sets of tiles */
+#define SLHA_B200_KERNEL_TILE 2       /* a thread takes a tile (MIX3) */
+#define SLHA_B200_KERNEL_WIDE 3       /* 16 rows or more a segment */
+#define SLHA_B200_KERNEL_ROWS 4       /* whole rows, up to four a pass */
+#define SLHA_B200_KERNEL_ROWS_WIDE 5  /* whole rows, 16 or more a segment */
+int32_t slha_b200_debug_last_score_kernel(uint32_t* out);
+/* Checking aid: with on != 0 the calling thread's score_topk calls stream short rows too,
+ * which are otherwise scored as a whole. */
+int32_t slha_b200_debug_stream_all_rows(int32_t on);
 /* Device timing of the fused score + top-k path: after timing_begin, each of
  * the calling thread's next `max_calls` slha_b200_score_topk /
  * slha_b200_pool_score_topk calls records CUDA events on its stream around the

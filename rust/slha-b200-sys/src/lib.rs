@@ -142,6 +142,8 @@ extern "C" {
     pub fn slha_b200_debug_force_generic_score(on: i32) -> i32;
     pub fn slha_b200_last_score_stats(out: *mut u64) -> i32;
     pub fn slha_b200_debug_last_score_set(out: *mut u32) -> i32;
+    pub fn slha_b200_debug_last_score_kernel(out: *mut u32) -> i32;
+    pub fn slha_b200_debug_stream_all_rows(on: i32) -> i32;
     pub fn slha_b200_timing_begin(max_calls: u32) -> i32;
     pub fn slha_b200_timing_end(score_ms: *mut f32, merge_ms: *mut f32, capacity: u32, n_out: *mut u32) -> i32;
     pub fn slha_b200_malloc(bytes: usize, out: *mut *mut c_void) -> i32;

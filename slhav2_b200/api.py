@@ -76,6 +76,8 @@ SIGNATURES = {
     "slha_b200_debug_force_generic_score": (_i32, [_i32]),
     "slha_b200_last_score_stats": (_i32, [_vp]),
     "slha_b200_debug_last_score_set": (_i32, [_vp]),
+    "slha_b200_debug_last_score_kernel": (_i32, [_vp]),
+    "slha_b200_debug_stream_all_rows": (_i32, [_i32]),
     "slha_b200_timing_begin": (_i32, [_u32]),
     "slha_b200_timing_end": (_i32, [_vp, _vp, _u32, _vp]),
     "slha_b200_malloc": (_i32, [_sz, C.POINTER(_vp)]),
@@ -214,6 +216,21 @@ def debug_last_score_set():
     out = np.zeros(1, np.uint32)
     _check(load_library().slha_b200_debug_last_score_set(ptr(out)))
     return int(out[0])
+
+
+KERNEL_STREAM, KERNEL_TILE, KERNEL_WIDE, KERNEL_ROWS, KERNEL_ROWS_WIDE = 1, 2, 3, 4, 5
+
+
+def debug_last_score_kernel():
+    """Checking aid: the kernel of this thread's latest tensor-core score_topk call (KERNEL_*; 0: none)."""
+    out = np.zeros(1, np.uint32)
+    _check(load_library().slha_b200_debug_last_score_kernel(ptr(out)))
+    return int(out[0])
+
+
+def debug_stream_all_rows(on):
+    """Checking aid: the calling thread's score_topk calls stream short rows too, which are otherwise scored as a whole."""
+    _check(load_library().slha_b200_debug_stream_all_rows(1 if on else 0))
 
 
 def timing_begin(max_calls):

@@ -67,6 +67,20 @@ int32_t slha_b200_debug_last_score_set(uint32_t* out) {
         return Status();
     });
 }
+int32_t slha_b200_debug_last_score_kernel(uint32_t* out) {
+    return ffi([&]() -> Status {
+        if (!out) return Status(SLHA_ERR_NULL, "slha_b200_debug_last_score_kernel received a NULL pointer");
+        Ctx* c;
+        SLHA_TRY(get_ctx(&c));
+        *out = last_score_kernel(c);
+        return Status();
+    });
+}
+int32_t slha_b200_debug_stream_all_rows(int32_t on) {
+    g_last_error[0] = 0;
+    debug_stream_all_rows(on != 0);
+    return SLHA_OK;
+}
 int32_t slha_b200_timing_begin(uint32_t max_calls) {
     return ffi([&]() -> Status {
         Ctx* c;

@@ -174,6 +174,8 @@ void debug_force_generic_score(bool on);  // calling thread only
 bool debug_general_paths();                // the calling thread's switch (also: host-driven enforce_budget phases)
 Status last_score_stats(Ctx* c, uint64_t* out4);
 uint32_t last_score_set(Ctx* c);
+uint32_t last_score_kernel(Ctx* c);
+void debug_stream_all_rows(bool on);  // calling thread only
 uint64_t plan_epoch();     // what a graph that captured score_topk on this thread has to compare with before it runs again
 void plan_was_captured();  // the thread's latest score_topk was captured
 bool timing_active();  // the calling thread records kernel events (slha_b200_timing_begin)

@@ -13,6 +13,7 @@ constexpr size_t MAX_SMEM = 227 * 1024;
 // slha_b200_debug_force_generic_score: the calling thread's score_topk calls skip the
 // tensor-core kernel (a checking aid: both kernels must give the same answers).
 thread_local bool g_force_generic = false;
+thread_local bool g_stream_all_rows = false;  // slha_b200_debug_stream_all_rows
 struct Plan;
 thread_local const Plan* g_last_stream_plan = nullptr;  // the calling thread's latest tensor-core call (for its counters)
 
@@ -1087,7 +1088,7 @@ Status score_topk_device(Ctx* c, const SciRustSlhaTile* tiles, const uint8_t* st
     if (k == 0 || k > 4096) return Status(SLHA_ERR_DIMENSION, "top-k: k must be in 1..4096");
     ctx_uses_plans(c);
     Plan* p = nullptr;
-    SLHA_TRY(build_plan(c, tiles, segs, n_segs, nq, k, codec_hint, /*allow_wide=*/state == nullptr, /*allow_rows=*/!prefer_generic, &p));
+    SLHA_TRY(build_plan(c, tiles, segs, n_segs, nq, k, codec_hint, /*allow_wide=*/state == nullptr, /*allow_rows=*/!prefer_generic && !g_stream_all_rows, &p));
     g_last_plan = p;
     if (p->rows) return score_topk_rows(c, p, tiles, state, d_q_coarse, d_q_sign, nq, k, d_out_index, d_out_score, d_out_count, codec_hint);
     const int nwarps = p->threads / 32;
@@ -1219,6 +1220,7 @@ void plan_was_captured() {
 }
 
 void debug_force_generic_score(bool on) { g_force_generic = on; }
+void debug_stream_all_rows(bool on) { g_stream_all_rows = on; }
 bool debug_general_paths() { return g_force_generic; }
 
 // Counters of the calling thread's latest score_topk call that used the tensor-core kernel.
@@ -1240,10 +1242,16 @@ Status last_score_stats(Ctx* c, uint64_t* out4) {
     return Status();
 }
 
+uint32_t last_score_kernel(Ctx* c) {
+    const Plan* p = g_last_stream_plan;
+    if (!p || p->device != c->device || !p->use_mma) return 0u;
+    if (p->rows) return p->wide ? SLHA_B200_KERNEL_ROWS_WIDE : SLHA_B200_KERNEL_ROWS;
+    return p->wide ? SLHA_B200_KERNEL_WIDE : p->kind == 4 ? SLHA_B200_KERNEL_TILE : SLHA_B200_KERNEL_STREAM;
+}
+
 // Tiles a warp of that call took at a time.
 uint32_t last_score_set(Ctx* c) {
-    const Plan* p = g_last_stream_plan;
-    return !p || p->device != c->device || !p->use_mma || p->wide || (!p->rows && p->kind == 4) ? 0u : (uint32_t)(MMA_SET_TILES * (p->rows ? 1 : p->sets));
+    return last_score_kernel(c) == SLHA_B200_KERNEL_STREAM ? (uint32_t)(MMA_SET_TILES * g_last_stream_plan->sets) : 0u;
 }
 
 bool timing_active() { return g_timing.calls < g_timing.max_calls; }

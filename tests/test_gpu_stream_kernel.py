@@ -183,8 +183,12 @@ def test_plain_shares_around_the_sets_of_sixteen_and_thirty_two(codec, nq):
     odd = rows[12]
     tiles[odd[0] + 400:odd[0] + 403] = H.random_tiles(3, 3 if codec != 3 else 4, seed=5)
     qc, qs = H.random_queries(nq * len(lens), 971)
-    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, nq * len(lens), k)
-    assert S.debug_last_score_set() == 16
+    S.debug_stream_all_rows(True)  # (such rows are scored as a whole otherwise)
+    try:
+        idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, nq * len(lens), k)
+        assert S.debug_last_score_set() == 16
+    finally:
+        S.debug_stream_all_rows(False)
     for tb, m, qb, _, base in rows:
         for j in range(qb, qb + nq):
             have = min(m, k)

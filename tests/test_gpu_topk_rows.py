@@ -9,7 +9,7 @@ from tests import helpers as H
 
 pytestmark = pytest.mark.gpu
 F = np.float32
-TAKEN = S.last_score_stats  # (rows of a whole-row plan are reported as sets of sixteen tiles with as many slots as the row has, in multiples of 32)
+TAKEN = S.last_score_stats  # (a whole-row plan has as many slots as the longest row has scores, in multiples of 32)
 
 
 def _check(tiles, rows, nq, k, qc, qs, state_cold=None):
@@ -18,6 +18,7 @@ def _check(tiles, rows, nq, k, qc, qs, state_cold=None):
     longest = max(r[1] for r in rows)
     idx, sc, cnt = S.score_topk(dt, seg, qc, qs, nq, k)
     assert TAKEN()["buffer_slots"] == (longest + 31) // 32 * 32
+    assert S.debug_last_score_kernel() in (S.KERNEL_ROWS, S.KERNEL_ROWS_WIDE) and S.debug_last_score_set() == 0
     flat = S.make_segments([(t, n, q, m, 0) for t, n, q, m, _ in rows])
     dense = S.score_segments(dt, flat, qc, qs, nq, np.zeros((nq, longest), F), np.arange(nq, dtype=np.uint64) * longest, longest, fill=0.0)
     for t, n, q0, m, base in rows:
