@@ -297,7 +297,7 @@ struct Cuts {
     }
 };
 
-// Whether a call's rows are scored as a whole (score_select.cuh) rather than streamed: rows of up to ROWS_MOST tiles, scores of 64 MB at most.  `passes`: tiles times
+// Whether a call's rows are scored as a whole (score_select.cuh) rather than streamed: rows of up to ROWS_MOST tiles, scores of 64 MB at most as they are laid out.  `passes`: tiles times
 // groups of four query rows, `wide`: 16 rows or more a segment, which the 64-row kernel takes (512 rows of 16 384 TQ3 tiles, k = 256 85 -> 47 us; 1232 of
 // 3553 MX tiles 111 -> 53).  Streaming reads a million tiles in 25 us where score_dense_kernel takes 40 (NF4 34, 59), but its set-up, first sets and compaction
 // cost about 20 us a call, and appending and merging a row 0.04 (k = 64) to 0.08 us (k = 1024), which selecting from whole rows costs hardly: in pico-
@@ -308,7 +308,8 @@ struct Cuts {
 //   200 / 308, 245 / 396, NF4 272 / 294, 273 / 369, 318 / 475.
 enum RowsRule { ROWS_NO, ROWS_YES, ROWS_UNLESS_NF4 };
 RowsRule rows_rule(uint64_t passes, bool wide, size_t nq, uint32_t longest, uint32_t k) {
-    if (longest == 0 || longest > ROWS_MOST || nq * (((uint64_t)longest + 31) / 32 * 32) > (16ull << 20)) return ROWS_NO;
+    const uint64_t unit = wide ? WIDE_M : 32;  // (the 64-row kernel writes blocks of 128 scores)
+    if (longest == 0 || longest > ROWS_MOST || nq * Cuts::whole(longest, unit) > (16ull << 20)) return ROWS_NO;
     if (wide || passes <= (k >= 512 ? 1280000 : 640000)) return ROWS_YES;
     const uint64_t saved = 18000000 + nq * (k >= 1024 ? 85000 : k >= 200 ? 75000 : k >= 32 ? 37000 : 25000);
     return 30 * passes <= saved ? ROWS_YES : 16 * passes <= saved ? ROWS_UNLESS_NF4 : ROWS_NO;

@@ -182,3 +182,18 @@ def test_equal_scores_and_one_far_from_the_rest_cost_no_multiple(n, k):
         took[shape] = float(np.median(S.timing_end(9)[1]))
         _check(tiles, [(0, n, 0, 2, 0)], 2, k, qc[:2], qs[:2])
     assert max(took["equal"], took["far"]) < 10 * took["differ"], took
+
+
+@pytest.mark.parametrize("n_seg,kernel", [(8190, S.KERNEL_ROWS_WIDE), (8200, S.KERNEL_WIDE)])
+def test_many_short_rows_of_the_64_row_kernel_stay_within_the_plan_s_memory(n_seg, kernel):
+    # 16 rows of 17 tiles a segment, which that kernel pads to 128 scores: 64 MB on either side
+    n, nq, k = 17, 16, 4
+    assert (n_seg * nq * 128 <= 16 << 20) == (kernel == S.KERNEL_ROWS_WIDE) and n_seg * nq * 32 < 16 << 20
+    tiles = H.random_tiles(3000, 1, seed=91)
+    qc, qs = (np.resize(x, (n_seg * nq,) + x.shape[1:]) for x in H.random_queries(61, 92))
+    rows = [(i % 2900, n, nq * i, nq, i) for i in range(n_seg)]
+    idx, sc, cnt = S.score_topk(S.to_device(tiles), S.make_segments(rows), qc, qs, n_seg * nq, k)
+    assert S.debug_last_score_kernel() == kernel and np.all(cnt == k)
+    for i in (0, 1, 4000, n_seg - 1):
+        want = ora.score_tiles(tiles[rows[i][0]:rows[i][0] + n], qc[nq * i + 3], qs[nq * i + 3])
+        assert np.all(np.abs(sc[nq * i + 3] - np.sort(want)[::-1][:k]) <= 2e-3) and np.all(np.abs(sc[nq * i + 3] - want[idx[nq * i + 3] - i]) <= 1e-3)
