@@ -14,6 +14,7 @@
 #include <cub/block/block_scan.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
+#include <chrono>
 #include <vector>
 
 #include "common.cuh"
@@ -1465,17 +1466,20 @@ static Status pool_step_memory(Pool* pl) {
     }
     return Status();
 }
-// Until a kernel on the stream has answered; an error of the stream, or its end without the answer, ends the wait too.
+// Until the stream's last kernel has answered.  The host polls for as long as a decode step's kernels may take (the answer is there some us before the runtime knows of the kernel's end), but
+// not where its threads are to sleep while they wait (cudaDeviceScheduleBlockingSync); behind more work than that it waits for the stream as everywhere.  The library's own stream is drained.
+constexpr long POLL_US = 200;
 template <typename There>
 static Status wait_answer(Ctx* c, There there) {
-    for (uint32_t i = 0; !there(); ++i) {
-        if (i % 4096 != 4095) continue;
-        const cudaError_t e = cudaStreamQuery(c->stream);
-        if (e == cudaErrorNotReady) continue;
-        SLHA_CUDA(e);
-        if (!there()) return Status(SLHA_ERR_DEVICE, "the kernel ended without an answer");
+    unsigned flags = 0;
+    SLHA_CUDA(cudaGetDeviceFlags(&flags));
+    if ((flags & cudaDeviceScheduleMask) != cudaDeviceScheduleBlockingSync) {
+        const auto since = std::chrono::steady_clock::now();
+        for (uint32_t i = 1; !there(); ++i)
+            if (i % 64 == 0 && std::chrono::steady_clock::now() - since > std::chrono::microseconds(POLL_US)) break;
     }
-    return Status();
+    if (!there() || c->own_stream) SLHA_CUDA(cudaStreamSynchronize(c->stream));
+    return there() ? Status() : Status(SLHA_ERR_DEVICE, "the kernel ended without an answer");
 }
 
 // One cooperative launch for all phases, one read-back of the counters.  Sets *done when the

@@ -219,3 +219,45 @@ def test_refused_calls_leave_the_page_for_short_outputs_free():
             S.score_topk(dt, good, dq, ds, 1, 5000, np.zeros((1, 5000), np.uint32), np.zeros((1, 5000), F), out[2])
     after = took()
     assert after < 1.25 * before, (before, after)
+
+
+_SLEEPER = """
+import ctypes, sys, time
+rt = ctypes.CDLL("libcudart.so.12")
+assert rt.cudaSetDevice(0) == 0 and rt.cudaSetDeviceFlags(4) == 0  # cudaDeviceScheduleBlockingSync
+import numpy as np
+import slhav2_b200 as S
+from tests import helpers as H
+from tests.test_gpu_streams import Streams
+gm = S.Model.from_projection(H.make_model_pair(128, seed=61)[1], 128, 61)
+keys = S.to_device(np.resize(H.gaussian_keys(67, 4096, 128), (262144, 128)))
+out = S.DeviceBuffer(262144 * 128)
+pool = S.TilePool(1000, 2**40)
+pool.append_keys(gm, H.gaussian_keys(68, 900, 128), S.CODEC_MIXED)
+with Streams(1) as st:
+    S.set_stream(st.all[0].value)
+    for call in (pool.stats, pool.enforce_budget):
+        call()
+        worst = 0.0
+        for _ in range(3):
+            for _ in range(60):
+                gm.encode_keys(keys, S.CODEC_NF4, n=262144, out=out)
+            wall, cpu = time.perf_counter(), time.thread_time()
+            call()
+            wall, cpu = time.perf_counter() - wall, time.thread_time() - cpu
+            assert wall > 0.01, wall
+            worst = max(worst, cpu / wall)
+        print(call.__name__, worst)
+        assert worst < 0.3, (call.__name__, worst)
+"""
+
+
+def test_a_thread_that_is_to_sleep_while_it_waits_does():
+    # calls behind 60 encodes of 0.7 ms, in a process whose device has cudaDeviceScheduleBlockingSync
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _SLEEPER], cwd=root, capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
