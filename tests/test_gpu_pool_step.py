@@ -261,3 +261,55 @@ def test_a_thread_that_is_to_sleep_while_it_waits_does():
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     r = subprocess.run([sys.executable, "-c", _SLEEPER], cwd=root, capture_output=True, text=True, timeout=120)
     assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("n,evict,skewed", [(500_003, 1, False), (500_003, 1, True), (16 * 148 * 512 - 1, 1, False), (16 * 148 * 512, 0, False), (16 * 148 * 512 + 1, 1, False)])
+def test_a_step_in_a_large_pool(n, evict, skewed):
+    # all sixteen slots of a thread's registers (148 SMs) and one more; skewed: one block holds no small key, so that the blocks' least keys bound nothing, more
+    # candidates than the list holds lie within the other bound, and the kernel leaves the work to the other one after its scans
+    rng = np.random.default_rng(n + evict)
+    gm = S.Model.from_projection(H.make_model_pair(128, seed=61)[1], 128, 61)
+    keys = S.to_device(np.resize(H.gaussian_keys(62, 4096, 128), (131072, 128)))
+    pools = [S.TilePool(n + 4000, 2**40, 1, evict, 4, 500) for _ in range(2)]
+    at = 0
+
+    def append(m):
+        nonlocal at
+        got = [p.append_keys(gm, keys, S.CODEC_MIXED, n=m, position_base=at) for p in pools]
+        assert np.array_equal(*got)
+        at += m
+
+    def step(budget):
+        within, launched = [], []
+        for i, p in enumerate(pools):
+            p.set_budget(int(budget))
+            S.debug_force_generic_score(bool(i))
+            before = S.launch_count()
+            try:
+                within.append(p.enforce_budget())
+            finally:
+                S.debug_force_generic_score(False)
+            launched.append(S.launch_count() - before)
+        assert within[0] == within[1] and pools[0].stats() == pools[1].stats()
+        return launched[0]
+
+    def live():
+        return pools[0].stats()["live_bytes"]
+
+    for b in range(0, n, 131072):
+        append(min(131072, n - b))
+    slots = np.arange(n, dtype=np.uint32)
+    sc = rng.standard_normal(n).astype(F)
+    if skewed:
+        sc[slots // 512 % 148 == 147] += 30
+    for p in pools:
+        p.observe_scores(slots, sc, 0.9)
+    step(96 * n)                           # everything is paged
+    for m, gone in ((8, 1), (8, 8), (1, 60), (20, 90)):
+        append(m)
+        kernels = step(live() - 32 * m - 96 * gone)
+        assert kernels == (2 if skewed and gone >= 60 else 1), (m, gone, kernels)
+    append(3)
+    assert step(live() - 32 * 2) == 1 and step(live()) == 1
+    for a, b in zip(pools[0].read(), pools[1].read()):
+        assert a.tobytes() == b.tobytes()
