@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     uint64_t* buf = reinterpret_cast<uint64_t*>(smem);                     // [cap]
     uint64_t* own = buf + cap + tid;                                       // [OWN], NT apart; then the candidates' places in their buckets
     int* hist = reinterpret_cast<int*>(buf + cap + row_own_slots(cap, NT, R));  // [ROW_BUCKETS + 1]
-    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket and 10, 11, 13 what a closer look at it needs, 5, 8, 9 of a selection step, 12 a bucket is crowded, 16.. warp totals
+    uint32_t* st = reinterpret_cast<uint32_t*>(hist + ROW_HIST_INTS);     // 0 candidates, 1 smallest and 2 largest score word, 3 bound's bucket and 10, 11, 13 what a closer look at it needs, 14 the bucket of a lower bound, 5, 8, 9 of a selection step, 12 a bucket is crowded, 16.. warp totals
     const uint32_t n = info.n;
     const float* row = a.scores + info.begin;
     // thread t holds the scores 4 (t + NT j) .. + 3
@@ -189,7 +189,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
     const float top = key_score(ranged ? st[2] : score_key(1.0f));
     if (sampled && ranged) {
         const float part = (float)k * (0.25f / (float)STEP);
-        const int want = (int)(1.25f * part + 3.0f * sqrtf(part)) + 2, most = (int)(cap * 3u / (16u * STEP));
+        const int want = (int)(1.25f * part + 3.0f * sqrtf(part)) + 2, most = (int)(cap * 3u / (16u * STEP)), safe = min(most, 3 * want);
         float inv = (float)ROW_BUCKETS / (top - low);  // (a range that overflows puts all in one bucket)
 #pragma unroll
         for (int j = 0; j < R; ++j) {
@@ -204,6 +204,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
                 st[3] = tid * PER + j + 1;
                 if (at + c[j] > most) st[13] = at + 1;
             }
+            if (R > 2 && at <= safe && at + c[j] > safe) st[14] = tid * PER + j;  // (shorter rows take 20 us without a bound)
             at += c[j];
             hist[tid * PER + j] = 0;
         }
@@ -324,9 +325,12 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         }
         __syncthreads();
         if (st[0] >= k || bound == -INFINITY) break;
-        bound = -INFINITY;  // (the sample misled)
+        // The sample misled: a bound that three times as many of it reach, in the end none.  (One of some thousand rows for small k; in a call of 32 rows of 32 768 the selection of all
+        // scores that follows without a bound took 102 us instead of 33.)
+        const float second = top - (float)st[14] * (top - low) / (float)ROW_BUCKETS;
+        bound = R > 2 && st[14] && second < bound ? second : -INFINITY;
         __syncthreads();
-        if (tid == 0) st[0] = 0u;
+        if (tid == 0) st[0] = st[14] = 0u;
         __syncthreads();
     }
     const uint32_t got = st[0], m = min(got, k);

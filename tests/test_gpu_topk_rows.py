@@ -197,3 +197,34 @@ def test_many_short_rows_of_the_64_row_kernel_stay_within_the_plan_s_memory(n_se
     for i in (0, 1, 4000, n_seg - 1):
         want = ora.score_tiles(tiles[rows[i][0]:rows[i][0] + n], qc[nq * i + 3], qs[nq * i + 3])
         assert np.all(np.abs(sc[nq * i + 3] - np.sort(want)[::-1][:k]) <= 2e-3) and np.all(np.abs(sc[nq * i + 3] - want[idx[nq * i + 3] - i]) <= 1e-3)
+
+
+@pytest.mark.parametrize("n,k,among", [(30000, 64, 20), (30000, 64, 64), (16384, 64, 25), (30000, 1024, 130), (5000, 64, 40)])
+def test_rows_whose_best_lie_where_the_sample_looks(n, k, among):
+    # `among` of the k best scores lie at places that are sampled (every fourth to sixteenth score), so that fewer than k reach the first bound; the lower one, or none, is enough
+    step = 4 if n > 16384 else 2 if n > 8192 else 1
+    place = np.arange(n)
+    sampled = np.flatnonzero((place % 4 == 0) & ((place // 4 % 512 + place // 2048) % step == 0))
+    rng = np.random.default_rng(n + k)
+    tiles = np.resize(H.random_tiles(1, 0, seed=93), n)
+    tiles["dynamic_lambda"] = 0
+    qc, qs = H.random_queries(1, 94)
+    sign = 1 if ora.score_tiles(tiles[:1], qc[0], qs[0])[0] > 0 else -1
+    qc = np.repeat(sign * qc, 128, 0)
+    best = np.concatenate([rng.choice(sampled, among, replace=False), rng.choice(np.setdiff1d(place, sampled), k - among, replace=False)])
+    scale = tiles["scale"] * rng.uniform(0.1, 1.0, n).astype(F)
+    scale[best] = tiles["scale"][0] * rng.uniform(1.5, 2.0, k).astype(F)
+    tiles["scale"] = scale
+    _check(tiles, [(0, n, 0, 2, 0)], 2, k, qc[:2], qs[[0, 0]])
+    if among < k:
+        seg, nq = S.make_segments([(0, n, 4 * i, 4, 0) for i in range(32)]), 128
+        args = S.to_device(qc), S.to_device(np.repeat(qs, nq, 0)), nq, k, S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * k * 4), S.DeviceBuffer(nq * 4)
+        took = {}
+        for name, t in (("placed", tiles), ("anywhere", tiles[rng.permutation(n)])):
+            dt = S.to_device(t)
+            S.score_topk(dt, seg, *args)
+            S.timing_begin(9)
+            for _ in range(9):
+                S.score_topk(dt, seg, *args)
+            took[name] = float(np.median(S.timing_end(9)[1]))
+        assert took["placed"] < 2.5 * took["anywhere"], took
