@@ -456,14 +456,22 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
             wide = wide && (segs[i].n_queries >= 16 || segs[i].n_tiles == 0);
             passes += (uint64_t)segs[i].n_tiles * ((segs[i].n_queries + 3) / 4);
         }
-        RowsRule rule = rows_rule(passes, wide && allow_wide, nq, longest, k);
-        if (rule == ROWS_UNLESS_NF4) {
+        // (NF4 tiles, which the 64-row kernel does not decode, are taken four rows at a time from the start: handed on by that kernel, whose work items are short, 40 rows on each of 2 x 20 000
+        // tiles k = 100 took 101 us a call instead of 40, 250 on 32 768 219 instead of 116)
+        wide = wide && allow_wide;
+        RowsRule rule = rows_rule(passes, wide, nq, longest, k);
+        if (rule == ROWS_UNLESS_NF4 || (rule == ROWS_YES && wide)) {
             SLHA_TRY(look());
             looked = true;
-            rule = p->kind == 0 ? ROWS_NO : ROWS_YES;
+            if (p->kind == 0) {
+                wide = false;
+                rule = rows_rule(passes, false, nq, longest, k) == ROWS_YES ? ROWS_YES : ROWS_NO;
+            } else {
+                rule = ROWS_YES;
+            }
         }
         if (rule == ROWS_YES) {
-            SLHA_TRY(build_rows_plan(c, p, segs, n_segs, nq, longest, allow_wide));
+            SLHA_TRY(build_rows_plan(c, p, segs, n_segs, nq, longest, wide));
             p->use_mma = true;
             p->key = std::move(key);
             p->device = c->device;

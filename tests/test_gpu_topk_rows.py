@@ -134,28 +134,31 @@ def test_many_rows_whose_segments_end_inside_a_block(codec, n_seg):
 
 
 def test_rows_handed_on_for_different_reasons():
-    # A segment of three blocks, the first of which begins on an NF4 tile and the others meet one, scored with 16 rows: alone, and behind 49 short NF4 segments
-    # and before others in shares of 50 blocks (on 148 SMs), where the CTA that hands its rows on for the first block does so last.  The same scores bit for bit.
+    # A segment of three blocks, the first of which begins on an NF4 tile and the others meet one, scored with 16 rows behind 49 short NF4 segments in shares of 50
+    # blocks (on 148 SMs, one share of others before them), where the CTA that hands its rows on for the first block does so last: the generic arithmetic, bit for bit.
     n, nq, k = 384, 16, 384
     mixed = H.random_tiles(n, 0, seed=85)
     nf4 = H.random_tiles(60, 2, seed=86)
     mixed[0], mixed[130:140], mixed[300] = nf4[59], nf4[49:59], nf4[58]
     rest = np.tile(H.random_tiles(2560, 0, seed=87), 2)
     tiles = np.concatenate([nf4[:49], mixed, rest])
-    rows = [(i, 1, nq * i, nq, 0) for i in range(49)] + [(49, n, nq * 49, nq, 0)]
-    for _ in range((148 * 50 - 52) // 4):
-        rows.append((49 + n + len(rows), 512, nq * len(rows), nq, 0))
+    at = 49 + n
+    rows = [(at + i, 512 if i < 12 else 256) for i in range(13)] + [(i, 1) for i in range(49)] + [(49, n)] + [(at + i, 512) for i in range((148 * 50 - 50 - 52) // 4)]
+    rows = [(tb, m, nq * i, nq, 0) for i, (tb, m) in enumerate(rows)]
     total = nq * len(rows)
     qc, qs = H.random_queries(total, 88)
-    own = slice(49 * nq, 50 * nq)
+    own = slice(62 * nq, 63 * nq)
     dt = S.to_device(tiles)
-    alone = S.score_topk(dt, S.make_segments([(49, n, 0, nq, 0)]), qc[own], qs[own], nq, k)
-    assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
+    S.debug_force_generic_score(True)
+    try:
+        alone = S.score_topk(dt, S.make_segments([(49, n, 0, nq, 0)]), qc[own], qs[own], nq, k)
+    finally:
+        S.debug_force_generic_score(False)
     want = ora.score_tiles(mixed, qc[own][3], qs[own][3])
     assert np.all(np.abs(alone[1][3] - want[alone[0][3]]) <= 1e-3)
     for _ in range(5):
         idx, sc, cnt = S.score_topk(dt, S.make_segments(rows), qc, qs, total, k)
-        assert S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
+        assert S.debug_last_score_kernel() == S.KERNEL_ROWS_WIDE and S.last_score_stats()["rows_handed_to_generic_kernel"] == nq
         assert np.all(cnt[own] == k) and np.array_equal(idx[own], alone[0]) and np.array_equal(sc[own].view(np.uint32), alone[1].view(np.uint32))
 
 
@@ -228,3 +231,18 @@ def test_rows_whose_best_lie_where_the_sample_looks(n, k, among):
                 S.score_topk(dt, seg, *args)
             took[name] = float(np.median(S.timing_end(9)[1]))
         assert took["placed"] < 2.5 * took["anywhere"], took
+
+
+@pytest.mark.parametrize("n,nq,k,kernel", [(3000, 64, 100, S.KERNEL_ROWS), (20000, 40, 500, S.KERNEL_ROWS), (32768, 250, 16, S.KERNEL_STREAM), (1000, 16, 16, S.KERNEL_ROWS)])
+def test_nf4_rows_of_many_queries_are_taken_four_at_a_time(n, nq, k, kernel):
+    # the 64-row kernel does not decode NF4: its short items, handed on, took twice as long as the kernels for four rows
+    tiles = H.random_tiles(n, 2, seed=95, warm_every=9)
+    qc, qs = H.random_queries(nq, 96)
+    dt, seg = S.to_device(tiles), S.make_segments([(0, n, 0, nq, 7)])
+    for _ in range(2):
+        idx, sc, cnt = S.score_topk(dt, seg, qc, qs, nq, k)
+        assert S.debug_last_score_kernel() == kernel and S.last_score_stats()["rows_handed_to_generic_kernel"] == 0
+    assert np.all(cnt == k)
+    for j in range(0, nq, 13):
+        want = ora.score_tiles(tiles, qc[j], qs[j])
+        assert np.all(np.abs(sc[j] - want[idx[j] - 7]) <= 1e-3 * (1 + np.abs(sc[j]))) and np.all(np.abs(sc[j] - np.sort(want)[::-1][:k]) <= 2e-3 * (1 + np.abs(sc[j])))
