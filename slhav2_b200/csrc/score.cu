@@ -303,7 +303,13 @@ struct ScoreArgs {
     uint32_t* gcount;             // per query row: candidates appended to the row's buffer
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
     uint32_t blocked;             // dense mode: item's scores lie in blocks of 128 tiles, block b's of its row q from list_begin + b * pad + 128 q on
-    uint32_t by_fours;            // score_dense_kernel: items are the 64-row kernel's, taken four rows at a time (item e: rows 4 (e mod 16) .. of items[e / 16])
+    // score_dense_kernel<true>, behind the 64-row kernel: whole streams (a segment's tiles, up to 64 query rows), which it cuts for itself: in groups of four rows, blocks of 128 tiles, unit_share of
+    // them a CTA in order.  (A list of those cuts would be twice as long as all that a dense call brings; the 64-row kernel's own cuts, four rows at a time, are a set-up for every two or
+    // three blocks: 40 rows on each of 2 x 20 000 NF4 tiles 98 us a call instead of 40.)
+    const WorkItem* streams;
+    const uint2* stream_at;       // [n_streams + 1] groups, blocks before a stream
+    uint32_t n_streams, unit_share;
+    uint32_t* handoff_any;        // 1 where that kernel handed rows on
     uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): bit 0, or bit 1 where that pass is to
     uint32_t handoff_as;          // score them in score_kernel's arithmetic (items that begin with an NF4 tile: always bit 0)
     const uint32_t* only_flagged; // dense mode: optional, per query row: only work items one of whose rows is flagged here
@@ -457,20 +463,47 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
     }
 }
 
-// Item e of a call of score_dense_kernel.
-__device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e) {
-    if (!a.by_fours) return a.stream_items[e];
-    WorkItem it = a.stream_items[e >> 4];
-    const uint32_t q = 4u * (e & 15u);
-    it.query_begin += q;
-    it.n_queries = it.n_queries > q ? min(4u, it.n_queries - q) : 0u;
-    it.list_begin += 128u * q;
-    return it;
+// The last stream that begins at or before x (of its groups, or of its blocks).
+template <bool BLOCKS>
+__device__ __forceinline__ uint32_t dense_stream(const ScoreArgs& a, uint32_t x) {
+    uint32_t lo = 0, hi = a.n_streams;
+    while (hi - lo > 1u) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if ((BLOCKS ? a.stream_at[mid].y : a.stream_at[mid].x) <= x) lo = mid;
+        else hi = mid;
+    }
+    return lo;
 }
-// (null: an item a CTA)
-__device__ __forceinline__ uint32_t dense_first(const ScoreArgs& a, uint32_t cta) {
-    const uint32_t i = a.cta_begin ? a.cta_begin[cta] : cta;
-    return a.by_fours ? 16u * i : i;
+// the group that a block belongs to
+__device__ __forceinline__ uint32_t dense_group(const ScoreArgs& a, uint32_t block) {
+    const uint32_t s = dense_stream<true>(a, block);
+    return a.stream_at[s].x + (block - a.stream_at[s].y) / ((a.streams[s].n_tiles + 127u) / 128u);
+}
+// A CTA's items of a call of score_dense_kernel: first .. end (null: an item a CTA).  PASS: behind the 64-row kernel; an item is what the CTA takes of a stream's group.
+template <bool PASS>
+__device__ __forceinline__ uint32_t dense_first(const ScoreArgs& a) {
+    if (PASS) return dense_group(a, blockIdx.x * a.unit_share);
+    return a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x;
+}
+template <bool PASS>
+__device__ __forceinline__ uint32_t dense_end(const ScoreArgs& a) {
+    if (PASS) return dense_group(a, min((blockIdx.x + 1u) * a.unit_share, a.stream_at[a.n_streams].y) - 1u) + 1u;
+    return a.cta_begin ? a.cta_begin[blockIdx.x + 1] : blockIdx.x + 1u;
+}
+template <bool PASS>
+__device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e) {
+    if (!PASS) return a.stream_items[e];
+    const uint32_t s = dense_stream<false>(a, e), q = 4u * (e - a.stream_at[s].x);
+    WorkItem it = a.streams[s];
+    const uint32_t blocks = (it.n_tiles + 127u) / 128u, at = a.stream_at[s].y + q / 4u * blocks, mine = blockIdx.x * a.unit_share;
+    const uint32_t lo = max(mine, at) - at, hi = min(mine + a.unit_share, at + blocks) - at;
+    it.query_begin += q;
+    it.n_queries = min(4u, it.n_queries - q);
+    it.list_begin += 128u * q;
+    it.tile_begin += 128u * lo;
+    it.index_base += 128u * lo;
+    it.n_tiles = min(it.n_tiles, 128u * hi) - 128u * lo;
+    return it;
 }
 
 // Work items that a dense kernel's CTA could not score on the tensor cores (a tile of another codec than its item's first, a query outside the fp16
@@ -481,8 +514,9 @@ __device__ __forceinline__ uint32_t undone_shift(uint32_t items) {
     return items <= 32u * UNDONE_WORDS ? 0u : 32u - (uint32_t)__clz((items - 1u) / (32u * UNDONE_WORDS));
 }
 // (one thread of the CTA)
+template <bool PASS>
 __device__ __forceinline__ void undone_add(const ScoreArgs& a, uint32_t* bits, uint32_t item) {
-    const uint32_t first = dense_first(a, blockIdx.x), e = (item - first) >> undone_shift(dense_first(a, blockIdx.x + 1) - first);
+    const uint32_t first = dense_first<PASS>(a), e = (item - first) >> undone_shift(dense_end<PASS>(a) - first);
     bits[e >> 5] |= 1u << (e & 31u);
 }
 // Dense scores of one work item by the whole CTA, rows query_begin .. + nq (four at most).  smem: 4 KB, and 4 KB a warp.
@@ -544,13 +578,14 @@ __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem&
     __syncthreads();
 }
 // What is left at a CTA's end (all of its shared memory but the bits is free).
+template <bool PASS>
 __device__ __noinline__ void finish_undone(const ScoreArgs& a, const uint32_t* bits, unsigned char* smem) {
     __syncthreads();
-    const uint32_t first = dense_first(a, blockIdx.x), items = dense_first(a, blockIdx.x + 1) - first, shift = undone_shift(items);
+    const uint32_t first = dense_first<PASS>(a), items = dense_end<PASS>(a) - first, shift = undone_shift(items);
     for (uint32_t e = 0; e < items; ++e) {
         const uint32_t bit = e >> shift;
         if (!(bits[bit >> 5] >> (bit & 31u) & 1u)) continue;
-        const WorkItem it = dense_item(a, first + e);
+        const WorkItem it = dense_item<PASS>(a, first + e);
         for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
     }
 }

@@ -65,9 +65,13 @@ Status launch_stream(Ctx* c, int kind, bool il, bool long_items, const ScoreArgs
 uint32_t stream_warp_tiles(int kind, int sets) { return kind == 4 ? ST_WT : (uint32_t)(MMA_SET_TILES * sets); }
 uint32_t stream_warps(int kind) { return (uint32_t)(kind == 4 ? ST_THREADS : STREAM_THREADS) / 32; }
 static_assert(ST_CHUNK == ST_WT, "a fresh chunk holds what a warp can append at once");
-Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
+template <bool PASS>
+Status launch_dense_t(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
     static thread_local bool configured[16] = {false};
-    return launch_tc(c, score_dense_kernel, configured, a, grid, ST_THREADS, st_smem_bytes(true), behind);
+    return launch_tc(c, score_dense_kernel<PASS>, configured, a, grid, ST_THREADS, st_smem_bytes(true), behind);
+}
+Status launch_dense(Ctx* c, const ScoreArgs& a, uint32_t grid, bool behind) {
+    return a.streams ? launch_dense_t<true>(c, a, grid, behind) : launch_dense_t<false>(c, a, grid, behind);
 }
 template <int KIND>
 Status launch_wide_t(Ctx* c, const ScoreArgs& a, uint32_t grid) {
@@ -254,7 +258,10 @@ struct Plan {
     uint32_t longest = 0;
     uint64_t row_stride = 0;
     RowInfo* d_rows = nullptr;
-    uint32_t* d_row_flags = nullptr;  // [nq] generic arithmetic, [nq] handed on by the 64-row kernel, [nq][2] statistics
+    uint32_t* d_row_flags = nullptr;  // [nq] generic arithmetic, [nq] handed on by the 64-row kernel, [nq][2] statistics, whether any row was handed on
+    WorkItem* d_streams = nullptr;    // of the pass over those, see Streams
+    uint2* d_stream_at = nullptr;
+    uint32_t n_streams = 0, unit_share = 1, streams_grid = 0;
     uint64_t last_use = 0;
     bool captured = false;  // a graph of the library's own names this plan's buffers (see plan_epoch)
 };
@@ -294,6 +301,24 @@ struct Cuts {
     }
     void finish() {
         if (cta.back() != (uint32_t)items.size()) cta.push_back((uint32_t)items.size());
+    }
+};
+
+// What the four-row kernel's pass behind the 64-row kernel is given, see ScoreArgs::streams.
+struct Streams {
+    std::vector<WorkItem> all;
+    std::vector<uint2> at{make_uint2(0u, 0u)};
+    uint32_t share = 1, grid = 0;
+    // (`place`, `step`: of whole rows in blocks)
+    void add(const SlhaB200Segment& s, uint32_t q0, uint32_t place = 0, uint32_t step = 0) {
+        const uint32_t rows = std::min<uint32_t>(WIDE_NQ, s.n_queries - q0), groups = (rows + 3) / 4;
+        all.push_back(WorkItem{s.tile_begin, s.n_tiles, s.index_base, s.query_begin + q0, rows, place, step});
+        at.push_back(make_uint2(at.back().x + groups, at.back().y + groups * ((s.n_tiles + 127u) / 128u)));
+    }
+    void finish(int sms, uint32_t least) {
+        const uint32_t blocks = at.back().y;
+        share = std::max(least, (blocks + (uint32_t)sms - 1) / (uint32_t)sms);
+        grid = (blocks + share - 1) / share;
     }
 };
 
@@ -344,12 +369,16 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     // Where the scores go: rows one behind the other, or where the 64-row kernel writes them, a block of 128 tiles' scores of all the item's rows together.
     p->row_stride = ((uint64_t)longest + 31) / 32 * 32;
     uint64_t floats = nq * p->row_stride;
+    Streams streams;
     if (wide) {
         floats = 0;
         size_t at = 0;
         for (size_t i = 0; i < n_segs; ++i)
             for (uint32_t q0 = 0; q0 < segs[i].n_queries && segs[i].n_tiles; q0 += WIDE_NQ) {
                 const uint32_t m = std::min<uint32_t>(WIDE_NQ, segs[i].n_queries - q0);
+                SlhaB200Segment s = segs[i];
+                s.index_base = 0;
+                streams.add(s, q0, (uint32_t)floats, 128 * m);
                 for (uint32_t q = 0; q < m; ++q) {
                     rows[segs[i].query_begin + q0 + q].begin = (uint32_t)(floats + 128 * q);
                     rows[segs[i].query_begin + q0 + q].step = 128 * m;
@@ -364,21 +393,27 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     } else {
         for (size_t q = 0; q < nq; ++q) rows[q].begin = (uint32_t)(q * p->row_stride);
     }
+    streams.finish(sms, 1);
     Blob tables;
-    const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows);
+    const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows), o_s = tables.add(streams.all), o_sa = tables.add(streams.at);
     SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
-    SLHA_TRY(p->b_gpivot.ensure(4 * nq * 4));
+    SLHA_TRY(p->b_gpivot.ensure((4 * nq + 1) * 4));
     SLHA_TRY(p->b_gbuf.ensure(floats * 4));
     unsigned char* dev = static_cast<unsigned char*>(p->b_tables.p);
     SLHA_TRY(ctx_copy_table(c, dev, tables.bytes.data(), tables.bytes.size()));
     p->d_row_flags = (uint32_t*)p->b_gpivot.p;
-    SLHA_CUDA(cudaMemsetAsync(p->d_row_flags, 0, 4 * nq * 4, c->stream));
+    SLHA_CUDA(cudaMemsetAsync(p->d_row_flags, 0, (4 * nq + 1) * 4, c->stream));
     p->d_items = reinterpret_cast<WorkItem*>(dev + o_n);
     p->wide = wide;
     p->n_items = (uint32_t)cuts.items.size();
     p->mma_grid = (uint32_t)cuts.cta.size() - 1;
     p->d_cta_begin = !wide && p->n_items == p->mma_grid ? nullptr : reinterpret_cast<uint32_t*>(dev + o_nc);  // (null: an item a CTA)
     p->d_rows = reinterpret_cast<RowInfo*>(dev + o_r);
+    p->d_streams = reinterpret_cast<WorkItem*>(dev + o_s);
+    p->d_stream_at = reinterpret_cast<uint2*>(dev + o_sa);
+    p->n_streams = (uint32_t)streams.all.size();
+    p->unit_share = streams.share;
+    p->streams_grid = streams.grid;
     p->longest = longest;
     p->rows = true;
     return Status();
@@ -993,10 +1028,13 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
         total += Cuts::whole(s.n_tiles, ST_M) * ((s.n_queries + 3) / 4);
         wtotal += Cuts::whole(s.n_tiles, WIDE_M) * ((s.n_queries + WIDE_NQ - 1) / WIDE_NQ);
     }
-    // (the four-row kernel's pass behind the 64-row kernel takes that one's items, four rows at a time)
     Cuts cuts(wide ? wtotal : total, sms, wide ? WIDE_M : ST_M, wide ? WIDE_M : ST_M * 4);
     for (size_t i = 0; i < n_segs; ++i) cuts.add(segs[i], wide ? WIDE_NQ : 4);
     cuts.finish();
+    Streams streams;
+    for (size_t i = 0; i < n_segs && wide; ++i)
+        for (uint32_t q0 = 0; q0 < segs[i].n_queries && segs[i].n_tiles; q0 += WIDE_NQ) streams.add(segs[i], q0);
+    streams.finish(sms, 4);
     std::vector<WorkItem> generic;  // runs of 4096 tiles where score_kernel takes the call
     if (g_force_generic)
         for (const WorkItem& s : cuts.items)
@@ -1009,7 +1047,8 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
             }
     Blob blob;
     const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta), o_gen = blob.add(generic);
-    const size_t o_tail = fills ? blob.add(tail) : 0, o_flag = wide ? blob.add(std::vector<uint32_t>(nq, 0u)) : 0;
+    const size_t o_tail = fills ? blob.add(tail) : 0, o_flag = wide ? blob.add(std::vector<uint32_t>(nq + 1, 0u)) : 0;
+    const size_t o_s = wide ? blob.add(streams.all) : 0, o_sa = wide ? blob.add(streams.at) : 0;
     const size_t o_rows = check ? 0 : blob.add(std::vector<uint64_t>(row_offsets, row_offsets + nq));
     unsigned char* dev;
     SLHA_TRY(send_tables(c, blob, &dev, check));
@@ -1035,14 +1074,18 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     const uint32_t grid = (uint32_t)cuts.cta.size() - 1;
     if (wide) {
         a.handoff = reinterpret_cast<uint32_t*>(dev + o_flag);
+        a.handoff_any = a.handoff + nq;
         a.handoff_as = 1u;
         SLHA_TRY(launch_wide_dense(c, a, grid, true));
         a.only_flagged = a.handoff;
-        a.by_fours = 1u;
+        a.streams = reinterpret_cast<const WorkItem*>(dev + o_s);
+        a.stream_at = reinterpret_cast<const uint2*>(dev + o_sa);
+        a.n_streams = (uint32_t)streams.all.size();
+        a.unit_share = streams.share;
     } else if (a.n_items == grid) {
         a.cta_begin = nullptr;
     }
-    if (!g_force_generic) return launch_dense(c, a, grid, true);
+    if (!g_force_generic) return launch_dense(c, a, wide ? streams.grid : grid, true);
     a.items = reinterpret_cast<const WorkItem*>(dev + o_gen);
     const int threads = 128, nwarps = threads / 32;
     return launch_score<false>(c, 4, a, (uint32_t)generic.size(), threads, score_smem_bytes(4, nwarps, false, 0), false);
@@ -1071,12 +1114,16 @@ static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, con
     if (p->wide) {
         a.blocked = 1u;
         a.handoff = p->d_row_flags + nq;
+        a.handoff_any = p->d_row_flags + 4 * nq;
         a.handoff_as = 2u;
         SLHA_TRY(launch_wide_dense(c, a, p->mma_grid, true));
         a.only_flagged = a.handoff;
-        a.by_fours = 1u;  // (the pass takes the same items, four rows at a time)
+        a.streams = p->d_streams;
+        a.stream_at = p->d_stream_at;
+        a.n_streams = p->n_streams;
+        a.unit_share = p->unit_share;
     }
-    SLHA_TRY(launch_dense(c, a, p->mma_grid, true));
+    SLHA_TRY(launch_dense(c, a, p->wide ? p->streams_grid : p->mma_grid, true));
     if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));
     RowsArgs r{a.scores, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, p->kp2, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
     SLHA_TRY(launch_rows(c, r, (uint32_t)nq, p->longest));

@@ -24,7 +24,7 @@ struct RowInfo {
 struct RowsArgs {
     const float* scores;
     const RowInfo* rows;
-    uint32_t* flag;          // [nq] a work item of the row took the generic arithmetic, [nq] it was handed on by the 64-row kernel (cleared here)
+    uint32_t* flag;          // [nq] a work item of the row took the generic arithmetic, [nq] it was handed on by the 64-row kernel, [4 nq] whether any was (cleared here)
     uint32_t* stats;         // [nq][2] candidates, the flag
     uint32_t k, kp2, cap;    // cap: slots for candidates, row_cap(k, kp2)
     uint32_t* out_index;
@@ -498,6 +498,7 @@ __global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
         a.stats[2 * Q] = got;
         a.stats[2 * Q + 1] = a.flag[Q];
         a.flag[Q] = a.flag[gridDim.x + Q] = 0u;
+        if (Q == 0) a.flag[4 * (size_t)gridDim.x] = 0u;
     }
 }
 

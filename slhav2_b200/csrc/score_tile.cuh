@@ -374,7 +374,7 @@ __device__ __forceinline__ uint32_t first_tile_flags(const ScoreArgs& a, const W
 // index_base + i; -inf for COLD slots) and nothing is filtered or appended.  IL: the work items are interleaved shares of
 // whole streams (see the planner).  A tile of another codec than KIND's, or a query outside the fp16 split, hands the
 // item's query rows to the generic kernel.
-template <int KIND, bool IL, bool DENSE, bool KINDS>
+template <int KIND, bool IL, bool DENSE, bool KINDS, bool PASS = false>
 __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, uint32_t item_id, uint32_t item_end, WorkItem& it, uint32_t& flags0, bool nf4_too = false) {
     constexpr int NWG = ST_WG, NWARPS = 4 * NWG, NACC = st_accs(KIND);
     constexpr uint32_t STRIDE = ST_TMEM, DCOL = st_d_col(KIND);
@@ -420,7 +420,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
 
     auto next_item = [&]() {  // false at the end, or at an item of another kind (the same in the whole CTA)
         if (++item_id >= item_end) return false;
-        it = DENSE ? dense_item(a, item_id) : a.stream_items[item_id];
+        it = DENSE ? dense_item<PASS>(a, item_id) : a.stream_items[item_id];
         if (KINDS) flags0 = first_tile_flags(a, it);
         return !KINDS || item_kind(flags0, nf4_too) == KIND;
     };
@@ -446,13 +446,13 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             if (j >= my_rounds) j -= my_rounds;
             return (j * il_n + il_c) * (uint32_t)NWG + (uint32_t)wg;
         };
-        if (DENSE && a.only_flagged) {  // a second pass: only the items one of whose rows the first pass handed over
+        if (PASS) {  // only the items one of whose rows the first pass handed over
             uint32_t f = 0;
             for (int q = 0; q < nq; ++q) f |= a.only_flagged[it.query_begin + q];
             if (!f) continue;  // (the same in the whole CTA)
             if (f & 2u) {
                 if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
-                if (tid == 0) undone_add(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
+                if (tid == 0) undone_add<PASS>(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
                 cta.undone = true;
                 continue;
             }
@@ -858,7 +858,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             // rows this CTA could not score on the tensor cores go to the generic kernel as a whole; of dense calls the item, at the CTA's end
             if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
             if (DENSE) {
-                if (tid == 0) undone_add(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
+                if (tid == 0) undone_add<PASS>(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
                 cta.undone = true;
             }
         }
@@ -890,22 +890,25 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_mix3_kernel(ScoreArgs a) 
 // Dense scores.  Every work item is decoded as what its first tile says (read here: a host that looked would wait for the
 // stream); a tile of another kind inside the item hands its rows over as everywhere.  An arena known to hold NF4 beside INT4
 // tiles is decoded as NF4 throughout.
+// PASS: behind the 64-row kernel, of the rows that it handed on.
+template <bool PASS>
 __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid_constant__ ScoreArgs a) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     dep_launch();
     dep_wait();
     if (a.refused && *a.refused) return;
-    uint32_t i = dense_first(a, blockIdx.x);
-    const uint32_t item_end = dense_first(a, blockIdx.x + 1);
-    if (a.only_flagged) {  // (a pass with nothing to do, as behind the 64-row kernel, ends here)
+    if (PASS && !*a.handoff_any) return;
+    uint32_t i = dense_first<PASS>(a);
+    const uint32_t item_end = dense_end<PASS>(a);
+    if (PASS) {  // (with nothing to do a CTA ends here)
         uint32_t f = 0;
         for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS) {
-            const WorkItem own = dense_item(a, e);
+            const WorkItem own = dense_item<PASS>(a, e);
             for (uint32_t q = 0; q < own.n_queries; ++q) f |= a.only_flagged[own.query_begin + q];
         }
         if (!__syncthreads_or(f != 0u)) return;
     }
-    WorkItem it = dense_item(a, i);
+    WorkItem it = dense_item<PASS>(a, i);
     uint32_t flags = first_tile_flags(a, it);  // (on its way while the CTA is set up, and the first item's queries with it)
     if (threadIdx.x < 4u * it.n_queries) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_coarse + (size_t)it.query_begin * D_C + 32u * threadIdx.x));
     if (threadIdx.x == 32) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_sign + (size_t)it.query_begin * 8));
@@ -916,17 +919,17 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     TileCta cta = tile_open<true>(smem_raw);
     for (;;) {
         switch (item_kind(flags, nf4_too)) {
-            case 0: i = tile_run<0, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
-            case 1: i = tile_run<1, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
-            case 2: i = tile_run<2, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
-            case 3: i = tile_run<3, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
-            default: i = tile_run<4, false, true, true>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 0: i = tile_run<0, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 1: i = tile_run<1, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 2: i = tile_run<2, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;
+            case 3: i = tile_run<3, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;
+            default: i = tile_run<4, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;
         }
         if (i >= item_end) break;
     }
     tile_close(cta);
     static_assert(4096 + (ST_THREADS / 32) * BLK_BYTES <= TileLayout<true>::UNDONE, "below the bits");
-    if (cta.undone) finish_undone(a, bits, smem_raw);
+    if (cta.undone) finish_undone<PASS>(a, bits, smem_raw);
 }
 
 }  // namespace

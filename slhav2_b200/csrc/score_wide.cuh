@@ -119,6 +119,7 @@ __device__ __forceinline__ void wide_sign_words(const uint4& x, uint32_t ta) {
 // Dense calls: an item's rows go to the four-row kernel's pass.  (CTAs that share the rows may hand them on for different reasons: the pass sees them all, whichever came last.)
 __device__ __forceinline__ void wide_hand_on(const ScoreArgs& a, const WorkItem& it, uint32_t as) {
     if (threadIdx.x < it.n_queries) atomicOr(a.handoff + it.query_begin + threadIdx.x, as);
+    if (threadIdx.x == 0) *a.handoff_any = 1u;
 }
 // what an item that wide_body did not score is handed on as: it is NF4 where its first tile is
 __device__ __forceinline__ uint32_t wide_hand_as(const ScoreArgs& a, const WorkItem& it) {

@@ -406,3 +406,36 @@ def test_segments_that_are_left_to_the_generic_arithmetic_leave_the_others_as_th
             for j in (nq * i, nq * i + nq - 1):
                 want = ora.score_tiles(mixed[m * i:m * i + m], qc[j], qs[j])
                 assert np.all(np.abs(now[0][j] - want) <= 1e-3 * (1 + np.abs(want))) and np.all(np.abs(now[2][j] - want[now[1][j]]) <= 1e-3)
+
+
+def test_nf4_rows_of_many_queries_cost_what_the_same_rows_cost_four_at_a_time():
+    # 40 rows a segment, handed on by the 64-row kernel and cut into equal shares again: shares end inside groups of four rows and at ragged ends
+    import time
+
+    n, nq, base = 20_013, 40, 9
+    tiles = H.random_tiles(2 * n, 2, seed=550, warm_every=11)
+    qc, qs = H.random_queries(2 * nq, 551)
+    dt, dq, ds = S.to_device(tiles), S.to_device(qc), S.to_device(qs)
+    row_len = n + base
+    off = S.to_device(np.arange(2 * nq, dtype=np.uint64) * row_len)
+    whole = S.make_segments([(0, n, 0, nq, base), (n, n, nq, nq, base)])
+    fours = S.make_segments([(i // 10 * n, n, 4 * i, 4, base) for i in range(20)])
+    outs, took = [], []
+    for seg in (whole, fours):
+        out = S.DeviceBuffer(2 * nq * row_len * 4)
+        out.upload(np.zeros(2 * nq * row_len, F))
+        for rep in range(2):
+            S.synchronize()
+            t = []
+            for _ in range(30):
+                t0 = time.perf_counter()
+                S.score_segments(dt, seg, dq, ds, 2 * nq, out, off, row_len)
+                S.synchronize()
+                t.append(time.perf_counter() - t0)
+        took.append(float(np.median(t)))
+        outs.append(out.download(F, 2 * nq * row_len).reshape(2 * nq, row_len))
+    assert outs[0].tobytes() == outs[1].tobytes()
+    for j in (0, 3, 39, 40, 77):
+        want = ora.score_tiles(tiles[j // nq * n:j // nq * n + n], qc[j], qs[j])
+        assert np.all(np.abs(outs[0][j, base:] - want) <= 1e-3 * (1 + np.abs(want)))
+    assert took[0] < 1.4 * took[1], took
