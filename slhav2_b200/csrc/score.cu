@@ -490,10 +490,11 @@ __device__ __forceinline__ uint32_t dense_end(const ScoreArgs& a) {
     if (PASS) return dense_group(a, min((blockIdx.x + 1u) * a.unit_share, a.stream_at[a.n_streams].y) - 1u) + 1u;
     return a.cta_begin ? a.cta_begin[blockIdx.x + 1] : blockIdx.x + 1u;
 }
+// s: item e's stream (PASS)
 template <bool PASS>
-__device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e) {
+__device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e, uint32_t s) {
     if (!PASS) return a.stream_items[e];
-    const uint32_t s = dense_stream<false>(a, e), q = 4u * (e - a.stream_at[s].x);
+    const uint32_t q = 4u * (e - a.stream_at[s].x);
     WorkItem it = a.streams[s];
     const uint32_t blocks = (it.n_tiles + 127u) / 128u, at = a.stream_at[s].y + q / 4u * blocks, mine = blockIdx.x * a.unit_share;
     const uint32_t lo = max(mine, at) - at, hi = min(mine + a.unit_share, at + blocks) - at;
@@ -585,7 +586,7 @@ __device__ __noinline__ void finish_undone(const ScoreArgs& a, const uint32_t* b
     for (uint32_t e = 0; e < items; ++e) {
         const uint32_t bit = e >> shift;
         if (!(bits[bit >> 5] >> (bit & 31u) & 1u)) continue;
-        const WorkItem it = dense_item<PASS>(a, first + e);
+        const WorkItem it = dense_item<PASS>(a, first + e, PASS ? dense_stream<false>(a, first + e) : 0u);
         for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
     }
 }

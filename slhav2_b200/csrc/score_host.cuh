@@ -202,6 +202,11 @@ struct Blob {
         if (!v.empty()) std::memcpy(bytes.data() + at, v.data(), v.size() * sizeof(T));
         return at;
     }
+    size_t zeros = 0;  // words of zeros behind them (the last to be added)
+    size_t add_zeros(size_t words) {
+        zeros = words;
+        return (bytes.size() + 15) / 16 * 16;
+    }
 };
 
 // The cached decomposition of one score_topk call shape.
@@ -306,16 +311,28 @@ struct Cuts {
 
 // What the four-row kernel's pass behind the 64-row kernel is given, see ScoreArgs::streams.
 struct Streams {
-    std::vector<WorkItem> all;
+    std::vector<WorkItem> all;  // (empty: the 64-row kernel's items themselves, of which most are whole streams where these are short)
     std::vector<uint2> at{make_uint2(0u, 0u)};
     uint32_t share = 1, grid = 0;
-    // (`place`, `step`: of whole rows in blocks)
-    void add(const SlhaB200Segment& s, uint32_t q0, uint32_t place = 0, uint32_t step = 0) {
-        const uint32_t rows = std::min<uint32_t>(WIDE_NQ, s.n_queries - q0), groups = (rows + 3) / 4;
-        all.push_back(WorkItem{s.tile_begin, s.n_tiles, s.index_base, s.query_begin + q0, rows, place, step});
-        at.push_back(make_uint2(at.back().x + groups, at.back().y + groups * ((s.n_tiles + 127u) / 128u)));
-    }
-    void finish(int sms, uint32_t least) {
+    // items: in the order of the streams, and of their tiles
+    void make(const std::vector<WorkItem>& items, int sms, uint32_t least) {
+        size_t streams = 0;
+        auto goes_on = [&](size_t i) {
+            if (i == 0) return false;
+            const WorkItem &w = items[i], &v = items[i - 1];
+            return w.query_begin == v.query_begin && w.n_queries == v.n_queries && w.tile_begin == v.tile_begin + v.n_tiles && w.index_base == v.index_base + v.n_tiles;
+        };
+        for (size_t i = 0; i < items.size(); ++i) streams += !goes_on(i);
+        const bool merge = 2 * streams <= items.size();
+        all.reserve(merge ? streams : 0);
+        at.reserve((merge ? streams : items.size()) + 1);
+        for (size_t i = 0; i < items.size();) {
+            WorkItem w = items[i++];
+            for (; merge && i < items.size() && goes_on(i); ++i) w.n_tiles += items[i].n_tiles;
+            const uint32_t groups = (w.n_queries + 3) / 4;
+            if (merge) all.push_back(w);
+            at.push_back(make_uint2(at.back().x + groups, at.back().y + groups * ((w.n_tiles + 127u) / 128u)));
+        }
         const uint32_t blocks = at.back().y;
         share = std::max(least, (blocks + (uint32_t)sms - 1) / (uint32_t)sms);
         grid = (blocks + share - 1) / share;
@@ -376,9 +393,6 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
         for (size_t i = 0; i < n_segs; ++i)
             for (uint32_t q0 = 0; q0 < segs[i].n_queries && segs[i].n_tiles; q0 += WIDE_NQ) {
                 const uint32_t m = std::min<uint32_t>(WIDE_NQ, segs[i].n_queries - q0);
-                SlhaB200Segment s = segs[i];
-                s.index_base = 0;
-                streams.add(s, q0, (uint32_t)floats, 128 * m);
                 for (uint32_t q = 0; q < m; ++q) {
                     rows[segs[i].query_begin + q0 + q].begin = (uint32_t)(floats + 128 * q);
                     rows[segs[i].query_begin + q0 + q].step = 128 * m;
@@ -393,7 +407,7 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     } else {
         for (size_t q = 0; q < nq; ++q) rows[q].begin = (uint32_t)(q * p->row_stride);
     }
-    streams.finish(sms, 1);
+    if (wide) streams.make(cuts.items, sms, 1);
     Blob tables;
     const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows), o_s = tables.add(streams.all), o_sa = tables.add(streams.at);
     SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
@@ -409,9 +423,9 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     p->mma_grid = (uint32_t)cuts.cta.size() - 1;
     p->d_cta_begin = !wide && p->n_items == p->mma_grid ? nullptr : reinterpret_cast<uint32_t*>(dev + o_nc);  // (null: an item a CTA)
     p->d_rows = reinterpret_cast<RowInfo*>(dev + o_r);
-    p->d_streams = reinterpret_cast<WorkItem*>(dev + o_s);
+    p->d_streams = streams.all.empty() ? p->d_items : reinterpret_cast<WorkItem*>(dev + o_s);
     p->d_stream_at = reinterpret_cast<uint2*>(dev + o_sa);
-    p->n_streams = (uint32_t)streams.all.size();
+    p->n_streams = (uint32_t)streams.at.size() - 1;
     p->unit_share = streams.share;
     p->streams_grid = streams.grid;
     p->longest = longest;
@@ -491,19 +505,14 @@ Status build_plan(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB200Segment* s
             wide = wide && (segs[i].n_queries >= 16 || segs[i].n_tiles == 0);
             passes += (uint64_t)segs[i].n_tiles * ((segs[i].n_queries + 3) / 4);
         }
-        // (NF4 tiles, which the 64-row kernel does not decode, are taken four rows at a time from the start: handed on by that kernel, whose work items are short, 40 rows on each of 2 x 20 000
-        // tiles k = 100 took 101 us a call instead of 40, 250 on 32 768 219 instead of 116)
+        // The 64-row kernel hands NF4 tiles on to score_dense_kernel, so whether they had better be streamed has to be known first, where the rule for four rows says so (250 NF4 rows on 32 768
+        // tiles, k = 16 100 us a call, 130 whole).  Elsewhere nobody looks: a new shape of other tiles would wait 18 us for what saves 5 of 34 on NF4 (64 rows on each of 4 x 3000).
         wide = wide && allow_wide;
         RowsRule rule = rows_rule(passes, wide, nq, longest, k);
-        if (rule == ROWS_UNLESS_NF4 || (rule == ROWS_YES && wide)) {
+        if (rule == ROWS_UNLESS_NF4 || (rule == ROWS_YES && wide && rows_rule(passes, false, nq, longest, k) != ROWS_YES)) {
             SLHA_TRY(look());
             looked = true;
-            if (p->kind == 0) {
-                wide = false;
-                rule = rows_rule(passes, false, nq, longest, k) == ROWS_YES ? ROWS_YES : ROWS_NO;
-            } else {
-                rule = ROWS_YES;
-            }
+            rule = p->kind == 0 ? ROWS_NO : ROWS_YES;
         }
         if (rule == ROWS_YES) {
             SLHA_TRY(build_rows_plan(c, p, segs, n_segs, nq, longest, wide));
@@ -854,12 +863,12 @@ struct TableParam {
 };
 constexpr uint32_t TABLE_SLICE = 2048;  // bytes a block copies (parameters are read one address at a time)
 template <int BYTES>
-__global__ void __launch_bounds__(256) table_kernel(const __grid_constant__ TableParam<BYTES> table, uint32_t n16, uint4* dst, const uint64_t* offsets, uint32_t nq, uint64_t scores_len,
+__global__ void __launch_bounds__(256) table_kernel(const __grid_constant__ TableParam<BYTES> table, uint32_t n16, uint32_t with_zeros, uint4* dst, const uint64_t* offsets, uint32_t nq, uint64_t scores_len,
                                                     uint32_t row_len, uint64_t* copy, uint32_t* refused, uint32_t* answer, uint32_t check_no) {
     dep_launch();
     dep_wait();
     const uint32_t i = blockIdx.x * (TABLE_SLICE / 16) + threadIdx.x;
-    if (threadIdx.x < TABLE_SLICE / 16 && i < n16) dst[i] = table.w[i];
+    if (threadIdx.x < TABLE_SLICE / 16 && i < with_zeros) dst[i] = i < n16 ? table.w[i] : make_uint4(0u, 0u, 0u, 0u);
     if (blockIdx.x || !offsets) return;
     bool bad = false;
     for (uint32_t q = threadIdx.x; q < nq; q += blockDim.x) {
@@ -880,13 +889,14 @@ Status launch_table_t(Ctx* c, const Blob& blob, uint4* dst, const uint64_t* offs
                       uint32_t check_no) {
     static thread_local TableParam<BYTES> table;
     std::memcpy(&table, blob.bytes.data(), blob.bytes.size());
-    const uint32_t n16 = (uint32_t)((blob.bytes.size() + 15) / 16), blocks = std::max<uint32_t>(1, (n16 * 16 + TABLE_SLICE - 1) / TABLE_SLICE);
-    SLHA_CUDA(launch_behind(table_kernel<BYTES>, dim3(blocks), dim3(256), 0, c->stream, table, n16, dst, offsets, nq, scores_len, row_len, copy, refused, answer, check_no));
+    const uint32_t n16 = (uint32_t)((blob.bytes.size() + 15) / 16), with_zeros = n16 + (uint32_t)((blob.zeros + 3) / 4);
+    const uint32_t blocks = std::max<uint32_t>(1, (uint32_t)(((uint64_t)with_zeros * 16 + TABLE_SLICE - 1) / TABLE_SLICE));
+    SLHA_CUDA(launch_behind(table_kernel<BYTES>, dim3(blocks), dim3(256), 0, c->stream, table, n16, with_zeros, dst, offsets, nq, scores_len, row_len, copy, refused, answer, check_no));
     count_launch();
     return Status();
 }
 // The call's tables to the device (*dev), and the check of `check`'s offsets, if any, with them.
-Status send_tables(Ctx* c, const Blob& blob, unsigned char** dev, RowCheck* check) {
+Status send_tables(Ctx* c, Blob& blob, unsigned char** dev, RowCheck* check) {
     SLHA_TRY(ctx_no_capture(c));
     const bool in_params = blob.bytes.size() <= 16384;
     uint64_t* copy = nullptr;
@@ -906,7 +916,8 @@ Status send_tables(Ctx* c, const Blob& blob, unsigned char** dev, RowCheck* chec
     const uint64_t* offsets = check ? check->offsets : nullptr;
     const uint32_t nq = check ? (uint32_t)check->nq : 0u, row_len = check ? check->row_len : 0u;
     const uint64_t len = check ? check->scores_len : 0ull;
-    if (in_params && !blob.bytes.empty()) SLHA_TRY(ctx_device_scratch(c, (blob.bytes.size() + 15) / 16 * 16, (void**)dev));
+    if (!in_params) blob.bytes.resize((blob.bytes.size() + 15) / 16 * 16 + 4 * blob.zeros);  // (uploaded with the rest)
+    if (in_params && !blob.bytes.empty()) SLHA_TRY(ctx_device_scratch(c, (blob.bytes.size() + 15) / 16 * 16 + (blob.zeros + 3) / 4 * 16, (void**)dev));
     else if (!blob.bytes.empty()) SLHA_TRY(ctx_upload(c, blob.bytes.data(), blob.bytes.size(), (void**)dev));
     uint4* dst = in_params ? reinterpret_cast<uint4*>(*dev) : nullptr;
     static const Blob none;
@@ -925,7 +936,8 @@ Status send_tables(Ctx* c, const Blob& blob, unsigned char** dev, RowCheck* chec
 }
 Status launch_row_check(Ctx* c, RowCheck* check) {
     unsigned char* dev = nullptr;
-    return send_tables(c, Blob(), &dev, check);
+    Blob none;
+    return send_tables(c, none, &dev, check);
 }
 // (The host polls the word: recording an event and waiting for it cost 3 us of a call of 17.)
 Status checked_offsets(Ctx* c, RowCheck& check, bool* refused) {
@@ -1032,9 +1044,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     for (size_t i = 0; i < n_segs; ++i) cuts.add(segs[i], wide ? WIDE_NQ : 4);
     cuts.finish();
     Streams streams;
-    for (size_t i = 0; i < n_segs && wide; ++i)
-        for (uint32_t q0 = 0; q0 < segs[i].n_queries && segs[i].n_tiles; q0 += WIDE_NQ) streams.add(segs[i], q0);
-    streams.finish(sms, 4);
+    if (wide) streams.make(cuts.items, sms, 4);
     std::vector<WorkItem> generic;  // runs of 4096 tiles where score_kernel takes the call
     if (g_force_generic)
         for (const WorkItem& s : cuts.items)
@@ -1047,9 +1057,10 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
             }
     Blob blob;
     const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta), o_gen = blob.add(generic);
-    const size_t o_tail = fills ? blob.add(tail) : 0, o_flag = wide ? blob.add(std::vector<uint32_t>(nq + 1, 0u)) : 0;
-    const size_t o_s = wide ? blob.add(streams.all) : 0, o_sa = wide ? blob.add(streams.at) : 0;
+    const size_t o_tail = fills ? blob.add(tail) : 0;
+    const size_t o_s = streams.all.empty() ? o_items : blob.add(streams.all), o_sa = wide ? blob.add(streams.at) : 0;
     const size_t o_rows = check ? 0 : blob.add(std::vector<uint64_t>(row_offsets, row_offsets + nq));
+    const size_t o_flag = wide ? blob.add_zeros(nq + 1) : 0;
     unsigned char* dev;
     SLHA_TRY(send_tables(c, blob, &dev, check));
     const unsigned long long* d_row_offsets = reinterpret_cast<const unsigned long long*>(check ? check->copy : reinterpret_cast<const uint64_t*>(dev + o_rows));
@@ -1080,7 +1091,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
         a.only_flagged = a.handoff;
         a.streams = reinterpret_cast<const WorkItem*>(dev + o_s);
         a.stream_at = reinterpret_cast<const uint2*>(dev + o_sa);
-        a.n_streams = (uint32_t)streams.all.size();
+        a.n_streams = (uint32_t)streams.at.size() - 1;
         a.unit_share = streams.share;
     } else if (a.n_items == grid) {
         a.cta_begin = nullptr;

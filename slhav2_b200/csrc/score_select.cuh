@@ -121,7 +121,7 @@ __device__ __forceinline__ const uint64_t* row_sort(uint64_t* buf, uint32_t cap,
 
 // R: 4 R scores a thread, n <= 4 R x threads
 template <int NT, int R>
-__global__ void __launch_bounds__(NT) topk_rows_kernel(RowsArgs a) {
+__global__ void __launch_bounds__(NT, R <= 2 ? 1536 / NT : R <= 8 ? 2 : 1) topk_rows_kernel(RowsArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     const RowInfo info = a.rows[blockIdx.x];  // (the plan's: no kernel writes it)
     dep_launch();

@@ -314,6 +314,7 @@ struct TileCta {
     uint32_t phase;    // of the warpgroup's mbarrier
     bool failed;       // a wait of this warp ran out
     bool undone;       // dense: an item was left, see undone_add
+    uint32_t stream;   // of the item (PASS)
 };
 template <bool DENSE>
 struct TileLayout {
@@ -350,6 +351,7 @@ __device__ __forceinline__ TileCta tile_open(unsigned char* smem_raw) {
     t.table = false;
     t.phase = 0u;
     t.failed = t.undone = false;
+    t.stream = 0u;
     return t;
 }
 __device__ __forceinline__ void tile_close(const TileCta& t) {
@@ -420,7 +422,8 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
 
     auto next_item = [&]() {  // false at the end, or at an item of another kind (the same in the whole CTA)
         if (++item_id >= item_end) return false;
-        it = DENSE ? dense_item<PASS>(a, item_id) : a.stream_items[item_id];
+        if (PASS && item_id >= a.stream_at[cta.stream + 1u].x) ++cta.stream;  // (every stream has a group)
+        it = DENSE ? dense_item<PASS>(a, item_id, cta.stream) : a.stream_items[item_id];
         if (KINDS) flags0 = first_tile_flags(a, it);
         return !KINDS || item_kind(flags0, nf4_too) == KIND;
     };
@@ -903,12 +906,13 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     if (PASS) {  // (with nothing to do a CTA ends here)
         uint32_t f = 0;
         for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS) {
-            const WorkItem own = dense_item<PASS>(a, e);
+            const WorkItem own = dense_item<PASS>(a, e, dense_stream<false>(a, e));
             for (uint32_t q = 0; q < own.n_queries; ++q) f |= a.only_flagged[own.query_begin + q];
         }
         if (!__syncthreads_or(f != 0u)) return;
     }
-    WorkItem it = dense_item<PASS>(a, i);
+    const uint32_t stream = PASS ? dense_stream<false>(a, i) : 0u;
+    WorkItem it = dense_item<PASS>(a, i, stream);
     uint32_t flags = first_tile_flags(a, it);  // (on its way while the CTA is set up, and the first item's queries with it)
     if (threadIdx.x < 4u * it.n_queries) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_coarse + (size_t)it.query_begin * D_C + 32u * threadIdx.x));
     if (threadIdx.x == 32) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_sign + (size_t)it.query_begin * 8));
@@ -917,6 +921,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     uint32_t* const bits = reinterpret_cast<uint32_t*>(tile_base(smem_raw) + TileLayout<true>::UNDONE);
     for (uint32_t w = threadIdx.x; w < min((item_end - i + 31u) / 32u, (uint32_t)UNDONE_WORDS); w += ST_THREADS) bits[w] = 0u;  // (ordered by tile_open's barrier)
     TileCta cta = tile_open<true>(smem_raw);
+    cta.stream = stream;
     for (;;) {
         switch (item_kind(flags, nf4_too)) {
             case 0: i = tile_run<0, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;

@@ -439,3 +439,16 @@ def test_nf4_rows_of_many_queries_cost_what_the_same_rows_cost_four_at_a_time():
         want = ora.score_tiles(tiles[j // nq * n:j // nq * n + n], qc[j], qs[j])
         assert np.all(np.abs(outs[0][j, base:] - want) <= 1e-3 * (1 + np.abs(want)))
     assert took[0] < 1.4 * took[1], took
+
+
+def test_segments_that_continue_one_another_in_the_tiles_but_not_in_the_row():
+    # NF4 rows of two segments each: the second takes the tiles behind the first's and writes them elsewhere in the row, beside ones that do go on
+    n, nq, row_len = 700, 16, 4000
+    tiles = H.random_tiles(4 * n, 2, seed=560)
+    qc, qs = H.random_queries(2 * nq, 561)
+    rows = [(0, n, 0, nq, 0), (n, n, 0, nq, 2000), (2 * n, n, nq, nq, 100), (3 * n, n, nq, nq, 100 + n)]
+    out = S.score_segments(S.to_device(tiles), S.make_segments(rows), qc, qs, 2 * nq, np.zeros((2 * nq, row_len), F), np.arange(2 * nq, dtype=np.uint64) * row_len, row_len)
+    for tb, m, q0, q, base in rows:
+        for j in range(q0, q0 + q, 5):
+            want = ora.score_tiles(tiles[tb:tb + m], qc[j], qs[j])
+            assert np.all(np.abs(out[j, base:base + m] - want) <= 1e-3 * (1 + np.abs(want)))
