@@ -246,3 +246,12 @@ def test_nf4_rows_of_many_queries(n, nq, k, kernel):
     for j in range(0, nq, 13):
         want = ora.score_tiles(tiles, qc[j], qs[j])
         assert np.all(np.abs(sc[j] - want[idx[j] - 7]) <= 1e-3 * (1 + np.abs(sc[j]))) and np.all(np.abs(sc[j] - np.sort(want)[::-1][:k]) <= 2e-3 * (1 + np.abs(sc[j])))
+
+
+@pytest.mark.parametrize("n,k", [(1, 1), (127, 64), (255, 255), (256, 300), (257, 64), (1000, 64), (1024, 17), (1025, 17), (900, 65)])
+def test_many_short_rows(n, k):
+    # from 1024 rows on, short ones of which little is selected take half as many threads each
+    rng = np.random.default_rng(n + k)
+    tiles = H.random_tiles(500, 4, seed=97, warm_every=9)[rng.integers(0, 500, 2 * n)]
+    qc, qs = H.random_queries(1030, 98)
+    _check(tiles, [(0, n, 0, 515, 3), (n, n - n // 5, 515, 515, 90)], 1030, k, qc, qs)
