@@ -303,12 +303,11 @@ struct ScoreArgs {
     uint32_t* gcount;             // per query row: candidates appended to the row's buffer
     uint32_t* gflag;              // per query row: 1 = the generic kernel scores the row's work items
     uint32_t blocked;             // dense mode: item's scores lie in blocks of 128 tiles, block b's of its row q from list_begin + b * pad + 128 q on
-    // score_dense_kernel<true>, behind the 64-row kernel: whole streams (a segment's tiles, up to 64 query rows), which it cuts for itself: in groups of four rows, blocks of 128 tiles, unit_share of
-    // them a CTA in order.  (A list of those cuts would be twice as long as all that a dense call brings; the 64-row kernel's own cuts, four rows at a time, are a set-up for every two or
-    // three blocks: 40 rows on each of 2 x 20 000 NF4 tiles 98 us a call instead of 40.)
+    // score_dense_kernel<true>, behind the 64-row kernel: whole streams (a segment's tiles, up to 64 query rows), of which it scores what was handed on, in groups of four rows and an equal
+    // share of their blocks of 128 tiles a CTA, see PassRange.  (A list of such shares would be twice as long as all that a dense call brings; the 64-row kernel's own items, four rows at a
+    // time, are a set-up for every two or three blocks: 40 rows on each of 2 x 20 000 NF4 tiles 98 us a call instead of 40.)
     const WorkItem* streams;
-    const uint2* stream_at;       // [n_streams + 1] groups, blocks before a stream
-    uint32_t n_streams, unit_share;
+    uint32_t n_streams, least_share;
     uint32_t* handoff_any;        // 1 where that kernel handed rows on
     uint32_t* handoff;            // dense mode of the 64-row kernel: rows for the four-row kernel's pass (only_flagged there): bit 0, or bit 1 where that pass is to
     uint32_t handoff_as;          // score them in score_kernel's arithmetic (items that begin with an NF4 tile: always bit 0)
@@ -463,41 +462,39 @@ __global__ void __launch_bounds__(256) score_kernel(ScoreArgs a) {
     }
 }
 
-// The last stream that begins at or before x (of its groups, or of its blocks).
-template <bool BLOCKS>
-__device__ __forceinline__ uint32_t dense_stream(const ScoreArgs& a, uint32_t x) {
-    uint32_t lo = 0, hi = a.n_streams;
-    while (hi - lo > 1u) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((BLOCKS ? a.stream_at[mid].y : a.stream_at[mid].x) <= x) lo = mid;
-        else hi = mid;
-    }
-    return lo;
+// A CTA's items of a call of score_dense_kernel: first .. end (null: an item a CTA).
+__device__ __forceinline__ uint32_t dense_first(const ScoreArgs& a) { return a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x; }
+__device__ __forceinline__ uint32_t dense_end(const ScoreArgs& a) { return a.cta_begin ? a.cta_begin[blockIdx.x + 1] : blockIdx.x + 1u; }
+
+// What a CTA of score_dense_kernel<true> takes of the groups that were handed on: blocks mine .. end of all of theirs, from group `left`'s lowest bit of a stream on, which begins at block `at`.
+struct PassRange {
+    uint32_t mine, end, stream, left, at;
+};
+struct PassWalk {
+    uint32_t stream, left, at, blocks;  // of the item: the stream, its groups from the item's on, blocks before the group, of the group
+};
+__device__ __forceinline__ uint32_t pass_blocks(const ScoreArgs& a, uint32_t stream) { return (a.streams[stream].n_tiles + 127u) / 128u; }
+// the groups of a stream that were handed on, a bit each (all lanes of a warp)
+__device__ __forceinline__ uint32_t pass_groups(const ScoreArgs& a, uint32_t stream) {
+    const uint32_t q = 4u * (threadIdx.x & 15u), n = a.streams[stream].n_queries, row = a.streams[stream].query_begin;
+    uint32_t f = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+        if (q + j < n) f |= a.only_flagged[row + q + j];
+    return __ballot_sync(0xFFFFFFFFu, f != 0u) & 0xFFFFu;
 }
-// the group that a block belongs to
-__device__ __forceinline__ uint32_t dense_group(const ScoreArgs& a, uint32_t block) {
-    const uint32_t s = dense_stream<true>(a, block);
-    return a.stream_at[s].x + (block - a.stream_at[s].y) / ((a.streams[s].n_tiles + 127u) / 128u);
+__device__ __forceinline__ PassWalk pass_first(const ScoreArgs& a, const PassRange& r) { return PassWalk{r.stream, r.left, r.at, pass_blocks(a, r.stream)}; }
+__device__ __forceinline__ bool pass_next(const ScoreArgs& a, const PassRange& r, PassWalk& w) {  // false: that was the last
+    w.at += w.blocks;
+    if (w.at >= r.end) return false;
+    w.left &= w.left - 1u;
+    while (!w.left) w.left = pass_groups(a, ++w.stream);  // (there is one: not all blocks have been passed)
+    w.blocks = pass_blocks(a, w.stream);
+    return true;
 }
-// A CTA's items of a call of score_dense_kernel: first .. end (null: an item a CTA).  PASS: behind the 64-row kernel; an item is what the CTA takes of a stream's group.
-template <bool PASS>
-__device__ __forceinline__ uint32_t dense_first(const ScoreArgs& a) {
-    if (PASS) return dense_group(a, blockIdx.x * a.unit_share);
-    return a.cta_begin ? a.cta_begin[blockIdx.x] : blockIdx.x;
-}
-template <bool PASS>
-__device__ __forceinline__ uint32_t dense_end(const ScoreArgs& a) {
-    if (PASS) return dense_group(a, min((blockIdx.x + 1u) * a.unit_share, a.stream_at[a.n_streams].y) - 1u) + 1u;
-    return a.cta_begin ? a.cta_begin[blockIdx.x + 1] : blockIdx.x + 1u;
-}
-// s: item e's stream (PASS)
-template <bool PASS>
-__device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e, uint32_t s) {
-    if (!PASS) return a.stream_items[e];
-    const uint32_t q = 4u * (e - a.stream_at[s].x);
-    WorkItem it = a.streams[s];
-    const uint32_t blocks = (it.n_tiles + 127u) / 128u, at = a.stream_at[s].y + q / 4u * blocks, mine = blockIdx.x * a.unit_share;
-    const uint32_t lo = max(mine, at) - at, hi = min(mine + a.unit_share, at + blocks) - at;
+__device__ __forceinline__ WorkItem pass_item(const ScoreArgs& a, const PassRange& r, const PassWalk& w) {
+    const uint32_t q = 4u * ((uint32_t)__ffs(w.left) - 1u), lo = max(r.mine, w.at) - w.at, hi = min(r.end, w.at + w.blocks) - w.at;
+    WorkItem it = a.streams[w.stream];
     it.query_begin += q;
     it.n_queries = min(4u, it.n_queries - q);
     it.list_begin += 128u * q;
@@ -506,20 +503,75 @@ __device__ __forceinline__ WorkItem dense_item(const ScoreArgs& a, uint32_t e, u
     it.n_tiles = min(it.n_tiles, 128u * hi) - 128u * lo;
     return it;
 }
+// The CTA's share (r in shared memory); false: there is none.  512 threads.
+__device__ __forceinline__ bool pass_range(const ScoreArgs& a, PassRange& r) {
+    __shared__ uint32_t sums[16];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    auto handed = [&](uint32_t s) -> uint32_t {  // blocks of a stream's groups that were
+        if (s >= a.n_streams) return 0u;
+        const WorkItem w = a.streams[s];
+        uint32_t groups = 0;
+        for (uint32_t q = 0; q < w.n_queries; q += 4) {
+            uint32_t f = 0;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j)
+                if (q + j < w.n_queries) f |= a.only_flagged[w.query_begin + q + j];
+            groups += f != 0u;
+        }
+        return groups * ((w.n_tiles + 127u) / 128u);
+    };
+    auto before = [&](uint32_t own, uint32_t& all) -> uint32_t {  // of the threads before this one
+        uint32_t incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if ((int)lane >= o) incl += y;
+        }
+        __syncthreads();
+        if (lane == 31) sums[warp] = incl;
+        __syncthreads();
+        const uint32_t x = lane < 16 ? sums[lane] : 0u;
+        all = __reduce_add_sync(0xFFFFFFFFu, x);
+        return incl - own + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? x : 0u);
+    };
+    uint32_t total = 0, own = 0, at = 0, all;
+    for (uint32_t s0 = 0; s0 < a.n_streams; s0 += 512u) {
+        own = handed(s0 + tid);
+        at = before(own, all);
+        total += all;
+    }
+    const uint32_t share = max(a.least_share, (total + gridDim.x - 1u) / gridDim.x), mine = blockIdx.x * share;
+    if (mine >= total) return false;
+    uint32_t base = 0;
+    for (uint32_t s0 = 0; s0 < a.n_streams; s0 += 512u) {
+        if (a.n_streams > 512u) {  // (else as it was)
+            own = handed(s0 + tid);
+            at = before(own, all);
+        }
+        if (mine - base < all) {  // (the same in every thread)
+            if (own && base + at <= mine && mine < base + at + own) r = PassRange{mine, min(mine + share, total), s0 + tid, 0u, base + at};
+            break;
+        }
+        base += all;
+    }
+    __syncthreads();
+    uint32_t left = pass_groups(a, r.stream), first = r.at;
+    const uint32_t blocks = pass_blocks(a, r.stream);
+    for (; first + blocks <= mine; first += blocks) left &= left - 1u;
+    __syncthreads();
+    if (tid == 0) {
+        r.left = left;
+        r.at = first;
+    }
+    __syncthreads();
+    return true;
+}
 
 // Work items that a dense kernel's CTA could not score on the tensor cores (a tile of another codec than its item's first, a query outside the fp16
-// split): a bit each in shared memory, to be scored in score_kernel's arithmetic once the CTA is through.  (In its loop the call would cost registers, 70 of which it spilled.)
-constexpr int UNDONE_WORDS = 4096;
-// 0: a bit an item, as for any call up to 19 million of them; above, 2^shift items share one
-__device__ __forceinline__ uint32_t undone_shift(uint32_t items) {
-    return items <= 32u * UNDONE_WORDS ? 0u : 32u - (uint32_t)__clz((items - 1u) / (32u * UNDONE_WORDS));
-}
-// (one thread of the CTA)
-template <bool PASS>
-__device__ __forceinline__ void undone_add(const ScoreArgs& a, uint32_t* bits, uint32_t item) {
-    const uint32_t first = dense_first<PASS>(a), e = (item - first) >> undone_shift(dense_end<PASS>(a) - first);
-    bits[e >> 5] |= 1u << (e & 31u);
-}
+// split): a bit each in shared memory, to be scored in score_kernel's arithmetic once the CTA is through.  (In its loop the call would cost registers, 70 of which it spilled.)  Items beyond the
+// 32 767th of a CTA share the last bit.
+constexpr int UNDONE_WORDS = 1024;
+__device__ __forceinline__ uint32_t undone_bit(uint32_t no) { return min(no, 32u * UNDONE_WORDS - 1u); }
 // Dense scores of one work item by the whole CTA, rows query_begin .. + nq (four at most).  smem: 4 KB, and 4 KB a warp.
 __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem& it, uint32_t query_begin, int nq, unsigned char* smem) {
     constexpr int G = 4;
@@ -578,16 +630,20 @@ __device__ __forceinline__ void generic_item(const ScoreArgs& a, const WorkItem&
     }
     __syncthreads();
 }
-// What is left at a CTA's end (all of its shared memory but the bits is free).
+// What is left at a CTA's end (all of its shared memory but the bits is free); range: PASS.
 template <bool PASS>
-__device__ __noinline__ void finish_undone(const ScoreArgs& a, const uint32_t* bits, unsigned char* smem) {
+__device__ __noinline__ void finish_undone(const ScoreArgs& a, const uint32_t* bits, const PassRange* range, unsigned char* smem) {
     __syncthreads();
-    const uint32_t first = dense_first<PASS>(a), items = dense_end<PASS>(a) - first, shift = undone_shift(items);
-    for (uint32_t e = 0; e < items; ++e) {
-        const uint32_t bit = e >> shift;
-        if (!(bits[bit >> 5] >> (bit & 31u) & 1u)) continue;
-        const WorkItem it = dense_item<PASS>(a, first + e, PASS ? dense_stream<false>(a, first + e) : 0u);
-        for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
+    const uint32_t first = dense_first(a), items = PASS ? 0u : dense_end(a) - first;
+    PassWalk w{};
+    if (PASS) w = pass_first(a, *range);
+    for (uint32_t e = 0; PASS || e < items; ++e) {
+        const uint32_t bit = undone_bit(e);
+        if (bits[bit >> 5] >> (bit & 31u) & 1u) {
+            const WorkItem it = PASS ? pass_item(a, *range, w) : a.stream_items[first + e];
+            for (uint32_t q = 0; q < it.n_queries; q += 4) generic_item(a, it, it.query_begin + q, (int)min(4u, it.n_queries - q), smem);
+        }
+        if (PASS && !pass_next(a, *range, w)) break;
     }
 }
 

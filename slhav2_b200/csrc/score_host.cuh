@@ -268,8 +268,7 @@ struct Plan {
     RowInfo* d_rows = nullptr;
     uint32_t* d_row_flags = nullptr;  // [nq] generic arithmetic, [nq] handed on by the 64-row kernel, [nq][2] statistics, whether any row was handed on
     WorkItem* d_streams = nullptr;    // of the pass over those, see Streams
-    uint2* d_stream_at = nullptr;
-    uint32_t n_streams = 0, unit_share = 1, streams_grid = 0;
+    uint32_t n_streams = 0, streams_grid = 0;
     uint64_t last_use = 0;
     bool captured = false;  // a graph of the library's own names this plan's buffers (see plan_epoch)
 };
@@ -312,33 +311,33 @@ struct Cuts {
     }
 };
 
-// What the four-row kernel's pass behind the 64-row kernel is given, see ScoreArgs::streams.
+// What the four-row kernel's pass behind the 64-row kernel is given (ScoreArgs::streams): that kernel's items put together to whole streams, or, where most are whole streams, the items
+// themselves (`all` stays empty).
 struct Streams {
-    std::vector<WorkItem> all;  // (empty: the 64-row kernel's items themselves, of which most are whole streams where these are short)
-    std::vector<uint2> at{make_uint2(0u, 0u)};
-    uint32_t share = 1, grid = 0;
+    std::vector<WorkItem> all;
+    uint32_t n = 0, grid = 0;
     // items: in the order of the streams, and of their tiles
-    void make(const std::vector<WorkItem>& items, int sms, uint32_t least) {
-        size_t streams = 0;
+    void make(const std::vector<WorkItem>& items, int sms) {
         auto goes_on = [&](size_t i) {
             if (i == 0) return false;
             const WorkItem &w = items[i], &v = items[i - 1];
             return w.query_begin == v.query_begin && w.n_queries == v.n_queries && w.tile_begin == v.tile_begin + v.n_tiles && w.index_base == v.index_base + v.n_tiles;
         };
-        for (size_t i = 0; i < items.size(); ++i) streams += !goes_on(i);
-        const bool merge = 2 * streams <= items.size();
-        all.reserve(merge ? streams : 0);
-        at.reserve((merge ? streams : items.size()) + 1);
-        for (size_t i = 0; i < items.size();) {
-            WorkItem w = items[i++];
-            for (; merge && i < items.size() && goes_on(i); ++i) w.n_tiles += items[i].n_tiles;
-            const uint32_t groups = (w.n_queries + 3) / 4;
-            if (merge) all.push_back(w);
-            at.push_back(make_uint2(at.back().x + groups, at.back().y + groups * ((w.n_tiles + 127u) / 128u)));
+        uint64_t blocks = 0;
+        for (size_t i = 0; i < items.size(); ++i) {
+            n += !goes_on(i);
+            blocks += (uint64_t)((items[i].n_queries + 3) / 4) * ((items[i].n_tiles + 127u) / 128u);
         }
-        const uint32_t blocks = at.back().y;
-        share = std::max(least, (blocks + (uint32_t)sms - 1) / (uint32_t)sms);
-        grid = (blocks + share - 1) / share;
+        grid = (uint32_t)std::min<uint64_t>(blocks, (uint64_t)sms);
+        if (2 * (size_t)n > items.size()) {
+            n = (uint32_t)items.size();
+            return;
+        }
+        all.reserve(n);
+        for (size_t i = 0; i < items.size(); ++i) {
+            if (goes_on(i)) all.back().n_tiles += items[i].n_tiles;
+            else all.push_back(items[i]);
+        }
     }
 };
 
@@ -410,9 +409,9 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     } else {
         for (size_t q = 0; q < nq; ++q) rows[q].begin = (uint32_t)(q * p->row_stride);
     }
-    if (wide) streams.make(cuts.items, sms, 1);
+    if (wide) streams.make(cuts.items, sms);
     Blob tables;
-    const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows), o_s = tables.add(streams.all), o_sa = tables.add(streams.at);
+    const size_t o_n = tables.add(cuts.items), o_nc = tables.add(cuts.cta), o_r = tables.add(rows), o_s = tables.add(streams.all);
     SLHA_TRY(p->b_tables.ensure(tables.bytes.size()));
     SLHA_TRY(p->b_gpivot.ensure((4 * nq + 1) * 4));
     SLHA_TRY(p->b_gbuf.ensure(floats * 4));
@@ -427,9 +426,7 @@ Status build_rows_plan(Ctx* c, Plan* p, const SlhaB200Segment* segs, size_t n_se
     p->d_cta_begin = !wide && p->n_items == p->mma_grid ? nullptr : reinterpret_cast<uint32_t*>(dev + o_nc);  // (null: an item a CTA)
     p->d_rows = reinterpret_cast<RowInfo*>(dev + o_r);
     p->d_streams = streams.all.empty() ? p->d_items : reinterpret_cast<WorkItem*>(dev + o_s);
-    p->d_stream_at = reinterpret_cast<uint2*>(dev + o_sa);
-    p->n_streams = (uint32_t)streams.at.size() - 1;
-    p->unit_share = streams.share;
+    p->n_streams = streams.n;
     p->streams_grid = streams.grid;
     p->longest = longest;
     p->rows = true;
@@ -1047,7 +1044,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     for (size_t i = 0; i < n_segs; ++i) cuts.add(segs[i], wide ? WIDE_NQ : 4);
     cuts.finish();
     Streams streams;
-    if (wide) streams.make(cuts.items, sms, 4);
+    if (wide) streams.make(cuts.items, sms);
     std::vector<WorkItem> generic;  // runs of 4096 tiles where score_kernel takes the call
     if (g_force_generic)
         for (const WorkItem& s : cuts.items)
@@ -1061,7 +1058,7 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
     Blob blob;
     const size_t o_items = blob.add(cuts.items), o_cta = blob.add(cuts.cta), o_gen = blob.add(generic);
     const size_t o_tail = fills ? blob.add(tail) : 0;
-    const size_t o_s = streams.all.empty() ? o_items : blob.add(streams.all), o_sa = wide ? blob.add(streams.at) : 0;
+    const size_t o_s = streams.all.empty() ? o_items : blob.add(streams.all);
     const size_t o_rows = check ? 0 : blob.add(std::vector<uint64_t>(row_offsets, row_offsets + nq));
     const size_t o_flag = wide ? blob.add_zeros(nq + 1) : 0;
     unsigned char* dev;
@@ -1093,9 +1090,8 @@ Status launch_score_segments(Ctx* c, const SciRustSlhaTile* tiles, const SlhaB20
         SLHA_TRY(launch_wide_dense(c, a, grid, true));
         a.only_flagged = a.handoff;
         a.streams = reinterpret_cast<const WorkItem*>(dev + o_s);
-        a.stream_at = reinterpret_cast<const uint2*>(dev + o_sa);
-        a.n_streams = (uint32_t)streams.at.size() - 1;
-        a.unit_share = streams.share;
+        a.n_streams = streams.n;
+        a.least_share = 4u;
     } else if (a.n_items == grid) {
         a.cta_begin = nullptr;
     }
@@ -1133,9 +1129,8 @@ static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, con
         SLHA_TRY(launch_wide_dense(c, a, p->mma_grid, true));
         a.only_flagged = a.handoff;
         a.streams = p->d_streams;
-        a.stream_at = p->d_stream_at;
         a.n_streams = p->n_streams;
-        a.unit_share = p->unit_share;
+        a.least_share = 1u;
     }
     SLHA_TRY(launch_dense(c, a, p->wide ? p->streams_grid : p->mma_grid, true));
     if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));

@@ -314,7 +314,8 @@ struct TileCta {
     uint32_t phase;    // of the warpgroup's mbarrier
     bool failed;       // a wait of this warp ran out
     bool undone;       // dense: an item was left, see undone_add
-    uint32_t stream;   // of the item (PASS)
+    PassWalk walk;     // PASS: where the item lies, of range
+    const PassRange* range;
 };
 template <bool DENSE>
 struct TileLayout {
@@ -351,7 +352,8 @@ __device__ __forceinline__ TileCta tile_open(unsigned char* smem_raw) {
     t.table = false;
     t.phase = 0u;
     t.failed = t.undone = false;
-    t.stream = 0u;
+    t.walk = PassWalk{};
+    t.range = nullptr;
     return t;
 }
 __device__ __forceinline__ void tile_close(const TileCta& t) {
@@ -421,9 +423,17 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
     bool failed = cta.failed;
 
     auto next_item = [&]() {  // false at the end, or at an item of another kind (the same in the whole CTA)
-        if (++item_id >= item_end) return false;
-        if (PASS && item_id >= a.stream_at[cta.stream + 1u].x) ++cta.stream;  // (every stream has a group)
-        it = DENSE ? dense_item<PASS>(a, item_id, cta.stream) : a.stream_items[item_id];
+        if (PASS) {
+            if (!pass_next(a, *cta.range, cta.walk)) {
+                item_id = item_end;
+                return false;
+            }
+            ++item_id;
+            it = pass_item(a, *cta.range, cta.walk);
+        } else {
+            if (++item_id >= item_end) return false;
+            it = a.stream_items[item_id];
+        }
         if (KINDS) flags0 = first_tile_flags(a, it);
         return !KINDS || item_kind(flags0, nf4_too) == KIND;
     };
@@ -449,13 +459,16 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             if (j >= my_rounds) j -= my_rounds;
             return (j * il_n + il_c) * (uint32_t)NWG + (uint32_t)wg;
         };
-        if (PASS) {  // only the items one of whose rows the first pass handed over
+        auto leave = [&]() {
+            const uint32_t bit = undone_bit(PASS ? item_id : item_id - dense_first(a));
+            reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE)[bit >> 5] |= 1u << (bit & 31u);
+        };
+        if (PASS) {  // (a group one of whose rows the 64-row kernel handed on)
             uint32_t f = 0;
             for (int q = 0; q < nq; ++q) f |= a.only_flagged[it.query_begin + q];
-            if (!f) continue;  // (the same in the whole CTA)
-            if (f & 2u) {
+            if (f & 2u) {  // (the same in the whole CTA)
                 if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
-                if (tid == 0) undone_add<PASS>(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
+                if (tid == 0) leave();
                 cta.undone = true;
                 continue;
             }
@@ -861,7 +874,7 @@ __device__ __forceinline__ uint32_t tile_run(const ScoreArgs& a, TileCta& cta, u
             // rows this CTA could not score on the tensor cores go to the generic kernel as a whole; of dense calls the item, at the CTA's end
             if (a.gflag && tid < nq) a.gflag[it.query_begin + tid] = 1u;
             if (DENSE) {
-                if (tid == 0) undone_add<PASS>(a, reinterpret_cast<uint32_t*>(base + TileLayout<true>::UNDONE), item_id);
+                if (tid == 0) leave();
                 cta.undone = true;
             }
         }
@@ -900,28 +913,23 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     dep_launch();
     dep_wait();
     if (a.refused && *a.refused) return;
-    if (PASS && !*a.handoff_any) return;
-    uint32_t i = dense_first<PASS>(a);
-    const uint32_t item_end = dense_end<PASS>(a);
-    if (PASS) {  // (with nothing to do a CTA ends here)
-        uint32_t f = 0;
-        for (uint32_t e = i + threadIdx.x; e < item_end; e += ST_THREADS) {
-            const WorkItem own = dense_item<PASS>(a, e, dense_stream<false>(a, e));
-            for (uint32_t q = 0; q < own.n_queries; ++q) f |= a.only_flagged[own.query_begin + q];
-        }
-        if (!__syncthreads_or(f != 0u)) return;
-    }
-    const uint32_t stream = PASS ? dense_stream<false>(a, i) : 0u;
-    WorkItem it = dense_item<PASS>(a, i, stream);
+    __shared__ PassRange range;
+    if (PASS && (!*a.handoff_any || !pass_range(a, range))) return;
+    uint32_t i = PASS ? 0u : dense_first(a);  // PASS: counted
+    const uint32_t first = i, item_end = PASS ? 0xFFFFFFFFu : dense_end(a);
+    PassWalk walk{};
+    if (PASS) walk = pass_first(a, range);
+    WorkItem it = PASS ? pass_item(a, range, walk) : a.stream_items[i];
     uint32_t flags = first_tile_flags(a, it);  // (on its way while the CTA is set up, and the first item's queries with it)
     if (threadIdx.x < 4u * it.n_queries) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_coarse + (size_t)it.query_begin * D_C + 32u * threadIdx.x));
     if (threadIdx.x == 32) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.q_sign + (size_t)it.query_begin * 8));
     if (threadIdx.x == 64 && a.row_offset) asm volatile("prefetch.global.L1 [%0];\n" ::"l"(a.row_offset + it.query_begin));
     const bool nf4_too = a.nf4_table == 1u || (a.nf4_table == 2u && (first_tile_flags(a, a.stream_items[0]) & F_NF4));
     uint32_t* const bits = reinterpret_cast<uint32_t*>(tile_base(smem_raw) + TileLayout<true>::UNDONE);
-    for (uint32_t w = threadIdx.x; w < min((item_end - i + 31u) / 32u, (uint32_t)UNDONE_WORDS); w += ST_THREADS) bits[w] = 0u;  // (ordered by tile_open's barrier)
+    for (uint32_t w = threadIdx.x; w < min(((PASS ? range.end - range.mine : item_end - first) + 31u) / 32u, (uint32_t)UNDONE_WORDS); w += ST_THREADS) bits[w] = 0u;  // (ordered by tile_open's barrier)
     TileCta cta = tile_open<true>(smem_raw);
-    cta.stream = stream;
+    cta.walk = walk;
+    cta.range = &range;
     for (;;) {
         switch (item_kind(flags, nf4_too)) {
             case 0: i = tile_run<0, false, true, true, PASS>(a, cta, i, item_end, it, flags, nf4_too); break;
@@ -934,7 +942,7 @@ __global__ void __launch_bounds__(ST_THREADS, 1) score_dense_kernel(const __grid
     }
     tile_close(cta);
     static_assert(4096 + (ST_THREADS / 32) * BLK_BYTES <= TileLayout<true>::UNDONE, "below the bits");
-    if (cta.undone) finish_undone<PASS>(a, bits, smem_raw);
+    if (cta.undone) finish_undone<PASS>(a, bits, &range, smem_raw);
 }
 
 }  // namespace

@@ -452,3 +452,33 @@ def test_segments_that_continue_one_another_in_the_tiles_but_not_in_the_row():
         for j in range(q0, q0 + q, 5):
             want = ora.score_tiles(tiles[tb:tb + m], qc[j], qs[j])
             assert np.all(np.abs(out[j, base:base + m] - want) <= 1e-3 * (1 + np.abs(want)))
+
+
+@pytest.mark.parametrize("n_seg,longest,share", [(40, 3000, 0.5), (700, 200, 0.3), (9, 20000, 0.12), (600, 40, 1.0)])
+def test_what_was_handed_on_is_shared_out_whatever_lies_between(n_seg, longest, share):
+    # segments of 16 to 70 rows, some of them NF4 (handed on by the 64-row kernel): those give what the same rows give in fours, bit for bit, the others the oracle's scores
+    rng = np.random.default_rng(n_seg)
+    nf4 = rng.random(n_seg) < share
+    base = {c: H.random_tiles(1000, c, seed=570 + c, warm_every=9) for c in (0, 2, 3, 5)}
+    rows, fours, parts, tb, qb = [], [], [], 0, 0
+    for i in range(n_seg):
+        n, nq = int(rng.integers(1, longest + 1)), int(rng.choice([16, 17, 40, 64, 70]))
+        parts.append(base[2 if nf4[i] else int(rng.choice([0, 3, 5]))][rng.integers(0, 1000, n)])
+        rows.append((tb, n, qb, nq, 0))
+        fours += [(tb, n, qb + q, min(4, nq - q), 0) for q in range(0, nq, 4)]
+        tb, qb = tb + n, qb + nq
+    tiles = np.concatenate(parts)
+    qc, qs = (np.resize(x, (qb,) + x.shape[1:]) for x in H.random_queries(211, 571))
+    row_len = max(r[1] for r in rows)
+    off = np.arange(qb, dtype=np.uint64) * row_len
+    dt = S.to_device(tiles)
+    out = S.score_segments(dt, S.make_segments(rows), qc, qs, qb, np.zeros((qb, row_len), F), off, row_len)
+    want = S.score_segments(dt, S.make_segments(fours), qc, qs, qb, np.zeros((qb, row_len), F), off, row_len)
+    of_nf4 = np.repeat(nf4, [r[3] for r in rows])
+    assert out[of_nf4].tobytes() == want[of_nf4].tobytes()
+    assert np.all(np.abs(out - want) <= 1e-4 * (1 + np.abs(want)))
+    for i in range(0, n_seg, max(1, n_seg // 12)):
+        t, n, q0, nq, _ = rows[i]
+        for j in (q0, q0 + nq - 1):
+            s = ora.score_tiles(tiles[t:t + n], qc[j], qs[j])
+            assert np.all(np.abs(out[j, :n] - s) <= 1e-3 * (1 + np.abs(s))) and np.all(out[j, n:] == 0)
