@@ -484,7 +484,7 @@ typedef struct SlhaB200Pool SlhaB200Pool;
 #define SLHA_B200_EVICT_IMPORTANCE 1
 
 typedef struct {
-    uint64_t capacity_tiles; /* slots reserved in HBM (128 B tile + 13 B bookkeeping each) */
+    uint64_t capacity_tiles; /* slots reserved in HBM (128 B tile + 21 B bookkeeping each) */
     uint64_t budget_bytes;   /* logical byte budget of enforce_budget */
     int32_t page_policy;
     int32_t evict_policy;

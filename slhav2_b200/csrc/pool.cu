@@ -1156,7 +1156,7 @@ __global__ void observe_pass3(PoolDev p, const uint32_t* slots, const float* sco
 // The three passes over all slots (observe_query) in one: a thread keeps its entries' terms and importances in registers between two grid barriers.  The shares, and so
 // the order of the sum, are pass 2's: half a CTA is one of its 256.  Latency bounds it, three loads' and two barriers': a million slots 22 us with the clear
 // and the three kernels, 13 with this one.
-constexpr int OBSERVE_PARTS = 256, OBSERVE_KEEP = 16;  // entries a thread, so up to 1 048 576 slots
+constexpr int OBSERVE_PARTS = 256, OBSERVE_KEEP = 16;  // entries a thread: up to 1 048 576 slots, since the parts of the sum, and with them its order, stay pass 2's 256
 __global__ void __launch_bounds__(512) observe_all_kernel(PoolDev p, const float* scores, uint64_t n, float temperature, ObserveTmp* tmp, float* partial) {
     cooperative_groups::grid_group grid = cooperative_groups::this_grid();
     __shared__ uint32_t red[3];

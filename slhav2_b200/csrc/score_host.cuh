@@ -350,6 +350,8 @@ struct Streams {
 //   NF4 126 / 114, 127 / 122, 143 / 140; 48 of 32 768 INT4 76 / 72, 79 / 85, 86 / 103, NF4 105 / 87, 109 / 99, 116 / 117; 96 of 32 768 INT4 131 / 114, 135 / 133, 147 / 157,
 //   mixed 129 / 124, 133 / 136, 144 / 157; 400 of 8192 INT4 141 / 165, 142 / 191, 181 / 234, NF4 201 / 186, 201 / 214, 241 / 256; 1000 of 4096 INT4 198 / 253,
 //   200 / 308, 245 / 396, NF4 272 / 294, 273 / 369, 318 / 475.
+// Up to 640 000 passes (1 280 000 from k = 512) whole rows are the faster ones however few they are: 19 x 32 768 tiles, one row each, k = 64, 1024 INT4 34 / 45, 37 / 78, NF4 45 / 47, 49 / 79;
+// 38 x 32 768, k = 512, 1024 INT4 50 / 94, 52 / 107, NF4 71 / 111, 73 / 131.  (Above, at k = 64, INT4 67 streamed, NF4 74.)
 enum RowsRule { ROWS_NO, ROWS_YES, ROWS_UNLESS_NF4 };
 RowsRule rows_rule(uint64_t passes, bool wide, size_t nq, uint32_t longest, uint32_t k) {
     const uint64_t unit = wide ? WIDE_M : 32;  // (the 64-row kernel writes blocks of 128 scores)

@@ -7,7 +7,7 @@
 // and those are compacted: up to ROW_RANKED are ordered by comparing each with all, more by buckets between the bound and the largest score of the
 // sample and by comparing inside a bucket, or, where that is crowded (equal scores, one far from the rest), by a radix sort.
 // Bound: the latencies between the block barriers, and for many rows the instructions a score costs.  us a call, streamed and merged / whole rows: 4096
-// INT4 tiles, k = 64 19.6 / 10.6, 8 x 8192 mixed tiles x 4 rows, k = 256 26.6 / 13.2, 8 x 16 384 TQ3 x 64 rows 85 / 47; the kernel itself about 8 us of the last.  With the
+// INT4 tiles, k = 64 19.6 / 10.6, 8 x 8192 mixed tiles x 4 rows, k = 256 26.6 / 13.0, 8 x 16 384 TQ3 x 64 rows 85 / 47 (with events between the two 34 of scores, 22 of selection).  With the
 // candidates ordered by buckets alone 13.6 and 48.1; with a histogram of the whole row in place of the sample 20 us for 512 rows of 16 384.
 #pragma once
 

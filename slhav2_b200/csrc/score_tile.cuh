@@ -6,13 +6,12 @@
 // the queries (scaled to one size, fp16 hi + lo columns, 22 bits or more) and the thread reads its finished coarse scores back.  Scale, lambda, flags
 // and scale bytes are each read by one thread, where the fragments of warp-level MMAs need them in four lanes each.
 //
-// Bound: the chain of a block (decode, TMEM store, eight or nine MMAs, read-back, filter or finish), 4000 cycles (MIX3 5200, NF4 6700) with four warpgroups in
-// flight, of which the instructions take 1700.  Dense scores of 8 x 131 072 mixed tiles, 4 rows: 4820 cycles a round -> 4020, one row 4250 -> 3330, an item's set-up 4900 ->
-// 3000, by the sums in pairs (f32x2), full adders in front of POPC, row addresses and slot states read ahead, the queries asked for before the tiles.
-// MIX3 top-k of 32 ragged segments (485 k tiles x 4 queries): 367 -> 72 us a call streamed (dense scores and a selection: 42); dense MIX3 scores of 8 x 4096
+// Bound: the chain of a block (decode, TMEM store, eight or nine MMAs, read-back, filter or finish) with four warpgroups in flight; a scheduler issues in 47 % of the cycles.  Dense scores
+// of 8 x 131 072 tiles, us a call for 4 rows / one: mixed 56 / 50 -> 42 / 36, NF4 78 / 72 -> 63 / 54, MIX3 65 / 60 -> 48 / 43 by the sums in pairs (f32x2), full adders in front of
+// POPC, row addresses and slot states read ahead, the queries asked for before the tiles.
+// MIX3 top-k of 32 ragged segments (485 k tiles x 4 queries): 367 -> 72 us a call streamed (dense scores and a selection: 40); dense MIX3 scores of 8 x 4096
 // tiles x 4 rows: 278 -> 17 us a call (6 of kernel).  Top-k of the codecs that score_stream_kernel
-// decodes, over long rows, stays there: with this kernel a call took 301 us against 292 us on 8.4 M MX-INT4 tiles and 573 us against 462 us on as many
-// NF4 tiles.
+// decodes, over long rows, stays there: on 8.4 M MX-INT4 tiles a call takes 308 us with this kernel and 237 with that one, on as many NF4 tiles earlier forms of both took 573 and 462.
 #pragma once
 
 namespace slha {
