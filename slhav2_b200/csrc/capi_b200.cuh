@@ -267,7 +267,9 @@ int32_t slha_b200_score_segments(const SciRustSlhaTile* tiles, const SlhaB200Seg
         if (dev_off && !st.ok()) {  // (what else was wrong is reported behind the offsets)
             bool bad;
             if (!check.launched) SLHA_TRY(launch_row_check(c, &check));
-            if (checked_offsets(c, check, &bad).ok() && bad) return Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+            if (checked_offsets(c, check, &bad).ok() && bad) st = Status(SLHA_ERR_DIMENSION, "slha_b200_score_segments: a row reaches beyond scores_len");
+            // (the kernels behind the check still read the thread's scratch, which a call on another stream only waits for where it was a caller's stream)
+            if (sync_by_default(c)) SLHA_CUDA(cudaStreamSynchronize(c->stream));
         }
         return st;
     });

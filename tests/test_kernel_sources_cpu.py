@@ -41,3 +41,12 @@ def test_a_kernel_whose_answer_the_host_polls_has_met_at_a_barrier_before_it_ans
         for m in re.finditer(answer, body):
             block = body[:m.start()]
             assert ".sync()" in block, (kernel, body[m.start():m.start() + 60])
+
+
+def test_a_dense_call_that_is_refused_drains_the_library_s_stream():
+    # Its kernels end on the check's word in the thread's scratch, which the thread's next call on another stream may write.
+    text = dict(_sources())["capi_b200.cuh"]
+    body = text[text.index("int32_t slha_b200_score_segments("):]
+    body = body[:body.index("\n}\n")]
+    refused = body[body.rindex("checked_offsets("):]
+    assert "return Status" not in refused and re.search(r"sync_by_default\(c\)\) SLHA_CUDA\(cudaStreamSynchronize", refused)
