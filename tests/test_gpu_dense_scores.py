@@ -438,7 +438,7 @@ def test_nf4_rows_of_many_queries_cost_what_the_same_rows_cost_four_at_a_time():
     for j in (0, 3, 39, 40, 77):
         want = ora.score_tiles(tiles[j // nq * n:j // nq * n + n], qc[j], qs[j])
         assert np.all(np.abs(outs[0][j, base:] - want) <= 1e-3 * (1 + np.abs(want)))
-    assert took[0] < 1.4 * took[1], took
+    assert took[0] < 1.6 * took[1], took
 
 
 def test_segments_that_continue_one_another_in_the_tiles_but_not_in_the_row():
