@@ -454,9 +454,10 @@ def test_segments_that_continue_one_another_in_the_tiles_but_not_in_the_row():
             assert np.all(np.abs(out[j, base:base + m] - want) <= 1e-3 * (1 + np.abs(want)))
 
 
-@pytest.mark.parametrize("n_seg,longest,share", [(40, 3000, 0.5), (700, 200, 0.3), (9, 20000, 0.12), (600, 40, 1.0)])
-def test_what_was_handed_on_is_shared_out_whatever_lies_between(n_seg, longest, share):
-    # segments of 16 to 70 rows, some of them NF4 (handed on by the 64-row kernel): those give what the same rows give in fours, bit for bit, the others the oracle's scores
+@pytest.mark.parametrize("n_seg,longest,share,huge", [(40, 3000, 0.5, 0), (700, 200, 0.3, 0), (9, 20000, 0.12, 0), (600, 40, 1.0, 0), (12, 9000, 0.3, 0.5), (800, 150, 0.1, 0.2), (1, 700, 0, 1), (3, 16384, 0, 1)])
+def test_what_was_handed_on_is_shared_out_whatever_lies_between(n_seg, longest, share, huge):
+    # segments of 16 to 70 rows, some of them NF4, some with a query row beyond the fp16 split (handed on by the 64-row kernel, in groups of unequal cost): those give what the same rows give in
+    # fours, bit for bit, the others the oracle's scores
     rng = np.random.default_rng(n_seg)
     nf4 = rng.random(n_seg) < share
     base = {c: H.random_tiles(1000, c, seed=570 + c, warm_every=9) for c in (0, 2, 3, 5)}
@@ -469,16 +470,24 @@ def test_what_was_handed_on_is_shared_out_whatever_lies_between(n_seg, longest, 
         tb, qb = tb + n, qb + nq
     tiles = np.concatenate(parts)
     qc, qs = (np.resize(x, (qb,) + x.shape[1:]) for x in H.random_queries(211, 571))
+    far, of_far = [], np.zeros(qb, bool)
+    for i in np.flatnonzero(rng.random(n_seg) < huge):
+        j = int(rng.integers(0, rows[i][3]))
+        far.append(rows[i][2] + j)
+        qc[far[-1], int(rng.integers(0, 100))] = rng.choice([1e30, -np.inf, np.nan])
+        of_far[rows[i][2] + j // 64 * 64:min(rows[i][2] + j // 64 * 64 + 64, rows[i][2] + rows[i][3])] = True
     row_len = max(r[1] for r in rows)
     off = np.arange(qb, dtype=np.uint64) * row_len
     dt = S.to_device(tiles)
     out = S.score_segments(dt, S.make_segments(rows), qc, qs, qb, np.zeros((qb, row_len), F), off, row_len)
     want = S.score_segments(dt, S.make_segments(fours), qc, qs, qb, np.zeros((qb, row_len), F), off, row_len)
     of_nf4 = np.repeat(nf4, [r[3] for r in rows])
-    assert out[of_nf4].tobytes() == want[of_nf4].tobytes()
-    assert np.all(np.abs(out - want) <= 1e-4 * (1 + np.abs(want)))
+    handed = of_nf4 | of_far
+    assert out[handed].tobytes() == want[handed].tobytes()
+    usual = np.setdiff1d(np.arange(qb), far)
+    assert np.all(np.abs(out[usual] - want[usual]) <= 1e-4 * (1 + np.abs(want[usual])))
     for i in range(0, n_seg, max(1, n_seg // 12)):
         t, n, q0, nq, _ = rows[i]
-        for j in (q0, q0 + nq - 1):
+        for j in set((q0, q0 + nq - 1)) - set(far):
             s = ora.score_tiles(tiles[t:t + n], qc[j], qs[j])
             assert np.all(np.abs(out[j, :n] - s) <= 1e-3 * (1 + np.abs(s))) and np.all(out[j, n:] == 0)
