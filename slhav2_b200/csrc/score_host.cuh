@@ -1136,7 +1136,7 @@ static Status score_topk_rows(Ctx* c, Plan* p, const SciRustSlhaTile* tiles, con
     }
     SLHA_TRY(launch_dense(c, a, p->wide ? p->streams_grid : p->mma_grid, true));
     if (timed) SLHA_CUDA(cudaEventRecord(tev[1], c->stream));
-    RowsArgs r{a.scores, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, p->kp2, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
+    RowsArgs r{a.scores, p->d_rows, p->d_row_flags, p->d_row_flags + 2 * nq, k, row_cap(k, p->kp2), d_out_index, d_out_score, d_out_count};
     SLHA_TRY(launch_rows(c, r, (uint32_t)nq, p->longest));
     if (timed) {
         SLHA_CUDA(cudaEventRecord(tev[2], c->stream));

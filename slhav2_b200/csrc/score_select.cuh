@@ -26,12 +26,12 @@ struct RowsArgs {
     const RowInfo* rows;
     uint32_t* flag;          // [nq] a work item of the row took the generic arithmetic, [nq] it was handed on by the 64-row kernel, [4 nq] whether any was (cleared here)
     uint32_t* stats;         // [nq][2] candidates, the flag
-    uint32_t k, kp2, cap;    // cap: slots for candidates, row_cap(k, kp2)
+    uint32_t k, cap;         // cap: slots for candidates, row_cap
     uint32_t* out_index;
     float* out_score;
     uint32_t* out_count;
 };
-// slots: what a sample's bound lets through, see below, and kp2 winners
+// slots: what a sample's bound lets through, see below, and k rounded up to a power of two at least
 inline uint32_t row_cap(uint32_t k, uint32_t kp2) { return std::max(kp2, std::min(4u * k + 1024u, 2u * k + 2560u)); }
 constexpr int ROW_HIST_INTS = ROW_BUCKETS + 64;
 // (the threads' own lists make room for the candidates by buckets)
